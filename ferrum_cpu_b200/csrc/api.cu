@@ -97,9 +97,9 @@ struct fc_qweight {
     int device;
     Arena arena;
     QMat w;
-    // scratch of the tensor-core path: bf16 hi / lo planes of the activations, status word
+    // scratch of the M >= 2 product: bf16 planes of the activations, status word
     Arena planes;
-    uint16_t *xhi = nullptr, *xlo = nullptr;
+    Planes x;
     int* status = nullptr;
     size_t plane_elems = 0;
 };
@@ -154,15 +154,12 @@ struct fc_model {
     float *lnfg = nullptr, *lnfb = nullptr;
     std::vector<LayerDev> layers;
     // prefill workspace for ws_rows rows
-    int ws_rows = 0, head_chunk = 0;
-    float *x = nullptr, *n = nullptr, *qkv = nullptr, *att = nullptr, *hid = nullptr, *logits = nullptr, *probs_d = nullptr;
+    int ws_rows = 0, ws_planes = 0;
+    float *x = nullptr, *n = nullptr, *qkv = nullptr, *att = nullptr, *logits = nullptr, *probs_d = nullptr;
     int *ids_d = nullptr, *targets_d = nullptr, *err_d = nullptr;
     double* lp_d = nullptr;
     uint8_t* gr_d = nullptr;
-    uint16_t *xhi = nullptr, *xlo = nullptr;   // bf16 planes of the current GEMM input
-    // tensor path: bf16 hi / lo planes of LayerNorm output, qkv, attention output, GELU output
-    uint16_t *nhi = nullptr, *nlo = nullptr, *qkvhi = nullptr, *qkvlo = nullptr;
-    uint16_t *atthi = nullptr, *attlo = nullptr, *hidhi = nullptr, *hidlo = nullptr;
+    Planes pn, pqkv, patt, phid;               // bf16 planes of LayerNorm output, qkv, attention output, GELU output
     void* head_stats = nullptr;                // fused head: per (row, 128-column tile) softmax records, 16 B each
     float* head_tlogit = nullptr;              // ... and the logit of each row's target
     int* tc_status = nullptr;                  // raised by a scoring kernel (tensor-core GEMM, attention, row tail) on a timeout
@@ -344,134 +341,111 @@ static int check_ids(const fc_model* m, const int32_t* ids, size_t n) {
 }
 
 // -------------------------------------------------------------------- prefill workspace
-static bool tensor_path(const fc_model* m);
-static int ensure_workspace(fc_model* m, int rows) {
-    if (rows <= m->ws_rows) return FC_OK;
+// bf16 planes a window forward splits its activations into: 3 hold an f32 exactly (FC_MATH_FP32), 2 to 2^-17 relative
+// (FC_MATH_BF16X3, for matrices whose rows are whole 64-wide k-blocks).
+static int model_planes(const fc_model* m) {
+    const fc_config& c = m->cfg;
+    return c.math_mode == FC_MATH_BF16X3 && c.d_model % 64 == 0 && c.d_ff % 64 == 0 ? 2 : 3;
+}
+// Whether the attention of a forward with `planes` planes runs on the tensor cores (heads of 64, two planes).
+static bool tensor_attention(const fc_model* m, int planes) { return planes == 2 && m->cfg.d_model == m->cfg.n_head * 64; }
+
+static int ensure_workspace(fc_model* m, int rows, int planes) {
+    if (rows <= m->ws_rows && planes <= m->ws_planes) return FC_OK;
+    rows = std::max(rows, m->ws_rows);
+    planes = std::max(planes, m->ws_planes);
+    FC_CUDA(cudaStreamSynchronize(m->st));
     m->ws_arena.release();
-    m->ws_rows = 0;
+    m->ws_rows = m->ws_planes = 0;
     const fc_config& c = m->cfg;
     const size_t R = rows, d = c.d_model, F = c.d_ff;
-    // fp32 mode: head logits are produced for head_chunk rows at a time (<= 1 GiB of f32). On the tensor-core
-    // path the head never writes logits (its epilogue leaves softmax records): one row is kept for predict_next.
-    size_t chunk = ((size_t)1 << 28) / (size_t)c.vocab;
-    chunk = std::max<size_t>(1, std::min<size_t>(chunk, R));
-    if (tensor_path(m)) chunk = 1;
     Arena& a = m->ws_arena;
     FC_TRY(a.alloc_n(&m->x, R * d));
-    FC_TRY(a.alloc_n(&m->n, R * d));
+    FC_TRY(a.alloc_n(&m->n, d));                            // predict_next: the last row through the final LayerNorm,
+    FC_TRY(a.alloc_n(&m->logits, (size_t)m->head.N_pad));   // and its logits
     FC_TRY(a.alloc_n(&m->qkv, R * 3 * d));
     FC_TRY(a.alloc_n(&m->att, R * d));
-    FC_TRY(a.alloc_n(&m->hid, R * F));
-    FC_TRY(a.alloc_n(&m->logits, chunk * (size_t)m->head.N_pad));
     FC_TRY(a.alloc_n(&m->ids_d, R));
     FC_TRY(a.alloc_n(&m->targets_d, R));
     FC_TRY(a.alloc_n(&m->lp_d, R));
     FC_TRY(a.alloc_n(&m->gr_d, R));
     FC_TRY(a.alloc_n(&m->err_d, 1));
     FC_TRY(a.alloc_n(&m->probs_d, (size_t)c.vocab));
-    if (c.math_mode == FC_MATH_BF16X3) {
-        // bf16 hi / lo planes of the widest GEMM input, and the kernel's status word
-        FC_TRY(a.alloc_n(&m->xhi, R * std::max(d, F)));
-        FC_TRY(a.alloc_n(&m->xlo, R * std::max(d, F)));
-        if (tensor_path(m)) {
-            FC_TRY(a.alloc_n(&m->nhi, R * d));       FC_TRY(a.alloc_n(&m->nlo, R * d));
-            FC_TRY(a.alloc_n(&m->qkvhi, R * 3 * d)); FC_TRY(a.alloc_n(&m->qkvlo, R * 3 * d));
-            FC_TRY(a.alloc_n(&m->atthi, R * d));     FC_TRY(a.alloc_n(&m->attlo, R * d));
-            FC_TRY(a.alloc_n(&m->hidhi, R * F));     FC_TRY(a.alloc_n(&m->hidlo, R * F));
-            FC_TRY(a.alloc(&m->head_stats, R * (size_t)((c.vocab + 127) / 128) * 16));
-            FC_TRY(a.alloc_n(&m->head_tlogit, R));
-        }
-    }
+    auto make = [&](Planes* p, size_t n) -> int {
+        for (int i = 0; i < planes; ++i) FC_TRY(a.alloc(&p->p[i], n * 2));
+        return FC_OK;
+    };
+    FC_TRY(make(&m->pn, R * d));
+    FC_TRY(make(&m->pqkv, R * 3 * d));
+    FC_TRY(make(&m->patt, R * d));
+    FC_TRY(make(&m->phid, R * F));
+    FC_TRY(a.alloc(&m->head_stats, R * (size_t)((c.vocab + 127) / 128) * 16));
+    FC_TRY(a.alloc_n(&m->head_tlogit, R));
     FC_TRY(a.alloc_n(&m->tc_status, 1));
     FC_CUDA(cudaMemsetAsync(m->tc_status, 0, sizeof(int), m->st));
     m->ws_rows = rows;
-    m->head_chunk = (int)chunk;
+    m->ws_planes = planes;
     return FC_OK;
 }
 
-static int gemm(fc_model* m, const QMat& w, const float* x, const float* bias, const float* res, int epi, float* y, int M, int ldy) {
-    // FC_MATH_BF16X3: split the activations into bf16 hi/lo planes, then the tcgen05 kernel
-    // (its k-blocks are 64 wide). FC_MATH_FP32, or a K that is not a multiple of 64: the
-    // fp32 CUDA-core kernel.
-    if (m->cfg.math_mode == FC_MATH_BF16X3 && w.K % 64 == 0) {
-        FC_TRY(launch_split_bf16(x, m->xhi, m->xlo, (size_t)M * w.K, m->st));
-        return launch_gemm_q8_bf16x3(w, m->xhi, m->xlo, bias, res, epi, y, M, ldy, m->tc_status, m->st);
-    }
-    return launch_gemm_q8_fp32(w, x, bias, res, epi, y, M, ldy, m->st);
-}
-
-// True when the whole window forward runs on tensor cores with bf16-plane activations.
-static bool tensor_path(const fc_model* m) {
-    const fc_config& c = m->cfg;
-    return c.math_mode == FC_MATH_BF16X3 && c.d_model == c.n_head * 64 && c.d_model % 64 == 0 && c.d_ff % 64 == 0;
-}
-
-// Sequential::forward (model.rs:51-71) through every block, on B windows of T rows whose ids
-// are already in m->ids_d. Leaves the residual stream in m->x.
-static int forward_blocks(fc_model* m, int B, int T) {
+// Sequential::forward (model.rs:51-71) through every block, on B windows of T rows whose ids are already in m->ids_d.
+// Leaves the residual stream in m->x. Between kernels activations are bf16 planes; only the residual stream is f32.
+// split_k: see launch_gemm_q8_tc. f32_qkv: the QKV product is written as f32 rows to m->qkv and on_qkv(layer) is called before the attention.
+template <class OnQkv>
+static int forward_blocks_with(fc_model* m, int B, int T, int planes, int* status, bool split_k, bool f32_qkv, OnQkv on_qkv) {
     const fc_config& c = m->cfg;
     const int R = B * T, d = c.d_model, F = c.d_ff;
     cudaStream_t st = m->st;
+    const bool tc_attn = tensor_attention(m, planes);
+    m->pn.n = m->pqkv.n = m->patt.n = m->phid.n = planes;
     FC_CUDA(cudaMemsetAsync(m->err_d, 0, sizeof(int), st));
     FC_TRY(launch_embed_rows(m->tok, m->pos, m->ids_d, R, T, m->x, m->err_d, st));
     // model.rs:58-68: with the statistics switched on, every layer's output is summarised as it appears
     m->stats_n = 0;
     auto layer_stats = [&]() -> int {
         if (!m->stats_on) return FC_OK;
-        return launch_layer_stats(m->x, nullptr, nullptr, (size_t)R * d, m->stats_scratch, m->stats_d + m->stats_n++, st);
+        return launch_layer_stats(m->x, Planes(), (size_t)R * d, m->stats_scratch, m->stats_d + m->stats_n++, st);
     };
     FC_TRY(layer_stats());
-    if (tensor_path(m)) {
-        // activations between kernels are bf16 hi / lo planes; only the residual stream is f32
-        for (int l = 0; l < c.n_layer; ++l) {
-            const LayerDev& L = m->layers[l];
-            FC_TRY(launch_layernorm_planes(m->x, L.ln1g, L.ln1b, R, d, m->nhi, m->nlo, st));
-            FC_TRY(launch_gemm_q8_bf16x3_ex(L.qkv, m->nhi, m->nlo, L.qkv_b, nullptr, EPI_NONE, nullptr, m->qkvhi, m->qkvlo, R, 3 * d, m->tc_status, st));
-            FC_TRY(launch_attn_prefill_tc(m->qkvhi, m->qkvlo, B, T, d, c.n_head, m->atthi, m->attlo, m->tc_status, st));
-            FC_TRY(launch_gemm_q8_bf16x3_ex(L.out, m->atthi, m->attlo, L.out_b, m->x, EPI_NONE, m->x, nullptr, nullptr, R, d, m->tc_status, st));
-            FC_TRY(launch_layernorm_planes(m->x, L.ln2g, L.ln2b, R, d, m->nhi, m->nlo, st));
-            FC_TRY(launch_gemm_q8_bf16x3_ex(L.up, m->nhi, m->nlo, L.up_b, nullptr, EPI_GELU, nullptr, m->hidhi, m->hidlo, R, F, m->tc_status, st));
-            FC_TRY(launch_gemm_q8_bf16x3_ex(L.down, m->hidhi, m->hidlo, L.down_b, m->x, EPI_NONE, m->x, nullptr, nullptr, R, d, m->tc_status, st));
-            FC_TRY(layer_stats());
-        }
-        return FC_OK;
-    }
     for (int l = 0; l < c.n_layer; ++l) {
         const LayerDev& L = m->layers[l];
-        FC_TRY(launch_layernorm(m->x, L.ln1g, L.ln1b, R, d, m->n, nullptr, st));
-        FC_TRY(gemm(m, L.qkv, m->n, L.qkv_b, nullptr, EPI_NONE, m->qkv, R, 3 * d));
-        FC_TRY(launch_attn_prefill(m->qkv, B, T, d, c.n_head, m->att, st));
-        FC_TRY(gemm(m, L.out, m->att, L.out_b, m->x, EPI_NONE, m->x, R, d));
-        FC_TRY(launch_layernorm(m->x, L.ln2g, L.ln2b, R, d, m->n, nullptr, st));
-        FC_TRY(gemm(m, L.up, m->n, L.up_b, nullptr, EPI_GELU, m->hid, R, F));
-        FC_TRY(gemm(m, L.down, m->hid, L.down_b, m->x, EPI_NONE, m->x, R, d));
+        FC_TRY(launch_layernorm_planes(m->x, L.ln1g, L.ln1b, R, d, m->pn, st));
+        if (tc_attn && !f32_qkv) {
+            FC_TRY(launch_gemm_q8_tc(L.qkv, m->pn, L.qkv_b, nullptr, EPI_NONE, nullptr, &m->pqkv, R, 3 * d, status, st, split_k));
+        } else {
+            FC_TRY(launch_gemm_q8_tc(L.qkv, m->pn, L.qkv_b, nullptr, EPI_NONE, m->qkv, nullptr, R, 3 * d, status, st, split_k));
+            FC_TRY(on_qkv(l));
+            if (tc_attn) FC_TRY(launch_split_planes(m->qkv, m->pqkv, (size_t)R * 3 * d, st));
+        }
+        if (tc_attn) {
+            FC_TRY(launch_attn_prefill_tc(m->pqkv, B, T, d, c.n_head, m->patt, status, st));
+        } else {
+            FC_TRY(launch_attn_prefill(m->qkv, B, T, d, c.n_head, m->att, st));
+            FC_TRY(launch_split_planes(m->att, m->patt, (size_t)R * d, st));
+        }
+        FC_TRY(launch_gemm_q8_tc(L.out, m->patt, L.out_b, m->x, EPI_NONE, m->x, nullptr, R, d, status, st, split_k));
+        FC_TRY(launch_layernorm_planes(m->x, L.ln2g, L.ln2b, R, d, m->pn, st));
+        FC_TRY(launch_gemm_q8_tc(L.up, m->pn, L.up_b, nullptr, EPI_GELU, nullptr, &m->phid, R, F, status, st, split_k));
+        FC_TRY(launch_gemm_q8_tc(L.down, m->phid, L.down_b, m->x, EPI_NONE, m->x, nullptr, R, d, status, st, split_k));
         FC_TRY(layer_stats());
     }
     return FC_OK;
 }
+static int forward_blocks(fc_model* m, int B, int T) {
+    return forward_blocks_with(m, B, T, model_planes(m), m->tc_status, false, false, [](int) { return FC_OK; });
+}
 
-// Forward + final LayerNorm + head + scoring tail for ids/targets already on the device.
-// lp_d/gr_d filled. Logit rows are ldl floats apart (ldl % 4 == 0 for vector stores).
+// Forward + final LayerNorm + head + scoring tail for ids/targets already on the device. lp_d/gr_d filled.
 static int score_device(fc_model* m, int B, int T) {
     const fc_config& c = m->cfg;
-    const int R = B * T, d = c.d_model, ldl = m->head.N_pad;
+    const int R = B * T, d = c.d_model;
     FC_TRY(forward_blocks(m, B, T));
-    if (tensor_path(m)) {
-        // the head's epilogue keeps (max, sum of exponentials, first argmax) per row and 128-column tile and the
-        // target's logit: [rows][V] logits never reach memory (scoring.rs:175-181 needs one number per row)
-        FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, R, d, m->nhi, m->nlo, m->st));
-        if (m->stats_on) FC_TRY(launch_layer_stats(nullptr, m->nhi, m->nlo, (size_t)R * d, m->stats_scratch, m->stats_d + m->stats_n++, m->st));
-        FC_TRY(launch_gemm_q8_bf16x3_score(m->head, m->nhi, m->nlo, m->targets_d, m->head_stats, m->head_tlogit, R, m->tc_status, m->st));
-        return launch_score_combine(m->head_stats, m->head_tlogit, m->targets_d, R, (c.vocab + 127) / 128, c.vocab, m->lp_d, m->gr_d, m->st);
-    }
-    FC_TRY(launch_layernorm(m->x, m->lnfg, m->lnfb, R, d, m->n, nullptr, m->st));
-    if (m->stats_on) FC_TRY(launch_layer_stats(m->n, nullptr, nullptr, (size_t)R * d, m->stats_scratch, m->stats_d + m->stats_n++, m->st));
-    for (int r0 = 0; r0 < R; r0 += m->head_chunk) {
-        const int rows = std::min(m->head_chunk, R - r0);
-        FC_TRY(gemm(m, m->head, m->n + (size_t)r0 * d, nullptr, nullptr, EPI_NONE, m->logits, rows, ldl));
-        FC_TRY(launch_score_rows(m->logits, ldl, c.vocab, m->targets_d + r0, rows, m->lp_d + r0, m->gr_d + r0, m->tc_status, m->st));
-    }
-    return FC_OK;
+    // the head's epilogue keeps (max, sum of exponentials, first argmax) per row and 128-column tile and the
+    // target's logit: [rows][V] logits never reach memory (scoring.rs:175-181 needs one number per row)
+    FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, R, d, m->pn, m->st));
+    if (m->stats_on) FC_TRY(launch_layer_stats(nullptr, m->pn, (size_t)R * d, m->stats_scratch, m->stats_d + m->stats_n++, m->st));
+    FC_TRY(launch_gemm_q8_tc_score(m->head, m->pn, m->targets_d, m->head_stats, m->head_tlogit, R, m->tc_status, m->st));
+    return launch_score_combine(m->head_stats, m->head_tlogit, m->targets_d, R, (c.vocab + 127) / 128, c.vocab, m->lp_d, m->gr_d, m->st);
 }
 
 }  // namespace fc
@@ -536,24 +510,27 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
         GemvOut o; o.out[0] = y_dev;
         return launch_gemv_q8(w->w, x_dev, bias_dev, nullptr, EPI_NONE, o, nullptr, st);
     }
-    if (math_mode == FC_MATH_BF16X3 && w->w.K % 64 == 0) {
-        // the bf16 planes of x and the status word live in the weight handle and grow on demand
-        fc_qweight* wm = const_cast<fc_qweight*>(w);
-        const size_t need = (size_t)M * w->w.K;
-        if (need > wm->plane_elems) {
-            FC_CUDA(cudaStreamSynchronize(st));
-            wm->planes.release();
-            wm->plane_elems = 0;
-            FC_TRY(wm->planes.alloc_n(&wm->xhi, need));
-            FC_TRY(wm->planes.alloc_n(&wm->xlo, need));
-            FC_TRY(wm->planes.alloc_n(&wm->status, 1));
-            FC_CUDA(cudaMemsetAsync(wm->status, 0, sizeof(int), st));
-            wm->plane_elems = need;
-        }
-        FC_TRY(launch_split_bf16(x_dev, wm->xhi, wm->xlo, need, st));
-        return launch_gemm_q8_bf16x3(w->w, wm->xhi, wm->xlo, bias_dev, nullptr, EPI_NONE, y_dev, M, w->w.N, wm->status, st);
+    // the bf16 planes of x and the status word live in the weight handle and grow on demand
+    fc_qweight* wm = const_cast<fc_qweight*>(w);
+    const int planes = math_mode == FC_MATH_BF16X3 && w->w.K % 64 == 0 ? 2 : 3;
+    const size_t need = (size_t)M * w->w.K;
+    if (need > wm->plane_elems || !wm->x.p[planes - 1]) {
+        FC_CUDA(cudaStreamSynchronize(st));
+        wm->planes.release();
+        const size_t elems = std::max(need, wm->plane_elems);
+        const int keep = std::max(planes, wm->x.p[2] ? 3 : 2);
+        wm->plane_elems = 0;
+        wm->x = Planes();
+        wm->status = nullptr;
+        for (int p = 0; p < keep; ++p) FC_TRY(wm->planes.alloc(&wm->x.p[p], elems * 2));
+        FC_TRY(wm->planes.alloc_n(&wm->status, 1));
+        FC_CUDA(cudaMemsetAsync(wm->status, 0, sizeof(int), st));
+        wm->plane_elems = elems;
     }
-    return launch_gemm_q8_fp32(w->w, x_dev, bias_dev, nullptr, EPI_NONE, y_dev, M, w->w.N, st);
+    Planes x = wm->x;
+    x.n = planes;
+    FC_TRY(launch_split_planes(x_dev, x, need, st));
+    return launch_gemm_q8_tc(w->w, x, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, wm->status, st);
 }
 
 int fc_q8_0_linear(int device, const float* x, const void* wq, const float* bias, float* y,
@@ -783,6 +760,14 @@ int fc_model_read_layer_stats(fc_model* m, fc_layer_stats* out, int cap) {
 // ---------------------------------------------------------------------------- scoring
 // Runs B windows x T rows through the model; double log-probs / flags stay on the device
 // until copied into the caller's arrays.
+static int check_tc_status(fc_model* m, const char* what) {
+    int status = 0;
+    FC_CUDA(cudaMemcpyAsync(&status, m->tc_status, sizeof(int), cudaMemcpyDeviceToHost, m->st));
+    FC_CUDA(cudaStreamSynchronize(m->st));
+    if (status == 0) return FC_OK;
+    cudaMemsetAsync(m->tc_status, 0, sizeof(int), m->st);
+    return fail(FC_E_TIMEOUT, "a bounded wait inside a tensor-core kernel of %s ran out (status %d)", what, status);
+}
 static int score_windows_impl(fc_model* m, const int32_t* ids, const int32_t* targets, int B, int T,
                               double* lp_host, uint8_t* gr_host) {
     const fc_config& c = m->cfg;
@@ -792,7 +777,7 @@ static int score_windows_impl(fc_model* m, const int32_t* ids, const int32_t* ta
     const int R = B * T;
     FC_TRY(check_ids(m, ids, (size_t)R));
     FC_CUDA(cudaSetDevice(m->device));
-    FC_TRY(ensure_workspace(m, R));
+    FC_TRY(ensure_workspace(m, R, model_planes(m)));
     cudaStream_t st = m->st;
     FC_CUDA(cudaMemcpyAsync(m->ids_d, ids, (size_t)R * 4, cudaMemcpyHostToDevice, st));
     FC_CUDA(cudaMemcpyAsync(m->targets_d, targets, (size_t)R * 4, cudaMemcpyHostToDevice, st));
@@ -950,18 +935,17 @@ int fc_predict_next(fc_model* m, const int32_t* ids, int n, float* probs) {
     if (n > c.ctx) return fail(FC_E_DIM, "Sequence length %d exceeds max_seq_len %d", n, c.ctx);
     FC_TRY(check_ids(m, ids, (size_t)n));
     FC_CUDA(cudaSetDevice(m->device));
-    FC_TRY(ensure_workspace(m, n));
+    FC_TRY(ensure_workspace(m, n, model_planes(m)));
     cudaStream_t st = m->st;
     FC_CUDA(cudaMemcpyAsync(m->ids_d, ids, (size_t)n * 4, cudaMemcpyHostToDevice, st));
     FC_TRY(forward_blocks(m, 1, n));
     FC_TRY(launch_layernorm(m->x + (size_t)(n - 1) * c.d_model, m->lnfg, m->lnfb, 1, c.d_model,
-                            m->n + (size_t)(n - 1) * c.d_model, nullptr, st));
+                            m->n, nullptr, st));
     GemvOut o; o.out[0] = m->logits;
-    FC_TRY(launch_gemv_q8(m->head, m->n + (size_t)(n - 1) * c.d_model, nullptr, nullptr, EPI_NONE, o, nullptr, st));
+    FC_TRY(launch_gemv_q8(m->head, m->n, nullptr, nullptr, EPI_NONE, o, nullptr, st));
     FC_TRY(launch_softmax_row(m->logits, c.vocab, m->probs_d, st));
     FC_CUDA(cudaMemcpyAsync(probs, m->probs_d, (size_t)c.vocab * 4, cudaMemcpyDeviceToHost, st));
-    FC_CUDA(cudaStreamSynchronize(st));
-    return FC_OK;
+    return check_tc_status(m, "predict_next");
 }
 
 // ----------------------------------------------------------------------------- streams
@@ -1080,17 +1064,17 @@ static int prime_batched(fc_stream* const* ss, int S, int n, int last_mode, int*
                          float* const* vcs_dev = nullptr) {
     fc_model* m = ss[0]->m;
     const fc_config& c = m->cfg;
-    const int d = c.d_model, F = c.d_ff, hd = d / c.n_head, R = S * n;
+    const int d = c.d_model, hd = d / c.n_head, R = S * n;
     *used = 0;
     if (R < kPrimeBatchMin || n < 2 || (hd != 32 && hd != 64)) return FC_OK;
     for (int i = 0; i < S; ++i)
         if (ss[i]->host_pos != 0) return FC_OK;
     cudaStream_t st = m->st;
-    FC_TRY(ensure_workspace(m, R));
+    // prompts keep f32 rounding (3 planes) unless the model's scoring mode is the 2-plane one and there are many rows
+    const int planes = R >= 256 && tensor_attention(m, model_planes(m)) ? 2 : 3;
+    FC_TRY(ensure_workspace(m, R, planes));
     for (int i = 0; i < S; ++i)
         FC_CUDA(cudaMemcpyAsync(m->ids_d + (size_t)i * n, ss[i]->queue, (size_t)n * sizeof(int), cudaMemcpyDeviceToDevice, st));
-    FC_CUDA(cudaMemsetAsync(m->err_d, 0, sizeof(int), st));
-    FC_TRY(launch_embed_rows(m->tok, m->pos, m->ids_d, R, n, m->x, m->err_d, st));
     const size_t layer_stride = (size_t)c.ctx * d;
     // rows [q | k | v] of window i -> cache positions 0..n-1 of stream i
     auto to_caches = [&](int l) -> int {
@@ -1104,34 +1088,7 @@ static int prime_batched(fc_stream* const* ss, int S, int n, int last_mode, int*
         }
         return FC_OK;
     };
-    if (tensor_path(m) && R >= 256) {
-        // many rows: the window forward of the scoring path (tcgen05 GEMMs and attention on bf16 hi / lo
-        // planes); the QKV product also leaves f32 rows, which feed the caches
-        for (int l = 0; l < c.n_layer; ++l) {
-            const LayerDev& L = m->layers[l];
-            FC_TRY(launch_layernorm_planes(m->x, L.ln1g, L.ln1b, R, d, m->nhi, m->nlo, st));
-            FC_TRY(launch_gemm_q8_bf16x3_ex(L.qkv, m->nhi, m->nlo, L.qkv_b, nullptr, EPI_NONE, m->qkv, nullptr, nullptr, R, 3 * d, m->tc_status, st));
-            FC_TRY(to_caches(l));
-            FC_TRY(launch_split_bf16(m->qkv, m->qkvhi, m->qkvlo, (size_t)R * 3 * d, st));
-            FC_TRY(launch_attn_prefill_tc(m->qkvhi, m->qkvlo, S, n, d, c.n_head, m->atthi, m->attlo, m->tc_status, st));
-            FC_TRY(launch_gemm_q8_bf16x3_ex(L.out, m->atthi, m->attlo, L.out_b, m->x, EPI_NONE, m->x, nullptr, nullptr, R, d, m->tc_status, st));
-            FC_TRY(launch_layernorm_planes(m->x, L.ln2g, L.ln2b, R, d, m->nhi, m->nlo, st));
-            FC_TRY(launch_gemm_q8_bf16x3_ex(L.up, m->nhi, m->nlo, L.up_b, nullptr, EPI_GELU, nullptr, m->hidhi, m->hidlo, R, F, m->tc_status, st));
-            FC_TRY(launch_gemm_q8_bf16x3_ex(L.down, m->hidhi, m->hidlo, L.down_b, m->x, EPI_NONE, m->x, nullptr, nullptr, R, d, m->tc_status, st));
-        }
-    } else {
-        for (int l = 0; l < c.n_layer; ++l) {
-            const LayerDev& L = m->layers[l];
-            FC_TRY(launch_layernorm(m->x, L.ln1g, L.ln1b, R, d, m->n, nullptr, st));
-            FC_TRY(launch_gemm_q8_fp32(L.qkv, m->n, L.qkv_b, nullptr, EPI_NONE, m->qkv, R, 3 * d, st));
-            FC_TRY(to_caches(l));
-            FC_TRY(launch_attn_prefill(m->qkv, S, n, d, c.n_head, m->att, st));
-            FC_TRY(launch_gemm_q8_fp32(L.out, m->att, L.out_b, m->x, EPI_NONE, m->x, R, d, st));
-            FC_TRY(launch_layernorm(m->x, L.ln2g, L.ln2b, R, d, m->n, nullptr, st));
-            FC_TRY(launch_gemm_q8_fp32(L.up, m->n, L.up_b, nullptr, EPI_GELU, m->hid, R, F, st));
-            FC_TRY(launch_gemm_q8_fp32(L.down, m->hid, L.down_b, m->x, EPI_NONE, m->x, R, d, st));
-        }
-    }
+    FC_TRY(forward_blocks_with(m, S, n, planes, S == 1 && ss[0]->status ? ss[0]->status : m->tc_status, true, true, to_caches));
     *used = 1;
     for (int i = 0; i < S; ++i) {
         fc_stream* s = ss[i];

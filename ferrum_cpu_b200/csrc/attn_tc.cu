@@ -367,10 +367,8 @@ int encode(CUtensorMap* map, const void* plane, size_t rows, size_t cols, int bo
 }
 }  // namespace
 
-// qkv_hi / qkv_lo: bf16 planes [B*T][H*64 + 2*KV*64] (q heads | k heads | v heads per row);
-// out_hi / out_lo: planes [B*T][H*64]. Query head h reads key / value head h / (H / KV).
-int launch_attn_prefill_tc_gqa(const void* qkv_hi, const void* qkv_lo, int B, int T, int H, int KV, void* out_hi, void* out_lo,
-                               int* status, cudaStream_t st) {
+// qkv: bf16 planes [B*T][H*64 + 2*KV*64] (q heads | k heads | v heads per row); out: planes [B*T][H*64]. Query head h reads key / value head h / (H / KV).
+int launch_attn_prefill_tc_gqa(const Planes& qkv, int B, int T, int H, int KV, const Planes& out, int* status, cudaStream_t st) {
     if (KV <= 0 || H % KV) return fail(FC_E_DIM, "n_heads %d must be a multiple of n_kv_heads %d", H, KV);
     static bool attr_set[64] = {};
     int dev = 0;
@@ -381,13 +379,13 @@ int launch_attn_prefill_tc_gqa(const void* qkv_hi, const void* qkv_lo, int B, in
     }
     const size_t R = (size_t)B * T, ld = (size_t)(H + 2 * KV) * HD;
     CUtensorMap qh, ql, kh, kl;
-    FC_TRY(encode(&qh, qkv_hi, R, ld, QT));
-    FC_TRY(encode(&ql, qkv_lo, R, ld, QT));
-    FC_TRY(encode(&kh, qkv_hi, R, ld, KT));
-    FC_TRY(encode(&kl, qkv_lo, R, ld, KT));
+    FC_TRY(encode(&qh, qkv.p[0], R, ld, QT));
+    FC_TRY(encode(&ql, qkv.p[1], R, ld, QT));
+    FC_TRY(encode(&kh, qkv.p[0], R, ld, KT));
+    FC_TRY(encode(&kl, qkv.p[1], R, ld, KT));
     AttnArgs a;
     a.T = T; a.k_col = H * HD; a.v_col = (H + KV) * HD; a.group = H / KV; a.ldo = H * HD;
-    a.out_hi = (uint16_t*)out_hi; a.out_lo = (uint16_t*)out_lo; a.status = status;
+    a.out_hi = (uint16_t*)out.p[0]; a.out_lo = (uint16_t*)out.p[1]; a.status = status;
     dim3 grid((T + QT - 1) / QT, H, B);
     attn_prefill_tc_kernel<<<grid, THREADS, SMEM_BYTES, st>>>(qh, ql, kh, kl, a);
     FC_LAUNCHED();
@@ -395,10 +393,9 @@ int launch_attn_prefill_tc_gqa(const void* qkv_hi, const void* qkv_lo, int B, in
 }
 
 // The multi-head form: planes [B*T][3d] in, [B*T][d] out.
-int launch_attn_prefill_tc(const void* qkv_hi, const void* qkv_lo, int B, int T, int d, int H, void* out_hi, void* out_lo,
-                           int* status, cudaStream_t st) {
+int launch_attn_prefill_tc(const Planes& qkv, int B, int T, int d, int H, const Planes& out, int* status, cudaStream_t st) {
     if (d != H * HD) return fail(FC_E_SHAPE, "tensor-core attention needs head_dim 64 (d = %d, H = %d)", d, H);
-    return launch_attn_prefill_tc_gqa(qkv_hi, qkv_lo, B, T, H, H, out_hi, out_lo, status, st);
+    return launch_attn_prefill_tc_gqa(qkv, B, T, H, H, out, status, st);
 }
 
 }  // namespace fc

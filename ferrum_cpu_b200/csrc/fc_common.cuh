@@ -87,10 +87,13 @@ constexpr int kRowPad = 128;
 
 enum Epilogue : int { EPI_NONE = 0, EPI_GELU = 1, EPI_SWIGLU = 2, EPI_SCORE = 3 };
 
-// activation.rs:9-12 (tanh GELU), same constants and association as the reference.
+// activation.rs:9-12 (tanh GELU): 0.5 x (1 + tanh(u)) with u = 0.7978846 (x + 0.044715 x^3). Since (1 + tanh(u)) / 2 is the
+// logistic function of 2u, that is x / (1 + exp(-2u)): a handful of instructions where tanhf takes some thirty, and
+// without the cancellation of 1 + tanh(u) for large negative u. exp2 and the quotient are the 2-ulp hardware forms.
 __device__ __forceinline__ float gelu_f(float x) {
     const float K = 0.7978846f;
-    return 0.5f * x * (1.0f + tanhf(K * (x + 0.044715f * x * x * x)));
+    const float u = K * (x + 0.044715f * x * x * x);
+    return __fdividef(x, 1.0f + exp2f(u * -2.885390082f));   // -2 log2(e)
 }
 
 // ---- decode-step device state (one per stream) ----------------------------------------
@@ -132,27 +135,27 @@ int launch_gemv_q8_wide(const QMat& w, const float* x, const float* norm_w, floa
 int launch_gemv_q8_stream(const QMat& w, const float* x, const float* norm_w, float eps, const float* bias, const float* residual,
                           int epi, float* out, const StepState* state, int* status, cudaStream_t st);
 
-// gemm_simt.cu — Y[M][N] = X[M][K]·Wᵀ + bias (+GELU) (+residual[M][N]), fp32 CUDA cores.
-int launch_gemm_q8_fp32(const QMat& w, const float* x, const float* bias, const float* residual, int epi,
-                        float* y, int M, int ldy, cudaStream_t st);
+// An f32 matrix as n bf16 planes whose sum it is: 2 planes hold it to 2^-17 relative (FC_MATH_BF16X3), 3 exactly
+// (FC_MATH_FP32). The form in which activations reach the tensor cores.
+struct Planes {
+    void* p[3] = {nullptr, nullptr, nullptr};
+    int n = 0;
+};
+int launch_split_planes(const float* x, const Planes& out, size_t n, cudaStream_t st);
+// gemm_tc.cu — Y[M][N] = X[M][K]·Wᵀ + bias (+GELU / SwiGLU) (+residual[M][N]) on tcgen05 tensor cores, the weight exact, X
+// as planes [M][K]. Output: f32 rows y, or (y == nullptr) planes yp for the next GEMM, as many as X has.
+// `status` is a device int raised to FC_E_TIMEOUT when a bounded wait runs out. split_k: few rows may split the K range
+// over CTAs; without it a row's result does not depend on how many rows share the launch (the scoring forward).
+int launch_gemm_q8_tc(const QMat& w, const Planes& x, const float* bias, const float* residual, int epi, float* y, const Planes* yp,
+                      int M, int ldy, int* status, cudaStream_t st, bool split_k = true);
 
-// gemm_tc.cu — the same product on tcgen05 tensor cores (bf16 3-term split, fp32 TMEM
-// accumulate). x_hi / x_lo are bf16 planes [M][K] made by launch_split_bf16; K % 64 == 0.
-// `status` is a device int raised to FC_E_TIMEOUT when a bounded wait runs out.
-int launch_split_bf16(const float* x, void* hi, void* lo, size_t n, cudaStream_t st);
-int launch_gemm_q8_bf16x3(const QMat& w, const void* x_hi, const void* x_lo, const float* bias, const float* residual,
-                          int epi, float* y, int M, int ldy, int* status, cudaStream_t st);
-// The same with a choice of output: f32 rows y, or (y == nullptr) bf16 hi / lo planes for the next GEMM.
-int launch_gemm_q8_bf16x3_ex(const QMat& w, const void* x_hi, const void* x_lo, const float* bias, const float* residual,
-                             int epi, float* y, void* y_hi, void* y_lo, int M, int ldy, int* status, cudaStream_t st);
-
-// The LM head fused with the statistics of the softmax tail (math mode FC_MATH_BF16X3): instead of logits the
+// The LM head fused with the statistics of the softmax tail: instead of logits the
 // epilogue leaves, per (row, 128-column tile), the tile's largest logit, the sum of exp(logit - that) and the first
 // column that attains it in stats [M][ceil(N / 128)] (16-byte records), and the logit of the row's target
 // (targets[M], -1: none) in tlogit [M]. launch_score_combine folds the records of a row in tile order into
 // ln(max(softmax(row)[target], 1e-12)) (f32 probability, f64 logarithm) and argmax_first(row) == target.
-int launch_gemm_q8_bf16x3_score(const QMat& w, const void* x_hi, const void* x_lo, const int* targets, void* stats, float* tlogit,
-                                int M, int* status, cudaStream_t st);
+int launch_gemm_q8_tc_score(const QMat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status,
+                            cudaStream_t st);
 int launch_score_combine(const void* stats, const float* tlogit, const int* targets, int M, int n_tiles, int V, double* logprob,
                          uint8_t* is_greedy, cudaStream_t st);
 
@@ -166,8 +169,8 @@ int launch_embed_rows(const QMat& tok, const float* pos_emb, const int* ids, int
                       int* error_flag, cudaStream_t st);
 int launch_layernorm(const float* x, const float* g, const float* b, int rows, int d, float* y,
                      const StepState* state, cudaStream_t st);
-// LayerNorm written as bf16 hi / lo planes [rows][d] for the tensor-core GEMM.
-int launch_layernorm_planes(const float* x, const float* g, const float* b, int rows, int d, void* hi, void* lo, cudaStream_t st);
+// LayerNorm written as bf16 planes [rows][d] for the tensor-core GEMM.
+int launch_layernorm_planes(const float* x, const float* g, const float* b, int rows, int d, const Planes& out, cudaStream_t st);
 // Decode tail over logits[V]: softmax statistics, optional probs[V], optional greedy select
 // (append to queue) — and always the end-of-step bookkeeping (pos, fed).
 int launch_step_tail(const float* logits, int V, float* probs_or_null, int do_select, int* queue, int queue_cap,
@@ -175,10 +178,6 @@ int launch_step_tail(const float* logits, int V, float* probs_or_null, int do_se
 // End-of-step bookkeeping alone (steps that skip the head).
 int launch_step_advance(StepState* state, cudaStream_t st);
 int launch_step_advance_pdl(StepState* state, cudaStream_t st);
-// Scoring tail: per row of logits[R][ldl], target id (or -1) -> logprob, is_greedy.
-// `status` (device int, may be null) is raised to FC_E_TIMEOUT when a bounded wait runs out.
-int launch_score_rows(const float* logits, int ldl, int V, const int* targets, int R, double* logprob,
-                      uint8_t* is_greedy, int* status, cudaStream_t st);
 int launch_softmax_row(const float* logits, int V, float* probs, cudaStream_t st);
 // sample.cu — one draw of sample_with_params on the device; see the kernel for the arguments.
 int launch_sample(const float* in, int V, int from_probs, const fc_sampling& prm, const int* recent, int n_recent,
@@ -205,8 +204,8 @@ struct LayerStatsDev {
     long long nan_count, inf_count, n;
 };
 size_t layer_stats_scratch_bytes();
-// x (f32), or (x == nullptr) bf16 hi / lo planes whose sum is the value; n elements; scratch: layer_stats_scratch_bytes().
-int launch_layer_stats(const float* x, const void* hi, const void* lo, size_t n, void* scratch, LayerStatsDev* out, cudaStream_t st);
+// x (f32), or (x == nullptr) bf16 planes whose sum is the value; n elements; scratch: layer_stats_scratch_bytes().
+int launch_layer_stats(const float* x, const Planes& planes, size_t n, void* scratch, LayerStatsDev* out, cudaStream_t st);
 
 // attn.cu
 int launch_attn_decode(const float* q, const float* kcache, const float* vcache, int d, int H, int ctx,
@@ -219,13 +218,11 @@ int launch_attn_decode_gqa(const float* q, const float* kcache, const float* vca
                            const StepState* state, float* out, cudaStream_t st);
 int launch_attn_prefill_gqa(const float* q, const float* k, const float* v, int B, int T, int ld, int H, int KV, int hd,
                             int ldo, float* out, cudaStream_t st);
-// attn_tc.cu — the same on tcgen05 (head_dim 64): bf16 hi / lo planes of qkv [B*T][3d] in,
-// planes of the attention output [B*T][d] out; `status` is raised on a timeout.
-int launch_attn_prefill_tc(const void* qkv_hi, const void* qkv_lo, int B, int T, int d, int H, void* out_hi, void* out_lo,
-                           int* status, cudaStream_t st);
+// attn_tc.cu — the same on tcgen05 (head_dim 64): bf16 planes (two) of qkv [B*T][3d] in, planes of the attention output
+// [B*T][d] out; `status` is raised on a timeout.
+int launch_attn_prefill_tc(const Planes& qkv, int B, int T, int d, int H, const Planes& out, int* status, cudaStream_t st);
 // Grouped-query form: planes [B*T][(H + 2 KV) * 64] in (q heads | k heads | v heads), [B*T][H * 64] out.
-int launch_attn_prefill_tc_gqa(const void* qkv_hi, const void* qkv_lo, int B, int T, int H, int KV, void* out_hi, void* out_lo,
-                               int* status, cudaStream_t st);
+int launch_attn_prefill_tc_gqa(const Planes& qkv, int B, int T, int H, int KV, const Planes& out, int* status, cudaStream_t st);
 
 // decode_batch.cu — one lock-step decode step for S <= kBatchMaxStreams streams.
 // Fragment-major copy of a Q8_0 matrix for the warp-level tensor-core product: per (16 rows,

@@ -1,507 +1,701 @@
-// Q8_0 GEMM on the 5th-generation tensor cores (math mode FC_MATH_BF16X3):
-//     Y[M][N] = X[M][K] · dequant(W[N][K])ᵀ + bias (+GELU) (+residual)
+// Q8_0 GEMM on the 5th-generation tensor cores:
+//     Y[M][N] = X[M][K] · dequant(W[N][K])ᵀ + bias (+GELU / SwiGLU) (+residual)
 //
-// Replaces ops::linear_forward (ferrum_core/src/ops.rs:233-256) for M >= 2 with the weight
-// kept packed. The reference multiplies f32 by f32; tcgen05 has no f32 operand kind, so both
-// operands are split into two bf16 terms (x = xh + xl, w = wh + wl, each exact to 2^-17
-// relative) and every 128x128x16 step issues three kind::f16 MMAs into the same fp32 TMEM
-// accumulator: xh·wh + xl·wh + xh·wl. The dropped xl·wl term is 2^-16 relative per product.
+// Replaces ops::linear_forward (ferrum_core/src/ops.rs:233-256) for M >= 2 with the weight kept packed. A Q8_0 level
+// is an 8-bit whole number and therefore exact in bf16, so the tensor core multiplies the LEVELS and the block scale is
+// applied afterwards: every 32-wide k-block is accumulated on its own in TMEM, and the warps that read it back fold it
+// into f32 registers with one fused multiply-add by the row's block scale. What is left to split is the activation:
+//     2 planes (math mode FC_MATH_BF16X3): x = x1 + x2 to 2^-17 relative, two MMAs per step
+//     3 planes (math mode FC_MATH_FP32):   x = x1 + x2 + x3 exactly (3 x 8 bits of significand), three MMAs per step
+// The weight is exact in both, d·q is never rounded. Dequantising the weight to bf16 hi + lo planes instead needs three
+// MMAs per step for 2-plane precision (and two weight planes in shared memory): measured on 32768 x 768 x 2304, that
+// form ran at 338 TFLOP/s of algorithmic work.
 //
-// Persistent kernel, one CTA per SM, 256 x 128 output tiles (two 128-row MMA tiles that share
-// one dequantised weight tile) taken round-robin, N fastest, so that the CTAs running together
-// share a few row panels of X in L2:
-//   warp 16     TMA producer: the two bf16 planes of the X tile (256 rows x 64 k, 128-byte
-//               swizzle) into the stage's A buffers, completing on the stage's mbarrier;
-//   warps 8-15  dequantise the 128 x 64 Q8_0 weight tile: w = d * q exactly as
-//               gguf::dequant_q8_0 (ferrum_core/src/gguf/dequant.rs:37-49), split into bf16
-//               hi/lo and stored in the same swizzled K-major layout the tensor core reads;
-//   warp 17     allocates all 512 TMEM columns (two buffers of two accumulators) and issues tcgen05.mma from one
-//               thread; tcgen05.commit frees the stage and finally publishes the accumulator;
-//   warps 0-7   epilogue of the previous tile while the next one is being multiplied, four warps (one per 32
-//               TMEM lanes) for each 128-row half: tcgen05.ld their accumulator lanes, bias / GELU /
-//               residual, then either f32 rows or the bf16 hi/lo planes the next GEMM consumes. (With four
-//               warps for the whole tile the epilogue outlasted the MMAs of the next tile and held its buffer.)
-// Every mbarrier wait is bounded by a cycle budget; when it runs out the kernel raises a
-// status word, releases its TMEM and returns.
+// The weight tile is the M operand of the MMA (TMEM lane = weight row) and the activation rows are its N operand
+// (TMEM column = activation row). A thread that drains TMEM thus needs ONE scale per k-block, its row's, and the number
+// of activation rows per tile is free in steps of 16 or 32.
 //
-// Bound: tensor pipe. 2·M·N·K algorithmic FLOP (6·M·N·K executed).
+// One CTA per SM, 640 threads in five warpgroups (registers 160 / 160 / 56 / 56 / 40 a thread):
+//   warps 0-7   drain: per k-block tcgen05.ld of their 32 lanes x half of the columns, f32x2 FMA into registers; after the
+//               last k-block bias / GELU / SwiGLU / residual or the softmax records, and the stores
+//   warps 8-15  weights: 32 levels of a row per thread, u8 -> bf16 (two logic operations and one packed add per pair),
+//               stored in the swizzled K-major layout the tensor core reads. With four warps (64 levels a thread) a stage
+//               took about 1600 cycles of latency, twice what the MMAs take
+//   warp 16     TMA: the activation planes of the stage (64 k each)
+//   warps 17-18 MMA issue, one for the even and one for the odd k-blocks; warp 17 owns the TMEM allocation (512 columns:
+//               four k-block buffers of up to 128 activation rows or three of 160, enough to hide the two barrier hops
+//               between a k-block's MMAs and its drain). What a k-block costs its issuer besides the MMAs (two barrier waits, a commit,
+//               fetching the loop's instructions again) is about 500 cycles, as long as the MMAs themselves: one issuer
+//               leaves the tensor pipe idle half of the time, two hide each other's.
+// CG = 2: a pair of CTAs shares a tile (tcgen05 cta_group::2): each holds its 128 of 256 weight rows and half of the
+// activation rows, so that the activation tile is read from L2 once for 256 weight rows and its operand reads from shared
+// memory halve. Up to 160 rows a tile: 192 and 256 leave two buffers and more accumulators than the drain warps' registers
+// hold beside their working set (32768 x 768 x 2304: 160 rows 354 us, 128 rows 388, 192 rows 376, 256 rows 467).
+// CG = 1 takes small problems: the K range may be split over a cluster of up to 8 CTAs whose partial sums meet through
+// distributed shared memory in rank order, so that a few activation rows still occupy the GPU and results stay
+// reproducible.
+//
+// Every wait is bounded; a wait that runs out raises the status word and all roles leave.
+// Bound: tensor pipe for large M (2·M·N·K algorithmic FLOP, planes x that executed), weight bytes for a few rows. Measured
+// with the split of X into planes (of the f32 form this replaced: CUDA-core FMA, 42 TFLOP/s):
+//     32768 x 768 x 2304   2 planes 348 us = 334 TFLOP/s   3 planes 369 us = 314 TFLOP/s
+//     32768 x 1024 x 4096  2 planes 746 us = 368 TFLOP/s   3 planes 791 us = 348 TFLOP/s
+//     4096 x 1024 x 4096   2 planes 109 us (126 before)    3 planes 112 us (811 before)
 #include <cuda.h>
-#include <cuda_bf16.h>
 
-#include "fc_common.cuh"
+#include <algorithm>
+#include <type_traits>
+
+#include "planes.cuh"
 
 namespace fc {
 
 namespace {
 
-constexpr int BM = 256, BN = 128, BK = 64;            // a CTA tile is two 128-row MMA tiles sharing one weight tile
-constexpr int STAGES = 2;
-constexpr int TILE_BYTES = 128 * BK * 2;                // one 128-row bf16 operand tile: 16 KiB
-constexpr int A_BYTES = 2 * TILE_BYTES;                 // one plane of the 256-row X tile
-constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * TILE_BYTES;   // A hi, A lo (256 rows each), B hi, B lo
-constexpr int EPI_WARPS = 8, DQ_WARPS = 8;   // epilogue: four warps (one per 32 TMEM lanes) for each 128-row half of the tile
-constexpr int TMA_WARP = EPI_WARPS + DQ_WARPS, MMA_WARP = TMA_WARP + 1;
-constexpr int THREADS = (MMA_WARP + 1) * 32;
-constexpr int TMEM_COLS = 512;                          // two buffers of two 128-column accumulators
-// bf16 x bf16 -> f32, M = 128, N = 128, both operands K-major
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+constexpr int BK = 64;                                  // k per stage: two Q8_0 blocks, one 128-byte swizzle row of bf16
+constexpr int Q_BYTES = 128 * BK * 2;                   // the CTA's weight tile of a stage
+constexpr int DRAIN_WARPS = 8, DQ_WARPS = 8;
+constexpr int TMA_WARP = DRAIN_WARPS + DQ_WARPS, MMA_WARP = TMA_WARP + 1;   // MMA_WARP and MMA_WARP + 1
+constexpr int THREADS = 640;
+constexpr int MAX_STAGES = 8;
+constexpr int TMEM_COLS = 512, MAX_BUFS = 4;            // k-block buffers of 128 or 160 columns
+constexpr int SCORE_BYTES = 4 * 128 * 16;               // per (32-row quarter, column) softmax records
+// Block scales travel to the drain warps through a ring of their own: a stage is free again when its MMAs have retired, and
+// the drain may be MAX_BUFS k-blocks behind those (two stages, three when it is in the middle of one).
+constexpr int SCALE_BYTES = 128 * 4, SCALE_EXTRA = 3;   // per slot: a row's two f16 scales; slots beyond the stages
+constexpr int SMEM_LIMIT = 227 * 1024;
 
-struct Bars {
-    unsigned long long full_a[STAGES];
-    unsigned long long full_b[STAGES];
-    unsigned long long empty[STAGES];
-    unsigned long long acc_full[2];
-    unsigned long long acc_empty[2];
-    uint32_t tmem_base;
-    volatile int abort;
+enum Mode : int { OUT_F32 = 0, OUT_PLANES = 1, OUT_GELU = 2 /* planes, after GELU */, OUT_SWIGLU = 3, OUT_SCORE = 4 };
+
+struct TcArgs {
+    const uint8_t* qu; const __half* d; int N, K, N_pad, M;
+    int nt;                   // activation rows of a tile
+    int stages, stage_bytes;
+    int bufs, acc_cols;       // TMEM buffers and their columns
+    int ksplit;               // CTAs of a cluster that share the K range (CG = 1)
+    const float* bias; const float* residual; int gelu;
+    float* y; int ldy;        // OUT_F32
+    uint16_t* yp[3];          // OUT_PLANES / OUT_GELU / OUT_SWIGLU: bf16 planes, ldy elements apart
+    // OUT_SCORE: per (row, 128-column tile) softmax statistics instead of the product (see launch_gemm_q8_tc_score)
+    const int* targets; float4* stats; float* tlogit;
+    int* status;
+    long long wait_cycles;    // budget of every mbarrier wait
+    int withhold;             // test hook: the TMA producer issues nothing, so the waits on its stages run out
 };
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /* alignment slack */ + (int)sizeof(Bars);
+
+// Barriers and flags at the end of the shared memory, by byte offset.
+constexpr int BAR_FULL = 0, BAR_EMPTY = BAR_FULL + 8 * MAX_STAGES, BAR_ACC_FULL = BAR_EMPTY + 8 * MAX_STAGES, BAR_ACC_EMPTY = BAR_ACC_FULL + 8 * MAX_BUFS;
+constexpr int BAR_TMEM = BAR_ACC_EMPTY + 8 * MAX_BUFS, BAR_ABORT = BAR_TMEM + 4, BAR_BYTES = BAR_ABORT + 4;
 
 __device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned long long* b, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s32(b)), "r"(count) : "memory");
+__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
 }
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* b, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(s32(b)), "r"(bytes) : "memory");
+// Barriers are named by their 32-bit shared address: a generic pointer would be converted again at every use.
+__device__ __forceinline__ void mbar_init(uint32_t b, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s32(b)) : "memory");
+__device__ __forceinline__ void mbar_expect_tx(uint32_t b, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
 }
-// A thread that finds the phase incomplete is suspended by the hardware for up to 2 us.
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* b, uint32_t parity) {
+// b: a shared::cluster address, this CTA's or a peer's.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t b) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(b) : "memory");
+}
+// Up to `tries` times: a thread that finds the phase incomplete is suspended by the hardware for a while (without a time
+// hint: with one, the wait is a software loop around nanosleep). The loop is four instructions, since a dozen warps sit in
+// such loops at any time and their polls compete with the drain warps for issue slots.
+__device__ __forceinline__ bool mbar_poll(uint32_t b, uint32_t parity, int tries) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .s32 n;\n\t"
+        "mov.s32 n, %3;\n"
+        "POLL_%=:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE_%=;\n\t"
+        "sub.s32 n, n, 1;\n\t"
+        "setp.gt.s32 q, n, 0;\n\t"
+        "@q bra POLL_%=;\n"
+        "DONE_%=:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(b), "r"(parity), "r"(tries) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool mbar_sleep(uint32_t b, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(s32(b)), "r"(parity), "r"(2000u) : "memory");
+        : "=r"(ok) : "r"(b), "r"(parity), "r"(1000u) : "memory");
     return ok != 0;
 }
-// Bounded wait. Returns false (after raising the status word) when the budget runs out or
-// another role of this CTA already gave up.
-__device__ bool wait_bar(Bars* bars, unsigned long long* b, uint32_t parity, int* status, long long budget) {
+// Bounded wait. Returns false (after raising the status word) when the budget runs out or another role of this CTA
+// already gave up. SLEEP: for the producers, which wait most of the time and are stages ahead.
+template <bool SLEEP = false>
+__device__ __forceinline__ bool wait_bar(uint32_t b, uint32_t parity, volatile int* abort, const TcArgs& a) {
+    if (__builtin_expect(SLEEP ? mbar_sleep(b, parity) : mbar_poll(b, parity, 256), 1)) return true;
     const long long t0 = clock64();
-    while (!mbar_try_wait(b, parity)) {
-        if (bars->abort) return false;
-        if (clock64() - t0 > budget) {
-            bars->abort = 1;
-            atomicExch(status, FC_E_TIMEOUT);
+    while (!(SLEEP ? mbar_sleep(b, parity) : mbar_poll(b, parity, 256))) {
+        if (*abort) return false;
+        if (clock64() - t0 > a.wait_cycles) {
+            *abort = 1;
+            atomicExch(a.status, FC_E_TIMEOUT);
             return false;
         }
     }
     return true;
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(s32(dst)), "l"(map), "r"(x), "r"(y), "r"(s32(bar)) : "memory");
+// mbar: shared::cluster address of the barrier the bytes complete on; with CG = 2 it may be the pair's other CTA's.
+template <int CG>
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t mbar) {
+    if (CG == 2)
+        asm volatile(
+            "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+            ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(mbar) : "memory");
+    else
+        asm volatile(
+            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+            ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(mbar) : "memory");
 }
 // K-major, 128-byte swizzle: 8-row atoms of 1024 bytes (SBO = 64 x 16 B), descriptor version 1.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)64 << 32) | ((uint64_t)1 << 46) |
            ((uint64_t)2 << 61);
 }
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(IDESC), "r"(accumulate) : "memory");
+template <int CG, bool ACCUMULATE>
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t dhi, uint32_t idesc) {
+    if (CG == 2)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+            "setp.ne.b32 p, %5, 0;\n\tmov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %4, p;\n\t}"
+            ::"r"(tmem_d), "r"(alo), "r"(blo), "r"(dhi), "r"(idesc), "n"(ACCUMULATE ? 1 : 0) : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+            "setp.ne.b32 p, %5, 0;\n\tmov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
+            ::"r"(tmem_d), "r"(alo), "r"(blo), "r"(dhi), "r"(idesc), "n"(ACCUMULATE ? 1 : 0) : "memory");
 }
-__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(bar)) : "memory");
+// Arrives on the barrier at this offset when the MMAs issued so far have retired (CG = 2: in both CTAs of the pair).
+template <int CG>
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+    if (CG == 2)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(bar), "h"((uint16_t)3) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-
-template <int B>
-__device__ __forceinline__ float qb(uint32_t w) {
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540 + B)) - 8388736.0f;
-}
-// Two values -> packed bf16 hi pair and lo pair (element 0 in the low half).
-__device__ __forceinline__ void split2(float w0, float w1, uint32_t* hi, uint32_t* lo) {
-    const __nv_bfloat162 h = __float22bfloat162_rn(make_float2(w0, w1));
-    const float2 hf = __bfloat1622float2(h);
-    const __nv_bfloat162 l = __float22bfloat162_rn(make_float2(w0 - hf.x, w1 - hf.y));
-    *hi = *(const uint32_t*)&h;
-    *lo = *(const uint32_t*)&l;
-}
-
-// 256-bit global accesses: one full 32-byte sector per lane and instruction.
-__device__ __forceinline__ void st256(void* p, const uint32_t* v) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
-}
-__device__ __forceinline__ void ld256(const void* p, uint32_t* v) {
-    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "l"(p) : "memory");
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-struct TcArgs {
-    const uint8_t* qu; const __half* d; int N, K;
-    const float* bias; const float* residual; int epi;
-    float* y;                 // f32 output rows, or null when the output goes to planes
-    uint16_t *yhi, *ylo;      // bf16 hi / lo output planes [M][ldy]
-    int M, ldy;
-    int* status;
-    // EPI_SCORE: per (row, N tile) softmax statistics instead of the product (see launch_gemm_q8_bf16x3_score)
-    const int* targets;
-    float4* stats;
-    float* tlogit;
-    long long wait_cycles;    // budget of every mbarrier wait
-    int withhold;             // test hook: the TMA producer issues nothing, so the waits on its stages run out
+// N consecutive columns of the warp's 32 lanes into r[o ..].
+template <int N, int CW>
+__device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint32_t (&r)[CW], const int o) {
+    if (N == 8) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {"
+            "%0, %1, %2, %3, %4, %5, %6, %7"
+            "}, [%8];"
+            : "=r"(r[o + 0]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7])
+            : "r"(taddr) : "memory");
+    }
+    if (N == 16) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {"
+            "%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15"
+            "}, [%16];"
+            : "=r"(r[o + 0]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7]),
+              "=r"(r[o + 8]), "=r"(r[o + 9]), "=r"(r[o + 10]), "=r"(r[o + 11]), "=r"(r[o + 12]), "=r"(r[o + 13]), "=r"(r[o + 14]), "=r"(r[o + 15])
+            : "r"(taddr) : "memory");
+    }
+    if (N == 32) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {"
+            "%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31"
+            "}, [%32];"
+            : "=r"(r[o + 0]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7]),
+              "=r"(r[o + 8]), "=r"(r[o + 9]), "=r"(r[o + 10]), "=r"(r[o + 11]), "=r"(r[o + 12]), "=r"(r[o + 13]), "=r"(r[o + 14]), "=r"(r[o + 15]),
+              "=r"(r[o + 16]), "=r"(r[o + 17]), "=r"(r[o + 18]), "=r"(r[o + 19]), "=r"(r[o + 20]), "=r"(r[o + 21]), "=r"(r[o + 22]), "=r"(r[o + 23]),
+              "=r"(r[o + 24]), "=r"(r[o + 25]), "=r"(r[o + 26]), "=r"(r[o + 27]), "=r"(r[o + 28]), "=r"(r[o + 29]), "=r"(r[o + 30]), "=r"(r[o + 31])
+            : "r"(taddr) : "memory");
+    }
+}
+template <int CW>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[CW]) {
+    tmem_ld_n<(CW >= 32 ? 32 : CW)>(taddr, r, 0);
+    if (CW > 32) tmem_ld_n<(CW > 32 ? CW - 32 : 8)>(taddr + 32, r, 32);
+}
+// The registers pass through the wait (eight at a time), so that nothing that reads them can be scheduled ahead of it.
+template <int CW>
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[CW]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < CW; i += 8)
+        asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]), "+r"(r[i + 7]));
+}
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) { return (uint64_t)hi << 32 | lo; }
+__device__ __forceinline__ float lo_f(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi_f(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float redux_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float ex2(float v) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// Finishes neighbouring activation rows m, m + 1 of this thread's weight row n, two at a time from row m0 on. Called by
+// whole warps whose lanes hold 32 consecutive n (plane outputs trade values between neighbouring lanes).
+template <int P, int MODE>
+struct Finish {
+    const TcArgs& a;
+    bool real, odd;
+    float bias;
+    size_t at;                // offset of (m, n) in the output (plane outputs: of the pair or row this lane stores)
+    __device__ __forceinline__ Finish(const TcArgs& a_, int n, int lane, int m0) : a(a_), real(n < a_.N), odd(lane & 1) {
+        bias = a.bias && real ? __ldg(a.bias + n) : 0.0f;
+        at = MODE == OUT_F32 ? (size_t)m0 * a.ldy + n
+                             : (size_t)(m0 + odd) * a.ldy + (MODE == OUT_SWIGLU ? n >> 1 : n & ~1);
+    }
+    // The residual of rows m + 2 i and m + 2 i + 1. Asked for ahead of a run of stores: the residual may be the output
+    // itself, so the compiler cannot move the loads of the next pair above the stores of this one.
+    __device__ __forceinline__ void residual(int i, int left, float& r0, float& r1) const {
+        const float* r = a.residual + at + (size_t)(2 * i) * a.ldy;
+        r0 = real && left > 0 ? r[0] : 0.0f;
+        r1 = real && left > 1 ? r[a.ldy] : 0.0f;
+    }
+    // left: rows from m on that exist (at least 1); r0, r1: their residual
+    __device__ __forceinline__ void operator()(int left, float v0, float v1, float r0 = 0.0f, float r1 = 0.0f) {
+        v0 += bias;
+        v1 += bias;
+        if (MODE == OUT_GELU) { v0 = gelu_f(v0); v1 = gelu_f(v1); }
+        if (MODE == OUT_F32) {
+            if (a.gelu) { v0 = gelu_f(v0); v1 = gelu_f(v1); }
+            if (real) {
+                float* y = a.y + at;
+                if (a.residual) { v0 = r0 + v0; v1 = r1 + v1; }
+                y[0] = v0;
+                if (left > 1) y[a.ldy] = v1;
+            }
+        } else if (MODE == OUT_SWIGLU) {
+            // rows (2j, 2j + 1) of the weight are (gate_j, up_j) (llm.rs:417-428): the even lane finishes row m, the odd
+            // lane row m + 1, each with one value from its neighbour
+            const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+            const float g = odd ? got : v0, u = odd ? v1 : got;
+            const float h = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), u);
+            if (real && (!odd || left > 1)) {
+                uint32_t w[P];
+                split2<P>(h, 0.0f, w);
+#pragma unroll
+                for (int p = 0; p < P; ++p) a.yp[p][at] = (uint16_t)w[p];
+            }
+        } else {
+            // lanes (2i, 2i + 1) hold neighbouring columns: after the trade the even lane owns row m of both, the odd
+            // lane row m + 1, and a half warp writes one 64-byte run
+            uint32_t w[P], out[P];
+            split2<P>(v0, v1, w);
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, __byte_perm(w[0], w[1], odd ? 0x5410 : 0x7632), 1);
+            out[0] = __byte_perm(w[0], got, odd ? 0x3254 : 0x5410);
+            out[1] = __byte_perm(w[1], got, odd ? 0x3276 : 0x7610);
+            if (P == 3) {
+                const uint32_t g2 = __shfl_xor_sync(0xffffffffu, w[P - 1], 1);
+                out[P - 1] = __byte_perm(w[P - 1], g2, odd ? 0x3276 : 0x5410);
+            }
+            if (real && (!odd || left > 1)) {
+#pragma unroll
+                for (int p = 0; p < P; ++p) *(uint32_t*)(a.yp[p] + at) = out[p];
+            }
+        }
+        at += 2 * (size_t)a.ldy;
+    }
 };
 
 }  // namespace
 
+// CW: columns a drain warp handles (its half of the nt columns, or more: what lies beyond its own is folded into registers
+// that nothing stores): 32, 64 or 80, loaded in one or two parts. A compile-time number, and no more than 80: with a branch
+// around each part, or with 128 columns, the compiler's moves and spills cost more than the larger tile saves.
+template <int CG, int P, int MODE, int CW>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_q8_bf16x3_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo, const TcArgs a) {
+gemm_q8_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
+                  const __grid_constant__ CUtensorMap map2, const TcArgs a) {
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    Bars* bars = (Bars*)(smem + STAGES * STAGE_BYTES);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nkb = a.K / BK;
-    const int tiles_n = (a.N + BN - 1) / BN, tiles_m = (a.M + BM - 1) / BM;
+    // offsets, not casts, so that every access below is known to be to shared memory
+    unsigned char* smem = smem_raw + ((1024 - (s32(smem_raw) & 1023)) & 1023);
+    __half* scales = (__half*)(smem + a.stages * a.stage_bytes);                 // [stages + SCALE_EXTRA][128 rows]
+    float4* recs = (float4*)((unsigned char*)scales + (a.stages + SCALE_EXTRA) * SCALE_BYTES);   // OUT_SCORE only
+    unsigned char* tail = (unsigned char*)recs + (MODE == OUT_SCORE ? SCORE_BYTES : 0);
+    volatile int* abort = (volatile int*)(tail + BAR_ABORT);
+    const uint32_t sb = s32(smem), full = s32(tail) + BAR_FULL, empty = s32(tail) + BAR_EMPTY;
+    const uint32_t acc_full = s32(tail) + BAR_ACC_FULL, acc_empty = s32(tail) + BAR_ACC_EMPTY;
+    // the warp index through a shuffle: everything computed from it is then known to be the same for the whole warp and
+    // stays out of the vector registers, of which the drain warps have none to spare
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int csize = CG == 2 ? 2 : a.ksplit;
+    const int rank = CG == 2 || csize > 1 ? (int)(blockIdx.x % csize) : 0;          // rank in the cluster (clusters are 1-d)
+    const int group = blockIdx.x / csize, n_groups = gridDim.x / csize;             // clusters take tiles in turn
+    const int tiles_n = (a.N + 128 * CG - 1) / (128 * CG), tiles_m = (a.M + a.nt - 1) / a.nt;
     const int n_tiles = tiles_n * tiles_m;
+    const int nb = a.K >> 5;                                                        // 32-wide k-blocks of a row
+    const int nst = (nb + 1) >> 1;                                                  // 64-wide stages of a row
+    // this CTA's share of the K range, in stages (all of it unless the cluster splits K)
+    const int st0 = CG == 2 ? 0 : rank * nst / csize, st1 = CG == 2 ? nst : (rank + 1) * nst / csize;
+    const int xr = a.nt / CG;                                                       // activation rows in this CTA's shared memory
+    const bool leader = CG == 1 || rank == 0;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(&bars->full_a[s], 1);
-            mbar_init(&bars->full_b[s], DQ_WARPS);
-            mbar_init(&bars->empty[s], 1);
+        for (int s = 0; s < a.stages; ++s) {
+            mbar_init(full + 8 * s, 1 + DQ_WARPS * CG);
+            mbar_init(empty + 8 * s, 2);
         }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&bars->acc_full[b], 1);
-            mbar_init(&bars->acc_empty[b], EPI_WARPS);
+        for (int b = 0; b < MAX_BUFS; ++b) {
+            mbar_init(acc_full + 8 * b, 1);
+            mbar_init(acc_empty + 8 * b, DRAIN_WARPS * CG);
         }
-        bars->abort = 0;
+        *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == MMA_WARP) {   // the MMA warp owns the tensor memory allocation
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&bars->tmem_base)), "r"((uint32_t)TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (warp == MMA_WARP) {   // the MMA warp owns the tensor memory allocation (with CG = 2 one warp of each CTA takes part)
+        if (CG == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tail + BAR_TMEM)), "r"((uint32_t)TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tail + BAR_TMEM)), "r"((uint32_t)TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (CG == 2 || csize > 1) {
+        __syncwarp();
+        cluster_sync();
+    }
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = bars->tmem_base;
+    const uint32_t tmem = *(volatile uint32_t*)(tail + BAR_TMEM);
 
-    if (warp == TMA_WARP) {
-        // ---------------------------------------------------------------- TMA producer
-        if (lane == 0 && !a.withhold) {
-            int it = 0;                                   // k-blocks issued so far, over all tiles
-            for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-                const int m0 = (tile / tiles_n) * BM;
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!wait_bar(bars, &bars->empty[s], ((it / STAGES) & 1) ^ 1, a.status, a.wait_cycles)) { tile = n_tiles; break; }
-                    unsigned char* st = smem + s * STAGE_BYTES;
-                    mbar_expect_tx(&bars->full_a[s], 2 * A_BYTES);
-                    tma_load_2d(st, &map_hi, kb * BK, m0, &bars->full_a[s]);
-                    tma_load_2d(st + A_BYTES, &map_lo, kb * BK, m0, &bars->full_a[s]);
+    // the barriers the pair's MMA issuers wait on are the leader's
+    const uint32_t full_leader = CG == 2 ? mapa(full, 0) : full, acc_empty_leader = CG == 2 ? mapa(acc_empty, 0) : acc_empty;
+
+    // Every role ends here: nobody leaves while a peer may still reach this CTA's shared memory or barriers. After an
+    // aborted wait, copies and MMAs may be in flight for a few microseconds more: outstay them.
+    auto leave = [&]() {
+        __syncwarp();
+        if (*abort) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < 200000) __nanosleep(200);
+        }
+        __syncwarp();
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (CG == 2 || csize > 1) cluster_sync();
+        else asm volatile("bar.sync 0, %0;" ::"n"(THREADS) : "memory");
+    };
+
+    if (warp >= TMA_WARP) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (warp == TMA_WARP && lane == 0 && !a.withhold) {
+            // ------------------------------------------------------------ TMA producer
+            int s = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int tile = group; tile < n_tiles && ok; tile += n_groups) {
+                const int m0 = (tile / tiles_n) * a.nt + (CG == 2 ? rank * xr : 0);
+                for (int kb = st0; kb < st1; ++kb) {
+                    ok = wait_bar<true>(empty + 8 * s, ph, abort, a);
+                    if (!ok) break;
+                    const uint32_t dst = sb + s * a.stage_bytes, bar = full_leader + 8 * s;
+                    if (leader) mbar_expect_tx(full + 8 * s, (uint32_t)(CG * P * xr * 128));
+                    tma_load_2d<CG>(dst, &map0, kb * BK, m0, bar);
+                    tma_load_2d<CG>(dst + xr * 128, &map1, kb * BK, m0, bar);
+                    if (P == 3) tma_load_2d<CG>(dst + 2 * xr * 128, &map2, kb * BK, m0, bar);
+                    if (++s == a.stages) { s = 0; ph ^= 1; }
                 }
             }
+        } else if ((warp == MMA_WARP || warp == MMA_WARP + 1) && lane == 0 && leader) {
+            // ------------------------------------------------------------ MMA issuers
+            const int h = warp - MMA_WARP;                          // the k-block of each stage that is this warp's
+            // bf16 x bf16 -> f32, M = 128 (256 for the pair), N = nt, both operands K-major
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.nt >> 3) << 17) | ((uint32_t)(8 * CG) << 24);
+            const uint64_t desc = smem_desc(sb + 64 * h);           // 32 k = 64 bytes
+            const uint32_t dhi = (uint32_t)(desc >> 32), plane = (uint32_t)xr * 8;   // descriptors count 16 bytes
+            const int total = (group < n_tiles ? (n_tiles - group + n_groups - 1) / n_groups : 0) * (st1 - st0);
+            uint32_t x = (uint32_t)desc, ph = 0, aph = 1;
+            int s = 0, kb = st0, buf = h;                           // buffers in k-block order over all tiles
+            for (int it = 0; it < total; ++it) {
+                const bool whole = 2 * kb + 1 < nb;
+                if (h == 0 || whole) {
+                    if (!wait_bar(acc_empty + 8 * buf, aph, abort, a)) break;
+                    if (!wait_bar(full + 8 * s, ph, abort, a)) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t q = x + P * plane, acc = tmem + buf * a.acc_cols;
+                    // the small terms first: they meet a small accumulator
+                    umma<CG, false>(acc, q, x + (P - 1) * plane, dhi, idesc);
+                    umma<CG, true>(acc, q + 2, x + (P - 1) * plane + 2, dhi, idesc);
+#pragma unroll
+                    for (int p = P - 2; p >= 0; --p) {
+                        umma<CG, true>(acc, q, x + p * plane, dhi, idesc);
+                        umma<CG, true>(acc, q + 2, x + p * plane + 2, dhi, idesc);
+                    }
+                    umma_commit<CG>(acc_full + 8 * buf);
+                } else if (!wait_bar(full + 8 * s, ph, abort, a)) {
+                    break;
+                }
+                umma_commit<CG>(empty + 8 * s);                      // frees the stage when both issuers' MMAs have retired
+                x += (uint32_t)a.stage_bytes / 16;
+                if (++s == a.stages) { s = 0; ph ^= 1; x = (uint32_t)desc; }
+                if (++kb == st1) kb = st0;
+                buf += whole ? 2 : 1;
+                if (buf >= a.bufs) { buf -= a.bufs; aph ^= 1; }
+            }
         }
-    } else if (warp == MMA_WARP) {
-        // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            int it = 0, ti = 0;
+        leave();
+        if (csize > 1 && CG == 1) cluster_sync();
+        if (warp == MMA_WARP) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS) : "memory");
+            else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS) : "memory");
+        }
+    } else if (warp >= DRAIN_WARPS) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        // ---------------------------------------------------------------- weight levels -> bf16
+        const int row = (threadIdx.x - DRAIN_WARPS * 32) >> 1, hk = threadIdx.x & 1;  // weight row of the CTA's tile, half of its 64 levels
+        int s = 0, slot = 0;
+        uint32_t ph = 1;
+        bool ok = true;
+        for (int tile = group; tile < n_tiles && ok; tile += n_groups) {
+            const int n = (tile % tiles_n) * (128 * CG) + (CG == 2 ? rank * 128 : 0) + row;
+            const bool real = n < a.N_pad;
+            const __half* dsrc = a.d + (size_t)(real ? n : 0) * nb;
+            const uint4* src = (const uint4*)(a.qu + (size_t)(real ? n : 0) * a.K);
+            const uint4 zero = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);   // biased zeros
+            // two stages of levels and scales are under way at any time, in two sets of registers that take turns: with one
+            // stage ahead, a stage could not come more often than an L2 round trip
+            struct Row { uint4 q[2]; __half d; } ra, rb;
+            auto fetch = [&](Row& r, int kb) {
+                const bool have = real && kb < st1 && 2 * kb + hk < nb;
+                if (have) r.d = dsrc[2 * kb + hk];
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    r.q[i] = have ? __ldg(src + (2 * kb + hk) * 2 + i) : make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);   // biased zeros
+            };
+            auto put = [&](Row& r, int kb) {
+                ok = wait_bar<true>(empty + 8 * s, ph, abort, a);
+                if (!ok) return;
+                scales[slot * 256 + row * 2 + hk] = r.d;
+                slot = slot == a.stages + SCALE_EXTRA - 1 ? 0 : slot + 1;
+                unsigned char* dst = smem + s * a.stage_bytes + P * xr * 128 + row * 128;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {                                       // 16-byte chunk: 8 levels
+                    const uint32_t w0 = (&r.q[c >> 1].x)[(c & 1) * 2], w1 = (&r.q[c >> 1].x)[(c & 1) * 2 + 1];
+                    uint32_t o[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        // u = q + 128 in 16-bit lanes. bf16 has 7 stored bits: 0x4300 | (u & 127) is 128 + (u & 127), and
+                        // bit 7 of u turns -256 (0xC380) into -128 (0xC300), so that the sum is q, exactly
+                        const uint32_t t = __byte_perm(i < 2 ? w0 : w1, 0, (i & 1) ? 0x4342 : 0x4140);
+                        const uint32_t hi = (t & 0x007F007Fu) | 0x43004300u, sub = (t & 0x00800080u) ^ 0xC380C380u;
+                        asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(o[i]) : "r"(hi), "r"(sub));
+                    }
+                    *(uint4*)(dst + (((hk * 4 + c) ^ (row & 7)) * 16)) = make_uint4(o[0], o[1], o[2], o[3]);   // 128-byte swizzle
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // generic writes -> tensor-core reads
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(full_leader + 8 * s);
+                // after the fence: it waits for every load under way, new ones included (1400 cycles a stage with them)
+                fetch(r, kb + 2);
+                if (++s == a.stages) { s = 0; ph ^= 1; }
+            };
+            fetch(ra, st0);
+            fetch(rb, st0 + 1);
+            for (int kb = st0; kb < st1 && ok; kb += 2) {
+                put(ra, kb);
+                if (ok && kb + 1 < st1) put(rb, kb + 1);
+            }
+        }
+        leave();
+        if (csize > 1 && CG == 1) cluster_sync();
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+        // ---------------------------------------------------------------- drain and finish
+        const int quarter = warp & 3, part = warp >> 2;                             // 32 TMEM lanes, half of the columns
+        const int cw = a.nt >> 1;                                                   // columns of this warp (a multiple of 8)
+        const uint32_t taddr0 = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part * cw);
+        const __half2* my_scale = (const __half2*)scales + quarter * 32 + lane;
+        int slot = 0;
+        uint32_t fph = 0;                                                           // phase of the acc_full barriers
+        int buf = 0;
+        for (int tile = group; tile < n_tiles; tile += n_groups) {
+            uint64_t acc[CW / 2];
+#pragma unroll
+            for (int i = 0; i < CW / 2; ++i) acc[i] = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++ti) {
-                const int buf = ti & 1;
-                // the epilogue must have drained this accumulator (two tiles ago)
-                ok = wait_bar(bars, &bars->acc_empty[buf], ((ti >> 1) & 1) ^ 1, a.status, a.wait_cycles);
+            __half2 sc = __half2half2(__float2half(0.0f));
+#pragma unroll 1
+            for (int b = 2 * st0; b < min(2 * st1, nb); ++b) {
+                ok = __all_sync(0xffffffffu, wait_bar(acc_full + 8 * buf, fph, abort, a));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc = tmem + (uint32_t)(buf * 2 * BN);     // rows 0..127 here, rows 128..255 at + BN
-                for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t par = (it / STAGES) & 1;
-                    ok = wait_bar(bars, &bars->full_a[s], par, a.status, a.wait_cycles) && wait_bar(bars, &bars->full_b[s], par, a.status, a.wait_cycles);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t base = s32(smem + s * STAGE_BYTES);
-                    const uint64_t bh = smem_desc(base + 2 * A_BYTES), bl = smem_desc(base + 2 * A_BYTES + TILE_BYTES);
+                constexpr int LW = CW > 40 ? CW / 2 : CW;                                // columns of one load
+                if (!(b & 1)) {
+                    sc = my_scale[slot * 128];
+                    slot = slot == a.stages + SCALE_EXTRA - 1 ? 0 : slot + 1;
+                }
+                const float scale = b & 1 ? __high2float(sc) : __low2float(sc);
+                const uint64_t sc2 = pack2(__float_as_uint(scale), __float_as_uint(scale));
 #pragma unroll
-                    for (int hm = 0; hm < 2; ++hm) {                     // the two 128-row halves of the X tile
-                        const uint64_t ah = smem_desc(base + hm * TILE_BYTES), al = smem_desc(base + A_BYTES + hm * TILE_BYTES);
-#pragma unroll
-                        for (int ks = 0; ks < BK / 16; ++ks) {
-                            const uint64_t adv = (uint64_t)(ks * 2);    // 32 bytes per k-step of 16 bf16
-                            umma(acc + hm * BN, ah + adv, bh + adv, (kb | ks) != 0);
-                            umma(acc + hm * BN, al + adv, bh + adv, 1);
-                            umma(acc + hm * BN, ah + adv, bl + adv, 1);
-                        }
+                for (int o = 0; o < CW; o += LW) {
+                    uint32_t r[LW];
+                    tmem_ld<LW>(taddr0 + (uint32_t)(buf * a.acc_cols + o), r);
+                    tmem_wait<LW>(r);
+                    if (o + LW == CW) {
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        if (lane == 0) mbar_arrive_cluster(acc_empty_leader + 8 * buf);
                     }
-                    umma_commit(&bars->empty[s]);                    // frees the stage when the MMAs retire
+#pragma unroll
+                    for (int i = 0; i < LW / 2; ++i) fma2(acc[o / 2 + i], pack2(r[2 * i], r[2 * i + 1]), sc2);
                 }
-                if (ok) umma_commit(&bars->acc_full[buf]);
+                if (++buf == a.bufs) { buf = 0; fph ^= 1; }
             }
-        }
-    } else if (warp >= EPI_WARPS) {
-        // ---------------------------------------------------------------- weight dequantisers
-        const int t = threadIdx.x - EPI_WARPS * 32;  // 0..255
-        const int row = t >> 1, half = t & 1;        // weight row of the tile, 32-wide half of the k-block
-        int it = 0;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-            const int n0 = (tile % tiles_n) * BN;
-            const size_t n = (size_t)(n0 + row);     // < N_pad (zero rows past N)
-            const uint8_t* qrow = a.qu + n * a.K + half * 32;
-            const __half* drow = a.d + n * (a.K >> 5) + half;
-            // two k-blocks of quants are kept in flight ahead of the one being converted; they
-            // rotate through named registers (an array indexed by kb & 1 would live in local memory)
-            const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
-            uint4 qa0 = z4, qc0 = z4, qa1 = z4, qc1 = z4;
-            float sc0 = 0.0f, sc1 = 0.0f;
-            if (0 < nkb) {
-                qa0 = __ldg((const uint4*)qrow);
-                qc0 = __ldg((const uint4*)qrow + 1);
-                sc0 = __half2float(__ldg(drow));
-            }
-            if (1 < nkb) {
-                qa1 = __ldg((const uint4*)(qrow + (size_t)BK));
-                qc1 = __ldg((const uint4*)(qrow + (size_t)BK) + 1);
-                sc1 = __half2float(__ldg(drow + 2));
-            }
-            for (int kb = 0; kb < nkb; ++kb, ++it) {
-                const int s = it % STAGES;
-                const uint4 c0 = qa0, c1 = qc0;
-                const float scale = sc0;
-                qa0 = qa1; qc0 = qc1; sc0 = sc1;
-                if (kb + 2 < nkb) {
-                    qa1 = __ldg((const uint4*)(qrow + (size_t)(kb + 2) * BK));
-                    qc1 = __ldg((const uint4*)(qrow + (size_t)(kb + 2) * BK) + 1);
-                    sc1 = __half2float(__ldg(drow + (kb + 2) * 2));
-                }
-                // the conversion runs before the stage is waited for: only the stores sit between
-                // the stage becoming free and becoming full again
-                const uint32_t ws[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-                uint4 hi[4], lo[4];
+            if (!ok) break;
+            const int n = (tile % tiles_n) * (128 * CG) + (CG == 2 ? rank * 128 : 0) + quarter * 32 + lane;
+            const int m0 = (tile / tiles_n) * a.nt + part * cw;
+            if (CG == 1 && csize > 1) {
+                // partial sums [column][128 rows] into the stage buffers: every MMA and copy of this CTA is done
+                float* sum = (float*)smem + (size_t)(part * cw) * 128 + quarter * 32 + lane;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {        // 16-byte chunk c of this half: 8 weights
-                    split2(scale * qb<0>(ws[2 * c]), scale * qb<1>(ws[2 * c]), &hi[c].x, &lo[c].x);
-                    split2(scale * qb<2>(ws[2 * c]), scale * qb<3>(ws[2 * c]), &hi[c].y, &lo[c].y);
-                    split2(scale * qb<0>(ws[2 * c + 1]), scale * qb<1>(ws[2 * c + 1]), &hi[c].z, &lo[c].z);
-                    split2(scale * qb<2>(ws[2 * c + 1]), scale * qb<3>(ws[2 * c + 1]), &hi[c].w, &lo[c].w);
-                }
-                if (!wait_bar(bars, &bars->empty[s], ((it / STAGES) & 1) ^ 1, a.status, a.wait_cycles)) { tile = n_tiles; break; }
-                unsigned char* bhi = smem + s * STAGE_BYTES + 2 * A_BYTES + row * 128;
-                unsigned char* blo = bhi + TILE_BYTES;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int chunk = ((half * 4 + c) ^ (row & 7)) * 16;   // 128-byte swizzle
-                    *(uint4*)(bhi + chunk) = hi[c];
-                    *(uint4*)(blo + chunk) = lo[c];
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> tensor-core reads
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars->full_b[s]);
-            }
-        }
-    } else {
-        // ---------------------------------------------------------------- epilogue (warps 0-7)
-        const bool vec_ok = (a.ldy & 3) == 0 && (((uintptr_t)a.y | (uintptr_t)a.residual) & 15) == 0;
-        // rows of 32 columns start on 32-byte boundaries: whole-sector accesses
-        const bool vec8_ok = (a.ldy & 7) == 0 && (((uintptr_t)a.y | (uintptr_t)a.residual) & 31) == 0;
-        int ti = 0;
-        // EPI_SCORE: running (largest logit, sum of exponentials relative to it, its first column) of this lane's row
-        // over the four 32-column chunks of a tile, and the row's target
-        float run_m = -INFINITY, run_s = 0.0f;
-        int run_i = 0x7fffffff, tgt = -1;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++ti) {
-            const int buf = ti & 1;
-            const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
-            if (!wait_bar(bars, &bars->acc_full[buf], (ti >> 1) & 1, a.status, a.wait_cycles)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int hm = warp >> 2, quarter = warp & 3;                // 128-row half of the tile, 32-lane quarter of TMEM
-#pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {                          // 32-column chunk
-                const int m = m0 + hm * 128 + quarter * 32 + lane;
-                uint32_t r[32];
-                const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((buf * 2 + hm) * BN + c * 32);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                    "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                      "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                      "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                    : "r"(taddr) : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (c == BN / 32 - 1) {
-                    // this warp's part of the accumulator is in registers: hand the TMEM buffer back to the MMA warp
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->acc_empty[buf]);
-                }
-                const int nb = n0 + c * 32;
-                if (a.epi == EPI_SCORE) {
-                    if (c == 0) {
-                        run_m = -INFINITY; run_s = 0.0f; run_i = 0x7fffffff;
-                        tgt = m < a.M ? __ldg(a.targets + m) : -1;
-                    }
-                    if (m < a.M && nb < a.N) {
-                        // this chunk's largest logit and its first column (columns past N do not exist)
-                        float cm = -INFINITY;
-                        int ci = 0x7fffffff;
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const float t = __uint_as_float(r[i]);
-                            if (nb + i < a.N && t > cm) { cm = t; ci = nb + i; }
-                        }
-                        if (cm > run_m) {                      // strictly larger: an equal later column never replaces an earlier one
-                            run_s *= expf(run_m - cm);          // run_m == -inf: run_s is 0 and stays 0
-                            run_m = cm;
-                            run_i = ci;
-                        }
-                        float e = 0.0f;
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (nb + i < a.N) e += expf(__uint_as_float(r[i]) - run_m);
-                        run_s += e;
-                        if (tgt >= nb && tgt < nb + 32) {
-                            float tl = 0.0f;
-#pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                                if (nb + i == tgt) tl = __uint_as_float(r[i]);
-                            a.tlogit[m] = tl;
-                        }
-                    }
-                    if (c == BN / 32 - 1 && m < a.M)
-                        a.stats[(size_t)m * tiles_n + (tile % tiles_n)] = make_float4(run_m, run_s, __int_as_float(run_i), 0.0f);
-                } else
-                if (m < a.M && nb < a.N) {
-                const bool full = nb + 32 <= a.N;
-                float v[32];
-                const size_t off = (size_t)m * a.ldy + nb;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    float t = __uint_as_float(r[i]);
-                    if (a.bias && (full || nb + i < a.N)) t += __ldg(a.bias + nb + i);
-                    if (a.epi == EPI_GELU) t = gelu_f(t);
-                    v[i] = t;
-                }
-                if (a.residual) {
-                    if (full && vec8_ok) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            uint32_t rr[8];
-                            ld256(a.residual + off + 8 * i, rr);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) v[8 * i + j] = __uint_as_float(rr[j]) + v[8 * i + j];
-                        }
-                    } else if (full && vec_ok) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const float4 rr = *(const float4*)(a.residual + off + 4 * i);
-                            v[4 * i] = rr.x + v[4 * i]; v[4 * i + 1] = rr.y + v[4 * i + 1];
-                            v[4 * i + 2] = rr.z + v[4 * i + 2]; v[4 * i + 3] = rr.w + v[4 * i + 3];
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (nb + i < a.N) v[i] = a.residual[off + i] + v[i];
+                for (int i = 0; i < CW / 2; ++i) {
+                    if (2 * i < cw) {
+                        sum[(2 * i) * 128] = lo_f(acc[i]);
+                        sum[(2 * i + 1) * 128] = hi_f(acc[i]);
                     }
                 }
-                if (a.y) {
-                    if (full && vec8_ok) {
+            } else if (MODE == OUT_SCORE) {
+                // softmax records of (activation row, 128 weight rows): each warp reduces its 32 lanes per column, the
+                // four quarters meet in shared memory. Lane l ends up with column 32 j + l of its warp.
+                const float kLog2e = 1.4426950408889634f;
+                const bool real = n < a.N;
+                const int nq = n - lane;
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");        // the records of the tile before are read
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            uint32_t w[8];
+                for (int j = 0; j < CW / 32; ++j) {
+                    float e[32], my_max = -INFINITY;
+                    int my_idx = 0x7fffffff;
+                    const int mt = m0 + j * 32 + lane;
+                    const int tgt = j * 32 + lane < cw && mt < a.M ? __ldg(a.targets + mt) : -1;
+                    const uint32_t hits = __ballot_sync(0xffffffffu, tgt >= nq && tgt < nq + 32);
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) w[j] = __float_as_uint(v[8 * i + j]);
-                            st256(a.y + off + 8 * i, w);
+                    for (int i = 0; i < 32; ++i) {
+                        const float v = (i & 1) ? hi_f(acc[j * 16 + i / 2]) : lo_f(acc[j * 16 + i / 2]);
+                        const float t = real ? v : -INFINITY;
+                        const float mx = redux_max(t);
+                        const uint32_t at = __ballot_sync(0xffffffffu, t == mx);
+                        e[i] = real ? ex2((v - mx) * kLog2e) : 0.0f;
+                        if (lane == i) { my_max = mx; my_idx = nq + __ffs(at) - 1; }
+                        if (hits >> i & 1) {                                         // some lane's row is the target of column i
+                            const int tg = __shfl_sync(0xffffffffu, tgt, i);
+                            if (n == tg) a.tlogit[m0 + j * 32 + i] = v;
                         }
-                    } else if (full && vec_ok) {
+                    }
+                    // transposing sum: 16 + 8 + 4 + 2 + 1 exchanges leave lane l with the sum of column l
 #pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            *(float4*)(a.y + off + 4 * i) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                    } else {
+                    for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (nb + i < a.N) a.y[off + i] = v[i];
+                        for (int i = 0; i < o; ++i) {
+                            const bool up = lane & o;
+                            const float keep = up ? e[i + o] : e[i], send = up ? e[i] : e[i + o];
+                            e[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                        }
+                    }
+                    if (j * 32 + lane < cw)
+                        recs[quarter * 128 + part * cw + j * 32 + lane] = make_float4(my_max, e[0], __int_as_float(nq < a.N ? my_idx : 0x7fffffff), 0.0f);
+                }
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");
+                const int c = quarter * 32 + lane, m = m0 + c;
+                const int t128 = (tile % tiles_n) * CG + (CG == 2 ? rank : 0), n128 = (a.N + 127) / 128;
+                if (c < cw && m < a.M && t128 < n128) {
+                    float mx = -INFINITY, sum = 0.0f;
+                    int idx = 0x7fffffff;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) mx = fmaxf(mx, recs[q * 128 + part * cw + c].x);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float4 r = recs[q * 128 + part * cw + c];
+                        if (r.x > -INFINITY || r.y != 0.0f) sum += r.y * ex2((r.x - mx) * kLog2e);
+                        if (r.x == mx) idx = min(idx, __float_as_int(r.z));
+                    }
+                    a.stats[(size_t)m * n128 + t128] = make_float4(mx, sum, __int_as_float(idx), 0.0f);
+                }
+            } else {
+                const int left = a.M - m0;
+                Finish<P, MODE> fin(a, n, lane, m0);
+                if (MODE == OUT_F32 && a.residual) {
+                    constexpr int RB = CW / 4;                                       // pairs per batch
+#pragma unroll
+                    for (int o = 0; o < CW / 2; o += RB) {
+                        float r[2 * RB];
+#pragma unroll
+                        for (int i = 0; i < RB; ++i) fin.residual(i, min(cw, left) - 2 * (o + i), r[2 * i], r[2 * i + 1]);
+#pragma unroll
+                        for (int i = 0; i < RB; ++i)
+                            if (2 * (o + i) < cw && 2 * (o + i) < left)
+                                fin(left - 2 * (o + i), lo_f(acc[o + i]), hi_f(acc[o + i]), r[2 * i], r[2 * i + 1]);
                     }
                 } else {
-                    if (a.epi == EPI_SWIGLU) {
-                        // columns (2j, 2j + 1) are (gate_j, up_j) (llm.rs:417-428): 16 gated values, planes [M][N / 2]
-                        uint32_t hi8[8], lo8[8];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const float g0 = v[4 * i], g1 = v[4 * i + 2];
-                            const float h0 = __fmul_rn(__fdiv_rn(g0, __fadd_rn(1.0f, expf(-g0))), v[4 * i + 1]);
-                            const float h1 = __fmul_rn(__fdiv_rn(g1, __fadd_rn(1.0f, expf(-g1))), v[4 * i + 3]);
-                            split2(h0, h1, &hi8[i], &lo8[i]);
-                        }
-                        const size_t o2 = (size_t)m * a.ldy + (nb >> 1);
-                        if ((((uintptr_t)a.yhi | (uintptr_t)a.ylo) & 31) == 0 && (a.ldy & 15) == 0) {
-                            st256(a.yhi + o2, hi8);
-                            st256(a.ylo + o2, lo8);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 2; ++i) {
-                                *(uint4*)(a.yhi + o2 + 8 * i) = make_uint4(hi8[4 * i], hi8[4 * i + 1], hi8[4 * i + 2], hi8[4 * i + 3]);
-                                *(uint4*)(a.ylo + o2 + 8 * i) = make_uint4(lo8[4 * i], lo8[4 * i + 1], lo8[4 * i + 2], lo8[4 * i + 3]);
-                            }
-                        }
-                    } else {
-                    // bf16 hi / lo planes for the next GEMM (ldy % 8 == 0, N % 32 == 0 for these outputs)
-                    uint32_t hi[16], lo[16];
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) split2(v[2 * i], v[2 * i + 1], &hi[i], &lo[i]);
-                    if ((((uintptr_t)a.yhi | (uintptr_t)a.ylo) & 31) == 0 && (a.ldy & 15) == 0) {
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            st256(a.yhi + off + 16 * i, hi + 8 * i);
-                            st256(a.ylo + off + 16 * i, lo + 8 * i);
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            *(uint4*)(a.yhi + off + 8 * i) = make_uint4(hi[4 * i], hi[4 * i + 1], hi[4 * i + 2], hi[4 * i + 3]);
-                            *(uint4*)(a.ylo + off + 8 * i) = make_uint4(lo[4 * i], lo[4 * i + 1], lo[4 * i + 2], lo[4 * i + 3]);
-                        }
-                    }
-                    }
+                    for (int i = 0; i < CW / 2; ++i)
+                        if (2 * i < cw && 2 * i < left) fin(left - 2 * i, lo_f(acc[i]), hi_f(acc[i]));
                 }
-                }
-                __syncwarp();      // the next tcgen05.ld is warp-collective
             }
         }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == MMA_WARP) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS) : "memory");
+        leave();
+        if (CG == 1 && csize > 1) {
+            // every rank of the cluster finishes its share of the columns, adding the partial sums in rank order
+            if (!*abort && group < n_tiles && MODE != OUT_SCORE) {
+                const int tile = group;
+                const int n = (tile % tiles_n) * 128 + quarter * 32 + lane, m0 = (tile / tiles_n) * a.nt;
+                const int share = ((a.nt + csize - 1) / csize + 1) & ~1, c1 = min(a.nt, (rank + 1) * share);
+                const uint32_t base = sb + (uint32_t)(quarter * 32 + lane) * 4;
+                for (int c = rank * share + 2 * part; c < c1; c += 4) {
+                    if (m0 + c >= a.M) break;
+                    float v0 = 0.0f, v1 = 0.0f;
+                    for (int r = 0; r < csize; ++r) {
+                        const uint32_t at = mapa(base + (uint32_t)c * 512, r);
+                        float p0, p1;
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(p0) : "r"(at) : "memory");
+                        asm volatile("ld.shared::cluster.f32 %0, [%1 + 512];" : "=f"(p1) : "r"(at) : "memory");
+                        v0 += p0;
+                        v1 += p1;
+                    }
+                    Finish<P, MODE> fin(a, n, lane, m0 + c);
+                    float r0 = 0.0f, r1 = 0.0f;
+                    if (MODE == OUT_F32 && a.residual) fin.residual(0, a.M - m0 - c, r0, r1);
+                    fin(a.M - m0 - c, v0, v1, r0, r1);
+                }
+            }
+            __syncwarp();
+            cluster_sync();
+        }
     }
 }
 
-// x[n] -> bf16 hi, lo planes with x = hi + lo to 2^-17 relative.
-__global__ void split_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, size_t n4) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
-        const float4 v = ((const float4*)x)[i];
-        uint2 h, l;
-        split2(v.x, v.y, &h.x, &l.x);
-        split2(v.z, v.w, &h.y, &l.y);
-        ((uint2*)hi)[i] = h;
-        ((uint2*)lo)[i] = l;
-    }
-}
-
-int launch_split_bf16(const float* x, void* hi, void* lo, size_t n, cudaStream_t st) {
-    if (n % 4) return fail(FC_E_SHAPE, "split_bf16: element count %zu is not a multiple of 4", n);
-    const size_t n4 = n / 4;
-    const int blocks = (int)((n4 + 255) / 256 < 148 * 8 ? (n4 + 255) / 256 : 148 * 8);
-    split_bf16_kernel<<<blocks > 0 ? blocks : 1, 256, 0, st>>>(x, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n4);
-    FC_LAUNCHED();
-    return FC_OK;
-}
-
+// ------------------------------------------------------------------------------------------------ host side
 namespace {
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int encode_plane(CUtensorMap* map, const void* plane, int M, int K) {
+int encode_plane(CUtensorMap* map, const void* plane, int M, int K, int box_rows) {
     static EncodeTiledFn fn = nullptr;
     if (!fn) {
         void* p = nullptr;
@@ -512,7 +706,7 @@ int encode_plane(CUtensorMap* map, const void* plane, int M, int K) {
     }
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
     const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)BM};   // 64 x 256: two 128-row MMA tiles
+    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)plane, dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -520,56 +714,143 @@ int encode_plane(CUtensorMap* map, const void* plane, int M, int K) {
     if (r != CUDA_SUCCESS) return fail(FC_E_CUDA, "cuTensorMapEncodeTiled failed (%d) for a [%d][%d] bf16 plane", (int)r, M, K);
     return FC_OK;
 }
-}  // namespace
 
-// x_hi / x_lo: bf16 planes [M][K] (16-byte aligned). Output: f32 rows y (ldy floats apart), or, when
-// y is null, bf16 planes y_hi / y_lo (N % 32 == 0, ldy % 8 == 0). status: device int, raised on timeout.
-static int launch_tc(const QMat& w, const void* x_hi, const void* x_lo, TcArgs a, int M, cudaStream_t st) {
-    static int sms[64] = {};
+struct TileChoice { int cg, nt, ksplit; };
+
+// Tile shape by estimated SM cycles: waves of tiles x (k-blocks x the slowest of the pipelines + what a tile costs once).
+// Per 32-wide k-block: tensor pipe planes * nt; shared-memory bandwidth (128 bytes a cycle: operand reads of the MMAs, the
+// TMA writes, the converted weights); the drain (tcgen05.ld and FMA, 32 lanes a cycle); the weight conversion.
+// split_k: the K range may be split over CTAs, which changes the order of the sums with the number of rows; callers whose
+// results may not depend on how many rows share a launch leave it out.
+TileChoice choose_tile(int M, int N, int K, int P, int mode, bool split_k, int sms) {
+    TileChoice best = {1, 16, 1};
+    double best_cost = 1e30;
+    const int nst = (K + 63) / 64;
+    auto consider = [&](int cg, int nt, int ks) {
+        const long tiles = (long)((N + 128 * cg - 1) / (128 * cg)) * ((M + nt - 1) / nt);
+        const long slots = sms / (cg * ks) < 1 ? 1 : sms / (cg * ks);
+        if (ks > 1 && (tiles > slots || ks > nst)) return;            // a split-K cluster runs one tile
+        const double waves = (double)((tiles + slots - 1) / slots);
+        const double xr = (double)nt / cg;
+        const double smem = (2.0 * P * (4096 + 32 * xr) + P * xr * 64 + 8192) / 128.0;
+        const double step = std::max(std::max((double)P * nt, smem), std::max(1.3 * nt + 110.0, 190.0));
+        const double steps = 2.0 * ((nst + ks - 1) / ks);
+        const double once = (mode == OUT_SCORE ? 16.0 : 9.0) * nt + 400.0;
+        const double cost = waves * (steps * step + once) + 2500.0 + (ks > 1 ? 1500.0 + 6.0 * nt : 0.0);
+        if (cost < best_cost) { best_cost = cost; best = {cg, nt, ks}; }
+    };
+    for (int nt = 16; nt <= 128; nt += 16)
+        for (int ks = 1; ks <= (split_k ? 8 : 1); ks *= 2) consider(1, nt, ks);
+    if (M > 64)
+        for (int nt = 64; nt <= (mode == OUT_SCORE ? 128 : 160); nt += 32) consider(2, nt, 1);   // records of 160 columns: 7 % slower head
+    return best;
+}
+
+template <int CG, int P, int MODE, int CW>
+int launch_one(const CUtensorMap (&map)[3], const TcArgs& a, int grid, int smem, cudaStream_t st) {
+    static bool ready[64] = {};
     int dev = 0;
     FC_CUDA(cudaGetDevice(&dev));
     if (dev >= 64) return fail(FC_E_ARG, "device %d out of range", dev);
-    if (!sms[dev]) {
-        FC_CUDA(cudaFuncSetAttribute(gemm_q8_bf16x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        FC_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
+    if (!ready[dev]) {
+        FC_CUDA(cudaFuncSetAttribute(gemm_q8_tc_kernel<CG, P, MODE, CW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
+        ready[dev] = true;
     }
-    CUtensorMap mh, ml;
-    FC_TRY(encode_plane(&mh, x_hi, M, w.K));
-    FC_TRY(encode_plane(&ml, x_lo, M, w.K));
-    a.qu = w.qu; a.d = w.d; a.N = w.N; a.K = w.K; a.M = M;
-    a.wait_cycles = g_debug.wait_cycles; a.withhold = g_debug.withhold;
-    const int n_tiles = ((w.N + BN - 1) / BN) * ((M + BM - 1) / BM);
-    const int grid = n_tiles < sms[dev] ? n_tiles : sms[dev];
-    gemm_q8_bf16x3_kernel<<<grid, THREADS, SMEM_BYTES, st>>>(mh, ml, a);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)(CG == 2 ? 2 : a.ksplit);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FC_CUDA(cudaLaunchKernelEx(&cfg, gemm_q8_tc_kernel<CG, P, MODE, CW>, map[0], map[1], map[2], a));
     FC_LAUNCHED();
     return FC_OK;
 }
 
-int launch_gemm_q8_bf16x3_ex(const QMat& w, const void* x_hi, const void* x_lo, const float* bias, const float* residual,
-                             int epi, float* y, void* y_hi, void* y_lo, int M, int ldy, int* status, cudaStream_t st) {
-    if (w.K % BK) return fail(FC_E_SHAPE, "the tensor-core GEMM needs K %% 64 == 0 (K = %d)", w.K);
-    if (!y && (!y_hi || !y_lo || (w.N & 31) || (ldy & 7) || residual))
-        return fail(FC_E_SHAPE, "plane output needs N %% 32 == 0, ldy %% 8 == 0 and no residual");
-    if (epi == EPI_SWIGLU && (y || ldy < w.N / 2)) return fail(FC_E_SHAPE, "the SwiGLU epilogue writes planes [M][N / 2]");
-    if (epi == EPI_SCORE) return fail(FC_E_ARG, "the scoring epilogue has its own entry");
-    TcArgs a = {};
-    a.bias = bias; a.residual = residual; a.epi = epi;
-    a.y = y; a.yhi = (uint16_t*)y_hi; a.ylo = (uint16_t*)y_lo; a.ldy = ldy; a.status = status;
-    return launch_tc(w, x_hi, x_lo, a, M, st);
+template <int MODE>
+int launch_tc(const QMat& w, const Planes& x, TcArgs a, int M, bool split_k, cudaStream_t st) {
+    static int sms[64] = {};
+    int dev = 0;
+    FC_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64) return fail(FC_E_ARG, "device %d out of range", dev);
+    if (!sms[dev]) FC_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
+    if (M <= 0) return FC_OK;
+    const int P = x.n;
+    if ((P != 2 && P != 3) || w.K % 32) return fail(FC_E_SHAPE, "the tensor-core GEMM takes 2 or 3 planes and K %% 32 == 0 (got %d, %d)", P, w.K);
+    const TileChoice t = choose_tile(M, w.N, w.K, P, MODE, split_k && MODE != OUT_SCORE, sms[dev]);
+    a.qu = w.qu; a.d = w.d; a.N = w.N; a.K = w.K; a.N_pad = w.N_pad; a.M = M;
+    a.nt = t.nt; a.ksplit = t.ksplit;
+    a.acc_cols = t.nt > 128 ? 160 : 128;
+    a.bufs = t.nt > 128 ? 3 : 4;
+    const int xr = t.nt / t.cg;
+    a.stage_bytes = P * xr * 128 + Q_BYTES;
+    const int fixed = 1024 /* alignment slack */ + SCALE_EXTRA * SCALE_BYTES + BAR_BYTES + (MODE == OUT_SCORE ? SCORE_BYTES : 0);
+    a.stages = std::min(MAX_STAGES, (SMEM_LIMIT - fixed) / (a.stage_bytes + SCALE_BYTES));
+    a.wait_cycles = g_debug.wait_cycles; a.withhold = g_debug.withhold;
+    CUtensorMap map[3];
+    for (int p = 0; p < P; ++p) FC_TRY(encode_plane(&map[p], x.p[p], M, w.K, xr));
+    if (P < 3) map[2] = map[1];
+    const int tiles = ((w.N + 128 * t.cg - 1) / (128 * t.cg)) * ((M + t.nt - 1) / t.nt);
+    const int csize = t.cg == 2 ? 2 : t.ksplit;
+    const int grid = std::min(tiles, sms[dev] / csize) * csize;
+    const int smem = a.stages * (a.stage_bytes + SCALE_BYTES) + fixed;
+    auto go = [&](auto cg, auto cw) -> int {
+        constexpr int CG = decltype(cg)::value, CW = decltype(cw)::value;
+        return P == 2 ? launch_one<CG, 2, MODE, CW>(map, a, grid, smem, st) : launch_one<CG, 3, MODE, CW>(map, a, grid, smem, st);
+    };
+    const std::integral_constant<int, 1> one;
+    const std::integral_constant<int, 2> two;
+    const std::integral_constant<int, MODE == OUT_SCORE ? 64 : 32> ws;
+    const std::integral_constant<int, 64> wm;
+    const std::integral_constant<int, MODE == OUT_SCORE ? 64 : 80> wl;
+    if (t.cg == 2) return t.nt > 128 ? go(two, wl) : t.nt > 64 ? go(two, wm) : go(two, ws);
+    return t.nt > 64 ? go(one, wm) : go(one, ws);
 }
 
-int launch_gemm_q8_bf16x3_score(const QMat& w, const void* x_hi, const void* x_lo, const int* targets, void* stats, float* tlogit,
-                                int M, int* status, cudaStream_t st) {
-    if (w.K % BK) return fail(FC_E_SHAPE, "the tensor-core GEMM needs K %% 64 == 0 (K = %d)", w.K);
+template <int P>
+__global__ void split_planes_kernel(const float* __restrict__ x, const Planes out, size_t n4) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x)
+        store_planes4<P>(out, i, ((const float4*)x)[i]);
+}
+}  // namespace
+
+int launch_split_planes(const float* x, const Planes& out, size_t n, cudaStream_t st) {
+    if (n % 4) return fail(FC_E_SHAPE, "split_planes: element count %zu is not a multiple of 4", n);
+    const size_t n4 = n / 4;
+    const int blocks = (int)std::max<size_t>(1, std::min<size_t>((n4 + 255) / 256, 148 * 8));
+    if (out.n == 3) split_planes_kernel<3><<<blocks, 256, 0, st>>>(x, out, n4);
+    else split_planes_kernel<2><<<blocks, 256, 0, st>>>(x, out, n4);
+    FC_LAUNCHED();
+    return FC_OK;
+}
+
+int launch_gemm_q8_tc(const QMat& w, const Planes& x, const float* bias, const float* residual, int epi, float* y, const Planes* yp,
+                      int M, int ldy, int* status, cudaStream_t st, bool split_k) {
+    TcArgs a = {};
+    a.bias = bias; a.residual = residual; a.gelu = epi == EPI_GELU; a.y = y; a.ldy = ldy; a.status = status;
+    if (yp) for (int p = 0; p < yp->n; ++p) a.yp[p] = (uint16_t*)yp->p[p];
+    if (epi == EPI_SWIGLU) {
+        if (y || !yp || yp->n != x.n || residual || (w.N & 1) || ldy < w.N / 2) return fail(FC_E_SHAPE, "the SwiGLU epilogue writes planes [M][N / 2]");
+        return launch_tc<OUT_SWIGLU>(w, x, a, M, split_k, st);
+    }
+    if (epi != EPI_NONE && epi != EPI_GELU) return fail(FC_E_ARG, "epilogue %d is not one of this entry's", epi);
+    if (y) return launch_tc<OUT_F32>(w, x, a, M, split_k, st);
+    if (!yp || yp->n != x.n || (w.N & 31) || (ldy & 7) || residual)
+        return fail(FC_E_SHAPE, "plane output needs N %% 32 == 0, ldy %% 8 == 0, as many planes as the input and no residual");
+    return epi == EPI_GELU ? launch_tc<OUT_GELU>(w, x, a, M, split_k, st) : launch_tc<OUT_PLANES>(w, x, a, M, split_k, st);
+}
+
+int launch_gemm_q8_tc_score(const QMat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status,
+                            cudaStream_t st) {
     if (!targets || !stats || !tlogit) return fail(FC_E_ARG, "the scoring epilogue needs targets, stats and tlogit");
     TcArgs a = {};
-    a.epi = EPI_SCORE; a.targets = targets; a.stats = (float4*)stats; a.tlogit = tlogit; a.status = status;
-    return launch_tc(w, x_hi, x_lo, a, M, st);
-}
-
-int launch_gemm_q8_bf16x3(const QMat& w, const void* x_hi, const void* x_lo, const float* bias, const float* residual,
-                          int epi, float* y, int M, int ldy, int* status, cudaStream_t st) {
-    return launch_gemm_q8_bf16x3_ex(w, x_hi, x_lo, bias, residual, epi, y, nullptr, nullptr, M, ldy, status, st);
+    a.targets = targets; a.stats = (float4*)stats; a.tlogit = tlogit; a.status = status;
+    return launch_tc<OUT_SCORE>(w, x, a, M, false, st);
 }
 
 // scoring.rs:175-181 from the per-tile records of the fused head: a warp per row folds the records in tile
@@ -680,10 +961,9 @@ extern "C" int fc_q8_0_linear_dev_noalloc(const fc_qweight* w, const float* x_de
     cudaStream_t st = (cudaStream_t)cuda_stream;
     // the status word keeps whatever the previous call left in it: start from zero
     FC_CUDA(cudaMemsetAsync(sc.status, 0, sizeof(int), st));
-    uint16_t* hi = sc.planes;
-    uint16_t* lo = sc.planes + kStaticPlaneElems;
-    FC_TRY(launch_split_bf16(x_dev, hi, lo, (size_t)M * mat->K, st));
-    FC_TRY(launch_gemm_q8_bf16x3(*mat, hi, lo, bias_dev, nullptr, EPI_NONE, y_dev, M, mat->N, sc.status, st));
+    const Planes x = {{sc.planes, sc.planes + kStaticPlaneElems, nullptr}, 2};
+    FC_TRY(launch_split_planes(x_dev, x, (size_t)M * mat->K, st));
+    FC_TRY(launch_gemm_q8_tc(*mat, x, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, mat->N, sc.status, st));
     if (timed_out) {
         FC_CUDA(cudaMemcpyAsync(timed_out, sc.status, sizeof(int), cudaMemcpyDeviceToHost, st));
         FC_CUDA(cudaStreamSynchronize(st));

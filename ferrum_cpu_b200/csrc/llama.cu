@@ -33,14 +33,12 @@ struct fc_llama {
     std::vector<LlamaLayerDev> layers;
     int q_dim = 0, kv_dim = 0, qkv_dim = 0;
     // window-forward workspace for ws_rows rows
-    int ws_rows = 0, head_chunk = 0;
+    int ws_rows = 0, ws_planes = 0, head_chunk = 0;
     float *x = nullptr, *n = nullptr, *qkv = nullptr, *att = nullptr, *gu = nullptr, *hid = nullptr, *logits = nullptr;
     int *ids_d = nullptr, *targets_d = nullptr, *err_d = nullptr, *tc_status = nullptr;
     double* lp_d = nullptr;
     uint8_t* gr_d = nullptr;
-    uint16_t *xhi = nullptr, *xlo = nullptr;
-    uint16_t *qkvhi = nullptr, *qkvlo = nullptr, *atthi = nullptr, *attlo = nullptr;   // planes around the tensor-core attention
-    uint16_t *hidhi = nullptr, *hidlo = nullptr;                                       // gated hidden state, written by the gate/up GEMM
+    Planes px, pqkv, patt, phid;     // bf16 planes: normalised rows, rotated q | k | v, attention output, gated hidden state
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_score_ms = 0.0f;
     bool force_fp32 = false;         // the batched prime keeps the cache rows at fp32 rounding
@@ -114,24 +112,20 @@ int upload_interleaved(Arena& ar, const void* a, const void* b, int rows, int K,
     return upload_q8(ar, buf.data(), 2 * rows, K, out, st);
 }
 
-int gemm(fc_llama* m, const QMat& w, const float* x, const float* bias, const float* res, float* y, int M, int ldy) {
-    if (m->cfg.math_mode == FC_MATH_BF16X3 && !m->force_fp32 && w.K % 64 == 0) {
-        FC_TRY(launch_split_bf16(x, m->xhi, m->xlo, (size_t)M * w.K, m->st));
-        return launch_gemm_q8_bf16x3(w, m->xhi, m->xlo, bias, res, EPI_NONE, y, M, ldy, m->tc_status, m->st);
-    }
-    return launch_gemm_q8_fp32(w, x, bias, res, EPI_NONE, y, M, ldy, m->st);
-}
-
-// The window attention runs on tcgen05 when the math mode allows it and heads are 64 wide (the
-// rotated q | k | v rows are split into bf16 planes for it; its output planes feed the wo GEMM).
-bool tensor_attention(const fc_llama* m) {
-    return m->cfg.math_mode == FC_MATH_BF16X3 && m->cfg.head_dim == 64 && m->cfg.d_model % 64 == 0;
+// bf16 planes the window forward splits its activations into: 3 hold an f32 exactly, 2 to 2^-17 relative (the math mode
+// FC_MATH_BF16X3, for matrices whose rows are whole 64-wide k-blocks).
+int model_planes(const fc_llama* m) {
+    const fc_llama_config& c = m->cfg;
+    return c.math_mode == FC_MATH_BF16X3 && !m->force_fp32 && c.d_model % 64 == 0 && c.d_ff % 64 == 0 && m->q_dim % 64 == 0 ? 2 : 3;
 }
 
 int ensure_workspace(fc_llama* m, int rows) {
-    if (rows <= m->ws_rows) return FC_OK;
+    const int planes = std::max(m->prec >= 0 ? 0 : model_planes(m), m->ws_planes);
+    if (rows <= m->ws_rows && planes <= m->ws_planes) return FC_OK;
+    rows = std::max(rows, m->ws_rows);
+    FC_CUDA(cudaStreamSynchronize(m->st));
     m->ws_arena.release();
-    m->ws_rows = 0;
+    m->ws_rows = m->ws_planes = 0;
     const fc_llama_config& c = m->cfg;
     const size_t R = rows, d = c.d_model, F = c.d_ff;
     size_t chunk = ((size_t)1 << 28) / (size_t)m->head.N_pad;   // logits for head_chunk rows at a time (<= 1 GiB)
@@ -141,8 +135,10 @@ int ensure_workspace(fc_llama* m, int rows) {
     FC_TRY(a.alloc_n(&m->n, R * d));
     FC_TRY(a.alloc_n(&m->qkv, R * (size_t)m->qkv_dim));
     FC_TRY(a.alloc_n(&m->att, R * (size_t)m->q_dim));
-    FC_TRY(a.alloc_n(&m->gu, R * 2 * F));
-    FC_TRY(a.alloc_n(&m->hid, R * F));
+    if (m->prec >= 0) {
+        FC_TRY(a.alloc_n(&m->gu, R * 2 * F));
+        FC_TRY(a.alloc_n(&m->hid, R * F));
+    }
     FC_TRY(a.alloc_n(&m->logits, chunk * (size_t)m->head.N_pad));
     FC_TRY(a.alloc_n(&m->ids_d, R));
     FC_TRY(a.alloc_n(&m->targets_d, R));
@@ -151,26 +147,23 @@ int ensure_workspace(fc_llama* m, int rows) {
     FC_TRY(a.alloc_n(&m->err_d, 1));
     FC_TRY(a.alloc_n(&m->tc_status, 1));
     FC_CUDA(cudaMemsetAsync(m->tc_status, 0, sizeof(int), m->st));
-    if (c.math_mode == FC_MATH_BF16X3) {
-        const size_t widest = std::max({d, F, (size_t)m->q_dim});
-        FC_TRY(a.alloc_n(&m->xhi, R * widest));
-        FC_TRY(a.alloc_n(&m->xlo, R * widest));
-        if (d % 64 == 0 && F % 64 == 0) {
-            FC_TRY(a.alloc_n(&m->hidhi, R * F));
-            FC_TRY(a.alloc_n(&m->hidlo, R * F));
-        }
-        if (tensor_attention(m)) {
-            FC_TRY(a.alloc_n(&m->qkvhi, R * (size_t)m->qkv_dim)); FC_TRY(a.alloc_n(&m->qkvlo, R * (size_t)m->qkv_dim));
-            FC_TRY(a.alloc_n(&m->atthi, R * (size_t)m->q_dim));   FC_TRY(a.alloc_n(&m->attlo, R * (size_t)m->q_dim));
-        }
-    }
+    auto make = [&](Planes* p, size_t n) -> int {
+        for (int i = 0; i < planes; ++i) FC_TRY(a.alloc(&p->p[i], n * 2));
+        return FC_OK;
+    };
+    FC_TRY(make(&m->px, R * d));
+    FC_TRY(make(&m->pqkv, R * (size_t)m->qkv_dim));
+    FC_TRY(make(&m->patt, R * (size_t)m->q_dim));
+    FC_TRY(make(&m->phid, R * F));
     m->ws_rows = rows;
+    m->ws_planes = planes;
     m->head_chunk = (int)chunk;
     return FC_OK;
 }
 
 // LlamaModel::forward_tokens (llm.rs:622-635) up to the final norm, for B windows of T rows
-// whose ids are in m->ids_d: every row r sits at position r % T. Leaves RMSNorm(h) in m->n.
+// whose ids are in m->ids_d: every row r sits at position r % T. Leaves RMSNorm(h) in m->n
+// and, for the Q8_0 model, its planes in m->px.
 // With `fill` (B == 1) the rotated keys and the values of every block become the cache's rows 0..T-1.
 int forward_rows_packed(fc_llama* m, int B, int T, fc_llama_cache* fill);
 int forward_rows(fc_llama* m, int B, int T, fc_llama_cache* fill = nullptr) {
@@ -180,53 +173,39 @@ int forward_rows(fc_llama* m, int B, int T, fc_llama_cache* fill = nullptr) {
     cudaStream_t st = m->st;
     FC_CUDA(cudaMemsetAsync(m->err_d, 0, sizeof(int), st));
     FC_TRY(launch_llama_embed_rows(m->tok, m->ids_d, R, m->x, m->err_d, st));
+    const int planes = model_planes(m);
+    m->px.n = m->pqkv.n = m->patt.n = m->phid.n = planes;
+    // the attention runs on tcgen05 on two planes and heads of 64; a cache fill needs the rotated f32 rows
+    const bool tc_attn = planes == 2 && c.head_dim == 64 && !fill && (size_t)m->qkv_dim * 4 <= 48 * 1024;
     for (int l = 0; l < c.n_layer; ++l) {
         const LlamaLayerDev& L = m->layers[l];
-        // LlamaBlock::forward_full (llm.rs:464-482)
-        const bool planes = m->cfg.math_mode == FC_MATH_BF16X3 && !m->force_fp32 && d % 64 == 0 && F % 64 == 0;
-        if (planes) {
-            // norms and the gate write the planes the next GEMM reads: no f32 copy of them, no split pass
-            FC_TRY(launch_llama_rmsnorm_planes(m->x, L.attn_norm, c.norm_eps, R, d, m->xhi, m->xlo, st));
-            FC_TRY(launch_gemm_q8_bf16x3(L.qkv, m->xhi, m->xlo, L.qkv_b, nullptr, EPI_NONE, m->qkv, R, m->qkv_dim, m->tc_status, st));
-        } else {
-            FC_TRY(launch_llama_rmsnorm(m->x, L.attn_norm, c.norm_eps, R, d, m->n, nullptr, st));
-            FC_TRY(gemm(m, L.qkv, m->n, L.qkv_b, nullptr, m->qkv, R, m->qkv_dim));
-        }
-        const bool tc_attn = tensor_attention(m) && !m->force_fp32 && !fill && (size_t)m->qkv_dim * 4 <= 48 * 1024;
+        // LlamaBlock::forward_full (llm.rs:464-482); norms and the gate write the planes the next GEMM reads
+        FC_TRY(launch_llama_rmsnorm_planes(m->x, L.attn_norm, c.norm_eps, R, d, m->px, st));
+        FC_TRY(launch_gemm_q8_tc(L.qkv, m->px, L.qkv_b, nullptr, EPI_NONE, m->qkv, nullptr, R, m->qkv_dim, m->tc_status, st, fill != nullptr));
         if (tc_attn) {
             // rotate and split in one pass: the attention reads planes, nothing reads the rotated f32 rows
             FC_TRY(launch_llama_rope_planes(m->qkv, R, m->qkv_dim, T, c.n_head, c.n_kv_head, m->q_dim, c.head_dim, c.rope_dim,
-                                            c.rope_type == FC_ROPE_NEOX, m->ftab, m->inv_linear, m->qkvhi, m->qkvlo, st));
+                                            c.rope_type == FC_ROPE_NEOX, m->ftab, m->inv_linear, m->pqkv, st));
+            FC_TRY(launch_attn_prefill_tc_gqa(m->pqkv, B, T, c.n_head, c.n_kv_head, m->patt, m->tc_status, st));
         } else {
             FC_TRY(launch_llama_rope_rows(m->qkv, R, m->qkv_dim, T, c.n_head, c.n_kv_head, m->q_dim, c.head_dim, c.rope_dim,
                                           c.rope_type == FC_ROPE_NEOX, m->ftab, m->inv_linear, st));
-        }
-        if (fill) {
-            const size_t layer_stride = (size_t)c.ctx * m->kv_dim;
-            FC_TRY(launch_llama_store_kv_rows(m->qkv, R, m->qkv_dim, m->q_dim, m->kv_dim, fill->kc + l * layer_stride,
-                                              fill->vc + l * layer_stride, st));
-        }
-        if (tc_attn) {
-            FC_TRY(launch_attn_prefill_tc_gqa(m->qkvhi, m->qkvlo, B, T, c.n_head, c.n_kv_head, m->atthi, m->attlo, m->tc_status, st));
-            FC_TRY(launch_gemm_q8_bf16x3(L.wo, m->atthi, m->attlo, nullptr, m->x, EPI_NONE, m->x, R, d, m->tc_status, st));
-        } else {
+            if (fill) {
+                const size_t layer_stride = (size_t)c.ctx * m->kv_dim;
+                FC_TRY(launch_llama_store_kv_rows(m->qkv, R, m->qkv_dim, m->q_dim, m->kv_dim, fill->kc + l * layer_stride,
+                                                  fill->vc + l * layer_stride, st));
+            }
             FC_TRY(launch_attn_prefill_gqa(m->qkv, m->qkv + m->q_dim, m->qkv + m->q_dim + m->kv_dim, B, T, m->qkv_dim, c.n_head,
                                            c.n_kv_head, c.head_dim, m->q_dim, m->att, st));
-            FC_TRY(gemm(m, L.wo, m->att, nullptr, m->x, m->x, R, d));
+            FC_TRY(launch_split_planes(m->att, m->patt, (size_t)R * m->q_dim, st));
         }
-        if (planes) {
-            FC_TRY(launch_llama_rmsnorm_planes(m->x, L.ffn_norm, c.norm_eps, R, d, m->xhi, m->xlo, st));
-            // the gate is the GEMM's epilogue: interleaved (gate, up) columns -> planes of the gated hidden state
-            FC_TRY(launch_gemm_q8_bf16x3_ex(L.gateup, m->xhi, m->xlo, nullptr, nullptr, EPI_SWIGLU, nullptr, m->hidhi, m->hidlo, R, F,
-                                            m->tc_status, st));
-            FC_TRY(launch_gemm_q8_bf16x3(L.down, m->hidhi, m->hidlo, nullptr, m->x, EPI_NONE, m->x, R, d, m->tc_status, st));
-        } else {
-            FC_TRY(launch_llama_rmsnorm(m->x, L.ffn_norm, c.norm_eps, R, d, m->n, nullptr, st));
-            FC_TRY(gemm(m, L.gateup, m->n, nullptr, nullptr, m->gu, R, 2 * F));
-            FC_TRY(launch_llama_swiglu(m->gu, R, F, m->hid, nullptr, st));
-            FC_TRY(gemm(m, L.down, m->hid, nullptr, m->x, m->x, R, d));
-        }
+        FC_TRY(launch_gemm_q8_tc(L.wo, m->patt, nullptr, m->x, EPI_NONE, m->x, nullptr, R, d, m->tc_status, st, fill != nullptr));
+        FC_TRY(launch_llama_rmsnorm_planes(m->x, L.ffn_norm, c.norm_eps, R, d, m->px, st));
+        // the gate is the GEMM's epilogue: interleaved (gate, up) columns -> planes of the gated hidden state
+        FC_TRY(launch_gemm_q8_tc(L.gateup, m->px, nullptr, nullptr, EPI_SWIGLU, nullptr, &m->phid, R, F, m->tc_status, st, fill != nullptr));
+        FC_TRY(launch_gemm_q8_tc(L.down, m->phid, nullptr, m->x, EPI_NONE, m->x, nullptr, R, d, m->tc_status, st, fill != nullptr));
     }
+    if (!fill) FC_TRY(launch_llama_rmsnorm_planes(m->x, m->out_norm, c.norm_eps, R, d, m->px, st));
     return launch_llama_rmsnorm(m->x, m->out_norm, c.norm_eps, R, d, m->n, nullptr, st);
 }
 
@@ -315,13 +294,21 @@ int check_status(fc_llama* m) {
     return FC_OK;
 }
 
+// Logits of rows r0 .. r0 + rows of the last forward_rows into m->logits (m->head.N_pad floats apart).
+int head_rows(fc_llama* m, int r0, int rows) {
+    const size_t off = (size_t)r0 * m->cfg.d_model;
+    if (m->prec >= 0) return lin_apply(m->packed_head, m->n + off, nullptr, nullptr, m->logits, m->head.N_pad, rows, m->st);
+    Planes x = m->px;
+    for (int p = 0; p < x.n; ++p) x.p[p] = (uint16_t*)x.p[p] + off;
+    return launch_gemm_q8_tc(m->head, x, nullptr, nullptr, EPI_NONE, m->logits, nullptr, rows, m->head.N_pad, m->tc_status, m->st, false);
+}
+
 // Head + scoring tail over the R rows whose normalised state is in m->n; targets in m->targets_d.
 int score_tail(fc_llama* m, int R) {
-    const int d = m->cfg.d_model, ldl = m->head.N_pad;
+    const int ldl = m->head.N_pad;
     for (int r0 = 0; r0 < R; r0 += m->head_chunk) {
         const int rows = std::min(m->head_chunk, R - r0);
-        if (m->prec >= 0) FC_TRY(lin_apply(m->packed_head, m->n + (size_t)r0 * d, nullptr, nullptr, m->logits, ldl, rows, m->st));
-        else FC_TRY(gemm(m, m->head, m->n + (size_t)r0 * d, nullptr, nullptr, m->logits, rows, ldl));
+        FC_TRY(head_rows(m, r0, rows));
         FC_TRY(launch_llama_score_rows(m->logits, ldl, m->cfg.vocab, m->targets_d + r0, rows, m->lp_d + r0, m->gr_d + r0, m->st));
     }
     return FC_OK;
@@ -460,14 +447,14 @@ int prime_window(fc_llama_cache* s, const int32_t* ids, int n) {
     fc_llama* m = s->m;
     const fc_llama_config& c = m->cfg;
     if (n > c.ctx) return fail(FC_E_DIM, "%d tokens do not fit the model's %d-token context window", n, c.ctx);
-    FC_TRY(ensure_workspace(m, n));
     cudaStream_t st = m->st;
-    FC_CUDA(cudaMemcpyAsync(m->ids_d, ids, (size_t)n * 4, cudaMemcpyHostToDevice, st));
-    FC_CUDA(cudaMemcpyAsync(s->queue, ids, (size_t)n * 4, cudaMemcpyHostToDevice, st));
     m->force_fp32 = true;
-    const int rc = forward_rows(m, 1, n, s);
+    int rc = ensure_workspace(m, n);
+    if (rc == FC_OK && cudaMemcpyAsync(m->ids_d, ids, (size_t)n * 4, cudaMemcpyHostToDevice, st) != cudaSuccess) rc = fail(FC_E_CUDA, "upload of the prompt failed");
+    if (rc == FC_OK) rc = forward_rows(m, 1, n, s);
     m->force_fp32 = false;
     FC_TRY(rc);
+    FC_CUDA(cudaMemcpyAsync(s->queue, ids, (size_t)n * 4, cudaMemcpyHostToDevice, st));
     llama_set_state_kernel<<<1, 1, 0, st>>>(s->state, n, n, n);
     FC_LAUNCHED();
     // logits of the last row: the final norm was applied by forward_rows
@@ -641,13 +628,12 @@ int fc_llama_forward_tokens(fc_llama* m, const int32_t* ids, int n, float* logit
     FC_CUDA(cudaSetDevice(m->device));
     FC_TRY(check_ids(m, ids, (size_t)n));
     FC_TRY(ensure_workspace(m, n));
-    const int d = m->cfg.d_model, V = m->cfg.vocab, ldl = m->head.N_pad;
+    const int V = m->cfg.vocab, ldl = m->head.N_pad;
     FC_CUDA(cudaMemcpyAsync(m->ids_d, ids, (size_t)n * 4, cudaMemcpyHostToDevice, m->st));
     FC_TRY(forward_rows(m, 1, n));
     for (int r0 = 0; r0 < n; r0 += m->head_chunk) {
         const int rows = std::min(m->head_chunk, n - r0);
-        if (m->prec >= 0) FC_TRY(lin_apply(m->packed_head, m->n + (size_t)r0 * d, nullptr, nullptr, m->logits, ldl, rows, m->st));
-        else FC_TRY(gemm(m, m->head, m->n + (size_t)r0 * d, nullptr, nullptr, m->logits, rows, ldl));
+        FC_TRY(head_rows(m, r0, rows));
         FC_CUDA(cudaMemcpy2DAsync(logits + (size_t)r0 * V, (size_t)V * 4, m->logits, (size_t)ldl * 4, (size_t)V * 4, rows,
                                   cudaMemcpyDeviceToHost, m->st));
     }

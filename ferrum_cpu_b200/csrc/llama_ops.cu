@@ -2,9 +2,9 @@
 // RMSNorm, rotary positions, the SwiGLU gate, the exact log-softmax scoring tail of
 // llm_score.rs and the greedy pick. All are HBM-bound elementwise / row-reduction work: one
 // block per row, coalesced accesses, fixed-order block reductions.
-#include <cuda_bf16.h>
 
 #include "llama_ops.cuh"
+#include "planes.cuh"
 #include "pdl.cuh"
 
 namespace fc {
@@ -100,25 +100,21 @@ __global__ void __launch_bounds__(256) llama_rmsnorm_kernel(const float* __restr
     const float inv = 1.0f / sqrtf(ms + eps);
     for (int c = threadIdx.x; c < d; c += blockDim.x) y[(size_t)blockIdx.x * d + c] = __fmul_rn(__fmul_rn(xr[c], inv), w[c]);
 }
-// The same with the result written as the bf16 hi / lo planes (y = hi + lo to 2^-17 relative)
-// that the tensor-core GEMM reads.
-__device__ __forceinline__ void store_planes(float y, __nv_bfloat16* hi, __nv_bfloat16* lo, size_t i) {
-    const __nv_bfloat16 h = __float2bfloat16_rn(y);
-    hi[i] = h;
-    lo[i] = __float2bfloat16_rn(y - __bfloat162float(h));
-}
+// The same with the result written as the P bf16 planes that the tensor-core GEMM reads.
+template <int P>
 __global__ void __launch_bounds__(256) llama_rmsnorm_planes_kernel(const float* __restrict__ x, const float* __restrict__ w, float eps,
-                                                                   int d, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
+                                                                   int d, const Planes out) {
     __shared__ float red[33];
     const float* xr = x + (size_t)blockIdx.x * d;
     float s = 0.0f;
     for (int c = threadIdx.x; c < d; c += blockDim.x) { const float v = xr[c]; s = fmaf(v, v, s); }
     const float ms = block_sum_t(s, red) / (float)d;
     const float inv = 1.0f / sqrtf(ms + eps);
-    for (int c = threadIdx.x; c < d; c += blockDim.x) store_planes(__fmul_rn(__fmul_rn(xr[c], inv), w[c]), hi, lo, (size_t)blockIdx.x * d + c);
+    for (int c = threadIdx.x; c < d; c += blockDim.x) store_planes<P>(out, (size_t)blockIdx.x * d + c, __fmul_rn(__fmul_rn(xr[c], inv), w[c]));
 }
-int launch_llama_rmsnorm_planes(const float* x, const float* w, float eps, int rows, int d, void* hi, void* lo, cudaStream_t st) {
-    llama_rmsnorm_planes_kernel<<<rows, 256, 0, st>>>(x, w, eps, d, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo);
+int launch_llama_rmsnorm_planes(const float* x, const float* w, float eps, int rows, int d, const Planes& out, cudaStream_t st) {
+    if (out.n == 3) llama_rmsnorm_planes_kernel<3><<<rows, 256, 0, st>>>(x, w, eps, d, out);
+    else llama_rmsnorm_planes_kernel<2><<<rows, 256, 0, st>>>(x, w, eps, d, out);
     FC_LAUNCHED();
     return FC_OK;
 }
@@ -162,8 +158,7 @@ __global__ void llama_rope_rows_kernel(float* __restrict__ qkv, int ld, int T, i
 // The same rotation with the row handed on as bf16 hi / lo planes (the input of the tensor-core
 // attention): the f32 row is staged in shared memory, rotated there and written once.
 __global__ void llama_rope_planes_kernel(const float* __restrict__ qkv, int ld, int T, int n_q, int n_kv, int k_off, int hd, int half,
-                                         int neox, const float2* __restrict__ ftab, float inv_linear,
-                                         __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
+                                         int neox, const float2* __restrict__ ftab, float inv_linear, const Planes out) {
     extern __shared__ float srow[];
     const int r = blockIdx.x, pos = r % T;
     const float* row = qkv + (size_t)r * ld;
@@ -177,14 +172,13 @@ __global__ void llama_rope_planes_kernel(const float* __restrict__ qkv, int ld, 
         rotate_pair(srow, ia, ib, rope_angle(pos, ftab[i], inv_linear));
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < ld; c += blockDim.x) store_planes(srow[c], hi, lo, (size_t)r * ld + c);
+    for (int c = threadIdx.x; c < ld; c += blockDim.x) store_planes<2>(out, (size_t)r * ld + c, srow[c]);
 }
 int launch_llama_rope_planes(const float* qkv, int R, int ld, int T, int n_q, int n_kv, int k_off, int hd, int rope_dim, int neox,
-                             const float2* ftab, float inv_linear, void* hi, void* lo, cudaStream_t st) {
+                             const float2* ftab, float inv_linear, const Planes& out, cudaStream_t st) {
     const size_t smem = (size_t)ld * sizeof(float);
     if (smem > 48 * 1024) return fail(FC_E_SHAPE, "fused q | k | v rows of %d floats exceed the rotation kernel's staging", ld);
-    llama_rope_planes_kernel<<<R, 256, smem, st>>>(qkv, ld, T, n_q, n_kv, k_off, hd, rope_dim / 2, neox, ftab, inv_linear,
-                                                   (__nv_bfloat16*)hi, (__nv_bfloat16*)lo);
+    llama_rope_planes_kernel<<<R, 256, smem, st>>>(qkv, ld, T, n_q, n_kv, k_off, hd, rope_dim / 2, neox, ftab, inv_linear, out);
     FC_LAUNCHED();
     return FC_OK;
 }

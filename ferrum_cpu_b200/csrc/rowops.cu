@@ -1,11 +1,10 @@
 // Row kernels of the forward path: embedding gather, LayerNorm, the decode tail
 // (softmax statistics + greedy select) and the scoring tail (per-target log-prob).
-#include <cuda_bf16.h>
 
 #include <algorithm>
 
-#include "fc_common.cuh"
 #include "pdl.cuh"
+#include "planes.cuh"
 
 namespace fc {
 
@@ -132,11 +131,10 @@ __global__ void layernorm_kernel(const float* __restrict__ x, const float* __res
     }
 }
 
-// The same LayerNorm with the result written as the bf16 hi / lo planes (y = hi + lo to 2^-17
-// relative) that the tensor-core GEMM reads.
-template <int PER>
+// The same LayerNorm with the result written as the P bf16 planes that the tensor-core GEMM reads.
+template <int PER, int P>
 __global__ void layernorm_planes_kernel(const float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ b,
-                                        int d, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
+                                        int d, const Planes out) {
     __shared__ float red[33];
     const float* xr = x + (size_t)blockIdx.x * d;
     float v[PER];
@@ -160,21 +158,15 @@ __global__ void layernorm_planes_kernel(const float* __restrict__ x, const float
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const int c = threadIdx.x + i * blockDim.x;
-        if (c < d) {
-            const float y = ((v[i] - mean) / sd) * g[c] + b[c];
-            const __nv_bfloat16 h = __float2bfloat16_rn(y);
-            hi[(size_t)blockIdx.x * d + c] = h;
-            lo[(size_t)blockIdx.x * d + c] = __float2bfloat16_rn(y - __bfloat162float(h));
-        }
+        if (c < d) store_planes<P>(out, (size_t)blockIdx.x * d + c, ((v[i] - mean) / sd) * g[c] + b[c]);
     }
 }
 
 // The same for rows of up to 1024 columns (a multiple of 128): a warp per row, the row in registers as 16-byte loads,
 // the two sums by shuffles (no block-wide synchronisation), the planes written 8 bytes per lane. Eight rows per CTA.
-template <int NV>
+template <int NV, int P>
 __global__ void __launch_bounds__(256) layernorm_planes_warp_kernel(const float* __restrict__ x, const float* __restrict__ g,
-                                                                    const float* __restrict__ b, int rows, int d,
-                                                                    __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
+                                                                    const float* __restrict__ b, int rows, int d, const Planes out) {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -202,41 +194,36 @@ __global__ void __launch_bounds__(256) layernorm_planes_warp_kernel(const float*
     const float sd = sqrtf(q / (float)d + 1e-5f);
     const float4* g4 = (const float4*)g;
     const float4* b4 = (const float4*)b;
-    uint2* h2 = (uint2*)(hi + (size_t)row * d);
-    uint2* l2 = (uint2*)(lo + (size_t)row * d);
 #pragma unroll
     for (int i = 0; i < NV; ++i)
         if (i < nv) {
             const float4 gg = __ldg(g4 + lane + 32 * i), bb = __ldg(b4 + lane + 32 * i);
-            const float y[4] = {((v[i].x - mean) / sd) * gg.x + bb.x, ((v[i].y - mean) / sd) * gg.y + bb.y,
-                                ((v[i].z - mean) / sd) * gg.z + bb.z, ((v[i].w - mean) / sd) * gg.w + bb.w};
-            __nv_bfloat16 hh[4], ll[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                hh[k] = __float2bfloat16_rn(y[k]);
-                ll[k] = __float2bfloat16_rn(y[k] - __bfloat162float(hh[k]));
-            }
-            h2[lane + 32 * i] = *(const uint2*)hh;
-            l2[lane + 32 * i] = *(const uint2*)ll;
+            store_planes4<P>(out, (size_t)row * (d >> 2) + lane + 32 * i,
+                             make_float4(((v[i].x - mean) / sd) * gg.x + bb.x, ((v[i].y - mean) / sd) * gg.y + bb.y,
+                                         ((v[i].z - mean) / sd) * gg.z + bb.z, ((v[i].w - mean) / sd) * gg.w + bb.w));
         }
 }
 
-int launch_layernorm_planes(const float* x, const float* g, const float* b, int rows, int d, void* hi, void* lo, cudaStream_t st) {
-    if (d % 128 == 0 && d <= 1024 && aligned16(x) && aligned16(g) && aligned16(b) && aligned16(hi) && aligned16(lo)) {
+template <int P>
+static int layernorm_planes(const float* x, const float* g, const float* b, int rows, int d, const Planes& out, cudaStream_t st) {
+    if (d % 128 == 0 && d <= 1024 && aligned16(x) && aligned16(g) && aligned16(b)) {
         const int blocks = (rows + 7) / 8;
-        if (d <= 512) layernorm_planes_warp_kernel<4><<<blocks, 256, 0, st>>>(x, g, b, rows, d, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo);
-        else layernorm_planes_warp_kernel<8><<<blocks, 256, 0, st>>>(x, g, b, rows, d, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo);
+        if (d <= 512) layernorm_planes_warp_kernel<4, P><<<blocks, 256, 0, st>>>(x, g, b, rows, d, out);
+        else layernorm_planes_warp_kernel<8, P><<<blocks, 256, 0, st>>>(x, g, b, rows, d, out);
         FC_LAUNCHED();
         return FC_OK;
     }
     const int threads = 256;
     const int per = (d + threads - 1) / threads;
-    if (per <= 4) layernorm_planes_kernel<4><<<rows, threads, 0, st>>>(x, g, b, d, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo);
-    else if (per <= 8) layernorm_planes_kernel<8><<<rows, threads, 0, st>>>(x, g, b, d, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo);
-    else if (per <= 16) layernorm_planes_kernel<16><<<rows, threads, 0, st>>>(x, g, b, d, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo);
+    if (per <= 4) layernorm_planes_kernel<4, P><<<rows, threads, 0, st>>>(x, g, b, d, out);
+    else if (per <= 8) layernorm_planes_kernel<8, P><<<rows, threads, 0, st>>>(x, g, b, d, out);
+    else if (per <= 16) layernorm_planes_kernel<16, P><<<rows, threads, 0, st>>>(x, g, b, d, out);
     else return fail(FC_E_SHAPE, "LayerNorm width %d exceeds 4096", d);
     FC_LAUNCHED();
     return FC_OK;
+}
+int launch_layernorm_planes(const float* x, const float* g, const float* b, int rows, int d, const Planes& out, cudaStream_t st) {
+    return out.n == 3 ? layernorm_planes<3>(x, g, b, rows, d, out, st) : layernorm_planes<2>(x, g, b, rows, d, out, st);
 }
 
 int launch_layernorm(const float* x, const float* g, const float* b, int rows, int d, float* y,
@@ -338,140 +325,6 @@ int launch_step_advance_pdl(StepState* state, cudaStream_t st) {
     return FC_OK;
 }
 
-// ------------------------------------------------------------------------------ scoring tail
-// scoring.rs:175-181: p = softmax(row)[target] in f32, clamp_prob (loss.rs:12-18), ln in
-// f64; greedy = argmax_first(row) == target, where the row is the probability row: the
-// first index whose exp(x - max) / sum equals the largest such value.
-__global__ void __launch_bounds__(256) score_rows_kernel(const float* __restrict__ logits, int ldl, int V,
-                                                         const int* __restrict__ targets, double* __restrict__ logprob,
-                                                         uint8_t* __restrict__ is_greedy) {
-    __shared__ float red[33];
-    __shared__ int ired[32];
-    const int r = blockIdx.x, target = targets[r];
-    if (target < 0 || target >= V) {
-        if (threadIdx.x == 0) { logprob[r] = 0.0; is_greedy[r] = 0; }
-        return;
-    }
-    const float* row = logits + (size_t)r * ldl;
-    float mx = -INFINITY;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) mx = fmaxf(mx, row[i]);
-    mx = block_max(mx, red);
-    float s = 0.0f;
-    int first = 0x7fffffff;          // first index whose probability ties the maximum's
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        const float e = expf(row[i] - mx);
-        s += e;
-        if (e == 1.0f && i < first) first = i;
-    }
-    const float sum = block_sum(s, red);
-    for (int o = 16; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-    if ((threadIdx.x & 31) == 0) ired[threadIdx.x >> 5] = first;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) first = min(first, ired[w]);
-        float p = expf(row[target] - mx) / sum;
-        if (p == p) p = fmaxf(p, 1e-12f);
-        logprob[r] = log((double)p);
-        is_greedy[r] = (uint8_t)(first == target);
-    }
-}
-
-// The same tail with the row staged in shared memory: one CTA per SM walks rows, fetches a
-// whole row of logits with one bulk async copy (a single pass over HBM, hundreds of KB in flight
-// per SM) and makes its three passes (max, sum of exponentials + first maximal index, target)
-// out of shared memory. Same arithmetic per row as score_rows_kernel with 1024 threads.
-// Bound: HBM, 4 * ldl bytes per scored row.
-constexpr int STAGED_THREADS = 1024;
-constexpr long long STAGED_WAIT_CYCLES = 4000000000LL;
-__global__ void __launch_bounds__(STAGED_THREADS, 1)
-score_rows_staged_kernel(const float* __restrict__ logits, int ldl, int V, const int* __restrict__ targets, int R,
-                         double* __restrict__ logprob, uint8_t* __restrict__ is_greedy, int* status) {
-    extern __shared__ __align__(16) float srow[];
-    __shared__ float red[33];
-    __shared__ int ired[32];
-    __shared__ unsigned long long bar;
-    const uint32_t bar_a = (uint32_t)__cvta_generic_to_shared(&bar);
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_a) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    const uint32_t bytes = (uint32_t)ldl * 4u;
-    uint32_t copies = 0;                                   // bulk copies issued so far (phase parity)
-    for (int r = blockIdx.x; r < R; r += gridDim.x) {
-        const int target = targets[r];
-        if (target < 0 || target >= V) {
-            if (threadIdx.x == 0) { logprob[r] = 0.0; is_greedy[r] = 0; }
-            continue;
-        }
-        bool failed = false;
-        if (threadIdx.x == 0) {
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_a), "r"(bytes) : "memory");
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"((uint32_t)__cvta_generic_to_shared(srow)), "l"(logits + (size_t)r * ldl), "r"(bytes), "r"(bar_a) : "memory");
-            const long long t0 = clock64();
-            for (;;) {
-                uint32_t ok;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-                    "selp.u32 %0, 1, 0, p;\n\t}"
-                    : "=r"(ok) : "r"(bar_a), "r"(copies & 1u), "r"(2000u) : "memory");
-                if (ok) break;
-                if (clock64() - t0 > STAGED_WAIT_CYCLES) { failed = true; break; }
-            }
-        }
-        ++copies;
-        if (__syncthreads_or(failed)) {                      // the row never arrived: report and stop
-            if (threadIdx.x == 0) atomicExch(status, FC_E_TIMEOUT);
-            break;
-        }
-        float mx = -INFINITY;
-        for (int i = threadIdx.x; i < V; i += STAGED_THREADS) mx = fmaxf(mx, srow[i]);
-        mx = block_max(mx, red);
-        float s = 0.0f;
-        int first = 0x7fffffff;          // first index whose probability ties the maximum's
-        for (int i = threadIdx.x; i < V; i += STAGED_THREADS) {
-            const float e = expf(srow[i] - mx);
-            s += e;
-            if (e == 1.0f && i < first) first = i;
-        }
-        const float sum = block_sum(s, red);
-        for (int o = 16; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-        if ((threadIdx.x & 31) == 0) ired[threadIdx.x >> 5] = first;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < STAGED_THREADS / 32; ++w) first = min(first, ired[w]);
-            float p = expf(srow[target] - mx) / sum;
-            if (p == p) p = fmaxf(p, 1e-12f);
-            logprob[r] = log((double)p);
-            is_greedy[r] = (uint8_t)(first == target);
-        }
-        __syncthreads();                                     // the row buffer is free for the next copy
-    }
-}
-
-int launch_score_rows(const float* logits, int ldl, int V, const int* targets, int R, double* logprob,
-                      uint8_t* is_greedy, int* status, cudaStream_t st) {
-    static int sms[64] = {};
-    const size_t smem = (size_t)ldl * 4;
-    int dev = 0;
-    FC_CUDA(cudaGetDevice(&dev));
-    // rows staged in shared memory when a row fits and the copy is legal (16-byte multiples)
-    if (status && dev < 64 && smem <= 200 * 1024 && (ldl & 3) == 0 && (((uintptr_t)logits) & 15) == 0 && R > 0) {
-        if (!sms[dev]) {
-            FC_CUDA(cudaFuncSetAttribute(score_rows_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            FC_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
-        }
-        score_rows_staged_kernel<<<R < sms[dev] ? R : sms[dev], STAGED_THREADS, smem, st>>>(logits, ldl, V, targets, R, logprob, is_greedy, status);
-        FC_LAUNCHED();
-        return FC_OK;
-    }
-    score_rows_kernel<<<R, 256, 0, st>>>(logits, ldl, V, targets, logprob, is_greedy);
-    FC_LAUNCHED();
-    return FC_OK;
-}
-
 __global__ void __launch_bounds__(1024) softmax_row_kernel(const float* __restrict__ logits, int V, float* __restrict__ probs) {
     __shared__ float red[33];
     float mx = -INFINITY;
@@ -491,15 +344,17 @@ int launch_softmax_row(const float* logits, int V, float* probs, cudaStream_t st
 // ------------------------------------------------------------------------------ layer statistics
 // verbose::stats + verbose::check_nan_inf (verbose.rs:85-110) of one layer output: min, max, f64 sum, and the
 // counts of NaN and Inf. Two stages with a fixed order (per-block partials, then one block), so the figures are
-// the same from run to run. planes_lo != null: the tensor is held as bf16 hi / lo planes, value = hi + lo.
+// the same from run to run. x == null: the tensor is held as bf16 planes, value = their sum.
 struct StatPart { float mn, mx; double sum; unsigned long long nan, inf; };
 
-__global__ void __launch_bounds__(256) layer_stats_partial_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ hi,
-                                                                  const __nv_bfloat16* __restrict__ lo, size_t n, StatPart* part) {
+__global__ void __launch_bounds__(256) layer_stats_partial_kernel(const float* __restrict__ x, const Planes pl, size_t n, StatPart* part) {
     __shared__ StatPart sh[256];
     StatPart p{INFINITY, -INFINITY, 0.0, 0ull, 0ull};
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float v = x ? x[i] : __bfloat162float(hi[i]) + __bfloat162float(lo[i]);
+        float v = 0.0f;
+        if (x) v = x[i];
+        else
+            for (int p = pl.n - 1; p >= 0; --p) v += __bfloat162float(((const __nv_bfloat16*)pl.p[p])[i]);
         if (v != v) { p.nan += 1; continue; }      // as the reference's comparisons, NaN never becomes min or max
         if (isinf(v)) p.inf += 1;
         p.mn = fminf(p.mn, v);
@@ -532,9 +387,9 @@ __global__ void layer_stats_final_kernel(const StatPart* part, int n_part, size_
 
 size_t layer_stats_scratch_bytes() { return 148 * sizeof(StatPart); }
 
-int launch_layer_stats(const float* x, const void* hi, const void* lo, size_t n, void* scratch, LayerStatsDev* out, cudaStream_t st) {
+int launch_layer_stats(const float* x, const Planes& planes, size_t n, void* scratch, LayerStatsDev* out, cudaStream_t st) {
     const int blocks = (int)std::min<size_t>(148, std::max<size_t>(1, (n + 255) / 256));
-    layer_stats_partial_kernel<<<blocks, 256, 0, st>>>(x, (const __nv_bfloat16*)hi, (const __nv_bfloat16*)lo, n, (StatPart*)scratch);
+    layer_stats_partial_kernel<<<blocks, 256, 0, st>>>(x, planes, n, (StatPart*)scratch);
     FC_LAUNCHED();
     layer_stats_final_kernel<<<1, 1, 0, st>>>((const StatPart*)scratch, blocks, n, out);
     FC_LAUNCHED();
