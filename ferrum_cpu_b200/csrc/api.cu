@@ -143,6 +143,53 @@ struct BatchCtx {
     cudaEvent_t fork = nullptr;
 };
 
+// One batch of scoring windows on its way: what the host sends and gets back, in pinned memory and on the device. Two of
+// them, so that the host prepares and harvests one batch while the GPU works on the other.
+struct ScoreSlot {
+    char *in_h = nullptr, *in_d = nullptr, *out_h = nullptr, *out_d = nullptr;
+    size_t in_cap = 0, out_cap = 0;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, done = nullptr;
+    int picked = 0;                  // scored rows
+    // in: ids [R] | positions [R] | window starts [B + 1] | scored rows [picked] | their targets [picked]
+    // out: status word (8 bytes) | f64 log-probs [picked] | greedy flags [picked]
+    int* status_d() const { return (int*)out_d; }
+    double* lp_d() const { return (double*)(out_d + 8); }
+    uint8_t* gr_d() const { return (uint8_t*)(out_d + 8 + 8 * (size_t)picked); }
+    const double* lp_h() const { return (const double*)(out_h + 8); }
+    const uint8_t* gr_h() const { return (const uint8_t*)(out_h + 8 + 8 * (size_t)picked); }
+    size_t out_bytes() const { return 8 + 9 * (size_t)picked; }
+    int reserve(size_t in_bytes, size_t out_bytes) {
+        if (!done) {
+            FC_CUDA(cudaEventCreate(&ev0));
+            FC_CUDA(cudaEventCreate(&ev1));
+            FC_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+        }
+        auto grow = [](char** h, char** d, size_t* cap, size_t want) -> int {
+            if (want <= *cap) return FC_OK;
+            if (*h) cudaFreeHost(*h);
+            if (*d) cudaFree(*d);
+            *h = *d = nullptr;
+            *cap = 0;
+            FC_CUDA(cudaMallocHost((void**)h, want));
+            FC_CUDA(cudaMalloc((void**)d, want));
+            *cap = want;
+            return FC_OK;
+        };
+        FC_TRY(grow(&in_h, &in_d, &in_cap, in_bytes));
+        return grow(&out_h, &out_d, &out_cap, out_bytes);
+    }
+    void release() {
+        if (in_h) cudaFreeHost(in_h);
+        if (out_h) cudaFreeHost(out_h);
+        if (in_d) cudaFree(in_d);
+        if (out_d) cudaFree(out_d);
+        if (ev0) cudaEventDestroy(ev0);
+        if (ev1) cudaEventDestroy(ev1);
+        if (done) cudaEventDestroy(done);
+        *this = ScoreSlot();
+    }
+};
+
 struct fc_model {
     fc_config cfg;
     int device;
@@ -156,9 +203,8 @@ struct fc_model {
     // prefill workspace for ws_rows rows
     int ws_rows = 0, ws_planes = 0;
     float *x = nullptr, *n = nullptr, *qkv = nullptr, *att = nullptr, *logits = nullptr, *probs_d = nullptr;
-    int *ids_d = nullptr, *targets_d = nullptr, *err_d = nullptr;
-    double* lp_d = nullptr;
-    uint8_t* gr_d = nullptr;
+    int *ids_d = nullptr, *err_d = nullptr;
+    ScoreSlot slot[2];
     Planes pn, pqkv, patt, phid;               // bf16 planes of LayerNorm output, qkv, attention output, GELU output
     void* head_stats = nullptr;                // fused head: per (row, 128-column tile) softmax records, 16 B each
     float* head_tlogit = nullptr;              // ... and the logit of each row's target
@@ -347,8 +393,8 @@ static int model_planes(const fc_model* m) {
     const fc_config& c = m->cfg;
     return c.math_mode == FC_MATH_BF16X3 && c.d_model % 64 == 0 && c.d_ff % 64 == 0 ? 2 : 3;
 }
-// Whether the attention of a forward with `planes` planes runs on the tensor cores (heads of 64, two planes).
-static bool tensor_attention(const fc_model* m, int planes) { return planes == 2 && m->cfg.d_model == m->cfg.n_head * 64; }
+// Whether the window attention runs on the tensor cores (heads of 64).
+static bool tensor_attention(const fc_model* m) { return m->cfg.d_model == m->cfg.n_head * 64; }
 
 static int ensure_workspace(fc_model* m, int rows, int planes) {
     if (rows <= m->ws_rows && planes <= m->ws_planes) return FC_OK;
@@ -366,9 +412,6 @@ static int ensure_workspace(fc_model* m, int rows, int planes) {
     FC_TRY(a.alloc_n(&m->qkv, R * 3 * d));
     FC_TRY(a.alloc_n(&m->att, R * d));
     FC_TRY(a.alloc_n(&m->ids_d, R));
-    FC_TRY(a.alloc_n(&m->targets_d, R));
-    FC_TRY(a.alloc_n(&m->lp_d, R));
-    FC_TRY(a.alloc_n(&m->gr_d, R));
     FC_TRY(a.alloc_n(&m->err_d, 1));
     FC_TRY(a.alloc_n(&m->probs_d, (size_t)c.vocab));
     auto make = [&](Planes* p, size_t n) -> int {
@@ -388,18 +431,20 @@ static int ensure_workspace(fc_model* m, int rows, int planes) {
     return FC_OK;
 }
 
-// Sequential::forward (model.rs:51-71) through every block, on B windows of T rows whose ids are already in m->ids_d.
+// Sequential::forward (model.rs:51-71) through every block, on the R rows of `win` (device arrays: their ids, and their
+// positions in the window, null: r % T).
 // Leaves the residual stream in m->x. Between kernels activations are bf16 planes; only the residual stream is f32.
 // split_k: see launch_gemm_q8_tc. f32_qkv: the QKV product is written as f32 rows to m->qkv and on_qkv(layer) is called before the attention.
 template <class OnQkv>
-static int forward_blocks_with(fc_model* m, int B, int T, int planes, int* status, bool split_k, bool f32_qkv, OnQkv on_qkv) {
+static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int* ids, const int* pos, int planes, int* status,
+                               bool split_k, bool f32_qkv, OnQkv on_qkv) {
     const fc_config& c = m->cfg;
-    const int R = B * T, d = c.d_model, F = c.d_ff;
+    const int d = c.d_model, F = c.d_ff;
     cudaStream_t st = m->st;
-    const bool tc_attn = tensor_attention(m, planes);
+    const bool tc_attn = tensor_attention(m);
     m->pn.n = m->pqkv.n = m->patt.n = m->phid.n = planes;
     FC_CUDA(cudaMemsetAsync(m->err_d, 0, sizeof(int), st));
-    FC_TRY(launch_embed_rows(m->tok, m->pos, m->ids_d, R, T, m->x, m->err_d, st));
+    FC_TRY(launch_embed_rows(m->tok, m->pos, ids, pos, R, win.T, m->x, m->err_d, st));
     // model.rs:58-68: with the statistics switched on, every layer's output is summarised as it appears
     m->stats_n = 0;
     auto layer_stats = [&]() -> int {
@@ -409,7 +454,7 @@ static int forward_blocks_with(fc_model* m, int B, int T, int planes, int* statu
     FC_TRY(layer_stats());
     for (int l = 0; l < c.n_layer; ++l) {
         const LayerDev& L = m->layers[l];
-        FC_TRY(launch_layernorm_planes(m->x, L.ln1g, L.ln1b, R, d, m->pn, st));
+        FC_TRY(launch_layernorm_planes(m->x, L.ln1g, L.ln1b, nullptr, R, d, m->pn, st));
         if (tc_attn && !f32_qkv) {
             FC_TRY(launch_gemm_q8_tc(L.qkv, m->pn, L.qkv_b, nullptr, EPI_NONE, nullptr, &m->pqkv, R, 3 * d, status, st, split_k));
         } else {
@@ -418,34 +463,34 @@ static int forward_blocks_with(fc_model* m, int B, int T, int planes, int* statu
             if (tc_attn) FC_TRY(launch_split_planes(m->qkv, m->pqkv, (size_t)R * 3 * d, st));
         }
         if (tc_attn) {
-            FC_TRY(launch_attn_prefill_tc(m->pqkv, B, T, d, c.n_head, m->patt, status, st));
+            FC_TRY(launch_attn_prefill_tc(m->pqkv, win, R, d, c.n_head, m->patt, status, st));
         } else {
-            FC_TRY(launch_attn_prefill(m->qkv, B, T, d, c.n_head, m->att, st));
+            FC_TRY(launch_attn_prefill(m->qkv, win, d, c.n_head, m->att, st));
             FC_TRY(launch_split_planes(m->att, m->patt, (size_t)R * d, st));
         }
         FC_TRY(launch_gemm_q8_tc(L.out, m->patt, L.out_b, m->x, EPI_NONE, m->x, nullptr, R, d, status, st, split_k));
-        FC_TRY(launch_layernorm_planes(m->x, L.ln2g, L.ln2b, R, d, m->pn, st));
+        FC_TRY(launch_layernorm_planes(m->x, L.ln2g, L.ln2b, nullptr, R, d, m->pn, st));
         FC_TRY(launch_gemm_q8_tc(L.up, m->pn, L.up_b, nullptr, EPI_GELU, nullptr, &m->phid, R, F, status, st, split_k));
         FC_TRY(launch_gemm_q8_tc(L.down, m->phid, L.down_b, m->x, EPI_NONE, m->x, nullptr, R, d, status, st, split_k));
         FC_TRY(layer_stats());
     }
     return FC_OK;
 }
-static int forward_blocks(fc_model* m, int B, int T) {
-    return forward_blocks_with(m, B, T, model_planes(m), m->tc_status, false, false, [](int) { return FC_OK; });
-}
-
-// Forward + final LayerNorm + head + scoring tail for ids/targets already on the device. lp_d/gr_d filled.
-static int score_device(fc_model* m, int B, int T) {
+// The forward of a scoring batch: blocks, final LayerNorm, head and scoring tail for the scored rows.
+static int score_device(fc_model* m, const ScoreSlot& s, const Windows& win, int R) {
     const fc_config& c = m->cfg;
-    const int R = B * T, d = c.d_model;
-    FC_TRY(forward_blocks(m, B, T));
+    const int d = c.d_model, n = s.picked;
+    const int *ids = (const int*)s.in_d, *pos = ids + R, *pick = pos + R + win.B + 1, *targets = pick + n;
+    FC_TRY(forward_blocks_with(m, win, R, ids, pos, model_planes(m), s.status_d(), false, false, [](int) { return FC_OK; }));
+    if (m->stats_on) {
+        FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, nullptr, R, d, m->pn, m->st));
+        FC_TRY(launch_layer_stats(nullptr, m->pn, (size_t)R * d, m->stats_scratch, m->stats_d + m->stats_n++, m->st));
+    }
     // the head's epilogue keeps (max, sum of exponentials, first argmax) per row and 128-column tile and the
     // target's logit: [rows][V] logits never reach memory (scoring.rs:175-181 needs one number per row)
-    FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, R, d, m->pn, m->st));
-    if (m->stats_on) FC_TRY(launch_layer_stats(nullptr, m->pn, (size_t)R * d, m->stats_scratch, m->stats_d + m->stats_n++, m->st));
-    FC_TRY(launch_gemm_q8_tc_score(m->head, m->pn, m->targets_d, m->head_stats, m->head_tlogit, R, m->tc_status, m->st));
-    return launch_score_combine(m->head_stats, m->head_tlogit, m->targets_d, R, (c.vocab + 127) / 128, c.vocab, m->lp_d, m->gr_d, m->st);
+    FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, n == R ? nullptr : pick, n, d, m->pn, m->st));
+    FC_TRY(launch_gemm_q8_tc_score(m->head, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
+    return launch_score_combine(m->head_stats, m->head_tlogit, targets, n, (c.vocab + 127) / 128, c.vocab, s.lp_d(), s.gr_d(), m->st);
 }
 
 }  // namespace fc
@@ -708,6 +753,7 @@ void fc_model_free(fc_model* m) {
     m->pool.clear();
     m->arena.release();
     m->ws_arena.release();
+    for (ScoreSlot& s : m->slot) s.release();
     if (m->batch.graph) cudaGraphExecDestroy(m->batch.graph);
     if (m->batch.graph4) cudaGraphExecDestroy(m->batch.graph4);
     for (cudaStream_t t : m->batch.side) cudaStreamDestroy(t);
@@ -768,33 +814,58 @@ static int check_tc_status(fc_model* m, const char* what) {
     cudaMemsetAsync(m->tc_status, 0, sizeof(int), m->st);
     return fail(FC_E_TIMEOUT, "a bounded wait inside a tensor-core kernel of %s ran out (status %d)", what, status);
 }
-static int score_windows_impl(fc_model* m, const int32_t* ids, const int32_t* targets, int B, int T,
-                              double* lp_host, uint8_t* gr_host) {
-    const fc_config& c = m->cfg;
-    if (B <= 0 || T <= 0) return fail(FC_E_SHAPE, "scoring needs B > 0 and T > 0 (got %d, %d)", B, T);
-    if (T > c.ctx) return fail(FC_E_DIM, "Sequence length %d exceeds max_seq_len %d", T, c.ctx);
-    if ((int64_t)B * T > (int64_t)1 << 24) return fail(FC_E_SHAPE, "too many rows in one forward: %lld", (long long)B * T);
-    const int R = B * T;
-    FC_TRY(check_ids(m, ids, (size_t)R));
-    FC_CUDA(cudaSetDevice(m->device));
-    FC_TRY(ensure_workspace(m, R, model_planes(m)));
-    cudaStream_t st = m->st;
-    FC_CUDA(cudaMemcpyAsync(m->ids_d, ids, (size_t)R * 4, cudaMemcpyHostToDevice, st));
-    FC_CUDA(cudaMemcpyAsync(m->targets_d, targets, (size_t)R * 4, cudaMemcpyHostToDevice, st));
-    FC_CUDA(cudaEventRecord(m->ev0, st));
-    FC_TRY(score_device(m, B, T));
-    FC_CUDA(cudaEventRecord(m->ev1, st));
-    FC_CUDA(cudaMemcpyAsync(lp_host, m->lp_d, (size_t)R * 8, cudaMemcpyDeviceToHost, st));
-    FC_CUDA(cudaMemcpyAsync(gr_host, m->gr_d, (size_t)R, cudaMemcpyDeviceToHost, st));
-    int tc_status = 0;
-    if (m->tc_status) FC_CUDA(cudaMemcpyAsync(&tc_status, m->tc_status, sizeof(int), cudaMemcpyDeviceToHost, st));
-    FC_CUDA(cudaStreamSynchronize(st));
-    if (tc_status != 0) {
-        cudaMemsetAsync(m->tc_status, 0, sizeof(int), st);
-        return fail(FC_E_TIMEOUT, "a bounded wait inside a scoring kernel ran out (status %d)", tc_status);
+// A batch of windows as the host builds it: the rows of all windows one after the other, without padding.
+struct ScoreBatch {
+    std::vector<int32_t> ids, pos, starts, pick, targets;
+    int longest = 0;
+    void clear() { ids.clear(); pos.clear(); starts.assign(1, 0); pick.clear(); targets.clear(); longest = 0; }
+    // n rows; returns the first row
+    int window(const int32_t* src, int n) {
+        const int at = (int)ids.size();
+        ids.insert(ids.end(), src, src + n);
+        for (int t = 0; t < n; ++t) pos.push_back(t);
+        starts.push_back(at + n);
+        longest = std::max(longest, n);
+        return at;
     }
+    void score(int row, int32_t target) { pick.push_back(row); targets.push_back(target); }
+};
+
+static int score_issue(fc_model* m, ScoreSlot& s, const ScoreBatch& b) {
+    const fc_config& c = m->cfg;
+    const size_t R = b.ids.size(), n = b.pick.size(), B = b.starts.size() - 1;
+    if (b.longest > c.ctx) return fail(FC_E_DIM, "Sequence length %d exceeds max_seq_len %d", b.longest, c.ctx);
+    if (R > (size_t)1 << 24) return fail(FC_E_SHAPE, "too many rows in one forward: %zu", R);
+    FC_TRY(check_ids(m, b.ids.data(), R));
+    FC_CUDA(cudaSetDevice(m->device));
+    FC_TRY(ensure_workspace(m, (int)R, model_planes(m)));
+    const size_t in_bytes = 4 * (2 * R + B + 1 + 2 * n);
+    s.picked = (int)n;
+    FC_TRY(s.reserve(in_bytes, s.out_bytes()));
+    char* at = s.in_h;
+    for (const std::vector<int32_t>* v : {&b.ids, &b.pos, &b.starts, &b.pick, &b.targets}) {
+        std::memcpy(at, v->data(), v->size() * 4);
+        at += v->size() * 4;
+    }
+    cudaStream_t st = m->st;
+    FC_CUDA(cudaMemcpyAsync(s.in_d, s.in_h, in_bytes, cudaMemcpyHostToDevice, st));
+    FC_CUDA(cudaMemsetAsync(s.out_d, 0, 8, st));
+    Windows win;
+    win.B = (int)B; win.T = b.longest; win.starts = (const int*)s.in_d + 2 * R;
+    FC_CUDA(cudaEventRecord(s.ev0, st));
+    if (n > 0) FC_TRY(score_device(m, s, win, (int)R));
+    FC_CUDA(cudaEventRecord(s.ev1, st));
+    FC_CUDA(cudaMemcpyAsync(s.out_h, s.out_d, s.out_bytes(), cudaMemcpyDeviceToHost, st));
+    FC_CUDA(cudaEventRecord(s.done, st));
+    return FC_OK;
+}
+
+static int score_harvest(fc_model* m, ScoreSlot& s) {
+    FC_CUDA(cudaEventSynchronize(s.done));
+    const int status = *(const int*)s.out_h;
+    if (status != 0) return fail(FC_E_TIMEOUT, "a bounded wait inside a scoring kernel ran out (status %d)", status);
     float ms = 0.0f;
-    FC_CUDA(cudaEventElapsedTime(&ms, m->ev0, m->ev1));
+    FC_CUDA(cudaEventElapsedTime(&ms, s.ev0, s.ev1));
     m->last_score_ms += ms;
     return FC_OK;
 }
@@ -802,10 +873,21 @@ static int score_windows_impl(fc_model* m, const int32_t* ids, const int32_t* ta
 int fc_score_windows(fc_model* m, const int32_t* ids, const int32_t* targets, int B, int T,
                      float* logprob, uint8_t* is_greedy) {
     if (!m || !ids || !targets || !logprob || !is_greedy) return fail(FC_E_ARG, "fc_score_windows: null argument");
+    if (B <= 0 || T <= 0) return fail(FC_E_SHAPE, "scoring needs B > 0 and T > 0 (got %d, %d)", B, T);
+    if (T > m->cfg.ctx) return fail(FC_E_DIM, "Sequence length %d exceeds max_seq_len %d", T, m->cfg.ctx);
+    if ((int64_t)B * T > (int64_t)1 << 24) return fail(FC_E_SHAPE, "too many rows in one forward: %lld", (long long)B * T);
     m->last_score_ms = 0.0f;
-    std::vector<double> lp((size_t)std::max(0, B) * std::max(0, T));
-    FC_TRY(score_windows_impl(m, ids, targets, B, T, lp.data(), is_greedy));
-    for (size_t i = 0; i < lp.size(); ++i) logprob[i] = (float)lp[i];
+    ScoreBatch b;
+    b.clear();
+    for (int i = 0; i < B; ++i) b.window(ids + (size_t)i * T, T);
+    for (int r = 0; r < B * T; ++r)
+        if (targets[r] >= 0 && targets[r] < m->cfg.vocab) b.score(r, targets[r]);
+    ScoreSlot& s = m->slot[0];
+    FC_TRY(score_issue(m, s, b));
+    FC_TRY(score_harvest(m, s));
+    std::fill(logprob, logprob + (size_t)B * T, 0.0f);
+    std::fill(is_greedy, is_greedy + (size_t)B * T, (uint8_t)0);
+    for (int i = 0; i < s.picked; ++i) { logprob[b.pick[i]] = (float)s.lp_h()[i]; is_greedy[b.pick[i]] = s.gr_h()[i]; }
     return FC_OK;
 }
 
@@ -827,40 +909,39 @@ void plan_windows(int seq, int n, int from, int T, std::vector<Window>* out) {
     }
 }
 
-// Scores every window of `plan` in batches; seq_ids(s) gives the ids of sequence s, seq_len(s)
-// its length. For each scored target calls add(seq, target, logprob, greedy).
+// Scores every window of `plan` in batches; seq_ids(s) gives the ids of sequence s, seq_len(s) its length. For each scored
+// target calls add(seq, target, logprob, greedy), in the order of the plan. The windows of a batch lie one after the other
+// without the reference's padding (scoring.rs:184-193 pads with id 0; under the causal mask no scored row sees a pad), and only
+// the rows that predict a target meet the head. A batch is harvested when the next one has been queued.
 template <class Ids, class Len, class Add>
 int run_plan_ragged(fc_model* m, const std::vector<Window>& plan, int batch, Ids seq_ids, Len seq_len, Add add) {
     const int T = m->cfg.ctx;
-    std::vector<int32_t> ids, targets;
-    std::vector<double> lp;
-    std::vector<uint8_t> gr;
-    for (size_t w0 = 0; w0 < plan.size(); w0 += batch) {
-        const int B = (int)std::min<size_t>(batch, plan.size() - w0);
-        // rows past the longest window of the batch are never read under the causal mask
-        int Tb = 1;
-        for (int b = 0; b < B; ++b) Tb = std::max(Tb, std::min(plan[w0 + b].start + T, seq_len(plan[w0 + b].seq)) - plan[w0 + b].start);
-        ids.assign((size_t)B * Tb, 0);          // right padding with id 0 (scoring.rs:188-190)
-        targets.assign((size_t)B * Tb, -1);
-        for (int b = 0; b < B; ++b) {
-            const Window& w = plan[w0 + b];
+    ScoreBatch b;
+    auto harvest = [&](size_t w0, ScoreSlot& s) -> int {
+        FC_TRY(score_harvest(m, s));
+        const double* lp = s.lp_h();
+        const uint8_t* gr = s.gr_h();
+        for (size_t w = w0; w < std::min(w0 + batch, plan.size()); ++w)
+            for (int t = plan[w].first; t < plan[w].end; ++t) add(plan[w].seq, t, *lp++, *gr++);
+        return FC_OK;
+    };
+    int rc = FC_OK;
+    size_t w0 = 0, waiting = plan.size();            // first window of the batch that is under way
+    for (int k = 0; w0 < plan.size() && rc == FC_OK; w0 += batch, k ^= 1) {
+        b.clear();
+        for (size_t i = w0; i < std::min(w0 + batch, plan.size()); ++i) {
+            const Window& w = plan[i];
             const int32_t* src = seq_ids(w.seq);
-            const int wl = std::min(w.start + T, seq_len(w.seq)) - w.start;
-            std::copy(src + w.start, src + w.start + wl, ids.begin() + (size_t)b * Tb);
-            for (int t = w.first; t < w.end; ++t) targets[(size_t)b * Tb + (t - 1 - w.start)] = src[t];
+            const int at = b.window(src + w.start, std::min(w.start + T, seq_len(w.seq)) - w.start);
+            for (int t = w.first; t < w.end; ++t) b.score(at + t - 1 - w.start, src[t]);
         }
-        lp.resize((size_t)B * Tb);
-        gr.resize((size_t)B * Tb);
-        FC_TRY(score_windows_impl(m, ids.data(), targets.data(), B, Tb, lp.data(), gr.data()));
-        for (int b = 0; b < B; ++b) {
-            const Window& w = plan[w0 + b];
-            for (int t = w.first; t < w.end; ++t) {
-                const size_t r = (size_t)b * Tb + (t - 1 - w.start);
-                add(w.seq, t, lp[r], gr[r]);
-            }
-        }
+        rc = score_issue(m, m->slot[k], b);
+        if (rc == FC_OK && waiting < plan.size()) rc = harvest(waiting, m->slot[k ^ 1]);
+        waiting = w0;
+        if (rc == FC_OK && w0 + batch >= plan.size()) rc = harvest(w0, m->slot[k]);
     }
-    return FC_OK;
+    if (rc != FC_OK) cudaStreamSynchronize(m->st);   // nothing of this call stays under way
+    return rc;
 }
 template <class Ids, class Add>
 int run_plan(fc_model* m, const std::vector<Window>& plan, int batch, Ids seq_ids, int n, Add add) {
@@ -938,7 +1019,9 @@ int fc_predict_next(fc_model* m, const int32_t* ids, int n, float* probs) {
     FC_TRY(ensure_workspace(m, n, model_planes(m)));
     cudaStream_t st = m->st;
     FC_CUDA(cudaMemcpyAsync(m->ids_d, ids, (size_t)n * 4, cudaMemcpyHostToDevice, st));
-    FC_TRY(forward_blocks(m, 1, n));
+    Windows win;
+    win.B = 1; win.T = n;
+    FC_TRY(forward_blocks_with(m, win, n, m->ids_d, nullptr, model_planes(m), m->tc_status, false, false, [](int) { return FC_OK; }));
     FC_TRY(launch_layernorm(m->x + (size_t)(n - 1) * c.d_model, m->lnfg, m->lnfb, 1, c.d_model,
                             m->n, nullptr, st));
     GemvOut o; o.out[0] = m->logits;
@@ -1071,7 +1154,7 @@ static int prime_batched(fc_stream* const* ss, int S, int n, int last_mode, int*
         if (ss[i]->host_pos != 0) return FC_OK;
     cudaStream_t st = m->st;
     // prompts keep f32 rounding (3 planes) unless the model's scoring mode is the 2-plane one and there are many rows
-    const int planes = R >= 256 && tensor_attention(m, model_planes(m)) ? 2 : 3;
+    const int planes = R >= 256 && tensor_attention(m) && model_planes(m) == 2 ? 2 : 3;
     FC_TRY(ensure_workspace(m, R, planes));
     for (int i = 0; i < S; ++i)
         FC_CUDA(cudaMemcpyAsync(m->ids_d + (size_t)i * n, ss[i]->queue, (size_t)n * sizeof(int), cudaMemcpyDeviceToDevice, st));
@@ -1088,7 +1171,9 @@ static int prime_batched(fc_stream* const* ss, int S, int n, int last_mode, int*
         }
         return FC_OK;
     };
-    FC_TRY(forward_blocks_with(m, S, n, planes, S == 1 && ss[0]->status ? ss[0]->status : m->tc_status, true, true, to_caches));
+    Windows win;
+    win.B = S; win.T = n;
+    FC_TRY(forward_blocks_with(m, win, R, m->ids_d, nullptr, planes, S == 1 && ss[0]->status ? ss[0]->status : m->tc_status, true, true, to_caches));
     *used = 1;
     for (int i = 0; i < S; ++i) {
         fc_stream* s = ss[i];

@@ -109,7 +109,7 @@ constexpr int KT = 64;   // keys per tile
 // h reads key/value head h / group; output rows are ldo floats apart.
 template <int HD>
 __global__ void __launch_bounds__(256) attn_prefill_kernel(const float* __restrict__ q, const float* __restrict__ k,
-                                                           const float* __restrict__ v, int T, int ld, int group, int ldo,
+                                                           const float* __restrict__ v, const Windows win, int ld, int group, int ldo,
                                                            float* __restrict__ out) {
     constexpr int LDS = HD + 4;                 // row stride in floats: 16-byte aligned, bank-shifted by 4
     extern __shared__ float4 sm4[];
@@ -119,10 +119,13 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const float* __restri
     const int h = blockIdx.y, b = blockIdx.z;
     const int qi = threadIdx.x >> 2, part = threadIdx.x & 3;
     const int i = qt * QT + qi;                 // query row within the window
+    const int T = win.length(b);
+    const size_t first = (size_t)win.begin(b);
+    if (qt * QT >= T) return;
     const size_t row3 = (size_t)ld;
-    const float* base = q + (size_t)b * T * row3 + (size_t)h * HD;
-    const float* kbase = k + (size_t)b * T * row3 + (size_t)(h / group) * HD;
-    const float* vbase = v + (size_t)b * T * row3 + (size_t)(h / group) * HD;
+    const float* base = q + first * row3 + (size_t)h * HD;
+    const float* kbase = k + first * row3 + (size_t)(h / group) * HD;
+    const float* vbase = v + first * row3 + (size_t)(h / group) * HD;
     const float scale = 1.0f / sqrtf((float)HD);
 
     float qreg[HD];
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const float* __restri
         o[c] = v;
     }
     if (i < T) {
-        float* op = out + ((size_t)b * T + i) * ldo + (size_t)h * HD;
+        float* op = out + (first + i) * ldo + (size_t)h * HD;
         // lane `part` stores its quarter of the head dimension
 #pragma unroll
         for (int c = 0; c < HD / 4; ++c)
@@ -220,15 +223,17 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const float* __restri
 // dimension, keys read straight from global memory. Slower than the tiled kernel; used for the
 // head widths that kernel is not instantiated for.
 __global__ void __launch_bounds__(256) attn_prefill_any_kernel(const float* __restrict__ q, const float* __restrict__ k,
-                                                               const float* __restrict__ v, int T, int ld, int group, int hd,
+                                                               const float* __restrict__ v, const Windows win, int ld, int group, int hd,
                                                                int ldo, float* __restrict__ out) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int i = (gridDim.x - 1 - blockIdx.x) * 8 + wid;      // late (long) rows first
     const int h = blockIdx.y, b = blockIdx.z;
+    const int T = win.length(b);
+    const size_t first = (size_t)win.begin(b);
     if (i >= T) return;
-    const float* qr = q + ((size_t)b * T + i) * ld + (size_t)h * hd;
-    const float* kb = k + (size_t)b * T * ld + (size_t)(h / group) * hd;
-    const float* vb = v + (size_t)b * T * ld + (size_t)(h / group) * hd;
+    const float* qr = q + (first + i) * ld + (size_t)h * hd;
+    const float* kb = k + first * ld + (size_t)(h / group) * hd;
+    const float* vb = v + first * ld + (size_t)(h / group) * hd;
     const float scale = 1.0f / sqrtf((float)hd);
     float qv[8], o[8];
 #pragma unroll
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(256) attn_prefill_any_kernel(const float* __re
         }
         m = mnew;
     }
-    float* op = out + ((size_t)b * T + i) * ldo + (size_t)h * hd;
+    float* op = out + (first + i) * ldo + (size_t)h * hd;
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
         const int c = lane + 32 * u;
@@ -268,21 +273,21 @@ __global__ void __launch_bounds__(256) attn_prefill_any_kernel(const float* __re
     }
 }
 
-int launch_attn_prefill_gqa(const float* q, const float* k, const float* v, int B, int T, int ld, int H, int KV, int hd,
+int launch_attn_prefill_gqa(const float* q, const float* k, const float* v, const Windows& w, int ld, int H, int KV, int hd,
                             int ldo, float* out, cudaStream_t st) {
     if (KV <= 0 || H % KV) return fail(FC_E_DIM, "n_heads %d must be a multiple of n_kv_heads %d", H, KV);
     const int group = H / KV;
-    dim3 grid((T + QT - 1) / QT, H, B);
+    dim3 grid((w.T + QT - 1) / QT, H, w.B);
     const bool aligned = ((ld | ldo) & 3) == 0 && ((((uintptr_t)q) | ((uintptr_t)k) | ((uintptr_t)v) | ((uintptr_t)out)) & 15) == 0;
     if (hd == 64 && aligned) {
         const size_t smem = (size_t)2 * KT * (64 + 4) * sizeof(float);
-        attn_prefill_kernel<64><<<grid, 256, smem, st>>>(q, k, v, T, ld, group, ldo, out);
+        attn_prefill_kernel<64><<<grid, 256, smem, st>>>(q, k, v, w, ld, group, ldo, out);
     } else if (hd == 32 && aligned) {
         const size_t smem = (size_t)2 * KT * (32 + 4) * sizeof(float);
-        attn_prefill_kernel<32><<<grid, 256, smem, st>>>(q, k, v, T, ld, group, ldo, out);
+        attn_prefill_kernel<32><<<grid, 256, smem, st>>>(q, k, v, w, ld, group, ldo, out);
     } else if (hd <= 256) {
-        dim3 g2((T + 7) / 8, H, B);
-        attn_prefill_any_kernel<<<g2, 256, 0, st>>>(q, k, v, T, ld, group, hd, ldo, out);
+        dim3 g2((w.T + 7) / 8, H, w.B);
+        attn_prefill_any_kernel<<<g2, 256, 0, st>>>(q, k, v, w, ld, group, hd, ldo, out);
     } else {
         return fail(FC_E_SHAPE, "window attention supports head_dim up to 256, got %d", hd);
     }
@@ -290,8 +295,8 @@ int launch_attn_prefill_gqa(const float* q, const float* k, const float* v, int 
     return FC_OK;
 }
 
-int launch_attn_prefill(const float* qkv, int B, int T, int d, int H, float* out, cudaStream_t st) {
-    return launch_attn_prefill_gqa(qkv, qkv + d, qkv + 2 * d, B, T, 3 * d, H, H, d / H, d, out, st);
+int launch_attn_prefill(const float* qkv, const Windows& w, int d, int H, float* out, cudaStream_t st) {
+    return launch_attn_prefill_gqa(qkv, qkv + d, qkv + 2 * d, w, 3 * d, H, H, d / H, d, out, st);
 }
 
 }  // namespace fc

@@ -4,28 +4,26 @@
 // (ferrum_core/src/layer/transformer.rs:395-477): S = Q Kᵀ / sqrt(hd), entries j > i masked,
 // row softmax, O = P V. The T x T probability matrix the reference keeps (`last_attention`,
 // transformer.rs:458-478) is never formed: keys are visited in tiles of 64 with an online
-// softmax. Both products run as bf16 3-term splits with fp32 accumulation (q = qh + ql,
-// k = kh + kl: qh·kh + ql·kh + qh·kl; the same for P·V), so they reproduce f32 products to
-// 2^-16 relative.
+// softmax. Both products run on bf16 planes with fp32 accumulation: with two planes as three products (q1·k1 + q1·k2 +
+// q2·k1; the same for P·V, so they reproduce f32 products to 2^-16 relative), with three planes (the f32 math mode) as six
+// (all of order up to 2^-16; what is dropped is 2^-24 of a product).
 //
-// Inputs are the bf16 hi / lo planes of the fused qkv rows [R][3d] written by the QKV GEMM;
-// the output is the pair of planes [R][d] the out-projection GEMM reads.
+// Inputs are the bf16 planes of the fused qkv rows [R][3d] written by the QKV GEMM; the output are the planes [R][d] the
+// out-projection GEMM reads. Windows of a batch may differ in length: they lie one after the other without padding.
 //
-// One CTA owns 128 query rows of one (window, head); two CTAs fit on an SM, so one's
-// softmax overlaps the other's MMAs.
+// One CTA owns 128 query rows of one (window, head); with two planes two CTAs fit on an SM, so one's softmax overlaps the
+// other's MMAs.
 //   warps 0-3   one query row per thread: tcgen05.ld the score tile, scale, mask, running
-//               max / sum, write P (bf16 hi / lo, 128-byte swizzle) to shared memory, then
+//               max / sum, write P (bf16 planes, 128-byte swizzle) to shared memory, then
 //               fold the P·V tile into the row's output registers;
 //   warp 4      TMA: Q once, then a K tile and a V tile (64 keys) per step;
-//   warp 5      tcgen05.mma issue: 12 MMAs for the score tile, 12 for P·V (V is consumed
+//   warp 5      tcgen05.mma issue: 12 (24) MMAs for the score tile, as many for P·V (V is consumed
 //               MN-major, exactly as TMA lays out its [keys][hd] rows).
 // Every mbarrier wait is bounded; on a timeout the status word is raised and the CTA leaves.
 //
 // Bound: tensor pipe / MUFU. 4·hd·T(T+1)/2 algorithmic FLOP per (window, head).
 #include <cuda.h>
-#include <cuda_bf16.h>
-
-#include "fc_common.cuh"
+#include "planes.cuh"
 
 namespace fc {
 
@@ -37,8 +35,11 @@ constexpr int KT = 64;                 // keys per step
 constexpr int Q_BYTES = QT * HD * 2;   // one bf16 plane of the Q tile: 16 KiB
 constexpr int KV_BYTES = KT * HD * 2;  // one bf16 plane of a K or V tile: 8 KiB
 constexpr int P_BYTES = QT * KT * 2;   // one bf16 plane of the P tile: 16 KiB
-constexpr int OFF_Q = 0, OFF_K = OFF_Q + 2 * Q_BYTES, OFF_V = OFF_K + 2 * KV_BYTES, OFF_P = OFF_V + 2 * KV_BYTES;
-constexpr int OFF_BARS = OFF_P + 2 * P_BYTES;
+// Shared memory of a CTA that works on P planes: 96 KB for two (two CTAs per SM), 144 KB for three.
+template <int P>
+struct Smem {
+    static constexpr int Q = 0, K = Q + P * Q_BYTES, V = K + P * KV_BYTES, PR = V + P * KV_BYTES, BARS = PR + P * P_BYTES;
+};
 constexpr int SOFTMAX_WARPS = 4, TMA_WARP = 4, MMA_WARP = 5, THREADS = 6 * 32;
 constexpr int TMEM_COLS = 128;         // score tile: columns 0..63, P·V tile: columns 64..127
 constexpr long long WAIT_CYCLES = 4000000000LL;
@@ -52,7 +53,8 @@ struct Bars {
     uint32_t tmem_base;
     volatile int abort;
 };
-constexpr int SMEM_BYTES = OFF_BARS + 1024 /* alignment slack */ + (int)sizeof(Bars);
+template <int P>
+constexpr int SMEM_BYTES = Smem<P>::BARS + 1024 /* alignment slack */ + (int)sizeof(Bars);
 
 __device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // 2^x on the special-function unit (2 ulp); 2^-inf = 0
@@ -124,37 +126,42 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
         : "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void split2(float w0, float w1, uint32_t* hi, uint32_t* lo) {
-    const __nv_bfloat162 h = __float22bfloat162_rn(make_float2(w0, w1));
-    const float2 hf = __bfloat1622float2(h);
-    const __nv_bfloat162 l = __float22bfloat162_rn(make_float2(w0 - hf.x, w1 - hf.y));
-    *hi = *(const uint32_t*)&h;
-    *lo = *(const uint32_t*)&l;
+// The products of planes i and j that a P-plane product keeps (i + j < P), the smallest first: they meet a small accumulator.
+template <int P, class F>
+__device__ __forceinline__ void each_term(F f) {
+#pragma unroll
+    for (int order = P - 1; order >= 0; --order)
+#pragma unroll
+        for (int i = 0; i <= order; ++i) f(i, order - i, order == P - 1 && i == 0);
 }
 
 struct AttnArgs {
-    int T;
+    Windows win;
     int k_col, v_col;            // first column of the key / value heads in the fused q | k | v planes
     int group;                   // query heads per key / value head (1: multi-head attention)
     int ldo;                     // row stride of the output planes (= query heads x 64)
-    uint16_t *out_hi, *out_lo;   // [R][ldo] bf16 planes
+    uint16_t* out[3];            // [R][ldo] bf16 planes
     int* status;
 };
 
 }  // namespace
 
-__global__ void __launch_bounds__(THREADS, 2)
-attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_hi, const __grid_constant__ CUtensorMap q_lo,
-                       const __grid_constant__ CUtensorMap kv_hi, const __grid_constant__ CUtensorMap kv_lo, const AttnArgs a) {
+struct AttnMaps { CUtensorMap q[3], kv[3]; };    // per plane: boxes of 128 query rows, of 64 key rows
+
+template <int P>
+__global__ void __launch_bounds__(THREADS, P == 2 ? 2 : 1)
+attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) {
+    constexpr int OFF_Q = Smem<P>::Q, OFF_K = Smem<P>::K, OFF_V = Smem<P>::V, OFF_P = Smem<P>::PR, OFF_BARS = Smem<P>::BARS;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     Bars* bars = (Bars*)(smem + OFF_BARS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int qt = (gridDim.x - 1) - blockIdx.x;          // long (late) query tiles first
     const int h = blockIdx.y, b = blockIdx.z;
-    const int row0 = b * a.T;                             // first row of the window in [R]
+    const int T = a.win.length(b), row0 = a.win.begin(b); // the window's rows in [R]
     const int q0 = qt * QT;                               // first query of the tile inside the window
-    const int last_q = min(a.T, q0 + QT) - 1;             // last valid query
+    if (q0 >= T) return;                                  // a window shorter than the longest
+    const int last_q = min(T, q0 + QT) - 1;               // last valid query
     const int n_kt = last_q / KT + 1;                     // key tiles 0..n_kt-1 cover keys 0..last_q
 
     if (threadIdx.x == 0) {
@@ -178,41 +185,37 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_hi, const __grid_co
 
     if (warp == TMA_WARP) {
         if (lane == 0) {
-            mbar_expect_tx(&bars->q_full, 2 * Q_BYTES);
-            tma_load_2d(smem + OFF_Q, &q_hi, h * HD, row0 + q0, &bars->q_full);
-            tma_load_2d(smem + OFF_Q + Q_BYTES, &q_lo, h * HD, row0 + q0, &bars->q_full);
+            mbar_expect_tx(&bars->q_full, P * Q_BYTES);
+#pragma unroll
+            for (int p = 0; p < P; ++p) tma_load_2d(smem + OFF_Q + p * Q_BYTES, &maps.q[p], h * HD, row0 + q0, &bars->q_full);
             for (int kt = 0; kt < n_kt; ++kt) {
                 const uint32_t par = (kt & 1) ^ 1;
                 if (!wait_bar(bars, &bars->k_empty, par, a.status)) break;
-                mbar_expect_tx(&bars->k_full, 2 * KV_BYTES);
-                tma_load_2d(smem + OFF_K, &kv_hi, a.k_col + (h / a.group) * HD, row0 + kt * KT, &bars->k_full);
-                tma_load_2d(smem + OFF_K + KV_BYTES, &kv_lo, a.k_col + (h / a.group) * HD, row0 + kt * KT, &bars->k_full);
+                mbar_expect_tx(&bars->k_full, P * KV_BYTES);
+#pragma unroll
+                for (int p = 0; p < P; ++p) tma_load_2d(smem + OFF_K + p * KV_BYTES, &maps.kv[p], a.k_col + (h / a.group) * HD, row0 + kt * KT, &bars->k_full);
                 if (!wait_bar(bars, &bars->v_empty, par, a.status)) break;
-                mbar_expect_tx(&bars->v_full, 2 * KV_BYTES);
-                tma_load_2d(smem + OFF_V, &kv_hi, a.v_col + (h / a.group) * HD, row0 + kt * KT, &bars->v_full);
-                tma_load_2d(smem + OFF_V + KV_BYTES, &kv_lo, a.v_col + (h / a.group) * HD, row0 + kt * KT, &bars->v_full);
+                mbar_expect_tx(&bars->v_full, P * KV_BYTES);
+#pragma unroll
+                for (int p = 0; p < P; ++p) tma_load_2d(smem + OFF_V + p * KV_BYTES, &maps.kv[p], a.v_col + (h / a.group) * HD, row0 + kt * KT, &bars->v_full);
             }
         }
     } else if (warp == MMA_WARP) {
         if (lane == 0) {
             const uint32_t sb = s32(smem);
-            const uint64_t qh = smem_desc(sb + OFF_Q), ql = smem_desc(sb + OFF_Q + Q_BYTES);
-            const uint64_t kh = smem_desc(sb + OFF_K), kl = smem_desc(sb + OFF_K + KV_BYTES);
-            const uint64_t vh = smem_desc(sb + OFF_V), vl = smem_desc(sb + OFF_V + KV_BYTES);
-            const uint64_t ph = smem_desc(sb + OFF_P), pl = smem_desc(sb + OFF_P + P_BYTES);
+            const uint64_t dq = smem_desc(sb + OFF_Q), dk = smem_desc(sb + OFF_K), dv = smem_desc(sb + OFF_V), dp = smem_desc(sb + OFF_P);
+            constexpr uint64_t QS = Q_BYTES / 16, KS = KV_BYTES / 16, PS = P_BYTES / 16;   // from plane to plane, in descriptor units
             bool ok = wait_bar(bars, &bars->q_full, 0, a.status);
             // score tile kt: its keys have landed and the softmax warps have read the previous one out of TMEM
             auto issue_scores = [&](int kt) -> bool {
                 const uint32_t par = kt & 1;
                 if (!(wait_bar(bars, &bars->k_full, par, a.status) && wait_bar(bars, &bars->s_empty, par ^ 1, a.status))) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                each_term<P>([&](int i, int j, bool first) {
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks) {
-                    const uint64_t adv = (uint64_t)(ks * 2);                 // 32 bytes along hd
-                    umma(tmem, qh + adv, kh + adv, IDESC_S, ks != 0);
-                    umma(tmem, ql + adv, kh + adv, IDESC_S, 1);
-                    umma(tmem, qh + adv, kl + adv, IDESC_S, 1);
-                }
+                    for (int ks = 0; ks < HD / 16; ++ks)                        // 32 bytes along hd per step
+                        umma(tmem, dq + i * QS + ks * 2, dk + j * KS + ks * 2, IDESC_S, !(first && ks == 0));
+                });
                 umma_commit(&bars->s_full);
                 umma_commit(&bars->k_empty);
                 return true;
@@ -231,14 +234,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_hi, const __grid_co
                      wait_bar(bars, &bars->o_empty, par ^ 1, a.status);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                each_term<P>([&](int i, int j, bool first) {
 #pragma unroll
-                for (int ks = 0; ks < KT / 16; ++ks) {
-                    const uint64_t pa = (uint64_t)(ks * 2);                  // 32 bytes along the keys of a P row
-                    const uint64_t va = (uint64_t)(ks * 128);                // 16 key rows of 128 bytes
-                    umma(tmem + HD, ph + pa, vh + va, IDESC_O, ks != 0);
-                    umma(tmem + HD, pl + pa, vh + va, IDESC_O, 1);
-                    umma(tmem + HD, ph + pa, vl + va, IDESC_O, 1);
-                }
+                    for (int ks = 0; ks < KT / 16; ++ks)                        // 32 bytes along the keys of a P row, 16 key rows of 128 bytes of V
+                        umma(tmem + HD, dp + i * PS + ks * 2, dv + j * KS + ks * 128, IDESC_O, !(first && ks == 0));
+                });
                 umma_commit(&bars->o_full);
                 umma_commit(&bars->v_empty);
             }
@@ -252,8 +252,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_hi, const __grid_co
 #pragma unroll
         for (int c = 0; c < HD; ++c) o[c] = 0.0f;
         float m = -INFINITY, l = 0.0f;
-        unsigned char* prow_hi = smem + OFF_P + r * 128;
-        unsigned char* prow_lo = prow_hi + P_BYTES;
+        unsigned char* prow = smem + OFF_P + r * 128;
         const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
         bool ok = true;
         for (int kt = 0; kt < n_kt && ok; ++kt) {
@@ -284,17 +283,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_hi, const __grid_co
             float psum = 0.0f;
 #pragma unroll
             for (int c = 0; c < KT / 8; ++c) {        // 16-byte chunk c of the P row: 8 keys
-                uint4 hi, lo;
                 float p[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) { p[e] = ex2_approx(fmaf(sv[8 * c + e], c2, off2)); psum += p[e]; }
-                split2(p[0], p[1], &hi.x, &lo.x);
-                split2(p[2], p[3], &hi.y, &lo.y);
-                split2(p[4], p[5], &hi.z, &lo.z);
-                split2(p[6], p[7], &hi.w, &lo.w);
-                const int chunk = (c ^ (r & 7)) * 16;  // 128-byte swizzle
-                *(uint4*)(prow_hi + chunk) = hi;
-                *(uint4*)(prow_lo + chunk) = lo;
+                uint32_t w[4][P];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) split2<P>(p[2 * e], p[2 * e + 1], w[e]);
+#pragma unroll
+                for (int t = 0; t < P; ++t)        // 128-byte swizzle
+                    *(uint4*)(prow + t * P_BYTES + (c ^ (r & 7)) * 16) = make_uint4(w[0][t], w[1][t], w[2][t], w[3][t]);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
@@ -317,18 +314,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_hi, const __grid_co
 #pragma unroll
             for (int c = 0; c < 32; ++c) { o[c] += __uint_as_float(s0[c]); o[32 + c] += __uint_as_float(s1[c]); }
         }
-        if (ok && qi < a.T) {
+        if (ok && qi < T) {
             const float inv = 1.0f / l;
             const size_t off = (size_t)(row0 + qi) * a.ldo + (size_t)h * HD;
 #pragma unroll
             for (int c = 0; c < HD / 8; ++c) {
-                uint4 hi, lo;
-                split2(o[8 * c] * inv, o[8 * c + 1] * inv, &hi.x, &lo.x);
-                split2(o[8 * c + 2] * inv, o[8 * c + 3] * inv, &hi.y, &lo.y);
-                split2(o[8 * c + 4] * inv, o[8 * c + 5] * inv, &hi.z, &lo.z);
-                split2(o[8 * c + 6] * inv, o[8 * c + 7] * inv, &hi.w, &lo.w);
-                *(uint4*)(a.out_hi + off + 8 * c) = hi;
-                *(uint4*)(a.out_lo + off + 8 * c) = lo;
+                uint32_t w[4][P];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) split2<P>(o[8 * c + 2 * e] * inv, o[8 * c + 2 * e + 1] * inv, w[e]);
+#pragma unroll
+                for (int t = 0; t < P; ++t) *(uint4*)(a.out[t] + off + 8 * c) = make_uint4(w[0][t], w[1][t], w[2][t], w[3][t]);
             }
         }
     }
@@ -367,35 +362,42 @@ int encode(CUtensorMap* map, const void* plane, size_t rows, size_t cols, int bo
 }
 }  // namespace
 
-// qkv: bf16 planes [B*T][H*64 + 2*KV*64] (q heads | k heads | v heads per row); out: planes [B*T][H*64]. Query head h reads key / value head h / (H / KV).
-int launch_attn_prefill_tc_gqa(const Planes& qkv, int B, int T, int H, int KV, const Planes& out, int* status, cudaStream_t st) {
+// qkv: bf16 planes [R][H*64 + 2*KV*64] (q heads | k heads | v heads per row); out: planes [R][H*64]. Query head h reads key /
+// value head h / (H / KV).
+template <int P>
+static int launch_attn_tc(const Planes& qkv, const Windows& w, int R, int H, int KV, const Planes& out, int* status, cudaStream_t st) {
     if (KV <= 0 || H % KV) return fail(FC_E_DIM, "n_heads %d must be a multiple of n_kv_heads %d", H, KV);
     static bool attr_set[64] = {};
     int dev = 0;
     FC_CUDA(cudaGetDevice(&dev));
     if (dev < 64 && !attr_set[dev]) {
-        FC_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        FC_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES<P>));
         attr_set[dev] = true;
     }
-    const size_t R = (size_t)B * T, ld = (size_t)(H + 2 * KV) * HD;
-    CUtensorMap qh, ql, kh, kl;
-    FC_TRY(encode(&qh, qkv.p[0], R, ld, QT));
-    FC_TRY(encode(&ql, qkv.p[1], R, ld, QT));
-    FC_TRY(encode(&kh, qkv.p[0], R, ld, KT));
-    FC_TRY(encode(&kl, qkv.p[1], R, ld, KT));
+    const size_t ld = (size_t)(H + 2 * KV) * HD;
+    AttnMaps maps;
     AttnArgs a;
-    a.T = T; a.k_col = H * HD; a.v_col = (H + KV) * HD; a.group = H / KV; a.ldo = H * HD;
-    a.out_hi = (uint16_t*)out.p[0]; a.out_lo = (uint16_t*)out.p[1]; a.status = status;
-    dim3 grid((T + QT - 1) / QT, H, B);
-    attn_prefill_tc_kernel<<<grid, THREADS, SMEM_BYTES, st>>>(qh, ql, kh, kl, a);
+    for (int p = 0; p < P; ++p) {
+        FC_TRY(encode(&maps.q[p], qkv.p[p], R, ld, QT));
+        FC_TRY(encode(&maps.kv[p], qkv.p[p], R, ld, KT));
+        a.out[p] = (uint16_t*)out.p[p];
+    }
+    a.win = w; a.k_col = H * HD; a.v_col = (H + KV) * HD; a.group = H / KV; a.ldo = H * HD;
+    a.status = status;
+    dim3 grid((w.T + QT - 1) / QT, H, w.B);
+    attn_prefill_tc_kernel<P><<<grid, THREADS, SMEM_BYTES<P>, st>>>(maps, a);
     FC_LAUNCHED();
     return FC_OK;
 }
 
-// The multi-head form: planes [B*T][3d] in, [B*T][d] out.
-int launch_attn_prefill_tc(const Planes& qkv, int B, int T, int d, int H, const Planes& out, int* status, cudaStream_t st) {
+int launch_attn_prefill_tc_gqa(const Planes& qkv, const Windows& w, int R, int H, int KV, const Planes& out, int* status, cudaStream_t st) {
+    return qkv.n == 3 ? launch_attn_tc<3>(qkv, w, R, H, KV, out, status, st) : launch_attn_tc<2>(qkv, w, R, H, KV, out, status, st);
+}
+
+// The multi-head form: planes [R][3d] in, [R][d] out.
+int launch_attn_prefill_tc(const Planes& qkv, const Windows& w, int R, int d, int H, const Planes& out, int* status, cudaStream_t st) {
     if (d != H * HD) return fail(FC_E_SHAPE, "tensor-core attention needs head_dim 64 (d = %d, H = %d)", d, H);
-    return launch_attn_prefill_tc_gqa(qkv, B, T, H, H, out, status, st);
+    return launch_attn_prefill_tc_gqa(qkv, w, R, H, H, out, status, st);
 }
 
 }  // namespace fc

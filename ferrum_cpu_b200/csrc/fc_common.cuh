@@ -137,6 +137,15 @@ int launch_gemv_q8_stream(const QMat& w, const float* x, const float* norm_w, fl
 
 // An f32 matrix as n bf16 planes whose sum it is: 2 planes hold it to 2^-17 relative (FC_MATH_BF16X3), 3 exactly
 // (FC_MATH_FP32). The form in which activations reach the tensor cores.
+// Windows of rows that share a forward pass: window b holds rows starts[b] .. starts[b + 1] (device array of B + 1), or, with
+// starts == nullptr, T rows each. T: rows of the longest.
+struct Windows {
+    int B = 0, T = 0;
+    const int* starts = nullptr;
+    __host__ __device__ int begin(int b) const { return starts ? starts[b] : b * T; }
+    __host__ __device__ int length(int b) const { return starts ? starts[b + 1] - starts[b] : T; }
+};
+
 struct Planes {
     void* p[3] = {nullptr, nullptr, nullptr};
     int n = 0;
@@ -165,12 +174,15 @@ const QMat* qweight_matrix(const fc_qweight* w, int* device);
 // rowops.cu
 int launch_embed_step(const QMat& tok, const float* pos_emb, int ctx, const int* queue, StepState* state,
                       float* x, cudaStream_t st);
-int launch_embed_rows(const QMat& tok, const float* pos_emb, const int* ids, int R, int T, float* x,
+// pos: each row's position in its window, or null: r % T.
+int launch_embed_rows(const QMat& tok, const float* pos_emb, const int* ids, const int* pos, int R, int T, float* x,
                       int* error_flag, cudaStream_t st);
 int launch_layernorm(const float* x, const float* g, const float* b, int rows, int d, float* y,
                      const StepState* state, cudaStream_t st);
-// LayerNorm written as bf16 planes [rows][d] for the tensor-core GEMM.
-int launch_layernorm_planes(const float* x, const float* g, const float* b, int rows, int d, const Planes& out, cudaStream_t st);
+// LayerNorm written as bf16 planes [rows][d] for the tensor-core GEMM. pick (may be null): row i of the output is row pick[i]
+// of x.
+int launch_layernorm_planes(const float* x, const float* g, const float* b, const int* pick, int rows, int d, const Planes& out,
+                            cudaStream_t st);
 // Decode tail over logits[V]: softmax statistics, optional probs[V], optional greedy select
 // (append to queue) — and always the end-of-step bookkeeping (pos, fed).
 int launch_step_tail(const float* logits, int V, float* probs_or_null, int do_select, int* queue, int queue_cap,
@@ -210,19 +222,19 @@ int launch_layer_stats(const float* x, const Planes& planes, size_t n, void* scr
 // attn.cu
 int launch_attn_decode(const float* q, const float* kcache, const float* vcache, int d, int H, int ctx,
                        const StepState* state, float* out, cudaStream_t st);
-// qkv [R][3d] (q | k | v per row), R = B·T, causal within each window of T rows.
-int launch_attn_prefill(const float* qkv, int B, int T, int d, int H, float* out, cudaStream_t st);
+// qkv [R][3d] (q | k | v per row), causal within each window.
+int launch_attn_prefill(const float* qkv, const Windows& w, int d, int H, float* out, cudaStream_t st);
 // Grouped-query forms (llm.rs:305-341): H query heads share KV key/value heads of width hd.
 // Decode: q [H*hd], caches [ctx][KV*hd]. Window: q, k, v rows ld floats apart, out rows ldo apart.
 int launch_attn_decode_gqa(const float* q, const float* kcache, const float* vcache, int H, int KV, int hd, int ctx,
                            const StepState* state, float* out, cudaStream_t st);
-int launch_attn_prefill_gqa(const float* q, const float* k, const float* v, int B, int T, int ld, int H, int KV, int hd,
+int launch_attn_prefill_gqa(const float* q, const float* k, const float* v, const Windows& w, int ld, int H, int KV, int hd,
                             int ldo, float* out, cudaStream_t st);
-// attn_tc.cu — the same on tcgen05 (head_dim 64): bf16 planes (two) of qkv [B*T][3d] in, planes of the attention output
-// [B*T][d] out; `status` is raised on a timeout.
-int launch_attn_prefill_tc(const Planes& qkv, int B, int T, int d, int H, const Planes& out, int* status, cudaStream_t st);
-// Grouped-query form: planes [B*T][(H + 2 KV) * 64] in (q heads | k heads | v heads), [B*T][H * 64] out.
-int launch_attn_prefill_tc_gqa(const Planes& qkv, int B, int T, int H, int KV, const Planes& out, int* status, cudaStream_t st);
+// attn_tc.cu — the same on tcgen05 (head_dim 64): bf16 planes (two or three) of qkv [R][3d] in, as many planes of the
+// attention output [R][d] out; `status` is raised on a timeout.
+int launch_attn_prefill_tc(const Planes& qkv, const Windows& w, int R, int d, int H, const Planes& out, int* status, cudaStream_t st);
+// Grouped-query form: planes [R][(H + 2 KV) * 64] in (q heads | k heads | v heads), [R][H * 64] out.
+int launch_attn_prefill_tc_gqa(const Planes& qkv, const Windows& w, int R, int H, int KV, const Planes& out, int* status, cudaStream_t st);
 
 // decode_batch.cu — one lock-step decode step for S <= kBatchMaxStreams streams.
 // Fragment-major copy of a Q8_0 matrix for the warp-level tensor-core product: per (16 rows,

@@ -173,29 +173,35 @@ int forward_rows(fc_llama* m, int B, int T, fc_llama_cache* fill = nullptr) {
     cudaStream_t st = m->st;
     FC_CUDA(cudaMemsetAsync(m->err_d, 0, sizeof(int), st));
     FC_TRY(launch_llama_embed_rows(m->tok, m->ids_d, R, m->x, m->err_d, st));
+    Windows win;
+    win.B = B; win.T = T;
     const int planes = model_planes(m);
     m->px.n = m->pqkv.n = m->patt.n = m->phid.n = planes;
-    // the attention runs on tcgen05 on two planes and heads of 64; a cache fill needs the rotated f32 rows
-    const bool tc_attn = planes == 2 && c.head_dim == 64 && !fill && (size_t)m->qkv_dim * 4 <= 48 * 1024;
+    // heads of 64 attend on tcgen05
+    const bool tc_attn = c.head_dim == 64 && (size_t)m->qkv_dim * 4 <= 48 * 1024;
     for (int l = 0; l < c.n_layer; ++l) {
         const LlamaLayerDev& L = m->layers[l];
         // LlamaBlock::forward_full (llm.rs:464-482); norms and the gate write the planes the next GEMM reads
         FC_TRY(launch_llama_rmsnorm_planes(m->x, L.attn_norm, c.norm_eps, R, d, m->px, st));
         FC_TRY(launch_gemm_q8_tc(L.qkv, m->px, L.qkv_b, nullptr, EPI_NONE, m->qkv, nullptr, R, m->qkv_dim, m->tc_status, st, fill != nullptr));
-        if (tc_attn) {
+        if (tc_attn && !fill) {
             // rotate and split in one pass: the attention reads planes, nothing reads the rotated f32 rows
             FC_TRY(launch_llama_rope_planes(m->qkv, R, m->qkv_dim, T, c.n_head, c.n_kv_head, m->q_dim, c.head_dim, c.rope_dim,
                                             c.rope_type == FC_ROPE_NEOX, m->ftab, m->inv_linear, m->pqkv, st));
-            FC_TRY(launch_attn_prefill_tc_gqa(m->pqkv, B, T, c.n_head, c.n_kv_head, m->patt, m->tc_status, st));
         } else {
             FC_TRY(launch_llama_rope_rows(m->qkv, R, m->qkv_dim, T, c.n_head, c.n_kv_head, m->q_dim, c.head_dim, c.rope_dim,
                                           c.rope_type == FC_ROPE_NEOX, m->ftab, m->inv_linear, st));
-            if (fill) {
-                const size_t layer_stride = (size_t)c.ctx * m->kv_dim;
-                FC_TRY(launch_llama_store_kv_rows(m->qkv, R, m->qkv_dim, m->q_dim, m->kv_dim, fill->kc + l * layer_stride,
-                                                  fill->vc + l * layer_stride, st));
-            }
-            FC_TRY(launch_attn_prefill_gqa(m->qkv, m->qkv + m->q_dim, m->qkv + m->q_dim + m->kv_dim, B, T, m->qkv_dim, c.n_head,
+            if (tc_attn) FC_TRY(launch_split_planes(m->qkv, m->pqkv, (size_t)R * m->qkv_dim, st));
+        }
+        if (fill) {
+            const size_t layer_stride = (size_t)c.ctx * m->kv_dim;
+            FC_TRY(launch_llama_store_kv_rows(m->qkv, R, m->qkv_dim, m->q_dim, m->kv_dim, fill->kc + l * layer_stride,
+                                              fill->vc + l * layer_stride, st));
+        }
+        if (tc_attn) {
+            FC_TRY(launch_attn_prefill_tc_gqa(m->pqkv, win, R, c.n_head, c.n_kv_head, m->patt, m->tc_status, st));
+        } else {
+            FC_TRY(launch_attn_prefill_gqa(m->qkv, m->qkv + m->q_dim, m->qkv + m->q_dim + m->kv_dim, win, m->qkv_dim, c.n_head,
                                            c.n_kv_head, c.head_dim, m->q_dim, m->att, st));
             FC_TRY(launch_split_planes(m->att, m->patt, (size_t)R * m->q_dim, st));
         }
@@ -259,6 +265,8 @@ int forward_rows_packed(fc_llama* m, int B, int T, fc_llama_cache* fill) {
     FC_CUDA(cudaMemsetAsync(m->err_d, 0, sizeof(int), st));
     if (m->native_tok) FC_TRY(launch_ggml_rows(m->native_tok, m->ids_d, nullptr, nullptr, c.ctx, R, m->x, m->err_d, st));
     else FC_TRY(launch_llama_embed_rows(m->tok, m->ids_d, R, m->x, m->err_d, st));
+    Windows win;
+    win.B = B; win.T = T;
     for (int l = 0; l < c.n_layer; ++l) {
         FC_TRY(packed_block(m, l, R, m->x, m->n, m->qkv, m->att, m->gu, m->hid, nullptr, [&]() -> int {
             FC_TRY(launch_llama_rope_rows(m->qkv, R, m->qkv_dim, T, c.n_head, c.n_kv_head, m->q_dim, c.head_dim, c.rope_dim,
@@ -268,7 +276,7 @@ int forward_rows_packed(fc_llama* m, int B, int T, fc_llama_cache* fill) {
                 FC_TRY(launch_llama_store_kv_rows(m->qkv, R, m->qkv_dim, m->q_dim, m->kv_dim, fill->kc + l * layer_stride,
                                                   fill->vc + l * layer_stride, st));
             }
-            return launch_attn_prefill_gqa(m->qkv, m->qkv + m->q_dim, m->qkv + m->q_dim + m->kv_dim, B, T, m->qkv_dim, c.n_head,
+            return launch_attn_prefill_gqa(m->qkv, m->qkv + m->q_dim, m->qkv + m->q_dim + m->kv_dim, win, m->qkv_dim, c.n_head,
                                            c.n_kv_head, c.head_dim, m->q_dim, m->att, st);
         }));
     }

@@ -155,8 +155,9 @@ __global__ void llama_rope_rows_kernel(float* __restrict__ qkv, int ld, int T, i
         rotate_pair(row, ia, ib, rope_angle(pos, ftab[i], inv_linear));
     }
 }
-// The same rotation with the row handed on as bf16 hi / lo planes (the input of the tensor-core
+// The same rotation with the row handed on as bf16 planes (the input of the tensor-core
 // attention): the f32 row is staged in shared memory, rotated there and written once.
+template <int P>
 __global__ void llama_rope_planes_kernel(const float* __restrict__ qkv, int ld, int T, int n_q, int n_kv, int k_off, int hd, int half,
                                          int neox, const float2* __restrict__ ftab, float inv_linear, const Planes out) {
     extern __shared__ float srow[];
@@ -172,13 +173,14 @@ __global__ void llama_rope_planes_kernel(const float* __restrict__ qkv, int ld, 
         rotate_pair(srow, ia, ib, rope_angle(pos, ftab[i], inv_linear));
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < ld; c += blockDim.x) store_planes<2>(out, (size_t)r * ld + c, srow[c]);
+    for (int c = threadIdx.x; c < ld; c += blockDim.x) store_planes<P>(out, (size_t)r * ld + c, srow[c]);
 }
 int launch_llama_rope_planes(const float* qkv, int R, int ld, int T, int n_q, int n_kv, int k_off, int hd, int rope_dim, int neox,
                              const float2* ftab, float inv_linear, const Planes& out, cudaStream_t st) {
     const size_t smem = (size_t)ld * sizeof(float);
     if (smem > 48 * 1024) return fail(FC_E_SHAPE, "fused q | k | v rows of %d floats exceed the rotation kernel's staging", ld);
-    llama_rope_planes_kernel<<<R, 256, smem, st>>>(qkv, ld, T, n_q, n_kv, k_off, hd, rope_dim / 2, neox, ftab, inv_linear, out);
+    if (out.n == 3) llama_rope_planes_kernel<3><<<R, 256, smem, st>>>(qkv, ld, T, n_q, n_kv, k_off, hd, rope_dim / 2, neox, ftab, inv_linear, out);
+    else llama_rope_planes_kernel<2><<<R, 256, smem, st>>>(qkv, ld, T, n_q, n_kv, k_off, hd, rope_dim / 2, neox, ftab, inv_linear, out);
     FC_LAUNCHED();
     return FC_OK;
 }

@@ -78,9 +78,9 @@ int launch_embed_step(const QMat& tok, const float* pos_emb, int ctx, const int*
     return FC_OK;
 }
 
-__global__ void embed_rows_kernel(QMat tok, const float* __restrict__ pos_emb, const int* __restrict__ ids,
+__global__ void embed_rows_kernel(QMat tok, const float* __restrict__ pos_emb, const int* __restrict__ ids, const int* __restrict__ pos,
                                   int T, float* __restrict__ x, int* error_flag) {
-    const int r = blockIdx.x, t = r % T;
+    const int r = blockIdx.x, t = pos ? pos[r] : r % T;
     int id = ids[r];
     if (id < 0 || id >= tok.N) {
         if (threadIdx.x == 0) atomicExch(error_flag, FC_E_DIM);
@@ -90,9 +90,9 @@ __global__ void embed_rows_kernel(QMat tok, const float* __restrict__ pos_emb, c
         x[(size_t)r * tok.K + c] = tok_value(tok, id, c) + pos_emb[(size_t)t * tok.K + c];
 }
 
-int launch_embed_rows(const QMat& tok, const float* pos_emb, const int* ids, int R, int T, float* x,
+int launch_embed_rows(const QMat& tok, const float* pos_emb, const int* ids, const int* pos, int R, int T, float* x,
                       int* error_flag, cudaStream_t st) {
-    embed_rows_kernel<<<R, 256, 0, st>>>(tok, pos_emb, ids, T, x, error_flag);
+    embed_rows_kernel<<<R, 256, 0, st>>>(tok, pos_emb, ids, pos, T, x, error_flag);
     FC_LAUNCHED();
     return FC_OK;
 }
@@ -134,9 +134,9 @@ __global__ void layernorm_kernel(const float* __restrict__ x, const float* __res
 // The same LayerNorm with the result written as the P bf16 planes that the tensor-core GEMM reads.
 template <int PER, int P>
 __global__ void layernorm_planes_kernel(const float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ b,
-                                        int d, const Planes out) {
+                                        const int* __restrict__ pick, int d, const Planes out) {
     __shared__ float red[33];
-    const float* xr = x + (size_t)blockIdx.x * d;
+    const float* xr = x + (size_t)(pick ? pick[blockIdx.x] : (int)blockIdx.x) * d;
     float v[PER];
     float s = 0.0f;
 #pragma unroll
@@ -166,12 +166,13 @@ __global__ void layernorm_planes_kernel(const float* __restrict__ x, const float
 // the two sums by shuffles (no block-wide synchronisation), the planes written 8 bytes per lane. Eight rows per CTA.
 template <int NV, int P>
 __global__ void __launch_bounds__(256) layernorm_planes_warp_kernel(const float* __restrict__ x, const float* __restrict__ g,
-                                                                    const float* __restrict__ b, int rows, int d, const Planes out) {
+                                                                    const float* __restrict__ b, const int* __restrict__ pick, int rows,
+                                                                    int d, const Planes out) {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int nv = d >> 7;                                  // 16-byte chunks per lane
-    const float4* xr = (const float4*)(x + (size_t)row * d);
+    const float4* xr = (const float4*)(x + (size_t)(pick ? pick[row] : row) * d);
     float4 v[NV];
     float s = 0.0f;
 #pragma unroll
@@ -205,25 +206,27 @@ __global__ void __launch_bounds__(256) layernorm_planes_warp_kernel(const float*
 }
 
 template <int P>
-static int layernorm_planes(const float* x, const float* g, const float* b, int rows, int d, const Planes& out, cudaStream_t st) {
+static int layernorm_planes(const float* x, const float* g, const float* b, const int* pick, int rows, int d, const Planes& out,
+                            cudaStream_t st) {
     if (d % 128 == 0 && d <= 1024 && aligned16(x) && aligned16(g) && aligned16(b)) {
         const int blocks = (rows + 7) / 8;
-        if (d <= 512) layernorm_planes_warp_kernel<4, P><<<blocks, 256, 0, st>>>(x, g, b, rows, d, out);
-        else layernorm_planes_warp_kernel<8, P><<<blocks, 256, 0, st>>>(x, g, b, rows, d, out);
+        if (d <= 512) layernorm_planes_warp_kernel<4, P><<<blocks, 256, 0, st>>>(x, g, b, pick, rows, d, out);
+        else layernorm_planes_warp_kernel<8, P><<<blocks, 256, 0, st>>>(x, g, b, pick, rows, d, out);
         FC_LAUNCHED();
         return FC_OK;
     }
     const int threads = 256;
     const int per = (d + threads - 1) / threads;
-    if (per <= 4) layernorm_planes_kernel<4, P><<<rows, threads, 0, st>>>(x, g, b, d, out);
-    else if (per <= 8) layernorm_planes_kernel<8, P><<<rows, threads, 0, st>>>(x, g, b, d, out);
-    else if (per <= 16) layernorm_planes_kernel<16, P><<<rows, threads, 0, st>>>(x, g, b, d, out);
+    if (per <= 4) layernorm_planes_kernel<4, P><<<rows, threads, 0, st>>>(x, g, b, pick, d, out);
+    else if (per <= 8) layernorm_planes_kernel<8, P><<<rows, threads, 0, st>>>(x, g, b, pick, d, out);
+    else if (per <= 16) layernorm_planes_kernel<16, P><<<rows, threads, 0, st>>>(x, g, b, pick, d, out);
     else return fail(FC_E_SHAPE, "LayerNorm width %d exceeds 4096", d);
     FC_LAUNCHED();
     return FC_OK;
 }
-int launch_layernorm_planes(const float* x, const float* g, const float* b, int rows, int d, const Planes& out, cudaStream_t st) {
-    return out.n == 3 ? layernorm_planes<3>(x, g, b, rows, d, out, st) : layernorm_planes<2>(x, g, b, rows, d, out, st);
+int launch_layernorm_planes(const float* x, const float* g, const float* b, const int* pick, int rows, int d, const Planes& out,
+                            cudaStream_t st) {
+    return out.n == 3 ? layernorm_planes<3>(x, g, b, pick, rows, d, out, st) : layernorm_planes<2>(x, g, b, pick, rows, d, out, st);
 }
 
 int launch_layernorm(const float* x, const float* g, const float* b, int rows, int d, float* y,
