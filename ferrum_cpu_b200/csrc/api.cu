@@ -552,8 +552,7 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
     FC_CUDA(cudaSetDevice(w->device));
     cudaStream_t st = (cudaStream_t)cuda_stream;
     if (M == 1) {
-        GemvOut o; o.out[0] = y_dev;
-        return launch_gemv_q8(w->w, x_dev, bias_dev, nullptr, EPI_NONE, o, nullptr, st);
+        return launch_gemv_row(w->w, x_dev, nullptr, 0.0f, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, st);
     }
     // the bf16 planes of x and the status word live in the weight handle and grow on demand
     fc_qweight* wm = const_cast<fc_qweight*>(w);

@@ -76,7 +76,7 @@ int upload_q8(Arena& ar, const void* host, int N, int K, QMat* out, cudaStream_t
 // The 34-byte GGML blocks are split at upload into two planes so that every row starts
 // on a 16-byte boundary:
 //   qu [N_pad][K]      uint8  = int8 quant XOR 0x80 (i.e. q + 128), K contiguous
-//   d  [N_pad][K/32]   f16    block scales
+//   d  [N_pad][K/32]   f16    block scales; null: levels alone (scale 1), as a packed QWeight keeps them
 // Rows N..N_pad-1 are zero scale / 0x80 quants (value 0) so tiles may read them.
 struct QMat {
     const uint8_t* qu = nullptr;
@@ -129,11 +129,25 @@ int launch_gemv_q8(const QMat& w, const float* x, const float* bias, const float
 int launch_gemv_q8_wide(const QMat& w, const float* x, const float* norm_w, float eps, const float* bias, const float* residual,
                         int epi, float* out, const StepState* state, cudaStream_t st);
 
-// gemv_stream.cu — the same contract on a persistent kernel that streams row tiles through a
-// shared-memory ring with bulk async copies; `status` (device int) is raised to FC_E_TIMEOUT when
-// a bounded wait runs out. Shapes the ring does not cover take launch_gemv_q8_wide.
-int launch_gemv_q8_stream(const QMat& w, const float* x, const float* norm_w, float eps, const float* bias, const float* residual,
-                          int epi, float* out, const StepState* state, int* status, cudaStream_t st);
+// gemv_row.cu — one activation row against up to three matrices (q | k | v, gate | up) of the same K. part.d: f16 scales per
+// 32 of k, or null with part.xscale [K]: the scale of input index k (then levels alone). Optional RMSNorm of x (norm_w, eps)
+// as it is staged; EPI_SWIGLU pairs rows (2i, 2i + 1) of one matrix, or row i of two, as (gate, up) and writes
+// part[0].out[i] = silu(gate) * up. Launched as a programmatic dependent.
+struct GemvPart {
+    const uint8_t* qu = nullptr;
+    const __half* d = nullptr;
+    const float* xscale = nullptr;
+    const float* bias = nullptr;
+    float* out = nullptr;
+    int N = 0;
+};
+int launch_gemv_row(const GemvPart* parts, int n_parts, int K, const float* x, const float* norm_w, float eps, const float* residual,
+                    int epi, const StepState* state, cudaStream_t st);
+inline int launch_gemv_row(const QMat& w, const float* x, const float* norm_w, float eps, const float* bias, const float* residual,
+                           int epi, float* out, const StepState* state, cudaStream_t st) {
+    const GemvPart p = {w.qu, w.d, nullptr, bias, out, w.N};
+    return launch_gemv_row(&p, 1, w.K, x, norm_w, eps, residual, epi, state, st);
+}
 
 // An f32 matrix as n bf16 planes whose sum it is: 2 planes hold it to 2^-17 relative (FC_MATH_BF16X3), 3 exactly
 // (FC_MATH_FP32). The form in which activations reach the tensor cores.
@@ -150,7 +164,8 @@ struct Planes {
     void* p[3] = {nullptr, nullptr, nullptr};
     int n = 0;
 };
-int launch_split_planes(const float* x, const Planes& out, size_t n, cudaStream_t st);
+// cols (may be null): column k of rows K wide is multiplied by cols[k] first.
+int launch_split_planes(const float* x, const Planes& out, size_t n, cudaStream_t st, const float* cols = nullptr, int K = 4);
 // gemm_tc.cu — Y[M][N] = X[M][K]·Wᵀ + bias (+GELU / SwiGLU) (+residual[M][N]) on tcgen05 tensor cores, the weight exact, X
 // as planes [M][K]. Output: f32 rows y, or (y == nullptr) planes yp for the next GEMM, as many as X has.
 // `status` is a device int raised to FC_E_TIMEOUT when a bounded wait runs out. split_k: few rows may split the K range
@@ -206,10 +221,12 @@ int ggml_weight_rows(const fc_ggml_weight* w);
 int ggml_weight_cols(const fc_ggml_weight* w);
 
 // Per-row-scale int8 / int4 linear on a packed matrix (rowq.cu): y[M][ldy] = [residual +] bias + x · W; bias and residual may
-// be null, residual may be y itself.
-int launch_rowq_linear(fc_rowq* w, const float* x, const float* bias, const float* residual, float* y, int ldy, int M, cudaStream_t st);
-int rowq_in(const fc_rowq* w);
-int rowq_out(const fc_rowq* w);
+// be null, residual may be y itself. scratch: three planes of M x K the caller lends (several rows), with the status word of
+// the product, or null: the weight's own.
+int launch_rowq_linear(fc_rowq* w, const float* x, const float* bias, const float* residual, float* y, int ldy, int M, cudaStream_t st,
+                       const Planes* scratch = nullptr, int* status = nullptr);
+// The matrix as rows of levels and its input scales, or false (shapes only the packed form covers).
+bool rowq_part(const fc_rowq* w, const float* bias, float* out, GemvPart* part);
 
 struct LayerStatsDev {
     float min, max, mean, pad;

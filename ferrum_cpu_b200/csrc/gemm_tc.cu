@@ -482,9 +482,10 @@ gemm_q8_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             // two stages of levels and scales are under way at any time, in two sets of registers that take turns: with one
             // stage ahead, a stage could not come more often than an L2 round trip
             struct Row { uint4 q[2]; __half d; } ra, rb;
+            ra.d = rb.d = __float2half(1.0f);                                       // a matrix of levels alone has no scales
             auto fetch = [&](Row& r, int kb) {
                 const bool have = real && kb < st1 && 2 * kb + hk < nb;
-                if (have) r.d = dsrc[2 * kb + hk];
+                if (have && a.d) r.d = dsrc[2 * kb + hk];
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
                     r.q[i] = have ? __ldg(src + (2 * kb + hk) * 2 + i) : make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);   // biased zeros
@@ -813,18 +814,24 @@ int launch_tc(const QMat& w, const Planes& x, TcArgs a, int M, bool split_k, cud
 }
 
 template <int P>
-__global__ void split_planes_kernel(const float* __restrict__ x, const Planes out, size_t n4) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x)
-        store_planes4<P>(out, i, ((const float4*)x)[i]);
+__global__ void split_planes_kernel(const float* __restrict__ x, const float* __restrict__ cols, int k4, const Planes out, size_t n4) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
+        float4 v = ((const float4*)x)[i];
+        if (cols) {
+            const float4 s = ((const float4*)cols)[i % k4];
+            v.x *= s.x; v.y *= s.y; v.z *= s.z; v.w *= s.w;
+        }
+        store_planes4<P>(out, i, v);
+    }
 }
 }  // namespace
 
-int launch_split_planes(const float* x, const Planes& out, size_t n, cudaStream_t st) {
-    if (n % 4) return fail(FC_E_SHAPE, "split_planes: element count %zu is not a multiple of 4", n);
+int launch_split_planes(const float* x, const Planes& out, size_t n, cudaStream_t st, const float* cols, int K) {
+    if (n % 4 || (cols && K % 4)) return fail(FC_E_SHAPE, "split_planes: element count %zu is not a multiple of 4", n);
     const size_t n4 = n / 4;
     const int blocks = (int)std::max<size_t>(1, std::min<size_t>((n4 + 255) / 256, 148 * 8));
-    if (out.n == 3) split_planes_kernel<3><<<blocks, 256, 0, st>>>(x, out, n4);
-    else split_planes_kernel<2><<<blocks, 256, 0, st>>>(x, out, n4);
+    if (out.n == 3) split_planes_kernel<3><<<blocks, 256, 0, st>>>(x, cols, K / 4, out, n4);
+    else split_planes_kernel<2><<<blocks, 256, 0, st>>>(x, cols, K / 4, out, n4);
     FC_LAUNCHED();
     return FC_OK;
 }

@@ -1,0 +1,265 @@
+// One activation row against quantised matrices: the projections of a decode step and the M = 1 linear.
+//
+//     y[n] = (residual[n] +) bias[n] + sum_k xhat[k] * w[n][k],   xhat = x, or RMSNorm(x) (llm.rs:57-64)
+//
+// Up to three matrices share the row (q | k | v, gate | up). A matrix is a QMat: int8 levels with an f16 scale per 32 of k
+// (Q8_0), or levels alone whose scale belongs to the input index (the per-row-scale QWeight of quant.rs:122-146): then
+// xhat[k] * scale[k] is staged per matrix (ops.rs:336-342).
+//
+// A step of a decoder is a chain of such products, each a few microseconds long, so what counts is how little happens
+// between "the row is there" and "the result is there":
+//  - a warp owns RB rows (or a K slice of them) from the first load to the dot product: lanes across k, 16 levels each. It
+//    asks for the first rows BEFORE it waits for the kernel ahead (weights depend on nothing), so small matrices are in
+//    registers when the activations appear; the next rows are asked for before the current ones are multiplied;
+//  - the row is staged in shared memory once (two block barriers with the norm, one without); from there on warps do not
+//    meet, unless K is wider than 2048 and `ks` of them share a row;
+//  - few rows take few warps per CTA, spread over all SMs.
+// Bound: HBM for wide matrices (N*K*34/32 or N*K bytes), otherwise the launch-to-launch latency.
+// (The kernel this replaced streamed 32 KB tiles through a shared-memory ring with a block barrier per tile: about 5.5 us
+// for every product of a step, however small.)
+#include <algorithm>
+
+#include "fc_common.cuh"
+#include "pdl.cuh"
+
+namespace fc {
+
+namespace {
+
+constexpr int MAX_WARPS = 16;
+constexpr int SLICE = 2048;      // k a warp covers: 4 chunks of 16 per lane
+
+template <int B>
+__device__ __forceinline__ float qbyte(uint32_t w) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540 + B)) - 8388736.0f;
+}
+// 16 quants (biased bytes) against 16 activations held in registers (shared by the rows of a task).
+__device__ __forceinline__ float dot16x(const uint4& w, const float4& x0, const float4& x1, const float4& x2, const float4& x3) {
+    float a = x0.x * qbyte<0>(w.x), b = x1.x * qbyte<0>(w.y), c2 = x2.x * qbyte<0>(w.z), e = x3.x * qbyte<0>(w.w);
+    a = fmaf(x0.y, qbyte<1>(w.x), a); b = fmaf(x1.y, qbyte<1>(w.y), b); c2 = fmaf(x2.y, qbyte<1>(w.z), c2); e = fmaf(x3.y, qbyte<1>(w.w), e);
+    a = fmaf(x0.z, qbyte<2>(w.x), a); b = fmaf(x1.z, qbyte<2>(w.y), b); c2 = fmaf(x2.z, qbyte<2>(w.z), c2); e = fmaf(x3.z, qbyte<2>(w.w), e);
+    a = fmaf(x0.w, qbyte<3>(w.x), a); b = fmaf(x1.w, qbyte<3>(w.y), b); c2 = fmaf(x2.w, qbyte<3>(w.z), c2); e = fmaf(x3.w, qbyte<3>(w.w), e);
+    return (a + b) + (c2 + e);
+}
+// Levels are read once: they need no place in L1.
+__device__ __forceinline__ uint4 ld_levels(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+struct RowArgs {
+    GemvPart part[3];
+    int parts, staged;           // staged: copies of the row in shared memory (one per part when the parts have input scales)
+    int K, ks;                   // ks: warps that share a row
+    const float* x; const float* norm_w; float eps;
+    const float* residual; int epi;
+    const StepState* state;
+    int tasks;
+};
+
+// NCH: 16-level chunks per lane of a row (slice). RB: rows per task; SwiGLU pairs gate row t with up row t.
+template <int NCH, int RB, bool SCALED>
+__global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowArgs a) {
+    extern __shared__ __align__(16) float4 xs[];             // [staged][K / 4] units of 16 bytes, swizzled
+    __shared__ float red[MAX_WARPS];
+    __shared__ float meet[2][MAX_WARPS][RB];
+    pdl_trigger();
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, warps = blockDim.x >> 5;
+    const int K = a.K, chunks = K >> 4, units = K >> 2, kb = K >> 5;
+    const int slice = wid % a.ks, per_slice = (chunks + a.ks - 1) / a.ks;
+    const int c_end = min(chunks, (slice + 1) * per_slice), c0 = slice * per_slice + lane;
+    const int groups = gridDim.x * (warps / a.ks);
+
+    struct Rows { uint4 q[RB][NCH]; __half d[RB][NCH]; };
+    // row of part p that slot r of task t works on; the last row again where there is none
+    auto row_of = [&](int t, int r, int& p) -> int {
+        if (a.epi == EPI_SWIGLU && a.parts == 2) { p = r; return t; }
+        p = 0;
+        while (p + 1 < a.parts) {
+            const int n = (a.part[p].N + RB - 1) / RB;
+            if (t < n) break;
+            t -= n;
+            ++p;
+        }
+        return t * RB + r;
+    };
+    auto fetch = [&](Rows& w, int t) {
+        if (t >= a.tasks) return;
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            int p;
+            const int n = row_of(t, r, p);
+            const size_t row = (size_t)min(n, a.part[p].N - 1);
+            const uint4* q = (const uint4*)(a.part[p].qu + row * K);
+#pragma unroll
+            for (int i = 0; i < NCH; ++i)
+                if (c0 + 32 * i < c_end) {
+                    w.q[r][i] = ld_levels(q + c0 + 32 * i);
+                    if (SCALED) w.d[r][i] = a.part[p].d[row * kb + ((c0 + 32 * i) >> 1)];
+                }
+        }
+    };
+    Rows wa, wb;
+    const int first = blockIdx.x * (warps / a.ks) + wid / a.ks;
+    fetch(wa, first);
+
+    pdl_wait();
+    const bool dead = a.state && (a.state->done | a.state->error);
+    // stage the row (a thread keeps the units it loads), normalising and scaling it on the way
+    float ss = 0.0f;
+    for (int u = tid; u < units; u += blockDim.x) {
+        const float4 v = ((const float4*)a.x)[u];
+        ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
+        xs[u ^ ((u >> 3) & 3)] = v;
+    }
+    float inv = 1.0f;
+    if (a.norm_w) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) red[wid] = ss;
+        __syncthreads();
+        float t = 0.0f;
+        for (int i = 0; i < warps; ++i) t += red[i];
+        inv = 1.0f / sqrtf(t / (float)K + a.eps);
+    }
+    if (a.norm_w || a.part[0].xscale)
+        for (int u = tid; u < units; u += blockDim.x) {
+            const int at = u ^ ((u >> 3) & 3);
+            float4 v = xs[at];
+            if (a.norm_w) {
+                const float4 w = ((const float4*)a.norm_w)[u];
+                v.x = __fmul_rn(__fmul_rn(v.x, inv), w.x); v.y = __fmul_rn(__fmul_rn(v.y, inv), w.y);
+                v.z = __fmul_rn(__fmul_rn(v.z, inv), w.z); v.w = __fmul_rn(__fmul_rn(v.w, inv), w.w);
+            }
+            for (int p = 0; p < a.staged; ++p) {
+                float4 o = v;
+                if (a.part[p].xscale) {
+                    const float4 s = ((const float4*)a.part[p].xscale)[u];
+                    o.x *= s.x; o.y *= s.y; o.z *= s.z; o.w *= s.w;
+                }
+                xs[(size_t)p * units + at] = o;
+            }
+        }
+    __syncthreads();
+
+    int buf = 0;
+    auto work = [&](const Rows& w, int t) {
+        float acc[RB];
+        int p[RB], n[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) { acc[r] = 0.0f; n[r] = row_of(t, r, p[r]); }
+        const bool split_x = a.staged > 1 && a.epi == EPI_SWIGLU;      // the two rows of a task have a staged row each
+#pragma unroll
+        for (int i = 0; i < NCH; ++i) {
+            const int c = c0 + 32 * i;
+            if (c < c_end) {
+                const int sw = (c >> 1) & 3;
+                const float4* xp = xs + (a.staged > 1 ? (size_t)p[0] * units : 0) + 4 * c;
+                float4 x0 = xp[0 ^ sw], x1 = xp[1 ^ sw], x2 = xp[2 ^ sw], x3 = xp[3 ^ sw];
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    if (r > 0 && split_x) { xp += units; x0 = xp[0 ^ sw]; x1 = xp[1 ^ sw]; x2 = xp[2 ^ sw]; x3 = xp[3 ^ sw]; }
+                    const float v = dot16x(w.q[r][i], x0, x1, x2, x3);
+                    acc[r] = SCALED ? fmaf(__half2float(w.d[r][i]), v, acc[r]) : acc[r] + v;
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+        if (a.ks > 1) {
+            // the slices of a row meet in slice order
+            if (lane == 0)
+#pragma unroll
+                for (int r = 0; r < RB; ++r) meet[buf][wid][r] = acc[r];
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + wid / a.ks), "r"(32 * a.ks) : "memory");
+            if (slice == 0)
+#pragma unroll
+                for (int r = 0; r < RB; ++r)
+                    for (int s = 1; s < a.ks; ++s) acc[r] += meet[buf][wid + s][r];
+            buf ^= 1;
+        }
+        if (slice != 0 || lane != 0 || dead) return;
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+            if (a.part[p[r]].bias && n[r] < a.part[p[r]].N) acc[r] += a.part[p[r]].bias[n[r]];
+        if (RB == 2 && a.epi == EPI_SWIGLU) {
+            a.part[0].out[t] = __fmul_rn(__fdiv_rn(acc[0], __fadd_rn(1.0f, expf(-acc[0]))), acc[RB - 1]);
+            return;
+        }
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+            if (n[r] < a.part[p[r]].N) {
+                float v = acc[r];
+                if (a.epi == EPI_GELU) v = gelu_f(v);
+                if (a.residual) v = a.residual[n[r]] + v;
+                a.part[p[r]].out[n[r]] = v;
+            }
+    };
+    for (int t = first; t < a.tasks; t += 2 * groups) {
+        fetch(wb, t + groups);
+        work(wa, t);
+        if (t + groups < a.tasks) {
+            fetch(wa, t + 2 * groups);
+            work(wb, t + groups);
+        }
+    }
+}
+
+template <int NCH, int RB>
+int launch_row_t(const RowArgs& a, int blocks, int threads, size_t smem, bool scaled, cudaStream_t st) {
+    static bool ready[64] = {};
+    int dev = 0;
+    FC_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64) return fail(FC_E_ARG, "device index %d", dev);
+    if (!ready[dev]) {
+        FC_CUDA(cudaFuncSetAttribute(gemv_row_kernel<NCH, RB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+        FC_CUDA(cudaFuncSetAttribute(gemv_row_kernel<NCH, RB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+        ready[dev] = true;
+    }
+    if (scaled) FC_CUDA(launch_pdl(gemv_row_kernel<NCH, RB, true>, dim3(blocks), dim3(threads), smem, st, a));
+    else FC_CUDA(launch_pdl(gemv_row_kernel<NCH, RB, false>, dim3(blocks), dim3(threads), smem, st, a));
+    ++g_launches;
+    return FC_OK;
+}
+
+}  // namespace
+
+int launch_gemv_row(const GemvPart* parts, int n_parts, int K, const float* x, const float* norm_w, float eps, const float* residual,
+                    int epi, const StepState* state, cudaStream_t st) {
+    if (n_parts < 1 || n_parts > 3 || K % 32 || K > 12288) return fail(FC_E_SHAPE, "gemv_row: %d parts, K = %d", n_parts, K);
+    static int sms[64] = {};
+    int dev = 0;
+    FC_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64) return fail(FC_E_ARG, "device index %d", dev);
+    if (!sms[dev]) FC_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
+    RowArgs a = {};
+    long rows = 0;
+    for (int p = 0; p < n_parts; ++p) { a.part[p] = parts[p]; rows += parts[p].N; }
+    a.parts = n_parts; a.K = K; a.x = x; a.norm_w = norm_w; a.eps = eps; a.residual = residual; a.epi = epi; a.state = state;
+    a.staged = parts[0].xscale ? n_parts : 1;
+    if (epi == EPI_SWIGLU && (residual || n_parts > 2 || (n_parts == 1 && (parts[0].N & 1)) || (n_parts == 2 && parts[0].N != parts[1].N)))
+        return fail(FC_E_SHAPE, "the SwiGLU epilogue pairs rows and takes no residual");
+    if (residual && n_parts > 1) return fail(FC_E_SHAPE, "gemv_row: a residual belongs to a single matrix");
+    a.ks = K <= SLICE ? 1 : K <= 2 * SLICE ? 2 : K <= 4 * SLICE ? 4 : 8;
+    const int per_slice = (K / 16 + a.ks - 1) / a.ks, nch = (per_slice + 31) / 32;
+    // two rows a task when every warp of the GPU gets at least two such tasks (they share the reads of the staged row)
+    const int rb = epi == EPI_SWIGLU || rows * a.ks >= 4L * MAX_WARPS * sms[dev] ? 2 : 1;
+    a.tasks = 0;
+    for (int p = 0; p < n_parts; ++p) a.tasks += (parts[p].N + rb - 1) / rb;
+    if (epi == EPI_SWIGLU && n_parts == 2) a.tasks = parts[0].N;
+    // few tasks: few warps per CTA, on all SMs
+    int warps = (int)std::min<long>(MAX_WARPS, ((long)a.tasks * a.ks + sms[dev] - 1) / sms[dev]);
+    warps = std::max(a.ks, (std::max(warps, 4) + a.ks - 1) / a.ks * a.ks);
+    const int blocks = std::min(sms[dev], (a.tasks * a.ks + warps - 1) / warps);
+    const size_t smem = (size_t)a.staged * K * 4;
+    const bool scaled = parts[0].d != nullptr;
+#define FC_ROW(N) (rb == 2 ? launch_row_t<N, 2>(a, blocks, warps * 32, smem, scaled, st) : launch_row_t<N, 1>(a, blocks, warps * 32, smem, scaled, st))
+    return nch == 1 ? FC_ROW(1) : nch == 2 ? FC_ROW(2) : nch == 3 ? FC_ROW(3) : FC_ROW(4);
+#undef FC_ROW
+}
+
+}  // namespace fc

@@ -38,6 +38,7 @@ struct fc_llama {
     int *ids_d = nullptr, *targets_d = nullptr, *err_d = nullptr, *tc_status = nullptr;
     double* lp_d = nullptr;
     uint8_t* gr_d = nullptr;
+    Planes pany;                     // packed model: the planes of whatever product runs next
     Planes px, pqkv, patt, phid;     // bf16 planes: normalised rows, rotated q | k | v, attention output, gated hidden state
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_score_ms = 0.0f;
@@ -120,7 +121,8 @@ int model_planes(const fc_llama* m) {
 }
 
 int ensure_workspace(fc_llama* m, int rows) {
-    const int planes = std::max(m->prec >= 0 ? 0 : model_planes(m), m->ws_planes);
+    const bool packed = m->prec == FC_Q_INT8 || m->prec == FC_Q_INT4;
+    const int planes = std::max(packed ? 3 : m->prec >= 0 ? 0 : model_planes(m), m->ws_planes);
     if (rows <= m->ws_rows && planes <= m->ws_planes) return FC_OK;
     rows = std::max(rows, m->ws_rows);
     FC_CUDA(cudaStreamSynchronize(m->st));
@@ -151,10 +153,15 @@ int ensure_workspace(fc_llama* m, int rows) {
         for (int i = 0; i < planes; ++i) FC_TRY(a.alloc(&p->p[i], n * 2));
         return FC_OK;
     };
-    FC_TRY(make(&m->px, R * d));
-    FC_TRY(make(&m->pqkv, R * (size_t)m->qkv_dim));
-    FC_TRY(make(&m->patt, R * (size_t)m->q_dim));
-    FC_TRY(make(&m->phid, R * F));
+    if (packed) {
+        FC_TRY(make(&m->pany, R * std::max({d, F, (size_t)m->q_dim})));
+        m->pany.n = 3;
+    } else {
+        FC_TRY(make(&m->px, R * d));
+        FC_TRY(make(&m->pqkv, R * (size_t)m->qkv_dim));
+        FC_TRY(make(&m->patt, R * (size_t)m->q_dim));
+        FC_TRY(make(&m->phid, R * F));
+    }
     m->ws_rows = rows;
     m->ws_planes = planes;
     m->head_chunk = (int)chunk;
@@ -215,8 +222,9 @@ int forward_rows(fc_llama* m, int B, int T, fc_llama_cache* fill = nullptr) {
     return launch_llama_rmsnorm(m->x, m->out_norm, c.norm_eps, R, d, m->n, nullptr, st);
 }
 
-int lin_apply(const fc_llama::Lin& l, const float* x, const float* bias, const float* residual, float* y, int ldy, int M, cudaStream_t st) {
-    return l.rq ? launch_rowq_linear(l.rq, x, bias, residual, y, ldy, M, st) : launch_ggml_linear(l.gw, x, bias, residual, y, ldy, M, st);
+int lin_apply(fc_llama* m, const fc_llama::Lin& l, const float* x, const float* bias, const float* residual, float* y, int ldy, int M) {
+    return l.rq ? launch_rowq_linear(l.rq, x, bias, residual, y, ldy, M, m->st, M > 1 ? &m->pany : nullptr, m->tc_status)
+                : launch_ggml_linear(l.gw, x, bias, residual, y, ldy, M, m->st);
 }
 
 // FeedForward::forward (llm.rs:417-428) on separate gate and up rows: h = silu(gate) * up.
@@ -246,16 +254,16 @@ int packed_block(fc_llama* m, int l, int R, float* x, float* n, float* qkv, floa
     cudaStream_t st = m->st;
     FC_TRY(launch_llama_rmsnorm(x, L.attn_norm, c.norm_eps, R, d, n, state, st));
     const float* b = L.qkv_b;
-    FC_TRY(lin_apply(P.wq, n, b, nullptr, qkv, m->qkv_dim, R, st));
-    FC_TRY(lin_apply(P.wk, n, b ? b + m->q_dim : nullptr, nullptr, qkv + m->q_dim, m->qkv_dim, R, st));
-    FC_TRY(lin_apply(P.wv, n, b ? b + m->q_dim + m->kv_dim : nullptr, nullptr, qkv + m->q_dim + m->kv_dim, m->qkv_dim, R, st));
+    FC_TRY(lin_apply(m, P.wq, n, b, nullptr, qkv, m->qkv_dim, R));
+    FC_TRY(lin_apply(m, P.wk, n, b ? b + m->q_dim : nullptr, nullptr, qkv + m->q_dim, m->qkv_dim, R));
+    FC_TRY(lin_apply(m, P.wv, n, b ? b + m->q_dim + m->kv_dim : nullptr, nullptr, qkv + m->q_dim + m->kv_dim, m->qkv_dim, R));
     FC_TRY(attend());
-    FC_TRY(lin_apply(P.wo, att, nullptr, x, x, d, R, st));
+    FC_TRY(lin_apply(m, P.wo, att, nullptr, x, x, d, R));
     FC_TRY(launch_llama_rmsnorm(x, L.ffn_norm, c.norm_eps, R, d, n, state, st));
-    FC_TRY(lin_apply(P.gate, n, nullptr, nullptr, gu, F, R, st));
-    FC_TRY(lin_apply(P.up, n, nullptr, nullptr, gu + (size_t)R * F, F, R, st));
+    FC_TRY(lin_apply(m, P.gate, n, nullptr, nullptr, gu, F, R));
+    FC_TRY(lin_apply(m, P.up, n, nullptr, nullptr, gu + (size_t)R * F, F, R));
     FC_TRY(launch_silu_mul(gu, gu + (size_t)R * F, (size_t)R * F, hid, st));
-    return lin_apply(P.down, hid, nullptr, x, x, d, R, st);
+    return lin_apply(m, P.down, hid, nullptr, x, x, d, R);
 }
 
 int forward_rows_packed(fc_llama* m, int B, int T, fc_llama_cache* fill) {
@@ -305,7 +313,7 @@ int check_status(fc_llama* m) {
 // Logits of rows r0 .. r0 + rows of the last forward_rows into m->logits (m->head.N_pad floats apart).
 int head_rows(fc_llama* m, int r0, int rows) {
     const size_t off = (size_t)r0 * m->cfg.d_model;
-    if (m->prec >= 0) return lin_apply(m->packed_head, m->n + off, nullptr, nullptr, m->logits, m->head.N_pad, rows, m->st);
+    if (m->prec >= 0) return lin_apply(m, m->packed_head, m->n + off, nullptr, nullptr, m->logits, m->head.N_pad, rows);
     Planes x = m->px;
     for (int p = 0; p < x.n; ++p) x.p[p] = (uint16_t*)x.p[p] + off;
     return launch_gemm_q8_tc(m->head, x, nullptr, nullptr, EPI_NONE, m->logits, nullptr, rows, m->head.N_pad, m->tc_status, m->st, false);
@@ -356,15 +364,15 @@ int launch_step(fc_llama_cache* s, int with_head) {
         float* kc = s->kc + l * layer_stride;
         float* vc = s->vc + l * layer_stride;
         // RMSNorm rides in the prologue of the projection that reads it, SwiGLU in the epilogue of gate/up
-        FC_TRY(launch_gemv_q8_stream(L.qkv, s->x, L.attn_norm, c.norm_eps, L.qkv_b, nullptr, EPI_NONE, s->qkv, s->state, s->status, st));
+        FC_TRY(launch_gemv_row(L.qkv, s->x, L.attn_norm, c.norm_eps, L.qkv_b, nullptr, EPI_NONE, s->qkv, s->state, st));
         FC_TRY(launch_llama_attn_decode(s->qkv, c.n_head, c.n_kv_head, c.head_dim, c.rope_dim, c.rope_type == FC_ROPE_NEOX, m->ftab,
                                         m->inv_linear, kc, vc, c.ctx, s->state, s->att, st));
-        FC_TRY(launch_gemv_q8_stream(L.wo, s->att, nullptr, 0.0f, nullptr, s->x, EPI_NONE, s->x, s->state, s->status, st));
-        FC_TRY(launch_gemv_q8_stream(L.gateup, s->x, L.ffn_norm, c.norm_eps, nullptr, nullptr, EPI_SWIGLU, s->hid, s->state, s->status, st));
-        FC_TRY(launch_gemv_q8_stream(L.down, s->hid, nullptr, 0.0f, nullptr, s->x, EPI_NONE, s->x, s->state, s->status, st));
+        FC_TRY(launch_gemv_row(L.wo, s->att, nullptr, 0.0f, nullptr, s->x, EPI_NONE, s->x, s->state, st));
+        FC_TRY(launch_gemv_row(L.gateup, s->x, L.ffn_norm, c.norm_eps, nullptr, nullptr, EPI_SWIGLU, s->hid, s->state, st));
+        FC_TRY(launch_gemv_row(L.down, s->hid, nullptr, 0.0f, nullptr, s->x, EPI_NONE, s->x, s->state, st));
     }
     if (with_head)
-        FC_TRY(launch_gemv_q8_stream(m->head, s->x, m->out_norm, c.norm_eps, nullptr, nullptr, EPI_NONE, s->logits, s->state, s->status, st));
+        FC_TRY(launch_gemv_row(m->head, s->x, m->out_norm, c.norm_eps, nullptr, nullptr, EPI_NONE, s->logits, s->state, st));
     return launch_step_advance_pdl(s->state, st);
 }
 
@@ -380,14 +388,36 @@ int launch_step_packed(fc_llama_cache* s, int with_head) {
     for (int l = 0; l < c.n_layer; ++l) {
         float* kc = s->kc + l * layer_stride;
         float* vc = s->vc + l * layer_stride;
+        const fc_llama::PackedLayer& P = m->packed[l];
+        const LlamaLayerDev& L = m->layers[l];
+        const float* b = L.qkv_b;
+        GemvPart in[3], gu[2], wo, down;
+        if (P.wq.rq && rowq_part(P.wq.rq, b, s->qkv, &in[0]) && rowq_part(P.wk.rq, b ? b + m->q_dim : nullptr, s->qkv + m->q_dim, &in[1]) &&
+            rowq_part(P.wv.rq, b ? b + m->q_dim + m->kv_dim : nullptr, s->qkv + m->q_dim + m->kv_dim, &in[2]) &&
+            rowq_part(P.wo.rq, nullptr, s->x, &wo) && rowq_part(P.gate.rq, nullptr, s->hid, &gu[0]) &&
+            rowq_part(P.up.rq, nullptr, s->hid, &gu[1]) && rowq_part(P.down.rq, nullptr, s->x, &down)) {
+            // five kernels, as the Q8_0 step: the norms are prologues, SwiGLU and the residual epilogues
+            FC_TRY(launch_gemv_row(in, 3, c.d_model, s->x, L.attn_norm, c.norm_eps, nullptr, EPI_NONE, s->state, st));
+            FC_TRY(launch_llama_attn_decode(s->qkv, c.n_head, c.n_kv_head, c.head_dim, c.rope_dim, c.rope_type == FC_ROPE_NEOX, m->ftab,
+                                            m->inv_linear, kc, vc, c.ctx, s->state, s->att, st));
+            FC_TRY(launch_gemv_row(&wo, 1, m->q_dim, s->att, nullptr, 0.0f, s->x, EPI_NONE, s->state, st));
+            FC_TRY(launch_gemv_row(gu, 2, c.d_model, s->x, L.ffn_norm, c.norm_eps, nullptr, EPI_SWIGLU, s->state, st));
+            FC_TRY(launch_gemv_row(&down, 1, c.d_ff, s->hid, nullptr, 0.0f, s->x, EPI_NONE, s->state, st));
+            continue;
+        }
         FC_TRY(packed_block(m, l, 1, s->x, s->n, s->qkv, s->att, s->gu, s->hid, nullptr, [&]() -> int {
             return launch_llama_attn_decode(s->qkv, c.n_head, c.n_kv_head, c.head_dim, c.rope_dim, c.rope_type == FC_ROPE_NEOX, m->ftab,
                                             m->inv_linear, kc, vc, c.ctx, s->state, s->att, st);
         }));
     }
     if (with_head) {
-        FC_TRY(launch_llama_rmsnorm(s->x, m->out_norm, c.norm_eps, 1, c.d_model, s->n, nullptr, st));
-        FC_TRY(lin_apply(m->packed_head, s->n, nullptr, nullptr, s->logits, m->head.N_pad, 1, st));
+        GemvPart head;
+        if (m->packed_head.rq && rowq_part(m->packed_head.rq, nullptr, s->logits, &head)) {
+            FC_TRY(launch_gemv_row(&head, 1, c.d_model, s->x, m->out_norm, c.norm_eps, nullptr, EPI_NONE, s->state, st));
+        } else {
+            FC_TRY(launch_llama_rmsnorm(s->x, m->out_norm, c.norm_eps, 1, c.d_model, s->n, nullptr, st));
+            FC_TRY(lin_apply(m, m->packed_head, s->n, nullptr, nullptr, s->logits, m->head.N_pad, 1));
+        }
     }
     return launch_step_advance_pdl(s->state, st);
 }
@@ -467,10 +497,10 @@ int prime_window(fc_llama_cache* s, const int32_t* ids, int n) {
     FC_LAUNCHED();
     // logits of the last row: the final norm was applied by forward_rows
     if (m->prec >= 0)
-        FC_TRY(lin_apply(m->packed_head, m->n + (size_t)(n - 1) * c.d_model, nullptr, nullptr, s->logits, m->head.N_pad, 1, st));
+        FC_TRY(lin_apply(m, m->packed_head, m->n + (size_t)(n - 1) * c.d_model, nullptr, nullptr, s->logits, m->head.N_pad, 1));
     else
-        FC_TRY(launch_gemv_q8_stream(m->head, m->n + (size_t)(n - 1) * c.d_model, nullptr, 0.0f, nullptr, nullptr, EPI_NONE, s->logits,
-                                     s->state, s->status, st));
+        FC_TRY(launch_gemv_row(m->head, m->n + (size_t)(n - 1) * c.d_model, nullptr, 0.0f, nullptr, nullptr, EPI_NONE, s->logits,
+                                     s->state, st));
     FC_TRY(check_status(m));
     s->host_pos = n;
     return FC_OK;

@@ -1,16 +1,18 @@
-// Per-row-scale int8 / int4 linear: ops::qlinear (ferrum_core/src/ops.rs:268-377) on a QWeight
-// (quant.rs:122-263) kept packed on the device.
+// Per-row-scale int8 / int4 linear: ops::qlinear (ferrum_core/src/ops.rs:268-377) on a QWeight (quant.rs:122-263).
 //
 //     y[i][j] = bias[j] + sum_p (x[i][p] * scale[p]) * level[p][j]
 //
-// The matrix is [K = in][N = out] with the outputs contiguous, so a thread owns a run of 4 to 16
-// packed bytes of every row — that many columns (int8) or twice as many (int4: the low nibbles
-// are columns b.., the high nibbles half+b..) — and walks down the rows: loads are coalesced
-// across the warp, no cross-thread reduction is needed, and the K dimension is cut into slices
-// so that a single activation row still fills the GPU. Slice partials are added in slice order.
-// Up to 8 activation rows share one pass over the weights.
+// The scale belongs to the input index, so it goes into the activation and what is left is a product with whole numbers.
+// A matrix whose input width is a multiple of 32 (every Linear of a model) is therefore turned at upload into rows of int8
+// levels, outputs first, the layout of a Q8_0 matrix without its block scales (QMat): one activation row runs on
+// gemv_row.cu, more on the tensor-core GEMM with x * scale split exactly into three bf16 planes. Measured on [2048][8192],
+// one row: 26 us (int8) and 36 us (int4) before, on the kernel below.
 //
-// Bound: HBM for M <= 8. Algorithmic bytes = K * row_bytes + 4K (scales) + 4 M (K + N).
+// Other widths keep the packed [in][out] form, outputs contiguous: a thread owns a run of 4 to 16 packed bytes of every row —
+// that many columns (int8) or twice as many (int4: the low nibbles are columns b.., the high nibbles half+b..) — and walks
+// down the rows: loads are coalesced across the warp, no cross-thread reduction is needed, and the K dimension is cut into
+// slices so that a single activation row still fills the GPU. Slice partials are added in slice order. Up to 8 activation
+// rows share one pass over the weights.
 #include <algorithm>
 
 #include "fc_common.cuh"
@@ -22,6 +24,11 @@ struct fc_rowq {
     fc::Arena arena;
     uint8_t* q = nullptr;
     float* scales = nullptr;
+    fc::QMat levels;               // the matrix as rows of levels [cols][rows]; qu null: the packed form `q` is what runs
+    fc::Arena pl;                  // planes of x * scale and the status word of the tensor-core product, grown on demand
+    fc::Planes planes;
+    size_t plane_elems = 0;
+    int* status = nullptr;
     // scratch: slice partials, grown on demand. A single activation row has a buffer of its own, whose size never
     // changes once it exists: a captured decode step keeps pointing at it whatever the batched calls do to the other.
     fc::Arena ws, ws1;
@@ -57,6 +64,30 @@ template <int W> struct Words;
 template <> struct Words<1> { using T = uint32_t; };
 template <> struct Words<2> { using T = uint2; };
 template <> struct Words<4> { using T = uint4; };
+
+// Packed rows [K][ld] -> levels [N_pad][K] biased to unsigned (level + 128), 32 x 32 tiles through shared memory; rows past N
+// are zeros.
+template <int INT4>
+__global__ void __launch_bounds__(256) rowq_levels_kernel(const uint8_t* __restrict__ q, int K, int N, int ld, int half, uint8_t* __restrict__ out) {
+    __shared__ uint8_t tile[32][33];
+    const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int i = ty; i < 32; i += 8) {
+        const int n = n0 + tx;
+        int level = 0;
+        if (n < N) {
+            const uint8_t* row = q + (size_t)(k0 + i) * ld;
+            if (INT4) {
+                const int nib = n < half ? row[n] & 15 : row[n - half] >> 4;
+                level = nib >= 8 ? nib - 16 : nib;
+            } else {
+                level = (int8_t)row[n];
+            }
+        }
+        tile[i][tx] = (uint8_t)(level + 128);
+    }
+    __syncthreads();
+    for (int i = ty; i < 32; i += 8) out[(size_t)(n0 + i) * K + k0 + tx] = tile[tx][i];
+}
 
 // grid: (runs of 4 W bytes of a row, k-slices, passes of MTT rows). A thread owns 4 W packed
 // bytes of every weight row: 4 W columns (int8) or 8 W (int4). One activation row takes 16-byte
@@ -216,13 +247,35 @@ int rowq_launch(fc_rowq* w, const float* x, const float* bias, const float* resi
 
 }  // namespace
 
-// y[M][ldy] (columns 0 .. cols-1) = [residual +] bias + x · W for a packed matrix; bias and residual may be null.
-int launch_rowq_linear(fc_rowq* w, const float* x, const float* bias, const float* residual, float* y, int ldy, int M, cudaStream_t st) {
-    if (ldy < w->cols) return fail(FC_E_SHAPE, "rowq linear: row stride %d below %d columns", ldy, w->cols);
-    return rowq_launch(w, x, bias, residual, y, ldy, M, st);
+bool rowq_part(const fc_rowq* w, const float* bias, float* out, GemvPart* part) {
+    if (!w->levels.qu) return false;
+    *part = GemvPart{w->levels.qu, nullptr, w->scales, bias, out, w->cols};
+    return true;
 }
-int rowq_in(const fc_rowq* w) { return w->rows; }
-int rowq_out(const fc_rowq* w) { return w->cols; }
+
+// y[M][ldy] (columns 0 .. cols-1) = [residual +] bias + x · W for a packed matrix; bias and residual may be null.
+int launch_rowq_linear(fc_rowq* w, const float* x, const float* bias, const float* residual, float* y, int ldy, int M, cudaStream_t st,
+                       const Planes* scratch, int* status) {
+    if (ldy < w->cols) return fail(FC_E_SHAPE, "rowq linear: row stride %d below %d columns", ldy, w->cols);
+    GemvPart part;
+    if (!rowq_part(w, bias, y, &part)) return rowq_launch(w, x, bias, residual, y, ldy, M, st);
+    if (M == 1) return launch_gemv_row(&part, 1, w->rows, x, nullptr, 0.0f, residual, EPI_NONE, nullptr, st);
+    const size_t need = (size_t)M * w->rows;
+    if (!scratch && need > w->plane_elems) {
+        FC_CUDA(cudaStreamSynchronize(st));
+        w->pl.release();
+        w->plane_elems = 0;
+        w->planes = Planes();
+        for (int p = 0; p < 3; ++p) FC_TRY(w->pl.alloc(&w->planes.p[p], need * 2));
+        FC_TRY(w->pl.alloc_n(&w->status, 1));
+        FC_CUDA(cudaMemsetAsync(w->status, 0, sizeof(int), st));
+        w->planes.n = 3;
+        w->plane_elems = need;
+    }
+    const Planes& p = scratch ? *scratch : w->planes;
+    FC_TRY(launch_split_planes(x, p, need, st, w->scales, w->rows));
+    return launch_gemm_q8_tc(w->levels, p, bias, residual, EPI_NONE, y, nullptr, M, ldy, scratch ? status : w->status, st);
+}
 }  // namespace fc
 
 using namespace fc;
@@ -239,15 +292,30 @@ int fc_rowq_upload(int device, const uint8_t* q, const float* scales, int rows, 
     w->device = device; w->rows = rows; w->cols = cols; w->kind = kind;
     const size_t rb = kind == FC_Q_INT4 ? (size_t)(cols + 1) / 2 : (size_t)cols;
     w->ld = (int)((rb + 15) & ~(size_t)15);
+    Arena packed;                  // given back when the rows of levels exist
     auto build = [&]() -> int {
-        FC_TRY(w->arena.alloc_n(&w->q, (size_t)rows * w->ld));
+        FC_TRY(packed.alloc_n(&w->q, (size_t)rows * w->ld));
         FC_TRY(w->arena.alloc_n(&w->scales, (size_t)rows));
         FC_CUDA(cudaMemset(w->q, 0, (size_t)rows * w->ld));
         FC_CUDA(cudaMemcpy2D(w->q, (size_t)w->ld, q, rb, rb, (size_t)rows, cudaMemcpyHostToDevice));
         FC_CUDA(cudaMemcpy(w->scales, scales, (size_t)rows * sizeof(float), cudaMemcpyHostToDevice));
+        if (rows % 32 == 0 && rows <= 12288) {
+            const int n_pad = (cols + kRowPad - 1) / kRowPad * kRowPad, half = (cols + 1) / 2;
+            uint8_t* qu = nullptr;
+            FC_TRY(w->arena.alloc_n(&qu, (size_t)n_pad * rows));
+            const dim3 grid(n_pad / 32, rows / 32);
+            if (kind == FC_Q_INT4) rowq_levels_kernel<1><<<grid, 256>>>(w->q, rows, cols, w->ld, half, qu);
+            else rowq_levels_kernel<0><<<grid, 256>>>(w->q, rows, cols, w->ld, half, qu);
+            FC_LAUNCHED();
+            FC_CUDA(cudaDeviceSynchronize());
+            w->levels.qu = qu; w->levels.N = cols; w->levels.K = rows; w->levels.N_pad = n_pad;
+            packed.release();
+            w->q = nullptr;
+        }
         return FC_OK;
     };
     const int rc = build();
+    w->arena.ptrs.insert(w->arena.ptrs.end(), packed.ptrs.begin(), packed.ptrs.end());
     if (rc != FC_OK) { fc_rowq_free(w); return rc; }
     *out = w;
     return FC_OK;
@@ -259,6 +327,7 @@ void fc_rowq_free(fc_rowq* w) {
     cudaDeviceSynchronize();
     w->ws.release();
     w->ws1.release();
+    w->pl.release();
     w->arena.release();
     delete w;
 }
@@ -269,7 +338,7 @@ int fc_rowq_linear_dev(const fc_rowq* w, const float* x_dev, const float* bias_d
         return fail(FC_E_ARG, "fc_rowq_linear_dev: x_dev, y_dev and bias_dev must be 16-byte aligned");
     if (M <= 0) return fail(FC_E_SHAPE, "fc_rowq_linear_dev: M = %d", M);
     FC_CUDA(cudaSetDevice(w->device));
-    return rowq_launch(const_cast<fc_rowq*>(w), x_dev, bias_dev, nullptr, y_dev, w->cols, M, (cudaStream_t)stream);
+    return launch_rowq_linear(const_cast<fc_rowq*>(w), x_dev, bias_dev, nullptr, y_dev, w->cols, M, (cudaStream_t)stream);
 }
 
 int fc_rowq_linear(const fc_rowq* w, const float* x, const float* bias, float* y, int M) {
@@ -286,7 +355,7 @@ int fc_rowq_linear(const fc_rowq* w, const float* x, const float* bias, float* y
     };
     copy(xd, x, (size_t)M * w->rows * 4, cudaMemcpyHostToDevice);
     copy(bd, bias, (size_t)w->cols * 4, cudaMemcpyHostToDevice);
-    if (rc == FC_OK) rc = rowq_launch(const_cast<fc_rowq*>(w), xd, bd, nullptr, yd, w->cols, M, nullptr);
+    if (rc == FC_OK) rc = launch_rowq_linear(const_cast<fc_rowq*>(w), xd, bd, nullptr, yd, w->cols, M, nullptr);
     if (rc == FC_OK && cudaDeviceSynchronize() != cudaSuccess) rc = fail(FC_E_CUDA, "fc_rowq_linear: the kernel failed");
     copy(y, yd, (size_t)M * w->cols * 4, cudaMemcpyDeviceToHost);
     a.release();
