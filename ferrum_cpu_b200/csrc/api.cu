@@ -1376,32 +1376,48 @@ int fc_generate_sampled(fc_stream* s, const int32_t* prompt, int n, int max_new,
     int made = 0;
     bool cancelled = false, timed = false;
     int rc = FC_OK;
+    // A draw appends its token to the queue on the device (or raises `done` on eos, which turns what follows into no-ops) and
+    // the feed reads it there, so the host reads back once per kDrawBatch draws; it polls `cancel` as often. A draw that
+    // makes the window outgrow the context goes alone: its re-prime starts on the host.
+    constexpr int kDrawBatch = 16;
+    auto draw = [&]() { return launch_sample(s->probs, c.vocab, 1, *params, s->queue, 0, s->rng_d, s->queue, s->queue_cap, s->state, nullptr, st); };
+    auto issue = [&](int k, bool feed) -> int {
+        for (int i = 1; i <= k; ++i) {
+            FC_TRY(draw());
+            // the feed (or re-prime) after the last requested token keeps the stream continuable, as the reference's call
+            // order does, but its distribution is not used here: it stays outside the timed region
+            if (made + i == max_new) { FC_CUDA(cudaEventRecord(s->ev1, st)); timed = true; }
+            if (feed) FC_TRY(run_steps(s, 1, STEP_PROBS, STEP_PROBS));   // feed(next): the distribution of the token after it
+        }
+        return FC_OK;
+    };
+    // Reads back what the draws appended to the window.
+    auto harvest = [&](bool* done) -> int {
+        StepState hs;
+        FC_TRY(read_state(s, &hs));
+        if (hs.error) return fail(hs.error, "decode step rejected a token or position on the device");
+        const int have = hs.tail - (int)window.size();
+        if (have > 0) {
+            window.resize(hs.tail);
+            FC_CUDA(cudaMemcpy(window.data() + hs.tail - have, s->queue + hs.tail - have, (size_t)have * 4, cudaMemcpyDeviceToHost));
+            for (int i = 0; i < have; ++i) out[made++] = window[hs.tail - have + i];
+        }
+        *done = hs.done != 0;
+        return FC_OK;
+    };
     while (made < max_new) {
         if (cancel && *cancel) { cancelled = true; break; }
-        // draw from the current distribution with the window as `recent`; the token is appended
-        // to the queue on the device, or `done` is raised on eos
-        rc = launch_sample(s->probs, c.vocab, 1, *params, s->queue, 0, s->rng_d, s->queue, s->queue_cap, s->state, nullptr, st);
-        if (rc != FC_OK) break;
-        StepState hs;
-        rc = read_state(s, &hs);
-        if (rc != FC_OK) break;
-        if (hs.error) { rc = fail(hs.error, "decode step rejected a token or position on the device"); break; }
-        if (hs.done) break;                                   // eos: nothing was appended
-        int32_t tok = 0;
-        if (cudaMemcpy(&tok, s->queue + hs.tail - 1, 4, cudaMemcpyDeviceToHost) != cudaSuccess) { rc = fail(FC_E_CUDA, "token download failed"); break; }
-        out[made++] = tok;
-        // the feed (or re-prime) after the last requested token keeps the stream continuable, as the reference's call
-        // order does, but its distribution is not used here: it stays outside the timed region
-        if (made == max_new) { FC_CUDA(cudaEventRecord(s->ev1, st)); timed = true; }
-        window.push_back(tok);
-        if ((int)window.size() > cap) {
+        const int k = std::min(std::min(max_new - made, kDrawBatch), cap - (int)window.size());
+        bool done = false;
+        rc = issue(std::max(k, 1), k > 0);
+        if (rc == FC_OK) rc = harvest(&done);
+        if (rc != FC_OK || done) break;                       // eos: nothing was appended
+        if (k <= 0) {
             // the window outgrew the context: keep the last cap/2 ids and re-prime (token_stream.rs:162-165)
             window.erase(window.begin(), window.end() - keep);
             rc = start_window();
-        } else {
-            rc = run_steps(s, 1, STEP_PROBS, STEP_PROBS);     // feed(next): the distribution of the token after it
+            if (rc != FC_OK) break;
         }
-        if (rc != FC_OK) break;
     }
     if (rc == FC_OK) {
         if (!timed) FC_CUDA(cudaEventRecord(s->ev1, st));

@@ -11,7 +11,11 @@
 // keeps an unspecified subset of them). A draw can therefore differ from the reference only
 // when r falls within rounding of a cumulative boundary.
 //
-// Bound: latency (one row of V floats, ~70 block-wide passes out of shared memory).
+// Bound: latency of one CTA: a row of V floats in shared memory costs V / 32 cycles a pass (0.8 us at V = 50257). Finding the
+// cuts by bisection of their bit patterns takes 31 such passes each (155 us a draw at V = 50257 with top-k 40 and top-p 0.95).
+// With a top-k of at most kListK the row is therefore passed five times only: the k-th largest of the threads' maxima bounds
+// the k-th largest value from below, and the few values that reach it go to a list on which every later step works: a
+// sampled token of a 12-layer, 768-wide model (V = 50257) takes 0.33 ms instead of 0.48 ms.
 #include <climits>
 
 #include "fc_common.cuh"
@@ -19,7 +23,10 @@
 namespace fc {
 
 namespace {
-constexpr int ST = 1024;   // threads
+constexpr int ST = 1024;       // threads
+constexpr int kList = 1024;    // candidates the list holds
+// Up to half as many as there are thread maxima: above that the bound drops into the bulk of a flat row and the list overflows.
+constexpr int kListK = 512;
 
 __device__ float bsum(float v, float* red) {
 #pragma unroll
@@ -63,6 +70,64 @@ __device__ unsigned long long next_u64(unsigned long long* state) {
     *state = x;
     return x * 0x2545F4914F6CDD1DULL;
 }
+// The rest of the pipeline on the n candidates of a top-k draw: (value, index) pairs in v / at, unordered, that contain every
+// value the top-k may keep. O(n^2 / ST) reads of shared memory, broadcast. sv / si: the list in index order.
+__device__ int draw_from_list(int n, float sum, const fc_sampling& prm, float* v, int* at, float* sv, int* si, float* red,
+                              unsigned long long* rng_state) {
+    __shared__ float r_draw;
+    __shared__ int found;
+    const int tid = threadIdx.x, n4 = (n + 3) & ~3;
+    if (tid == 0) {
+        r_draw = (float)(next_u64(rng_state) >> 40) / 16777216.0f;   // rng.rs:37-40
+        found = 0x7fffffff;
+    }
+    for (int q = n + tid; q < n4; q += ST) { v[q] = -1.0f; at[q] = 0x7fffffff; sv[q] = 0.0f; si[q] = 0x7fffffff; }
+    __syncthreads();
+    // 3. top-k: a value stays when fewer than k are larger
+    float p = tid < n ? v[tid] / sum : 0.0f;
+    if (tid < n) {
+        const int mine = at[tid];
+        int rank = 0, larger = 0;
+        for (int q = 0; q < n4; q += 4) {
+            const float4 o = *(const float4*)(v + q);
+            const int4 i = *(const int4*)(at + q);
+            rank += (i.x < mine) + (i.y < mine) + (i.z < mine) + (i.w < mine);
+            // by quotient, as the filter sees them; equal numerators have equal quotients
+            larger += (o.x > v[tid] && o.x / sum > p) + (o.y > v[tid] && o.y / sum > p) + (o.z > v[tid] && o.z / sum > p) + (o.w > v[tid] && o.w / sum > p);
+        }
+        sv[rank] = larger < prm.top_k ? p : 0.0f;
+        si[rank] = mine;
+    }
+    __syncthreads();
+    p = tid < n ? sv[tid] : 0.0f;
+    // 4. top-p: the largest value down to which the mass reaches top_p
+    if (prm.top_p < 1.0f) {
+        float mass = 0.0f;
+        if (p > 0.0f)
+            for (int q = 0; q < n4; q += 4) {
+                const float4 o = *(const float4*)(sv + q);
+                mass += ((o.x >= p ? o.x : 0.0f) + (o.y >= p ? o.y : 0.0f)) + ((o.z >= p ? o.z : 0.0f) + (o.w >= p ? o.w : 0.0f));
+            }
+        const float cut = bmax(p > 0.0f && mass >= prm.top_p ? p : 0.0f, red);
+        if (p < cut) p = 0.0f;
+        if (tid < n) sv[tid] = p;
+        __syncthreads();
+    }
+    // 5. renormalise and draw: the mass in index order, as pick_by_mass adds it (sampling.rs:106-121)
+    const float sum2 = bsum(p, red);
+    p /= sum2;
+    if (tid < n) sv[tid] = p;
+    __syncthreads();
+    if (p > 0.0f) {
+        float cum = 0.0f;
+        for (int q = 0; q <= tid; ++q) cum += sv[q];
+        if (r_draw <= cum) atomicMin(&found, tid);
+    }
+    __syncthreads();
+    if (found != 0x7fffffff) return si[found];
+    // rounding left the total a hair under r: the last index that has any mass
+    return max(0, (int)bmax(p > 0.0f ? (float)si[tid] : -1.0f, red));
+}
 // total order of slm/sampling.rs:96-104 (f32::total_cmp) as a signed key
 __device__ __forceinline__ int order_key(float f) {
     const int b = __float_as_int(f);
@@ -83,21 +148,47 @@ sample_kernel(const float* __restrict__ in, int V, int from_probs, fc_sampling p
     const int tid = threadIdx.x;
     if (state && (state->done | state->error)) return;
     const int n_recent = state ? state->tail : n_recent_fixed;
+    __shared__ __align__(16) float lv[kList], lsv[kList];
+    __shared__ __align__(16) int li[kList], lsi[kList];
+    __shared__ int listed;
 
-    for (int i = tid; i < V; i += ST) w[i] = from_probs ? logf(fmaxf(in[i], 1e-12f)) : in[i];
+    const auto logit = [&](float v) { return from_probs ? logf(fmaxf(v, 1e-12f)) : v; };
+    const int V4 = ((uintptr_t)in & 15) ? 0 : V >> 2;        // a stream's buffers are aligned, a caller's pointer may not be
+#pragma unroll 4
+    for (int i = tid; i < V4; i += ST) {
+        const float4 v = ((const float4*)in)[i];
+        ((float4*)w)[i] = make_float4(logit(v.x), logit(v.y), logit(v.z), logit(v.w));
+    }
+    for (int i = 4 * V4 + tid; i < V; i += ST) w[i] = logit(in[i]);
+    if (tid == 0) listed = 0;
     __syncthreads();
     // 1. repetition penalty, once per occurrence: the thread that holds the first occurrence of
     // an id applies it as many times as the id occurs
     const float rp = prm.repetition_penalty;
     if (fabsf(rp - 1.0f) > 1.1920929e-7f && rp > 0.0f) {
+        // a window of up to kList ids is read from shared memory, four at a time
+        const bool staged = n_recent <= kList;
+        const int n4 = staged ? (n_recent + 3) & ~3 : 0;
+        if (staged) {
+            for (int q = tid; q < n4; q += ST) li[q] = q < n_recent ? recent[q] : -1;
+            __syncthreads();
+        }
         for (int j = tid; j < n_recent; j += ST) {
             const int tok = recent[j];
             if (tok < 0 || tok >= V) continue;
-            bool first = true;
-            for (int q = 0; q < j && first; ++q) first = recent[q] != tok;
-            if (!first) continue;
-            int count = 0;
-            for (int q = j; q < n_recent; ++q) count += recent[q] == tok;
+            int before = 0, count = 0;
+            for (int q = 0; q < n4; q += 4) {
+                const int4 o = *(const int4*)(li + q);
+                const int a = o.x == tok, b = o.y == tok, c = o.z == tok, e = o.w == tok;
+                before += (a & (q < j)) + (b & (q + 1 < j)) + (c & (q + 2 < j)) + (e & (q + 3 < j));
+                count += a + b + c + e;
+            }
+            for (int q = 0; !staged && q < n_recent; ++q) {
+                const int a = recent[q] == tok;
+                before += a & (q < j);
+                count += a;
+            }
+            if (before) continue;
             float l = w[tok];
             for (int c = 0; c < count; ++c) l = l > 0.0f ? l / rp : l * rp;
             w[tok] = l;
@@ -130,23 +221,45 @@ sample_kernel(const float* __restrict__ in, int V, int from_probs, fc_sampling p
         float mx = -INFINITY;
         for (int i = tid; i < V; i += ST) mx = fmaxf(mx, w[i]);
         mx = bmax(mx, red);
-        float s = 0.0f;
+        float s = 0.0f, top = 0.0f;
+#pragma unroll 4
         for (int i = tid; i < V; i += ST) {
             const float e = expf((w[i] - mx) / t);
             w[i] = e;
             s += e;
+            top = fmaxf(top, e);
         }
         const float sum = bsum(s, red);
+        const bool cut_k = prm.top_k > 0 && prm.top_k < V;
+        int n_list = kList + 1;
+        if (cut_k && prm.top_k <= kListK && sum > 1e-10f) {
+            // the k-th largest of the threads' maxima: at least k values reach it. A few units in the last place below it, so
+            // that whatever ties with it after the division by the sum is in the list too.
+            unsigned T = 0;
+            for (int bit = 30; bit >= 0; --bit)
+                if (__syncthreads_count(__float_as_uint(top) >= (T | (1u << bit))) >= prm.top_k) T |= 1u << bit;
+            T = max(T, 5u) - 4;
+            if (__float_as_uint(top) >= T)
+                for (int i = tid; i < V; i += ST)
+                    if (__float_as_uint(w[i]) >= T) {
+                        const int q = atomicAdd(&listed, 1);
+                        if (q < kList) { lv[q] = w[i]; li[q] = i; }
+                    }
+            __syncthreads();
+            n_list = listed;
+        }
         if (!(sum > 1e-10f)) {
             // degenerate mass: uniform fallback (sampling.rs:160-167)
             if (tid == 0) found = (int)(next_u64(rng_state) % (unsigned long long)V);
             __syncthreads();
             token = found;
+        } else if (n_list <= kList) {
+            token = draw_from_list(n_list, sum, prm, lv, li, lsv, lsi, red, rng_state);
         } else {
             for (int i = tid; i < V; i += ST) w[i] /= sum;
             __syncthreads();
             // 3. top-k: the k-th largest probability by bisection on its bit pattern
-            if (prm.top_k > 0 && prm.top_k < V) {
+            if (cut_k) {
                 unsigned T = 0;
                 for (int bit = 30; bit >= 0; --bit) {
                     const unsigned cand = T | (1u << bit);

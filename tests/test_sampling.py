@@ -86,6 +86,23 @@ def test_draws_follow_the_reference_distribution_on_vocabulary_sized_rows(kw):
     assert same >= 20      # most draws agree index for index
 
 
+@pytest.mark.parametrize("V,k,levels", [(5, 2, 0), (1023, 40, 0), (1025, 512, 0), (4099, 512, 0), (4099, 513, 0), (50257, 1, 0), (50257, 40, 7),
+                                        (50257, 512, 1)])
+def test_top_k_draws_at_the_edges_of_the_candidate_list(V, k, levels):
+    """Rows at and around the thread count, k at the list's limit and past it, rows of few distinct values (ties that
+    overflow the list): what is drawn carries mass, and where no tie or rounding decides it is the reference's token."""
+    logits = synth.Rng(V + k).normal(V, 2.5)
+    if levels:
+        logits = np.floor(logits / 2.5 * levels).astype(np.float32)
+    kw = dict(temperature=0.8, top_k=k, top_p=0.95, repetition_penalty=1.1)
+    recent = synth.token_ids(9, 150, V)
+    p, _ = _cdf64(logits, recent, **{**kw, "top_p": 1.0})
+    for seed in range(1, 9):
+        want, got = _pair(logits, seed, recent=recent, **kw)
+        assert p[got] > 0.0
+        assert got == want or levels or k > 40
+
+
 def test_greedy_with_penalty_matches_exactly_on_vocabulary_sized_rows():
     V = 50257
     logp = synth.Rng(6).normal(V, 2.5)
