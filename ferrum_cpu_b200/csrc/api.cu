@@ -237,11 +237,13 @@ struct fc_stream {
     int queue_cap = 0;
     StepState* state = nullptr;
     int host_pos = 0;
-    cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
-    int graph_nodes[3] = {0, 0, 0};
+    cudaGraphExec_t graph[2][3] = {};   // [one step, kChainSteps steps][mode]
+    int graph_nodes[2][3] = {};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_decode_ms = 0.0f;
     // persistent decode kernel: exchange buffers, grid barrier word, status word
+    float* qkv = nullptr;                  // decode chain: the step's q | k | v row, or null (shapes it does not cover)
+    float2* stats = nullptr;
     float *partg = nullptr, *x1g = nullptr, *statg = nullptr;
     unsigned* bar = nullptr;
     int* status = nullptr;
@@ -263,8 +265,33 @@ namespace fc {
 // ------------------------------------------------------------------------- decode step
 enum StepMode { STEP_NOHEAD = 0, STEP_SELECT = 1, STEP_PROBS = 2 };
 
-// One token through every block: the kernel sequence of CachedTransformer::feed
-// (slm/cached.rs:100-125) -> TransformerBlock::forward_with_cache (transformer.rs:221-294).
+// One token through every block as a chain of dependent launches, five a layer: CachedTransformer::feed (slm/cached.rs:100-125)
+// -> TransformerBlock::forward_with_cache (transformer.rs:221-294). LayerNorm is the prologue of the product that reads it,
+// bias, GELU and residual are epilogues, and the weights of a kernel are asked for while the one ahead of it runs. The
+// embedding starts when everything ahead of it is complete, so the attention may read state and caches early.
+static int launch_chain(fc_stream* s, int mode) {
+    fc_model* m = s->m;
+    const fc_config& c = m->cfg;
+    cudaStream_t st = m->st;
+    const int d = c.d_model, hd = d / c.n_head;
+    const size_t layer_stride = (size_t)c.ctx * d;
+    FC_TRY(launch_embed_step(m->tok, m->pos, c.ctx, s->queue, s->state, s->x, st));
+    for (int l = 0; l < c.n_layer; ++l) {
+        const LayerDev& L = m->layers[l];
+        FC_TRY(launch_gemv_row(L.qkv, s->x, RowNorm{L.ln1g, L.ln1b, 1e-5f}, L.qkv_b, nullptr, EPI_NONE, s->qkv, s->state, st));
+        FC_TRY(launch_attn_step(s->qkv, c.n_head, c.n_head, hd, 0, 0, nullptr, 1.0f, s->kc + l * layer_stride, s->vc + l * layer_stride, c.ctx,
+                                s->state, s->att, st));
+        FC_TRY(launch_gemv_row(L.out, s->att, RowNorm(), L.out_b, s->x, EPI_NONE, s->x, s->state, st));
+        FC_TRY(launch_gemv_row(L.up, s->x, RowNorm{L.ln2g, L.ln2b, 1e-5f}, L.up_b, nullptr, EPI_GELU, s->hid, s->state, st));
+        FC_TRY(launch_gemv_row(L.down, s->hid, RowNorm(), L.down_b, s->x, EPI_NONE, s->x, s->state, st));
+    }
+    if (mode == STEP_NOHEAD) return launch_step_advance_pdl(s->state, st);
+    int n_stats = 0;
+    FC_TRY(launch_gemv_row(m->head, s->x, RowNorm{m->lnfg, m->lnfb, 1e-5f}, nullptr, nullptr, EPI_NONE, s->logits, s->state, st, s->stats, &n_stats));
+    return launch_step_finish(s->logits, c.vocab, s->stats, n_stats, mode == STEP_PROBS ? s->probs : nullptr, s->queue, s->queue_cap, s->state, st);
+}
+
+// The same for the shapes the chain does not cover (heads of other widths than 32, 64 and 128, odd row lengths).
 static int launch_step(fc_stream* s, int mode) {
     fc_model* m = s->m;
     const fc_config& c = m->cfg;
@@ -298,24 +325,27 @@ static int launch_step(fc_stream* s, int mode) {
 
 // The launch-bound step is captured once per mode into a CUDA graph and replayed; every
 // per-step quantity (token, position) is read from device state, so no node is updated.
-static int run_step(fc_stream* s, int mode) {
-    if (!s->graph[mode]) {
+constexpr int kChainSteps = 8;
+static int run_step(fc_stream* s, int mode, bool several = false) {
+    cudaGraphExec_t& graph = s->graph[several][mode];
+    if (!graph) {
         cudaStream_t st = s->m->st;
         cudaGraph_t g = nullptr;
         const int64_t before = g_launches;
         FC_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        const int rc = launch_step(s, mode);
+        int rc = FC_OK;
+        for (int i = 0; i < (several ? kChainSteps : 1) && rc == FC_OK; ++i) rc = s->qkv ? launch_chain(s, mode) : launch_step(s, mode);
         const cudaError_t e = cudaStreamEndCapture(st, &g);
-        s->graph_nodes[mode] = (int)(g_launches - before);
+        s->graph_nodes[several][mode] = (int)(g_launches - before);
         g_launches = before;
         if (rc != FC_OK) { if (g) cudaGraphDestroy(g); return rc; }
         FC_CUDA(e);
-        const cudaError_t ei = cudaGraphInstantiate(&s->graph[mode], g, 0);
+        const cudaError_t ei = cudaGraphInstantiate(&graph, g, 0);
         cudaGraphDestroy(g);
         FC_CUDA(ei);
     }
-    FC_CUDA(cudaGraphLaunch(s->graph[mode], s->m->st));
-    g_launches += s->graph_nodes[mode];
+    FC_CUDA(cudaGraphLaunch(graph, s->m->st));
+    g_launches += s->graph_nodes[several][mode];
     return FC_OK;
 }
 
@@ -354,6 +384,14 @@ static int run_steps(fc_stream* s, int n, int mode, int last_mode) {
         return run_mega(s, n, head_from, last_mode == STEP_SELECT, last_mode == STEP_PROBS);
     }
     for (int i = 0; i < n; ++i) FC_TRY(run_step(s, i + 1 == n ? last_mode : mode));
+    return FC_OK;
+}
+
+// n steps of a generation. The chain of dependent launches is ahead of the persistent kernel wherever it covers the model.
+static int decode_steps(fc_stream* s, int n, int mode) {
+    if (!s->qkv) return run_steps(s, n, mode, mode);
+    for (; n >= kChainSteps; n -= kChainSteps) FC_TRY(run_step(s, mode, true));
+    for (int i = 0; i < n; ++i) FC_TRY(run_step(s, mode));
     return FC_OK;
 }
 
@@ -549,10 +587,13 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
     if (M < 0) return fail(FC_E_SHAPE, "fc_q8_0_linear_dev: M = %d", M);
     if (M == 0) return FC_OK;
     if (math_mode != FC_MATH_FP32 && math_mode != FC_MATH_BF16X3) return fail(FC_E_ARG, "unknown math_mode %d", math_mode);
-    FC_CUDA(cudaSetDevice(w->device));
+    // asking is cheaper than setting, and nearly every call finds its device current
+    int current = -1;
+    FC_CUDA(cudaGetDevice(&current));
+    if (current != w->device) FC_CUDA(cudaSetDevice(w->device));
     cudaStream_t st = (cudaStream_t)cuda_stream;
     if (M == 1) {
-        return launch_gemv_row(w->w, x_dev, nullptr, 0.0f, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, st);
+        return launch_gemv_row(w->w, x_dev, RowNorm(), bias_dev, nullptr, EPI_NONE, y_dev, nullptr, st);
     }
     // the bf16 planes of x and the status word live in the weight handle and grow on demand
     fc_qweight* wm = const_cast<fc_qweight*>(w);
@@ -1031,6 +1072,10 @@ int fc_predict_next(fc_model* m, const int32_t* ids, int n, float* probs) {
 }
 
 // ----------------------------------------------------------------------------- streams
+static bool chain_covers(const fc_config& c) {
+    return c.d_model % 32 == 0 && c.d_ff % 32 == 0 && c.d_model <= 12288 && c.d_ff <= 12288 && attn_step_covers(c.d_model / c.n_head, c.ctx);
+}
+
 int fc_stream_create(fc_model* m, fc_stream** out) {
     if (!m || !out) return fail(FC_E_ARG, "fc_stream_create: null argument");
     *out = nullptr;
@@ -1052,6 +1097,10 @@ int fc_stream_create(fc_model* m, fc_stream** out) {
     if (rc == FC_OK) rc = a.alloc_n(&s->probs, (size_t)c.vocab);
     if (rc == FC_OK) rc = a.alloc_n(&s->queue, (size_t)s->queue_cap);
     if (rc == FC_OK) rc = a.alloc_n(&s->state, 1);
+    if (rc == FC_OK && chain_covers(c)) {
+        rc = a.alloc_n(&s->stats, kRowStats);
+        if (rc == FC_OK) rc = a.alloc_n(&s->qkv, (size_t)3 * c.d_model);
+    }
     if (rc == FC_OK && m->mega_grid > 0) {
         const int hd = c.d_model / c.n_head;
         s->attn_splits = std::max(1, std::min(8, m->mega_grid / c.n_head));
@@ -1078,7 +1127,8 @@ void fc_stream_free(fc_stream* s) {
     cudaStreamSynchronize(s->m->st);
     if (s->cs) { cudaStreamSynchronize(s->cs); cudaStreamDestroy(s->cs); }
     if (s->cs_done) cudaEventDestroy(s->cs_done);
-    for (int i = 0; i < 3; ++i) if (s->graph[i]) cudaGraphExecDestroy(s->graph[i]);
+    for (auto& set : s->graph)
+        for (cudaGraphExec_t g : set) if (g) cudaGraphExecDestroy(g);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     s->arena.release();
@@ -1300,11 +1350,11 @@ int fc_generate_greedy(fc_stream* s, const int32_t* prompt, int n, int max_new, 
             // selecting feeds i..max_new-1, as many as stay inside the context
             const int k = std::min(std::min(max_new - i, 32), cap - win_start_len - gen_win + 1);
             if (k >= 1) {
-                FC_TRY(run_steps(s, k, STEP_SELECT, STEP_SELECT));
+                FC_TRY(decode_steps(s, k, STEP_SELECT));
                 gen_win += k;
                 i += k;
             } else {
-                FC_TRY(run_steps(s, 1, STEP_PROBS, STEP_PROBS));   // the last feed selects nothing
+                FC_TRY(decode_steps(s, 1, STEP_PROBS));   // the last feed selects nothing
                 i += 1;
             }
         }
@@ -1387,7 +1437,7 @@ int fc_generate_sampled(fc_stream* s, const int32_t* prompt, int n, int max_new,
             // the feed (or re-prime) after the last requested token keeps the stream continuable, as the reference's call
             // order does, but its distribution is not used here: it stays outside the timed region
             if (made + i == max_new) { FC_CUDA(cudaEventRecord(s->ev1, st)); timed = true; }
-            if (feed) FC_TRY(run_steps(s, 1, STEP_PROBS, STEP_PROBS));   // feed(next): the distribution of the token after it
+            if (feed) FC_TRY(decode_steps(s, 1, STEP_PROBS));   // feed(next): the distribution of the token after it
         }
         return FC_OK;
     };

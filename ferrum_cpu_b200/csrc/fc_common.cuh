@@ -130,8 +130,7 @@ int launch_gemv_q8_wide(const QMat& w, const float* x, const float* norm_w, floa
                         int epi, float* out, const StepState* state, cudaStream_t st);
 
 // gemv_row.cu — one activation row against up to three matrices (q | k | v, gate | up) of the same K. part.d: f16 scales per
-// 32 of k, or null with part.xscale [K]: the scale of input index k (then levels alone). Optional RMSNorm of x (norm_w, eps)
-// as it is staged; EPI_SWIGLU pairs rows (2i, 2i + 1) of one matrix, or row i of two, as (gate, up) and writes
+// 32 of k, or null with part.xscale [K]: the scale of input index k (then levels alone); EPI_SWIGLU pairs rows (2i, 2i + 1) of one matrix, or row i of two, as (gate, up) and writes
 // part[0].out[i] = silu(gate) * up. Launched as a programmatic dependent.
 struct GemvPart {
     const uint8_t* qu = nullptr;
@@ -141,13 +140,26 @@ struct GemvPart {
     float* out = nullptr;
     int N = 0;
 };
-int launch_gemv_row(const GemvPart* parts, int n_parts, int K, const float* x, const float* norm_w, float eps, const float* residual,
-                    int epi, const StepState* state, cudaStream_t st);
-inline int launch_gemv_row(const QMat& w, const float* x, const float* norm_w, float eps, const float* bias, const float* residual,
-                           int epi, float* out, const StepState* state, cudaStream_t st) {
+// What becomes of the row on its way into shared memory: nothing (w null), RMSNorm (b null) or LayerNorm.
+struct RowNorm {
+    const float *w = nullptr, *b = nullptr;
+    float eps = 0.0f;
+};
+// stats (kRowStats entries): per CTA the largest output and the sum of exp(output - largest); *n_stats: CTAs.
+constexpr int kRowStats = 1024;
+int launch_gemv_row(const GemvPart* parts, int n_parts, int K, const float* x, const RowNorm& norm, const float* residual, int epi,
+                    const StepState* state, cudaStream_t st, float2* stats = nullptr, int* n_stats = nullptr);
+inline int launch_gemv_row(const QMat& w, const float* x, const RowNorm& norm, const float* bias, const float* residual, int epi,
+                           float* out, const StepState* state, cudaStream_t st, float2* stats = nullptr, int* n_stats = nullptr) {
     const GemvPart p = {w.qu, w.d, nullptr, bias, out, w.N};
-    return launch_gemv_row(&p, 1, w.K, x, norm_w, eps, residual, epi, state, st);
+    return launch_gemv_row(&p, 1, w.K, x, norm, residual, epi, state, st, stats, n_stats);
 }
+
+// attn_step.cu — one attention step over the caches, one CTA per query head; ftab null: no rotation. The state and the cached
+// rows are read ahead of its wait: some kernel of the step before it has to wait for all of the step before.
+bool attn_step_covers(int hd, int ctx);
+int launch_attn_step(const float* qkv, int n_q, int n_kv, int hd, int rope_dim, int neox, const float2* ftab, float inv_linear,
+                     float* kc, float* vc, int ctx, const StepState* state, float* out, cudaStream_t st);
 
 // An f32 matrix as n bf16 planes whose sum it is: 2 planes hold it to 2^-17 relative (FC_MATH_BF16X3), 3 exactly
 // (FC_MATH_FP32). The form in which activations reach the tensor cores.
@@ -200,6 +212,9 @@ int launch_layernorm_planes(const float* x, const float* g, const float* b, cons
                             cudaStream_t st);
 // Decode tail over logits[V]: softmax statistics, optional probs[V], optional greedy select
 // (append to queue) — and always the end-of-step bookkeeping (pos, fed).
+// The tail behind a head product with stats: probabilities (probs set) or the greedy pick, then the step's advance.
+int launch_step_finish(const float* logits, int V, const float2* stats, int n_stats, float* probs_or_null, int* queue, int queue_cap,
+                       StepState* state, cudaStream_t st);
 int launch_step_tail(const float* logits, int V, float* probs_or_null, int do_select, int* queue, int queue_cap,
                      StepState* state, float* sel_logit_or_null, cudaStream_t st);
 // End-of-step bookkeeping alone (steps that skip the head).

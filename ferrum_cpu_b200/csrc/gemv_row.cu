@@ -1,6 +1,6 @@
 // One activation row against quantised matrices: the projections of a decode step and the M = 1 linear.
 //
-//     y[n] = (residual[n] +) bias[n] + sum_k xhat[k] * w[n][k],   xhat = x, or RMSNorm(x) (llm.rs:57-64)
+//     y[n] = (residual[n] +) bias[n] + sum_k xhat[k] * w[n][k],   xhat = x, RMSNorm(x) (llm.rs:57-64) or LayerNorm(x) (layer/norm.rs:46-82)
 //
 // Up to three matrices share the row (q | k | v, gate | up). A matrix is a QMat: int8 levels with an f16 scale per 32 of k
 // (Q8_0), or levels alone whose scale belongs to the input index (the per-row-scale QWeight of quant.rs:122-146): then
@@ -27,6 +27,7 @@ namespace fc {
 namespace {
 
 constexpr int MAX_WARPS = 16;
+constexpr int UN = 2;            // 16-byte units of the row a thread stages from registers
 constexpr int SLICE = 2048;      // k a warp covers: 4 chunks of 16 per lane
 
 template <int B>
@@ -49,21 +50,28 @@ __device__ __forceinline__ uint4 ld_levels(const uint4* p) {
     return v;
 }
 
-struct RowArgs {
+struct RowArgs {                 // small: a launch costs the host more with every few words of arguments
     GemvPart part[3];
-    int parts, staged;           // staged: copies of the row in shared memory (one per part when the parts have input scales)
-    int K, ks;                   // ks: warps that share a row
-    const float* x; const float* norm_w; float eps;
-    const float* residual; int epi;
+    const float *x, *nw, *nb, *residual;
     const StepState* state;
-    int tasks;
+    float2* stats;               // per CTA: largest output and sum of exp(output - largest), or null
+    int K, tasks;
+    float eps;
+    uint8_t parts, staged;       // staged: copies of the row in shared memory (one per part when the parts have input scales)
+    uint8_t ks, epi;             // ks: warps that share a row
 };
 
+__device__ __forceinline__ float sq4(const float4& v, float m) {
+    const float a = v.x - m, b = v.y - m, c = v.z - m, d = v.w - m;
+    return fmaf(a, a, fmaf(b, b, fmaf(c, c, d * d)));
+}
+
+// NORM: the row is normalised (and stats are taken): code that a plain product should not have to fetch.
 // NCH: 16-level chunks per lane of a row (slice). RB: rows per task; SwiGLU pairs gate row t with up row t.
-template <int NCH, int RB, bool SCALED>
+template <int NCH, int RB, bool SCALED, bool NORM>
 __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowArgs a) {
     extern __shared__ __align__(16) float4 xs[];             // [staged][K / 4] units of 16 bytes, swizzled
-    __shared__ float red[MAX_WARPS];
+    __shared__ __align__(16) float red[3][MAX_WARPS];
     __shared__ float meet[2][MAX_WARPS][RB];
     pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, warps = blockDim.x >> 5;
@@ -105,45 +113,119 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
     const int first = blockIdx.x * (warps / a.ks) + wid / a.ks;
     fetch(wa, first);
 
-    pdl_wait();
-    const bool dead = a.state && (a.state->done | a.state->error);
-    // stage the row (a thread keeps the units it loads), normalising and scaling it on the way
-    float ss = 0.0f;
-    for (int u = tid; u < units; u += blockDim.x) {
-        const float4 v = ((const float4*)a.x)[u];
-        ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
-        xs[u ^ ((u >> 3) & 3)] = v;
-    }
-    float inv = 1.0f;
-    if (a.norm_w) {
+    // the first task's bias, by the lane that adds it: behind the dot product it would cost an L2 round trip
+    const bool finisher = slice == 0 && lane == 0;
+    float bias0[RB], res0[RB];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane == 0) red[wid] = ss;
-        __syncthreads();
-        float t = 0.0f;
-        for (int i = 0; i < warps; ++i) t += red[i];
-        inv = 1.0f / sqrtf(t / (float)K + a.eps);
+    for (int r = 0; r < RB; ++r) {
+        bias0[r] = res0[r] = 0.0f;
+        if (!finisher || first >= a.tasks) continue;
+        int p;
+        const int n = row_of(first, r, p);
+        if (n < a.part[p].N && a.part[p].bias) bias0[r] = a.part[p].bias[n];
     }
-    if (a.norm_w || a.part[0].xscale)
-        for (int u = tid; u < units; u += blockDim.x) {
-            const int at = u ^ ((u >> 3) & 3);
-            float4 v = xs[at];
-            if (a.norm_w) {
-                const float4 w = ((const float4*)a.norm_w)[u];
-                v.x = __fmul_rn(__fmul_rn(v.x, inv), w.x); v.y = __fmul_rn(__fmul_rn(v.y, inv), w.y);
-                v.z = __fmul_rn(__fmul_rn(v.z, inv), w.z); v.w = __fmul_rn(__fmul_rn(v.w, inv), w.w);
-            }
-            for (int p = 0; p < a.staged; ++p) {
-                float4 o = v;
-                if (a.part[p].xscale) {
-                    const float4 s = ((const float4*)a.part[p].xscale)[u];
-                    o.x *= s.x; o.y *= s.y; o.z *= s.z; o.w *= s.w;
-                }
-                xs[(size_t)p * units + at] = o;
-            }
+    // this thread's units of the norm's parameters
+    const float *nw = NORM ? a.nw : nullptr, *nb = NORM ? a.nb : nullptr;
+    float4 gw[UN], gb[UN];
+#pragma unroll
+    for (int i = 0; i < UN; ++i) {
+        const int u = tid + i * blockDim.x;
+        if (nw && u < units) gw[i] = ((const float4*)nw)[u];
+        if (nb && u < units) gb[i] = ((const float4*)nb)[u];
+    }
+
+    pdl_wait();
+    float4 v[UN];
+#pragma unroll
+    for (int i = 0; i < UN; ++i) {
+        const int u = tid + i * blockDim.x;
+        v[i] = u < units ? ((const float4*)a.x)[u] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    if (a.residual && finisher && first < a.tasks)
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            int p;
+            const int n = row_of(first, r, p);
+            if (n < a.part[p].N) res0[r] = a.residual[n];
         }
+    const bool dead = a.state && (a.state->done | a.state->error);
+    // stage the row: a thread's first UN units stay in registers until they are normalised, further ones are read again
+    const int more = tid + UN * blockDim.x;
+    float mean = 0.0f, inv = 1.0f;
+    if (nw) {
+        auto warp_sum = [&](float t) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            return t;
+        };
+        float sum = 0.0f, m_w = 0.0f, q = 0.0f;
+        int n_w = 0;
+        if (nb) {
+            // LayerNorm: every warp takes the mean of its own elements and the squares around it; one barrier, then the warps'
+            // figures are merged around the common mean (n_w (m_w - mean)^2 is what a warp's own mean left out)
+#pragma unroll
+            for (int i = 0; i < UN; ++i) sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+            for (int u = more; u < units; u += blockDim.x) {
+                const float4 t = ((const float4*)a.x)[u];
+                sum += (t.x + t.y) + (t.z + t.w);
+            }
+            sum = warp_sum(sum);
+            for (int u = wid * 32; u < units; u += blockDim.x) n_w += 4 * min(32, units - u);
+            m_w = n_w > 0 ? sum / (float)n_w : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < UN; ++i)
+            if (tid + i * (int)blockDim.x < units) q += sq4(v[i], m_w);
+        for (int u = more; u < units; u += blockDim.x) q += sq4(((const float4*)a.x)[u], m_w);
+        q = warp_sum(q);
+        if (lane == 0) { red[0][wid] = m_w; red[1][wid] = q; red[2][wid] = (float)n_w; }
+        if (tid >= warps && tid < MAX_WARPS) red[0][tid] = red[1][tid] = red[2][tid] = 0.0f;
+        __syncthreads();
+        // every thread merges for itself: a fixed count, so that the reads are wide and the sums are trees
+        auto total = [&](auto f) {
+            float t[MAX_WARPS / 4];
+#pragma unroll
+            for (int w = 0; w < MAX_WARPS / 4; ++w) t[w] = f(((const float4*)red[0])[w], ((const float4*)red[1])[w], ((const float4*)red[2])[w]);
+            return (t[0] + t[1]) + (t[2] + t[3]);
+        };
+        if (nb) {
+            mean = total([](const float4& m, const float4&, const float4& n) { return fmaf(n.x, m.x, n.y * m.y) + fmaf(n.z, m.z, n.w * m.w); }) / (float)K;
+            auto off = [&](float m, float q, float n) { const float dm = m - mean; return fmaf(n * dm, dm, q); };
+            const float m2 = total([&](const float4& m, const float4& q, const float4& n) {
+                return (off(m.x, q.x, n.x) + off(m.y, q.y, n.y)) + (off(m.z, q.z, n.z) + off(m.w, q.w, n.w));
+            });
+            inv = sqrtf(m2 / (float)K + a.eps);            // the reference divides by the deviation
+        } else {
+            inv = 1.0f / sqrtf(total([](const float4&, const float4& q, const float4&) { return (q.x + q.y) + (q.z + q.w); }) / (float)K + a.eps);
+        }
+    }
+    auto put = [&](int u, float4 t, const float4& g, const float4& b) {
+        if (nb) {
+            t.x = ((t.x - mean) / inv) * g.x + b.x; t.y = ((t.y - mean) / inv) * g.y + b.y;
+            t.z = ((t.z - mean) / inv) * g.z + b.z; t.w = ((t.w - mean) / inv) * g.w + b.w;
+        } else if (nw) {
+            t.x = __fmul_rn(__fmul_rn(t.x, inv), g.x); t.y = __fmul_rn(__fmul_rn(t.y, inv), g.y);
+            t.z = __fmul_rn(__fmul_rn(t.z, inv), g.z); t.w = __fmul_rn(__fmul_rn(t.w, inv), g.w);
+        }
+        const int at = u ^ ((u >> 3) & 3);
+        if (!a.part[0].xscale) { xs[at] = t; return; }
+        for (int p = 0; p < a.staged; ++p) {
+            const float4 s = ((const float4*)a.part[p].xscale)[u];
+            xs[(size_t)p * units + at] = make_float4(t.x * s.x, t.y * s.y, t.z * s.z, t.w * s.w);
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < UN; ++i)
+        if (tid + i * (int)blockDim.x < units) put(tid + i * blockDim.x, v[i], gw[i], gb[i]);
+    for (int u = more; u < units; u += blockDim.x) {
+        float4 g = {}, b = {};
+        if (nw) g = ((const float4*)nw)[u];
+        if (nb) b = ((const float4*)nb)[u];
+        put(u, ((const float4*)a.x)[u], g, b);
+    }
     __syncthreads();
 
+    float top = -INFINITY, mass = 0.0f;                      // a.stats: over the outputs of this lane
     int buf = 0;
     auto work = [&](const Rows& w, int t) {
         float acc[RB];
@@ -182,10 +264,11 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
                     for (int s = 1; s < a.ks; ++s) acc[r] += meet[buf][wid + s][r];
             buf ^= 1;
         }
-        if (slice != 0 || lane != 0 || dead) return;
+        if (!finisher || dead) return;
 #pragma unroll
         for (int r = 0; r < RB; ++r)
-            if (a.part[p[r]].bias && n[r] < a.part[p[r]].N) acc[r] += a.part[p[r]].bias[n[r]];
+            if (t == first) acc[r] += bias0[r];
+            else if (a.part[p[r]].bias && n[r] < a.part[p[r]].N) acc[r] += a.part[p[r]].bias[n[r]];
         if (RB == 2 && a.epi == EPI_SWIGLU) {
             a.part[0].out[t] = __fmul_rn(__fdiv_rn(acc[0], __fadd_rn(1.0f, expf(-acc[0]))), acc[RB - 1]);
             return;
@@ -195,8 +278,12 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
             if (n[r] < a.part[p[r]].N) {
                 float v = acc[r];
                 if (a.epi == EPI_GELU) v = gelu_f(v);
-                if (a.residual) v = a.residual[n[r]] + v;
+                if (a.residual) v = (t == first ? res0[r] : a.residual[n[r]]) + v;
                 a.part[p[r]].out[n[r]] = v;
+                if (NORM && a.stats) {
+                    if (v > top) { mass *= expf(top - v); top = v; }
+                    mass += expf(v - top);
+                }
             }
     };
     for (int t = first; t < a.tasks; t += 2 * groups) {
@@ -207,29 +294,46 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
             work(wb, t + groups);
         }
     }
+    if (NORM && a.stats) {
+        __syncthreads();
+        if (lane == 0) { red[0][wid] = top; red[1][wid] = mass; }
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < warps; ++w) top = fmaxf(top, red[0][w]);
+            mass = 0.0f;
+            for (int w = 0; w < warps; ++w)
+                if (red[1][w] != 0.0f) mass += red[1][w] * expf(red[0][w] - top);
+            a.stats[blockIdx.x] = make_float2(top, mass);
+        }
+    }
 }
 
-template <int NCH, int RB>
-int launch_row_t(const RowArgs& a, int blocks, int threads, size_t smem, bool scaled, cudaStream_t st) {
+template <int NCH, int RB, bool SCALED, bool NORM>
+int launch_row_t(const RowArgs& a, int blocks, int threads, size_t smem, int dev, cudaStream_t st) {
     static bool ready[64] = {};
-    int dev = 0;
-    FC_CUDA(cudaGetDevice(&dev));
-    if (dev >= 64) return fail(FC_E_ARG, "device index %d", dev);
     if (!ready[dev]) {
-        FC_CUDA(cudaFuncSetAttribute(gemv_row_kernel<NCH, RB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-        FC_CUDA(cudaFuncSetAttribute(gemv_row_kernel<NCH, RB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+        FC_CUDA(cudaFuncSetAttribute(gemv_row_kernel<NCH, RB, SCALED, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
         ready[dev] = true;
     }
-    if (scaled) FC_CUDA(launch_pdl(gemv_row_kernel<NCH, RB, true>, dim3(blocks), dim3(threads), smem, st, a));
-    else FC_CUDA(launch_pdl(gemv_row_kernel<NCH, RB, false>, dim3(blocks), dim3(threads), smem, st, a));
+    FC_CUDA(launch_pdl(gemv_row_kernel<NCH, RB, SCALED, NORM>, dim3(blocks), dim3(threads), smem, st, a));
     ++g_launches;
     return FC_OK;
+}
+template <int NCH>
+int launch_row(int rb, bool scaled, const RowArgs& a, int blocks, int threads, size_t smem, int dev, cudaStream_t st) {
+    auto go = [&](auto f) { return f(a, blocks, threads, smem, dev, st); };
+    if (a.nw) {
+        if (scaled) return go(rb == 2 ? launch_row_t<NCH, 2, true, true> : launch_row_t<NCH, 1, true, true>);
+        return go(rb == 2 ? launch_row_t<NCH, 2, false, true> : launch_row_t<NCH, 1, false, true>);
+    }
+    if (scaled) return go(rb == 2 ? launch_row_t<NCH, 2, true, false> : launch_row_t<NCH, 1, true, false>);
+    return go(rb == 2 ? launch_row_t<NCH, 2, false, false> : launch_row_t<NCH, 1, false, false>);
 }
 
 }  // namespace
 
-int launch_gemv_row(const GemvPart* parts, int n_parts, int K, const float* x, const float* norm_w, float eps, const float* residual,
-                    int epi, const StepState* state, cudaStream_t st) {
+int launch_gemv_row(const GemvPart* parts, int n_parts, int K, const float* x, const RowNorm& norm, const float* residual, int epi,
+                    const StepState* state, cudaStream_t st, float2* stats, int* n_stats) {
     if (n_parts < 1 || n_parts > 3 || K % 32 || K > 12288) return fail(FC_E_SHAPE, "gemv_row: %d parts, K = %d", n_parts, K);
     static int sms[64] = {};
     int dev = 0;
@@ -239,10 +343,11 @@ int launch_gemv_row(const GemvPart* parts, int n_parts, int K, const float* x, c
     RowArgs a = {};
     long rows = 0;
     for (int p = 0; p < n_parts; ++p) { a.part[p] = parts[p]; rows += parts[p].N; }
-    a.parts = n_parts; a.K = K; a.x = x; a.norm_w = norm_w; a.eps = eps; a.residual = residual; a.epi = epi; a.state = state;
+    a.parts = n_parts; a.K = K; a.x = x; a.nw = norm.w; a.nb = norm.b; a.eps = norm.eps; a.stats = stats; a.residual = residual; a.epi = epi; a.state = state;
     a.staged = parts[0].xscale ? n_parts : 1;
     if (epi == EPI_SWIGLU && (residual || n_parts > 2 || (n_parts == 1 && (parts[0].N & 1)) || (n_parts == 2 && parts[0].N != parts[1].N)))
         return fail(FC_E_SHAPE, "the SwiGLU epilogue pairs rows and takes no residual");
+    if (stats && !norm.w) return fail(FC_E_ARG, "gemv_row: stats belong to a product with a norm");
     if (residual && n_parts > 1) return fail(FC_E_SHAPE, "gemv_row: a residual belongs to a single matrix");
     a.ks = K <= SLICE ? 1 : K <= 2 * SLICE ? 2 : K <= 4 * SLICE ? 4 : 8;
     const int per_slice = (K / 16 + a.ks - 1) / a.ks, nch = (per_slice + 31) / 32;
@@ -253,13 +358,13 @@ int launch_gemv_row(const GemvPart* parts, int n_parts, int K, const float* x, c
     if (epi == EPI_SWIGLU && n_parts == 2) a.tasks = parts[0].N;
     // few tasks: few warps per CTA, on all SMs
     int warps = (int)std::min<long>(MAX_WARPS, ((long)a.tasks * a.ks + sms[dev] - 1) / sms[dev]);
-    warps = std::max(a.ks, (std::max(warps, 4) + a.ks - 1) / a.ks * a.ks);
+    warps = std::max((int)a.ks, (std::max(warps, 4) + a.ks - 1) / a.ks * a.ks);
     const int blocks = std::min(sms[dev], (a.tasks * a.ks + warps - 1) / warps);
+    if (n_stats) *n_stats = blocks;
     const size_t smem = (size_t)a.staged * K * 4;
     const bool scaled = parts[0].d != nullptr;
-#define FC_ROW(N) (rb == 2 ? launch_row_t<N, 2>(a, blocks, warps * 32, smem, scaled, st) : launch_row_t<N, 1>(a, blocks, warps * 32, smem, scaled, st))
-    return nch == 1 ? FC_ROW(1) : nch == 2 ? FC_ROW(2) : nch == 3 ? FC_ROW(3) : FC_ROW(4);
-#undef FC_ROW
+    auto go = nch == 1 ? launch_row<1> : nch == 2 ? launch_row<2> : nch == 3 ? launch_row<3> : launch_row<4>;
+    return go(rb, scaled, a, blocks, warps * 32, smem, dev, st);
 }
 
 }  // namespace fc

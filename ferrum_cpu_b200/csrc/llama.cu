@@ -349,6 +349,15 @@ int check_window(const fc_llama* m, int window) {
     return FC_OK;
 }
 
+int launch_attention(fc_llama_cache* s, float* kc, float* vc) {
+    fc_llama* m = s->m;
+    const fc_llama_config& c = m->cfg;
+    auto go = attn_step_covers(c.head_dim, c.ctx) ? launch_attn_step : launch_llama_attn_decode;
+    return go(s->qkv, c.n_head, c.n_kv_head, c.head_dim, c.rope_dim, c.rope_type == FC_ROPE_NEOX, m->ftab, m->inv_linear, kc, vc, c.ctx,
+              s->state, s->att, m->st);
+}
+
+
 // ---------------------------------------------------------------------------- decode step
 // LlamaModel::forward_one (llm.rs:610-618) -> LlamaBlock::forward_one (llm.rs:451-461) as a
 // kernel sequence; every per-step quantity is read from device state so the captured graph is
@@ -364,15 +373,14 @@ int launch_step(fc_llama_cache* s, int with_head) {
         float* kc = s->kc + l * layer_stride;
         float* vc = s->vc + l * layer_stride;
         // RMSNorm rides in the prologue of the projection that reads it, SwiGLU in the epilogue of gate/up
-        FC_TRY(launch_gemv_row(L.qkv, s->x, L.attn_norm, c.norm_eps, L.qkv_b, nullptr, EPI_NONE, s->qkv, s->state, st));
-        FC_TRY(launch_llama_attn_decode(s->qkv, c.n_head, c.n_kv_head, c.head_dim, c.rope_dim, c.rope_type == FC_ROPE_NEOX, m->ftab,
-                                        m->inv_linear, kc, vc, c.ctx, s->state, s->att, st));
-        FC_TRY(launch_gemv_row(L.wo, s->att, nullptr, 0.0f, nullptr, s->x, EPI_NONE, s->x, s->state, st));
-        FC_TRY(launch_gemv_row(L.gateup, s->x, L.ffn_norm, c.norm_eps, nullptr, nullptr, EPI_SWIGLU, s->hid, s->state, st));
-        FC_TRY(launch_gemv_row(L.down, s->hid, nullptr, 0.0f, nullptr, s->x, EPI_NONE, s->x, s->state, st));
+        FC_TRY(launch_gemv_row(L.qkv, s->x, RowNorm{L.attn_norm, nullptr, c.norm_eps}, L.qkv_b, nullptr, EPI_NONE, s->qkv, s->state, st));
+        FC_TRY(launch_attention(s, kc, vc));
+        FC_TRY(launch_gemv_row(L.wo, s->att, RowNorm(), nullptr, s->x, EPI_NONE, s->x, s->state, st));
+        FC_TRY(launch_gemv_row(L.gateup, s->x, RowNorm{L.ffn_norm, nullptr, c.norm_eps}, nullptr, nullptr, EPI_SWIGLU, s->hid, s->state, st));
+        FC_TRY(launch_gemv_row(L.down, s->hid, RowNorm(), nullptr, s->x, EPI_NONE, s->x, s->state, st));
     }
     if (with_head)
-        FC_TRY(launch_gemv_row(m->head, s->x, m->out_norm, c.norm_eps, nullptr, nullptr, EPI_NONE, s->logits, s->state, st));
+        FC_TRY(launch_gemv_row(m->head, s->x, RowNorm{m->out_norm, nullptr, c.norm_eps}, nullptr, nullptr, EPI_NONE, s->logits, s->state, st));
     return launch_step_advance_pdl(s->state, st);
 }
 
@@ -397,23 +405,21 @@ int launch_step_packed(fc_llama_cache* s, int with_head) {
             rowq_part(P.wo.rq, nullptr, s->x, &wo) && rowq_part(P.gate.rq, nullptr, s->hid, &gu[0]) &&
             rowq_part(P.up.rq, nullptr, s->hid, &gu[1]) && rowq_part(P.down.rq, nullptr, s->x, &down)) {
             // five kernels, as the Q8_0 step: the norms are prologues, SwiGLU and the residual epilogues
-            FC_TRY(launch_gemv_row(in, 3, c.d_model, s->x, L.attn_norm, c.norm_eps, nullptr, EPI_NONE, s->state, st));
-            FC_TRY(launch_llama_attn_decode(s->qkv, c.n_head, c.n_kv_head, c.head_dim, c.rope_dim, c.rope_type == FC_ROPE_NEOX, m->ftab,
-                                            m->inv_linear, kc, vc, c.ctx, s->state, s->att, st));
-            FC_TRY(launch_gemv_row(&wo, 1, m->q_dim, s->att, nullptr, 0.0f, s->x, EPI_NONE, s->state, st));
-            FC_TRY(launch_gemv_row(gu, 2, c.d_model, s->x, L.ffn_norm, c.norm_eps, nullptr, EPI_SWIGLU, s->state, st));
-            FC_TRY(launch_gemv_row(&down, 1, c.d_ff, s->hid, nullptr, 0.0f, s->x, EPI_NONE, s->state, st));
+            FC_TRY(launch_gemv_row(in, 3, c.d_model, s->x, RowNorm{L.attn_norm, nullptr, c.norm_eps}, nullptr, EPI_NONE, s->state, st));
+            FC_TRY(launch_attention(s, kc, vc));
+            FC_TRY(launch_gemv_row(&wo, 1, m->q_dim, s->att, RowNorm(), s->x, EPI_NONE, s->state, st));
+            FC_TRY(launch_gemv_row(gu, 2, c.d_model, s->x, RowNorm{L.ffn_norm, nullptr, c.norm_eps}, nullptr, EPI_SWIGLU, s->state, st));
+            FC_TRY(launch_gemv_row(&down, 1, c.d_ff, s->hid, RowNorm(), s->x, EPI_NONE, s->state, st));
             continue;
         }
         FC_TRY(packed_block(m, l, 1, s->x, s->n, s->qkv, s->att, s->gu, s->hid, nullptr, [&]() -> int {
-            return launch_llama_attn_decode(s->qkv, c.n_head, c.n_kv_head, c.head_dim, c.rope_dim, c.rope_type == FC_ROPE_NEOX, m->ftab,
-                                            m->inv_linear, kc, vc, c.ctx, s->state, s->att, st);
+            return launch_attention(s, kc, vc);
         }));
     }
     if (with_head) {
         GemvPart head;
         if (m->packed_head.rq && rowq_part(m->packed_head.rq, nullptr, s->logits, &head)) {
-            FC_TRY(launch_gemv_row(&head, 1, c.d_model, s->x, m->out_norm, c.norm_eps, nullptr, EPI_NONE, s->state, st));
+            FC_TRY(launch_gemv_row(&head, 1, c.d_model, s->x, RowNorm{m->out_norm, nullptr, c.norm_eps}, nullptr, EPI_NONE, s->state, st));
         } else {
             FC_TRY(launch_llama_rmsnorm(s->x, m->out_norm, c.norm_eps, 1, c.d_model, s->n, nullptr, st));
             FC_TRY(lin_apply(m, m->packed_head, s->n, nullptr, nullptr, s->logits, m->head.N_pad, 1));
@@ -499,7 +505,7 @@ int prime_window(fc_llama_cache* s, const int32_t* ids, int n) {
     if (m->prec >= 0)
         FC_TRY(lin_apply(m, m->packed_head, m->n + (size_t)(n - 1) * c.d_model, nullptr, nullptr, s->logits, m->head.N_pad, 1));
     else
-        FC_TRY(launch_gemv_row(m->head, m->n + (size_t)(n - 1) * c.d_model, nullptr, 0.0f, nullptr, nullptr, EPI_NONE, s->logits,
+        FC_TRY(launch_gemv_row(m->head, m->n + (size_t)(n - 1) * c.d_model, RowNorm(), nullptr, nullptr, EPI_NONE, s->logits,
                                      s->state, st));
     FC_TRY(check_status(m));
     s->host_pos = n;

@@ -69,8 +69,8 @@ int launch_llama_embed_rows(const QMat& tok, const int* ids, int R, float* x, in
 // forward_one (llm.rs:610-618): the queued token at the cache position. A full context is
 // refused like a bad id (generation stops at the window, llm.rs:720-730).
 __global__ void llama_embed_step_kernel(QMat tok, int ctx, const int* __restrict__ queue, StepState* st, float* __restrict__ x) {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();       // only now: the attention reads state and caches ahead of its own wait
     if (st->done | st->error) return;
     const int pos = st->pos, id = queue[st->fed];
     if (id < 0 || id >= tok.N || pos >= ctx) {
@@ -136,9 +136,6 @@ __device__ __forceinline__ void rotate_pair(float* x, int ia, int ib, float thet
     const float a = x[ia], b = x[ib];
     x[ia] = __fsub_rn(__fmul_rn(a, c), __fmul_rn(b, s));
     x[ib] = __fadd_rn(__fmul_rn(a, s), __fmul_rn(b, c));
-}
-__device__ __forceinline__ float rope_angle(int pos, float2 f, float inv_linear) {
-    return __fmul_rn(__fdiv_rn(__fmul_rn((float)pos, f.x), f.y), inv_linear);
 }
 
 // Window form: row r of the fused [R][ld] buffer sits at position r % T; its first n_q heads

@@ -4,6 +4,11 @@
 
 namespace fc {
 
+// Angle of a rotary pair at a position; the table holds (numerator, denominator) of its frequency.
+__device__ __forceinline__ float rope_angle(int pos, float2 f, float inv_linear) {
+    return __fmul_rn(__fdiv_rn(__fmul_rn((float)pos, f.x), f.y), inv_linear);
+}
+
 int launch_llama_embed_rows(const QMat& tok, const int* ids, int R, float* x, int* error_flag, cudaStream_t st);
 // Rotation of window rows with the result written as bf16 hi / lo planes [R][ld] (the f32 rows stay as they were).
 int launch_llama_rope_planes(const float* qkv, int R, int ld, int T, int n_q, int n_kv, int k_off, int hd, int rope_dim, int neox,

@@ -60,6 +60,8 @@ __device__ __forceinline__ float tok_value(const QMat& tok, int id, int c) {
 
 __global__ void embed_step_kernel(QMat tok, const float* __restrict__ pos_emb, int ctx,
                                   const int* __restrict__ queue, StepState* st, float* __restrict__ x) {
+    pdl_wait();
+    pdl_trigger();       // only now: the chain's attention reads state and caches ahead of its own wait
     if (st->done | st->error) return;
     const int pos = st->pos, id = queue[st->fed];
     // embedding.rs:71-82 and transformer.rs:237-242: bad id / full cache are errors, not traps
@@ -73,8 +75,8 @@ __global__ void embed_step_kernel(QMat tok, const float* __restrict__ pos_emb, i
 
 int launch_embed_step(const QMat& tok, const float* pos_emb, int ctx, const int* queue, StepState* state,
                       float* x, cudaStream_t st) {
-    embed_step_kernel<<<1, 256, 0, st>>>(tok, pos_emb, ctx, queue, state, x);
-    FC_LAUNCHED();
+    FC_CUDA(launch_pdl(embed_step_kernel, dim3(1), dim3(256), 0, st, tok, pos_emb, ctx, queue, state, x));
+    ++g_launches;
     return FC_OK;
 }
 
@@ -306,6 +308,96 @@ int launch_step_tail(const float* logits, int V, float* probs_or_null, int do_se
                      StepState* state, float* sel_logit_or_null, cudaStream_t st) {
     step_tail_kernel<<<1, 1024, 0, st>>>(logits, V, probs_or_null, do_select, queue, queue_cap, state, sel_logit_or_null);
     FC_LAUNCHED();
+    return FC_OK;
+}
+
+// The tail of a step whose head product left, per CTA, its largest logit and the mass around it: the softmax needs no pass of
+// its own. M and S of the whole row, by every warp for itself.
+__device__ __forceinline__ float2 row_stats(const float2* __restrict__ stats, int n) {
+    const int lane = threadIdx.x & 31;
+    float top = -INFINITY, mass = 0.0f;
+    for (int i = lane; i < n; i += 32) {
+        const float2 s = stats[i];
+        if (s.x > top) { mass *= expf(top - s.x); top = s.x; }
+        if (s.y != 0.0f) mass += s.y * expf(s.x - top);
+    }
+    float all = top;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) all = fmaxf(all, __shfl_xor_sync(0xffffffffu, all, o));
+    mass = mass != 0.0f ? mass * expf(top - all) : 0.0f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
+    return make_float2(all, mass);
+}
+// Greedy pick: first index of the largest ln(max(p, 1e-12)). Rounding can make neighbours of the largest logit tie with it, but
+// nothing 0.01 below it (p there is at least 1 % smaller, and the largest p is at least 1 / V), so only those are evaluated.
+__global__ void __launch_bounds__(1024) step_pick_kernel(const float* __restrict__ logits, int V, const float2* __restrict__ stats, int n_stats,
+                                                         int* __restrict__ queue, int queue_cap, StepState* st) {
+    __shared__ ArgPair pred[32];
+    pdl_trigger();
+    pdl_wait();
+    if (st->done | st->error) return;
+    const float2 ms = row_stats(stats, n_stats);
+    ArgPair best{-INFINITY, 0x7fffffff};
+    auto look = [&](float l, int i) {
+        if (l >= ms.x - 0.01f) best = better(best, ArgPair{logf(fmaxf(expf(l - ms.x) / ms.y, 1e-12f)), i});
+    };
+    const int V4 = V >> 2;
+    for (int i0 = threadIdx.x; i0 < V4; i0 += 7 * blockDim.x) {
+        float4 l[7];                     // 28 K logits on their way at a time
+#pragma unroll
+        for (int k = 0; k < 7; ++k) {
+            const int i = i0 + k * blockDim.x;
+            l[k] = i < V4 ? ((const float4*)logits)[i] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        }
+#pragma unroll
+        for (int k = 0; k < 7; ++k) {
+            const int i = 4 * (i0 + k * blockDim.x);
+            if (fmaxf(fmaxf(l[k].x, l[k].y), fmaxf(l[k].z, l[k].w)) < ms.x - 0.01f) continue;
+            look(l[k].x, i); look(l[k].y, i + 1); look(l[k].z, i + 2); look(l[k].w, i + 3);
+        }
+    }
+    if ((int)threadIdx.x < (V & 3)) look(logits[4 * V4 + threadIdx.x], 4 * V4 + threadIdx.x);
+    auto warp_best = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            best = better(best, ArgPair{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
+    };
+    warp_best();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0) pred[wid] = best;
+    __syncthreads();
+    if (wid != 0) return;
+    best = pred[lane];
+    warp_best();
+    if (lane != 0) return;
+    if (best.i == st->eos) {
+        st->done = 1;
+    } else if (st->tail < queue_cap) {
+        queue[st->tail] = best.i;
+        st->tail += 1;
+    } else {
+        st->error = FC_E_DIM;
+    }
+    st->pos += 1;
+    st->fed += 1;
+}
+__global__ void __launch_bounds__(256) step_probs_kernel(const float* __restrict__ logits, int V, const float2* __restrict__ stats, int n_stats,
+                                                         float* __restrict__ probs, StepState* st) {
+    pdl_trigger();
+    pdl_wait();
+    if (st->done | st->error) return;
+    const float2 ms = row_stats(stats, n_stats);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x) probs[i] = expf(logits[i] - ms.x) / ms.y;
+    if (blockIdx.x == 0 && threadIdx.x == 0) { st->pos += 1; st->fed += 1; }
+}
+int launch_step_finish(const float* logits, int V, const float2* stats, int n_stats, float* probs_or_null, int* queue, int queue_cap,
+                       StepState* state, cudaStream_t st) {
+    if (probs_or_null)
+        FC_CUDA(launch_pdl(step_probs_kernel, dim3(std::min(148, (V + 255) / 256)), dim3(256), 0, st, logits, V, stats, n_stats, probs_or_null, state));
+    else
+        FC_CUDA(launch_pdl(step_pick_kernel, dim3(1), dim3(1024), 0, st, logits, V, stats, n_stats, queue, queue_cap, state));
+    ++g_launches;
     return FC_OK;
 }
 

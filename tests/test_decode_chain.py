@@ -1,0 +1,44 @@
+"""The chain of dependent launches that decodes one token (gemv_row.cu, attn_step.cu, the pick), against the oracle."""
+import numpy as np
+import pytest
+
+import ferrum_cpu_b200 as fcb
+from ferrum_cpu_b200 import synth
+from ferrum_cpu_b200.llama import CudaLlama
+from tests import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("d,heads,ff,ctx,prompt,new", [(32, 1, 64, 16, 1, 14), (96, 3, 160, 64, 60, 9), (64, 1, 96, 512, 345, 20),
+                                                      (256, 4, 4128, 40, 17, 20)])
+def test_decode_chain_at_its_edges(d, heads, ff, ctx, prompt, new):
+    """Greedy tokens of the decode chain against the oracle: heads of 32 and 64, the first positions, caches that outgrow
+    the rows the attention holds in shared memory, a window that slides, rows wider than one slice and odd vocabularies."""
+    sm = synth.SynthModel(2, d, heads, ff, ctx, 515, seed=d + ff, perturb=True)
+    om, gm = O.OracleModel(sm), fcb.CudaSlm(sm.config, sm.weights)
+    window, want = list(synth.token_ids(4, prompt, 515)), []
+    dist = om.prime(window)
+    for _ in range(new):
+        want.append(int(np.argmax(dist)))
+        window.append(want[-1])
+        if len(window) > ctx:
+            window = window[-(ctx // 2):]
+            dist = om.prime(window)
+        else:
+            dist = om.feed(want[-1])
+    got, _ = gm.generate_tokens(synth.token_ids(4, prompt, 515), new)
+    assert list(got) == want
+    gm.close()
+    om.close()
+
+
+@pytest.mark.parametrize("hd,heads,kv,rope_dim,rope_type", [(128, 2, 1, 128, 0), (128, 2, 2, 96, 1), (32, 3, 1, 30, 0), (64, 8, 2, 64, 1)])
+def test_rotary_steps_match_the_oracle_past_the_held_rows(hd, heads, kv, rope_dim, rope_type):
+    sm = synth.SynthLlama(515, 96, 2, heads, kv, hd, 160, 416, seed=hd + kv, perturb=True, rope_dim=rope_dim, rope_type=rope_type)
+    om, gm = O.OracleLlama(sm, threads=4), CudaLlama.from_synth(sm)
+    cache = gm.new_cache()
+    om.clear()
+    for t, tok in enumerate(synth.token_ids(2, 400, 515)):
+        got, want = gm.forward_one(tok, cache), om.forward_one(tok)
+        assert np.abs(got - want).max() < 2e-4, t
