@@ -572,29 +572,45 @@ __global__ void __launch_bounds__(1024) pick_batch_kernel(const float* __restric
     const float* row = logits + (size_t)s * ldl;
     const float4* row4 = (const float4*)row;           // ldl % 4 == 0: rows start on 16-byte boundaries
     const int V4 = V >> 2;
-    float mx = -INFINITY;
-    for (int i = threadIdx.x; i < V4; i += blockDim.x) {
-        const float4 v = row4[i];
-        mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
-    }
-    for (int i = 4 * V4 + threadIdx.x; i < V; i += blockDim.x) mx = fmaxf(mx, row[i]);
-    mx = block_max(mx, red);
-    float e = 0.0f;
-    for (int i = threadIdx.x; i < V4; i += blockDim.x) {
-        const float4 v = row4[i];
-        e += (expf(v.x - mx) + expf(v.y - mx)) + (expf(v.z - mx) + expf(v.w - mx));
-    }
-    for (int i = 4 * V4 + threadIdx.x; i < V; i += blockDim.x) e += expf(row[i] - mx);
-    const float sum = block_sum(e, red);
+    // 28 K logits on their way at a time: with one load after the other the passes over a row were a chain of L2 round trips
+    auto sweep = [&](auto f) {
+        for (int i0 = threadIdx.x; i0 < V4; i0 += 7 * blockDim.x) {
+            float4 l[7];
+#pragma unroll
+            for (int k = 0; k < 7; ++k) {
+                const int i = i0 + k * blockDim.x;
+                l[k] = i < V4 ? row4[i] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+            }
+#pragma unroll
+            for (int k = 0; k < 7; ++k) f(l[k], 4 * (i0 + k * blockDim.x));
+        }
+    };
+    const int rest = 4 * V4 + threadIdx.x;
+    const float lrest = rest < V ? row[rest] : -INFINITY;
+    // largest logit and sum of exponentials in one pass: the sum follows a thread's running maximum
+    float top = -INFINITY, e = 0.0f;
+    sweep([&](const float4& v, int) {
+        const float m = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
+        if (m > top) { e *= expf(top - m); top = m; }
+        if (top > -INFINITY) e += (expf(v.x - top) + expf(v.y - top)) + (expf(v.z - top) + expf(v.w - top));
+    });
+    if (lrest > top) { e *= expf(top - lrest); top = lrest; }
+    if (lrest > -INFINITY) e += expf(lrest - top);
+    const float mx = block_max(top, red);
+    const float sum = block_sum(e > 0.0f ? e * expf(top - mx) : 0.0f, red);
     // Only a logit within rounding distance of the largest one can tie its probability after the
     // f32 exp and division; everything more than 0.01 below it has a strictly smaller probability
     // (the largest probability is at least 1 / V, far above the 1e-12 floor), so the full formula
     // is evaluated for those candidates only.
     ArgPair best{-INFINITY, 0x7fffffff};
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        const float l = row[i];
-        if (l >= mx - 0.01f) best = better(best, ArgPair{logf(fmaxf(expf(l - mx) / sum, 1e-12f)), i});
-    }
+    auto look = [&](float l, int i) {
+        if (l >= mx - 0.01f && i < V) best = better(best, ArgPair{logf(fmaxf(expf(l - mx) / sum, 1e-12f)), i});
+    };
+    sweep([&](const float4& v, int i) {
+        if (!(fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)) >= mx - 0.01f)) return;
+        look(v.x, i); look(v.y, i + 1); look(v.z, i + 2); look(v.w, i + 3);
+    });
+    look(lrest, rest);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) best = better(best, ArgPair{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
