@@ -202,7 +202,7 @@ struct fc_model {
     std::vector<LayerDev> layers;
     // prefill workspace for ws_rows rows
     int ws_rows = 0, ws_planes = 0;
-    float *x = nullptr, *n = nullptr, *qkv = nullptr, *att = nullptr, *logits = nullptr, *probs_d = nullptr;
+    float *x = nullptr, *qkv = nullptr, *att = nullptr, *logits = nullptr, *probs_d = nullptr;
     int *ids_d = nullptr, *err_d = nullptr;
     ScoreSlot slot[2];
     Planes pn, pqkv, patt, phid;               // bf16 planes of LayerNorm output, qkv, attention output, GELU output
@@ -232,7 +232,7 @@ struct fc_stream {
     fc_model* m;
     Arena arena;
     float *kc = nullptr, *vc = nullptr;  // [L][ctx][d]
-    float *x = nullptr, *n = nullptr, *q = nullptr, *att = nullptr, *hid = nullptr, *logits = nullptr, *probs = nullptr;
+    float *x = nullptr, *q = nullptr, *att = nullptr, *hid = nullptr, *logits = nullptr, *probs = nullptr;
     int* queue = nullptr;
     int queue_cap = 0;
     StepState* state = nullptr;
@@ -242,8 +242,8 @@ struct fc_stream {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_decode_ms = 0.0f;
     // persistent decode kernel: exchange buffers, grid barrier word, status word
-    float* qkv = nullptr;                  // decode chain: the step's q | k | v row, or null (shapes it does not cover)
-    float2* stats = nullptr;
+    float* qkv = nullptr;                  // the step's q | k | v row
+    float2* stats = nullptr;               // softmax statistics of its logits
     float *partg = nullptr, *x1g = nullptr, *statg = nullptr;
     unsigned* bar = nullptr;
     int* status = nullptr;
@@ -265,11 +265,20 @@ namespace fc {
 // ------------------------------------------------------------------------- decode step
 enum StepMode { STEP_NOHEAD = 0, STEP_SELECT = 1, STEP_PROBS = 2 };
 
+// Final LayerNorm, head and the selection of a step, on one row.
+static int launch_head(fc_stream* s, const float* x, int mode) {
+    fc_model* m = s->m;
+    int n_stats = 0;
+    FC_TRY(launch_gemv_row(m->head, x, RowNorm{m->lnfg, m->lnfb, 1e-5f}, nullptr, nullptr, EPI_NONE, s->logits, s->state, m->st, s->stats, &n_stats));
+    return launch_step_finish(s->logits, m->cfg.vocab, s->stats, n_stats, mode == STEP_PROBS ? s->probs : nullptr, s->queue, s->queue_cap, s->state,
+                              m->st);
+}
+
 // One token through every block as a chain of dependent launches, five a layer: CachedTransformer::feed (slm/cached.rs:100-125)
 // -> TransformerBlock::forward_with_cache (transformer.rs:221-294). LayerNorm is the prologue of the product that reads it,
 // bias, GELU and residual are epilogues, and the weights of a kernel are asked for while the one ahead of it runs. The
 // embedding starts when everything ahead of it is complete, so the attention may read state and caches early.
-static int launch_chain(fc_stream* s, int mode) {
+static int launch_step(fc_stream* s, int mode) {
     fc_model* m = s->m;
     const fc_config& c = m->cfg;
     cudaStream_t st = m->st;
@@ -286,41 +295,7 @@ static int launch_chain(fc_stream* s, int mode) {
         FC_TRY(launch_gemv_row(L.down, s->hid, RowNorm(), L.down_b, s->x, EPI_NONE, s->x, s->state, st));
     }
     if (mode == STEP_NOHEAD) return launch_step_advance_pdl(s->state, st);
-    int n_stats = 0;
-    FC_TRY(launch_gemv_row(m->head, s->x, RowNorm{m->lnfg, m->lnfb, 1e-5f}, nullptr, nullptr, EPI_NONE, s->logits, s->state, st, s->stats, &n_stats));
-    return launch_step_finish(s->logits, c.vocab, s->stats, n_stats, mode == STEP_PROBS ? s->probs : nullptr, s->queue, s->queue_cap, s->state, st);
-}
-
-// The same for the shapes the chain does not cover (heads of other widths than 32, 64 and 128, odd row lengths).
-static int launch_step(fc_stream* s, int mode) {
-    fc_model* m = s->m;
-    const fc_config& c = m->cfg;
-    cudaStream_t st = m->st;
-    const int d = c.d_model;
-    const size_t layer_stride = (size_t)c.ctx * d;
-    FC_TRY(launch_embed_step(m->tok, m->pos, c.ctx, s->queue, s->state, s->x, st));
-    for (int l = 0; l < c.n_layer; ++l) {
-        const LayerDev& L = m->layers[l];
-        float* kc = s->kc + l * layer_stride;
-        float* vc = s->vc + l * layer_stride;
-        FC_TRY(launch_layernorm(s->x, L.ln1g, L.ln1b, 1, d, s->n, s->state, st));
-        GemvOut o;
-        o.out[0] = s->q; o.out[1] = kc; o.out[2] = vc; o.seg = d; o.pos_stride = d;
-        FC_TRY(launch_gemv_q8(L.qkv, s->n, L.qkv_b, nullptr, EPI_NONE, o, s->state, st));
-        FC_TRY(launch_attn_decode(s->q, kc, vc, d, c.n_head, c.ctx, s->state, s->att, st));
-        GemvOut ox; ox.out[0] = s->x;
-        FC_TRY(launch_gemv_q8(L.out, s->att, L.out_b, s->x, EPI_NONE, ox, s->state, st));
-        FC_TRY(launch_layernorm(s->x, L.ln2g, L.ln2b, 1, d, s->n, s->state, st));
-        GemvOut oh; oh.out[0] = s->hid;
-        FC_TRY(launch_gemv_q8(L.up, s->n, L.up_b, nullptr, EPI_GELU, oh, s->state, st));
-        FC_TRY(launch_gemv_q8(L.down, s->hid, L.down_b, s->x, EPI_NONE, ox, s->state, st));
-    }
-    if (mode == STEP_NOHEAD) return launch_step_advance(s->state, st);
-    FC_TRY(launch_layernorm(s->x, m->lnfg, m->lnfb, 1, d, s->n, s->state, st));
-    GemvOut ol; ol.out[0] = s->logits;
-    FC_TRY(launch_gemv_q8(m->head, s->n, nullptr, nullptr, EPI_NONE, ol, s->state, st));
-    return launch_step_tail(s->logits, c.vocab, mode == STEP_PROBS ? s->probs : nullptr, mode == STEP_SELECT ? 1 : 0,
-                            s->queue, s->queue_cap, s->state, nullptr, st);
+    return launch_head(s, s->x, mode);
 }
 
 // The launch-bound step is captured once per mode into a CUDA graph and replayed; every
@@ -334,7 +309,7 @@ static int run_step(fc_stream* s, int mode, bool several = false) {
         const int64_t before = g_launches;
         FC_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         int rc = FC_OK;
-        for (int i = 0; i < (several ? kChainSteps : 1) && rc == FC_OK; ++i) rc = s->qkv ? launch_chain(s, mode) : launch_step(s, mode);
+        for (int i = 0; i < (several ? kChainSteps : 1) && rc == FC_OK; ++i) rc = launch_step(s, mode);
         const cudaError_t e = cudaStreamEndCapture(st, &g);
         s->graph_nodes[several][mode] = (int)(g_launches - before);
         g_launches = before;
@@ -389,7 +364,8 @@ static int run_steps(fc_stream* s, int n, int mode, int last_mode) {
 
 // n steps of a generation. The chain of dependent launches is ahead of the persistent kernel wherever it covers the model.
 static int decode_steps(fc_stream* s, int n, int mode) {
-    if (!s->qkv) return run_steps(s, n, mode, mode);
+    const fc_config& c = s->m->cfg;
+    if (!attn_step_covers(c.d_model / c.n_head, c.ctx)) return run_steps(s, n, mode, mode);
     for (; n >= kChainSteps; n -= kChainSteps) FC_TRY(run_step(s, mode, true));
     for (int i = 0; i < n; ++i) FC_TRY(run_step(s, mode));
     return FC_OK;
@@ -445,8 +421,7 @@ static int ensure_workspace(fc_model* m, int rows, int planes) {
     const size_t R = rows, d = c.d_model, F = c.d_ff;
     Arena& a = m->ws_arena;
     FC_TRY(a.alloc_n(&m->x, R * d));
-    FC_TRY(a.alloc_n(&m->n, d));                            // predict_next: the last row through the final LayerNorm,
-    FC_TRY(a.alloc_n(&m->logits, (size_t)m->head.N_pad));   // and its logits
+    FC_TRY(a.alloc_n(&m->logits, (size_t)m->head.N_pad));   // predict_next
     FC_TRY(a.alloc_n(&m->qkv, R * 3 * d));
     FC_TRY(a.alloc_n(&m->att, R * d));
     FC_TRY(a.alloc_n(&m->ids_d, R));
@@ -1062,20 +1037,14 @@ int fc_predict_next(fc_model* m, const int32_t* ids, int n, float* probs) {
     Windows win;
     win.B = 1; win.T = n;
     FC_TRY(forward_blocks_with(m, win, n, m->ids_d, nullptr, model_planes(m), m->tc_status, false, false, [](int) { return FC_OK; }));
-    FC_TRY(launch_layernorm(m->x + (size_t)(n - 1) * c.d_model, m->lnfg, m->lnfb, 1, c.d_model,
-                            m->n, nullptr, st));
-    GemvOut o; o.out[0] = m->logits;
-    FC_TRY(launch_gemv_q8(m->head, m->n, nullptr, nullptr, EPI_NONE, o, nullptr, st));
+    FC_TRY(launch_gemv_row(m->head, m->x + (size_t)(n - 1) * c.d_model, RowNorm{m->lnfg, m->lnfb, 1e-5f}, nullptr, nullptr, EPI_NONE, m->logits,
+                           nullptr, st));
     FC_TRY(launch_softmax_row(m->logits, c.vocab, m->probs_d, st));
     FC_CUDA(cudaMemcpyAsync(probs, m->probs_d, (size_t)c.vocab * 4, cudaMemcpyDeviceToHost, st));
     return check_tc_status(m, "predict_next");
 }
 
 // ----------------------------------------------------------------------------- streams
-static bool chain_covers(const fc_config& c) {
-    return c.d_model % 32 == 0 && c.d_ff % 32 == 0 && c.d_model <= 12288 && c.d_ff <= 12288 && attn_step_covers(c.d_model / c.n_head, c.ctx);
-}
-
 int fc_stream_create(fc_model* m, fc_stream** out) {
     if (!m || !out) return fail(FC_E_ARG, "fc_stream_create: null argument");
     *out = nullptr;
@@ -1089,7 +1058,6 @@ int fc_stream_create(fc_model* m, fc_stream** out) {
     int rc = a.alloc_n(&s->kc, cache);
     if (rc == FC_OK) rc = a.alloc_n(&s->vc, cache);
     if (rc == FC_OK) rc = a.alloc_n(&s->x, (size_t)c.d_model);
-    if (rc == FC_OK) rc = a.alloc_n(&s->n, (size_t)c.d_model);
     if (rc == FC_OK) rc = a.alloc_n(&s->q, (size_t)c.d_model);
     if (rc == FC_OK) rc = a.alloc_n(&s->att, (size_t)c.d_model);
     if (rc == FC_OK) rc = a.alloc_n(&s->hid, (size_t)c.d_ff);
@@ -1097,10 +1065,8 @@ int fc_stream_create(fc_model* m, fc_stream** out) {
     if (rc == FC_OK) rc = a.alloc_n(&s->probs, (size_t)c.vocab);
     if (rc == FC_OK) rc = a.alloc_n(&s->queue, (size_t)s->queue_cap);
     if (rc == FC_OK) rc = a.alloc_n(&s->state, 1);
-    if (rc == FC_OK && chain_covers(c)) {
-        rc = a.alloc_n(&s->stats, kRowStats);
-        if (rc == FC_OK) rc = a.alloc_n(&s->qkv, (size_t)3 * c.d_model);
-    }
+    if (rc == FC_OK) rc = a.alloc_n(&s->stats, kRowStats);
+    if (rc == FC_OK) rc = a.alloc_n(&s->qkv, (size_t)3 * c.d_model);
     if (rc == FC_OK && m->mega_grid > 0) {
         const int hd = c.d_model / c.n_head;
         s->attn_splits = std::max(1, std::min(8, m->mega_grid / c.n_head));
@@ -1234,11 +1200,7 @@ static int prime_batched(fc_stream* const* ss, int S, int n, int last_mode, int*
         // the head sees the last row only; its tail advances the position by one
         bump_state_kernel<<<1, 1, 0, st>>>(s->state, n - 1);
         FC_LAUNCHED();
-        FC_TRY(launch_layernorm(m->x + ((size_t)i * n + n - 1) * d, m->lnfg, m->lnfb, 1, d, s->n, s->state, st));
-        GemvOut ol; ol.out[0] = s->logits;
-        FC_TRY(launch_gemv_q8(m->head, s->n, nullptr, nullptr, EPI_NONE, ol, s->state, st));
-        FC_TRY(launch_step_tail(s->logits, c.vocab, last_mode == STEP_PROBS ? s->probs : nullptr, last_mode == STEP_SELECT ? 1 : 0,
-                                s->queue, s->queue_cap, s->state, nullptr, st));
+        FC_TRY(launch_head(s, m->x + ((size_t)i * n + n - 1) * d, last_mode));
     }
     return FC_OK;
 }

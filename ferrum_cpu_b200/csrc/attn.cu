@@ -1,102 +1,9 @@
-// Causal multi-head attention: the single-query KV-cached form used by decode, and the
-// full-window form used by scoring/prefill. fp32 throughout; the T x T probability matrix
+// Causal multi-head attention over whole windows (scoring, prefill) on CUDA cores, fp32 throughout; the T x T probability matrix
 // the reference stores (transformer.rs:458-478 `last_attention`) is never materialised.
 #include "fc_common.cuh"
 #include "pdl.cuh"
 
 namespace fc {
-
-// --------------------------------------------------------------------------- decode form
-// layer/transformer.rs:246-283 forward_with_cache, per head h: scores[j] = (q_h · k_h(j)) *
-// 1/sqrt(hd) over the len cached rows, softmax (max, exp, sum), out_h = sum_j (e_j/sum) v_h(j).
-// One block per query head. Cache rows are kvd floats apart; query head h reads key/value head
-// h / group (grouped-query attention, llm.rs:305-341; group == 1 is the GPT-2 form).
-__global__ void __launch_bounds__(256) attn_decode_kernel(const float* __restrict__ q, const float* __restrict__ kc,
-                                                          const float* __restrict__ vc, int kvd, int group, int hd, int ctx,
-                                                          const StepState* st, float* __restrict__ out) {
-    extern __shared__ float sm[];   // scores[ctx] | q_h[hd] | red[64] | part[8][hd]
-    pdl_trigger();
-    pdl_wait();
-    if (st->done | st->error) return;
-    const int len = st->pos + 1;    // the new row was appended by the QKV GEMV
-    const int h = blockIdx.x, hs = h * hd, ks = (h / group) * hd;
-    float* sc = sm;
-    float* qh = sm + ctx;
-    float* red = qh + hd;
-    float* part = red + 64;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int c = threadIdx.x; c < hd; c += blockDim.x) qh[c] = q[hs + c];
-    __syncthreads();
-    const float scale = 1.0f / sqrtf((float)hd);
-    // scores: one warp per cached row, lanes across the head dimension
-    float mx = -INFINITY;
-    for (int j = wid; j < len; j += nw) {
-        const float* kr = kc + (size_t)j * kvd + ks;
-        float dot = 0.0f;
-        for (int c = lane; c < hd; c += 32) dot = fmaf(qh[c], kr[c], dot);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        const float s = dot * scale;
-        if (lane == 0) sc[j] = s;
-        mx = fmaxf(mx, s);
-    }
-    if (lane == 0) red[wid] = mx;
-    __syncthreads();
-    mx = red[0];
-    for (int w = 1; w < nw; ++w) mx = fmaxf(mx, red[w]);
-    __syncthreads();
-    float s = 0.0f;
-    for (int j = threadIdx.x; j < len; j += blockDim.x) {
-        const float e = expf(sc[j] - mx);
-        sc[j] = e;
-        s += e;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) red[32 + wid] = s;
-    __syncthreads();
-    float sum = 0.0f;
-    for (int w = 0; w < nw; ++w) sum += red[32 + w];
-    // out: thread (g, c) accumulates rows j = g, g+G, ... for dimension c, then the G
-    // partials are added in a fixed order.
-    const int G = blockDim.x / hd;   // hd <= blockDim.x
-    const int g = threadIdx.x / hd, c = threadIdx.x - g * hd;
-    if (g < G) {
-        float acc = 0.0f;
-        for (int j = g; j < len; j += G) acc = fmaf(sc[j] / sum, vc[(size_t)j * kvd + ks + c], acc);
-        part[g * hd + c] = acc;
-    }
-    __syncthreads();
-    if (threadIdx.x < hd) {
-        float acc = 0.0f;
-        for (int gg = 0; gg < G; ++gg) acc += part[gg * hd + threadIdx.x];
-        out[hs + threadIdx.x] = acc;
-    }
-}
-
-int launch_attn_decode_gqa(const float* q, const float* kcache, const float* vcache, int H, int KV, int hd, int ctx,
-                           const StepState* state, float* out, cudaStream_t st) {
-    if (hd > 256) return fail(FC_E_SHAPE, "head_dim %d exceeds 256", hd);
-    const int threads = 256;
-    const size_t smem = (size_t)(ctx + hd + 64 + (threads / hd) * hd) * sizeof(float);
-    if (smem > 200 * 1024) return fail(FC_E_SHAPE, "context %d exceeds what the decode attention holds in shared memory", ctx);
-    if (smem > 48 * 1024) FC_CUDA(cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    FC_CUDA(launch_pdl(attn_decode_kernel, dim3(H), dim3(threads), smem, st, q, kcache, vcache, KV * hd, H / KV, hd, ctx, state, out));
-    ++g_launches;
-    return FC_OK;
-}
-
-int launch_attn_decode(const float* q, const float* kcache, const float* vcache, int d, int H, int ctx,
-                       const StepState* state, float* out, cudaStream_t st) {
-    const int hd = d / H, threads = 256;
-    if (hd > 256) return fail(FC_E_SHAPE, "head_dim %d exceeds 256", hd);
-    const size_t smem = (size_t)(ctx + hd + 64 + (threads / hd) * hd) * sizeof(float);
-    if (smem > 200 * 1024) return fail(FC_E_SHAPE, "context %d exceeds what the decode attention holds in shared memory", ctx);
-    if (smem > 48 * 1024) FC_CUDA(cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attn_decode_kernel<<<H, threads, smem, st>>>(q, kcache, vcache, d, 1, hd, ctx, state, out);
-    FC_LAUNCHED();
-    return FC_OK;
-}
 
 // --------------------------------------------------------------------------- window form
 // layer/transformer.rs:395-477 per (window b, head h): S = Q Kᵀ · 1/sqrt(hd), entries j > i

@@ -171,10 +171,11 @@ int launch(const float* qkv, int n_q, int n_kv, int half, int neox, const float2
 }  // namespace
 
 // Other widths of a head, and contexts whose scores alone fill shared memory, keep the kernels that read the caches in place.
-bool attn_step_covers(int hd, int ctx) { return (hd == 32 || hd == 64 || hd == 128) && ctx <= 32768; }
+bool attn_step_covers(int hd, int ctx) { return (hd == 32 || hd == 64 || hd == 128) && (size_t)ctx * 4 <= kSmem; }
 
 int launch_attn_step(const float* qkv, int n_q, int n_kv, int hd, int rope_dim, int neox, const float2* ftab, float inv_linear,
                      float* kc, float* vc, int ctx, const StepState* state, float* out, cudaStream_t st) {
+    if (!attn_step_covers(hd, ctx)) return fail(FC_E_SHAPE, "attention step: heads of %d, context %d", hd, ctx);
     auto go = hd == 32 ? launch<32> : hd == 64 ? launch<64> : launch<128>;
     return go(qkv, n_q, n_kv, rope_dim / 2, neox, ftab, inv_linear, kc, vc, ctx, state, out, st);
 }

@@ -113,22 +113,6 @@ struct StepState {
 // repack.cu
 int launch_repack_q8(const uint8_t* raw, int N, int K, int N_pad, uint8_t* qu, __half* d, cudaStream_t st);
 
-// gemv.cu — y = W·x + bias (+GELU) (+residual), one activation row.
-struct GemvOut {
-    // Row n of the result goes to out[n / seg][n % seg]; segments 1 and 2 (K and V rows of
-    // the fused QKV matrix) are offset by pos * pos_stride floats, pos read from `state`.
-    float* out[3] = {nullptr, nullptr, nullptr};
-    int seg = 0;
-    size_t pos_stride = 0;
-};
-int launch_gemv_q8(const QMat& w, const float* x, const float* bias, const float* residual, int epi,
-                   const GemvOut& out, const StepState* state, cudaStream_t st);
-
-// Split-K form for wide matrices: optional RMSNorm of x (norm_w, eps) as it is staged; epi
-// EPI_SWIGLU pairs rows (2i, 2i+1) as (gate, up) and writes out[i] = silu(gate) * up.
-int launch_gemv_q8_wide(const QMat& w, const float* x, const float* norm_w, float eps, const float* bias, const float* residual,
-                        int epi, float* out, const StepState* state, cudaStream_t st);
-
 // gemv_row.cu — one activation row against up to three matrices (q | k | v, gate | up) of the same K. part.d: f16 scales per
 // 32 of k, or null with part.xscale [K]: the scale of input index k (then levels alone); EPI_SWIGLU pairs rows (2i, 2i + 1) of one matrix, or row i of two, as (gate, up) and writes
 // part[0].out[i] = silu(gate) * up. Launched as a programmatic dependent.
@@ -204,8 +188,6 @@ int launch_embed_step(const QMat& tok, const float* pos_emb, int ctx, const int*
 // pos: each row's position in its window, or null: r % T.
 int launch_embed_rows(const QMat& tok, const float* pos_emb, const int* ids, const int* pos, int R, int T, float* x,
                       int* error_flag, cudaStream_t st);
-int launch_layernorm(const float* x, const float* g, const float* b, int rows, int d, float* y,
-                     const StepState* state, cudaStream_t st);
 // LayerNorm written as bf16 planes [rows][d] for the tensor-core GEMM. pick (may be null): row i of the output is row pick[i]
 // of x.
 int launch_layernorm_planes(const float* x, const float* g, const float* b, const int* pick, int rows, int d, const Planes& out,
@@ -215,10 +197,7 @@ int launch_layernorm_planes(const float* x, const float* g, const float* b, cons
 // The tail behind a head product with stats: probabilities (probs set) or the greedy pick, then the step's advance.
 int launch_step_finish(const float* logits, int V, const float2* stats, int n_stats, float* probs_or_null, int* queue, int queue_cap,
                        StepState* state, cudaStream_t st);
-int launch_step_tail(const float* logits, int V, float* probs_or_null, int do_select, int* queue, int queue_cap,
-                     StepState* state, float* sel_logit_or_null, cudaStream_t st);
 // End-of-step bookkeeping alone (steps that skip the head).
-int launch_step_advance(StepState* state, cudaStream_t st);
 int launch_step_advance_pdl(StepState* state, cudaStream_t st);
 int launch_softmax_row(const float* logits, int V, float* probs, cudaStream_t st);
 // sample.cu — one draw of sample_with_params on the device; see the kernel for the arguments.
@@ -252,14 +231,10 @@ size_t layer_stats_scratch_bytes();
 int launch_layer_stats(const float* x, const Planes& planes, size_t n, void* scratch, LayerStatsDev* out, cudaStream_t st);
 
 // attn.cu
-int launch_attn_decode(const float* q, const float* kcache, const float* vcache, int d, int H, int ctx,
-                       const StepState* state, float* out, cudaStream_t st);
 // qkv [R][3d] (q | k | v per row), causal within each window.
 int launch_attn_prefill(const float* qkv, const Windows& w, int d, int H, float* out, cudaStream_t st);
 // Grouped-query forms (llm.rs:305-341): H query heads share KV key/value heads of width hd.
 // Decode: q [H*hd], caches [ctx][KV*hd]. Window: q, k, v rows ld floats apart, out rows ldo apart.
-int launch_attn_decode_gqa(const float* q, const float* kcache, const float* vcache, int H, int KV, int hd, int ctx,
-                           const StepState* state, float* out, cudaStream_t st);
 int launch_attn_prefill_gqa(const float* q, const float* k, const float* v, const Windows& w, int ld, int H, int KV, int hd,
                             int ldo, float* out, cudaStream_t st);
 // attn_tc.cu — the same on tcgen05 (head_dim 64): bf16 planes (two or three) of qkv [R][3d] in, as many planes of the

@@ -102,38 +102,7 @@ int launch_embed_rows(const QMat& tok, const float* pos_emb, const int* ids, con
 // ------------------------------------------------------------------------------ LayerNorm
 // layer/norm.rs:46-82: mean, then the variance of (x - mean), std = sqrt(var + 1e-5),
 // y = ((x - mean) / std) * gamma + beta. One block per row; the row is held in registers.
-template <int PER>
-__global__ void layernorm_kernel(const float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ b,
-                                 int d, float* __restrict__ y, const StepState* st) {
-    __shared__ float red[33];
-    if (st && (st->done | st->error)) return;
-    const float* xr = x + (size_t)blockIdx.x * d;
-    float v[PER];
-    float s = 0.0f;
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int c = threadIdx.x + i * blockDim.x;
-        v[i] = c < d ? xr[c] : 0.0f;
-        s += v[i];
-    }
-    const float mean = block_sum(s, red) / (float)d;
-    float q = 0.0f;
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int c = threadIdx.x + i * blockDim.x;
-        const float t = v[i] - mean;
-        q += c < d ? t * t : 0.0f;
-    }
-    const float var = block_sum(q, red) / (float)d;
-    const float sd = sqrtf(var + 1e-5f);
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int c = threadIdx.x + i * blockDim.x;
-        if (c < d) y[(size_t)blockIdx.x * d + c] = ((v[i] - mean) / sd) * g[c] + b[c];
-    }
-}
-
-// The same LayerNorm with the result written as the P bf16 planes that the tensor-core GEMM reads.
+// The result is written as the P bf16 planes that the tensor-core GEMM reads.
 template <int PER, int P>
 __global__ void layernorm_planes_kernel(const float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ b,
                                         const int* __restrict__ pick, int d, const Planes out) {
@@ -231,18 +200,6 @@ int launch_layernorm_planes(const float* x, const float* g, const float* b, cons
     return out.n == 3 ? layernorm_planes<3>(x, g, b, pick, rows, d, out, st) : layernorm_planes<2>(x, g, b, pick, rows, d, out, st);
 }
 
-int launch_layernorm(const float* x, const float* g, const float* b, int rows, int d, float* y,
-                     const StepState* state, cudaStream_t st) {
-    const int threads = 256;
-    const int per = (d + threads - 1) / threads;
-    if (per <= 4) layernorm_kernel<4><<<rows, threads, 0, st>>>(x, g, b, d, y, state);
-    else if (per <= 8) layernorm_kernel<8><<<rows, threads, 0, st>>>(x, g, b, d, y, state);
-    else if (per <= 16) layernorm_kernel<16><<<rows, threads, 0, st>>>(x, g, b, d, y, state);
-    else return fail(FC_E_SHAPE, "LayerNorm width %d exceeds 4096", d);
-    FC_LAUNCHED();
-    return FC_OK;
-}
-
 // ------------------------------------------------------------------------------ decode tail
 // ops.rs:478-502 softmax_rows on one row, then (when selecting) token_stream.rs:134 +
 // sampling.rs:96-104,147: logit_i = ln(max(p_i, 1e-12)), first index of the largest.
@@ -251,64 +208,6 @@ struct ArgPair { float v; int i; };
 __device__ __forceinline__ ArgPair better(ArgPair a, ArgPair b) {
     // larger value wins; equal values: smaller index (first on ties)
     return (b.v > a.v || (b.v == a.v && b.i < a.i)) ? b : a;
-}
-
-__global__ void __launch_bounds__(1024) step_tail_kernel(const float* __restrict__ logits, int V, float* __restrict__ probs,
-                                                         int do_select, int* __restrict__ queue, int queue_cap,
-                                                         StepState* st, float* sel_logit) {
-    __shared__ float red[33];
-    __shared__ ArgPair pred[32];
-    if (st->done | st->error) return;
-    float mx = -INFINITY;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) mx = fmaxf(mx, logits[i]);
-    mx = block_max(mx, red);
-    float s = 0.0f;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) s += expf(logits[i] - mx);
-    const float sum = block_sum(s, red);
-    if (probs)
-        for (int i = threadIdx.x; i < V; i += blockDim.x) probs[i] = expf(logits[i] - mx) / sum;
-    if (do_select) {
-        ArgPair best{-INFINITY, 0x7fffffff};
-        for (int i = threadIdx.x; i < V; i += blockDim.x) {
-            const float p = expf(logits[i] - mx) / sum;
-            best = better(best, ArgPair{logf(fmaxf(p, 1e-12f)), i});
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            ArgPair other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
-            best = better(best, other);
-        }
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        if (lane == 0) pred[wid] = best;
-        __syncthreads();
-        if (wid == 0) {
-            best = lane < (int)((blockDim.x + 31) >> 5) ? pred[lane] : ArgPair{-INFINITY, 0x7fffffff};
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                ArgPair other{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
-                best = better(best, other);
-            }
-            if (lane == 0) {
-                if (sel_logit) sel_logit[st->tail < queue_cap ? st->tail : queue_cap - 1] = best.v;
-                if (best.i == st->eos) {
-                    st->done = 1;
-                } else if (st->tail < queue_cap) {
-                    queue[st->tail] = best.i;
-                    st->tail += 1;
-                } else {
-                    st->error = FC_E_DIM;
-                }
-            }
-        }
-    }
-    if (threadIdx.x == 0) { st->pos += 1; st->fed += 1; }
-}
-
-int launch_step_tail(const float* logits, int V, float* probs_or_null, int do_select, int* queue, int queue_cap,
-                     StepState* state, float* sel_logit_or_null, cudaStream_t st) {
-    step_tail_kernel<<<1, 1024, 0, st>>>(logits, V, probs_or_null, do_select, queue, queue_cap, state, sel_logit_or_null);
-    FC_LAUNCHED();
-    return FC_OK;
 }
 
 // The tail of a step whose head product left, per CTA, its largest logit and the mass around it: the softmax needs no pass of
@@ -408,12 +307,7 @@ __global__ void step_advance_kernel(StepState* st) {
     st->pos += 1;
     st->fed += 1;
 }
-int launch_step_advance(StepState* state, cudaStream_t st) {
-    step_advance_kernel<<<1, 1, 0, st>>>(state);
-    FC_LAUNCHED();
-    return FC_OK;
-}
-// The same as a programmatic dependent of the kernel ahead (steps whose kernels all wait first).
+// A programmatic dependent of the kernel ahead (steps whose kernels all wait first).
 int launch_step_advance_pdl(StepState* state, cudaStream_t st) {
     FC_CUDA(launch_pdl(step_advance_kernel, dim3(1), dim3(1), 0, st, state));
     ++g_launches;
