@@ -37,8 +37,8 @@ extern "C" {
 #define FC_E_ARG (-7)       /* null handle / null required pointer */
 
 /* Math modes of the prefill GEMM. Decode always runs fp32 FMA on CUDA cores. */
-#define FC_MATH_FP32 0      /* fp32 CUDA-core GEMM (exactly rounded products) */
-#define FC_MATH_BF16X3 1    /* tcgen05 kind::f16 bf16 operands, 3-term split, fp32 TMEM accumulate */
+#define FC_MATH_FP32 0      /* tcgen05 kind::f16, activations as three bf16 planes (their f32 value exactly), f32 accumulate */
+#define FC_MATH_BF16X3 1    /* the same with two planes (2^-17 relative) */
 
 /* Dimensions of a gpt2-architecture GGUF (ferrum_core/src/loader/gpt2.rs:201-215). */
 typedef struct fc_config {
