@@ -8,7 +8,8 @@
 // into shared memory), and after the wait only this step's q, k and v are missing. Keys are stored at a stride of 4 mod 8
 // units of 16 bytes, so that the 4 lanes that share a key and the 8 keys of a warp's sweep read every bank once; values are
 // read row by row and need no padding. Rows that do not fit in shared memory are read where they are.
-// 256 threads, so that the kernel fits on an SM beside a product of up to 96 registers a thread and really does start early.
+// 256 threads, and q, k and v asked for ahead of the check of the state: a step of 12 layers of width 768 takes 226.6 us; with
+// 512 threads and the loads behind the check 232.6 us.
 #include <algorithm>
 #include <atomic>
 

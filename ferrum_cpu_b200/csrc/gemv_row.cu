@@ -133,6 +133,13 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
         if (nw && u < units) gw[i] = ((const float4*)nw)[u];
         if (nb && u < units) gb[i] = ((const float4*)nb)[u];
     }
+    // and, where the scales belong to the input index, those of its first unit (behind the wait each copy of the row would
+    // cost an L2 round trip: 16 layers of width 512, int8, 64 tokens: 20.0 instead of 23.5 ms)
+    float4 sx[3];
+    if constexpr (!SCALED)
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+            if (p < a.staged && a.part[p].xscale && tid < units) sx[p] = ((const float4*)a.part[p].xscale)[tid];
 
     pdl_wait();
     float4 v[UN];
@@ -208,9 +215,12 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
             t.z = __fmul_rn(__fmul_rn(t.z, inv), g.z); t.w = __fmul_rn(__fmul_rn(t.w, inv), g.w);
         }
         const int at = u ^ ((u >> 3) & 3);
-        if (!a.part[0].xscale) { xs[at] = t; return; }
-        for (int p = 0; p < a.staged; ++p) {
-            const float4 s = ((const float4*)a.part[p].xscale)[u];
+        if (SCALED || !a.part[0].xscale) { xs[at] = t; return; }
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            if (p >= a.staged) break;
+            float4 s = sx[p];
+            if (u != tid) s = ((const float4*)a.part[p].xscale)[u];
             xs[(size_t)p * units + at] = make_float4(t.x * s.x, t.y * s.y, t.z * s.z, t.w * s.w);
         }
     };
