@@ -70,8 +70,8 @@ struct fc_llama_cache {
     StepState* state = nullptr;
     int* status = nullptr;                // raised by a kernel whose bounded wait ran out
     int host_pos = 0;
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};   // [0]: step without the head, [1]: with it
-    int graph_nodes[2] = {0, 0};
+    cudaGraphExec_t graph[3] = {};   // [0]: step without the head, [1]: with it, [2]: kFreeSteps times the greedy pick and [1]
+    int graph_nodes[3] = {};
     bool packed_warm[2] = {false, false};   // packed model: the uncaptured first step of each kind has run
     unsigned long long* rng_d = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -428,30 +428,43 @@ int launch_step_packed(fc_llama_cache* s, int with_head) {
     return launch_step_advance_pdl(s->state, st);
 }
 
-int run_step(fc_llama_cache* s, int with_head) {
-    const bool packed = s->m->prec >= 0;
-    if (packed && !s->packed_warm[with_head]) {
-        s->packed_warm[with_head] = true;
-        return launch_step_packed(s, with_head);
-    }
-    if (!s->graph[with_head]) {
-        cudaStream_t st = s->m->st;
+// Greedy tokens that need nothing from the host share a graph: between two graphs the GPU waits for the next one's launch.
+constexpr int kFreeSteps = 8;
+
+int run_graph(fc_llama_cache* s, int which) {
+    if (!s->graph[which]) {
+        const fc_llama* m = s->m;
+        cudaStream_t st = m->st;
         cudaGraph_t g = nullptr;
         const int64_t before = g_launches;
+        auto step = [&](int with_head) { return m->prec >= 0 ? launch_step_packed(s, with_head) : launch_step(s, with_head); };
         FC_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        const int rc = packed ? launch_step_packed(s, with_head) : launch_step(s, with_head);
+        int rc = FC_OK;
+        if (which < 2) rc = step(which);
+        for (int i = 0; which == 2 && i < kFreeSteps && rc == FC_OK; ++i) {
+            rc = launch_llama_pick(s->logits, m->cfg.vocab, s->queue, s->queue_cap, s->state, st);
+            if (rc == FC_OK) rc = step(1);
+        }
         const cudaError_t e = cudaStreamEndCapture(st, &g);
-        s->graph_nodes[with_head] = (int)(g_launches - before);
+        s->graph_nodes[which] = (int)(g_launches - before);
         g_launches = before;
         if (rc != FC_OK) { if (g) cudaGraphDestroy(g); return rc; }
         FC_CUDA(e);
-        const cudaError_t ei = cudaGraphInstantiate(&s->graph[with_head], g, 0);
+        const cudaError_t ei = cudaGraphInstantiate(&s->graph[which], g, 0);
         cudaGraphDestroy(g);
         FC_CUDA(ei);
     }
-    FC_CUDA(cudaGraphLaunch(s->graph[with_head], s->m->st));
-    g_launches += s->graph_nodes[with_head];
+    FC_CUDA(cudaGraphLaunch(s->graph[which], s->m->st));
+    g_launches += s->graph_nodes[which];
     return FC_OK;
+}
+
+int run_step(fc_llama_cache* s, int with_head) {
+    if (s->m->prec >= 0 && !s->packed_warm[with_head]) {
+        s->packed_warm[with_head] = true;
+        return launch_step_packed(s, with_head);
+    }
+    return run_graph(s, with_head);
 }
 
 __global__ void llama_set_state_kernel(StepState* st, int pos, int fed, int tail) {
@@ -897,6 +910,14 @@ int fc_llama_generate(fc_llama_cache* s, const int32_t* prompt, int n, int max_n
     bool cancelled = false, timed = false;
     while (made < max_new) {
         if (cancel && *cancel) { cancelled = true; break; }
+        // all but the last tokens of a free run, once a packed step has run uncaptured
+        if (free_run && max_new - made > kFreeSteps && (m->prec < 0 || s->packed_warm[1])) {
+            rc = run_graph(s, 2);
+            if (rc != FC_OK) break;
+            made += kFreeSteps;
+            s->host_pos += kFreeSteps;
+            continue;
+        }
         // recent = prompt + tokens so far = the queue (llm.rs:740-751)
         rc = plain_greedy ? launch_llama_pick(s->logits, c.vocab, s->queue, s->queue_cap, s->state, st)
                           : launch_sample(s->logits, c.vocab, 0, *params, s->queue, 0, s->rng_d, s->queue, s->queue_cap, s->state,

@@ -447,8 +447,8 @@ __global__ void __launch_bounds__(1024) llama_pick_kernel(const float* __restric
     }
 }
 int launch_llama_pick(const float* logits, int V, int* queue, int queue_cap, StepState* state, cudaStream_t st) {
-    llama_pick_kernel<<<1, 1024, 0, st>>>(logits, V, queue, queue_cap, state);
-    FC_LAUNCHED();
+    FC_CUDA(launch_pdl(llama_pick_kernel, dim3(1), dim3(1024), 0, st, logits, V, queue, queue_cap, state));
+    ++g_launches;
     return FC_OK;
 }
 
