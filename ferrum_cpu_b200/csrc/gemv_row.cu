@@ -12,8 +12,9 @@
 //  - a warp owns RB rows (or a K slice of them) from the first load to the dot product: lanes across k, 16 levels each. It
 //    asks for the first rows BEFORE it waits for the kernel ahead (weights depend on nothing), so small matrices are in
 //    registers when the activations appear; the next rows are asked for before the current ones are multiplied;
-//  - the norm's parameters, the input scales and the first bias are asked for before that wait too, the first residual right
-//    after it: later each of them would cost an L2 round trip;
+//  - the norm's parameters, the input scales and, inside a model, the first bias are asked for before that wait too, the first
+//    residual (and a caller's bias, which may be what the kernel ahead writes) right after it: later each of them would cost
+//    an L2 round trip;
 //  - the row is staged in shared memory once, out of registers (two block barriers with a norm, one without; every thread
 //    merges the warps' sums itself, over a fixed count with wide reads: with loops over the warps and a division each, 24
 //    LayerNorms cost 50 us of a step of width 768, now 27). From there on warps do not meet, unless K is wider than 2048 and
@@ -24,6 +25,7 @@
 // (The kernel this replaced streamed 32 KB tiles through a shared-memory ring with a block barrier per tile: about 5.5 us
 // for every product of a step, however small.)
 #include <algorithm>
+#include <type_traits>
 
 #include "fc_common.cuh"
 #include "pdl.cuh"
@@ -72,9 +74,11 @@ __device__ __forceinline__ float sq4(const float4& v, float m) {
     return fmaf(a, a, fmaf(b, b, fmaf(c, c, d * d)));
 }
 
-// NORM: the row is normalised (and stats are taken): code that a plain product should not have to fetch.
+// What a product is. NORM: the row is normalised (and stats are taken), code that a plain product should not have to fetch.
+// ALONE: a caller's own product, whose bias may be the output of the kernel ahead: it is asked for behind the wait, with the row.
+enum Kind { PLAIN, NORM, ALONE };
 // NCH: 16-level chunks per lane of a row (slice). RB: rows per task; SwiGLU pairs gate row t with up row t.
-template <int NCH, int RB, bool SCALED, bool NORM>
+template <int NCH, int RB, bool SCALED, Kind KIND>
 __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowArgs a) {
     extern __shared__ __align__(16) float4 xs[];             // [staged][K / 4] units of 16 bytes, swizzled
     __shared__ __align__(16) float red[3][MAX_WARPS];
@@ -122,16 +126,20 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
     // the first task's bias, by the lane that adds it: behind the dot product it would cost an L2 round trip
     const bool finisher = slice == 0 && lane == 0;
     float bias0[RB], res0[RB];
+    auto first_bias = [&]() {
 #pragma unroll
-    for (int r = 0; r < RB; ++r) {
-        bias0[r] = res0[r] = 0.0f;
-        if (!finisher || first >= a.tasks) continue;
-        int p;
-        const int n = row_of(first, r, p);
-        if (n < a.part[p].N && a.part[p].bias) bias0[r] = a.part[p].bias[n];
-    }
+        for (int r = 0; r < RB; ++r) {
+            if (!finisher || first >= a.tasks) continue;
+            int p;
+            const int n = row_of(first, r, p);
+            if (n < a.part[p].N && a.part[p].bias) bias0[r] = a.part[p].bias[n];
+        }
+    };
+#pragma unroll
+    for (int r = 0; r < RB; ++r) bias0[r] = res0[r] = 0.0f;
+    if (KIND != ALONE) first_bias();
     // this thread's units of the norm's parameters
-    const float *nw = NORM ? a.nw : nullptr, *nb = NORM ? a.nb : nullptr;
+    const float *nw = KIND == NORM ? a.nw : nullptr, *nb = KIND == NORM ? a.nb : nullptr;
     float4 gw[UN], gb[UN];
 #pragma unroll
     for (int i = 0; i < UN; ++i) {
@@ -154,6 +162,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
         const int u = tid + i * blockDim.x;
         v[i] = u < units ? ((const float4*)a.x)[u] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
+    if (KIND == ALONE) first_bias();
     if (a.residual && finisher && first < a.tasks)
 #pragma unroll
         for (int r = 0; r < RB; ++r) {
@@ -296,7 +305,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
                 if (a.epi == EPI_GELU) v = gelu_f(v);
                 if (a.residual) v = (t == first ? res0[r] : a.residual[n[r]]) + v;
                 a.part[p[r]].out[n[r]] = v;
-                if (NORM && a.stats) {
+                if (KIND == NORM && a.stats) {
                     if (v > top) { mass *= expf(top - v); top = v; }
                     mass += expf(v - top);
                 }
@@ -310,7 +319,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
             work(wb, t + groups);
         }
     }
-    if (NORM && a.stats) {
+    if (KIND == NORM && a.stats) {
         __syncthreads();
         if (lane == 0) { red[0][wid] = top; red[1][wid] = mass; }
         __syncthreads();
@@ -324,26 +333,29 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
     }
 }
 
-template <int NCH, int RB, bool SCALED, bool NORM>
+template <int NCH, int RB, bool SCALED, Kind KIND>
 int launch_row_t(const RowArgs& a, int blocks, int threads, size_t smem, int dev, cudaStream_t st) {
     static bool ready[64] = {};
     if (!ready[dev]) {
-        FC_CUDA(cudaFuncSetAttribute(gemv_row_kernel<NCH, RB, SCALED, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+        FC_CUDA(cudaFuncSetAttribute(gemv_row_kernel<NCH, RB, SCALED, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
         ready[dev] = true;
     }
-    FC_CUDA(launch_pdl(gemv_row_kernel<NCH, RB, SCALED, NORM>, dim3(blocks), dim3(threads), smem, st, a));
+    FC_CUDA(launch_pdl(gemv_row_kernel<NCH, RB, SCALED, KIND>, dim3(blocks), dim3(threads), smem, st, a));
     ++g_launches;
     return FC_OK;
 }
 template <int NCH>
 int launch_row(int rb, bool scaled, const RowArgs& a, int blocks, int threads, size_t smem, int dev, cudaStream_t st) {
     auto go = [&](auto f) { return f(a, blocks, threads, smem, dev, st); };
-    if (a.nw) {
-        if (scaled) return go(rb == 2 ? launch_row_t<NCH, 2, true, true> : launch_row_t<NCH, 1, true, true>);
-        return go(rb == 2 ? launch_row_t<NCH, 2, false, true> : launch_row_t<NCH, 1, false, true>);
-    }
-    if (scaled) return go(rb == 2 ? launch_row_t<NCH, 2, true, false> : launch_row_t<NCH, 1, true, false>);
-    return go(rb == 2 ? launch_row_t<NCH, 2, false, false> : launch_row_t<NCH, 1, false, false>);
+    auto of = [&](auto kind) {
+        constexpr Kind KIND = decltype(kind)::value;
+        if (scaled) return go(rb == 2 ? launch_row_t<NCH, 2, true, KIND> : launch_row_t<NCH, 1, true, KIND>);
+        return go(rb == 2 ? launch_row_t<NCH, 2, false, KIND> : launch_row_t<NCH, 1, false, KIND>);
+    };
+    if (a.nw) return of(std::integral_constant<Kind, NORM>());
+    // without the state of a decode step the product is a caller's own, on the caller's pointers
+    if (!a.state) return of(std::integral_constant<Kind, ALONE>());
+    return of(std::integral_constant<Kind, PLAIN>());
 }
 
 }  // namespace
