@@ -114,6 +114,7 @@ SIGNATURES = {
     "fc_decode_batch": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_int32, C.c_void_p, C.c_void_p]),
     "fc_last_batch_ms": (C.c_float, [C.c_void_p]),
     "fc_last_batch_prime_ms": (C.c_float, [C.c_void_p]),
+    "fc_debug_withhold_scratch": (C.c_int, [C.c_int]),
     "fc_debug_set_wait_budget": (C.c_int, [C.c_longlong, C.c_int]),
     "fc_score_sequences_multi": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p]),
     "fc_decode_batch_multi": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_int32, C.c_void_p, C.c_void_p]),

@@ -97,11 +97,7 @@ struct fc_qweight {
     int device;
     Arena arena;
     QMat w;
-    // scratch of the M >= 2 product: bf16 planes of the activations, status word
-    Arena planes;
-    Planes x;
-    int* status = nullptr;
-    size_t plane_elems = 0;
+    StatusWord status;   // of the products on callers' streams
 };
 
 namespace fc {
@@ -539,8 +535,11 @@ int fc_qweight_upload(int device, const void* wq, int N, int K, fc_qweight** out
     FC_TRY(select_device(device));
     fc_qweight* w = new fc_qweight;
     w->device = device;
-    const int rc = upload_q8(w->arena, wq, N, K, &w->w, 0);
-    if (rc != FC_OK) { w->arena.release(); delete w; return rc; }
+    int rc = scratch_retain(device);
+    if (rc != FC_OK) { delete w; return rc; }
+    rc = w->status.create();
+    if (rc == FC_OK) rc = upload_q8(w->arena, wq, N, K, &w->w, 0);
+    if (rc != FC_OK) { fc_qweight_free(w); return rc; }
     *out = w;
     return FC_OK;
 }
@@ -550,7 +549,8 @@ void fc_qweight_free(fc_qweight* w) {
     cudaSetDevice(w->device);
     cudaDeviceSynchronize();
     w->arena.release();
-    w->planes.release();
+    w->status.destroy();
+    scratch_release(w->device);
     delete w;
 }
 
@@ -570,27 +570,20 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
     if (M == 1) {
         return launch_gemv_row(w->w, x_dev, RowNorm(), bias_dev, nullptr, EPI_NONE, y_dev, nullptr, st);
     }
-    // the bf16 planes of x and the status word live in the weight handle and grow on demand
-    fc_qweight* wm = const_cast<fc_qweight*>(w);
+    FC_TRY(const_cast<fc_qweight*>(w)->status.check("an earlier call on this weight"));
     const int planes = math_mode == FC_MATH_BF16X3 && w->w.K % 64 == 0 ? 2 : 3;
-    const size_t need = (size_t)M * w->w.K;
-    if (need > wm->plane_elems || !wm->x.p[planes - 1]) {
-        FC_CUDA(cudaStreamSynchronize(st));
-        wm->planes.release();
-        const size_t elems = std::max(need, wm->plane_elems);
-        const int keep = std::max(planes, wm->x.p[2] ? 3 : 2);
-        wm->plane_elems = 0;
-        wm->x = Planes();
-        wm->status = nullptr;
-        for (int p = 0; p < keep; ++p) FC_TRY(wm->planes.alloc(&wm->x.p[p], elems * 2));
-        FC_TRY(wm->planes.alloc_n(&wm->status, 1));
-        FC_CUDA(cudaMemsetAsync(wm->status, 0, sizeof(int), st));
-        wm->plane_elems = elems;
+    const size_t n = (size_t)M * w->w.K;
+    CallScratch scratch;
+    Planes x;
+    FC_TRY(take_planes(scratch, x, planes, n, w->device, st));
+    if (!scratch.p) {
+        // no memory for the planes: the rows one by one, which need none
+        for (int m = 0; m < M; ++m)
+            FC_TRY(launch_gemv_row(w->w, x_dev + (size_t)m * w->w.K, RowNorm(), bias_dev, nullptr, EPI_NONE, y_dev + (size_t)m * w->w.N, nullptr, st));
+        return FC_OK;
     }
-    Planes x = wm->x;
-    x.n = planes;
-    FC_TRY(launch_split_planes(x_dev, x, need, st));
-    return launch_gemm_q8_tc(w->w, x, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, wm->status, st);
+    FC_TRY(launch_split_planes(x_dev, x, n, st));
+    return launch_gemm_q8_tc(w->w, x, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, w->status.dev, st);
 }
 
 int fc_q8_0_linear(int device, const float* x, const void* wq, const float* bias, float* y,
@@ -613,11 +606,7 @@ int fc_q8_0_linear(int device, const float* x, const void* wq, const float* bias
         if (bias) copy(bd, bias, (size_t)N * 4, cudaMemcpyHostToDevice);
         if (rc == FC_OK) rc = fc_q8_0_linear_dev(w, xd, bd, yd, M, math_mode, nullptr);
         if (rc == FC_OK && cudaDeviceSynchronize() != cudaSuccess) rc = cuda_fail(cudaGetLastError(), "fc_q8_0_linear kernel", __FILE__, __LINE__);
-        if (rc == FC_OK && w->status) {
-            int status = 0;
-            copy(&status, w->status, sizeof(int), cudaMemcpyDeviceToHost);
-            if (rc == FC_OK && status != 0) rc = fail(FC_E_TIMEOUT, "a bounded wait inside the tensor-core GEMM ran out (status %d)", status);
-        }
+        if (rc == FC_OK) rc = w->status.check("fc_q8_0_linear");
         copy(y, yd, (size_t)M * N * 4, cudaMemcpyDeviceToHost);
         tmp.release();
     }
@@ -1873,6 +1862,11 @@ int fc_decode_batch_multi(fc_model* const* models, int n_models, int n_streams, 
     return run_on_models(n_models, n_streams, [&](int i, int a, int b) {
         return fc_decode_batch(models[i], b - a, prompts + (size_t)a * prompt_len, prompt_len, max_new, eos, out + (size_t)a * max_new, n_out + a);
     });
+}
+
+int fc_debug_withhold_scratch(int on) {
+    g_debug.withhold_scratch = on != 0;
+    return FC_OK;
 }
 
 int fc_debug_set_wait_budget(long long cycles, int withhold_producers) {

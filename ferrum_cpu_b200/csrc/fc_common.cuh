@@ -46,6 +46,7 @@ inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 struct DebugKnobs {
     long long wait_cycles = 4000000000LL;   // ~2 s at 1.9 GHz
     int withhold = 0;
+    int withhold_scratch = 0;               // CallScratch finds no memory
 };
 extern DebugKnobs g_debug;
 
@@ -64,6 +65,28 @@ struct Arena {
         for (void* p : ptrs) cudaFree(p);
         ptrs.clear();
     }
+};
+// scratch.cu — device memory of one call, taken and given back in the order of its stream. take leaves p null when there is no
+// memory; the other failures are errors. A device's pool lives while weights are retained on it.
+int scratch_retain(int device);
+void scratch_release(int device);
+struct CallScratch {
+    void* p = nullptr;
+    int take(int device, size_t bytes, cudaStream_t st);
+    CallScratch() = default;
+    CallScratch(const CallScratch&) = delete;
+    CallScratch& operator=(const CallScratch&) = delete;
+    ~CallScratch();
+private:
+    cudaStream_t st_ = nullptr;
+};
+// A word of pinned host memory that kernels raise and the host reads without a copy.
+struct StatusWord {
+    volatile int* host = nullptr;
+    int* dev = nullptr;
+    int create();
+    void destroy();
+    int check(const char* what);   // FC_E_TIMEOUT, once, after a kernel raised it
 };
 struct QMat;
 // Makes `device` current; refuses anything but an sm_100 part (there is no other code path).
@@ -160,6 +183,8 @@ struct Planes {
     void* p[3] = {nullptr, nullptr, nullptr};
     int n = 0;
 };
+// Planes of n elements out of a call's scratch; scratch.p stays null when there is no memory.
+int take_planes(CallScratch& scratch, Planes& x, int planes, size_t n, int device, cudaStream_t st);
 // cols (may be null): column k of rows K wide is multiplied by cols[k] first.
 int launch_split_planes(const float* x, const Planes& out, size_t n, cudaStream_t st, const float* cols = nullptr, int K = 4);
 // gemm_tc.cu — Y[M][N] = X[M][K]·Wᵀ + bias (+GELU / SwiGLU) (+residual[M][N]) on tcgen05 tensor cores, the weight exact, X

@@ -25,10 +25,7 @@ struct fc_rowq {
     uint8_t* q = nullptr;
     float* scales = nullptr;
     fc::QMat levels;               // the matrix as rows of levels [cols][rows]; qu null: the packed form `q` is what runs
-    fc::Arena pl;                  // planes of x * scale and the status word of the tensor-core product, grown on demand
-    fc::Planes planes;
-    size_t plane_elems = 0;
-    int* status = nullptr;
+    fc::StatusWord status;         // of the tensor-core products on callers' streams
     // scratch: slice partials, grown on demand. A single activation row has a buffer of its own, whose size never
     // changes once it exists: a captured decode step keeps pointing at it whatever the batched calls do to the other.
     fc::Arena ws, ws1;
@@ -260,21 +257,26 @@ int launch_rowq_linear(fc_rowq* w, const float* x, const float* bias, const floa
     GemvPart part;
     if (!rowq_part(w, bias, y, &part)) return rowq_launch(w, x, bias, residual, y, ldy, M, st);
     if (M == 1) return launch_gemv_row(&part, 1, w->rows, x, RowNorm(), residual, EPI_NONE, nullptr, st);
-    const size_t need = (size_t)M * w->rows;
-    if (!scratch && need > w->plane_elems) {
-        FC_CUDA(cudaStreamSynchronize(st));
-        w->pl.release();
-        w->plane_elems = 0;
-        w->planes = Planes();
-        for (int p = 0; p < 3; ++p) FC_TRY(w->pl.alloc(&w->planes.p[p], need * 2));
-        FC_TRY(w->pl.alloc_n(&w->status, 1));
-        FC_CUDA(cudaMemsetAsync(w->status, 0, sizeof(int), st));
-        w->planes.n = 3;
-        w->plane_elems = need;
+    const size_t n = (size_t)M * w->rows;
+    CallScratch own;
+    Planes p;
+    if (scratch) {
+        p = *scratch;
+    } else {
+        FC_TRY(w->status.check("an earlier call on this weight"));
+        FC_TRY(take_planes(own, p, 3, n, w->device, st));
+        if (!own.p) {
+            // no memory for the planes: the rows one by one, which need none
+            for (int m = 0; m < M; ++m) {
+                part.out = y + (size_t)m * ldy;
+                FC_TRY(launch_gemv_row(&part, 1, w->rows, x + (size_t)m * w->rows, RowNorm(), residual ? residual + (size_t)m * ldy : nullptr,
+                                       EPI_NONE, nullptr, st));
+            }
+            return FC_OK;
+        }
     }
-    const Planes& p = scratch ? *scratch : w->planes;
-    FC_TRY(launch_split_planes(x, p, need, st, w->scales, w->rows));
-    return launch_gemm_q8_tc(w->levels, p, bias, residual, EPI_NONE, y, nullptr, M, ldy, scratch ? status : w->status, st);
+    FC_TRY(launch_split_planes(x, p, n, st, w->scales, w->rows));
+    return launch_gemm_q8_tc(w->levels, p, bias, residual, EPI_NONE, y, nullptr, M, ldy, scratch ? status : w->status.dev, st);
 }
 }  // namespace fc
 
@@ -292,8 +294,11 @@ int fc_rowq_upload(int device, const uint8_t* q, const float* scales, int rows, 
     w->device = device; w->rows = rows; w->cols = cols; w->kind = kind;
     const size_t rb = kind == FC_Q_INT4 ? (size_t)(cols + 1) / 2 : (size_t)cols;
     w->ld = (int)((rb + 15) & ~(size_t)15);
+    int rc = scratch_retain(device);
+    if (rc != FC_OK) { delete w; return rc; }
     Arena packed;                  // given back when the rows of levels exist
     auto build = [&]() -> int {
+        FC_TRY(w->status.create());
         FC_TRY(packed.alloc_n(&w->q, (size_t)rows * w->ld));
         FC_TRY(w->arena.alloc_n(&w->scales, (size_t)rows));
         FC_CUDA(cudaMemset(w->q, 0, (size_t)rows * w->ld));
@@ -314,7 +319,7 @@ int fc_rowq_upload(int device, const uint8_t* q, const float* scales, int rows, 
         }
         return FC_OK;
     };
-    const int rc = build();
+    rc = build();
     w->arena.ptrs.insert(w->arena.ptrs.end(), packed.ptrs.begin(), packed.ptrs.end());
     if (rc != FC_OK) { fc_rowq_free(w); return rc; }
     *out = w;
@@ -327,8 +332,9 @@ void fc_rowq_free(fc_rowq* w) {
     cudaDeviceSynchronize();
     w->ws.release();
     w->ws1.release();
-    w->pl.release();
     w->arena.release();
+    w->status.destroy();
+    scratch_release(w->device);
     delete w;
 }
 
@@ -357,6 +363,7 @@ int fc_rowq_linear(const fc_rowq* w, const float* x, const float* bias, float* y
     copy(bd, bias, (size_t)w->cols * 4, cudaMemcpyHostToDevice);
     if (rc == FC_OK) rc = launch_rowq_linear(const_cast<fc_rowq*>(w), xd, bd, nullptr, yd, w->cols, M, nullptr);
     if (rc == FC_OK && cudaDeviceSynchronize() != cudaSuccess) rc = fail(FC_E_CUDA, "fc_rowq_linear: the kernel failed");
+    if (rc == FC_OK) rc = const_cast<fc_rowq*>(w)->status.check("fc_rowq_linear");
     copy(y, yd, (size_t)M * w->cols * 4, cudaMemcpyDeviceToHost);
     a.release();
     return rc;

@@ -180,5 +180,6 @@ extern "C" {
     pub fn fc_take_launch_count() -> i64;
     pub fn fc_last_decode_ms(s: *const fc_stream) -> f32;
     pub fn fc_last_score_ms(m: *const fc_model) -> f32;
+    pub fn fc_debug_withhold_scratch(on: c_int) -> c_int;
     pub fn fc_debug_set_wait_budget(cycles: i64, withhold_producers: c_int) -> c_int;
 }

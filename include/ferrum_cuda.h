@@ -149,9 +149,20 @@ int fc_q8_0_linear(int device, const float* x, const void* wq, const float* bias
 /* The same with the weight resident: upload once, multiply many times on device
  * pointers (x_dev, bias_dev, y_dev are device memory on the weight's GPU). The kernels read and
  * write them with 16-byte vector accesses: a pointer that is not 16-byte aligned (a sub-view at an
- * odd element offset, say) is refused with FC_E_ARG before anything is launched. This entry cannot
- * report a device-side timeout (it returns before the kernel ends); an fc_qweight handle is used
- * by one host thread at a time, like every other handle. */
+ * odd element offset, say) is refused with FC_E_ARG before anything is launched. An fc_qweight
+ * handle is used by one host thread at a time, like every other handle; the streams it is used on may
+ * be several, and calls on them may overlap.
+ * Operands are read and written in the stream's order, bias_dev included: it may be what the call ahead
+ * on the stream writes. With M >= 2 the rows of x are first split into bf16 planes (two in
+ * FC_MATH_BF16X3 when K is a multiple of 64, else three: 4 or 6 bytes an element). That scratch belongs
+ * to the call, not to the weight: it is taken from a pool in the order of the stream and given back in
+ * the same order, so that a call may be captured into a graph without a call before it (it becomes an
+ * allocation node; such a graph cannot be a child node). Between calls the pool keeps 256 MiB at most
+ * for all weights of a device and gives everything back with the last of them. Where there is no
+ * memory for it, the rows run one by one on the kernel of M = 1, which needs none.
+ * A device-side wait that runs out (M >= 2, both math modes) can only be seen after the kernel has
+ * ended: it is reported as FC_E_TIMEOUT by the next call with M >= 2 on the handle, which launches
+ * nothing. */
 int fc_qweight_upload(int device, const void* wq, int N, int K, fc_qweight** out);
 void fc_qweight_free(fc_qweight* w);
 int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bias_dev, float* y_dev,
@@ -162,11 +173,10 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
  *
  * Who needs it: a serving loop that handed all free device memory to its own pool at
  * start-up, so a cudaMalloc inside the library would fail; or a latency-critical thread that
- * cannot afford cudaMalloc taking the driver's allocation lock and synchronising with other
- * work on the device. fc_q8_0_linear_dev grows its scratch (the two bf16 planes the
- * activations are split into, plus a status word) with cudaMalloc on demand; this entry point
- * keeps that scratch in a fixed array inside the library instead and calls no cudaMalloc,
- * cudaFree or allocating library routine.
+ * cannot afford an allocation taking the driver's lock. fc_q8_0_linear_dev takes its scratch (the
+ * bf16 planes the activations are split into) from a memory pool that grows on demand; this
+ * entry point keeps that scratch in a fixed array inside the library instead and calls no
+ * allocating or freeing routine.
  *
  * Limits and rules:
  *  - M * K <= 4 194 304 activations per call (FC_E_SHAPE beyond that: split the rows over
@@ -474,7 +484,9 @@ void fc_rowq_free(fc_rowq* w);
  * cols are the handle's). */
 int fc_rowq_linear(const fc_rowq* w, const float* x, const float* bias, float* y, int M);
 /* The same on device pointers, asynchronous on `stream` (a cudaStream_t, or NULL). x_dev, bias_dev and
- * y_dev must be 16-byte aligned (FC_E_ARG otherwise). */
+ * y_dev must be 16-byte aligned (FC_E_ARG otherwise). Operands, scratch, streams and timeouts as
+ * fc_q8_0_linear_dev has them, where rows is a multiple of 32 (12288 at most). Other widths run on a kernel
+ * whose scratch grows in the handle: one stream at a time, and a call of that size before a capture. */
 int fc_rowq_linear_dev(const fc_rowq* w, const float* x_dev, const float* bias_dev, float* y_dev, int M, void* stream);
 
 /* ---- introspection used by the benchmark ----------------------------------------- */
@@ -498,6 +510,8 @@ float fc_last_score_ms(const fc_model* m);
  * Nothing faults, traps or waits without a limit. Not for production use: restore
  * (4000000000, 0) afterwards. */
 int fc_debug_set_wait_budget(long long cycles, int withhold_producers);
+/* With on != 0 the products on callers' streams find no memory for their scratch (restore with 0). */
+int fc_debug_withhold_scratch(int on);
 
 #ifdef __cplusplus
 }

@@ -1,5 +1,5 @@
 """The resident-weight linears on device pointers as a program strings them together: one call's output as the next one's
-operand on a stream."""
+operand on a stream, calls on several streams, captured calls, and what they keep."""
 import ctypes as C
 
 import numpy as np
@@ -7,6 +7,7 @@ import pytest
 
 import ferrum_cpu_b200 as fcb
 from ferrum_cpu_b200 import _lib, engine, synth
+from tests.test_timeouts import short_waits_without_producers
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +44,124 @@ def test_single_row_bias_is_the_output_of_the_call_ahead(make, n, k_long):
     assert np.abs(y2.cpu().numpy() - want).max() <= 24 * 2.0 ** -24 * 4 * np.abs(want).max()
     w1.close()
     w2.close()
+
+
+def run_linear(w, x, bias, y, math_mode, stream):
+    args = (x.data_ptr(), bias.data_ptr(), y.data_ptr(), x.shape[0])
+    s = C.c_void_p(stream.cuda_stream)
+    w.linear_dev(*args, stream=s) if isinstance(w, engine.RowQWeight) else w.linear_dev(*args, math_mode, s)
+
+
+# largest error over the largest result against f64, as test_gemm_tiles.py has it for the two math modes
+KINDS = [(q8_weight, _lib.FC_MATH_FP32, 2e-6), (q8_weight, _lib.FC_MATH_BF16X3, 3e-5), (rowq_weight, None, 2e-6)]
+
+
+def close_to(y, x, f, tol):
+    want = x.double().cpu().numpy() @ f.T
+    return np.abs(y.cpu().numpy() - want).max() <= tol * np.abs(want).max()
+
+
+@pytest.mark.parametrize("make,math_mode,tol", KINDS)
+def test_calls_on_two_streams_share_nothing(make, math_mode, tol):
+    """The same weight on two streams without an order between them, with rows of their own."""
+    import torch
+
+    n, k, m = 640, 1024, 2048
+    w, f = make(n, k, 3)
+    xs = [[torch.randn(m, k, device="cuda") for _ in range(6)] for _ in range(2)]
+    ys = [[torch.zeros(m, n, device="cuda") for _ in range(6)] for _ in range(2)]
+    zero, streams = torch.zeros(n, device="cuda"), [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for i in range(6):
+        for s in range(2):
+            run_linear(w, xs[s][i], zero, ys[s][i], math_mode, streams[s])
+    torch.cuda.synchronize()
+    assert all(close_to(ys[s][i], xs[s][i], f, tol) for s in range(2) for i in range(6))
+    w.close()
+
+
+@pytest.mark.parametrize("make,math_mode,tol", KINDS)
+def test_first_call_may_be_captured(make, math_mode, tol):
+    import torch
+
+    n, k, m = 300, 512, 77
+    w, f = make(n, k, 4)
+    x, zero, y = torch.randn(m, k, device="cuda"), torch.zeros(n, device="cuda"), torch.zeros(m, n, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run_linear(w, x, zero, y, math_mode, torch.cuda.current_stream())
+    for _ in range(3):
+        x.normal_()
+        graph.replay()
+        run_linear(w, torch.randn(4 * m, k, device="cuda"), zero, torch.empty(4 * m, n, device="cuda"), math_mode, torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        assert close_to(y, x, f, tol)
+    del graph
+    w.close()
+
+
+@pytest.mark.parametrize("make,math_mode,tol", KINDS)
+def test_without_memory_for_scratch_the_rows_run_one_by_one(make, math_mode, tol):
+    import torch
+
+    n, k, m = 129, 544, 9
+    w, f = make(n, k, 5)
+    x, zero, y = torch.randn(m, k, device="cuda"), torch.zeros(n, device="cuda"), torch.zeros(m, n, device="cuda")
+    _lib.lib().fc_debug_withhold_scratch(1)
+    try:
+        run_linear(w, x, zero, y, math_mode, torch.cuda.current_stream())
+    finally:
+        _lib.lib().fc_debug_withhold_scratch(0)
+    torch.cuda.synchronize()
+    assert close_to(y, x, f, tol)
+    w.close()
+
+
+def test_weights_share_a_bounded_scratch():
+    """Eight weights of 96 MiB of scratch a call: what stays allocated is the pool's 256 MiB at most, not a buffer per weight."""
+    import torch
+
+    n, k, m = 32, 4096, 4096
+    weights = [q8_weight(n, k, 6)[0] for _ in range(8)]
+    x, zero, y = torch.randn(m, k, device="cuda"), torch.zeros(n, device="cuda"), torch.zeros(m, n, device="cuda")
+    torch.cuda.synchronize()
+    free, _ = torch.cuda.mem_get_info()
+    for w in weights:
+        run_linear(w, x, zero, y, _lib.FC_MATH_FP32, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] <= (256 + 32) << 20
+    for w in weights:
+        w.close()
+
+
+@pytest.mark.parametrize("make,math_mode,tol", KINDS)
+def test_a_wait_that_ran_out_is_reported_by_the_next_call(make, math_mode, tol):
+    import torch
+
+    n, k, m = 256, 768, 300
+    w, f = make(n, k, 7)
+    x, zero, y = torch.randn(m, k, device="cuda"), torch.zeros(n, device="cuda"), torch.zeros(m, n, device="cuda")
+    stream = torch.cuda.current_stream()
+    with short_waits_without_producers():
+        run_linear(w, x, zero, y, math_mode, stream)
+        torch.cuda.synchronize()                             # the kernel has returned; the context is intact
+    with pytest.raises(fcb.FerrumCudaError) as e:
+        run_linear(w, x, zero, y, math_mode, stream)
+    assert e.value.code == _lib.FC_E_TIMEOUT
+    run_linear(w, x, zero, y, math_mode, stream)
+    torch.cuda.synchronize()
+    assert close_to(y, x, f, tol)
+    w.close()
+
+
+def test_host_entry_reports_a_wait_that_ran_out():
+    w, f = rowq_weight(256, 768, 8)
+    x = np.random.default_rng(8).standard_normal((300, 768)).astype(np.float32)
+    with short_waits_without_producers():
+        with pytest.raises(fcb.FerrumCudaError) as e:
+            w.linear(x, np.zeros(256, np.float32))
+        assert e.value.code == _lib.FC_E_TIMEOUT
+    want = x.astype(np.float64) @ f.T
+    assert np.abs(w.linear(x, np.zeros(256, np.float32)) - want).max() <= 2e-6 * np.abs(want).max()
+    w.close()
