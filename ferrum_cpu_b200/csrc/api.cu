@@ -237,12 +237,12 @@ struct fc_stream {
     int graph_nodes[2][3] = {};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_decode_ms = 0.0f;
-    // persistent decode kernel: exchange buffers, grid barrier word, status word
+    int* status = nullptr;                 // raised by a kernel of its prime or its steps whose bounded wait ran out
+    // persistent decode kernel: exchange buffers, grid barrier word
     float* qkv = nullptr;                  // the step's q | k | v row
     float2* stats = nullptr;               // softmax statistics of its logits
     float *partg = nullptr, *x1g = nullptr, *statg = nullptr;
     unsigned* bar = nullptr;
-    int* status = nullptr;
     int attn_splits = 1;
     int use_mega = 0;
     // fc_decode_batch: index of the parameter table (grid size) this stream's launches use, and
@@ -380,11 +380,11 @@ static int set_state(fc_stream* s, int pos, int fed, int tail, int eos, int keep
 static int read_state(fc_stream* s, StepState* out) {
     int status = 0;
     FC_CUDA(cudaMemcpyAsync(out, s->state, sizeof(StepState), cudaMemcpyDeviceToHost, s->m->st));
-    if (s->status) FC_CUDA(cudaMemcpyAsync(&status, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->m->st));
+    FC_CUDA(cudaMemcpyAsync(&status, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->m->st));
     FC_CUDA(cudaStreamSynchronize(s->m->st));
     if (status != 0) {
         cudaMemsetAsync(s->status, 0, sizeof(int), s->m->st);
-        return fail(FC_E_TIMEOUT, "a bounded wait inside the persistent decode kernel ran out (status %d)", status);
+        return fail(FC_E_TIMEOUT, "a bounded wait inside the prime or the persistent decode kernel ran out (status %d)", status);
     }
     return FC_OK;
 }
@@ -1056,6 +1056,8 @@ int fc_stream_create(fc_model* m, fc_stream** out) {
     if (rc == FC_OK) rc = a.alloc_n(&s->state, 1);
     if (rc == FC_OK) rc = a.alloc_n(&s->stats, kRowStats);
     if (rc == FC_OK) rc = a.alloc_n(&s->qkv, (size_t)3 * c.d_model);
+    if (rc == FC_OK) rc = a.alloc_n(&s->status, 1);
+    if (rc == FC_OK && cudaMemsetAsync(s->status, 0, sizeof(int), m->st) != cudaSuccess) rc = fail(FC_E_CUDA, "status word initialisation failed");
     if (rc == FC_OK && m->mega_grid > 0) {
         const int hd = c.d_model / c.n_head;
         s->attn_splits = std::max(1, std::min(8, m->mega_grid / c.n_head));
@@ -1063,8 +1065,6 @@ int fc_stream_create(fc_model* m, fc_stream** out) {
         if (rc == FC_OK) rc = a.alloc_n(&s->x1g, (size_t)c.d_model);
         if (rc == FC_OK) rc = a.alloc_n(&s->statg, (size_t)m->mega_grid * 4);
         if (rc == FC_OK) rc = a.alloc_n(&s->bar, 1);
-        if (rc == FC_OK) rc = a.alloc_n(&s->status, 1);
-        if (rc == FC_OK && cudaMemsetAsync(s->status, 0, sizeof(int), m->st) != cudaSuccess) rc = fail(FC_E_CUDA, "status word initialisation failed");
         if (rc == FC_OK) rc = a.alloc_n(&s->trace, (size_t)m->mega_grid * kTraceCap);
         s->use_mega = 1;
     }
@@ -1177,7 +1177,8 @@ static int prime_batched(fc_stream* const* ss, int S, int n, int last_mode, int*
     };
     Windows win;
     win.B = S; win.T = n;
-    FC_TRY(forward_blocks_with(m, win, R, m->ids_d, nullptr, planes, S == 1 && ss[0]->status ? ss[0]->status : m->tc_status, true, true, to_caches));
+    // a wait that runs out: fc_decode_batch reads the model's word, read_state the stream's
+    FC_TRY(forward_blocks_with(m, win, R, m->ids_d, nullptr, planes, kcs_dev ? m->tc_status : ss[0]->status, true, true, to_caches));
     *used = 1;
     for (int i = 0; i < S; ++i) {
         fc_stream* s = ss[i];
@@ -1763,7 +1764,11 @@ int fc_decode_batch(fc_model* m, int n_streams, const int32_t* prompts, int prom
             FC_TRY(batch_head_and_pick(m, batch_view(m, 0, S, 0, st), eos, b.x, nullptr, 0, nullptr, nullptr, 0));
         } else {
             // prompts too short for a window forward: token by token per stream; the last step selects token 1
-            for (int i = 0; i < S; ++i) FC_TRY(run_steps(wv[i], prompt_len, STEP_NOHEAD, STEP_SELECT));
+            for (int i = 0; i < S; ++i) {
+                StepState hs;
+                FC_TRY(run_steps(wv[i], prompt_len, STEP_NOHEAD, STEP_SELECT));
+                FC_TRY(read_state(wv[i], &hs));
+            }
             FC_TRY(launch_gather_first(b.queues, b.states, prompt_len, S, b.cur, b.done, b.n_out, b.out_tok, b.out_cap, b.pos, st));
         }
         FC_CUDA(cudaEventRecord(m->ev_prime, st));
@@ -1792,6 +1797,7 @@ int fc_decode_batch(fc_model* m, int n_streams, const int32_t* prompts, int prom
             FC_CUDA(cudaEventElapsedTime(&pm, w0 > 0 ? m->ev1 : m->ev0, m->ev_prime));
             m->last_batch_prime_ms += pm;
         }
+        if (used) FC_TRY(check_tc_status(m, "the prime of fc_decode_batch"));
         for (int i = 0; i < S; ++i)
             if (done[i] == 2) return fail(FC_E_CUDA, "fc_decode_batch: stream %d produced no finite logit", w0 + i);
         for (int i = 0; i < S; ++i) {

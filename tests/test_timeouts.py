@@ -81,3 +81,24 @@ def test_persistent_decode_times_out_and_recovers():
         assert np.abs(np.log(np.maximum(pg, 1e-12)) - np.log(np.maximum(po, 1e-12))).max() < 2e-4
     assert gm.cached_len() == 6
     gm.close()
+
+
+@pytest.mark.parametrize("ctx", [128, 1100])
+def test_prime_times_out_and_recovers(ctx):
+    """A prompt of one stream, on a model with the persistent kernel and on one without, and the prompts of a batch: each call
+    reports the wait itself and leaves nothing behind for the next one."""
+    sm = synth.SynthModel(1, 64, 2, 128, ctx, 96, seed=5, perturb=True)
+    gm, om = fcb.CudaSlm(sm.config, sm.weights), O.OracleModel(sm, threads=2)
+    ids = synth.token_ids(6, 33, 96)
+    prompts = np.stack([ids[:16], ids[16:32], ids[1:17]])
+    gm.decode_batch(prompts, 2)
+    for call in (lambda: gm.prime(ids), lambda: gm.generate_tokens(ids, 5), lambda: gm.decode_batch(prompts, 5)):
+        with short_waits_without_producers():
+            with pytest.raises(fcb.FerrumCudaError) as e:
+                call()
+            assert e.value.code == _lib.FC_E_TIMEOUT
+        gm.predict_next(ids)                         # the model's own status word is clear
+    assert np.array_equal(gm.generate_tokens(ids, 5)[0], om.generate_greedy(ids, 5)[0])
+    for got, p in zip(gm.decode_batch(prompts, 5), prompts):
+        assert np.array_equal(got, om.generate_greedy(p, 5)[0])
+    gm.close()
