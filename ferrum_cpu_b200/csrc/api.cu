@@ -244,7 +244,7 @@ struct fc_stream {
     float *partg = nullptr, *x1g = nullptr, *statg = nullptr;
     unsigned* bar = nullptr;
     int attn_splits = 1;
-    int use_mega = 0;
+    int mode = FC_DECODE_AUTO;
     // fc_decode_batch: index of the parameter table (grid size) this stream's launches use, and
     // the CUDA stream they go to (null: the model's)
     int table = 0;
@@ -350,7 +350,7 @@ static int run_mega(fc_stream* s, int n, int head_from, int select, int probs) {
 // n steps, the last one in `last_mode`, the ones before it in `mode`.
 static int run_steps(fc_stream* s, int n, int mode, int last_mode) {
     if (n <= 0) return FC_OK;
-    if (s->use_mega) {
+    if (s->m->mega_grid > 0 && s->mode != FC_DECODE_PER_KERNEL) {
         const int head_from = mode != STEP_NOHEAD ? 0 : (last_mode != STEP_NOHEAD ? n - 1 : n);
         return run_mega(s, n, head_from, last_mode == STEP_SELECT, last_mode == STEP_PROBS);
     }
@@ -358,10 +358,10 @@ static int run_steps(fc_stream* s, int n, int mode, int last_mode) {
     return FC_OK;
 }
 
-// n steps of a generation. The chain of dependent launches is ahead of the persistent kernel wherever it covers the model.
+// n steps of a generation. Left to itself (FC_DECODE_AUTO) it takes the chain of dependent launches; the persistent kernel where
+// it was asked for, and where its timeline was.
 static int decode_steps(fc_stream* s, int n, int mode) {
-    const fc_config& c = s->m->cfg;
-    if (!attn_step_covers(c.d_model / c.n_head, c.ctx)) return run_steps(s, n, mode, mode);
+    if (s->m->mega_grid > 0 && (s->mode == FC_DECODE_PERSISTENT || (s->mode == FC_DECODE_AUTO && s->trace_on))) return run_steps(s, n, mode, mode);
     for (; n >= kChainSteps; n -= kChainSteps) FC_TRY(run_step(s, mode, true));
     for (int i = 0; i < n; ++i) FC_TRY(run_step(s, mode));
     return FC_OK;
@@ -1066,7 +1066,6 @@ int fc_stream_create(fc_model* m, fc_stream** out) {
         if (rc == FC_OK) rc = a.alloc_n(&s->statg, (size_t)m->mega_grid * 4);
         if (rc == FC_OK) rc = a.alloc_n(&s->bar, 1);
         if (rc == FC_OK) rc = a.alloc_n(&s->trace, (size_t)m->mega_grid * kTraceCap);
-        s->use_mega = 1;
     }
     if (rc == FC_OK && (cudaEventCreate(&s->ev0) != cudaSuccess || cudaEventCreate(&s->ev1) != cudaSuccess)) rc = fail(FC_E_CUDA, "event creation failed");
     if (rc == FC_OK) rc = set_state(s, 0, 0, 0, -1, 0);
@@ -1125,8 +1124,8 @@ int fc_stream_set_mode(fc_stream* s, int mode) {
     if (!s) return fail(FC_E_ARG, "fc_stream_set_mode: null stream");
     if (mode == FC_DECODE_PERSISTENT && s->m->mega_grid <= 0)
         return fail(FC_E_SHAPE, "the persistent decode kernel does not support this model shape");
-    if (mode != FC_DECODE_PERSISTENT && mode != FC_DECODE_PER_KERNEL) return fail(FC_E_ARG, "unknown decode mode %d", mode);
-    s->use_mega = mode == FC_DECODE_PERSISTENT;
+    if (mode != FC_DECODE_PERSISTENT && mode != FC_DECODE_PER_KERNEL && mode != FC_DECODE_AUTO) return fail(FC_E_ARG, "unknown decode mode %d", mode);
+    s->mode = mode;
     return FC_OK;
 }
 float fc_last_decode_ms(const fc_stream* s) { return s ? s->last_decode_ms : 0.0f; }

@@ -283,7 +283,8 @@ class CudaSlm:
         return t if absolute or not n else t - t[0]
 
     def set_decode_mode(self, mode):
-        """0: persistent decode kernel (default), 1: one kernel per layer operation."""
+        """0: persistent decode kernel, 1: chain of launches, 2: the chain for generations and the persistent kernel for feeds (a
+        new stream)."""
         check(_lib.lib().fc_stream_set_mode(self._stream(), mode))
 
     def cached_len(self):

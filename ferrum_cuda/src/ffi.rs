@@ -20,6 +20,7 @@ pub const FC_MATH_FP32: c_int = 0;
 pub const FC_MATH_BF16X3: c_int = 1;
 pub const FC_DECODE_PERSISTENT: c_int = 0;
 pub const FC_DECODE_PER_KERNEL: c_int = 1;
+pub const FC_DECODE_AUTO: c_int = 2;
 pub const FC_ROPE_NORM: c_int = 0;
 pub const FC_ROPE_NEOX: c_int = 1;
 pub const FC_GGML_Q4_0: c_int = 2;

@@ -267,13 +267,17 @@ int fc_predict_next(fc_model* m, const int32_t* ids, int n, float* probs);
 int fc_stream_create(fc_model* m, fc_stream** out);   /* cached.rs:45-64 try_new */
 void fc_stream_free(fc_stream* s);
 int fc_stream_reset(fc_stream* s);                    /* cached.rs:93-98 */
-/* How fc_feed / fc_prime / fc_generate_greedy run a token on the GPU. Both compute the same
- * CachedTransformer::feed; the per-kernel form exists to cross-check the persistent one.
- *   FC_DECODE_PERSISTENT: one cooperative kernel per batch of tokens (default when the model
- *                         shape fits it: d_model <= 1024, d_ff <= 4096, ctx <= 1024);
- *   FC_DECODE_PER_KERNEL: one kernel per layer operation, replayed from a CUDA graph. */
+/* How fc_feed / fc_prime / fc_generate_greedy / fc_generate_sampled run a token on the GPU. Both forms
+ * compute the same CachedTransformer::feed.
+ *   FC_DECODE_PERSISTENT: one cooperative kernel per batch of tokens, for every token (model shapes that
+ *                         fit it: d_model <= 1024, d_ff <= 4096, ctx <= 1024; FC_E_SHAPE otherwise);
+ *   FC_DECODE_PER_KERNEL: a chain of dependent launches, five per block, replayed from a CUDA graph;
+ *   FC_DECODE_AUTO (a new stream): the chain for the tokens of a generation, and for the rest the
+ *                         persistent kernel where the shape fits it. With tracing on, generations take
+ *                         the persistent kernel too. */
 #define FC_DECODE_PERSISTENT 0
 #define FC_DECODE_PER_KERNEL 1
+#define FC_DECODE_AUTO 2
 int fc_stream_set_mode(fc_stream* s, int mode);
 /* Tracing (the reference's per-layer verbose log, verbose.rs:11-110, has no timing; this is
  * its device-side counterpart). When on, the persistent decode kernel records the GPU's

@@ -42,3 +42,31 @@ def test_rotary_steps_match_the_oracle_past_the_held_rows(hd, heads, kv, rope_di
     for t, tok in enumerate(synth.token_ids(2, 400, 515)):
         got, want = gm.forward_one(tok, cache), om.forward_one(tok)
         assert np.abs(got - want).max() < 2e-4, t
+
+
+def test_generation_runs_in_the_mode_it_was_asked_for():
+    """fc_stream_set_mode holds for generations: one cooperative launch per batch of tokens, or a chain of launches per token; a
+    new stream takes the chain, and the persistent kernel while its timeline is recorded."""
+    sm = synth.named("tiny", seed=0, perturb=True)
+    gm = fcb.CudaSlm(sm.config, sm.weights)
+    prompt = synth.token_ids(17, 9, sm.dims[5])          # primed as a window: every traced token is a generated one
+    tokens, launches = {}, {}
+    gm.reset()                                           # makes the stream
+    for mode in (None, 0, 1, 2):
+        if mode is not None:
+            gm.set_decode_mode(mode)
+        fcb.take_launch_count()
+        tokens[mode] = list(gm.generate_tokens(prompt, 24)[0])
+        launches[mode] = fcb.take_launch_count()
+    assert tokens[None] == tokens[0] == tokens[1] == tokens[2]
+    per_token = 5 * sm.dims[0] + 3                       # embedding, five a block, head, pick
+    assert launches[None] == launches[1] == launches[2] >= 24 * per_token
+    assert launches[1] - launches[0] >= 23 * per_token   # 24 feeds in one launch
+    for mode, traced in ((2, True), (0, True), (1, False)):
+        gm.set_decode_mode(mode)
+        gm.set_trace(True)
+        fcb.take_launch_count()
+        gm.generate_tokens(prompt, 24)
+        gm.set_trace(False)
+        assert (fcb.take_launch_count() < launches[1]) == traced
+    gm.close()
