@@ -233,8 +233,9 @@ struct fc_stream {
     int queue_cap = 0;
     StepState* state = nullptr;
     int host_pos = 0;
-    cudaGraphExec_t graph[2][3] = {};   // [one step, kChainSteps steps][mode]
-    int graph_nodes[2][3] = {};
+    cudaGraphExec_t graph[2][2][3] = {};   // [heads with a CTA each, shared ones][one step, kChainSteps steps][mode]
+    int graph_nodes[2][2][3] = {};
+    int attn_split = 1, split_from = 0;    // CTAs that share a head from position split_from on
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_decode_ms = 0.0f;
     int* status = nullptr;                 // raised by a kernel of its prime or its steps whose bounded wait ran out
@@ -274,7 +275,7 @@ static int launch_head(fc_stream* s, const float* x, int mode) {
 // -> TransformerBlock::forward_with_cache (transformer.rs:221-294). LayerNorm is the prologue of the product that reads it,
 // bias, GELU and residual are epilogues, and the weights of a kernel are asked for while the one ahead of it runs. The
 // embedding starts when everything ahead of it is complete, so the attention may read state and caches early.
-static int launch_step(fc_stream* s, int mode) {
+static int launch_step(fc_stream* s, int mode, int split) {
     fc_model* m = s->m;
     const fc_config& c = m->cfg;
     cudaStream_t st = m->st;
@@ -285,7 +286,7 @@ static int launch_step(fc_stream* s, int mode) {
         const LayerDev& L = m->layers[l];
         FC_TRY(launch_gemv_row(L.qkv, s->x, RowNorm{L.ln1g, L.ln1b, 1e-5f}, L.qkv_b, nullptr, EPI_NONE, s->qkv, s->state, st));
         FC_TRY(launch_attn_step(s->qkv, c.n_head, c.n_head, hd, 0, 0, nullptr, 1.0f, s->kc + l * layer_stride, s->vc + l * layer_stride, c.ctx,
-                                s->state, s->att, st));
+                                split, s->state, s->att, st));
         FC_TRY(launch_gemv_row(L.out, s->att, RowNorm(), L.out_b, s->x, EPI_NONE, s->x, s->state, st));
         FC_TRY(launch_gemv_row(L.up, s->x, RowNorm{L.ln2g, L.ln2b, 1e-5f}, L.up_b, nullptr, EPI_GELU, s->hid, s->state, st));
         FC_TRY(launch_gemv_row(L.down, s->hid, RowNorm(), L.down_b, s->x, EPI_NONE, s->x, s->state, st));
@@ -296,18 +297,21 @@ static int launch_step(fc_stream* s, int mode) {
 
 // The launch-bound step is captured once per mode into a CUDA graph and replayed; every
 // per-step quantity (token, position) is read from device state, so no node is updated.
+// pos: the position of the (first) step, which decides how many CTAs a head has.
 constexpr int kChainSteps = 8;
-static int run_step(fc_stream* s, int mode, bool several = false) {
-    cudaGraphExec_t& graph = s->graph[several][mode];
+static int run_step(fc_stream* s, int mode, int pos, bool several = false) {
+    const bool shared = pos + (several ? kChainSteps : 1) > s->split_from;
+    cudaGraphExec_t& graph = s->graph[shared][several][mode];
+    int& nodes = s->graph_nodes[shared][several][mode];
     if (!graph) {
         cudaStream_t st = s->m->st;
         cudaGraph_t g = nullptr;
         const int64_t before = g_launches;
         FC_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         int rc = FC_OK;
-        for (int i = 0; i < (several ? kChainSteps : 1) && rc == FC_OK; ++i) rc = launch_step(s, mode);
+        for (int i = 0; i < (several ? kChainSteps : 1) && rc == FC_OK; ++i) rc = launch_step(s, mode, shared ? s->attn_split : 1);
         const cudaError_t e = cudaStreamEndCapture(st, &g);
-        s->graph_nodes[several][mode] = (int)(g_launches - before);
+        nodes = (int)(g_launches - before);
         g_launches = before;
         if (rc != FC_OK) { if (g) cudaGraphDestroy(g); return rc; }
         FC_CUDA(e);
@@ -316,7 +320,7 @@ static int run_step(fc_stream* s, int mode, bool several = false) {
         FC_CUDA(ei);
     }
     FC_CUDA(cudaGraphLaunch(graph, s->m->st));
-    g_launches += s->graph_nodes[several][mode];
+    g_launches += nodes;
     return FC_OK;
 }
 
@@ -347,23 +351,23 @@ static int run_mega(fc_stream* s, int n, int head_from, int select, int probs) {
     return launch_decode_mega(p, tab.grid, st);
 }
 
-// n steps, the last one in `last_mode`, the ones before it in `mode`.
-static int run_steps(fc_stream* s, int n, int mode, int last_mode) {
+// n steps from position pos on, the last one in `last_mode`, the ones before it in `mode`.
+static int run_steps(fc_stream* s, int n, int mode, int last_mode, int pos) {
     if (n <= 0) return FC_OK;
     if (s->m->mega_grid > 0 && s->mode != FC_DECODE_PER_KERNEL) {
         const int head_from = mode != STEP_NOHEAD ? 0 : (last_mode != STEP_NOHEAD ? n - 1 : n);
         return run_mega(s, n, head_from, last_mode == STEP_SELECT, last_mode == STEP_PROBS);
     }
-    for (int i = 0; i < n; ++i) FC_TRY(run_step(s, i + 1 == n ? last_mode : mode));
+    for (int i = 0; i < n; ++i) FC_TRY(run_step(s, i + 1 == n ? last_mode : mode, pos + i));
     return FC_OK;
 }
 
-// n steps of a generation. Left to itself (FC_DECODE_AUTO) it takes the chain of dependent launches; the persistent kernel where
+// n steps of a generation from position pos on. Left to itself (FC_DECODE_AUTO) it takes the chain of dependent launches; the persistent kernel where
 // it was asked for, and where its timeline was.
-static int decode_steps(fc_stream* s, int n, int mode) {
-    if (s->m->mega_grid > 0 && (s->mode == FC_DECODE_PERSISTENT || (s->mode == FC_DECODE_AUTO && s->trace_on))) return run_steps(s, n, mode, mode);
-    for (; n >= kChainSteps; n -= kChainSteps) FC_TRY(run_step(s, mode, true));
-    for (int i = 0; i < n; ++i) FC_TRY(run_step(s, mode));
+static int decode_steps(fc_stream* s, int n, int mode, int pos) {
+    if (s->m->mega_grid > 0 && (s->mode == FC_DECODE_PERSISTENT || (s->mode == FC_DECODE_AUTO && s->trace_on))) return run_steps(s, n, mode, mode, pos);
+    for (; n >= kChainSteps; n -= kChainSteps, pos += kChainSteps) FC_TRY(run_step(s, mode, pos, true));
+    for (int i = 0; i < n; ++i) FC_TRY(run_step(s, mode, pos + i));
     return FC_OK;
 }
 
@@ -1058,8 +1062,9 @@ int fc_stream_create(fc_model* m, fc_stream** out) {
     if (rc == FC_OK) rc = a.alloc_n(&s->qkv, (size_t)3 * c.d_model);
     if (rc == FC_OK) rc = a.alloc_n(&s->status, 1);
     if (rc == FC_OK && cudaMemsetAsync(s->status, 0, sizeof(int), m->st) != cudaSuccess) rc = fail(FC_E_CUDA, "status word initialisation failed");
+    const int hd = c.d_model / c.n_head;
+    if (rc == FC_OK) rc = attn_step_split(c.n_head, hd, c.ctx, &s->attn_split, &s->split_from);
     if (rc == FC_OK && m->mega_grid > 0) {
-        const int hd = c.d_model / c.n_head;
         s->attn_splits = std::max(1, std::min(8, m->mega_grid / c.n_head));
         rc = a.alloc_n(&s->partg, (size_t)c.n_head * s->attn_splits * (hd + 2));
         if (rc == FC_OK) rc = a.alloc_n(&s->x1g, (size_t)c.d_model);
@@ -1081,8 +1086,9 @@ void fc_stream_free(fc_stream* s) {
     cudaStreamSynchronize(s->m->st);
     if (s->cs) { cudaStreamSynchronize(s->cs); cudaStreamDestroy(s->cs); }
     if (s->cs_done) cudaEventDestroy(s->cs_done);
-    for (auto& set : s->graph)
-        for (cudaGraphExec_t g : set) if (g) cudaGraphExecDestroy(g);
+    for (auto& form : s->graph)
+        for (auto& set : form)
+            for (cudaGraphExec_t g : set) if (g) cudaGraphExecDestroy(g);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     s->arena.release();
@@ -1200,7 +1206,7 @@ static int feed_queued(fc_stream* s, int n, int last_mode) {
     int used = 0;
     FC_TRY(prime_batched(&s, 1, n, last_mode, &used));
     if (used) return FC_OK;
-    return run_steps(s, n, STEP_NOHEAD, last_mode);
+    return run_steps(s, n, STEP_NOHEAD, last_mode, s->host_pos);
 }
 
 static int feed_ids(fc_stream* s, const int32_t* ids, int n, float* probs) {
@@ -1301,11 +1307,11 @@ int fc_generate_greedy(fc_stream* s, const int32_t* prompt, int n, int max_new, 
             // selecting feeds i..max_new-1, as many as stay inside the context
             const int k = std::min(std::min(max_new - i, 32), cap - win_start_len - gen_win + 1);
             if (k >= 1) {
-                FC_TRY(decode_steps(s, k, STEP_SELECT));
+                FC_TRY(decode_steps(s, k, STEP_SELECT, win_start_len + gen_win - 1));
                 gen_win += k;
                 i += k;
             } else {
-                FC_TRY(decode_steps(s, 1, STEP_PROBS));   // the last feed selects nothing
+                FC_TRY(decode_steps(s, 1, STEP_PROBS, win_start_len + gen_win - 1));   // the last feed selects nothing
                 i += 1;
             }
         }
@@ -1388,7 +1394,7 @@ int fc_generate_sampled(fc_stream* s, const int32_t* prompt, int n, int max_new,
             // the feed (or re-prime) after the last requested token keeps the stream continuable, as the reference's call
             // order does, but its distribution is not used here: it stays outside the timed region
             if (made + i == max_new) { FC_CUDA(cudaEventRecord(s->ev1, st)); timed = true; }
-            if (feed) FC_TRY(decode_steps(s, 1, STEP_PROBS));   // feed(next): the distribution of the token after it
+            if (feed) FC_TRY(decode_steps(s, 1, STEP_PROBS, (int)window.size() + i - 1));   // feed(next): the distribution of the token after it
         }
         return FC_OK;
     };
@@ -1765,7 +1771,7 @@ int fc_decode_batch(fc_model* m, int n_streams, const int32_t* prompts, int prom
             // prompts too short for a window forward: token by token per stream; the last step selects token 1
             for (int i = 0; i < S; ++i) {
                 StepState hs;
-                FC_TRY(run_steps(wv[i], prompt_len, STEP_NOHEAD, STEP_SELECT));
+                FC_TRY(run_steps(wv[i], prompt_len, STEP_NOHEAD, STEP_SELECT, 0));
                 FC_TRY(read_state(wv[i], &hs));
             }
             FC_TRY(launch_gather_first(b.queues, b.states, prompt_len, S, b.cur, b.done, b.n_out, b.out_tok, b.out_cap, b.pos, st));

@@ -162,11 +162,14 @@ inline int launch_gemv_row(const QMat& w, const float* x, const RowNorm& norm, c
     return launch_gemv_row(&p, 1, w.K, x, norm, residual, epi, state, st, stats, n_stats);
 }
 
-// attn_step.cu — one attention step over the caches, one CTA per query head; ftab null: no rotation. The state and the cached
-// rows are read ahead of its wait: some kernel of the step before it has to wait for all of the step before.
+// attn_step.cu — one attention step over the caches, `split` CTAs per query head; ftab null: no rotation. The state and the
+// cached rows are read ahead of its wait: some kernel of the step before it has to wait for all of the step before.
+// attn_step_split: the CTAs that share a head at long positions (1: it stays with one), and the position from which on that is
+// the faster form; either form takes every position.
 bool attn_step_covers(int hd, int ctx);
+int attn_step_split(int n_q, int hd, int ctx, int* split, int* from);
 int launch_attn_step(const float* qkv, int n_q, int n_kv, int hd, int rope_dim, int neox, const float2* ftab, float inv_linear,
-                     float* kc, float* vc, int ctx, const StepState* state, float* out, cudaStream_t st);
+                     float* kc, float* vc, int ctx, int split, const StepState* state, float* out, cudaStream_t st);
 
 // An f32 matrix as n bf16 planes whose sum it is: 2 planes hold it to 2^-17 relative (FC_MATH_BF16X3), 3 exactly
 // (FC_MATH_FP32). The form in which activations reach the tensor cores.

@@ -70,8 +70,10 @@ struct fc_llama_cache {
     StepState* state = nullptr;
     int* status = nullptr;                // raised by a kernel whose bounded wait ran out
     int host_pos = 0;
-    cudaGraphExec_t graph[3] = {};   // [0]: step without the head, [1]: with it, [2]: kFreeSteps times the greedy pick and [1]
-    int graph_nodes[3] = {};
+    // [heads with a CTA each, shared ones][0: step without the head, 1: with it, 2: kFreeSteps times the greedy pick and 1]
+    cudaGraphExec_t graph[2][3] = {};
+    int graph_nodes[2][3] = {};
+    int attn_split = 1, split_from = 0;     // CTAs that share a head from position split_from on
     bool packed_warm[2] = {false, false};   // packed model: the uncaptured first step of each kind has run
     unsigned long long* rng_d = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -349,20 +351,21 @@ int check_window(const fc_llama* m, int window) {
     return FC_OK;
 }
 
-int launch_attention(fc_llama_cache* s, float* kc, float* vc) {
+int launch_attention(fc_llama_cache* s, float* kc, float* vc, int split) {
     fc_llama* m = s->m;
     const fc_llama_config& c = m->cfg;
-    auto go = attn_step_covers(c.head_dim, c.ctx) ? launch_attn_step : launch_llama_attn_decode;
-    return go(s->qkv, c.n_head, c.n_kv_head, c.head_dim, c.rope_dim, c.rope_type == FC_ROPE_NEOX, m->ftab, m->inv_linear, kc, vc, c.ctx,
-              s->state, s->att, m->st);
+    if (attn_step_covers(c.head_dim, c.ctx))
+        return launch_attn_step(s->qkv, c.n_head, c.n_kv_head, c.head_dim, c.rope_dim, c.rope_type == FC_ROPE_NEOX, m->ftab, m->inv_linear,
+                                kc, vc, c.ctx, split, s->state, s->att, m->st);
+    return launch_llama_attn_decode(s->qkv, c.n_head, c.n_kv_head, c.head_dim, c.rope_dim, c.rope_type == FC_ROPE_NEOX, m->ftab, m->inv_linear,
+                                    kc, vc, c.ctx, s->state, s->att, m->st);
 }
-
 
 // ---------------------------------------------------------------------------- decode step
 // LlamaModel::forward_one (llm.rs:610-618) -> LlamaBlock::forward_one (llm.rs:451-461) as a
 // kernel sequence; every per-step quantity is read from device state so the captured graph is
 // replayed unchanged.
-int launch_step(fc_llama_cache* s, int with_head) {
+int launch_step(fc_llama_cache* s, int with_head, int split) {
     fc_llama* m = s->m;
     const fc_llama_config& c = m->cfg;
     cudaStream_t st = m->st;
@@ -374,7 +377,7 @@ int launch_step(fc_llama_cache* s, int with_head) {
         float* vc = s->vc + l * layer_stride;
         // RMSNorm rides in the prologue of the projection that reads it, SwiGLU in the epilogue of gate/up
         FC_TRY(launch_gemv_row(L.qkv, s->x, RowNorm{L.attn_norm, nullptr, c.norm_eps}, L.qkv_b, nullptr, EPI_NONE, s->qkv, s->state, st));
-        FC_TRY(launch_attention(s, kc, vc));
+        FC_TRY(launch_attention(s, kc, vc, split));
         FC_TRY(launch_gemv_row(L.wo, s->att, RowNorm(), nullptr, s->x, EPI_NONE, s->x, s->state, st));
         FC_TRY(launch_gemv_row(L.gateup, s->x, RowNorm{L.ffn_norm, nullptr, c.norm_eps}, nullptr, nullptr, EPI_SWIGLU, s->hid, s->state, st));
         FC_TRY(launch_gemv_row(L.down, s->hid, RowNorm(), nullptr, s->x, EPI_NONE, s->x, s->state, st));
@@ -386,7 +389,7 @@ int launch_step(fc_llama_cache* s, int with_head) {
 
 // The same step on the packed model, one kernel per operation. The first step of a cache runs uncaptured, so that the
 // packed linears' single-row scratch exists before the step is captured.
-int launch_step_packed(fc_llama_cache* s, int with_head) {
+int launch_step_packed(fc_llama_cache* s, int with_head, int split) {
     fc_llama* m = s->m;
     const fc_llama_config& c = m->cfg;
     cudaStream_t st = m->st;
@@ -406,14 +409,14 @@ int launch_step_packed(fc_llama_cache* s, int with_head) {
             rowq_part(P.up.rq, nullptr, s->hid, &gu[1]) && rowq_part(P.down.rq, nullptr, s->x, &down)) {
             // five kernels, as the Q8_0 step: the norms are prologues, SwiGLU and the residual epilogues
             FC_TRY(launch_gemv_row(in, 3, c.d_model, s->x, RowNorm{L.attn_norm, nullptr, c.norm_eps}, nullptr, EPI_NONE, s->state, st));
-            FC_TRY(launch_attention(s, kc, vc));
+            FC_TRY(launch_attention(s, kc, vc, split));
             FC_TRY(launch_gemv_row(&wo, 1, m->q_dim, s->att, RowNorm(), s->x, EPI_NONE, s->state, st));
             FC_TRY(launch_gemv_row(gu, 2, c.d_model, s->x, RowNorm{L.ffn_norm, nullptr, c.norm_eps}, nullptr, EPI_SWIGLU, s->state, st));
             FC_TRY(launch_gemv_row(&down, 1, c.d_ff, s->hid, RowNorm(), s->x, EPI_NONE, s->state, st));
             continue;
         }
         FC_TRY(packed_block(m, l, 1, s->x, s->n, s->qkv, s->att, s->gu, s->hid, nullptr, [&]() -> int {
-            return launch_attention(s, kc, vc);
+            return launch_attention(s, kc, vc, split);
         }));
     }
     if (with_head) {
@@ -431,13 +434,18 @@ int launch_step_packed(fc_llama_cache* s, int with_head) {
 // Greedy tokens that need nothing from the host share a graph: between two graphs the GPU waits for the next one's launch.
 constexpr int kFreeSteps = 8;
 
-int run_graph(fc_llama_cache* s, int which) {
-    if (!s->graph[which]) {
+// pos: the position of the (first) step
+int run_graph(fc_llama_cache* s, int which, int pos) {
+    const bool shared = pos + (which == 2 ? kFreeSteps : 1) > s->split_from;
+    cudaGraphExec_t& graph = s->graph[shared][which];
+    int& nodes = s->graph_nodes[shared][which];
+    if (!graph) {
         const fc_llama* m = s->m;
         cudaStream_t st = m->st;
         cudaGraph_t g = nullptr;
         const int64_t before = g_launches;
-        auto step = [&](int with_head) { return m->prec >= 0 ? launch_step_packed(s, with_head) : launch_step(s, with_head); };
+        const int split = shared ? s->attn_split : 1;
+        auto step = [&](int with_head) { return m->prec >= 0 ? launch_step_packed(s, with_head, split) : launch_step(s, with_head, split); };
         FC_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         int rc = FC_OK;
         if (which < 2) rc = step(which);
@@ -446,25 +454,25 @@ int run_graph(fc_llama_cache* s, int which) {
             if (rc == FC_OK) rc = step(1);
         }
         const cudaError_t e = cudaStreamEndCapture(st, &g);
-        s->graph_nodes[which] = (int)(g_launches - before);
+        nodes = (int)(g_launches - before);
         g_launches = before;
         if (rc != FC_OK) { if (g) cudaGraphDestroy(g); return rc; }
         FC_CUDA(e);
-        const cudaError_t ei = cudaGraphInstantiate(&s->graph[which], g, 0);
+        const cudaError_t ei = cudaGraphInstantiate(&graph, g, 0);
         cudaGraphDestroy(g);
         FC_CUDA(ei);
     }
-    FC_CUDA(cudaGraphLaunch(s->graph[which], s->m->st));
-    g_launches += s->graph_nodes[which];
+    FC_CUDA(cudaGraphLaunch(graph, s->m->st));
+    g_launches += nodes;
     return FC_OK;
 }
 
-int run_step(fc_llama_cache* s, int with_head) {
+int run_step(fc_llama_cache* s, int with_head, int pos) {
     if (s->m->prec >= 0 && !s->packed_warm[with_head]) {
         s->packed_warm[with_head] = true;
-        return launch_step_packed(s, with_head);
+        return launch_step_packed(s, with_head, pos + 1 > s->split_from ? s->attn_split : 1);
     }
-    return run_graph(s, with_head);
+    return run_graph(s, with_head, pos);
 }
 
 __global__ void llama_set_state_kernel(StepState* st, int pos, int fed, int tail) {
@@ -491,7 +499,7 @@ int feed_ids(fc_llama_cache* s, const int32_t* ids, int n, int head_on_last) {
     FC_CUDA(cudaMemcpyAsync(s->queue + s->host_pos, ids, (size_t)n * 4, cudaMemcpyHostToDevice, m->st));
     llama_set_state_kernel<<<1, 1, 0, m->st>>>(s->state, s->host_pos, s->host_pos, s->host_pos + n);
     FC_LAUNCHED();
-    for (int i = 0; i < n; ++i) FC_TRY(run_step(s, head_on_last && i + 1 == n));
+    for (int i = 0; i < n; ++i) FC_TRY(run_step(s, head_on_last && i + 1 == n, s->host_pos + i));
     s->host_pos += n;
     return FC_OK;
 }
@@ -818,6 +826,7 @@ int fc_llama_cache_create(fc_llama* m, fc_llama_cache** out) {
         FC_TRY(a.alloc_n(&s->state, 1));
         FC_TRY(a.alloc_n(&s->status, 1));
         FC_CUDA(cudaMemsetAsync(s->status, 0, sizeof(int), m->st));
+        FC_TRY(attn_step_split(c.n_head, c.head_dim, c.ctx, &s->attn_split, &s->split_from));
         FC_TRY(a.alloc_n(&s->rng_d, 1));
         FC_CUDA(cudaEventCreate(&s->ev0));
         FC_CUDA(cudaEventCreate(&s->ev1));
@@ -833,7 +842,8 @@ void fc_llama_cache_free(fc_llama_cache* s) {
     if (!s) return;
     cudaSetDevice(s->device);
     cudaDeviceSynchronize();              // the model (and its stream) may already be gone
-    for (auto& g : s->graph) if (g) cudaGraphExecDestroy(g);
+    for (auto& form : s->graph)
+        for (cudaGraphExec_t g : form) if (g) cudaGraphExecDestroy(g);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     s->arena.release();
@@ -912,7 +922,7 @@ int fc_llama_generate(fc_llama_cache* s, const int32_t* prompt, int n, int max_n
         if (cancel && *cancel) { cancelled = true; break; }
         // all but the last tokens of a free run, once a packed step has run uncaptured
         if (free_run && max_new - made > kFreeSteps && (m->prec < 0 || s->packed_warm[1])) {
-            rc = run_graph(s, 2);
+            rc = run_graph(s, 2, s->host_pos);
             if (rc != FC_OK) break;
             made += kFreeSteps;
             s->host_pos += kFreeSteps;
@@ -936,7 +946,7 @@ int fc_llama_generate(fc_llama_cache* s, const int32_t* prompt, int n, int max_n
         // the forward of the last requested token keeps the cache continuable (llm.rs:750-751); its logits are not used
         // here, so it stays outside the timed region
         if (made == max_new) { FC_CUDA(cudaEventRecord(s->ev1, st)); timed = true; }
-        rc = run_step(s, 1);                                 // forward_one(next), the last token included (llm.rs:750-751)
+        rc = run_step(s, 1, s->host_pos);                    // forward_one(next), the last token included (llm.rs:750-751)
         if (rc != FC_OK) break;
         s->host_pos += 1;
     }

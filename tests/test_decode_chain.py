@@ -11,10 +11,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("d,heads,ff,ctx,prompt,new", [(32, 1, 64, 16, 1, 14), (96, 3, 160, 64, 60, 9), (64, 1, 96, 512, 345, 20),
-                                                      (256, 4, 4128, 40, 17, 20)])
+                                                      (256, 4, 4128, 40, 17, 20), (64, 1, 96, 1024, 889, 12), (96, 3, 64, 1024, 1010, 10)])
 def test_decode_chain_at_its_edges(d, heads, ff, ctx, prompt, new):
-    """Greedy tokens of the decode chain against the oracle: heads of 32 and 64, the first positions, caches that outgrow
-    the rows the attention holds in shared memory, a window that slides, rows wider than one slice and odd vocabularies."""
+    """Greedy tokens of the decode chain against the oracle: heads of 32 and 64, the first positions, caches long enough
+    for several CTAs a head, a window that slides, rows wider than one slice and odd vocabularies."""
     sm = synth.SynthModel(2, d, heads, ff, ctx, 515, seed=d + ff, perturb=True)
     om, gm = O.OracleModel(sm), fcb.CudaSlm(sm.config, sm.weights)
     window, want = list(synth.token_ids(4, prompt, 515)), []
