@@ -1384,9 +1384,9 @@ int fc_generate_sampled(fc_stream* s, const int32_t* prompt, int n, int max_new,
     bool cancelled = false, timed = false;
     int rc = FC_OK;
     // A draw appends its token to the queue on the device (or raises `done` on eos, which turns what follows into no-ops) and
-    // the feed reads it there, so the host reads back once per kDrawBatch draws; it polls `cancel` as often. A draw that
-    // makes the window outgrow the context goes alone: its re-prime starts on the host.
-    constexpr int kDrawBatch = 16;
+    // the feed reads it there, so the host reads back once per `batch` draws; with a cancel flag, which is polled before every
+    // draw, that is each one. A draw that makes the window outgrow the context goes alone: its re-prime starts on the host.
+    const int batch = cancel ? 1 : 16;
     auto draw = [&]() { return launch_sample(s->probs, c.vocab, 1, *params, s->queue, 0, s->rng_d, s->queue, s->queue_cap, s->state, nullptr, st); };
     auto issue = [&](int k, bool feed) -> int {
         for (int i = 1; i <= k; ++i) {
@@ -1414,7 +1414,7 @@ int fc_generate_sampled(fc_stream* s, const int32_t* prompt, int n, int max_new,
     };
     while (made < max_new) {
         if (cancel && *cancel) { cancelled = true; break; }
-        const int k = std::min(std::min(max_new - made, kDrawBatch), cap - (int)window.size());
+        const int k = std::min(std::min(max_new - made, batch), cap - (int)window.size());
         bool done = false;
         rc = issue(std::max(k, 1), k > 0);
         if (rc == FC_OK) rc = harvest(&done);

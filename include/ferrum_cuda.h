@@ -299,7 +299,7 @@ int fc_prime(fc_stream* s, const int32_t* ids, int n, float* probs);
 /* token_stream.rs:66-189 with temperature <= 0: keep the last ctx prompt ids, prime, then
  * per step argmax_first(ln(max(p,1e-12))) (sampling.rs:96-104,147), stop before emitting
  * `eos` (pass -1 for none), re-prime on the last ctx/2 ids when the window outgrows ctx,
- * else feed. `cancel` (may be NULL) is polled on the host between steps
+ * else feed. `cancel` (may be NULL) is polled on the host between launches of up to 32 steps
  * (sampling.rs:69-73); when seen set the call returns FC_E_CANCELLED with *n_out tokens
  * valid. out: host [max_new]. */
 int fc_generate_greedy(fc_stream* s, const int32_t* prompt, int n, int max_new, int32_t eos,
@@ -326,7 +326,8 @@ int fc_sample_logits(int device, const float* logits, int n, const fc_sampling* 
  * prompt ids, then per token draw from ln(max(p, 1e-12)) of the current distribution with the
  * window's ids as `recent`, stop on eos, re-prime on the last ctx/2 ids when the window
  * outgrows the context. The sampler and the generator state stay on the device between
- * tokens; *rng_state returns advanced. */
+ * tokens; *rng_state returns advanced. `cancel` (may be NULL) is polled on the host before every draw;
+ * without it the host reads tokens back 16 at a time. */
 int fc_generate_sampled(fc_stream* s, const int32_t* prompt, int n, int max_new, int32_t eos, const fc_sampling* params,
                         uint64_t* rng_state, const volatile int32_t* cancel, int32_t* out, int* n_out);
 /* n_streams independent greedy generations on one GPU: prompts [n_streams][prompt_len], out

@@ -1,13 +1,15 @@
 """Device sampler (sample.cu) against the oracle's restatement of slm/sampling.rs:124-210."""
+import ctypes as C
 import os
 import sys
+import threading
 
 import numpy as np
 import pytest
 
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 import ferrum_cpu_b200 as fcb  # noqa: E402
-from ferrum_cpu_b200 import synth  # noqa: E402
+from ferrum_cpu_b200 import _lib, synth  # noqa: E402
 from tests import oracle as O  # noqa: E402
 
 pytestmark = pytest.mark.gpu
@@ -153,3 +155,30 @@ def test_generate_sampled_follows_the_reference_loop():
     assert np.array_equal(g0, g1)
     gm.close()
     om.close()
+
+
+def test_cancel_is_polled_before_every_draw():
+    """A flag set when the first token arrives ends the generation at any later token, not at the end of a batch of 16."""
+    sm = synth.named("tiny", seed=0, perturb=True)
+    gm = fcb.CudaSlm(sm.config, sm.weights)
+    prompt, new = synth.token_ids(3, 9, sm.dims[5]), 100
+    params, made = fcb.sampling(0.8, 40, 0.95, 1.1), []
+    for seed in range(8):
+        out, cancel, n_out, over = np.full(new, -1, np.int32), np.zeros(1, np.int32), C.c_int(), threading.Event()
+
+        def watch():
+            while out[0] < 0 and not over.is_set():
+                pass
+            cancel[0] = 1
+
+        t = threading.Thread(target=watch)
+        t.start()
+        rc = _lib.lib().fc_generate_sampled(gm._stream(), prompt.ctypes.data, len(prompt), new, -1, C.byref(params),
+                                            C.byref(C.c_uint64(seed + 1)), cancel.ctypes.data, out.ctypes.data, C.byref(n_out))
+        over.set()
+        t.join()
+        assert rc in (_lib.FC_OK, _lib.FC_E_CANCELLED)
+        assert np.array_equal(out[:n_out.value], gm.generate_sampled(prompt, new, params, seed + 1)[0][:n_out.value])
+        made.append(n_out.value)
+    assert any(n % 16 and n < new for n in made), made
+    gm.close()
