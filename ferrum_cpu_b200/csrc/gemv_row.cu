@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
                 a.part[p[r]].out[n[r]] = v;
                 if (KIND == NORM && a.stats) {
                     if (v > top) { mass *= expf(top - v); top = v; }
-                    mass += expf(v - top);
+                    if (v != -INFINITY) mass += expf(v - top);
                 }
             }
     };

@@ -230,6 +230,7 @@ __device__ __forceinline__ float2 row_stats(const float2* __restrict__ stats, in
 }
 // Greedy pick: first index of the largest ln(max(p, 1e-12)). Rounding can make neighbours of the largest logit tie with it, but
 // nothing 0.01 below it (p there is at least 1 % smaller, and the largest p is at least 1 / V), so only those are evaluated.
+// A row with a NaN or an infinity, or of -inf alone, has no mass to compare: every p is NaN, all tie at the floor, the first wins.
 __global__ void __launch_bounds__(1024) step_pick_kernel(const float* __restrict__ logits, int V, const float2* __restrict__ stats, int n_stats,
                                                          int* __restrict__ queue, int queue_cap, StepState* st) {
     __shared__ ArgPair pred[32];
@@ -241,7 +242,9 @@ __global__ void __launch_bounds__(1024) step_pick_kernel(const float* __restrict
     auto look = [&](float l, int i) {
         if (l >= ms.x - 0.01f) best = better(best, ArgPair{logf(fmaxf(expf(l - ms.x) / ms.y, 1e-12f)), i});
     };
-    const int V4 = V >> 2;
+    const bool comparable = ms.y > 0.0f;
+    if (!comparable) best = ArgPair{0.0f, 0};
+    const int V4 = comparable ? V >> 2 : 0;
     for (int i0 = threadIdx.x; i0 < V4; i0 += 7 * blockDim.x) {
         float4 l[7];                     // 28 K logits on their way at a time
 #pragma unroll
@@ -256,7 +259,7 @@ __global__ void __launch_bounds__(1024) step_pick_kernel(const float* __restrict
             look(l[k].x, i); look(l[k].y, i + 1); look(l[k].z, i + 2); look(l[k].w, i + 3);
         }
     }
-    if ((int)threadIdx.x < (V & 3)) look(logits[4 * V4 + threadIdx.x], 4 * V4 + threadIdx.x);
+    if (comparable && (int)threadIdx.x < (V & 3)) look(logits[4 * V4 + threadIdx.x], 4 * V4 + threadIdx.x);
     auto warp_best = [&]() {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)

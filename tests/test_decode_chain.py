@@ -70,3 +70,31 @@ def test_generation_runs_in_the_mode_it_was_asked_for():
         gm.set_trace(False)
         assert (fcb.take_launch_count() < launches[1]) == traced
     gm.close()
+
+
+@pytest.mark.parametrize("rows", ["nan", "minus infinity"])
+def test_pick_on_rows_that_are_not_finite(rows):
+    """A row of NaN has no largest probability: ln(max(p, 1e-12)) is the floor everywhere and index 0 is picked. Logits of -inf
+    have probability 0, wherever they stand."""
+    sm = synth.SynthModel(1, 64, 1, 96, 64, 1031, seed=9, perturb=True)
+    if rows == "nan":
+        sm.out_norm_g[:] = np.nan
+    else:
+        # the first 300 rows meet -3e38 with a weight of 2, the others with 0
+        table = synth.q8_0_dequantize(sm.token_embd, 1031 * 64).reshape(1031, 64)
+        table[:300, 0], table[300:, 0] = 2.0, 0.0
+        sm.token_embd[:] = synth.q8_0_quantize(table)
+        sm.out_norm_g[0], sm.out_norm_b[0] = 0.0, -3e38
+    om, gm = O.OracleModel(sm), fcb.CudaSlm(sm.config, sm.weights)
+    prompt = synth.token_ids(8, 12, 1031)
+    want = om.generate_greedy(prompt, 12)[0]
+    assert (want == 0).all() if rows == "nan" else (want >= 300).all()
+    gm.set_decode_mode(1)
+    assert np.array_equal(gm.generate_tokens(prompt, 12)[0], want)
+    if rows == "nan":
+        gm.set_decode_mode(0)
+        assert np.array_equal(gm.generate_tokens(prompt, 12)[0], want)
+    else:
+        assert np.array_equal(gm.generate_sampled(prompt, 12, fcb.sampling(temperature=0.0), 1)[0], want)
+    gm.close()
+    om.close()
