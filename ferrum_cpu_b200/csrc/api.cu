@@ -499,6 +499,7 @@ static int score_device(fc_model* m, const ScoreSlot& s, const Windows& win, int
         FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, nullptr, R, d, m->pn, m->st));
         FC_TRY(launch_layer_stats(nullptr, m->pn, (size_t)R * d, m->stats_scratch, m->stats_d + m->stats_n++, m->st));
     }
+    if (n == 0) return FC_OK;               // the forward was for its statistics
     // the head's epilogue keeps (max, sum of exponentials, first argmax) per row and 128-column tile and the
     // target's logit: [rows][V] logits never reach memory (scoring.rs:175-181 needs one number per row)
     FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, n == R ? nullptr : pick, n, d, m->pn, m->st));
@@ -861,7 +862,7 @@ static int score_issue(fc_model* m, ScoreSlot& s, const ScoreBatch& b) {
     Windows win;
     win.B = (int)B; win.T = b.longest; win.starts = (const int*)s.in_d + 2 * R;
     FC_CUDA(cudaEventRecord(s.ev0, st));
-    if (n > 0) FC_TRY(score_device(m, s, win, (int)R));
+    if (n > 0 || m->stats_on) FC_TRY(score_device(m, s, win, (int)R));
     FC_CUDA(cudaEventRecord(s.ev1, st));
     FC_CUDA(cudaMemcpyAsync(s.out_h, s.out_d, s.out_bytes(), cudaMemcpyDeviceToHost, st));
     FC_CUDA(cudaEventRecord(s.done, st));

@@ -75,6 +75,10 @@ def test_layer_stats_records(mode):
     assert st[0]["min"] == emb.min() and st[0]["max"] == emb.max() and abs(st[0]["mean"] - emb.mean(dtype=np.float64)) < 1e-6
     # the final LayerNorm of a row has (gain-weighted) zero mean and unit scale: a sanity range, not a parity claim
     assert abs(st[-1]["mean"]) < 0.5 and st[-1]["max"] < 10 and st[-1]["min"] > -10
+    # a forward without a scored row has the same records
+    gm.set_layer_stats(True)
+    gm.score_windows(ids[None], np.full((1, 32), -1, np.int32))
+    assert gm.layer_stats() == st
     gm.set_layer_stats(False)
     gm.token_logprobs(ids, 1)
     assert gm.layer_stats() == []
