@@ -20,12 +20,6 @@ static thread_local char g_err[512] = "";
 thread_local int64_t g_launches = 0;
 DebugKnobs g_debug;
 
-void set_error(const char* fmt, ...) {
-    va_list ap;
-    va_start(ap, fmt);
-    vsnprintf(g_err, sizeof g_err, fmt, ap);
-    va_end(ap);
-}
 const char* g_err_text() { return g_err; }
 int fail(int code, const char* fmt, ...) {
     va_list ap;

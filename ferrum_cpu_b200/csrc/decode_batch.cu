@@ -44,12 +44,6 @@ constexpr int RED_LD = 33;
 __device__ __forceinline__ void pdl_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-__device__ __forceinline__ uint4 ld_stream16(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
 // bytes (b0, b1) of w (biased quants q + 128) -> two exact f16 values (q0, q1): 0x6400 | b is
 // 1024 + b, and 1152 = 1024 + 128 is subtracted.
 template <int HI>

@@ -1014,9 +1014,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_mega_kernel(const __grid_co
     }
 }
 
-size_t mega_smem_bytes() { return SMEM_BYTES; }
 int mega_head_rows_max() { return MAX_ROWS_HEAD; }
-int mega_threads() { return THREADS; }
 
 int mega_supported(const fc_config& c) {
     const int hd = c.d_model / c.n_head;

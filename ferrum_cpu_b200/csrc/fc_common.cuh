@@ -13,7 +13,6 @@
 namespace fc {
 
 // ---- errors -------------------------------------------------------------------------
-void set_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
 int fail(int code, const char* fmt, ...);
 const char* g_err_text();   // the calling thread's last error text
@@ -108,7 +107,7 @@ struct QMat {
 };
 constexpr int kRowPad = 128;
 
-enum Epilogue : int { EPI_NONE = 0, EPI_GELU = 1, EPI_SWIGLU = 2, EPI_SCORE = 3 };
+enum Epilogue : int { EPI_NONE = 0, EPI_GELU = 1, EPI_SWIGLU = 2 };
 
 // activation.rs:9-12 (tanh GELU): 0.5 x (1 + tanh(u)) with u = 0.7978846 (x + 0.044715 x^3). Since (1 + tanh(u)) / 2 is the
 // logistic function of 2u, that is x / (1 + exp(-2u)): a handful of instructions where tanhf takes some thirty, and
@@ -171,8 +170,6 @@ int attn_step_split(int n_q, int hd, int ctx, int* split, int* from);
 int launch_attn_step(const float* qkv, int n_q, int n_kv, int hd, int rope_dim, int neox, const float2* ftab, float inv_linear,
                      float* kc, float* vc, int ctx, int split, const StepState* state, float* out, cudaStream_t st);
 
-// An f32 matrix as n bf16 planes whose sum it is: 2 planes hold it to 2^-17 relative (FC_MATH_BF16X3), 3 exactly
-// (FC_MATH_FP32). The form in which activations reach the tensor cores.
 // Windows of rows that share a forward pass: window b holds rows starts[b] .. starts[b + 1] (device array of B + 1), or, with
 // starts == nullptr, T rows each. T: rows of the longest.
 struct Windows {
@@ -182,6 +179,8 @@ struct Windows {
     __host__ __device__ int length(int b) const { return starts ? starts[b + 1] - starts[b] : T; }
 };
 
+// An f32 matrix as n bf16 planes whose sum it is: 2 planes hold it to 2^-17 relative (FC_MATH_BF16X3), 3 exactly
+// (FC_MATH_FP32). The form in which activations reach the tensor cores.
 struct Planes {
     void* p[3] = {nullptr, nullptr, nullptr};
     int n = 0;
@@ -239,8 +238,6 @@ int launch_ggml_linear(const fc_ggml_weight* w, const float* x, const float* bia
                        cudaStream_t st);
 int launch_ggml_rows(const fc_ggml_weight* w, const int* ids, StepState* state, const int* queue, int ctx, int R, float* x,
                      int* error_flag, cudaStream_t st);
-int ggml_weight_rows(const fc_ggml_weight* w);
-int ggml_weight_cols(const fc_ggml_weight* w);
 
 // Per-row-scale int8 / int4 linear on a packed matrix (rowq.cu): y[M][ldy] = [residual +] bias + x · W; bias and residual may
 // be null, residual may be y itself. scratch: three planes of M x K the caller lends (several rows), with the status word of

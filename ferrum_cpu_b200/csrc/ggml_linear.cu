@@ -285,9 +285,6 @@ int launch_ggml_rows(const fc_ggml_weight* w, const int* ids, StepState* state, 
     return FC_OK;
 }
 
-int ggml_weight_rows(const fc_ggml_weight* w) { return w->N; }
-int ggml_weight_cols(const fc_ggml_weight* w) { return w->K; }
-
 }  // namespace fc
 
 using namespace fc;

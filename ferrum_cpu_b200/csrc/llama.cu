@@ -68,7 +68,6 @@ struct fc_llama_cache {
     int* queue = nullptr;
     int queue_cap = 0;
     StepState* state = nullptr;
-    int* status = nullptr;                // raised by a kernel whose bounded wait ran out
     int host_pos = 0;
     // [heads with a CTA each, shared ones][0: step without the head, 1: with it, 2: kFreeSteps times the greedy pick and 1]
     cudaGraphExec_t graph[2][3] = {};
@@ -480,14 +479,8 @@ __global__ void llama_set_state_kernel(StepState* st, int pos, int fed, int tail
 }
 
 int read_state(fc_llama_cache* s, StepState* out) {
-    int status = 0;
     FC_CUDA(cudaMemcpyAsync(out, s->state, sizeof(StepState), cudaMemcpyDeviceToHost, s->m->st));
-    FC_CUDA(cudaMemcpyAsync(&status, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->m->st));
     FC_CUDA(cudaStreamSynchronize(s->m->st));
-    if (status != 0) {
-        cudaMemsetAsync(s->status, 0, sizeof(int), s->m->st);
-        return fail(FC_E_TIMEOUT, "a bounded wait inside the streaming GEMV ran out (status %d)", status);
-    }
     return FC_OK;
 }
 
@@ -824,8 +817,6 @@ int fc_llama_cache_create(fc_llama* m, fc_llama_cache** out) {
         s->queue_cap = c.ctx + 1;
         FC_TRY(a.alloc_n(&s->queue, (size_t)s->queue_cap));
         FC_TRY(a.alloc_n(&s->state, 1));
-        FC_TRY(a.alloc_n(&s->status, 1));
-        FC_CUDA(cudaMemsetAsync(s->status, 0, sizeof(int), m->st));
         FC_TRY(attn_step_split(c.n_head, c.head_dim, c.ctx, &s->attn_split, &s->split_from));
         FC_TRY(a.alloc_n(&s->rng_d, 1));
         FC_CUDA(cudaEventCreate(&s->ev0));

@@ -336,25 +336,6 @@ int launch_llama_attn_decode(const float* qkv, int n_q, int n_kv, int hd, int ro
     return FC_OK;
 }
 
-// --------------------------------------------------------------------------------- SwiGLU
-// FeedForward::forward (llm.rs:417-428): h = (g / (1 + exp(-g))) * u on rows of interleaved
-// (gate_i, up_i) pairs, the row order of the fused gate/up matrix.
-__global__ void llama_swiglu_kernel(const float* __restrict__ gu, int F, float* __restrict__ h, const StepState* st) {
-    if (st && (st->done | st->error)) return;
-    const float* row = gu + (size_t)blockIdx.y * 2 * F;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < F) {
-        const float g = row[2 * c], u = row[2 * c + 1];
-        h[(size_t)blockIdx.y * F + c] = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), u);
-    }
-}
-int launch_llama_swiglu(const float* gu, int rows, int F, float* h, const StepState* state, cudaStream_t st) {
-    dim3 grid((F + 255) / 256, rows);
-    llama_swiglu_kernel<<<grid, 256, 0, st>>>(gu, F, h, state);
-    FC_LAUNCHED();
-    return FC_OK;
-}
-
 // --------------------------------------------------------------------------- scoring tail
 // log_prob (llm_score.rs:35-39): ln softmax(row)[target] in f64 with no probability floor —
 // max in f32, sum of exp((f64)x - max) in f64, x[target] - max - ln(sum); and

@@ -27,7 +27,6 @@ int launch_llama_attn_decode(const float* qkv, int n_q, int n_kv, int hd, int ro
                              float* kc, float* vc, int ctx, const StepState* state, float* out, cudaStream_t st);
 // RMSNorm written as the bf16 planes [rows][d] of the tensor-core GEMM.
 int launch_llama_rmsnorm_planes(const float* x, const float* w, float eps, int rows, int d, const Planes& out, cudaStream_t st);
-int launch_llama_swiglu(const float* gu, int rows, int F, float* h, const StepState* state, cudaStream_t st);
 int launch_llama_score_rows(const float* logits, int ldl, int V, const int* targets, int R, double* logprob, uint8_t* is_greedy,
                             cudaStream_t st);
 int launch_llama_pick(const float* logits, int V, int* queue, int queue_cap, StepState* state, cudaStream_t st);

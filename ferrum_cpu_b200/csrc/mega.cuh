@@ -99,9 +99,7 @@ struct MegaParams {
     int withhold;              // test hook: the producer warps copy nothing
 };
 
-size_t mega_smem_bytes();
 int mega_head_rows_max();   // most LM-head rows one CTA can own
-int mega_threads();
 int mega_supported(const fc_config& c);
 int mega_max_grid(int* grid);
 int launch_decode_mega(const MegaParams& p, int grid, cudaStream_t st);
