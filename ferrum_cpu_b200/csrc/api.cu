@@ -567,7 +567,7 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
     if (current != w->device) FC_CUDA(cudaSetDevice(w->device));
     cudaStream_t st = (cudaStream_t)cuda_stream;
     if (M == 1) {
-        return launch_gemv_row(w->w, x_dev, RowNorm(), bias_dev, nullptr, EPI_NONE, y_dev, nullptr, st);
+        return launch_gemv_alone(GemvPart{w->w.qu, w->w.d, nullptr, bias_dev, y_dev, w->w.N}, w->w.K, x_dev, st);
     }
     FC_TRY(const_cast<fc_qweight*>(w)->status.check("an earlier call on this weight"));
     const int planes = math_mode == FC_MATH_BF16X3 && w->w.K % 64 == 0 ? 2 : 3;

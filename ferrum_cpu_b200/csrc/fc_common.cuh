@@ -161,6 +161,9 @@ inline int launch_gemv_row(const QMat& w, const float* x, const RowNorm& norm, c
     return launch_gemv_row(&p, 1, w.K, x, norm, residual, epi, state, st, stats, n_stats);
 }
 
+// gemv_wide.cu — a caller's own row product, on the kernel for its size. The weight's rows are padded to kRowPad.
+int launch_gemv_alone(const GemvPart& part, int K, const float* x, cudaStream_t st);
+
 // attn_step.cu — one attention step over the caches, `split` CTAs per query head; ftab null: no rotation. The state and the
 // cached rows are read ahead of its wait: some kernel of the step before it has to wait for all of the step before.
 // attn_step_split: the CTAs that share a head at long positions (1: it stays with one), and the position from which on that is

@@ -256,6 +256,7 @@ int launch_rowq_linear(fc_rowq* w, const float* x, const float* bias, const floa
     if (ldy < w->cols) return fail(FC_E_SHAPE, "rowq linear: row stride %d below %d columns", ldy, w->cols);
     GemvPart part;
     if (!rowq_part(w, bias, y, &part)) return rowq_launch(w, x, bias, residual, y, ldy, M, st);
+    if (M == 1 && !residual) return launch_gemv_alone(part, w->rows, x, st);
     if (M == 1) return launch_gemv_row(&part, 1, w->rows, x, RowNorm(), residual, EPI_NONE, nullptr, st);
     const size_t n = (size_t)M * w->rows;
     CallScratch own;

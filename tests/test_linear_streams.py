@@ -165,3 +165,23 @@ def test_host_entry_reports_a_wait_that_ran_out():
     want = x.astype(np.float64) @ f.T
     assert np.abs(w.linear(x, np.zeros(256, np.float32)) - want).max() <= 2e-6 * np.abs(want).max()
     w.close()
+
+
+@pytest.mark.parametrize("make", [q8_weight, rowq_weight])
+@pytest.mark.parametrize("n,k", [(4096, 96), (4097, 32), (4130, 4128), (8191, 768), (16383, 512), (16384, 512), (16390, 544), (24575, 544),
+                                 (24576, 544), (24579, 1056), (50257, 96)])
+def test_single_row_against_matrices_of_many_rows(make, n, k):
+    """The sizes at which the row product changes its kernel, last rows that fill no half warp, rows of fewer chunks than lanes and
+    no multiple of them; the bias is the output of the call ahead."""
+    import torch
+
+    w, f = make(n, k, n + k)
+    x = torch.from_numpy(np.random.default_rng(k).standard_normal((2, k)).astype(np.float32)).cuda()
+    zero, y1, y2 = torch.zeros(n, device="cuda"), torch.full((n,), np.nan, device="cuda"), torch.full((n + 64,), np.nan, device="cuda")
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    w.linear_dev(x[0].data_ptr(), zero.data_ptr(), y1.data_ptr(), 1, stream=stream)
+    w.linear_dev(x[1].data_ptr(), y1.data_ptr(), y2.data_ptr(), 1, stream=stream)
+    want = x.double().cpu().numpy().sum(axis=0) @ f.T
+    assert np.abs(y2[:n].cpu().numpy() - want).max() <= 24 * 2.0 ** -24 * 4 * np.abs(want).max()
+    assert torch.isnan(y2[n:]).all()
+    w.close()
