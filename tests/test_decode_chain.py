@@ -98,3 +98,18 @@ def test_pick_on_rows_that_are_not_finite(rows):
         assert np.array_equal(gm.generate_sampled(prompt, 12, fcb.sampling(temperature=0.0), 1)[0], want)
     gm.close()
     om.close()
+
+
+@pytest.mark.parametrize("heads,kv,hd,ctx,prompt", [(2, 1, 128, 2048, 1640), (4, 1, 32, 6144, 5500)])
+def test_shared_heads_past_the_held_rows(heads, kv, hd, ctx, prompt):
+    """Positions at which even the parts of a shared head outgrow its CTAs' shared memory: 8 of them hold about 188 rows each of
+    width 128, about 650 of width 32."""
+    sm = synth.SynthLlama(515, 96, 1, heads, kv, hd, 160, ctx, seed=hd, perturb=True)
+    om, gm = O.OracleLlama(sm, threads=4), CudaLlama.from_synth(sm)
+    cache, ids = gm.new_cache(), synth.token_ids(2, prompt + 3, 515)
+    om.clear()
+    for tok in ids[:prompt]:
+        om.forward_one(tok)
+    gm.prime(ids[:prompt], cache, want_logits=False)
+    for tok in ids[prompt:]:
+        assert np.abs(gm.forward_one(tok, cache) - om.forward_one(tok)).max() < 2e-4
