@@ -566,21 +566,16 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
     FC_CUDA(cudaGetDevice(&current));
     if (current != w->device) FC_CUDA(cudaSetDevice(w->device));
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    if (M == 1) {
-        return launch_gemv_alone(GemvPart{w->w.qu, w->w.d, nullptr, bias_dev, y_dev, w->w.N}, w->w.K, x_dev, st);
-    }
+    const GemvPart part = {w->w.qu, w->w.d, nullptr, bias_dev, y_dev, w->w.N};
+    if (M == 1) return launch_gemv_alone(part, w->w.K, x_dev, st);
+    if (few_rows(w->w.N, w->w.K, M)) return launch_rows_alone(part, w->w.K, x_dev, M, st);
     FC_TRY(const_cast<fc_qweight*>(w)->status.check("an earlier call on this weight"));
     const int planes = math_mode == FC_MATH_BF16X3 && w->w.K % 64 == 0 ? 2 : 3;
     const size_t n = (size_t)M * w->w.K;
     CallScratch scratch;
     Planes x;
     FC_TRY(take_planes(scratch, x, planes, n, w->device, st));
-    if (!scratch.p) {
-        // no memory for the planes: the rows one by one, which need none
-        for (int m = 0; m < M; ++m)
-            FC_TRY(launch_gemv_row(w->w, x_dev + (size_t)m * w->w.K, RowNorm(), bias_dev, nullptr, EPI_NONE, y_dev + (size_t)m * w->w.N, nullptr, st));
-        return FC_OK;
-    }
+    if (!scratch.p) return launch_rows_alone(part, w->w.K, x_dev, M, st);   // no memory for the planes
     FC_TRY(launch_split_planes(x_dev, x, n, st));
     return launch_gemm_q8_tc(w->w, x, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, w->status.dev, st);
 }

@@ -161,8 +161,11 @@ inline int launch_gemv_row(const QMat& w, const float* x, const RowNorm& norm, c
     return launch_gemv_row(&p, 1, w.K, x, norm, residual, epi, state, st, stats, n_stats);
 }
 
-// gemv_wide.cu — a caller's own row product, on the kernel for its size. The weight's rows are padded to kRowPad.
+// rows_alone.cu — a caller's own product of one row or few (y rows N apart), on the kernel for its size; M rows need no scratch
+// there. The weight's rows are padded to kRowPad. few_rows: whether they are better off there than on the GEMM.
 int launch_gemv_alone(const GemvPart& part, int K, const float* x, cudaStream_t st);
+bool few_rows(int N, int K, int M);
+int launch_rows_alone(GemvPart part, int K, const float* x, int M, cudaStream_t st);
 
 // attn_step.cu — one attention step over the caches, `split` CTAs per query head; ftab null: no rotation. The state and the
 // cached rows are read ahead of its wait: some kernel of the step before it has to wait for all of the step before.

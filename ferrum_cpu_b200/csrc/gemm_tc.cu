@@ -36,11 +36,17 @@
 // reproducible.
 //
 // Every wait is bounded; a wait that runs out raises the status word and all roles leave.
-// Bound: tensor pipe for large M (2·M·N·K algorithmic FLOP, planes x that executed), weight bytes for a few rows. Measured
-// with the split of X into planes (of the f32 form this replaced: CUDA-core FMA, 42 TFLOP/s):
+// Bound: weight bytes for a few rows, the drain for many (2·M·N·K algorithmic FLOP, planes x that executed). Measured with the
+// split of X into planes (of the f32 form this replaced: CUDA-core FMA, 42 TFLOP/s):
 //     32768 x 768 x 2304   2 planes 348 us = 334 TFLOP/s   3 planes 369 us = 314 TFLOP/s
 //     32768 x 1024 x 4096  2 planes 746 us = 368 TFLOP/s   3 planes 791 us = 348 TFLOP/s
 //     4096 x 1024 x 4096   2 planes 109 us (126 before)    3 planes 112 us (811 before)
+// Half as many MMAs again cost 3 to 6 %: the tensor pipe is active 33 % (2 planes) and 49 % (3) of the cycles. Where the roles
+// wait, in cycles by clock64 around the waits, 4096 x 1024 x 4096 in pair tiles of 160, 2 / 3 planes: a 64-wide stage takes about
+// 1710 / 1795, its MMAs 640 / 960; an issuer waits 610 / 547 of it for an accumulator buffer and 254 / 268 for a stage, the TMA
+// warp 1141 / 1115 and the converters 651 / 719 for a free stage. The drain spends 201 / 219 of the 733 / 767 cycles of a
+// 32-wide k-block on its wait, which is about what a wait on a completed phase costs: it is the role the others wait for.
+// Longer rows dilute the epilogue (193 cycles a k-block at K = 1024, 65 at 3072) and nothing else.
 #include <cuda.h>
 
 #include <algorithm>
@@ -718,9 +724,11 @@ int encode_plane(CUtensorMap* map, const void* plane, int M, int K, int box_rows
 
 struct TileChoice { int cg, nt, ksplit; };
 
-// Tile shape by estimated SM cycles: waves of tiles x (k-blocks x the slowest of the pipelines + what a tile costs once).
+// Tile shape by a score in SM cycles: waves of tiles x (k-blocks x the slowest of the pipelines + what a tile costs once).
 // Per 32-wide k-block: tensor pipe planes * nt; shared-memory bandwidth (128 bytes a cycle: operand reads of the MMAs, the
-// TMA writes, the converted weights); the drain (tcgen05.ld and FMA, 32 lanes a cycle); the weight conversion.
+// TMA writes, the converted weights); the drain (tcgen05.ld and FMA, 32 lanes a cycle); the weight conversion. The score ranks
+// shapes, it does not predict times: it counts throughputs, and what a k-block really takes is the latency of the drain's
+// chain (wait, tcgen05.ld, FMA; see above): about 860 cycles with 160 rows where the score has 350 for two planes, 500 for three.
 // split_k: the K range may be split over CTAs, which changes the order of the sums with the number of rows; callers whose
 // results may not depend on how many rows share a launch leave it out.
 TileChoice choose_tile(int M, int N, int K, int P, int mode, bool split_k, int sms) {

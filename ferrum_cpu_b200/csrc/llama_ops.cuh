@@ -10,7 +10,7 @@ __device__ __forceinline__ float rope_angle(int pos, float2 f, float inv_linear)
 }
 
 int launch_llama_embed_rows(const QMat& tok, const int* ids, int R, float* x, int* error_flag, cudaStream_t st);
-// Rotation of window rows with the result written as bf16 hi / lo planes [R][ld] (the f32 rows stay as they were).
+// Rotation of window rows with the result written as bf16 planes [R][ld] (the f32 rows stay as they were).
 int launch_llama_rope_planes(const float* qkv, int R, int ld, int T, int n_q, int n_kv, int k_off, int hd, int rope_dim, int neox,
                              const float2* ftab, float inv_linear, const Planes& out, cudaStream_t st);
 int launch_llama_embed_step(const QMat& tok, int ctx, const int* queue, StepState* state, float* x, cudaStream_t st);

@@ -258,6 +258,8 @@ int launch_rowq_linear(fc_rowq* w, const float* x, const float* bias, const floa
     if (!rowq_part(w, bias, y, &part)) return rowq_launch(w, x, bias, residual, y, ldy, M, st);
     if (M == 1 && !residual) return launch_gemv_alone(part, w->rows, x, st);
     if (M == 1) return launch_gemv_row(&part, 1, w->rows, x, RowNorm(), residual, EPI_NONE, nullptr, st);
+    // a caller's own product: rows `cols` apart, no residual
+    if (!scratch && few_rows(w->cols, w->rows, M)) return launch_rows_alone(part, w->rows, x, M, st);
     const size_t n = (size_t)M * w->rows;
     CallScratch own;
     Planes p;
@@ -266,15 +268,7 @@ int launch_rowq_linear(fc_rowq* w, const float* x, const float* bias, const floa
     } else {
         FC_TRY(w->status.check("an earlier call on this weight"));
         FC_TRY(take_planes(own, p, 3, n, w->device, st));
-        if (!own.p) {
-            // no memory for the planes: the rows one by one, which need none
-            for (int m = 0; m < M; ++m) {
-                part.out = y + (size_t)m * ldy;
-                FC_TRY(launch_gemv_row(&part, 1, w->rows, x + (size_t)m * w->rows, RowNorm(), residual ? residual + (size_t)m * ldy : nullptr,
-                                       EPI_NONE, nullptr, st));
-            }
-            return FC_OK;
-        }
+        if (!own.p) return launch_rows_alone(part, w->rows, x, M, st);      // no memory for the planes
     }
     FC_TRY(launch_split_planes(x, p, n, st, w->scales, w->rows));
     return launch_gemm_q8_tc(w->levels, p, bias, residual, EPI_NONE, y, nullptr, M, ldy, scratch ? status : w->status.dev, st);

@@ -36,7 +36,8 @@ extern "C" {
 #define FC_E_CANCELLED (-6) /* the cancel flag was seen set */
 #define FC_E_ARG (-7)       /* null handle / null required pointer */
 
-/* Math modes of the prefill GEMM. Decode always runs fp32 FMA on CUDA cores. */
+/* Math modes of the window forward (scoring, primes) and of the linears with M >= 2. Decode steps are
+ * f32-equivalent in both. */
 #define FC_MATH_FP32 0      /* tcgen05 kind::f16, activations as three bf16 planes (their f32 value exactly), f32 accumulate */
 #define FC_MATH_BF16X3 1    /* the same with two planes (2^-17 relative) */
 
@@ -153,16 +154,17 @@ int fc_q8_0_linear(int device, const float* x, const void* wq, const float* bias
  * handle is used by one host thread at a time, like every other handle; the streams it is used on may
  * be several, and calls on them may overlap.
  * Operands are read and written in the stream's order, bias_dev included: it may be what the call ahead
- * on the stream writes. With M >= 2 the rows of x are first split into bf16 planes (two in
+ * on the stream writes. Few rows (K <= 3072 and M <= 4, or M * N * K below 2^25 with K rounded up to 256)
+ * run on f32 FMA in both math modes and need no scratch. More are first split into bf16 planes (two in
  * FC_MATH_BF16X3 when K is a multiple of 64, else three: 4 or 6 bytes an element). That scratch belongs
  * to the call, not to the weight: it is taken from a pool in the order of the stream and given back in
  * the same order, so that a call may be captured into a graph without a call before it (it becomes an
  * allocation node; such a graph cannot be a child node). Between calls the pool keeps 256 MiB at most
  * for all weights of a device and gives everything back with the last of them. Where there is no
- * memory for it, the rows run one by one on the kernel of M = 1, which needs none.
- * A device-side wait that runs out (M >= 2, both math modes) can only be seen after the kernel has
- * ended: it is reported as FC_E_TIMEOUT by the next call with M >= 2 on the handle, which launches
- * nothing. */
+ * memory for it, all rows run on the kernels that need none.
+ * A device-side wait of the tensor-core product that runs out (both math modes) can only be seen after the
+ * kernel has ended: it is reported as FC_E_TIMEOUT by the next call on the handle that takes the tensor
+ * cores, which then launches nothing. */
 int fc_qweight_upload(int device, const void* wq, int N, int K, fc_qweight** out);
 void fc_qweight_free(fc_qweight* w);
 int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bias_dev, float* y_dev,
@@ -410,8 +412,9 @@ int fc_llama_create(const fc_llama_config* cfg, const fc_llama_weights* w, int d
  * gguf/llama.rs:13-27,164-171): each Q8_0 matrix is decoded, transposed to [in][out] and packed by
  * QWeight::from_f32 (quant.rs:164-212) to per-input-row int8 (FC_Q_INT8) or int4 (FC_Q_INT4) - the LM head too, the
  * tied one from the transposed embedding (gguf/llama.rs:304-311) - and every forward runs ops::qlinear
- * (ops.rs:316-377) on them; the embedding table stays as stored. All fc_llama_* calls work on the result; the decode
- * step runs one kernel per operation. */
+ * (ops.rs:316-377) on them; the embedding table stays as stored. All fc_llama_* calls work on the result. Matrices
+ * whose input width is a multiple of 32 (at most 12288) become rows of levels on the device and run the decode step of
+ * the Q8_0 model, five kernels a block; other widths run one kernel per operation. */
 int fc_llama_create_packed(const fc_llama_config* cfg, const fc_llama_weights* w, int device, int kind, fc_llama** out);
 void fc_llama_free(fc_llama* m);
 /* Gguf::load_llama (gguf/llama.rs:164-339) for `llama` and `qwen2` files whose projections are

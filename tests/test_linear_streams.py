@@ -84,7 +84,7 @@ def test_calls_on_two_streams_share_nothing(make, math_mode, tol):
 def test_first_call_may_be_captured(make, math_mode, tol):
     import torch
 
-    n, k, m = 300, 512, 77
+    n, k, m = 300, 512, 277
     w, f = make(n, k, 4)
     x, zero, y = torch.randn(m, k, device="cuda"), torch.zeros(n, device="cuda"), torch.zeros(m, n, device="cuda")
     torch.cuda.synchronize()
@@ -102,10 +102,11 @@ def test_first_call_may_be_captured(make, math_mode, tol):
 
 
 @pytest.mark.parametrize("make,math_mode,tol", KINDS)
-def test_without_memory_for_scratch_the_rows_run_one_by_one(make, math_mode, tol):
+@pytest.mark.parametrize("rows_k", [544, 3104])
+def test_without_memory_for_scratch_the_rows_need_none(make, math_mode, tol, rows_k):
     import torch
 
-    n, k, m = 129, 544, 9
+    n, k, m = 1290, rows_k, 45
     w, f = make(n, k, 5)
     x, zero, y = torch.randn(m, k, device="cuda"), torch.zeros(n, device="cuda"), torch.zeros(m, n, device="cuda")
     _lib.lib().fc_debug_withhold_scratch(1)
@@ -184,4 +185,28 @@ def test_single_row_against_matrices_of_many_rows(make, n, k):
     want = x.double().cpu().numpy().sum(axis=0) @ f.T
     assert np.abs(y2[:n].cpu().numpy() - want).max() <= 24 * 2.0 ** -24 * 4 * np.abs(want).max()
     assert torch.isnan(y2[n:]).all()
+    w.close()
+
+
+@pytest.mark.parametrize("make", [q8_weight, rowq_weight])
+@pytest.mark.parametrize("m,n,k", [(2, 1, 32), (2, 4097, 288), (3, 515, 96), (4, 33, 3072), (4, 2050, 544), (5, 129, 256), (7, 31, 1056), (13, 700, 800),
+                                   (64, 500, 96), (3, 300, 3104), (30, 4096, 256), (33, 4096, 256)])
+def test_few_rows_without_scratch(make, m, n, k):
+    """Rows that fill no block of four, weight rows that fill no half warp, chunks that fill no lane, and the sizes on either side of
+    the change to the GEMM; the bias is the output of the call ahead."""
+    import torch
+
+    w, f = make(n, k, n + k)
+    x = torch.from_numpy(np.random.default_rng(m).standard_normal((m, k)).astype(np.float32)).cuda()
+    zero, y1 = torch.zeros(n, device="cuda"), torch.full((n,), np.nan, device="cuda")
+    y = torch.full((m * n + 64,), np.nan, device="cuda")
+    stream = torch.cuda.current_stream()
+    run_linear(w, x[:1], zero, y1, _lib.FC_MATH_FP32, stream)
+    w_args = (x.data_ptr(), y1.data_ptr(), y.data_ptr(), m)
+    s = C.c_void_p(stream.cuda_stream)
+    w.linear_dev(*w_args, stream=s) if isinstance(w, engine.RowQWeight) else w.linear_dev(*w_args, _lib.FC_MATH_FP32, s)
+    xs = x.double().cpu().numpy()
+    want = xs @ f.T + xs[0] @ f.T
+    assert np.abs(y[:m * n].cpu().numpy().reshape(m, n) - want).max() <= 2e-6 * np.abs(want).max()
+    assert torch.isnan(y[m * n:]).all()
     w.close()
