@@ -1755,7 +1755,7 @@ int fc_decode_batch(fc_model* m, int n_streams, const int32_t* prompts, int prom
             // the head sees the last row of every window: final LayerNorm, one product for all streams, pick of token 1
             const int d = c.d_model;
             FC_TRY(launch_gather_last_rows(m->x, S, prompt_len, d, b.x, st));
-            FC_TRY(launch_batch_init(S, prompt_len, b.done, b.n_out, b.cur, b.pos, st));
+            FC_TRY(launch_batch_init(S, prompt_len, m->tc_status, b.done, b.n_out, b.cur, b.pos, st));
             FC_TRY(batch_head_and_pick(m, batch_view(m, 0, S, 0, st), eos, b.x, nullptr, 0, nullptr, nullptr, 0));
         } else {
             // prompts too short for a window forward: token by token per stream; the last step selects token 1
@@ -1792,7 +1792,7 @@ int fc_decode_batch(fc_model* m, int n_streams, const int32_t* prompts, int prom
             FC_CUDA(cudaEventElapsedTime(&pm, w0 > 0 ? m->ev1 : m->ev0, m->ev_prime));
             m->last_batch_prime_ms += pm;
         }
-        if (used) FC_TRY(check_tc_status(m, "the prime of fc_decode_batch"));
+        if (done[0] == 3) return check_tc_status(m, "the prime of fc_decode_batch");
         for (int i = 0; i < S; ++i)
             if (done[i] == 2) return fail(FC_E_CUDA, "fc_decode_batch: stream %d produced no finite logit", w0 + i);
         for (int i = 0; i < S; ++i) {

@@ -681,10 +681,11 @@ __global__ void gather_last_rows_kernel(const float* __restrict__ x, int n, int 
     for (int c = threadIdx.x; c < d; c += blockDim.x) out[(size_t)s * d + c] = src[c];
 }
 
-__global__ void batch_init_kernel(int S, int pos0, int* done, int* n_out, int* cur, int* pos) {
+// A prime whose bounded wait ran out (status) has nothing to go on from: its streams start as done = 3.
+__global__ void batch_init_kernel(int S, int pos0, const int* status, int* done, int* n_out, int* cur, int* pos) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < kBatchMaxStreams) pos[s] = pos0;             // one position word per group of the step
-    if (s < S) { done[s] = 0; n_out[s] = 0; cur[s] = 0; }
+    if (s < S) { done[s] = *status != 0 ? 3 : 0; n_out[s] = 0; cur[s] = 0; }
 }
 
 template <int NT, int RG, int MAXT = 512>
@@ -820,8 +821,8 @@ int launch_gather_last_rows(const float* x, int S, int n, int d, float* out, cud
     return FC_OK;
 }
 
-int launch_batch_init(int S, int pos0, int* done, int* n_out, int* cur, int* pos, cudaStream_t st) {
-    batch_init_kernel<<<(S + 63) / 64, 64, 0, st>>>(S, pos0, done, n_out, cur, pos);
+int launch_batch_init(int S, int pos0, const int* status, int* done, int* n_out, int* cur, int* pos, cudaStream_t st) {
+    batch_init_kernel<<<(S + 63) / 64, 64, 0, st>>>(S, pos0, status, done, n_out, cur, pos);
     FC_LAUNCHED();
     return FC_OK;
 }

@@ -318,7 +318,7 @@ int launch_pick_batch(const float* logits, int ldl, int V, int S, int eos, int* 
                       int* pos, int advance, cudaStream_t st);
 int launch_scatter_kv(const float* qkv, float* const* kcs, float* const* vcs, size_t layer_off, int S, int n, int d, cudaStream_t st);
 int launch_gather_last_rows(const float* x, int S, int n, int d, float* out, cudaStream_t st);
-int launch_batch_init(int S, int pos0, int* done, int* n_out, int* cur, int* pos, cudaStream_t st);
+int launch_batch_init(int S, int pos0, const int* status, int* done, int* n_out, int* cur, int* pos, cudaStream_t st);
 int launch_gather_first(int* const* queues, StepState* const* states, int prompt_len, int S, int* cur, int* done, int* n_out,
                         int* out, int out_cap, int* pos, cudaStream_t st);
 
