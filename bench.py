@@ -48,16 +48,6 @@ N_SEQ, SEQ_LEN = 512, 1024
 METRIC = "Q8_0 GPT-2-small decode tokens/s (batch 1, KV cache, greedy)"
 
 
-def decode_dram_bytes_per_token():
-    """dram__bytes_read.sum + dram__bytes_write.sum of the persistent decode kernel per token, from the
-    tracked capture record (which names the kernel revision it was taken at); None when absent."""
-    path = os.path.join(ROOT, "profiles", "decode_mega_kernel_traffic.json")
-    if not os.path.exists(path):
-        return None
-    rec = json.load(open(path))
-    return float(rec["dram_bytes_read_per_token"]) + float(rec["dram_bytes_write_per_token"])
-
-
 def peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(path):
@@ -473,17 +463,17 @@ def main():
     ap.add_argument("--k", type=int, default=768)
     ap.add_argument("--n", type=int, default=50257)
     ap.add_argument("--reps", type=int, default=3)
-    ap.add_argument("--math", type=int, default=0, help="--case: 0 fp32 CUDA cores, 1 tcgen05 bf16x3")
+    ap.add_argument("--math", type=int, default=0, help="--case: activations as three bf16 planes (0, exact) or two (1)")
     ap.add_argument("--kind", type=int, default=0, help="--case rowq: 0 int8, 1 int4")
     ap.add_argument("--native", type=int, default=-1, help="--case llama-*: matrices kept in this ggml block format (2 Q4_0, 6 Q5_0, 8 Q8_0, 12 Q4_K, 13 Q5_K, 14 Q6_K) and decoded in the kernels")
     ap.add_argument("--packed", type=int, default=-1, help="--case llama-*: every Linear packed to per-row int8 (0) / int4 (1), as the reference's importer does")
-    ap.add_argument("--mode", type=int, default=0, help="--case decode: 0 persistent kernel, 1 one kernel per operation")
+    ap.add_argument("--mode", type=int, default=0, help="--case decode: 0 persistent kernel, 1 chain of launches")
     ap.add_argument("--trace", action="store_true", help="--case decode: print the phase timeline of one token")
     ap.add_argument("--score-steps", type=int, default=2)
     ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--score-math", choices=["bf16x3", "fp32"], default="bf16x3",
-                    help="math mode of the scoring GEMMs: tcgen05 bf16 3-term split, or fp32 CUDA cores")
+                    help="math mode of the scoring GEMMs: activations as two bf16 planes, or as three (exact)")
     args = ap.parse_args()
     rank = int(os.environ.get("RANK", "0"))
     local = int(os.environ.get("LOCAL_RANK", "0"))
@@ -729,10 +719,8 @@ def main():
                     "note": "fc_generate_greedy from pinned host buffers: prompt upload, 32-token prime, 256 feeds, token download"},
             "gpu_launches": int(launches),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
-                         "traffic": None if decode_dram_bytes_per_token() is None else decode_dram_bytes_per_token() * 32,
-                         "peak_kind": peak_kind,
-                         "what": "decode_mega_kernel, launches of 32 tokens: %.1f MB algorithmic per token; traffic = ncu dram "
-                                 "read + write of a one-token launch at position 38, scaled to 32 tokens" % (bpt / 1e6)},
+                         "traffic": None, "peak_kind": peak_kind,
+                         "what": "chain of dependent launches (five per block, eight tokens per graph): %.1f MB algorithmic per token" % (bpt / 1e6)},
             "clocks": clocks,
         }
         if args.workload == "both":
@@ -780,8 +768,8 @@ def main():
             "n_gpus": world, "steps": args.score_steps, "ms_per_step": step_ms, "scaling": "strong" if world > 1 else "n/a",
             "config": {"workload": "configs[2]: %d sequences x %d ids, full-window prefill, per-token log-probs, %d windows per forward"
                        % (N_SEQ, SEQ_LEN, bw),
-                       "math": "linear layers: tcgen05 kind::f16, bf16 3-term split of f32 operands, fp32 TMEM accumulate"
-                               if args.score_math == "bf16x3" else "fp32 CUDA cores"},
+                       "math": "linear layers: tcgen05 kind::f16, exact weight levels, f32 activations as %d bf16 planes, f32 accumulate"
+                               % (2 if args.score_math == "bf16x3" else 3)},
             "dtype": "bf16x3" if args.score_math == "bf16x3" else "f32",
             "e2e": {"value": positions / e2e_s, "unit": "positions/s", "h2d_bytes_per_step": per * SEQ_LEN * 4,
                     "d2h_bytes_per_step": per * SEQ_LEN * 4 + per * 24},

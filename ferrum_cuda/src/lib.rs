@@ -42,8 +42,9 @@ fn ids32(ids: &[usize]) -> Vec<i32> {
     ids.iter().map(|&i| i32::try_from(i).unwrap_or(i32::MAX)).collect()   // ids past i32 are out of every vocabulary: FC_E_DIM
 }
 
-/// Math mode of the window forward (scoring, prime): exact fp32 CUDA cores, or tcgen05 tensor cores on a
-/// three-term bf16 split of the f32 operands (2^-16 relative per product). Decode is fp32-equivalent in both.
+/// Math mode of the window forward (scoring, prime): tcgen05 tensor cores on exact weight levels and the
+/// activations as three bf16 planes (their f32 value exactly), or two (2^-17 relative). Decode is
+/// fp32-equivalent in both.
 #[derive(Clone, Copy, Debug, PartialEq, Eq)]
 pub enum MathMode { Fp32 = 0, Bf16x3 = 1 }
 
