@@ -1136,10 +1136,10 @@ __global__ void bump_state_kernel(StepState* st, int by) {
 // cache the same rows come out of ONE window forward (TransformerBlock::forward,
 // layer/transformer.rs:314-534, equals forward_with_cache row by row: transformer.rs:669-716),
 // so the n ids in queue[0..n) of each of the S streams go through every block as S windows of
-// n rows in fp32, each block's K and V rows are copied into the streams' caches, and only the
+// n rows, each block's K and V rows are copied into the streams' caches, and only the
 // last row of a window meets the head.
-// Very short prompts stay on the token-by-token path (one persistent-kernel launch); up to 64
-// rows the GEMMs run on small tiles so that every SM gets one.
+// Very short prompts stay on the token-by-token path (one persistent-kernel launch); with few
+// rows the GEMMs split K over a cluster so that more SMs take part.
 // Returns FC_OK with *used = 0 when the shape is not covered (the caller feeds token by token).
 constexpr int kPrimeBatchMin = 8;
 static int prime_batched(fc_stream* const* ss, int S, int n, int last_mode, int* used, float* const* kcs_dev = nullptr,

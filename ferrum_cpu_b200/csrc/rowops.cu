@@ -1,5 +1,5 @@
 // Row kernels of the forward path: embedding gather, LayerNorm, the decode tail
-// (softmax statistics + greedy select) and the scoring tail (per-target log-prob).
+// (probabilities or greedy select behind a head that left statistics) and the layer statistics.
 
 #include <algorithm>
 

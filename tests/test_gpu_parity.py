@@ -366,7 +366,7 @@ def test_small_scoring_is_batch_invariant_and_causal(small):
     assert np.array_equal(lpb[0, :600], lp1[0, :600]) and not np.array_equal(lpb[0, 600:], lp1[0, 600:])
 
 
-# ---- tensor-core math mode (bf16 3-term split on tcgen05) ----------------------------------
+# ---- two-plane math mode (activations as two bf16 planes) -----------------------------------
 @pytest.mark.parametrize("m,k,n", [(2, 64, 96), (129, 192, 257), (128, 768, 128), (512, 768, 3072), (300, 3072, 768),
                                    (4096, 1024, 4096)])
 def test_q8_0_linear_bf16x3_matches_engine(m, k, n):
@@ -379,7 +379,7 @@ def test_q8_0_linear_bf16x3_matches_engine(m, k, n):
     scale = np.abs(want).max()
     err = np.abs(got - want).max()
     assert err <= 1e-4 * scale, f"max abs err {err:.3e} vs scale {scale:.3e}"
-    # the fp32 CUDA-core kernel is the yardstick: both modes agree far inside the tolerance
+    # the f32 mode is the yardstick: both modes agree far inside the tolerance
     got32 = fcb.q8_0_linear(x, wq, bias, n, math_mode=fcb.FC_MATH_FP32)
     assert np.abs(got - got32).max() <= 1e-4 * scale
 
