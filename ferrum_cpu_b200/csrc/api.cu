@@ -2,6 +2,7 @@
 // the KV-cached decode driver. Host logic above the kernels mirrors, in C++, the Rust items
 // cited in include/ferrum_cuda.h.
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -65,21 +66,33 @@ int upload_q8(Arena& ar, const void* host, int N, int K, QMat* out, cudaStream_t
     uint8_t* raw = nullptr;
     uint8_t* qu = nullptr;
     __half* d = nullptr;
-    FC_CUDA(cudaMalloc((void**)&raw, raw_bytes));
+    const size_t top_at = (raw_bytes + 15) & ~(size_t)15;   // the largest scale's word behind the blocks
+    unsigned top = 0;
+    FC_CUDA(cudaMalloc((void**)&raw, top_at + 16));
     int rc = ar.alloc_n(&qu, (size_t)N_pad * K);
     if (rc == FC_OK) rc = ar.alloc_n(&d, (size_t)N_pad * (K / 32));
     if (rc == FC_OK && cudaMemcpyAsync(raw, host, raw_bytes, cudaMemcpyHostToDevice, st) != cudaSuccess)
         rc = fail(FC_E_CUDA, "upload of a Q8_0 tensor failed");
-    if (rc == FC_OK) rc = launch_repack_q8(raw, N, K, N_pad, qu, d, st);
+    if (rc == FC_OK && cudaMemsetAsync(raw + top_at, 0, 16, st) != cudaSuccess) rc = fail(FC_E_CUDA, "upload of a Q8_0 tensor failed");
+    if (rc == FC_OK) rc = launch_repack_q8(raw, N, K, N_pad, qu, d, (unsigned*)(raw + top_at), st);
+    if (rc == FC_OK && cudaMemcpyAsync(&top, raw + top_at, sizeof(top), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+        rc = fail(FC_E_CUDA, "repack of a Q8_0 tensor failed");
     if (rc == FC_OK && cudaStreamSynchronize(st) != cudaSuccess) rc = fail(FC_E_CUDA, "repack of a Q8_0 tensor failed");
     cudaFree(raw);
     FC_TRY(rc);
     out->qu = qu; out->d = d; out->N = N; out->K = K; out->N_pad = N_pad;
+    out->f16_exact = top < 0x5FFFu;                          // up to 511.5, and 511.5 x 128 < 65504
     return FC_OK;
 }
 
+// A block's matrices as f16 planes and the scales of the activation planes that meet them (gemm_f16.cu).
+struct LayerF16 {
+    F16Mat qkv, out, up, down;
+    float n1 = 0.0f, att = 0.0f, n2 = 0.0f, hid = 0.0f;
+};
 struct LayerDev {
     QMat qkv, out, up, down;
+    LayerF16 f16;
     float *qkv_b, *out_b, *up_b, *down_b, *ln1g, *ln1b, *ln2g, *ln2b;
 };
 
@@ -190,6 +203,9 @@ struct fc_model {
     float* pos = nullptr;
     float *lnfg = nullptr, *lnfb = nullptr;
     std::vector<LayerDev> layers;
+    bool f16 = false;                          // the two-plane mode runs on f16 planes: LayerDev::f16, and
+    F16Mat head_f16;
+    float lnf_scale = 0.0f;
     // prefill workspace for ws_rows rows
     int ws_rows = 0, ws_planes = 0;
     float *x = nullptr, *qkv = nullptr, *att = nullptr, *logits = nullptr, *probs_d = nullptr;
@@ -401,6 +417,67 @@ static int model_planes(const fc_model* m) {
     const fc_config& c = m->cfg;
     return c.math_mode == FC_MATH_BF16X3 && c.d_model % 64 == 0 && c.d_ff % 64 == 0 ? 2 : 3;
 }
+// The matrices of a two-plane model as f16 planes, and the scales of the activation planes. A scale is the largest power of two
+// that keeps scale x bound within f16, where the bound holds for every input: a LayerNorm's row has norm at most sqrt(d) max|g| +
+// |b|, an element of a product at most the norm of its weight row times that (+ bias), a mixture of value rows and GELU at
+// most what goes into them. The 1 % is for rounding. Without memory for the planes (4 bytes a weight), with a matrix that f16
+// cannot hold or a bound that is not a finite number, the model stays on the level GEMM.
+static int build_f16(fc_model* m, const fc_weights* w) {
+    const fc_config& c = m->cfg;
+    const int d = c.d_model, F = c.d_ff;
+    bool ok = m->head.f16_exact;
+    size_t weights = (size_t)c.vocab * d;
+    for (const LayerDev& L : m->layers) {
+        ok = ok && L.qkv.f16_exact && L.out.f16_exact && L.up.f16_exact && L.down.f16_exact;
+        weights += (size_t)4 * d * d + (size_t)2 * d * F;
+    }
+    if (!ok) return FC_OK;
+    void* mem = nullptr;
+    const size_t tops_at = weights * 4, tops_bytes = (size_t)c.n_layer * 2 * sizeof(unsigned);
+    const cudaError_t e = cudaMalloc(&mem, tops_at + tops_bytes);
+    if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); return FC_OK; }
+    FC_CUDA(e);
+    m->arena.ptrs.push_back(mem);
+    unsigned* tops_d = (unsigned*)((char*)mem + tops_at);
+    FC_CUDA(cudaMemsetAsync(tops_d, 0, tops_bytes, m->st));
+    char* at = (char*)mem;
+    auto make = [&](const QMat& q, F16Mat* f, int from, unsigned* top) -> int {
+        const size_t bytes = (size_t)q.N * q.K * 2;
+        *f = F16Mat{at, at + bytes, q.N, q.K};
+        at += 2 * bytes;
+        return launch_f16_planes(nullptr, 0, 4, Planes(), nullptr, q, *f, from, top, m->st);
+    };
+    FC_TRY(make(m->head, &m->head_f16, 0, nullptr));
+    for (int l = 0; l < c.n_layer; ++l) {
+        LayerDev& L = m->layers[l];
+        FC_TRY(make(L.qkv, &L.f16.qkv, 2 * d, tops_d + 2 * l));     // the value rows
+        FC_TRY(make(L.out, &L.f16.out, 0, nullptr));
+        FC_TRY(make(L.up, &L.f16.up, 0, tops_d + 2 * l + 1));
+        FC_TRY(make(L.down, &L.f16.down, 0, nullptr));
+    }
+    std::vector<float> tops((size_t)c.n_layer * 2);
+    FC_CUDA(cudaMemcpyAsync(tops.data(), tops_d, tops_bytes, cudaMemcpyDeviceToHost, m->st));
+    FC_CUDA(cudaStreamSynchronize(m->st));
+    auto most = [](const float* v, size_t n) { double t = 0; for (size_t i = 0; i < n; ++i) t = v[i] != v[i] ? INFINITY : std::max(t, std::fabs((double)v[i])); return t; };
+    auto norm = [](const float* v, size_t n) { double t = 0; for (size_t i = 0; i < n; ++i) t += (double)v[i] * v[i]; return std::sqrt(t); };
+    auto scale = [&](double bound) -> float {
+        bound *= 1.01;
+        ok = ok && bound < 1e30;                                     // false for NaN too
+        return ok && bound > 0 ? (float)std::exp2(std::min(15.0, std::floor(std::log2(65504.0 / bound)))) : 1.0f;
+    };
+    const double root = std::sqrt((double)d);
+    for (int l = 0; l < c.n_layer; ++l) {
+        const fc_layer_weights& s = w->layers[l];
+        LayerF16& f = m->layers[l].f16;
+        f.n1 = scale(root * most(s.ln1_g, d) + most(s.ln1_b, d));
+        f.n2 = scale(root * most(s.ln2_g, d) + most(s.ln2_b, d));
+        f.att = scale(std::sqrt((double)tops[2 * l]) * (root * most(s.ln1_g, d) + norm(s.ln1_b, d)) + most(s.attn_qkv_b + 2 * d, d));
+        f.hid = scale(std::sqrt((double)tops[2 * l + 1]) * (root * most(s.ln2_g, d) + norm(s.ln2_b, d)) + most(s.ffn_up_b, F));
+    }
+    m->lnf_scale = scale(root * most(w->out_norm_g, d) + most(w->out_norm_b, d));
+    m->f16 = ok;
+    return FC_OK;
+}
 // Whether the window attention runs on the tensor cores (heads of 64).
 static bool tensor_attention(const fc_model* m) { return m->cfg.d_model == m->cfg.n_head * 64; }
 
@@ -449,7 +526,12 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
     const int d = c.d_model, F = c.d_ff;
     cudaStream_t st = m->st;
     const bool tc_attn = tensor_attention(m);
+    const bool f16 = planes == 2 && m->f16;
     m->pn.n = m->pqkv.n = m->patt.n = m->phid.n = planes;
+    auto product = [&](const QMat& q, const F16Mat& h, const Planes& x, const float* bias, const float* residual, int epi, float* y, const Planes* yp) {
+        return f16 ? launch_gemm_f16(h, x, nullptr, bias, residual, epi, y, yp, R, q.N, status, st)
+                   : launch_gemm_q8_tc(q, x, bias, residual, epi, y, yp, R, q.N, status, st, split_k);
+    };
     FC_CUDA(cudaMemsetAsync(m->err_d, 0, sizeof(int), st));
     FC_TRY(launch_embed_rows(m->tok, m->pos, ids, pos, R, win.T, m->x, m->err_d, st));
     // model.rs:58-68: with the statistics switched on, every layer's output is summarised as it appears
@@ -461,11 +543,14 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
     FC_TRY(layer_stats());
     for (int l = 0; l < c.n_layer; ++l) {
         const LayerDev& L = m->layers[l];
+        m->pn.scale = f16 ? L.f16.n1 : 0.0f;
+        m->patt.scale = f16 ? L.f16.att : 0.0f;
+        m->phid.scale = f16 ? L.f16.hid : 0.0f;
         FC_TRY(launch_layernorm_planes(m->x, L.ln1g, L.ln1b, nullptr, R, d, m->pn, st));
         if (tc_attn && !f32_qkv) {
-            FC_TRY(launch_gemm_q8_tc(L.qkv, m->pn, L.qkv_b, nullptr, EPI_NONE, nullptr, &m->pqkv, R, 3 * d, status, st, split_k));
+            FC_TRY(product(L.qkv, L.f16.qkv, m->pn, L.qkv_b, nullptr, EPI_NONE, nullptr, &m->pqkv));
         } else {
-            FC_TRY(launch_gemm_q8_tc(L.qkv, m->pn, L.qkv_b, nullptr, EPI_NONE, m->qkv, nullptr, R, 3 * d, status, st, split_k));
+            FC_TRY(product(L.qkv, L.f16.qkv, m->pn, L.qkv_b, nullptr, EPI_NONE, m->qkv, nullptr));
             FC_TRY(on_qkv(l));
             if (tc_attn) FC_TRY(launch_split_planes(m->qkv, m->pqkv, (size_t)R * 3 * d, st));
         }
@@ -473,12 +558,13 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
             FC_TRY(launch_attn_prefill_tc(m->pqkv, win, R, d, c.n_head, m->patt, status, st));
         } else {
             FC_TRY(launch_attn_prefill(m->qkv, win, d, c.n_head, m->att, st));
-            FC_TRY(launch_split_planes(m->att, m->patt, (size_t)R * d, st));
+            FC_TRY(f16 ? launch_split_f16(m->att, m->patt, (size_t)R * d, st) : launch_split_planes(m->att, m->patt, (size_t)R * d, st));
         }
-        FC_TRY(launch_gemm_q8_tc(L.out, m->patt, L.out_b, m->x, EPI_NONE, m->x, nullptr, R, d, status, st, split_k));
+        FC_TRY(product(L.out, L.f16.out, m->patt, L.out_b, m->x, EPI_NONE, m->x, nullptr));
+        m->pn.scale = f16 ? L.f16.n2 : 0.0f;
         FC_TRY(launch_layernorm_planes(m->x, L.ln2g, L.ln2b, nullptr, R, d, m->pn, st));
-        FC_TRY(launch_gemm_q8_tc(L.up, m->pn, L.up_b, nullptr, EPI_GELU, nullptr, &m->phid, R, F, status, st, split_k));
-        FC_TRY(launch_gemm_q8_tc(L.down, m->phid, L.down_b, m->x, EPI_NONE, m->x, nullptr, R, d, status, st, split_k));
+        FC_TRY(product(L.up, L.f16.up, m->pn, L.up_b, nullptr, EPI_GELU, nullptr, &m->phid));
+        FC_TRY(product(L.down, L.f16.down, m->phid, L.down_b, m->x, EPI_NONE, m->x, nullptr));
         FC_TRY(layer_stats());
     }
     return FC_OK;
@@ -489,6 +575,7 @@ static int score_device(fc_model* m, const ScoreSlot& s, const Windows& win, int
     const int d = c.d_model, n = s.picked;
     const int *ids = (const int*)s.in_d, *pos = ids + R, *pick = pos + R + win.B + 1, *targets = pick + n;
     FC_TRY(forward_blocks_with(m, win, R, ids, pos, model_planes(m), s.status_d(), false, false, [](int) { return FC_OK; }));
+    m->pn.scale = 0.0f;
     if (m->stats_on) {
         FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, nullptr, R, d, m->pn, m->st));
         FC_TRY(launch_layer_stats(nullptr, m->pn, (size_t)R * d, m->stats_scratch, m->stats_d + m->stats_n++, m->st));
@@ -496,8 +583,11 @@ static int score_device(fc_model* m, const ScoreSlot& s, const Windows& win, int
     if (n == 0) return FC_OK;               // the forward was for its statistics
     // the head's epilogue keeps (max, sum of exponentials, first argmax) per row and 128-column tile and the
     // target's logit: [rows][V] logits never reach memory (scoring.rs:175-181 needs one number per row)
+    const bool f16 = m->pn.n == 2 && m->f16;
+    if (f16) m->pn.scale = m->lnf_scale;
     FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, n == R ? nullptr : pick, n, d, m->pn, m->st));
-    FC_TRY(launch_gemm_q8_tc_score(m->head, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
+    if (f16) FC_TRY(launch_gemm_f16_score(m->head_f16, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
+    else FC_TRY(launch_gemm_q8_tc_score(m->head, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
     return launch_score_combine(m->head_stats, m->head_tlogit, targets, n, (c.vocab + 127) / 128, c.vocab, s.lp_d(), s.gr_d(), m->st);
 }
 
@@ -574,6 +664,20 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
     const size_t n = (size_t)M * w->w.K;
     CallScratch scratch;
     Planes x;
+    if (planes == 2 && w->w.f16_exact && f16_rows(w->w.K, M)) {
+        // both operands as f16 planes, and the rows' scales behind them
+        const size_t nw = (size_t)w->w.N * w->w.K;
+        FC_TRY(scratch.take(w->device, 4 * (n + nw + M), st));
+        if (scratch.p) {
+            __half* p = (__half*)scratch.p;
+            const F16Mat wp = {p, p + nw, w->w.N, w->w.K};
+            p += 2 * nw;
+            x.p[0] = p; x.p[1] = p + n; x.n = 2; x.scale = 1.0f;
+            float* row_inv = (float*)(p + 2 * n);
+            FC_TRY(launch_f16_planes(x_dev, M, w->w.K, x, row_inv, w->w, wp, 0, nullptr, st));
+            return launch_gemm_f16(wp, x, row_inv, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, w->status.dev, st);
+        }
+    }
     FC_TRY(take_planes(scratch, x, planes, n, w->device, st));
     if (!scratch.p) return launch_rows_alone(part, w->w.K, x_dev, M, st);   // no memory for the planes
     FC_TRY(launch_split_planes(x_dev, x, n, st));
@@ -638,6 +742,7 @@ static int model_build(fc_model* m, const fc_weights* w) {
         FC_TRY(upload_f32(a, s.ln2_g, d, &L.ln2g, st));
         FC_TRY(upload_f32(a, s.ln2_b, d, &L.ln2b, st));
     }
+    if (model_planes(m) == 2) FC_TRY(build_f16(m, w));
     if (mega_supported(c)) {
         int full = 0;
         FC_TRY(mega_max_grid(&full));

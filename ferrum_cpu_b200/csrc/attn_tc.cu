@@ -22,8 +22,7 @@
 // Every mbarrier wait is bounded; on a timeout the status word is raised and the CTA leaves.
 //
 // Bound: tensor pipe / MUFU. 4·hd·T(T+1)/2 algorithmic FLOP per (window, head).
-#include <cuda.h>
-#include "planes.cuh"
+#include "tc.cuh"
 
 namespace fc {
 
@@ -140,7 +139,8 @@ struct AttnArgs {
     int k_col, v_col;            // first column of the key / value heads in the fused q | k | v planes
     int group;                   // query heads per key / value head (1: multi-head attention)
     int ldo;                     // row stride of the output planes (= query heads x 64)
-    uint16_t* out[3];            // [R][ldo] bf16 planes
+    uint16_t* out[3];            // [R][ldo] bf16 planes, or
+    float out_scale;             // not 0: two f16 planes of out_scale times the output
     int* status;
 };
 
@@ -155,7 +155,7 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     Bars* bars = (Bars*)(smem + OFF_BARS);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int qt = (gridDim.x - 1) - blockIdx.x;          // long (late) query tiles first
     const int h = blockIdx.y, b = blockIdx.z;
     const int T = a.win.length(b), row0 = a.win.begin(b); // the window's rows in [R]
@@ -181,10 +181,10 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = bars->tmem_base;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
 
     if (warp == TMA_WARP) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             mbar_expect_tx(&bars->q_full, P * Q_BYTES);
 #pragma unroll
             for (int p = 0; p < P; ++p) tma_load_2d(smem + OFF_Q + p * Q_BYTES, &maps.q[p], h * HD, row0 + q0, &bars->q_full);
@@ -201,7 +201,7 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
             }
         }
     } else if (warp == MMA_WARP) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t sb = s32(smem);
             const uint64_t dq = smem_desc(sb + OFF_Q), dk = smem_desc(sb + OFF_K), dv = smem_desc(sb + OFF_V), dp = smem_desc(sb + OFF_P);
             constexpr uint64_t QS = Q_BYTES / 16, KS = KV_BYTES / 16, PS = P_BYTES / 16;   // from plane to plane, in descriptor units
@@ -321,7 +321,12 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
             for (int c = 0; c < HD / 8; ++c) {
                 uint32_t w[4][P];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) split2<P>(o[8 * c + 2 * e] * inv, o[8 * c + 2 * e + 1] * inv, w[e]);
+                for (int e = 0; e < 4; ++e) {
+                    const float v0 = o[8 * c + 2 * e] * inv, v1 = o[8 * c + 2 * e + 1] * inv;
+                    if constexpr (P == 2)
+                        if (a.out_scale != 0.0f) { split2_f16(v0 * a.out_scale, v1 * a.out_scale, w[e]); continue; }
+                    split2<P>(v0, v1, w[e]);
+                }
 #pragma unroll
                 for (int t = 0; t < P; ++t) *(uint4*)(a.out[t] + off + 8 * c) = make_uint4(w[0][t], w[1][t], w[2][t], w[3][t]);
             }
@@ -383,6 +388,7 @@ static int launch_attn_tc(const Planes& qkv, const Windows& w, int R, int H, int
         a.out[p] = (uint16_t*)out.p[p];
     }
     a.win = w; a.k_col = H * HD; a.v_col = (H + KV) * HD; a.group = H / KV; a.ldo = H * HD;
+    a.out_scale = out.scale;
     a.status = status;
     dim3 grid((w.T + QT - 1) / QT, H, w.B);
     attn_prefill_tc_kernel<P><<<grid, THREADS, SMEM_BYTES<P>, st>>>(maps, a);

@@ -104,8 +104,14 @@ struct QMat {
     const uint8_t* qu = nullptr;
     const __half* d = nullptr;
     int N = 0, K = 0, N_pad = 0;
+    bool f16_exact = false;   // two f16 planes hold every weight exactly (largest scale x 128 within f16); else unknown
 };
 constexpr int kRowPad = 128;
+// A Q8_0 matrix as two f16 planes [N][K] whose sum it is, exactly (gemm_f16.cu).
+struct F16Mat {
+    void *hi = nullptr, *lo = nullptr;
+    int N = 0, K = 0;
+};
 
 enum Epilogue : int { EPI_NONE = 0, EPI_GELU = 1, EPI_SWIGLU = 2 };
 
@@ -133,7 +139,8 @@ struct StepState {
 
 // ---- kernel launchers (each returns FC_OK or FC_E_CUDA) --------------------------------
 // repack.cu
-int launch_repack_q8(const uint8_t* raw, int N, int K, int N_pad, uint8_t* qu, __half* d, cudaStream_t st);
+// top: a zeroed word, raised to the bits of the largest |scale|.
+int launch_repack_q8(const uint8_t* raw, int N, int K, int N_pad, uint8_t* qu, __half* d, unsigned* top, cudaStream_t st);
 
 // gemv_row.cu — one activation row against up to three matrices (q | k | v, gate | up) of the same K. part.d: f16 scales per
 // 32 of k, or null with part.xscale [K]: the scale of input index k (then levels alone); EPI_SWIGLU pairs rows (2i, 2i + 1) of one matrix, or row i of two, as (gate, up) and writes
@@ -186,10 +193,12 @@ struct Windows {
 };
 
 // An f32 matrix as n bf16 planes whose sum it is: 2 planes hold it to 2^-17 relative (FC_MATH_BF16X3), 3 exactly
-// (FC_MATH_FP32). The form in which activations reach the tensor cores.
+// (FC_MATH_FP32). The form in which activations reach the tensor cores. With a scale (a power of two) they are two f16 planes of
+// scale times the matrix, for gemm_f16.cu; whoever sets it vouches for scale x values within f16's range.
 struct Planes {
     void* p[3] = {nullptr, nullptr, nullptr};
     int n = 0;
+    float scale = 0.0f;
 };
 // Planes of n elements out of a call's scratch; scratch.p stays null when there is no memory.
 int take_planes(CallScratch& scratch, Planes& x, int planes, size_t n, int device, cudaStream_t st);
@@ -211,6 +220,19 @@ int launch_gemm_q8_tc_score(const QMat& w, const Planes& x, const int* targets, 
                             cudaStream_t st);
 int launch_score_combine(const void* stats, const float* tlogit, const int* targets, int M, int n_tiles, int V, double* logprob,
                          uint8_t* is_greedy, cudaStream_t st);
+
+// gemm_f16.cu — the same two entries on weights and activations as f16 planes. row_inv (may be null): 1 / scale of each row of x in
+// place of x.scale. Plane output: bf16, or behind GELU f16 of yp->scale. A row's result does not depend on the rows beside it.
+int launch_gemm_f16(const F16Mat& w, const Planes& x, const float* row_inv, const float* bias, const float* residual, int epi, float* y, const Planes* yp,
+                    int M, int ldy, int* status, cudaStream_t st);
+int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st);
+// x [M][K] as f16 planes scaled row by row (row_inv [M]: 1 / scale) and w as exact f16 planes, in one launch; either may be empty.
+// top (may be null): raised to the bits of the largest square norm of the weight rows from `from` on (finite and positive).
+int launch_f16_planes(const float* x, int M, int K, const Planes& out, float* row_inv, const QMat& w, const F16Mat& planes, int from, unsigned* top,
+                      cudaStream_t st);
+// Whether a caller's own two-plane product of M rows is better off there.
+bool f16_rows(int K, int M);
+int launch_split_f16(const float* x, const Planes& out, size_t n, cudaStream_t st);
 
 // api.cu — the matrix and device behind a resident-weight handle.
 const QMat* qweight_matrix(const fc_qweight* w, int* device);

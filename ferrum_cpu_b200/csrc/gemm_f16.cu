@@ -1,0 +1,579 @@
+// Q8_0 GEMM with the weight as two f16 planes:
+//     Y[M][N] = X[M][K] · dequant(W[N][K])ᵀ + bias (+GELU) (+residual), or the softmax records of the LM head
+//
+// The product of the two-plane math mode (FC_MATH_BF16X3). A Q8_0 weight d·q has at most 19 significant bits (11 of the f16
+// scale, 8 of the level) and is a whole multiple of 2^-24, so hi = f16(d·q) and lo = d·q - hi hold it EXACTLY, as long as
+// d·128 does not overflow f16 (QMat::f16_exact, checked at upload). An activation, scaled by a power of two that keeps it in
+// range, is hi + lo to 2^-24 relative: as close as f32 itself. Three MMAs per step, hi·hi + hi·lo + lo·hi, drop 2^-24 of a
+// product, and no scale is left to apply: k-blocks add up in TMEM, and the tensor pipe is what bounds the kernel.
+//
+// gemm_tc.cu multiplies the levels instead (two MMAs per step with bf16 planes of x) and has to fold every 32-wide k-block
+// into registers by the block's scale: its drain is what bounds it, at half the rate of the pipe, and its two bf16 planes of x
+// leave 2^-17. It stays for the f32 mode, whose sums may not be truncated as often as here (below), for matrices that f16
+// does not hold, and for few rows of a caller's own, where 4 bytes a weight would be what counts.
+//
+// The tensor core truncates its f32 sums: towards zero, once per MMA. Over all of K that is 1.05e-9 of the result per k (measured
+// on one MMA per 16 k: 1.1e-6 at K = 1024, 4.2e-6 at 4096; three times as much here), where two bf16 planes of x are 2.5e-6 off
+// whatever K is. So sums stay in TMEM for KGROUP stages and then go into f32 registers, rounded to nearest. Error against 64 bits at
+// K = 1024 (relative, 2-norm): 3.8e-7 with 2 stages a group, 7.6e-7 with 4, 1.7e-6 with 8; 4096 x 1024 x 4096 takes the same time with
+// 4 as with 8.
+//
+// One CTA per SM, 640 threads (registers 104 a thread of the drain, 64 of the others):
+//   warps 0-15  drain: a group's sums from TMEM into registers (lane = weight row, column = activation row); after the last
+//               group bias / GELU / residual or the softmax records, and the stores. With 8 warps of twice the columns the GELU
+//               epilogue was latency-bound: 32768 x 768 x 3072 390 us, now 298
+//   warp 16     TMA: both planes of the weight and of the activations, 64 k a stage
+//   warp 17     MMA issue and the TMEM allocation: two buffers of up to 256 columns, so that a group is read while the next runs.
+//               One elected thread (tc.cuh: elect_one) issues an MMA in about 30 cycles; behind lane == 0 it took 74
+// CG = 2: a pair of CTAs shares a tile of 256 weight rows (each holds 128 of them and half of the activation rows). CG = 1
+// takes few rows. The order of a row's sums depends on K alone, so a row's result does not depend on the rows beside it.
+//
+// Bound: the tensor pipe at the clock the power limit leaves. A stage of a 256-row tile takes 1547 cycles, its MMAs 1536. In a loop of
+// their own, with the planes made (levels in gemm_tc.cu): 4096 x 1024 x 4096 73 us (109), 32768 x 768 x 2304 239 us = 1.46 PFLOP/s executed
+// (348), 32768 x 3072 x 768 322 us (450).
+//
+// Every wait is bounded; a wait that runs out raises the status word and all roles leave.
+#include <algorithm>
+#include <type_traits>
+
+#include "pdl.cuh"
+#include "tc.cuh"
+
+namespace fc {
+
+using namespace tc;
+
+namespace {
+
+constexpr int BK = 64;                                  // k per stage: one 128-byte swizzle row of f16
+constexpr int KGROUP = 4;                               // stages whose sums stay in TMEM
+constexpr int W_BYTES = 128 * BK * 2;                   // one plane of the CTA's weight tile of a stage
+constexpr int DRAIN_WARPS = 16, TMA_WARP = 16, MMA_WARP = 17, THREADS = 640;
+constexpr int MAX_STAGES = 6;
+constexpr int TMEM_COLS = 512, ACC_COLS = 256;
+constexpr int SMEM_LIMIT = 227 * 1024;
+
+enum Mode : int { OUT_F32 = 0, OUT_BF16 = 1 /* bf16 planes */, OUT_GELU = 2 /* f16 planes, after GELU */, OUT_SCORE = 3 };
+
+struct F16Args {
+    int N, K, M, stages;
+    const float* bias; const float* residual; int gelu;
+    float inv;                // what takes the scale of x out of a sum (a power of two)
+    const float* row_inv;     // the same per activation row, or null
+    float* y; int ldy;        // OUT_F32
+    uint16_t* yp[2];          // OUT_BF16, OUT_GELU: planes, ldy elements apart
+    float out_scale;          // OUT_GELU: scale of the planes
+    const int* targets; float4* stats; float* tlogit;      // OUT_SCORE
+    int* status;
+    long long wait_cycles;
+    int withhold;
+};
+
+constexpr int BAR_FULL = 0, BAR_EMPTY = BAR_FULL + 8 * MAX_STAGES, BAR_ACC_FULL = BAR_EMPTY + 8 * MAX_STAGES, BAR_ACC_EMPTY = BAR_ACC_FULL + 16;
+constexpr int BAR_TMEM = BAR_ACC_EMPTY + 16, BAR_ABORT = BAR_TMEM + 4, BAR_BYTES = BAR_ABORT + 4;
+
+__device__ __forceinline__ void add2(uint64_t& acc, uint64_t v) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(v)); }
+
+}  // namespace
+
+// CW: columns (activation rows) of a drain warp, a quarter of the tile's.
+template <int CG, int CW, int MODE>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ CUtensorMap wl, const __grid_constant__ CUtensorMap xh,
+                const __grid_constant__ CUtensorMap xl, const F16Args a) {
+    constexpr int NT = 4 * CW, XR = NT / CG;                                        // activation rows of a tile, of this CTA's memory
+    constexpr int X_BYTES = XR * BK * 2, STAGE = 2 * W_BYTES + 2 * X_BYTES;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024 - (s32(smem_raw) & 1023)) & 1023);
+    float4* recs = (float4*)(smem + a.stages * STAGE);                              // OUT_SCORE: [4 quarters][NT]
+    unsigned char* tail = (unsigned char*)recs + (MODE == OUT_SCORE ? 4 * NT * 16 : 0);
+    volatile int* abort = (volatile int*)(tail + BAR_ABORT);
+    const uint32_t sb = s32(smem), full = s32(tail) + BAR_FULL, empty = s32(tail) + BAR_EMPTY;
+    const uint32_t acc_full = s32(tail) + BAR_ACC_FULL, acc_empty = s32(tail) + BAR_ACC_EMPTY;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int rank = CG == 2 ? (int)(blockIdx.x & 1) : 0;
+    const int group = blockIdx.x / CG, n_groups = gridDim.x / CG;                   // CTAs or pairs take tiles in turn
+    const int tiles_n = (a.N + 128 * CG - 1) / (128 * CG), tiles_m = (a.M + NT - 1) / NT;
+    const int n_tiles = tiles_n * tiles_m;
+    const int nst = (a.K + BK - 1) / BK;
+    const bool leader = rank == 0;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < a.stages; ++s) {
+            mbar_init(full + 8 * s, 1);
+            mbar_init(empty + 8 * s, 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(acc_full + 8 * b, 1);
+            mbar_init(acc_empty + 8 * b, DRAIN_WARPS * CG);
+        }
+        *abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == MMA_WARP) {
+        if (CG == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tail + BAR_TMEM)), "r"((uint32_t)TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tail + BAR_TMEM)), "r"((uint32_t)TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (CG == 2) {
+        __syncwarp();
+        cluster_sync();
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *(volatile uint32_t*)(tail + BAR_TMEM), 0);
+    pdl_wait();                                                                     // set up while the kernel ahead still ran
+    // the barriers the pair's MMA issuer waits on are the leader's
+    const uint32_t full_leader = CG == 2 ? mapa(full, 0) : full, acc_empty_leader = CG == 2 ? mapa(acc_empty, 0) : acc_empty;
+
+    // Every role ends here: nobody leaves while a peer may still reach this CTA's shared memory or barriers. After an
+    // aborted wait, copies and MMAs may be in flight for a few microseconds more: outstay them.
+    auto leave = [&]() {
+        __syncwarp();
+        if (*abort) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < 200000) __nanosleep(200);
+        }
+        __syncwarp();
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (CG == 2) cluster_sync();
+        else asm volatile("bar.sync 0, %0;" ::"n"(THREADS) : "memory");
+    };
+
+    if (warp >= TMA_WARP) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+        if (warp == TMA_WARP && !a.withhold && elect_one()) {
+            // ------------------------------------------------------------ TMA producer
+            int s = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int tile = group; tile < n_tiles && ok; tile += n_groups) {
+                const int n0 = (tile % tiles_n) * (128 * CG) + rank * 128, m0 = (tile / tiles_n) * NT + rank * XR;
+                for (int kb = 0; kb < nst; ++kb) {
+                    ok = wait_bar(empty + 8 * s, ph, abort, a);
+                    if (!ok) break;
+                    const uint32_t dst = sb + s * STAGE, bar = full_leader + 8 * s;
+                    if (leader) mbar_expect_tx(full + 8 * s, (uint32_t)(CG * STAGE));
+                    tma_load_2d<CG>(dst, &wh, kb * BK, n0, bar);
+                    tma_load_2d<CG>(dst + W_BYTES, &wl, kb * BK, n0, bar);
+                    tma_load_2d<CG>(dst + 2 * W_BYTES, &xh, kb * BK, m0, bar);
+                    tma_load_2d<CG>(dst + 2 * W_BYTES + X_BYTES, &xl, kb * BK, m0, bar);
+                    if (++s == a.stages) { s = 0; ph ^= 1; }
+                }
+            }
+        } else if (warp == MMA_WARP && leader && elect_one()) {
+            // ------------------------------------------------------------ MMA issuer
+            // f16 x f16 -> f32, M = 128 (256 for the pair), N = NT, both operands K-major
+            constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(8 * CG) << 24);
+            const uint64_t desc = smem_desc(sb);
+            const uint32_t dhi = (uint32_t)(desc >> 32);
+            uint32_t w = (uint32_t)desc, ph = 0, aph = 1;
+            int s = 0, buf = 0;
+            bool ok = true;
+            for (int tile = group; tile < n_tiles && ok; tile += n_groups) {
+                for (int kb = 0; kb < nst && ok; ++kb) {
+                    const bool first = kb % KGROUP == 0, last = kb % KGROUP == KGROUP - 1 || kb == nst - 1;
+                    ok = (!first || wait_bar(acc_empty + 8 * buf, aph, abort, a)) && wait_bar(full + 8 * s, ph, abort, a);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t acc = tmem + buf * ACC_COLS, x = w + 2 * W_BYTES / 16;      // descriptors count 16 bytes
+                    // the small terms first: they meet a small accumulator
+                    if (first) umma<CG, false>(acc, w + W_BYTES / 16, x, dhi, idesc);
+                    else umma<CG, true>(acc, w + W_BYTES / 16, x, dhi, idesc);
+#pragma unroll
+                    for (int k = 1; k < BK / 16; ++k) umma<CG, true>(acc, w + W_BYTES / 16 + 2 * k, x + 2 * k, dhi, idesc);
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k) umma<CG, true>(acc, w + 2 * k, x + X_BYTES / 16 + 2 * k, dhi, idesc);
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k) umma<CG, true>(acc, w + 2 * k, x + 2 * k, dhi, idesc);
+                    umma_commit<CG>(empty + 8 * s);
+                    if (last) {
+                        umma_commit<CG>(acc_full + 8 * buf);
+                        buf ^= 1;
+                        if (buf == 0) aph ^= 1;
+                    }
+                    w += STAGE / 16;
+                    if (++s == a.stages) { s = 0; ph ^= 1; w = (uint32_t)desc; }
+                }
+            }
+        }
+        leave();
+        if (warp == MMA_WARP) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS) : "memory");
+            else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS) : "memory");
+        }
+        return;
+    }
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    // -------------------------------------------------------------------- drain and finish
+    const int quarter = warp & 3, part = warp >> 2;                                 // 32 TMEM lanes, a quarter of the columns
+    const uint32_t taddr0 = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part * CW);
+    uint32_t fph = 0;
+    int buf = 0;
+    for (int tile = group; tile < n_tiles; tile += n_groups) {
+        uint64_t acc[CW / 2];
+#pragma unroll
+        for (int i = 0; i < CW / 2; ++i) acc[i] = 0;
+        bool ok = true;
+#pragma unroll 1
+        for (int kb = 0; kb < nst; kb += KGROUP) {
+            ok = __all_sync(0xffffffffu, wait_bar(acc_full + 8 * buf, fph, abort, a));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            constexpr int LW = CW % 32 == 0 ? 32 : CW % 16 == 0 ? 16 : 8;
+#pragma unroll
+            for (int o = 0; o < CW; o += LW) {
+                uint32_t r[LW];
+                tmem_ld_n<LW>(taddr0 + (uint32_t)(buf * ACC_COLS + o), r, 0);
+                tmem_wait<LW>(r);
+                if (o + LW == CW) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    if (lane == 0) mbar_arrive_cluster(acc_empty_leader + 8 * buf);
+                }
+#pragma unroll
+                for (int i = 0; i < LW / 2; ++i) add2(acc[o / 2 + i], pack2(r[2 * i], r[2 * i + 1]));
+            }
+            buf ^= 1;
+            if (buf == 0) fph ^= 1;
+        }
+        if (!ok) break;
+        const int n = (tile % tiles_n) * (128 * CG) + rank * 128 + quarter * 32 + lane;
+        const int m0 = (tile / tiles_n) * NT + part * CW, left = a.M - m0;
+        const bool real = n < a.N;
+        const float bias = a.bias && real ? __ldg(a.bias + n) : 0.0f;
+        if constexpr (MODE == OUT_SCORE) {
+            // softmax records of (activation row, 128 weight rows): each warp reduces its 32 lanes per column, the
+            // four quarters meet in shared memory. Lanes l and l + 16 end up with column 16 j + l of its warp.
+            const float kLog2e = 1.4426950408889634f;
+            const int nq = n - lane;
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");            // the records of the tile before are read
+#pragma unroll
+            for (int j = 0; j < CW / 16; ++j) {
+                float e[16], my_max = -INFINITY;
+                int my_idx = 0x7fffffff;
+                const int mt = m0 + j * 16 + (lane & 15);
+                const int tgt = mt < a.M ? __ldg(a.targets + mt) : -1;
+                const uint32_t hits = __ballot_sync(0xffffffffu, tgt >= nq && tgt < nq + 32);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const float v = ((i & 1) ? hi_f(acc[j * 8 + i / 2]) : lo_f(acc[j * 8 + i / 2])) * a.inv;
+                    const float t = real ? v : -INFINITY;
+                    const float mx = redux_max(t);
+                    const uint32_t at = __ballot_sync(0xffffffffu, t == mx);
+                    e[i] = real ? ex2((v - mx) * kLog2e) : 0.0f;
+                    if ((lane & 15) == i) { my_max = mx; my_idx = nq + __ffs(at) - 1; }
+                    if (hits >> i & 1) {                                             // some lane's row is the target of column i
+                        const int tg = __shfl_sync(0xffffffffu, tgt, i);
+                        if (n == tg) a.tlogit[m0 + j * 16 + i] = v;
+                    }
+                }
+                // transposing sum: 8 + 4 + 2 + 1 exchanges leave lanes l and l + 16 with halves of the sum of column l
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) {
+#pragma unroll
+                    for (int i = 0; i < o; ++i) {
+                        const bool up = lane & o;
+                        const float keep = up ? e[i + o] : e[i], send = up ? e[i] : e[i + o];
+                        e[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    }
+                }
+                e[0] += __shfl_xor_sync(0xffffffffu, e[0], 16);
+                if (lane < 16)
+                    recs[quarter * NT + part * CW + j * 16 + lane] = make_float4(my_max, e[0], __int_as_float(nq < a.N ? my_idx : 0x7fffffff), 0.0f);
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");
+            const int c = quarter * 32 + lane, m = m0 + c;
+            const int t128 = (tile % tiles_n) * CG + rank, n128 = (a.N + 127) / 128;
+            if (c < CW && m < a.M && t128 < n128) {
+                float mx = -INFINITY, sum = 0.0f;
+                int idx = 0x7fffffff;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) mx = fmaxf(mx, recs[q * NT + part * CW + c].x);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float4 r = recs[q * NT + part * CW + c];
+                    if (r.x > -INFINITY || r.y != 0.0f) sum += r.y * ex2((r.x - mx) * kLog2e);
+                    if (r.x == mx) idx = min(idx, __float_as_int(r.z));
+                }
+                a.stats[(size_t)m * n128 + t128] = make_float4(mx, sum, __int_as_float(idx), 0.0f);
+            }
+        } else if constexpr (MODE == OUT_F32) {
+            // the residual may be the output itself, so the compiler cannot move loads above the stores ahead of them: a batch
+            // of them is asked for first
+            constexpr int RB = CW < 16 ? CW : 16;                            // columns per batch
+            float* y = a.y + (size_t)m0 * a.ldy + n;
+            const float* rp = a.residual + (size_t)m0 * a.ldy + n;
+            float mine[(CW + 31) / 32];                                              // lane l: 1 / scale of columns l, l + 32, ..
+#pragma unroll
+            for (int j = 0; j < (CW + 31) / 32; ++j) mine[j] = a.row_inv && 32 * j + lane < left ? __ldg(a.row_inv + m0 + 32 * j + lane) : a.inv;
+#pragma unroll
+            for (int o = 0; o < CW; o += RB) {
+                if (o >= left) break;
+                float res[RB];
+#pragma unroll
+                for (int i = 0; i < RB; ++i) {
+                    res[i] = a.residual && real && o + i < left ? *rp : 0.0f;
+                    rp += a.ldy;
+                }
+#pragma unroll
+                for (int i = 0; i < RB; ++i) {
+                    const float inv = __shfl_sync(0xffffffffu, mine[(o + i) / 32], (o + i) & 31);
+                    float v = fmaf((i & 1) ? hi_f(acc[(o + i) / 2]) : lo_f(acc[(o + i) / 2]), inv, bias);
+                    if (a.gelu) v = gelu_f(v);
+                    if (a.residual) v = res[i] + v;
+                    if (real && o + i < left) *y = v;
+                    y += a.ldy;
+                }
+            }
+        } else {
+            // lanes (2i, 2i + 1) hold neighbouring columns of the output: after the trade the even lane owns row m of both, the
+            // odd lane row m + 1, and a half warp writes one 64-byte run
+            const int odd = lane & 1;
+            size_t at = (size_t)(m0 + odd) * a.ldy + (n & ~1);
+#pragma unroll
+            for (int i = 0; i < CW / 2; ++i) {
+                if (2 * i < left) {
+                    float v0 = fmaf(lo_f(acc[i]), a.inv, bias), v1 = fmaf(hi_f(acc[i]), a.inv, bias);
+                    uint32_t w[2];
+                    if (MODE == OUT_GELU) split2_f16(gelu_f(v0) * a.out_scale, gelu_f(v1) * a.out_scale, w);
+                    else split2<2>(v0, v1, w);
+                    const uint32_t got = __shfl_xor_sync(0xffffffffu, __byte_perm(w[0], w[1], odd ? 0x5410 : 0x7632), 1);
+                    const uint32_t o0 = __byte_perm(w[0], got, odd ? 0x3254 : 0x5410), o1 = __byte_perm(w[1], got, odd ? 0x3276 : 0x7610);
+                    if (real && 2 * i + odd < left) {
+                        *(uint32_t*)(a.yp[0] + at) = o0;
+                        *(uint32_t*)(a.yp[1] + at) = o1;
+                    }
+                }
+                at += 2 * (size_t)a.ldy;
+            }
+        }
+    }
+    leave();
+}
+
+// Rows of x as f16 planes, each scaled by a power of two that brings its largest element into [2^14, 2^15), and rows of a Q8_0
+// matrix as exact f16 planes; a warp per row. top (null or a zeroed word): bits of the largest square norm among the weight rows from
+// `from` on.
+__global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict__ x, int M, int K, __half* __restrict__ xh, __half* __restrict__ xl,
+                                                         float* __restrict__ row_inv, const QMat w, __half* __restrict__ wh,
+                                                         __half* __restrict__ wl, int from, unsigned* __restrict__ top) {
+    constexpr int HELD = 8;
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row < M) {
+        const float4* src = (const float4*)(x + (size_t)row * K);
+        const int units = K >> 2;
+        float big = 0.0f;
+        // NaN falls out of the maximum: such a row is NaN at any scale
+        auto most = [&](const float4& v) { big = fmaxf(fmaxf(big, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w))); };
+        float4 held[HELD];                                    // a lane's first units stay in registers
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) held[i] = lane + 32 * i < units ? src[lane + 32 * i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) most(held[i]);
+        for (int u = lane + 32 * HELD; u < units; u += 32) most(src[u]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+        // 2^(14 - exponent), its exponent kept where it and its inverse are normal numbers
+        const int e = (int)(__float_as_uint(big) >> 23);
+        const int se = big == 0.0f || e == 255 ? 127 : min(max(127 + 14 + 127 - e, 1), 253);
+        const float s = __uint_as_float((uint32_t)se << 23);
+        auto put = [&](int u, const float4& v) {
+            uint32_t p[2], q[2];
+            split2_f16(v.x * s, v.y * s, p);
+            split2_f16(v.z * s, v.w * s, q);
+            ((uint2*)(xh + (size_t)row * K))[u] = make_uint2(p[0], q[0]);
+            ((uint2*)(xl + (size_t)row * K))[u] = make_uint2(p[1], q[1]);
+        };
+#pragma unroll
+        for (int i = 0; i < HELD; ++i)
+            if (lane + 32 * i < units) put(lane + 32 * i, held[i]);
+        for (int u = lane + 32 * HELD; u < units; u += 32) put(u, src[u]);
+        if (lane == 0) row_inv[row] = __uint_as_float((uint32_t)(254 - se) << 23);
+        return;
+    }
+    const int n = row - M;
+    if (n >= w.N) return;
+    const uint4* q = (const uint4*)(w.qu + (size_t)n * w.K);
+    const __half* d = w.d + (size_t)n * (w.K >> 5);
+    float norm = 0.0f;
+#pragma unroll 2
+    for (int c = lane; c < w.K >> 4; c += 32) {
+        const uint4 u = q[c];
+        const __half2 d2 = __half2half2(d[c >> 1]);
+        uint32_t hi[8], lo[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            // 0x6400 | u is 1024 + u in f16: less 1152 it is the level, exactly
+            const uint32_t t = __byte_perm((&u.x)[i >> 1], 0x64646464u, (i & 1) ? 0x4342 : 0x4140);
+            const __half2 lv = __hsub2(*(const __half2*)&t, __half2half2(__ushort_as_half((unsigned short)0x6480)));
+            const __half2 h = __hmul2(lv, d2), r = __hfma2(lv, d2, __hneg2(h));       // the rounding's remainder, exactly
+            hi[i] = *(const uint32_t*)&h;
+            lo[i] = *(const uint32_t*)&r;
+            if (top) {
+                const float2 f = __half22float2(h);
+                norm = fmaf(f.x, f.x, fmaf(f.y, f.y, norm));
+            }
+        }
+        uint4 *ph = (uint4*)(wh + (size_t)n * w.K) + 2 * c, *pl = (uint4*)(wl + (size_t)n * w.K) + 2 * c;
+        ph[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        ph[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+        pl[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        pl[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+    }
+    if (top && n >= from) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) norm += __shfl_xor_sync(0xffffffffu, norm, o);
+        if (lane == 0) atomicMax(top, __float_as_uint(norm));                          // squares: the order of the bits is theirs
+    }
+}
+
+// x [n] as f16 planes of out.scale times its values.
+__global__ void __launch_bounds__(256) split_f16_kernel(const float4* __restrict__ x, uint2* __restrict__ hi, uint2* __restrict__ lo, float scale, size_t n4) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
+        const float4 v = x[i];
+        uint32_t p[2], q[2];
+        split2_f16(v.x * scale, v.y * scale, p);
+        split2_f16(v.z * scale, v.w * scale, q);
+        hi[i] = make_uint2(p[0], q[0]);
+        lo[i] = make_uint2(p[1], q[1]);
+    }
+}
+
+namespace {
+
+struct TileChoice { int cg, nt; };
+
+// Tile shape by waves of tiles x (stages x the cycles of a stage + the epilogue behind the last). What a stage takes, by clock64 in
+// the issuer: a pair with 64 rows 648, 128 rows 798, 192 rows 1165, 256 rows 1547 (the MMAs alone 384, 768, 1152, 1536), a single CTA with 32
+// rows 951, where reading the weight operand is what counts. 128 rows are entered dearer than that: with several waves the card's
+// power limit counts, and a narrow tile moves more bytes for the same sums (32768 x 768 x 2304: 255 us, 192 rows 239, 256 rows 242).
+TileChoice choose_tile(int M, int N, int K, int mode, int sms) {
+    TileChoice best = {2, 64};
+    double best_cost = 1e30;
+    const int nst = (K + BK - 1) / BK;
+    auto consider = [&](int cg, int nt, double step) {
+        const long tiles = (long)((N + 128 * cg - 1) / (128 * cg)) * ((M + nt - 1) / nt);
+        const long slots = std::max(1, sms / cg);
+        const double cost = (double)((tiles + slots - 1) / slots) * nst * step + 15.0 * nt;
+        if (cost < best_cost) { best_cost = cost; best = {cg, nt}; }
+    };
+    if (mode != OUT_SCORE) consider(1, 32, 950.0);
+    consider(2, 64, 650.0);
+    consider(2, 128, 900.0);
+    consider(2, 192, 1165.0);
+    consider(2, 256, 1547.0);
+    return best;
+}
+
+template <int CG, int CW, int MODE>
+int launch_one(const CUtensorMap (&map)[4], F16Args a, int tiles, int sms, cudaStream_t st) {
+    constexpr int NT = 4 * CW, STAGE = 2 * W_BYTES + 2 * (NT / CG) * BK * 2;
+    constexpr int FIXED = 1024 /* alignment slack */ + BAR_BYTES + (MODE == OUT_SCORE ? 4 * NT * 16 : 0);
+    constexpr int STAGES = (SMEM_LIMIT - FIXED) / STAGE < MAX_STAGES ? (SMEM_LIMIT - FIXED) / STAGE : MAX_STAGES;
+    constexpr int SMEM = STAGES * STAGE + FIXED;
+    static bool ready[64] = {};
+    int dev = 0;
+    FC_CUDA(cudaGetDevice(&dev));
+    if (!ready[dev & 63]) {
+        FC_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<CG, CW, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        ready[dev & 63] = true;
+    }
+    a.stages = STAGES;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(std::min(tiles, sms / CG) * CG));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CG;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    FC_CUDA(cudaLaunchKernelEx(&cfg, gemm_f16_kernel<CG, CW, MODE>, map[0], map[1], map[2], map[3], a));
+    FC_LAUNCHED();
+    return FC_OK;
+}
+
+template <int MODE>
+int launch_f16(const F16Mat& w, const Planes& x, F16Args a, int M, cudaStream_t st) {
+    static int sms[64] = {};
+    int dev = 0;
+    FC_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64) return fail(FC_E_ARG, "device %d out of range", dev);
+    if (!sms[dev]) FC_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
+    if (M <= 0) return FC_OK;
+    if (x.n != 2 || x.scale == 0.0f || !w.hi || w.K % 32) return fail(FC_E_SHAPE, "the f16 GEMM takes two f16 planes of either side and K %% 32 == 0 (K = %d)", w.K);
+    const TileChoice t = choose_tile(M, w.N, w.K, MODE, sms[dev]);
+    a.N = w.N; a.K = w.K; a.M = M;
+    a.inv = 1.0f / x.scale;
+    a.wait_cycles = g_debug.wait_cycles; a.withhold = g_debug.withhold;
+    CUtensorMap map[4];
+    FC_TRY(encode_plane(&map[0], w.hi, w.N, w.K, 128, true));
+    FC_TRY(encode_plane(&map[1], w.lo, w.N, w.K, 128, true));
+    FC_TRY(encode_plane(&map[2], x.p[0], M, w.K, t.nt / t.cg, true));
+    FC_TRY(encode_plane(&map[3], x.p[1], M, w.K, t.nt / t.cg, true));
+    const int tiles = ((w.N + 128 * t.cg - 1) / (128 * t.cg)) * ((M + t.nt - 1) / t.nt);
+    if (t.cg == 2)
+        return t.nt == 256 ? launch_one<2, 64, MODE>(map, a, tiles, sms[dev], st)
+             : t.nt == 192 ? launch_one<2, 48, MODE>(map, a, tiles, sms[dev], st)
+             : t.nt == 128 ? launch_one<2, 32, MODE>(map, a, tiles, sms[dev], st) : launch_one<2, 16, MODE>(map, a, tiles, sms[dev], st);
+    if constexpr (MODE != OUT_SCORE) return launch_one<1, 8, MODE>(map, a, tiles, sms[dev], st);
+    return fail(FC_E_SHAPE, "no scoring tile of %d rows", t.nt);
+}
+
+}  // namespace
+
+// A call of its own pays for turning the weight into planes, 5 bytes a weight, and has no split of K for few rows. Us on this kernel
+// (on the levels): 512 rows x 1024 x 2048 18.6 (20.8), x 4096 24.8 (24.8); 256 rows 17.1 (18.7), 20.8 (20.9); K = 3072, N = 1024: 512 rows
+// 32.3 (26.8), 1024 rows 33.0 (37.2), 1536 rows 43.6 (49.3); N = 4096: 512 rows 53.7 (47.4), 1024 rows 82 (81), 1536 rows 103 (119).
+bool f16_rows(int K, int M) { return M >= 512 && M >= K / 2; }
+
+int launch_f16_planes(const float* x, int M, int K, const Planes& out, float* row_inv, const QMat& w, const F16Mat& planes, int from, unsigned* top,
+                      cudaStream_t st) {
+    if (K % 4 || w.K % 16) return fail(FC_E_SHAPE, "f16 planes: row lengths %d, %d", K, w.K);
+    f16_planes_kernel<<<(M + w.N + 7) / 8, 256, 0, st>>>(x, M, K, (__half*)out.p[0], (__half*)out.p[1], row_inv, w, (__half*)planes.hi, (__half*)planes.lo,
+                                                         from, top);
+    FC_LAUNCHED();
+    return FC_OK;
+}
+
+int launch_split_f16(const float* x, const Planes& out, size_t n, cudaStream_t st) {
+    if (n % 4 || out.n != 2 || out.scale == 0.0f) return fail(FC_E_SHAPE, "split_f16: %zu elements into %d planes", n, out.n);
+    const size_t n4 = n / 4;
+    split_f16_kernel<<<(int)std::max<size_t>(1, std::min<size_t>((n4 + 255) / 256, 148 * 8)), 256, 0, st>>>(
+        (const float4*)x, (uint2*)out.p[0], (uint2*)out.p[1], out.scale, n4);
+    FC_LAUNCHED();
+    return FC_OK;
+}
+
+int launch_gemm_f16(const F16Mat& w, const Planes& x, const float* row_inv, const float* bias, const float* residual, int epi, float* y, const Planes* yp,
+                    int M, int ldy, int* status, cudaStream_t st) {
+    F16Args a = {};
+    a.bias = bias; a.residual = residual; a.gelu = epi == EPI_GELU; a.row_inv = row_inv; a.y = y; a.ldy = ldy; a.status = status;
+    if (epi != EPI_NONE && epi != EPI_GELU) return fail(FC_E_ARG, "epilogue %d is not one of this entry's", epi);
+    if (y) return launch_f16<OUT_F32>(w, x, a, M, st);
+    if (!yp || yp->n != 2 || (w.N & 31) || (ldy & 7) || residual || row_inv || (epi == EPI_GELU) != (yp->scale != 0.0f))
+        return fail(FC_E_SHAPE, "plane output needs N %% 32 == 0, ldy %% 8 == 0, two planes (f16 behind GELU, else bf16) and no residual");
+    for (int p = 0; p < 2; ++p) a.yp[p] = (uint16_t*)yp->p[p];
+    a.out_scale = yp->scale;
+    return epi == EPI_GELU ? launch_f16<OUT_GELU>(w, x, a, M, st) : launch_f16<OUT_BF16>(w, x, a, M, st);
+}
+
+int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st) {
+    if (!targets || !stats || !tlogit) return fail(FC_E_ARG, "the scoring epilogue needs targets, stats and tlogit");
+    F16Args a = {};
+    a.targets = targets; a.stats = (float4*)stats; a.tlogit = tlogit; a.status = status;
+    return launch_f16<OUT_SCORE>(w, x, a, M, st);
+}
+
+}  // namespace fc

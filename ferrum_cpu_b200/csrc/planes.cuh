@@ -25,20 +25,37 @@ __device__ __forceinline__ void split2(float v0, float v1, uint32_t (&w)[P]) {
         }
     }
 }
+// Two f32 values -> f16 hi and lo terms: together 2^-24 relative, while the values stay below 65504 and lo above 2^-24.
+__device__ __forceinline__ void split2_f16(float v0, float v1, uint32_t (&w)[2]) {
+    const __half2 h = __floats2half2_rn(v0, v1);
+    const float2 hf = __half22float2(h);
+    const __half2 l = __floats2half2_rn(v0 - hf.x, v1 - hf.y);
+    w[0] = *(const uint32_t*)&h;
+    w[1] = *(const uint32_t*)&l;
+}
+constexpr int F16X2 = -2;   // in the place of a number of planes: two f16 planes of out.scale times the value
 template <int P>
 __device__ __forceinline__ void store_planes(const Planes& out, size_t i, float v) {
-    uint32_t w[P];
-    split2<P>(v, 0.0f, w);
+    constexpr int N = P == F16X2 ? 2 : P;
+    uint32_t w[N];
+    if constexpr (P == F16X2) split2_f16(v * out.scale, 0.0f, w);
+    else split2<P>(v, 0.0f, w);
 #pragma unroll
-    for (int p = 0; p < P; ++p) ((uint16_t*)out.p[p])[i] = (uint16_t)w[p];
+    for (int p = 0; p < N; ++p) ((uint16_t*)out.p[p])[i] = (uint16_t)w[p];
 }
 template <int P>
 __device__ __forceinline__ void store_planes4(const Planes& out, size_t i4, float4 v) {   // elements 4 i4 .. 4 i4 + 3
-    uint32_t a[P], b[P];
-    split2<P>(v.x, v.y, a);
-    split2<P>(v.z, v.w, b);
+    constexpr int N = P == F16X2 ? 2 : P;
+    uint32_t a[N], b[N];
+    if constexpr (P == F16X2) {
+        split2_f16(v.x * out.scale, v.y * out.scale, a);
+        split2_f16(v.z * out.scale, v.w * out.scale, b);
+    } else {
+        split2<P>(v.x, v.y, a);
+        split2<P>(v.z, v.w, b);
+    }
 #pragma unroll
-    for (int p = 0; p < P; ++p) ((uint2*)out.p[p])[i4] = make_uint2(a[p], b[p]);
+    for (int p = 0; p < N; ++p) ((uint2*)out.p[p])[i4] = make_uint2(a[p], b[p]);
 }
 
 }  // namespace fc

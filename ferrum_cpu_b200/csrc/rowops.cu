@@ -197,6 +197,7 @@ static int layernorm_planes(const float* x, const float* g, const float* b, cons
 }
 int launch_layernorm_planes(const float* x, const float* g, const float* b, const int* pick, int rows, int d, const Planes& out,
                             cudaStream_t st) {
+    if (out.scale != 0.0f) return layernorm_planes<F16X2>(x, g, b, pick, rows, d, out, st);
     return out.n == 3 ? layernorm_planes<3>(x, g, b, pick, rows, d, out, st) : layernorm_planes<2>(x, g, b, pick, rows, d, out, st);
 }
 
