@@ -193,7 +193,7 @@ __device__ void make_work(Work* w, int N, int K, int c, int G) {
     mega_cta_rows(N, K, c, G, &w->r0, &w->r1);
     w->rpi = rows_per_item(K);
     w->gran = mega_row_gran(K);
-    w->iters = max(1, K >> 8);
+    w->iters = (K + 255) >> 8;
     const int n = w->r1 - w->r0;
     const int last = n > 0 ? n - ((n - 1) / w->rpi) * w->rpi : 0;
     w->ks_full = pick_ksplit(w->rpi, w->iters);
