@@ -73,7 +73,6 @@ __global__ void __launch_bounds__(THREADS, 1) attn_step_kernel(const float* __re
     __shared__ float red[2][WARPS];
     __shared__ float peer_o[MAX_SPLIT][HD], peer_ml[MAX_SPLIT][2];   // rank 0: each part's output, largest score and mass
     const int split = SPLIT ? n_split : 1;
-    pdl_trigger();
     if (SPLIT) cluster_arrive();                              // a CTA's shared memory may be written once all have started
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int h = SPLIT ? blockIdx.x / split : blockIdx.x, rank = SPLIT ? blockIdx.x - h * split : 0, group = n_q / n_kv, kvh = h / group, kv_dim = n_kv * HD;
@@ -98,6 +97,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_step_kernel(const float* __re
     if (pair) sincosf(rope_angle(pos, ftab[t], inv_linear), &s, &c);
 
     pdl_wait();
+    pdl_trigger();       // not ahead of the wait: what the kernel behind asks for would queue up before this one's row
     // asked for ahead of the check of the state, which is as far away
     const float* src = qkv + (role == 0 ? (size_t)h * HD : (size_t)n_q * HD + (size_t)(role == 2) * kv_dim + (size_t)kvh * HD);
     const int ia = pair ? (neox ? t : 2 * t) : t, ib = neox ? t + half : 2 * t + 1;

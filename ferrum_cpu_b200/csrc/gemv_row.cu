@@ -83,7 +83,6 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
     extern __shared__ __align__(16) float4 xs[];             // [staged][K / 4] units of 16 bytes, swizzled
     __shared__ __align__(16) float red[3][MAX_WARPS];
     __shared__ float meet[2][MAX_WARPS][RB];
-    pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, warps = blockDim.x >> 5;
     const int K = a.K, chunks = K >> 4, units = K >> 2, kb = K >> 5;
     const int slice = wid % a.ks, per_slice = (chunks + a.ks - 1) / a.ks;
@@ -156,6 +155,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1) gemv_row_kernel(const RowAr
             if (p < a.staged && a.part[p].xscale && tid < units) sx[p] = ((const float4*)a.part[p].xscale)[tid];
 
     pdl_wait();
+    pdl_trigger();       // not ahead of the wait: what the kernel behind asks for would queue up before this one's row
     float4 v[UN];
 #pragma unroll
     for (int i = 0; i < UN; ++i) {

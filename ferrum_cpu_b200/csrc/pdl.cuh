@@ -2,7 +2,9 @@
 // its preamble) before the kernel ahead of it in the stream has finished. Inside such a kernel
 // pdl_wait() blocks until the kernel ahead has completed and its writes are visible; everything
 // that reads or writes data another kernel of the chain touches comes after it, on every path,
-// so completion stays transitive along the chain. pdl_trigger() lets the kernel behind start.
+// so completion stays transitive along the chain. pdl_trigger() lets the kernel behind start: in a chain of short products behind
+// the wait, not ahead of it. Started earlier, the next kernel asks for its weights just when this one asks for its row, which then
+// comes late (16 blocks of 512, int8 levels, 64 tokens: 19.7 ms, triggered behind the wait 17.5; 4 blocks of 128: 3.87 and 3.65).
 // Both are no-ops in a kernel that was launched the ordinary way.
 #pragma once
 #include "fc_common.cuh"
