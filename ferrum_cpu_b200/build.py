@@ -11,7 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libferrum_cuda.so")
-SOURCES = ["codec.cpp", "gguf_load.cpp", "repack.cu", "scratch.cu", "gemv_row.cu", "rows_alone.cu", "rowops.cu", "attn.cu", "attn_step.cu", "attn_step_split.cu", "gemm_tc.cu", "gemm_f16.cu", "attn_tc.cu", "decode_mega.cu", "decode_batch.cu", "sample.cu", "llama_ops.cu", "llama.cu", "rowq.cu", "ggml_linear.cu", "api.cu"]
+SOURCES = ["codec.cpp", "gguf_load.cpp", "repack.cu", "scratch.cu", "gemv_row.cu", "rows_alone.cu", "rowops.cu", "attn.cu", "attn_step.cu", "block_step.cu", "head_row.cu", "attn_step_split.cu", "gemm_tc.cu", "gemm_f16.cu", "attn_tc.cu", "decode_mega.cu", "decode_batch.cu", "sample.cu", "llama_ops.cu", "llama.cu", "rowq.cu", "ggml_linear.cu", "api.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",

@@ -2,6 +2,7 @@
 // the KV-cached decode driver. Host logic above the kernels mirrors, in C++, the Rust items
 // cited in include/ferrum_cuda.h.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -245,6 +246,8 @@ struct fc_stream {
     int host_pos = 0;
     cudaGraphExec_t graph[2][2][3] = {};   // [heads with a CTA each, shared ones][one step, kChainSteps steps][mode]
     int graph_nodes[2][2][3] = {};
+    long long graph_wait = 0;              // the wait budget and the test hook the graphs were captured with
+    int graph_withhold = 0;
     int attn_split = 1, split_from = 0;    // CTAs that share a head from position split_from on
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_decode_ms = 0.0f;
@@ -252,6 +255,7 @@ struct fc_stream {
     // persistent decode kernel: exchange buffers, grid barrier word
     float* qkv = nullptr;                  // the step's q | k | v row
     float2* stats = nullptr;               // softmax statistics of its logits
+    float *parts_a = nullptr, *parts_m = nullptr;   // what the halves of a block leave to add (block_step.cu); null: shapes it does not cover
     float *partg = nullptr, *x1g = nullptr, *statg = nullptr;
     unsigned* bar = nullptr;
     int attn_splits = 1;
@@ -273,10 +277,12 @@ namespace fc {
 enum StepMode { STEP_NOHEAD = 0, STEP_SELECT = 1, STEP_PROBS = 2 };
 
 // Final LayerNorm, head and the selection of a step, on one row.
-static int launch_head(fc_stream* s, const float* x, int mode) {
+// tail: the row as the halves of the last block left it (null: x is whole).
+static int launch_head(fc_stream* s, const float* x, int mode, const BlockRow* tail = nullptr) {
     fc_model* m = s->m;
     int n_stats = 0;
-    FC_TRY(launch_gemv_row(m->head, x, RowNorm{m->lnfg, m->lnfb, 1e-5f}, nullptr, nullptr, EPI_NONE, s->logits, s->state, m->st, s->stats, &n_stats));
+    if (tail) FC_TRY(launch_head_row(m->head, *tail, s->logits, s->stats, &n_stats, s->state, m->st));
+    else FC_TRY(launch_gemv_row(m->head, x, RowNorm{m->lnfg, m->lnfb, 1e-5f}, nullptr, nullptr, EPI_NONE, s->logits, s->state, m->st, s->stats, &n_stats));
     return launch_step_finish(s->logits, m->cfg.vocab, s->stats, n_stats, mode == STEP_PROBS ? s->probs : nullptr, s->queue, s->queue_cap, s->state,
                               m->st);
 }
@@ -292,6 +298,22 @@ static int launch_step(fc_stream* s, int mode, int split) {
     const int d = c.d_model, hd = d / c.n_head;
     const size_t layer_stride = (size_t)c.ctx * d;
     FC_TRY(launch_embed_step(m->tok, m->pos, c.ctx, s->queue, s->state, s->x, st));
+    if (s->parts_a) {
+        // two launches a layer (block_step.cu); what a half leaves to add is added by the next one
+        BlockRow r = {s->x, nullptr, nullptr, nullptr, nullptr, nullptr, 0, d};
+        for (int l = 0; l < c.n_layer; ++l) {
+            const LayerDev& L = m->layers[l];
+            r.g = L.ln1g; r.b = L.ln1b;
+            r.x_out = l ? s->att : nullptr;                  // the first row is whole as it is
+            FC_TRY(launch_attn_half(r, c.n_head, L.qkv, L.qkv_b, L.out, s->kc + l * layer_stride, s->vc + l * layer_stride, c.ctx, s->parts_a, s->state,
+                                    s->status, st));
+            r = {l ? s->att : s->x, s->parts_a, L.out_b, s->q, L.ln2g, L.ln2b, c.n_head, d};
+            FC_TRY(launch_mlp_half(r, L.up, L.up_b, L.down, s->parts_m, s->state, s->status, st));
+            r = {s->q, s->parts_m, L.down_b, nullptr, m->lnfg, m->lnfb, block_step_slices(c.d_ff), d};
+        }
+        if (mode == STEP_NOHEAD) return launch_step_advance_pdl(s->state, st);
+        return launch_head(s, nullptr, mode, &r);
+    }
     for (int l = 0; l < c.n_layer; ++l) {
         const LayerDev& L = m->layers[l];
         FC_TRY(launch_gemv_row(L.qkv, s->x, RowNorm{L.ln1g, L.ln1b, 1e-5f}, L.qkv_b, nullptr, EPI_NONE, s->qkv, s->state, st));
@@ -305,12 +327,27 @@ static int launch_step(fc_stream* s, int mode, int split) {
     return launch_head(s, s->x, mode);
 }
 
+static void drop_graphs(fc_stream* s) {
+    for (auto& form : s->graph)
+        for (auto& set : form)
+            for (cudaGraphExec_t& g : set) {
+                if (g) cudaGraphExecDestroy(g);
+                g = nullptr;
+            }
+}
+
 // The launch-bound step is captured once per mode into a CUDA graph and replayed; every
 // per-step quantity (token, position) is read from device state, so no node is updated.
 // pos: the position of the (first) step, which decides how many CTAs a head has.
 constexpr int kChainSteps = 8;
 static int run_step(fc_stream* s, int mode, int pos, bool several = false) {
     const bool shared = pos + (several ? kChainSteps : 1) > s->split_from;
+    if (s->graph_wait != g_debug.wait_cycles || s->graph_withhold != g_debug.withhold) {
+        FC_CUDA(cudaStreamSynchronize(s->m->st));
+        drop_graphs(s);
+        s->graph_wait = g_debug.wait_cycles;
+        s->graph_withhold = g_debug.withhold;
+    }
     cudaGraphExec_t& graph = s->graph[shared][several][mode];
     int& nodes = s->graph_nodes[shared][several][mode];
     if (!graph) {
@@ -398,7 +435,7 @@ static int read_state(fc_stream* s, StepState* out) {
     FC_CUDA(cudaStreamSynchronize(s->m->st));
     if (status != 0) {
         cudaMemsetAsync(s->status, 0, sizeof(int), s->m->st);
-        return fail(FC_E_TIMEOUT, "a bounded wait inside the prime or the persistent decode kernel ran out (status %d)", status);
+        return fail(FC_E_TIMEOUT, "a bounded wait inside the prime or a decode step ran out (status %d)", status);
     }
     return FC_OK;
 }
@@ -1159,6 +1196,11 @@ int fc_stream_create(fc_model* m, fc_stream** out) {
     if (rc == FC_OK && cudaMemsetAsync(s->status, 0, sizeof(int), m->st) != cudaSuccess) rc = fail(FC_E_CUDA, "status word initialisation failed");
     const int hd = c.d_model / c.n_head;
     if (rc == FC_OK) rc = attn_step_split(c.n_head, hd, c.ctx, &s->attn_split, &s->split_from);
+    if (rc == FC_OK && block_step_covers(c.d_model, c.n_head, c.d_ff, c.ctx)) {
+        rc = a.alloc_n(&s->parts_a, (size_t)c.n_head * c.d_model);
+        if (rc == FC_OK) rc = a.alloc_n(&s->parts_m, (size_t)block_step_slices(c.d_ff) * c.d_model);
+        s->split_from = INT_MAX;
+    }
     if (rc == FC_OK && m->mega_grid > 0) {
         s->attn_splits = std::max(1, std::min(8, m->mega_grid / c.n_head));
         rc = a.alloc_n(&s->partg, (size_t)c.n_head * s->attn_splits * (hd + 2));
@@ -1181,9 +1223,7 @@ void fc_stream_free(fc_stream* s) {
     cudaStreamSynchronize(s->m->st);
     if (s->cs) { cudaStreamSynchronize(s->cs); cudaStreamDestroy(s->cs); }
     if (s->cs_done) cudaEventDestroy(s->cs_done);
-    for (auto& form : s->graph)
-        for (auto& set : form)
-            for (cudaGraphExec_t g : set) if (g) cudaGraphExecDestroy(g);
+    drop_graphs(s);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     s->arena.release();

@@ -183,6 +183,24 @@ int attn_step_split(int n_q, int hd, int ctx, int* split, int* from);
 int launch_attn_step(const float* qkv, int n_q, int n_kv, int hd, int rope_dim, int neox, const float2* ftab, float inv_linear,
                      float* kc, float* vc, int ctx, int split, const StepState* state, float* out, cudaStream_t st);
 
+// block_step.cu — a GPT-2 block of a decode step in two launches, each on the row x + (part[0] + .. + part[n_part - 1] + bias), left in
+// x_out (null: nowhere), behind LayerNorm (g, b). The attention half leaves parts [n_head][d], the MLP half [block_step_slices][d]. The
+// state and the cached rows are read ahead of the wait, as in launch_attn_step. `status` is raised when a bounded wait runs out.
+struct BlockRow {
+    const float *x, *part, *bias;
+    float* x_out;
+    const float *g, *b;
+    int n_part, d;
+};
+bool block_step_covers(int d, int n_head, int F, int ctx);
+int block_step_slices(int F);
+int launch_attn_half(const BlockRow& r, int n_head, const QMat& qkv, const float* qkv_b, const QMat& out, float* kc, float* vc, int ctx, float* parts,
+                     StepState* state, int* status, cudaStream_t st);
+int launch_mlp_half(const BlockRow& r, const QMat& up, const float* up_b, const QMat& down, float* parts, StepState* state, int* status, cudaStream_t st);
+
+// head_row.cu — the product behind those: logits and, per CTA, the largest and the mass around it (kRowStats entries at most).
+int launch_head_row(const QMat& w, const BlockRow& r, float* logits, float2* stats, int* n_stats, const StepState* state, cudaStream_t st);
+
 // Windows of rows that share a forward pass: window b holds rows starts[b] .. starts[b + 1] (device array of B + 1), or, with
 // starts == nullptr, T rows each. T: rows of the longest.
 struct Windows {

@@ -1,0 +1,61 @@
+"""The decode step of two launches a block (block_step.cu, head_row.cu) against the oracle and against the other forms of a step."""
+import numpy as np
+import pytest
+
+import ferrum_cpu_b200 as fcb
+from ferrum_cpu_b200 import _lib, synth
+from tests import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+# rows that do not fill a warp's units or the threads' shares, two and three hidden units a warp, one to sixteen slices of them,
+# clusters with fewer positions than CTAs, and contexts their shares do not divide
+@pytest.mark.parametrize("d,heads,ff,ctx,prompt,new,vocab", [(512, 8, 2048, 40, 1, 30, 515), (640, 10, 2560, 61, 3, 50, 515), (768, 12, 3072, 24, 9, 14, 4099),
+                                                             (896, 14, 4608, 200, 190, 9, 515), (1024, 16, 256, 70, 8, 40, 515)])
+def test_tokens_and_probabilities(d, heads, ff, ctx, prompt, new, vocab):
+    sm = synth.SynthModel(2, d, heads, ff, ctx, vocab, seed=d + ff, perturb=True)
+    om, gm = O.OracleModel(sm), fcb.CudaSlm(sm.config, sm.weights)
+    ids = synth.token_ids(4, prompt, vocab)
+    want, margin = om.generate_greedy(ids, new)
+    fcb.take_launch_count()
+    got, _ = gm.generate_tokens(ids, new)
+    assert fcb.take_launch_count() < 8 * new + 100          # seven launches a step: two a block, embedding, head, pick
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert a == b or margin[i] < 1e-4, i
+        if a != b:
+            break
+    gm.set_decode_mode(1)                                   # feeds take the same step
+    om.prime(ids), gm.prime(ids)
+    for t in want[: min(len(want), ctx - prompt)]:
+        assert np.abs(gm.feed(t) - om.feed(t)).max() < 2e-5
+    gm.close()
+    om.close()
+
+
+def test_scores_of_minus_infinity_and_huge_rows():
+    """A row without a finite logit ends as it does in the step of five launches: no id beyond the vocabulary, no hang."""
+    sm = synth.SynthModel(1, 512, 8, 2048, 32, 515, seed=3)
+    sm.position_embd[:] = np.float32(3e38)
+    gm = fcb.CudaSlm(sm.config, sm.weights)
+    got, _ = gm.generate_tokens(synth.token_ids(1, 2, 515), 5)
+    assert ((got >= 0) & (got < 515)).all()
+    gm.close()
+
+
+def test_a_wait_that_runs_out_feeds_nothing():
+    sm = synth.SynthModel(2, 512, 8, 2048, 64, 515, seed=5, perturb=True)
+    om, gm = O.OracleModel(sm), fcb.CudaSlm(sm.config, sm.weights)
+    gm.set_decode_mode(1)
+    ids = synth.token_ids(2, 3, 515)
+    om.prime(ids), gm.prime(ids)
+    _lib.check(_lib.lib().fc_debug_set_wait_budget(200000, 1))
+    try:
+        with pytest.raises(fcb.FerrumCudaError) as e:
+            gm.feed(7)
+    finally:
+        _lib.check(_lib.lib().fc_debug_set_wait_budget(4000000000, 0))
+    assert e.value.code == _lib.FC_E_TIMEOUT and gm.cached_len() == 3
+    assert np.abs(gm.feed(7) - om.feed(7)).max() < 2e-5
+    gm.close()
+    om.close()
