@@ -204,7 +204,7 @@ struct fc_model {
     float* pos = nullptr;
     float *lnfg = nullptr, *lnfb = nullptr;
     std::vector<LayerDev> layers;
-    bool f16 = false;                          // the two-plane mode runs on f16 planes: LayerDev::f16, and
+    bool f16 = false;                          // window forwards run on f16 planes: LayerDev::f16, and
     F16Mat head_f16;
     float lnf_scale = 0.0f;
     // prefill workspace for ws_rows rows
@@ -454,7 +454,9 @@ static int model_planes(const fc_model* m) {
     const fc_config& c = m->cfg;
     return c.math_mode == FC_MATH_BF16X3 && c.d_model % 64 == 0 && c.d_ff % 64 == 0 ? 2 : 3;
 }
-// The matrices of a two-plane model as f16 planes, and the scales of the activation planes. A scale is the largest power of two
+// Width from which on the f32 mode runs on f16 planes: its sums there are no further from 64 bits than those of the level GEMM.
+constexpr int kExactF16 = 512;
+// The matrices of a model as f16 planes (a two-plane model, or one whose products are long enough), and the scales of the activation planes. A scale is the largest power of two
 // that keeps scale x bound within f16, where the bound holds for every input: a LayerNorm's row has norm at most sqrt(d) max|g| +
 // |b|, an element of a product at most the norm of its weight row times that (+ bias), a mixture of value rows and GELU at
 // most what goes into them. The 1 % is for rounding. Without memory for the planes (4 bytes a weight), with a matrix that f16
@@ -563,10 +565,14 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
     const int d = c.d_model, F = c.d_ff;
     cudaStream_t st = m->st;
     const bool tc_attn = tensor_attention(m);
-    const bool f16 = planes == 2 && m->f16;
-    m->pn.n = m->pqkv.n = m->patt.n = m->phid.n = planes;
+    // f16 planes, unless a few rows are better off where K is split over CTAs
+    const bool f16 = m->f16 && (planes == 2 || d >= kExactF16) && (!split_k || R >= 256);
+    m->pqkv.n = planes;
+    m->pn.n = m->patt.n = m->phid.n = f16 ? 2 : planes;
+    m->pn.lift = m->patt.lift = f16_lift(d, planes == 3);
+    m->phid.lift = f16_lift(F, planes == 3);
     auto product = [&](const QMat& q, const F16Mat& h, const Planes& x, const float* bias, const float* residual, int epi, float* y, const Planes* yp) {
-        return f16 ? launch_gemm_f16(h, x, nullptr, bias, residual, epi, y, yp, R, q.N, status, st)
+        return f16 ? launch_gemm_f16(h, x, nullptr, bias, residual, epi, y, yp, R, q.N, status, st, planes == 3)
                    : launch_gemm_q8_tc(q, x, bias, residual, epi, y, yp, R, q.N, status, st, split_k);
     };
     FC_CUDA(cudaMemsetAsync(m->err_d, 0, sizeof(int), st));
@@ -612,6 +618,8 @@ static int score_device(fc_model* m, const ScoreSlot& s, const Windows& win, int
     const int d = c.d_model, n = s.picked;
     const int *ids = (const int*)s.in_d, *pos = ids + R, *pick = pos + R + win.B + 1, *targets = pick + n;
     FC_TRY(forward_blocks_with(m, win, R, ids, pos, model_planes(m), s.status_d(), false, false, [](int) { return FC_OK; }));
+    const bool f16 = m->f16;
+    m->pn.n = model_planes(m);
     m->pn.scale = 0.0f;
     if (m->stats_on) {
         FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, nullptr, R, d, m->pn, m->st));
@@ -620,10 +628,13 @@ static int score_device(fc_model* m, const ScoreSlot& s, const Windows& win, int
     if (n == 0) return FC_OK;               // the forward was for its statistics
     // the head's epilogue keeps (max, sum of exponentials, first argmax) per row and 128-column tile and the
     // target's logit: [rows][V] logits never reach memory (scoring.rs:175-181 needs one number per row)
-    const bool f16 = m->pn.n == 2 && m->f16;
-    if (f16) m->pn.scale = m->lnf_scale;
+    if (f16) {
+        m->pn.n = 2;
+        m->pn.scale = m->lnf_scale;
+        m->pn.lift = f16_lift(d, model_planes(m) == 3);
+    }
     FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, n == R ? nullptr : pick, n, d, m->pn, m->st));
-    if (f16) FC_TRY(launch_gemm_f16_score(m->head_f16, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
+    if (f16) FC_TRY(launch_gemm_f16_score(m->head_f16, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st, model_planes(m) == 3));
     else FC_TRY(launch_gemm_q8_tc_score(m->head, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
     return launch_score_combine(m->head_stats, m->head_tlogit, targets, n, (c.vocab + 127) / 128, c.vocab, s.lp_d(), s.gr_d(), m->st);
 }
@@ -709,10 +720,10 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
             __half* p = (__half*)scratch.p;
             const F16Mat wp = {p, p + nw, w->w.N, w->w.K};
             p += 2 * nw;
-            x.p[0] = p; x.p[1] = p + n; x.n = 2; x.scale = 1.0f;
+            x.p[0] = p; x.p[1] = p + n; x.n = 2; x.scale = 1.0f; x.lift = f16_lift(w->w.K, false);
             float* row_inv = (float*)(p + 2 * n);
             FC_TRY(launch_f16_planes(x_dev, M, w->w.K, x, row_inv, w->w, wp, 0, nullptr, st));
-            return launch_gemm_f16(wp, x, row_inv, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, w->status.dev, st);
+            return launch_gemm_f16(wp, x, row_inv, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, w->status.dev, st, false);
         }
     }
     FC_TRY(take_planes(scratch, x, planes, n, w->device, st));
@@ -779,7 +790,7 @@ static int model_build(fc_model* m, const fc_weights* w) {
         FC_TRY(upload_f32(a, s.ln2_g, d, &L.ln2g, st));
         FC_TRY(upload_f32(a, s.ln2_b, d, &L.ln2b, st));
     }
-    if (model_planes(m) == 2) FC_TRY(build_f16(m, w));
+    if (model_planes(m) == 2 || (d >= kExactF16 && d % 64 == 0 && F % 64 == 0)) FC_TRY(build_f16(m, w));
     if (mega_supported(c)) {
         int full = 0;
         FC_TRY(mega_max_grid(&full));

@@ -140,7 +140,7 @@ struct AttnArgs {
     int group;                   // query heads per key / value head (1: multi-head attention)
     int ldo;                     // row stride of the output planes (= query heads x 64)
     uint16_t* out[3];            // [R][ldo] bf16 planes, or
-    float out_scale;             // not 0: two f16 planes of out_scale times the output
+    float out_scale, out_lift;   // not 0: two f16 planes of out_scale (1 + out_lift) times the output
     int* status;
 };
 
@@ -323,12 +323,17 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float v0 = o[8 * c + 2 * e] * inv, v1 = o[8 * c + 2 * e + 1] * inv;
-                    if constexpr (P == 2)
-                        if (a.out_scale != 0.0f) { split2_f16(v0 * a.out_scale, v1 * a.out_scale, w[e]); continue; }
-                    split2<P>(v0, v1, w[e]);
+                    if (a.out_scale != 0.0f) {
+                        uint32_t t[2];
+                        split2_f16(v0 * a.out_scale, v1 * a.out_scale, a.out_lift, t);
+                        w[e][0] = t[0]; w[e][1] = t[1];
+                    } else {
+                        split2<P>(v0, v1, w[e]);
+                    }
                 }
 #pragma unroll
-                for (int t = 0; t < P; ++t) *(uint4*)(a.out[t] + off + 8 * c) = make_uint4(w[0][t], w[1][t], w[2][t], w[3][t]);
+                for (int t = 0; t < P; ++t)
+                    if (a.out[t]) *(uint4*)(a.out[t] + off + 8 * c) = make_uint4(w[0][t], w[1][t], w[2][t], w[3][t]);
             }
         }
     }
@@ -385,10 +390,10 @@ static int launch_attn_tc(const Planes& qkv, const Windows& w, int R, int H, int
     for (int p = 0; p < P; ++p) {
         FC_TRY(encode(&maps.q[p], qkv.p[p], R, ld, QT));
         FC_TRY(encode(&maps.kv[p], qkv.p[p], R, ld, KT));
-        a.out[p] = (uint16_t*)out.p[p];
+        a.out[p] = p < out.n ? (uint16_t*)out.p[p] : nullptr;
     }
     a.win = w; a.k_col = H * HD; a.v_col = (H + KV) * HD; a.group = H / KV; a.ldo = H * HD;
-    a.out_scale = out.scale;
+    a.out_scale = out.scale; a.out_lift = out.lift;
     a.status = status;
     dim3 grid((w.T + QT - 1) / QT, H, w.B);
     attn_prefill_tc_kernel<P><<<grid, THREADS, SMEM_BYTES<P>, st>>>(maps, a);

@@ -1,22 +1,28 @@
 // Q8_0 GEMM with the weight as two f16 planes:
 //     Y[M][N] = X[M][K] · dequant(W[N][K])ᵀ + bias (+GELU) (+residual), or the softmax records of the LM head
 //
-// The product of the two-plane math mode (FC_MATH_BF16X3). A Q8_0 weight d·q has at most 19 significant bits (11 of the f16
-// scale, 8 of the level) and is a whole multiple of 2^-24, so hi = f16(d·q) and lo = d·q - hi hold it EXACTLY, as long as
-// d·128 does not overflow f16 (QMat::f16_exact, checked at upload). An activation, scaled by a power of two that keeps it in
-// range, is hi + lo to 2^-24 relative: as close as f32 itself. Three MMAs per step, hi·hi + hi·lo + lo·hi, drop 2^-24 of a
-// product, and no scale is left to apply: k-blocks add up in TMEM, and the tensor pipe is what bounds the kernel.
+// The product of the two-plane math mode (FC_MATH_BF16X3), and of window forwards in the f32 mode. A Q8_0 weight d·q has at most 19
+// significant bits (11 of the f16 scale, 8 of the level) and is a whole multiple of 2^-24, so hi = f16(d·q) and lo = d·q - hi hold it
+// EXACTLY, as long as d·128 does not overflow f16 (QMat::f16_exact, checked at upload). An activation, scaled by a power of two
+// that keeps it in range, is hi + lo to 2^-23 relative. Three MMAs per step, hi·hi + hi·lo + lo·hi, drop 2^-24 of a product, and no
+// scale is left to apply: k-blocks add up in TMEM, and the tensor pipe is what bounds the kernel.
 //
 // gemm_tc.cu multiplies the levels instead (two MMAs per step with bf16 planes of x) and has to fold every 32-wide k-block
 // into registers by the block's scale: its drain is what bounds it, at half the rate of the pipe, and its two bf16 planes of x
-// leave 2^-17. It stays for the f32 mode, whose sums may not be truncated as often as here (below), for matrices that f16
-// does not hold, and for few rows of a caller's own, where 4 bytes a weight would be what counts.
+// leave 2^-17. It stays for the f32 linear, for narrow models in the f32 mode (below a width of 512 its sums are the more exact
+// ones), for matrices that f16 does not hold, and for few rows of a prime or of a caller's own, which it splits over K.
 //
 // The tensor core truncates its f32 sums: towards zero, once per MMA. Over all of K that is 1.05e-9 of the result per k (measured
 // on one MMA per 16 k: 1.1e-6 at K = 1024, 4.2e-6 at 4096; three times as much here), where two bf16 planes of x are 2.5e-6 off
-// whatever K is. So sums stay in TMEM for KGROUP stages and then go into f32 registers, rounded to nearest. Error against 64 bits at
-// K = 1024 (relative, 2-norm): 3.8e-7 with 2 stages a group, 7.6e-7 with 4, 1.7e-6 with 8; 4096 x 1024 x 4096 takes the same time with
-// 4 as with 8.
+// whatever K is. So sums stay in TMEM for KGROUP stages and then go into f32 registers, rounded to nearest. What they lose on the way is
+// on average the same share of a sum (2.8e-7 with two stages a group, 6.7e-7 with four), and the activations are lifted by it
+// (f16_lift). Error against 64 bits (relative, 2-norm) at K = 1024: two-plane mode 5.0e-7 (levels and bf16 planes: 2.5e-6; groups of 8:
+// 1.7e-6, and no faster).
+//
+// The f32 mode (FC_MATH_FP32) of models of width 512 and more is the same kernel with one stage a group, drained once per 12
+// MMAs. Its error at K = 768 / 1024 / 3072 / 4096: 1.08e-7 / 1.15e-7 / 1.54e-7 / 1.70e-7 (levels with three bf16 planes: 1.03e-7 / 1.15e-7 /
+// 1.84e-7 / 2.10e-7); of the log-probabilities of 12 x 768 and 24 x 1024 on windows of 32, 256 and 1024 ids 3.3e-8 / 3.3e-8 / 3.2e-8 and 3.7e-8 /
+// 3.6e-8 / 3.5e-8 (3.4e-8 / 3.3e-8 / 3.3e-8 and 3.7e-8 / 3.7e-8 / 3.7e-8). Groups of half a stage are no more exact (1.3e-7 at 768) and slower.
 //
 // One CTA per SM, 640 threads (registers 104 a thread of the drain, 64 of the others):
 //   warps 0-15  drain: a group's sums from TMEM into registers (lane = weight row, column = activation row); after the last
@@ -46,7 +52,7 @@ using namespace tc;
 namespace {
 
 constexpr int BK = 64;                                  // k per stage: one 128-byte swizzle row of f16
-constexpr int KGROUP = 4;                               // stages whose sums stay in TMEM
+constexpr int KGROUP = 4;                               // stages whose sums stay in TMEM in the two-plane mode; in the f32 mode one
 constexpr int W_BYTES = 128 * BK * 2;                   // one plane of the CTA's weight tile of a stage
 constexpr int DRAIN_WARPS = 16, TMA_WARP = 16, MMA_WARP = 17, THREADS = 640;
 constexpr int MAX_STAGES = 6;
@@ -57,12 +63,13 @@ enum Mode : int { OUT_F32 = 0, OUT_BF16 = 1 /* bf16 planes */, OUT_GELU = 2 /* f
 
 struct F16Args {
     int N, K, M, stages;
+    int exact;                // the f32 mode
     const float* bias; const float* residual; int gelu;
     float inv;                // what takes the scale of x out of a sum (a power of two)
     const float* row_inv;     // the same per activation row, or null
     float* y; int ldy;        // OUT_F32
-    uint16_t* yp[2];          // OUT_BF16, OUT_GELU: planes, ldy elements apart
-    float out_scale;          // OUT_GELU: scale of the planes
+    uint16_t* yp[3];          // OUT_BF16 (two planes, or three), OUT_GELU (two): planes, ldy elements apart
+    float out_scale, out_lift;   // OUT_GELU: scale and lift of the planes
     const int* targets; float4* stats; float* tlogit;      // OUT_SCORE
     int* status;
     long long wait_cycles;
@@ -173,11 +180,13 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
             const uint64_t desc = smem_desc(sb);
             const uint32_t dhi = (uint32_t)(desc >> 32);
             uint32_t w = (uint32_t)desc, ph = 0, aph = 1;
+            const int per_group = a.exact ? 1 : KGROUP;
             int s = 0, buf = 0;
             bool ok = true;
             for (int tile = group; tile < n_tiles && ok; tile += n_groups) {
-                for (int kb = 0; kb < nst && ok; ++kb) {
-                    const bool first = kb % KGROUP == 0, last = kb % KGROUP == KGROUP - 1 || kb == nst - 1;
+                for (int kb = 0, in_group = 0; kb < nst && ok; ++kb) {
+                    const bool first = in_group == 0, last = ++in_group == per_group || kb == nst - 1;
+                    if (last) in_group = 0;
                     ok = (!first || wait_bar(acc_empty + 8 * buf, aph, abort, a)) && wait_bar(full + 8 * s, ph, abort, a);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -214,6 +223,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
     // -------------------------------------------------------------------- drain and finish
     const int quarter = warp & 3, part = warp >> 2;                                 // 32 TMEM lanes, a quarter of the columns
     const uint32_t taddr0 = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part * CW);
+    const int groups = a.exact ? nst : (nst + KGROUP - 1) / KGROUP;
     uint32_t fph = 0;
     int buf = 0;
     for (int tile = group; tile < n_tiles; tile += n_groups) {
@@ -222,7 +232,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
         for (int i = 0; i < CW / 2; ++i) acc[i] = 0;
         bool ok = true;
 #pragma unroll 1
-        for (int kb = 0; kb < nst; kb += KGROUP) {
+        for (int g = 0; g < groups; ++g) {
             ok = __all_sync(0xffffffffu, wait_bar(acc_full + 8 * buf, fph, abort, a));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -340,14 +350,27 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
             for (int i = 0; i < CW / 2; ++i) {
                 if (2 * i < left) {
                     float v0 = fmaf(lo_f(acc[i]), a.inv, bias), v1 = fmaf(hi_f(acc[i]), a.inv, bias);
-                    uint32_t w[2];
-                    if (MODE == OUT_GELU) split2_f16(gelu_f(v0) * a.out_scale, gelu_f(v1) * a.out_scale, w);
-                    else split2<2>(v0, v1, w);
+                    uint32_t w[3];
+                    if (MODE == OUT_GELU) {
+                        uint32_t t[2];
+                        split2_f16(gelu_f(v0) * a.out_scale, gelu_f(v1) * a.out_scale, a.out_lift, t);
+                        w[0] = t[0]; w[1] = t[1];
+                    } else if (a.yp[2]) {
+                        split2<3>(v0, v1, w);
+                    } else {
+                        uint32_t t[2];
+                        split2<2>(v0, v1, t);
+                        w[0] = t[0]; w[1] = t[1]; w[2] = 0;
+                    }
                     const uint32_t got = __shfl_xor_sync(0xffffffffu, __byte_perm(w[0], w[1], odd ? 0x5410 : 0x7632), 1);
                     const uint32_t o0 = __byte_perm(w[0], got, odd ? 0x3254 : 0x5410), o1 = __byte_perm(w[1], got, odd ? 0x3276 : 0x7610);
                     if (real && 2 * i + odd < left) {
                         *(uint32_t*)(a.yp[0] + at) = o0;
                         *(uint32_t*)(a.yp[1] + at) = o1;
+                    }
+                    if (MODE == OUT_BF16 && a.yp[2]) {
+                        const uint32_t g2 = __shfl_xor_sync(0xffffffffu, w[2], 1);
+                        if (real && 2 * i + odd < left) *(uint32_t*)(a.yp[2] + at) = __byte_perm(w[2], g2, odd ? 0x3276 : 0x5410);
                     }
                 }
                 at += 2 * (size_t)a.ldy;
@@ -360,7 +383,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
 // Rows of x as f16 planes, each scaled by a power of two that brings its largest element into [2^14, 2^15), and rows of a Q8_0
 // matrix as exact f16 planes; a warp per row. top (null or a zeroed word): bits of the largest square norm among the weight rows from
 // `from` on.
-__global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict__ x, int M, int K, __half* __restrict__ xh, __half* __restrict__ xl,
+__global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict__ x, int M, int K, float lift, __half* __restrict__ xh, __half* __restrict__ xl,
                                                          float* __restrict__ row_inv, const QMat w, __half* __restrict__ wh,
                                                          __half* __restrict__ wl, int from, unsigned* __restrict__ top) {
     constexpr int HELD = 8;
@@ -386,8 +409,8 @@ __global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict
         const float s = __uint_as_float((uint32_t)se << 23);
         auto put = [&](int u, const float4& v) {
             uint32_t p[2], q[2];
-            split2_f16(v.x * s, v.y * s, p);
-            split2_f16(v.z * s, v.w * s, q);
+            split2_f16(v.x * s, v.y * s, lift, p);
+            split2_f16(v.z * s, v.w * s, lift, q);
             ((uint2*)(xh + (size_t)row * K))[u] = make_uint2(p[0], q[0]);
             ((uint2*)(xl + (size_t)row * K))[u] = make_uint2(p[1], q[1]);
         };
@@ -435,12 +458,12 @@ __global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict
 }
 
 // x [n] as f16 planes of out.scale times its values.
-__global__ void __launch_bounds__(256) split_f16_kernel(const float4* __restrict__ x, uint2* __restrict__ hi, uint2* __restrict__ lo, float scale, size_t n4) {
+__global__ void __launch_bounds__(256) split_f16_kernel(const float4* __restrict__ x, uint2* __restrict__ hi, uint2* __restrict__ lo, float scale, float lift, size_t n4) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
         const float4 v = x[i];
         uint32_t p[2], q[2];
-        split2_f16(v.x * scale, v.y * scale, p);
-        split2_f16(v.z * scale, v.w * scale, q);
+        split2_f16(v.x * scale, v.y * scale, lift, p);
+        split2_f16(v.z * scale, v.w * scale, lift, q);
         hi[i] = make_uint2(p[0], q[0]);
         lo[i] = make_uint2(p[1], q[1]);
     }
@@ -505,7 +528,7 @@ int launch_one(const CUtensorMap (&map)[4], F16Args a, int tiles, int sms, cudaS
 }
 
 template <int MODE>
-int launch_f16(const F16Mat& w, const Planes& x, F16Args a, int M, cudaStream_t st) {
+int launch_f16(const F16Mat& w, const Planes& x, F16Args a, int M, bool exact, cudaStream_t st) {
     static int sms[64] = {};
     int dev = 0;
     FC_CUDA(cudaGetDevice(&dev));
@@ -516,6 +539,7 @@ int launch_f16(const F16Mat& w, const Planes& x, F16Args a, int M, cudaStream_t 
     const TileChoice t = choose_tile(M, w.N, w.K, MODE, sms[dev]);
     a.N = w.N; a.K = w.K; a.M = M;
     a.inv = 1.0f / x.scale;
+    a.exact = exact;
     a.wait_cycles = g_debug.wait_cycles; a.withhold = g_debug.withhold;
     CUtensorMap map[4];
     FC_TRY(encode_plane(&map[0], w.hi, w.N, w.K, 128, true));
@@ -541,7 +565,7 @@ bool f16_rows(int K, int M) { return M >= 512 && M >= K / 2; }
 int launch_f16_planes(const float* x, int M, int K, const Planes& out, float* row_inv, const QMat& w, const F16Mat& planes, int from, unsigned* top,
                       cudaStream_t st) {
     if (K % 4 || w.K % 16) return fail(FC_E_SHAPE, "f16 planes: row lengths %d, %d", K, w.K);
-    f16_planes_kernel<<<(M + w.N + 7) / 8, 256, 0, st>>>(x, M, K, (__half*)out.p[0], (__half*)out.p[1], row_inv, w, (__half*)planes.hi, (__half*)planes.lo,
+    f16_planes_kernel<<<(M + w.N + 7) / 8, 256, 0, st>>>(x, M, K, out.lift, (__half*)out.p[0], (__half*)out.p[1], row_inv, w, (__half*)planes.hi, (__half*)planes.lo,
                                                          from, top);
     FC_LAUNCHED();
     return FC_OK;
@@ -551,29 +575,29 @@ int launch_split_f16(const float* x, const Planes& out, size_t n, cudaStream_t s
     if (n % 4 || out.n != 2 || out.scale == 0.0f) return fail(FC_E_SHAPE, "split_f16: %zu elements into %d planes", n, out.n);
     const size_t n4 = n / 4;
     split_f16_kernel<<<(int)std::max<size_t>(1, std::min<size_t>((n4 + 255) / 256, 148 * 8)), 256, 0, st>>>(
-        (const float4*)x, (uint2*)out.p[0], (uint2*)out.p[1], out.scale, n4);
+        (const float4*)x, (uint2*)out.p[0], (uint2*)out.p[1], out.scale, out.lift, n4);
     FC_LAUNCHED();
     return FC_OK;
 }
 
 int launch_gemm_f16(const F16Mat& w, const Planes& x, const float* row_inv, const float* bias, const float* residual, int epi, float* y, const Planes* yp,
-                    int M, int ldy, int* status, cudaStream_t st) {
+                    int M, int ldy, int* status, cudaStream_t st, bool exact) {
     F16Args a = {};
     a.bias = bias; a.residual = residual; a.gelu = epi == EPI_GELU; a.row_inv = row_inv; a.y = y; a.ldy = ldy; a.status = status;
     if (epi != EPI_NONE && epi != EPI_GELU) return fail(FC_E_ARG, "epilogue %d is not one of this entry's", epi);
-    if (y) return launch_f16<OUT_F32>(w, x, a, M, st);
-    if (!yp || yp->n != 2 || (w.N & 31) || (ldy & 7) || residual || row_inv || (epi == EPI_GELU) != (yp->scale != 0.0f))
-        return fail(FC_E_SHAPE, "plane output needs N %% 32 == 0, ldy %% 8 == 0, two planes (f16 behind GELU, else bf16) and no residual");
-    for (int p = 0; p < 2; ++p) a.yp[p] = (uint16_t*)yp->p[p];
-    a.out_scale = yp->scale;
-    return epi == EPI_GELU ? launch_f16<OUT_GELU>(w, x, a, M, st) : launch_f16<OUT_BF16>(w, x, a, M, st);
+    if (y) return launch_f16<OUT_F32>(w, x, a, M, exact, st);
+    if (!yp || (epi == EPI_GELU && yp->n != 2) || (w.N & 31) || (ldy & 7) || residual || row_inv || (epi == EPI_GELU) != (yp->scale != 0.0f))
+        return fail(FC_E_SHAPE, "plane output needs N %% 32 == 0, ldy %% 8 == 0, bf16 planes (behind GELU two f16 planes) and no residual");
+    for (int p = 0; p < yp->n; ++p) a.yp[p] = (uint16_t*)yp->p[p];
+    a.out_scale = yp->scale; a.out_lift = yp->lift;
+    return epi == EPI_GELU ? launch_f16<OUT_GELU>(w, x, a, M, exact, st) : launch_f16<OUT_BF16>(w, x, a, M, exact, st);
 }
 
-int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st) {
+int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st, bool exact) {
     if (!targets || !stats || !tlogit) return fail(FC_E_ARG, "the scoring epilogue needs targets, stats and tlogit");
     F16Args a = {};
     a.targets = targets; a.stats = (float4*)stats; a.tlogit = tlogit; a.status = status;
-    return launch_f16<OUT_SCORE>(w, x, a, M, st);
+    return launch_f16<OUT_SCORE>(w, x, a, M, exact, st);
 }
 
 }  // namespace fc
