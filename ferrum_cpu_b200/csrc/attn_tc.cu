@@ -22,6 +22,7 @@
 // Every mbarrier wait is bounded; on a timeout the status word is raised and the CTA leaves.
 //
 // Bound: tensor pipe / MUFU. 4·hd·T(T+1)/2 algorithmic FLOP per (window, head).
+#include "pdl.cuh"
 #include "tc.cuh"
 
 namespace fc {
@@ -160,7 +161,10 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
     const int h = blockIdx.y, b = blockIdx.z;
     const int T = a.win.length(b), row0 = a.win.begin(b); // the window's rows in [R]
     const int q0 = qt * QT;                               // first query of the tile inside the window
-    if (q0 >= T) return;                                  // a window shorter than the longest
+    if (q0 >= T) {                                        // a window shorter than the longest
+        pdl_wait();
+        return;
+    }
     const int last_q = min(T, q0 + QT) - 1;               // last valid query
     const int n_kt = last_q / KT + 1;                     // key tiles 0..n_kt-1 cover keys 0..last_q
 
@@ -182,6 +186,8 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
+    pdl_wait();                                           // set up while the kernel ahead still ran
+    pdl_trigger();
 
     if (warp == TMA_WARP) {
         if (tc::elect_one()) {
@@ -396,7 +402,7 @@ static int launch_attn_tc(const Planes& qkv, const Windows& w, int R, int H, int
     a.out_scale = out.scale; a.out_lift = out.lift;
     a.status = status;
     dim3 grid((w.T + QT - 1) / QT, H, w.B);
-    attn_prefill_tc_kernel<P><<<grid, THREADS, SMEM_BYTES<P>, st>>>(maps, a);
+    FC_CUDA(launch_pdl(attn_prefill_tc_kernel<P>, grid, dim3(THREADS), SMEM_BYTES<P>, st, maps, a));
     FC_LAUNCHED();
     return FC_OK;
 }

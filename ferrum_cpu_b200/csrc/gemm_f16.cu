@@ -135,6 +135,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = __shfl_sync(0xffffffffu, *(volatile uint32_t*)(tail + BAR_TMEM), 0);
     pdl_wait();                                                                     // set up while the kernel ahead still ran
+    pdl_trigger();
     // the barriers the pair's MMA issuer waits on are the leader's
     const uint32_t full_leader = CG == 2 ? mapa(full, 0) : full, acc_empty_leader = CG == 2 ? mapa(acc_empty, 0) : acc_empty;
 

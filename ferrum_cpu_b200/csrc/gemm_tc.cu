@@ -50,6 +50,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "pdl.cuh"
 #include "tc.cuh"
 
 namespace fc {
@@ -221,6 +222,8 @@ gemm_q8_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = __shfl_sync(0xffffffffu, *(volatile uint32_t*)(tail + BAR_TMEM), 0);
+    pdl_wait();                                             // set up while the kernel ahead still ran
+    pdl_trigger();
 
     // the barriers the pair's MMA issuers wait on are the leader's
     const uint32_t full_leader = CG == 2 ? mapa(full, 0) : full, acc_empty_leader = CG == 2 ? mapa(acc_empty, 0) : acc_empty;
@@ -577,12 +580,14 @@ int launch_one(const CUtensorMap (&map)[3], const TcArgs& a, int grid, int smem,
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)(CG == 2 ? 2 : a.ksplit);
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     FC_CUDA(cudaLaunchKernelEx(&cfg, gemm_q8_tc_kernel<CG, P, MODE, CW>, map[0], map[1], map[2], a));
     FC_LAUNCHED();
     return FC_OK;

@@ -107,6 +107,8 @@ template <int PER, int P>
 __global__ void layernorm_planes_kernel(const float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ b,
                                         const int* __restrict__ pick, int d, const Planes out) {
     __shared__ float red[33];
+    pdl_wait();
+    pdl_trigger();
     const float* xr = x + (size_t)(pick ? pick[blockIdx.x] : (int)blockIdx.x) * d;
     float v[PER];
     float s = 0.0f;
@@ -141,6 +143,8 @@ __global__ void __launch_bounds__(256) layernorm_planes_warp_kernel(const float*
                                                                     int d, const Planes out) {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_trigger();
     if (row >= rows) return;
     const int nv = d >> 7;                                  // 16-byte chunks per lane
     const float4* xr = (const float4*)(x + (size_t)(pick ? pick[row] : row) * d);
@@ -181,17 +185,15 @@ static int layernorm_planes(const float* x, const float* g, const float* b, cons
                             cudaStream_t st) {
     if (d % 128 == 0 && d <= 1024 && aligned16(x) && aligned16(g) && aligned16(b)) {
         const int blocks = (rows + 7) / 8;
-        if (d <= 512) layernorm_planes_warp_kernel<4, P><<<blocks, 256, 0, st>>>(x, g, b, pick, rows, d, out);
-        else layernorm_planes_warp_kernel<8, P><<<blocks, 256, 0, st>>>(x, g, b, pick, rows, d, out);
+        FC_CUDA(launch_pdl(d <= 512 ? layernorm_planes_warp_kernel<4, P> : layernorm_planes_warp_kernel<8, P>, dim3(blocks), dim3(256), 0, st, x, g, b, pick, rows, d, out));
         FC_LAUNCHED();
         return FC_OK;
     }
     const int threads = 256;
     const int per = (d + threads - 1) / threads;
-    if (per <= 4) layernorm_planes_kernel<4, P><<<rows, threads, 0, st>>>(x, g, b, pick, d, out);
-    else if (per <= 8) layernorm_planes_kernel<8, P><<<rows, threads, 0, st>>>(x, g, b, pick, d, out);
-    else if (per <= 16) layernorm_planes_kernel<16, P><<<rows, threads, 0, st>>>(x, g, b, pick, d, out);
-    else return fail(FC_E_SHAPE, "LayerNorm width %d exceeds 4096", d);
+    if (per > 16) return fail(FC_E_SHAPE, "LayerNorm width %d exceeds 4096", d);
+    FC_CUDA(launch_pdl(per <= 4 ? layernorm_planes_kernel<4, P> : per <= 8 ? layernorm_planes_kernel<8, P> : layernorm_planes_kernel<16, P>, dim3(rows),
+                       dim3(threads), 0, st, x, g, b, pick, d, out));
     FC_LAUNCHED();
     return FC_OK;
 }
