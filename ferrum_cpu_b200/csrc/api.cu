@@ -565,8 +565,9 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
     const int d = c.d_model, F = c.d_ff;
     cudaStream_t st = m->st;
     const bool tc_attn = tensor_attention(m);
-    // f16 planes, unless a few rows are better off where K is split over CTAs
-    const bool f16 = m->f16 && (planes == 2 || d >= kExactF16) && (!split_k || R >= 256);
+    // f16 planes, unless a few rows are better off where K is split over CTAs (prompts of 64 / 101 / 250 ids, 12 x 768: 1014 / 1033 / 1120 us
+    // on them, 932 / 1207 / 1469 split; 24 x 1024: 2273 / 2315 / 2506 and 2235 / 2449 / 3123)
+    const bool f16 = m->f16 && (planes == 2 || d >= kExactF16) && (!split_k || R > 64);
     m->pqkv.n = planes;
     m->pn.n = m->patt.n = m->phid.n = f16 ? 2 : planes;
     m->pn.lift = m->patt.lift = f16_lift(d, planes == 3);
