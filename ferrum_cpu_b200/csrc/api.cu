@@ -277,11 +277,14 @@ namespace fc {
 enum StepMode { STEP_NOHEAD = 0, STEP_SELECT = 1, STEP_PROBS = 2 };
 
 // Final LayerNorm, head and the selection of a step, on one row.
+static StepMat step_mat(const QMat& q, const float* bias = nullptr, int row = 0) {
+    return StepMat{q.qu + (size_t)row * q.K, q.d + (size_t)row * (q.K / 32), nullptr, bias ? bias + row : nullptr, 1};
+}
 // tail: the row as the halves of the last block left it (null: x is whole).
 static int launch_head(fc_stream* s, const float* x, int mode, const BlockRow* tail = nullptr) {
     fc_model* m = s->m;
     int n_stats = 0;
-    if (tail) FC_TRY(launch_head_row(m->head, *tail, s->logits, s->stats, &n_stats, s->state, m->st));
+    if (tail) FC_TRY(launch_head_row(step_mat(m->head), m->head.N, *tail, s->logits, s->stats, &n_stats, s->state, m->st));
     else FC_TRY(launch_gemv_row(m->head, x, RowNorm{m->lnfg, m->lnfb, 1e-5f}, nullptr, nullptr, EPI_NONE, s->logits, s->state, m->st, s->stats, &n_stats));
     return launch_step_finish(s->logits, m->cfg.vocab, s->stats, n_stats, mode == STEP_PROBS ? s->probs : nullptr, s->queue, s->queue_cap, s->state,
                               m->st);
@@ -305,11 +308,12 @@ static int launch_step(fc_stream* s, int mode, int split) {
             const LayerDev& L = m->layers[l];
             r.g = L.ln1g; r.b = L.ln1b;
             r.x_out = l ? s->att : nullptr;                  // the first row is whole as it is
-            FC_TRY(launch_attn_half(r, c.n_head, L.qkv, L.qkv_b, L.out, s->kc + l * layer_stride, s->vc + l * layer_stride, c.ctx, s->parts_a, s->state,
-                                    s->status, st));
+            const StepMat qkv[3] = {step_mat(L.qkv, L.qkv_b), step_mat(L.qkv, L.qkv_b, d), step_mat(L.qkv, L.qkv_b, 2 * d)}, up[2] = {step_mat(L.up, L.up_b), {}};
+            FC_TRY(launch_attn_half(r, c.n_head, c.n_head, StepRope(), qkv, step_mat(L.out), s->kc + l * layer_stride, s->vc + l * layer_stride, c.ctx,
+                                    s->parts_a, s->state, s->status, st));
             r = {l ? s->att : s->x, s->parts_a, L.out_b, s->q, L.ln2g, L.ln2b, c.n_head, d};
-            FC_TRY(launch_mlp_half(r, L.up, L.up_b, L.down, s->parts_m, s->state, s->status, st));
-            r = {s->q, s->parts_m, L.down_b, nullptr, m->lnfg, m->lnfb, block_step_slices(c.d_ff), d};
+            FC_TRY(launch_mlp_half(r, up, step_mat(L.down), c.d_ff, s->parts_m, s->state, s->status, st));
+            r = {s->q, s->parts_m, L.down_b, nullptr, m->lnfg, m->lnfb, block_step_slices(c.d_ff, false), d};
         }
         if (mode == STEP_NOHEAD) return launch_step_advance_pdl(s->state, st);
         return launch_head(s, nullptr, mode, &r);
@@ -1208,9 +1212,9 @@ int fc_stream_create(fc_model* m, fc_stream** out) {
     if (rc == FC_OK && cudaMemsetAsync(s->status, 0, sizeof(int), m->st) != cudaSuccess) rc = fail(FC_E_CUDA, "status word initialisation failed");
     const int hd = c.d_model / c.n_head;
     if (rc == FC_OK) rc = attn_step_split(c.n_head, hd, c.ctx, &s->attn_split, &s->split_from);
-    if (rc == FC_OK && block_step_covers(c.d_model, c.n_head, c.d_ff, c.ctx)) {
+    if (rc == FC_OK && block_step_covers(c.d_model, c.n_head, c.d_ff, c.ctx, false)) {
         rc = a.alloc_n(&s->parts_a, (size_t)c.n_head * c.d_model);
-        if (rc == FC_OK) rc = a.alloc_n(&s->parts_m, (size_t)block_step_slices(c.d_ff) * c.d_model);
+        if (rc == FC_OK) rc = a.alloc_n(&s->parts_m, (size_t)block_step_slices(c.d_ff, false) * c.d_model);
         s->split_from = INT_MAX;
     }
     if (rc == FC_OK && m->mega_grid > 0) {

@@ -1,8 +1,8 @@
-// A block of a GPT-2 decode step in two launches: layer/transformer.rs:221-294 for one token.
+// A block of a decode step in two launches: layer/transformer.rs:221-294 (GPT-2) and llm.rs:258-428 (Llama) for one token.
 //
 //     attention half   x = x0 + (parts + bias); q | k | v = Wqkv LN1(x) + b; append k, v; att = softmax(q Kᵀ / sqrt(hd)) V;
 //                      parts_a[h] = Wo[:, head h] att_h                               one cluster of CTAs a head
-//     MLP half         x = x0 + (parts_a + bias); hid = gelu(Wup LN2(x) + b);
+//     MLP half         x = x0 + (parts_a + bias); hid = gelu(Wup LN2(x) + b) or silu(Wgate RMS(x)) Wup RMS(x);
 //                      parts_m[c] = Wdown[:, slice c] hid_c                           one cluster of CTAs a slice of the hidden units
 //
 // One launch per operation (five a block) costs 16 us a block of width 768, of which the bytes explain 2: each launch pays its
@@ -24,7 +24,7 @@
 #include <algorithm>
 #include <atomic>
 
-#include "fc_common.cuh"
+#include "llama_ops.cuh"
 #include "pdl.cuh"
 
 namespace fc {
@@ -125,7 +125,7 @@ __device__ __forceinline__ bool received(const uint64_t* bar, const Waits& w) {
     const long long t0 = clock64();
     while (!poll())
         if (clock64() - t0 > w.cycles) {
-            atomicExch(w.status, FC_E_TIMEOUT);
+            if (w.status) atomicExch(w.status, FC_E_TIMEOUT);
             w.state->error = FC_E_TIMEOUT;
             return false;
         }
@@ -144,38 +144,46 @@ struct RowIn {
     float* x_out;                    // where the first cluster leaves it (null: nowhere)
     const float *g, *b;
     int n_part, d;
+    float eps;
 };
-struct Cols { const uint8_t* qu; const __half* d; int K; };   // a matrix whose columns are shared out
+// What a model's blocks are made of: LayerNorm, a head of its own for every query, GELU (GPT2); RMSNorm, rotated and grouped heads, SwiGLU
+// (LLAMA), the same on matrices of levels alone whose scales belong to the input index (LEVELS): the row is then staged once per
+// matrix that reads it, with its scales.
+enum Kind { GPT2, LLAMA, LEVELS };
 
 // Staged row: units of 16 bytes; eight consecutive lanes that read two of them each at a stride of 32 bytes meet every bank once.
 __device__ __forceinline__ int at16(int i) { return i ^ ((i >> 3) & 1); }
 
 // Shared memory of the row: what arrives (xr, stat, on bar), what is added up (add), the normalised row (xs).
+template <int COPIES>
 struct RowSmem {
-    float4 xr[MAX_D / 4], xs[MAX_D / 4], add[W][32];
+    float4 xr[MAX_D / 4], xs[COPIES][MAX_D / 4], add[W][32];
     float2 stat[MAX_C];
     uint64_t bar;
     __device__ __forceinline__ uint32_t bytes(int d, int C) const { return (uint32_t)(4 * d + 8 * C); }
 };
 // ahead: what does not depend on the kernel ahead; stage: the normalised row in s.xs, behind two block barriers. A CTA adds at most 32
 // units of 16 bytes.
-template <int C>
+template <int C, bool RMS, int COPIES>
 struct RowNormed {
-    float4 g, b, pb;
+    float4 g, b, pb, scale[COPIES];
     float inv_mine, inv_d;
-    __device__ __forceinline__ void ahead(const RowIn& r, int rank) {
+    __device__ __forceinline__ void ahead(const RowIn& r, int rank, const StepMat* mats) {
         const int tid = threadIdx.x, units = r.d >> 2, mine = units / C;
         inv_d = 1.0f / (float)r.d;
         inv_mine = (float)C * inv_d;
         g = b = pb = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (tid < units) {
             g = ((const float4*)r.g)[tid];
-            b = ((const float4*)r.b)[tid];
+            if (!RMS) b = ((const float4*)r.b)[tid];
+            if (COPIES > 1)
+#pragma unroll
+                for (int i = 0; i < COPIES; ++i) scale[i] = ((const float4*)mats[i].xscale)[tid];
         }
-        if (r.n_part && tid / 32 < C && (tid & 31) < mine) pb = ((const float4*)r.bias)[rank * mine + (tid & 31)];
+        if (r.n_part && r.bias && tid / 32 < C && (tid & 31) < mine) pb = ((const float4*)r.bias)[rank * mine + (tid & 31)];
     }
     // false: the row never came
-    __device__ __forceinline__ bool stage(const RowIn& r, RowSmem& s, int rank, bool first, bool& dead, Waits& waits) {
+    __device__ __forceinline__ bool stage(const RowIn& r, RowSmem<COPIES>& s, int rank, bool first, bool& dead, Waits& waits) {
         const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, units = r.d >> 2, mine = units / C, u = rank * mine + lane;
         // warp w adds rows w - 1 and w - 1 + W; row -1 is x
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -200,7 +208,7 @@ struct RowNormed {
             for (int i = 1; i < W; ++i) t = add4(t, s.add[i][lane]);            // rows that are not there: zeros
             v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (lane < mine) v = add4(s.add[0][lane], t);
-            const float m = warp_sum((v.x + v.y) + (v.z + v.w)) * inv_mine;
+            const float m = RMS ? 0.0f : warp_sum((v.x + v.y) + (v.z + v.w)) * inv_mine;
             float q = 0.0f;
             if (lane < mine) { const float a = v.x - m, c = v.y - m, e = v.z - m, f = v.w - m; q = (a * a + c * c) + (e * e + f * f); }
             q = warp_sum(q);
@@ -219,41 +227,50 @@ struct RowNormed {
         float sum = 0.0f, q = 0.0f, dev = 0.0f;
 #pragma unroll
         for (int i = 0; i < C; ++i) { sum += st[i].x; q += st[i].y; }
-        const float mean = sum / (float)C;
+        const float mean = RMS ? 0.0f : sum / (float)C;
+        if (!RMS)
 #pragma unroll
-        for (int i = 0; i < C; ++i) { const float dm = st[i].x - mean; dev = fmaf(dm, dm, dev); }
-        const float sd = sqrtf(fmaf(fmaf((float)(4 * mine), dev, q), inv_d, 1e-5f));     // the reference divides by the deviation
+            for (int i = 0; i < C; ++i) { const float dm = st[i].x - mean; dev = fmaf(dm, dm, dev); }
+        const float sd = sqrtf(fmaf(fmaf((float)(4 * mine), dev, q), inv_d, r.eps));
         if (tid < units) {
-            const float4 x = s.xr[tid];
-            s.xs[at16(tid)] = make_float4(((x.x - mean) / sd) * g.x + b.x, ((x.y - mean) / sd) * g.y + b.y, ((x.z - mean) / sd) * g.z + b.z,
-                                          ((x.w - mean) / sd) * g.w + b.w);
+            float4 x = s.xr[tid];
+            if (RMS) {
+                const float inv = 1.0f / sd;
+                x = make_float4(__fmul_rn(__fmul_rn(x.x, inv), g.x), __fmul_rn(__fmul_rn(x.y, inv), g.y), __fmul_rn(__fmul_rn(x.z, inv), g.z),
+                                __fmul_rn(__fmul_rn(x.w, inv), g.w));
+            } else {                                           // the reference divides by the deviation
+                x = make_float4(((x.x - mean) / sd) * g.x + b.x, ((x.y - mean) / sd) * g.y + b.y, ((x.z - mean) / sd) * g.z + b.z,
+                                ((x.w - mean) / sd) * g.w + b.w);
+            }
+#pragma unroll
+            for (int i = 0; i < COPIES; ++i)
+                s.xs[i][at16(tid)] = COPIES == 1 ? x : make_float4(x.x * scale[i].x, x.y * scale[i].y, x.z * scale[i].z, x.w * scale[i].w);
         }
         return __syncthreads_and(ok);
     }
 };
 
 // RB rows of a matrix against the staged row, by one warp: lanes across k, 8 levels a unit, NU units a lane.
-template <int NU, int RB>
+template <int NU, int RB, bool SCALED>
 struct WarpRows {
     uint2 q[RB][NU];
     __half d[RB][NU];
     float bias[RB];
-    __device__ __forceinline__ void ahead(const Cols& w, const float* b, const int (&row)[RB]) {
-        const int lane = threadIdx.x & 31, units = w.K >> 3;
+    // row r of this matrix becomes the warp's row `slot`
+    __device__ __forceinline__ void ahead(int slot, const StepMat& m, int r, int K) {
+        const int lane = threadIdx.x & 31, units = K >> 3;
+        const size_t at = (size_t)r * m.stride;
+        const uint2* src = (const uint2*)(m.qu + at * K);
 #pragma unroll
-        for (int r = 0; r < RB; ++r) {
-            const uint2* src = (const uint2*)(w.qu + (size_t)row[r] * w.K);
-            const __half* ds = w.d + (size_t)row[r] * (w.K >> 5);
-#pragma unroll
-            for (int i = 0; i < NU; ++i) {
-                const int u = lane + 32 * i;
-                q[r][i] = u < units ? ld_once(src + u) : make_uint2(0x80808080u, 0x80808080u);
-                d[r][i] = u < units ? ds[u >> 2] : __ushort_as_half((unsigned short)0);
-            }
-            bias[r] = b[row[r]];
+        for (int i = 0; i < NU; ++i) {
+            const int u = lane + 32 * i;
+            q[slot][i] = u < units ? ld_once(src + u) : make_uint2(0x80808080u, 0x80808080u);
+            if (SCALED) d[slot][i] = u < units ? m.d[at * (K >> 5) + (u >> 2)] : __ushort_as_half((unsigned short)0);
         }
+        bias[slot] = m.bias ? m.bias[r] : 0.0f;
     }
-    __device__ __forceinline__ void run(const float4* xs, int units, float (&out)[RB]) const {
+    // odd_xs: the staged row of rows 1, 3, .. (the two of a SwiGLU pair have matrices of their own)
+    __device__ __forceinline__ void run(const float4* xs, const float4* odd_xs, int units, float (&out)[RB]) const {
         const int lane = threadIdx.x & 31;
 #pragma unroll
         for (int r = 0; r < RB; ++r) out[r] = 0.0f;
@@ -262,11 +279,13 @@ struct WarpRows {
             const int u = lane + 32 * i;
             if (u >= units) break;
             const ulonglong2 x0 = *(const ulonglong2*)&xs[at16(2 * u)], x1 = *(const ulonglong2*)&xs[at16(2 * u + 1)];
+            ulonglong2 y0 = x0, y1 = x1;
+            if (odd_xs != xs) { y0 = *(const ulonglong2*)&odd_xs[at16(2 * u)]; y1 = *(const ulonglong2*)&odd_xs[at16(2 * u + 1)]; }
 #pragma unroll
             for (int r = 0; r < RB; ++r) {
                 uint64_t t = 0;
-                fma8(t, q[r][i].x, q[r][i].y, x0, x1);
-                out[r] = fmaf(__half2float(d[r][i]), both(t), out[r]);
+                fma8(t, q[r][i].x, q[r][i].y, r & 1 ? y0 : x0, r & 1 ? y1 : x1);
+                out[r] = SCALED ? fmaf(__half2float(d[r][i]), both(t), out[r]) : out[r] + both(t);
             }
         }
 #pragma unroll
@@ -276,24 +295,28 @@ struct WarpRows {
 
 struct AttnHalf {
     RowIn in;
-    Cols qkv, out;
-    const float* qkv_b;
+    StepMat qkv[3], out;
+    StepRope rope;
     float *kc, *vc, *parts;          // parts [heads][d]
-    int ctx, cap;                    // cap: cached rows a CTA may hold
+    int n_head, n_kv, ctx, cap;      // cap: cached rows a CTA may hold; further ones are read where they are
     Waits waits;
 };
 
 // Heads of HD, C = HD / 8 CTAs each, 24 rows of q, k and v a CTA: two for each of the first 12 warps.
-template <int HD, int NU>
+template <int HD, int NU, Kind KIND>
 __global__ void __launch_bounds__(T, 2) attn_half_kernel(const AttnHalf a) {
+    constexpr bool RMS = KIND != GPT2;
+    constexpr int COPIES = KIND == LEVELS ? 3 : 1;
+    constexpr bool FAR = RMS;                                  // rows beyond the held ones may occur
     constexpr int C = HD / 8, U = HD / 4, KS = HD == 64 ? 80 : HD + 16;   // key rows at a stride of 4 mod 8 units of 16 bytes
-    extern __shared__ __align__(16) float sm[];                // K [cap][KS] | V [cap][HD] | scores [cap]
-    __shared__ __align__(16) RowSmem rs;
+    extern __shared__ __align__(16) float sm[];                // K [cap][KS] | V [cap][HD] | scores of the part
+    __shared__ __align__(16) RowSmem<COPIES> rs;
     __shared__ __align__(16) float qkv[3][HD], part[W][HD], att[HD], peer_o[C][HD];
     __shared__ float2 peer_ml[C];
     __shared__ float red[2][W];
     __shared__ uint64_t bars[2];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, h = blockIdx.x / C, rank = blockIdx.x % C, d = a.in.d;
+    const int kvh = RMS ? h / (a.n_head / a.n_kv) : h, kv_dim = RMS ? a.n_kv * HD : d;
     if (tid == 0) {
         expect(&rs.bar, rs.bytes(d, C));
         expect(&bars[0], 3 * HD * 4);
@@ -305,13 +328,14 @@ __global__ void __launch_bounds__(T, 2) attn_half_kernel(const AttnHalf a) {
     // rows i = 2 wid, 2 wid + 1 of this CTA's 24: row rank * 8 + i % 8 of the head's q, k or v
     const bool has_rows = wid < 12;
     const int i0 = 2 * wid;
-    WarpRows<NU, 2> w;
+    WarpRows<NU, 2, KIND != LEVELS> w;
     if (has_rows) {
-        const int first = (i0 >> 3) * d + h * HD + rank * 8 + (i0 & 7), rows[2] = {first, first + 1};
-        w.ahead(a.qkv, a.qkv_b, rows);
+        const int first = (i0 < 8 ? h : kvh) * HD + rank * 8 + (i0 & 7);
+        w.ahead(0, a.qkv[i0 >> 3], first, d);
+        w.ahead(1, a.qkv[i0 >> 3], first + 1, d);
     }
-    RowNormed<C> row;
-    row.ahead(a.in, rank);
+    RowNormed<C, RMS, COPIES> row;
+    row.ahead(a.in, rank, a.qkv);
     // output rows of this CTA: TPR threads a row, 16 columns each, T / TPR rows a pass
     constexpr int UNITS = HD / 16, TPR = UNITS, PASSES = (MAX_D / C * TPR + T - 1) / T;
     const int per_cta = d / C, sub = tid % TPR, unit = h * UNITS + sub;
@@ -322,19 +346,25 @@ __global__ void __launch_bounds__(T, 2) attn_half_kernel(const AttnHalf a) {
         const int n = tid / TPR + i * (T / TPR);
         if (n >= per_cta) continue;
         oq[i] = ld_once((const uint4*)(a.out.qu + (size_t)(rank * per_cta + n) * d) + unit);
-        od[i] = __half2float(a.out.d[(size_t)(rank * per_cta + n) * (d >> 5) + (unit >> 1)]);
+        od[i] = KIND == LEVELS ? 1.0f : __half2float(a.out.d[(size_t)(rank * per_cta + n) * (d >> 5) + (unit >> 1)]);
     }
+    const float out_scale = KIND == LEVELS && tid < HD ? a.out.xscale[h * HD + tid] : 1.0f;
     // this CTA's part of the positions 0..pos; the last one of the last part is this step's row
     const int pos = a.waits.state->pos, last = min(pos, a.ctx - 1);
     const int per = (int)((unsigned)(last + C) / (unsigned)C), begin = rank * per, len = max(0, min(per, last + 1 - begin));
     const int own = begin + len == last + 1 && len > 0 ? len - 1 : -1;
     float *kt = sm, *vt = sm + (size_t)a.cap * KS, *sc = vt + (size_t)a.cap * HD;
+    const float *kg = a.kc + (size_t)begin * kv_dim + (size_t)kvh * HD, *vg = a.vc + (size_t)begin * kv_dim + (size_t)kvh * HD;
     {
-        const float *kg = a.kc + (size_t)begin * d + (size_t)h * HD, *vg = a.vc + (size_t)begin * d + (size_t)h * HD;
-        const int held = own >= 0 ? own : len;
-        for (int i = tid; i < held * U; i += T) copy16(kt + (i / U) * KS + (i % U) * 4, kg + (size_t)(i / U) * d + (i % U) * 4);
-        for (int i = tid; i < held * U; i += T) copy16(vt + i * 4, vg + (size_t)(i / U) * d + (i % U) * 4);
+        const int held = min(own >= 0 ? own : len, a.cap);
+        for (int i = tid; i < held * U; i += T) copy16(kt + (i / U) * KS + (i % U) * 4, kg + (size_t)(i / U) * kv_dim + (i % U) * 4);
+        for (int i = tid; i < held * U; i += T) copy16(vt + i * 4, vg + (size_t)(i / U) * kv_dim + (i % U) * 4);
     }
+    // threads of the first two warps rotate a pair each, of q, then of k
+    const int pair = tid & 31;
+    const bool turns = RMS && tid < 64 && pair < a.rope.half;
+    float sn = 0.0f, cs = 1.0f;
+    if (turns) sincosf(rope_angle(pos, a.rope.ftab[pair], a.rope.inv_linear), &sn, &cs);
 
     cluster_wait();                                            // all have started
     pdl_wait();
@@ -346,7 +376,8 @@ __global__ void __launch_bounds__(T, 2) attn_half_kernel(const AttnHalf a) {
     dead |= pos >= a.ctx;
     if (has_rows) {
         float r[2];
-        w.run(rs.xs, d >> 3, r);
+        const float4* xs = rs.xs[COPIES == 1 ? 0 : i0 >> 3];
+        w.run(xs, xs, d >> 3, r);
         // every CTA of the cluster gets every row: lane l sends to rank l
         if (lane < C) {
             float* to = &qkv[i0 >> 3][rank * 8 + (i0 & 7)];
@@ -354,10 +385,25 @@ __global__ void __launch_bounds__(T, 2) attn_half_kernel(const AttnHalf a) {
             send(to + 1, &bars[0], lane, r[1]);
         }
     }
-    bool ok = received(&bars[0], waits);
-    if (rank == 0 && tid < 2 * HD && ok && !dead) {
+    bool ok = true;
+    if (!RMS) {
+        ok = received(&bars[0], waits);
+    } else {
+        if (tid < 64) {
+            ok = received(&bars[0], waits);
+            if (turns) {
+                float* v = qkv[tid >> 5];
+                const int i = a.rope.neox ? pair : 2 * pair, j = a.rope.neox ? pair + a.rope.half : i + 1;
+                const float x = v[i], y = v[j];
+                v[i] = __fsub_rn(__fmul_rn(x, cs), __fmul_rn(y, sn));
+                v[j] = __fadd_rn(__fmul_rn(x, sn), __fmul_rn(y, cs));
+            }
+        }
+        ok = __syncthreads_and(ok);
+    }
+    if (rank == 0 && (!RMS || kvh * (a.n_head / a.n_kv) == h) && tid < 2 * HD && ok && !dead) {
         const int k = tid / HD;
-        (k ? a.vc : a.kc)[(size_t)pos * d + (size_t)h * HD + tid % HD] = qkv[1 + k][tid % HD];
+        (k ? a.vc : a.kc)[(size_t)pos * kv_dim + (size_t)kvh * HD + tid % HD] = qkv[1 + k][tid % HD];
     }
     // scores: 4 lanes a key
     const float scale = 1.0f / sqrtf((float)HD);
@@ -370,12 +416,16 @@ __global__ void __launch_bounds__(T, 2) attn_half_kernel(const AttnHalf a) {
         const int j = j0 + key0;
         float dot = 0.0f, dot2 = 0.0f;
         if (j < len) {
-            const float4* k4 = (const float4*)(j == own ? qkv[1] : kt + (size_t)j * KS);
+            auto dots = [&](const float4* k4) {
 #pragma unroll
-            for (int u = 0; u < U / 4; u += 2) {
-                dot = dot4(q[u], k4[u * 4 + sl], dot);
-                dot2 = dot4(q[u + 1], k4[u * 4 + 4 + sl], dot2);
-            }
+                for (int u = 0; u < U / 4; u += 2) {
+                    dot = dot4(q[u], k4[u * 4 + sl], dot);
+                    dot2 = dot4(q[u + 1], k4[u * 4 + 4 + sl], dot2);
+                }
+            };
+            // apart, so that the rows in shared memory are read as such
+            if (FAR && j >= a.cap && j != own) dots((const float4*)(kg + (size_t)j * kv_dim));
+            else dots((const float4*)(j == own ? qkv[1] : kt + j * KS));
         }
         dot += dot2;
         dot += __shfl_xor_sync(0xffffffffu, dot, 1);
@@ -403,7 +453,9 @@ __global__ void __launch_bounds__(T, 2) attn_half_kernel(const AttnHalf a) {
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 2
     for (int j = tid / U; j < len; j += R) {
-        const float4 v = ((const float4*)(j == own ? qkv[2] : vt + (size_t)j * HD))[col];
+        float4 v;
+        if (FAR && j >= a.cap && j != own) v = ((const float4*)(vg + (size_t)j * kv_dim))[col];
+        else v = ((const float4*)(j == own ? qkv[2] : vt + j * HD))[col];
         const float p = expf(sc[j] - M0);
         L += p;
         acc.x = fmaf(p, v.x, acc.x); acc.y = fmaf(p, v.y, acc.y); acc.z = fmaf(p, v.z, acc.z); acc.w = fmaf(p, v.w, acc.w);
@@ -454,7 +506,7 @@ __global__ void __launch_bounds__(T, 2) attn_half_kernel(const AttnHalf a) {
         for (int k = C / 2; k > 0; k >>= 1)
 #pragma unroll
             for (int i = 0; i < k; ++i) { f[i] += f[i + k]; o[i] += o[i + k]; }
-        att[tid] = o[0] / f[0];
+        att[tid] = KIND == LEVELS ? (o[0] / f[0]) * out_scale : o[0] / f[0];
     }
     if (!__syncthreads_and(ok)) { outstay(); return; }
     ulonglong2 ov[4];
@@ -472,20 +524,21 @@ __global__ void __launch_bounds__(T, 2) attn_half_kernel(const AttnHalf a) {
 
 struct MlpHalf {
     RowIn in;
-    Cols up, down;
-    const float* up_b;
+    StepMat up[2], down;             // up, or gate and up
     float* parts;                    // [slices][d]
-    int slice;                       // hidden units of a cluster
+    int slice, F;                    // hidden units of a cluster, of all
     Waits waits;
 };
 
-// Clusters of 8; a warp computes RB rows of up; 16 threads share RD rows of down, 16 columns of them each: the reads of the hidden units
+// Clusters of 8; a warp computes RB rows of up (of gate and up in turn: RB / 2 hidden units); 16 threads share RD rows of down, 16 columns of them each: the reads of the hidden units
 // from shared memory are what a product of so few columns would else be bound by (with a row a thread 1300 cycles).
-template <int NU, int RB, int RD>
+template <int NU, int RB, int RD, Kind KIND>
 __global__ void __launch_bounds__(T, 2) mlp_half_kernel(const MlpHalf a) {
+    constexpr bool RMS = KIND != GPT2;
+    constexpr int COPIES = KIND == LEVELS ? 2 : 1, HB = RMS ? RB / 2 : RB;   // HB: hidden units of a warp
     constexpr int C = 8, GROUPS = T / 16;               // RD x GROUPS rows of down: at least d / 8
     extern __shared__ __align__(16) unsigned char cols[];      // this CTA's rows of the slice's columns of down
-    __shared__ __align__(16) RowSmem rs;
+    __shared__ __align__(16) RowSmem<COPIES> rs;
     __shared__ __align__(16) float hid[MAX_SLICE];
     __shared__ uint64_t bar;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, c = blockIdx.x / C, rank = blockIdx.x % C, d = a.in.d;
@@ -496,24 +549,33 @@ __global__ void __launch_bounds__(T, 2) mlp_half_kernel(const MlpHalf a) {
     }
     __syncwarp();
     cluster_arrive();
-    const int share = a.slice / C, u0 = wid * RB;              // this warp's first unit of the CTA's share
-    int rows[RB];
+    const int share = a.slice / C, u0 = wid * HB;              // this warp's first unit of the CTA's share
+    WarpRows<NU, RB, KIND != LEVELS> w;
+    float down_scale[HB];
 #pragma unroll
-    for (int i = 0; i < RB; ++i) rows[i] = c * a.slice + rank * share + min(u0 + i, share - 1);
-    WarpRows<NU, RB> w;
-    w.ahead(a.up, a.up_b, rows);
-    RowNormed<C> row;
-    row.ahead(a.in, rank);
+    for (int i = 0; i < HB; ++i) {
+        const int f = c * a.slice + rank * share + min(u0 + i, share - 1);
+        if (RMS) {
+            w.ahead(2 * i, a.up[0], f, d);
+            w.ahead(2 * i + 1, a.up[1], f, d);
+        } else {
+            w.ahead(i, a.up[0], f, d);
+        }
+        down_scale[i] = KIND == LEVELS ? a.down.xscale[f] : 1.0f;
+    }
+    RowNormed<C, RMS, COPIES> row;
+    row.ahead(a.in, rank, a.up);
     const int per_cta = d / C, units = a.slice >> 4, unit = tid & 15;
     for (int i = tid; i < per_cta * units; i += T) {
         const int n = i / units, u = i % units;
-        copy16(cols + i * 16, a.down.qu + (size_t)(rank * per_cta + n) * a.down.K + c * a.slice + u * 16);
+        copy16(cols + i * 16, a.down.qu + (size_t)(rank * per_cta + n) * a.F + c * a.slice + u * 16);
     }
     float dd[RD];
 #pragma unroll
     for (int i = 0; i < RD; ++i) {
         const int n = tid / 16 + i * GROUPS;
-        dd[i] = n < per_cta && unit < units ? __half2float(a.down.d[(size_t)(rank * per_cta + n) * (a.down.K >> 5) + ((c * units + unit) >> 1)]) : 0.0f;
+        dd[i] = KIND == LEVELS ? 1.0f
+              : n < per_cta && unit < units ? __half2float(a.down.d[(size_t)(rank * per_cta + n) * (a.F >> 5) + ((c * units + unit) >> 1)]) : 0.0f;
     }
 
     cluster_wait();                                            // all have started
@@ -524,12 +586,15 @@ __global__ void __launch_bounds__(T, 2) mlp_half_kernel(const MlpHalf a) {
     pdl_trigger();
     if (!came) { outstay(); return; }
     float r[RB];
-    w.run(rs.xs, d >> 3, r);
+    w.run(rs.xs[0], rs.xs[COPIES - 1], d >> 3, r);
 #pragma unroll
-    for (int i = 0; i < RB; ++i)
+    for (int i = 0; i < HB; ++i)
         if (lane < C && u0 + i < share) {
             const int e = rank * share + u0 + i;
-            send(&hid[e ^ ((e >> 3) & 12)], &bar, lane, gelu_f(r[i]));
+            float v;
+            if constexpr (RMS) v = __fmul_rn(__fdiv_rn(r[2 * i], __fadd_rn(1.0f, expf(-r[2 * i]))), r[2 * i + 1]);
+            else v = gelu_f(r[i]);
+            send(&hid[e ^ ((e >> 3) & 12)], &bar, lane, KIND == LEVELS ? v * down_scale[i] : v);
         }
     if (!received(&bar, waits)) { outstay(); return; }
     // eight threads that read the same quarter of their units meet every bank once: quarter j of unit u lies at j ^ (u / 2) % 4
@@ -582,44 +647,64 @@ int launch_clusters(K kernel, int grid, int cluster, size_t smem, cudaStream_t s
     return FC_OK;
 }
 
-// Clusters that share the hidden units: as many as leave a warp two or three of them.
-int mlp_slices(int F) {
+// Clusters that share the hidden units: as many as leave a warp two or three rows of up, or of gate and up two or four.
+int mlp_slices(int F, bool gated) {
     for (int n : {16, 8, 4, 2, 1}) {
-        const int share = F / (n * 8), rb = (share + W - 1) / W;
-        if (F % (n * 8) == 0 && F / n % 32 == 0 && F / n <= 256 && (rb == 2 || rb == 3)) return n;
+        const int share = F / (n * 8), per_warp = (share + W - 1) / W;
+        if (F % (n * 8) == 0 && F / n % 32 == 0 && F / n <= 256 && per_warp <= (gated ? 2 : 3) && per_warp >= (gated ? 1 : 2)) return n;
     }
     return 0;
 }
-size_t attn_half_smem(int hd, int ctx) { return (size_t)((ctx + hd / 8 - 1) / (hd / 8)) * ((hd == 64 ? 80 : hd + 16) + hd + 1) * 4; }
+constexpr int HELD = 128;      // cached rows a CTA holds: two CTAs an SM
+int attn_cap(int ctx) { return std::min(HELD, (ctx + 7) / 8); }
+size_t attn_half_smem(int ctx) { return ((size_t)attn_cap(ctx) * (80 + 64) + (size_t)((ctx + 7) / 8)) * 4; }
 
 }  // namespace
 
 // Heads of 64 (8 CTAs each), rows of 512 to 1024 in multiples of 128, hidden units that split evenly. Us a token on two launches a block (on
-// five): 12 x 768 at 32 positions 140 (217), at 256 142 (237), at 900 153 (255); 24 x 1024 317 (447), 322 (488), 339 (533). Narrower rows keep a
+// five): 12 x 768 at 32 positions 140 (217), at 256 142 (237), at 900 153 (255); 24 x 1024 317 (447), 322 (488), 339 (533); Llama, 16 x 512, int8 levels, 33 + 64 tokens 12.8 ms (17.3). Narrower rows keep a
 // launch per operation, which is what a step of 128 columns is counted in.
-bool block_step_covers(int d, int n_head, int F, int ctx) {
-    return d % 128 == 0 && d >= 512 && d <= MAX_D && n_head * 64 == d && n_head <= MAX_PARTS && mlp_slices(F) > 0 && attn_half_smem(64, ctx) <= 80 * 1024;
+bool block_step_covers(int d, int n_head, int F, int ctx, bool gated) {
+    return d % 128 == 0 && d >= 512 && d <= MAX_D && n_head * 64 == d && n_head <= MAX_PARTS && mlp_slices(F, gated) > 0 &&
+           (gated ? attn_half_smem(ctx) <= 90 * 1024 : ctx <= 8 * HELD);
 }
-int block_step_slices(int F) { return mlp_slices(F); }
+int block_step_slices(int F, bool gated) { return mlp_slices(F, gated); }
 
-int launch_attn_half(const BlockRow& r, int n_head, const QMat& qkv, const float* qkv_b, const QMat& out, float* kc, float* vc, int ctx, float* parts,
-                     StepState* state, int* status, cudaStream_t st) {
+int launch_attn_half(const BlockRow& r, int n_head, int n_kv, const StepRope& rope, const StepMat (&qkv)[3], const StepMat& out, float* kc, float* vc, int ctx,
+                     float* parts, StepState* state, int* status, cudaStream_t st) {
     constexpr int HD = 64, C = HD / 8;
     const int d = r.d;
-    const AttnHalf a = {{r.x, r.part, r.bias, r.x_out, r.g, r.b, r.n_part, d}, {qkv.qu, qkv.d, d}, {out.qu, out.d, d}, qkv_b, kc, vc, parts, ctx,
-                        (ctx + C - 1) / C, {status, state, g_debug.wait_cycles, g_debug.withhold}};
-    auto go = [&](auto kernel) { return launch_clusters(kernel, n_head * C, C, attn_half_smem(HD, ctx), st, a); };
-    return d > 768 ? go(attn_half_kernel<HD, 4>) : d > 512 ? go(attn_half_kernel<HD, 3>) : go(attn_half_kernel<HD, 2>);
+    const AttnHalf a = {{r.x, r.part, r.bias, r.x_out, r.g, r.b, r.n_part, d, r.eps}, {qkv[0], qkv[1], qkv[2]}, out, rope, kc, vc, parts, n_head, n_kv, ctx,
+                        attn_cap(ctx), {status, state, g_debug.wait_cycles, g_debug.withhold}};
+    auto go = [&](auto kernel) { return launch_clusters(kernel, n_head * C, C, attn_half_smem(ctx), st, a); };
+    auto of = [&](auto kind) {
+        constexpr Kind K = decltype(kind)::value;
+        return d > 768 ? go(attn_half_kernel<HD, 4, K>) : d > 512 ? go(attn_half_kernel<HD, 3, K>) : go(attn_half_kernel<HD, 2, K>);
+    };
+    if (r.b) return of(std::integral_constant<Kind, GPT2>());
+    return out.xscale ? of(std::integral_constant<Kind, LEVELS>()) : of(std::integral_constant<Kind, LLAMA>());
 }
 
-int launch_mlp_half(const BlockRow& r, const QMat& up, const float* up_b, const QMat& down, float* parts, StepState* state, int* status, cudaStream_t st) {
-    const int d = r.d, F = up.N, slices = mlp_slices(F), slice = F / slices, rb = (slice / 8 + W - 1) / W;
-    const MlpHalf a = {{r.x, r.part, r.bias, r.x_out, r.g, r.b, r.n_part, d}, {up.qu, up.d, d}, {down.qu, down.d, F}, up_b, parts, slice,
+int launch_mlp_half(const BlockRow& r, const StepMat (&up)[2], const StepMat& down, int F, float* parts, StepState* state, int* status, cudaStream_t st) {
+    const bool gated = !r.b;
+    const int d = r.d, slices = mlp_slices(F, gated), slice = F / slices, per_warp = (slice / 8 + W - 1) / W;
+    const MlpHalf a = {{r.x, r.part, r.bias, r.x_out, r.g, r.b, r.n_part, d, r.eps}, {up[0], up[1]}, down, parts, slice, F,
                        {status, state, g_debug.wait_cycles, g_debug.withhold}};
     auto go = [&](auto kernel) { return launch_clusters(kernel, slices * 8, 8, (size_t)(d / 8) * slice, st, a); };
-    if (d > 768) return rb == 2 ? go(mlp_half_kernel<4, 2, 6>) : go(mlp_half_kernel<4, 3, 6>);
-    if (d > 512) return rb == 2 ? go(mlp_half_kernel<3, 2, 4>) : go(mlp_half_kernel<3, 3, 4>);
-    return rb == 2 ? go(mlp_half_kernel<2, 2, 4>) : go(mlp_half_kernel<2, 3, 4>);
+    // FEW, MANY: rows of a warp
+    auto of = [&](auto kind, auto few, auto many) {
+        constexpr Kind K = decltype(kind)::value;
+        constexpr int FEW = decltype(few)::value, MANY = decltype(many)::value;
+        const bool more = per_warp * (gated ? 2 : 1) > FEW;
+        if (d > 768) return more ? go(mlp_half_kernel<4, MANY, 6, K>) : go(mlp_half_kernel<4, FEW, 6, K>);
+        if (d > 512) return more ? go(mlp_half_kernel<3, MANY, 4, K>) : go(mlp_half_kernel<3, FEW, 4, K>);
+        return more ? go(mlp_half_kernel<2, MANY, 4, K>) : go(mlp_half_kernel<2, FEW, 4, K>);
+    };
+    const std::integral_constant<int, 2> two;
+    const std::integral_constant<int, 3> three;
+    const std::integral_constant<int, 4> four;
+    if (!gated) return of(std::integral_constant<Kind, GPT2>(), two, three);
+    return down.xscale ? of(std::integral_constant<Kind, LEVELS>(), two, four) : of(std::integral_constant<Kind, LLAMA>(), two, four);
 }
 
 }  // namespace fc

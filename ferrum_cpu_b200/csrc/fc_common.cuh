@@ -183,23 +183,38 @@ int attn_step_split(int n_q, int hd, int ctx, int* split, int* from);
 int launch_attn_step(const float* qkv, int n_q, int n_kv, int hd, int rope_dim, int neox, const float2* ftab, float inv_linear,
                      float* kc, float* vc, int ctx, int split, const StepState* state, float* out, cudaStream_t st);
 
-// block_step.cu — a GPT-2 block of a decode step in two launches, each on the row x + (part[0] + .. + part[n_part - 1] + bias), left in
-// x_out (null: nowhere), behind LayerNorm (g, b). The attention half leaves parts [n_head][d], the MLP half [block_step_slices][d]. The
-// state and the cached rows are read ahead of the wait, as in launch_attn_step. `status` is raised when a bounded wait runs out.
+// block_step.cu — a block of a decode step in two launches, each on the row x + (part[0] + .. + part[n_part - 1] + bias), left in
+// x_out (null: nowhere), behind LayerNorm (g, b) or RMSNorm (b null: a Llama block; bias may be null). The attention half leaves parts
+// [n_head][d], the MLP half [block_step_slices][d]. The state and the cached rows are read ahead of the wait, as in launch_attn_step.
+// `status` (may be null) and the state's error are raised when a bounded wait runs out.
 struct BlockRow {
     const float *x, *part, *bias;
     float* x_out;
     const float *g, *b;
     int n_part, d;
+    float eps = 1e-5f;
 };
-bool block_step_covers(int d, int n_head, int F, int ctx);
-int block_step_slices(int F);
-int launch_attn_half(const BlockRow& r, int n_head, const QMat& qkv, const float* qkv_b, const QMat& out, float* kc, float* vc, int ctx, float* parts,
-                     StepState* state, int* status, cudaStream_t st);
-int launch_mlp_half(const BlockRow& r, const QMat& up, const float* up_b, const QMat& down, float* parts, StepState* state, int* status, cudaStream_t st);
+// A matrix of such a block: row r lies at r x stride; d: f16 scales per 32 of k, or null with xscale, the scale of input index k.
+struct StepMat {
+    const uint8_t* qu = nullptr;
+    const __half* d = nullptr;
+    const float *xscale = nullptr, *bias = nullptr;
+    int stride = 1;
+};
+struct StepRope {
+    int half = 0, neox = 0;
+    const float2* ftab = nullptr;
+    float inv_linear = 1.0f;
+};
+bool block_step_covers(int d, int n_head, int F, int ctx, bool gated);
+int block_step_slices(int F, bool gated);
+int launch_attn_half(const BlockRow& r, int n_head, int n_kv, const StepRope& rope, const StepMat (&qkv)[3], const StepMat& out, float* kc, float* vc, int ctx,
+                     float* parts, StepState* state, int* status, cudaStream_t st);
+int launch_mlp_half(const BlockRow& r, const StepMat (&up)[2] /* up, or gate and up */, const StepMat& down, int F, float* parts, StepState* state, int* status,
+                    cudaStream_t st);
 
-// head_row.cu — the product behind those: logits and, per CTA, the largest and the mass around it (kRowStats entries at most).
-int launch_head_row(const QMat& w, const BlockRow& r, float* logits, float2* stats, int* n_stats, const StepState* state, cudaStream_t st);
+// head_row.cu — the product behind those: N logits and, with stats, per CTA the largest and the mass around it (kRowStats entries at most).
+int launch_head_row(const StepMat& w, int N, const BlockRow& r, float* logits, float2* stats, int* n_stats, const StepState* state, cudaStream_t st);
 
 // Windows of rows that share a forward pass: window b holds rows starts[b] .. starts[b + 1] (device array of B + 1), or, with
 // starts == nullptr, T rows each. T: rows of the longest.

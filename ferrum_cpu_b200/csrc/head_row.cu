@@ -34,13 +34,15 @@ __device__ __forceinline__ float warp_sum(float t) {
 
 struct HeadArgs {
     const uint8_t* qu; const __half* d; int N, K;
-    const float *x, *part, *bias, *g, *b;
+    const float *x, *part, *bias, *g, *b, *xscale;
     int n_part;
+    float eps;
     float* out; float2* stats;
     const StepState* state;
 };
 
-template <int NU>
+// RMS: RMSNorm in LayerNorm's place. SCALED: f16 scales per 32 of k, else levels alone and the scales of the input indices.
+template <int NU, bool RMS, bool SCALED>
 __global__ void __launch_bounds__(T, 1) head_row_kernel(const HeadArgs a) {
     constexpr int DEPTH = NU <= 2 ? 4 : NU == 3 ? 3 : 2;     // tasks in flight: as many as the registers hold
     extern __shared__ __align__(16) float4 add[];            // [n_part + 1][K / 4]
@@ -59,17 +61,18 @@ __global__ void __launch_bounds__(T, 1) head_row_kernel(const HeadArgs a) {
             for (int u = 0; u < NU; ++u) {
                 if (lane + 32 * u >= units) continue;
                 asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(r.q[i][u].x), "=r"(r.q[i][u].y) : "l"(q + lane + 32 * u));
-                r.d[i][u] = d[(lane + 32 * u) >> 2];
+                if (SCALED) r.d[i][u] = d[(lane + 32 * u) >> 2];
             }
         }
     };
 #pragma unroll
     for (int i = 0; i < DEPTH; ++i) fetch(w[i], first + i * step);
-    float4 g = {}, b = {}, pb = {};
+    float4 g = {}, b = {}, pb = {}, xs = {};
     if (tid < quads) {
         g = ((const float4*)a.g)[tid];
-        b = ((const float4*)a.b)[tid];
-        if (a.n_part) pb = ((const float4*)a.bias)[tid];
+        if (!RMS) b = ((const float4*)a.b)[tid];
+        if (!SCALED) xs = ((const float4*)a.xscale)[tid];
+        if (a.n_part && a.bias) pb = ((const float4*)a.bias)[tid];
     }
 
     pdl_wait();
@@ -92,7 +95,7 @@ __global__ void __launch_bounds__(T, 1) head_row_kernel(const HeadArgs a) {
     }
     // every warp takes the mean of its own elements and the squares around it; merged around the common mean
     auto count = [&](int wi) { return (float)min(max(K - 128 * wi, 0), 128); };
-    const float n_w = count(wid), m_w = n_w > 0.0f ? warp_sum((v.x + v.y) + (v.z + v.w)) / n_w : 0.0f;
+    const float n_w = count(wid), m_w = !RMS && n_w > 0.0f ? warp_sum((v.x + v.y) + (v.z + v.w)) / n_w : 0.0f;
     float q = 0.0f;
     if (tid < quads) { const float e = v.x - m_w, f = v.y - m_w, h = v.z - m_w, k = v.w - m_w; q = (e * e + f * f) + (h * h + k * k); }
     q = warp_sum(q);
@@ -101,13 +104,21 @@ __global__ void __launch_bounds__(T, 1) head_row_kernel(const HeadArgs a) {
     float mean = 0.0f, m2 = 0.0f;
 #pragma unroll
     for (int i = 0; i < W; ++i) mean += count(i) * red[0][i];
-    mean /= (float)K;
+    mean = RMS ? 0.0f : mean / (float)K;
 #pragma unroll
     for (int i = 0; i < W; ++i) { const float dm = red[0][i] - mean; m2 += fmaf(count(i) * dm, dm, red[1][i]); }
-    const float sd = sqrtf(m2 / (float)K + 1e-5f);
-    if (tid < quads)
-        add[tid] = make_float4(((v.x - mean) / sd) * g.x + b.x, ((v.y - mean) / sd) * g.y + b.y, ((v.z - mean) / sd) * g.z + b.z,
-                               ((v.w - mean) / sd) * g.w + b.w);
+    const float sd = sqrtf(m2 / (float)K + a.eps);
+    if (tid < quads) {
+        if (RMS) {
+            const float inv = 1.0f / sd;
+            v = make_float4(__fmul_rn(__fmul_rn(v.x, inv), g.x), __fmul_rn(__fmul_rn(v.y, inv), g.y), __fmul_rn(__fmul_rn(v.z, inv), g.z),
+                            __fmul_rn(__fmul_rn(v.w, inv), g.w));
+        } else {
+            v = make_float4(((v.x - mean) / sd) * g.x + b.x, ((v.y - mean) / sd) * g.y + b.y, ((v.z - mean) / sd) * g.z + b.z, ((v.w - mean) / sd) * g.w + b.w);
+        }
+        if (!SCALED) { v.x *= xs.x; v.y *= xs.y; v.z *= xs.z; v.w *= xs.w; }
+        add[tid] = v;
+    }
     __syncthreads();
     uint64_t x[NU][4];
 #pragma unroll
@@ -131,7 +142,8 @@ __global__ void __launch_bounds__(T, 1) head_row_kernel(const HeadArgs a) {
                 fma_pair<2>(acc, r.q[i][u].x, x[u][1]);
                 fma_pair<0>(acc, r.q[i][u].y, x[u][2]);
                 fma_pair<2>(acc, r.q[i][u].y, x[u][3]);
-                s[i] = fmaf(__half2float(r.d[i][u]), __uint_as_float((uint32_t)acc) + __uint_as_float((uint32_t)(acc >> 32)), s[i]);
+                const float t = __uint_as_float((uint32_t)acc) + __uint_as_float((uint32_t)(acc >> 32));
+                s[i] = SCALED ? fmaf(__half2float(r.d[i][u]), t, s[i]) : s[i] + t;
             }
         }
         // one value a lane: lanes below 16 end up with row 0, the others with row 1
@@ -155,6 +167,7 @@ __global__ void __launch_bounds__(T, 1) head_row_kernel(const HeadArgs a) {
                 fetch(w[i], k + DEPTH * step);
             }
         }
+    if (!a.stats) return;
     // the two lanes of a warp that finish rows, then the warps
     const float other = __shfl_xor_sync(0xffffffffu, top, 16), m = fmaxf(top, other);
     mass = mass == 0.0f ? 0.0f : mass * expf(top - m);
@@ -174,25 +187,31 @@ __global__ void __launch_bounds__(T, 1) head_row_kernel(const HeadArgs a) {
 
 }  // namespace
 
-int launch_head_row(const QMat& w, const BlockRow& r, float* logits, float2* stats, int* n_stats, const StepState* state, cudaStream_t st) {
-    if (r.d != w.K || w.K % 128 || w.K > 1024 || r.n_part > MAX_PARTS || !w.d) return fail(FC_E_SHAPE, "head row: K = %d, %d rows to add", w.K, r.n_part);
+int launch_head_row(const StepMat& w, int N, const BlockRow& r, float* logits, float2* stats, int* n_stats, const StepState* state, cudaStream_t st) {
+    const int K = r.d;
+    if (K % 128 || K > 1024 || r.n_part > MAX_PARTS || (!w.d && (!w.xscale || r.b))) return fail(FC_E_SHAPE, "head row: K = %d, %d rows to add", K, r.n_part);
     static int sms[64] = {};
     int dev = 0;
     FC_CUDA(cudaGetDevice(&dev));
     if (dev >= 64) return fail(FC_E_ARG, "device index %d", dev);
     if (!sms[dev]) FC_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
-    const HeadArgs a = {w.qu, w.d, w.N, w.K, r.x, r.part, r.bias, r.g, r.b, r.n_part, logits, stats, state};
-    const int blocks = std::min(sms[dev], ((w.N + RB - 1) / RB + W - 1) / W);
-    *n_stats = blocks;
-    const size_t smem = (size_t)(r.n_part + 1) * w.K * 4;
+    const HeadArgs a = {w.qu, w.d, N, K, r.x, r.part, r.bias, r.g, r.b, w.xscale, r.n_part, r.eps, logits, stats, state};
+    const int blocks = std::min(sms[dev], ((N + RB - 1) / RB + W - 1) / W);
+    if (n_stats) *n_stats = blocks;
+    const size_t smem = (size_t)(r.n_part + 1) * K * 4;
     auto go = [&](auto kernel) -> int {
         FC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (MAX_PARTS + 1) * 1024 * 4));
         FC_CUDA(launch_pdl(kernel, dim3(blocks), dim3(T), smem, st, a));
         ++g_launches;
         return FC_OK;
     };
-    const int nu = (w.K + 255) / 256;
-    return nu == 1 ? go(head_row_kernel<1>) : nu == 2 ? go(head_row_kernel<2>) : nu == 3 ? go(head_row_kernel<3>) : go(head_row_kernel<4>);
+    const int nu = (K + 255) / 256;
+    auto of = [&](auto rms, auto scaled) {
+        constexpr bool R = decltype(rms)::value, S = decltype(scaled)::value;
+        return nu == 1 ? go(head_row_kernel<1, R, S>) : nu == 2 ? go(head_row_kernel<2, R, S>) : nu == 3 ? go(head_row_kernel<3, R, S>) : go(head_row_kernel<4, R, S>);
+    };
+    if (r.b) return of(std::false_type(), std::true_type());
+    return w.d ? of(std::true_type(), std::true_type()) : of(std::true_type(), std::false_type());
 }
 
 }  // namespace fc

@@ -7,6 +7,8 @@
 #include <vector>
 
 #include "llama_native.h"
+#include <climits>
+
 #include "llama_ops.cuh"
 
 using namespace fc;
@@ -73,6 +75,9 @@ struct fc_llama_cache {
     cudaGraphExec_t graph[2][3] = {};
     int graph_nodes[2][3] = {};
     int attn_split = 1, split_from = 0;     // CTAs that share a head from position split_from on
+    float* parts = nullptr;                 // block_step.cu: what the halves leave to add, and two rows; null: shapes it does not cover
+    long long graph_wait = 0;               // the wait budget and the test hook the graphs were captured with
+    int graph_withhold = 0;
     bool packed_warm[2] = {false, false};   // packed model: the uncaptured first step of each kind has run
     unsigned long long* rng_d = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -364,7 +369,73 @@ int launch_attention(fc_llama_cache* s, float* kc, float* vc, int split) {
 // LlamaModel::forward_one (llm.rs:610-618) -> LlamaBlock::forward_one (llm.rs:451-461) as a
 // kernel sequence; every per-step quantity is read from device state so the captured graph is
 // replayed unchanged.
+// A block's matrices for block_step.cu; false where one of them has another form.
+bool step_mats(const fc_llama* m, int l, StepMat (&qkv)[3], StepMat* wo, StepMat (&gu)[2], StepMat* down) {
+    const LlamaLayerDev& L = m->layers[l];
+    const float* b = L.qkv_b;
+    const int at[3] = {0, m->q_dim, m->q_dim + m->kv_dim};
+    if (m->prec < 0) {
+        auto rows = [](const QMat& q, int row, int stride, const float* bias) {
+            return StepMat{q.qu + (size_t)row * q.K, q.d + (size_t)row * (q.K / 32), nullptr, bias, stride};
+        };
+        for (int i = 0; i < 3; ++i) qkv[i] = rows(L.qkv, at[i], 1, b ? b + at[i] : nullptr);
+        for (int i = 0; i < 2; ++i) gu[i] = rows(L.gateup, i, 2, nullptr);
+        *wo = rows(L.wo, 0, 1, nullptr);
+        *down = rows(L.down, 0, 1, nullptr);
+        return true;
+    }
+    const fc_llama::PackedLayer& P = m->packed[l];
+    auto mat = [](const fc_llama::Lin& w, const float* bias, StepMat* out) {
+        GemvPart part;
+        if (!w.rq || !rowq_part(w.rq, nullptr, nullptr, &part)) return false;
+        *out = StepMat{part.qu, nullptr, part.xscale, bias, 1};
+        return true;
+    };
+    return mat(P.wq, b, &qkv[0]) && mat(P.wk, b ? b + at[1] : nullptr, &qkv[1]) && mat(P.wv, b ? b + at[2] : nullptr, &qkv[2]) &&
+           mat(P.wo, nullptr, wo) && mat(P.gate, nullptr, &gu[0]) && mat(P.up, nullptr, &gu[1]) && mat(P.down, nullptr, down);
+}
+// The step in two launches a block.
+int launch_step_halves(fc_llama_cache* s, int with_head) {
+    fc_llama* m = s->m;
+    const fc_llama_config& c = m->cfg;
+    cudaStream_t st = m->st;
+    const int d = c.d_model, slices = block_step_slices(c.d_ff, true);
+    const size_t layer_stride = (size_t)c.ctx * m->kv_dim;
+    float *parts_a = s->parts, *parts_m = parts_a + (size_t)c.n_head * d, *row_a = parts_m + (size_t)slices * d, *row_m = row_a + d;
+    const StepRope rope = {c.rope_dim / 2, c.rope_type == FC_ROPE_NEOX, m->ftab, m->inv_linear};
+    FC_TRY(launch_llama_embed_step(m->tok, c.ctx, s->queue, s->state, s->x, st));
+    BlockRow r = {s->x, nullptr, nullptr, nullptr, nullptr, nullptr, 0, d, c.norm_eps};
+    for (int l = 0; l < c.n_layer; ++l) {
+        StepMat qkv[3], gu[2], wo, down;
+        if (!step_mats(m, l, qkv, &wo, gu, &down)) return fail(FC_E_SHAPE, "block %d is not covered", l);
+        r.g = m->layers[l].attn_norm;
+        r.x_out = l ? row_a : nullptr;                       // the first row is whole as it is
+        FC_TRY(launch_attn_half(r, c.n_head, c.n_kv_head, rope, qkv, wo, s->kc + l * layer_stride, s->vc + l * layer_stride, c.ctx, parts_a, s->state, nullptr, st));
+        r = {l ? row_a : s->x, parts_a, nullptr, row_m, m->layers[l].ffn_norm, nullptr, c.n_head, d, c.norm_eps};
+        FC_TRY(launch_mlp_half(r, gu, down, c.d_ff, parts_m, s->state, nullptr, st));
+        r = {row_m, parts_m, nullptr, nullptr, m->out_norm, nullptr, slices, d, c.norm_eps};
+    }
+    if (with_head) {
+        StepMat head = {m->head.qu, m->head.d, nullptr, nullptr, 1};
+        GemvPart part;
+        if (m->prec >= 0 && m->packed_head.rq && rowq_part(m->packed_head.rq, nullptr, nullptr, &part)) head = {part.qu, nullptr, part.xscale, nullptr, 1};
+        FC_TRY(launch_head_row(head, c.vocab, r, s->logits, nullptr, nullptr, s->state, st));
+    }
+    return launch_step_advance_pdl(s->state, st);
+}
+// Whether it takes every matrix of the model.
+bool halves_cover(const fc_llama* m) {
+    const fc_llama_config& c = m->cfg;
+    if (m->native_tok || m->prec == fc_llama::kNative || c.head_dim != 64 || !block_step_covers(c.d_model, c.n_head, c.d_ff, c.ctx, true)) return false;
+    StepMat qkv[3], gu[2], wo, down;
+    for (int l = 0; l < c.n_layer; ++l)
+        if (!step_mats(m, l, qkv, &wo, gu, &down)) return false;
+    GemvPart part;
+    return m->prec < 0 || (m->packed_head.rq && rowq_part(m->packed_head.rq, nullptr, nullptr, &part));
+}
+
 int launch_step(fc_llama_cache* s, int with_head, int split) {
+    if (s->parts) return launch_step_halves(s, with_head);
     fc_llama* m = s->m;
     const fc_llama_config& c = m->cfg;
     cudaStream_t st = m->st;
@@ -389,6 +460,7 @@ int launch_step(fc_llama_cache* s, int with_head, int split) {
 // The same step on the packed model, one kernel per operation. The first step of a cache runs uncaptured, so that the
 // packed linears' single-row scratch exists before the step is captured.
 int launch_step_packed(fc_llama_cache* s, int with_head, int split) {
+    if (s->parts) return launch_step_halves(s, with_head);
     fc_llama* m = s->m;
     const fc_llama_config& c = m->cfg;
     cudaStream_t st = m->st;
@@ -433,9 +505,23 @@ int launch_step_packed(fc_llama_cache* s, int with_head, int split) {
 // Greedy tokens that need nothing from the host share a graph: between two graphs the GPU waits for the next one's launch.
 constexpr int kFreeSteps = 8;
 
+void drop_graphs(fc_llama_cache* s) {
+    for (auto& form : s->graph)
+        for (cudaGraphExec_t& g : form) {
+            if (g) cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+}
+
 // pos: the position of the (first) step
 int run_graph(fc_llama_cache* s, int which, int pos) {
     const bool shared = pos + (which == 2 ? kFreeSteps : 1) > s->split_from;
+    if (s->graph_wait != g_debug.wait_cycles || s->graph_withhold != g_debug.withhold) {
+        FC_CUDA(cudaStreamSynchronize(s->m->st));
+        drop_graphs(s);
+        s->graph_wait = g_debug.wait_cycles;
+        s->graph_withhold = g_debug.withhold;
+    }
     cudaGraphExec_t& graph = s->graph[shared][which];
     int& nodes = s->graph_nodes[shared][which];
     if (!graph) {
@@ -818,6 +904,10 @@ int fc_llama_cache_create(fc_llama* m, fc_llama_cache** out) {
         FC_TRY(a.alloc_n(&s->queue, (size_t)s->queue_cap));
         FC_TRY(a.alloc_n(&s->state, 1));
         FC_TRY(attn_step_split(c.n_head, c.head_dim, c.ctx, &s->attn_split, &s->split_from));
+        if (halves_cover(m)) {
+            FC_TRY(a.alloc_n(&s->parts, (size_t)(c.n_head + block_step_slices(c.d_ff, true) + 2) * c.d_model));
+            s->split_from = INT_MAX;
+        }
         FC_TRY(a.alloc_n(&s->rng_d, 1));
         FC_CUDA(cudaEventCreate(&s->ev0));
         FC_CUDA(cudaEventCreate(&s->ev1));
@@ -833,8 +923,7 @@ void fc_llama_cache_free(fc_llama_cache* s) {
     if (!s) return;
     cudaSetDevice(s->device);
     cudaDeviceSynchronize();              // the model (and its stream) may already be gone
-    for (auto& form : s->graph)
-        for (cudaGraphExec_t g : form) if (g) cudaGraphExecDestroy(g);
+    drop_graphs(s);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     s->arena.release();

@@ -4,6 +4,7 @@ import pytest
 
 import ferrum_cpu_b200 as fcb
 from ferrum_cpu_b200 import _lib, synth
+from ferrum_cpu_b200.llama import CudaLlama
 from tests import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -59,3 +60,37 @@ def test_a_wait_that_runs_out_feeds_nothing():
     assert np.abs(gm.feed(7) - om.feed(7)).max() < 2e-5
     gm.close()
     om.close()
+
+
+# both pairings of the rotation with and without a tail that is not rotated, grouped heads, weights as stored and on rows of levels,
+# and caches longer than a CTA of a head holds
+@pytest.mark.parametrize("d,heads,kv,ff,ctx,rope_dim,rope_type,prec", [(512, 8, 2, 2048, 40, 64, 0, None), (512, 8, 8, 1024, 33, 48, 1, 0),
+                                                                       (640, 10, 1, 1280, 50, 64, 1, 1), (768, 12, 4, 3072, 40, 64, 0, 0),
+                                                                       (1024, 16, 4, 3072, 24, 64, 0, None)])
+def test_llama_steps(d, heads, kv, ff, ctx, rope_dim, rope_type, prec):
+    sm = synth.SynthLlama(515, d, 2, heads, kv, 64, ff, ctx, seed=d + kv, perturb=True, rope_dim=rope_dim, rope_type=rope_type)
+    om, gm = O.OracleLlama(sm, threads=4, **({} if prec is None else {"prec": prec})), CudaLlama.from_synth(sm, prec=prec)
+    cache = gm.new_cache()
+    om.clear()
+    for t, tok in enumerate(synth.token_ids(2, ctx, 515)):
+        if t == 1:
+            fcb.take_launch_count()
+        got, want = gm.forward_one(tok, cache), om.forward_one(tok)
+        assert np.abs(got - want).max() < 2e-4 * max(1.0, float(np.abs(want).max())), t
+        if t == 1:
+            assert fcb.take_launch_count() <= 8             # embedding, two a block, head, advance, state
+    gm.close()
+
+
+def test_llama_steps_past_the_held_rows():
+    sm = synth.SynthLlama(515, 512, 1, 8, 2, 64, 512, 1400, seed=9, perturb=True, rope_dim=64, rope_type=0)
+    om, gm = O.OracleLlama(sm, threads=4), CudaLlama.from_synth(sm)
+    ids = synth.token_ids(2, 1300, 515)
+    cache = gm.new_cache()
+    om.clear()
+    for t, tok in enumerate(ids):
+        want = om.forward_one(tok)
+        got = gm.forward_one(tok, cache)
+        if t % 97 == 0 or t > 1290:
+            assert np.abs(got - want).max() < 2e-4, t
+    gm.close()
