@@ -89,7 +89,7 @@ int upload_q8(Arena& ar, const void* host, int N, int K, QMat* out, cudaStream_t
 // A block's matrices as f16 planes and the scales of the activation planes that meet them (gemm_f16.cu).
 struct LayerF16 {
     F16Mat qkv, out, up, down;
-    float n1 = 0.0f, att = 0.0f, n2 = 0.0f, hid = 0.0f;
+    float n1 = 0.0f, heads = 0.0f, att = 0.0f, n2 = 0.0f, hid = 0.0f;
 };
 struct LayerDev {
     QMat qkv, out, up, down;
@@ -476,7 +476,7 @@ static int build_f16(fc_model* m, const fc_weights* w) {
     }
     if (!ok) return FC_OK;
     void* mem = nullptr;
-    const size_t tops_at = weights * 4, tops_bytes = (size_t)c.n_layer * 2 * sizeof(unsigned);
+    const size_t tops_at = weights * 4, tops_bytes = (size_t)c.n_layer * 3 * sizeof(unsigned);
     const cudaError_t e = cudaMalloc(&mem, tops_at + tops_bytes);
     if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); return FC_OK; }
     FC_CUDA(e);
@@ -493,12 +493,13 @@ static int build_f16(fc_model* m, const fc_weights* w) {
     FC_TRY(make(m->head, &m->head_f16, 0, nullptr));
     for (int l = 0; l < c.n_layer; ++l) {
         LayerDev& L = m->layers[l];
-        FC_TRY(make(L.qkv, &L.f16.qkv, 2 * d, tops_d + 2 * l));     // the value rows
+        FC_TRY(make(L.qkv, &L.f16.qkv, 0, tops_d + 3 * l));
+        FC_TRY(launch_f16_planes(nullptr, 0, 4, Planes(), nullptr, L.qkv, L.f16.qkv, 2 * d, tops_d + 3 * l + 1, m->st));   // the value rows alone
         FC_TRY(make(L.out, &L.f16.out, 0, nullptr));
-        FC_TRY(make(L.up, &L.f16.up, 0, tops_d + 2 * l + 1));
+        FC_TRY(make(L.up, &L.f16.up, 0, tops_d + 3 * l + 2));
         FC_TRY(make(L.down, &L.f16.down, 0, nullptr));
     }
-    std::vector<float> tops((size_t)c.n_layer * 2);
+    std::vector<float> tops((size_t)c.n_layer * 3);
     FC_CUDA(cudaMemcpyAsync(tops.data(), tops_d, tops_bytes, cudaMemcpyDeviceToHost, m->st));
     FC_CUDA(cudaStreamSynchronize(m->st));
     auto most = [](const float* v, size_t n) { double t = 0; for (size_t i = 0; i < n; ++i) t = v[i] != v[i] ? INFINITY : std::max(t, std::fabs((double)v[i])); return t; };
@@ -514,8 +515,9 @@ static int build_f16(fc_model* m, const fc_weights* w) {
         LayerF16& f = m->layers[l].f16;
         f.n1 = scale(root * most(s.ln1_g, d) + most(s.ln1_b, d));
         f.n2 = scale(root * most(s.ln2_g, d) + most(s.ln2_b, d));
-        f.att = scale(std::sqrt((double)tops[2 * l]) * (root * most(s.ln1_g, d) + norm(s.ln1_b, d)) + most(s.attn_qkv_b + 2 * d, d));
-        f.hid = scale(std::sqrt((double)tops[2 * l + 1]) * (root * most(s.ln2_g, d) + norm(s.ln2_b, d)) + most(s.ffn_up_b, F));
+        f.heads = scale(std::sqrt((double)tops[3 * l]) * (root * most(s.ln1_g, d) + norm(s.ln1_b, d)) + most(s.attn_qkv_b, 3 * (size_t)d));
+        f.att = scale(std::sqrt((double)tops[3 * l + 1]) * (root * most(s.ln1_g, d) + norm(s.ln1_b, d)) + most(s.attn_qkv_b + 2 * d, d));
+        f.hid = scale(std::sqrt((double)tops[3 * l + 2]) * (root * most(s.ln2_g, d) + norm(s.ln2_b, d)) + most(s.ffn_up_b, F));
     }
     m->lnf_scale = scale(root * most(w->out_norm_g, d) + most(w->out_norm_b, d));
     m->f16 = ok;
@@ -572,6 +574,9 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
     // f16 planes, unless a few rows are better off where K is split over CTAs (prompts of 64 / 101 / 250 ids, 12 x 768: 1014 / 1033 / 1120 us
     // on them, 932 / 1207 / 1469 split; 24 x 1024: 2273 / 2315 / 2506 and 2235 / 2449 / 3123)
     const bool f16 = m->f16 && (planes == 2 || d >= kExactF16) && (!split_k || R > 64);
+    // the attention of the f32 mode keeps three bf16 planes: two of f16 take 9 % off a batch of mixed requests, but its log-probabilities are up to
+    // 16 % further from 64 bits then (those of the two-plane mode half as far as with bf16: 8.5e-8 for 1.6e-7)
+    const bool f16_heads = f16 && planes == 2;
     m->pqkv.n = planes;
     m->pn.n = m->patt.n = m->phid.n = f16 ? 2 : planes;
     m->pn.lift = m->patt.lift = f16_lift(d, planes == 3);
@@ -592,6 +597,7 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
     for (int l = 0; l < c.n_layer; ++l) {
         const LayerDev& L = m->layers[l];
         m->pn.scale = f16 ? L.f16.n1 : 0.0f;
+        m->pqkv.scale = f16_heads ? L.f16.heads : 0.0f;
         m->patt.scale = f16 ? L.f16.att : 0.0f;
         m->phid.scale = f16 ? L.f16.hid : 0.0f;
         FC_TRY(launch_layernorm_planes(m->x, L.ln1g, L.ln1b, nullptr, R, d, m->pn, st));
@@ -600,7 +606,7 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
         } else {
             FC_TRY(product(L.qkv, L.f16.qkv, m->pn, L.qkv_b, nullptr, EPI_NONE, m->qkv, nullptr));
             FC_TRY(on_qkv(l));
-            if (tc_attn) FC_TRY(launch_split_planes(m->qkv, m->pqkv, (size_t)R * 3 * d, st));
+            if (tc_attn) FC_TRY(f16_heads ? launch_split_f16(m->qkv, m->pqkv, (size_t)R * 3 * d, st) : launch_split_planes(m->qkv, m->pqkv, (size_t)R * 3 * d, st));
         }
         if (tc_attn) {
             FC_TRY(launch_attn_prefill_tc(m->pqkv, win, R, d, c.n_head, m->patt, status, st));

@@ -6,7 +6,8 @@
 // transformer.rs:458-478) is never formed: keys are visited in tiles of 64 with an online
 // softmax. Both products run on bf16 planes with fp32 accumulation: with two planes as three products (q1·k1 + q1·k2 +
 // q2·k1; the same for P·V, so they reproduce f32 products to 2^-16 relative), with three planes (the f32 math mode) as six
-// (all of order up to 2^-16; what is dropped is 2^-24 of a product).
+// (all of order up to 2^-16; what is dropped is 2^-24 of a product). Two f16 planes of a scale times the values (gemm_f16.cu) take the
+// same three products as two of bf16 and hold 2^-23.
 //
 // Inputs are the bf16 planes of the fused qkv rows [R][3d] written by the QKV GEMM; the output are the planes [R][d] the
 // out-projection GEMM reads. Windows of a batch may differ in length: they lie one after the other without padding.
@@ -43,9 +44,10 @@ struct Smem {
 constexpr int SOFTMAX_WARPS = 4, TMA_WARP = 4, MMA_WARP = 5, THREADS = 6 * 32;
 constexpr int TMEM_COLS = 128;         // score tile: columns 0..63, P·V tile: columns 64..127
 constexpr long long WAIT_CYCLES = 4000000000LL;
-// bf16 x bf16 -> f32, M = 128, N = 64; B K-major for Q·Kᵀ, MN-major (bit 16) for P·V
-constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KT >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
-constexpr uint32_t IDESC_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
+// f32 sums, M = 128, N = 64; B K-major for Q·Kᵀ, MN-major (bit 16) for P·V
+constexpr uint32_t BF16 = (1u << 7) | (1u << 10);        // operand types; without: f16
+constexpr uint32_t IDESC_S = (1u << 4) | ((uint32_t)(KT >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
+constexpr uint32_t IDESC_O = (1u << 4) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
 
 struct Bars {
     unsigned long long q_full, k_full, v_full, k_empty, v_empty;
@@ -141,6 +143,7 @@ struct AttnArgs {
     int group;                   // query heads per key / value head (1: multi-head attention)
     int ldo;                     // row stride of the output planes (= query heads x 64)
     uint16_t* out[3];            // [R][ldo] bf16 planes, or
+    float unscale;               // f16 planes: 1 / their scale
     float out_scale, out_lift;   // not 0: two f16 planes of out_scale (1 + out_lift) times the output
     int* status;
 };
@@ -149,7 +152,8 @@ struct AttnArgs {
 
 struct AttnMaps { CUtensorMap q[3], kv[3]; };    // per plane: boxes of 128 query rows, of 64 key rows
 
-template <int P>
+// F16: two f16 planes of a scale times the values, else bf16 planes.
+template <int P, bool F16>
 __global__ void __launch_bounds__(THREADS, P == 2 ? 2 : 1)
 attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) {
     constexpr int OFF_Q = Smem<P>::Q, OFF_K = Smem<P>::K, OFF_V = Smem<P>::V, OFF_P = Smem<P>::PR, OFF_BARS = Smem<P>::BARS;
@@ -220,7 +224,7 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
                 each_term<P>([&](int i, int j, bool first) {
 #pragma unroll
                     for (int ks = 0; ks < HD / 16; ++ks)                        // 32 bytes along hd per step
-                        umma(tmem, dq + i * QS + ks * 2, dk + j * KS + ks * 2, IDESC_S, !(first && ks == 0));
+                        umma(tmem, dq + i * QS + ks * 2, dk + j * KS + ks * 2, IDESC_S | (F16 ? 0u : BF16), !(first && ks == 0));
                 });
                 umma_commit(&bars->s_full);
                 umma_commit(&bars->k_empty);
@@ -243,7 +247,7 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
                 each_term<P>([&](int i, int j, bool first) {
 #pragma unroll
                     for (int ks = 0; ks < KT / 16; ++ks)                        // 32 bytes along the keys of a P row, 16 key rows of 128 bytes of V
-                        umma(tmem + HD, dp + i * PS + ks * 2, dv + j * KS + ks * 128, IDESC_O, !(first && ks == 0));
+                        umma(tmem + HD, dp + i * PS + ks * 2, dv + j * KS + ks * 128, IDESC_O | (F16 ? 0u : BF16), !(first && ks == 0));
                 });
                 umma_commit(&bars->o_full);
                 umma_commit(&bars->v_empty);
@@ -253,7 +257,9 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
         // ------------------------------------------------------------------ softmax warps
         const int r = warp * 32 + lane;               // query row inside the tile
         const int qi = q0 + r;                        // query index inside the window
-        const float c2 = 0.125f * 1.4426950408889634f;   // 1 / sqrt(64) times log2(e)
+        const float c2 = 0.125f * 1.4426950408889634f * (F16 ? a.unscale * a.unscale : 1.0f);   // 1 / sqrt(64) times log2(e)
+        // f16 planes of 2^12 times the probabilities (the mass with them), so that the second plane of a small one is not lost
+        constexpr float LIFT = F16 ? 12.0f : 0.0f;
         float o[HD];
 #pragma unroll
         for (int c = 0; c < HD; ++c) o[c] = 0.0f;
@@ -285,7 +291,7 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
             }
             const float mn = fmaxf(m, tmax);          // finite from the first tile on (key 0 <= every query)
             const float corr = exp2f((m - mn) * c2);
-            const float off2 = -mn * c2;
+            const float off2 = LIFT - mn * c2;
             float psum = 0.0f;
 #pragma unroll
             for (int c = 0; c < KT / 8; ++c) {        // 16-byte chunk c of the P row: 8 keys
@@ -294,7 +300,10 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
                 for (int e = 0; e < 8; ++e) { p[e] = ex2_approx(fmaf(sv[8 * c + e], c2, off2)); psum += p[e]; }
                 uint32_t w[4][P];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) split2<P>(p[2 * e], p[2 * e + 1], w[e]);
+                for (int e = 0; e < 4; ++e) {
+                    if constexpr (F16) split2_f16(p[2 * e], p[2 * e + 1], 0.0f, w[e]);
+                    else split2<P>(p[2 * e], p[2 * e + 1], w[e]);
+                }
 #pragma unroll
                 for (int t = 0; t < P; ++t)        // 128-byte swizzle
                     *(uint4*)(prow + t * P_BYTES + (c ^ (r & 7)) * 16) = make_uint4(w[0][t], w[1][t], w[2][t], w[3][t]);
@@ -321,7 +330,7 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
             for (int c = 0; c < 32; ++c) { o[c] += __uint_as_float(s0[c]); o[32 + c] += __uint_as_float(s1[c]); }
         }
         if (ok && qi < T) {
-            const float inv = 1.0f / l;
+            const float inv = F16 ? a.unscale / l : 1.0f / l;
             const size_t off = (size_t)(row0 + qi) * a.ldo + (size_t)h * HD;
 #pragma unroll
             for (int c = 0; c < HD / 8; ++c) {
@@ -357,7 +366,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 // A [rows][cols] bf16 plane viewed through boxes of 64 columns x box_rows rows, 128-byte swizzle.
-int encode(CUtensorMap* map, const void* plane, size_t rows, size_t cols, int box_rows) {
+int encode(CUtensorMap* map, const void* plane, size_t rows, size_t cols, int box_rows, bool f16) {
     static EncodeTiledFn fn = nullptr;
     if (!fn) {
         void* p = nullptr;
@@ -370,7 +379,7 @@ int encode(CUtensorMap* map, const void* plane, size_t rows, size_t cols, int bo
     const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
     const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)plane, dims, strides, box, estr,
+    const CUresult r = fn(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)plane, dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(FC_E_CUDA, "cuTensorMapEncodeTiled failed (%d) for a [%zu][%zu] bf16 plane", (int)r, rows, cols);
@@ -380,35 +389,37 @@ int encode(CUtensorMap* map, const void* plane, size_t rows, size_t cols, int bo
 
 // qkv: bf16 planes [R][H*64 + 2*KV*64] (q heads | k heads | v heads per row); out: planes [R][H*64]. Query head h reads key /
 // value head h / (H / KV).
-template <int P>
+template <int P, bool F16>
 static int launch_attn_tc(const Planes& qkv, const Windows& w, int R, int H, int KV, const Planes& out, int* status, cudaStream_t st) {
     if (KV <= 0 || H % KV) return fail(FC_E_DIM, "n_heads %d must be a multiple of n_kv_heads %d", H, KV);
     static bool attr_set[64] = {};
     int dev = 0;
     FC_CUDA(cudaGetDevice(&dev));
     if (dev < 64 && !attr_set[dev]) {
-        FC_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES<P>));
+        FC_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<P, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES<P>));
         attr_set[dev] = true;
     }
     const size_t ld = (size_t)(H + 2 * KV) * HD;
     AttnMaps maps;
     AttnArgs a;
     for (int p = 0; p < P; ++p) {
-        FC_TRY(encode(&maps.q[p], qkv.p[p], R, ld, QT));
-        FC_TRY(encode(&maps.kv[p], qkv.p[p], R, ld, KT));
+        FC_TRY(encode(&maps.q[p], qkv.p[p], R, ld, QT, F16));
+        FC_TRY(encode(&maps.kv[p], qkv.p[p], R, ld, KT, F16));
         a.out[p] = p < out.n ? (uint16_t*)out.p[p] : nullptr;
     }
     a.win = w; a.k_col = H * HD; a.v_col = (H + KV) * HD; a.group = H / KV; a.ldo = H * HD;
+    a.unscale = F16 ? 1.0f / qkv.scale : 1.0f;
     a.out_scale = out.scale; a.out_lift = out.lift;
     a.status = status;
     dim3 grid((w.T + QT - 1) / QT, H, w.B);
-    FC_CUDA(launch_pdl(attn_prefill_tc_kernel<P>, grid, dim3(THREADS), SMEM_BYTES<P>, st, maps, a));
+    FC_CUDA(launch_pdl(attn_prefill_tc_kernel<P, F16>, grid, dim3(THREADS), SMEM_BYTES<P>, st, maps, a));
     FC_LAUNCHED();
     return FC_OK;
 }
 
 int launch_attn_prefill_tc_gqa(const Planes& qkv, const Windows& w, int R, int H, int KV, const Planes& out, int* status, cudaStream_t st) {
-    return qkv.n == 3 ? launch_attn_tc<3>(qkv, w, R, H, KV, out, status, st) : launch_attn_tc<2>(qkv, w, R, H, KV, out, status, st);
+    if (qkv.scale != 0.0f) return launch_attn_tc<2, true>(qkv, w, R, H, KV, out, status, st);
+    return qkv.n == 3 ? launch_attn_tc<3, false>(qkv, w, R, H, KV, out, status, st) : launch_attn_tc<2, false>(qkv, w, R, H, KV, out, status, st);
 }
 
 // The multi-head form: planes [R][3d] in, [R][d] out.

@@ -327,7 +327,7 @@ int launch_attn_prefill(const float* qkv, const Windows& w, int d, int H, float*
 // Decode: q [H*hd], caches [ctx][KV*hd]. Window: q, k, v rows ld floats apart, out rows ldo apart.
 int launch_attn_prefill_gqa(const float* q, const float* k, const float* v, const Windows& w, int ld, int H, int KV, int hd,
                             int ldo, float* out, cudaStream_t st);
-// attn_tc.cu — the same on tcgen05 (head_dim 64): bf16 planes (two or three) of qkv [R][3d] in, as many planes of the
+// attn_tc.cu — the same on tcgen05 (head_dim 64): planes (two or three of bf16, two of f16) of qkv [R][3d] in, as many planes of the
 // attention output [R][d] out; `status` is raised on a timeout.
 int launch_attn_prefill_tc(const Planes& qkv, const Windows& w, int R, int d, int H, const Planes& out, int* status, cudaStream_t st);
 // Grouped-query form: planes [R][(H + 2 KV) * 64] in (q heads | k heads | v heads), [R][H * 64] out.

@@ -59,7 +59,7 @@ constexpr int MAX_STAGES = 6;
 constexpr int TMEM_COLS = 512, ACC_COLS = 256;
 constexpr int SMEM_LIMIT = 227 * 1024;
 
-enum Mode : int { OUT_F32 = 0, OUT_BF16 = 1 /* bf16 planes */, OUT_GELU = 2 /* f16 planes, after GELU */, OUT_SCORE = 3 };
+enum Mode : int { OUT_F32 = 0, OUT_PLANES = 1 /* bf16 planes, or f16 planes of a scale */, OUT_GELU = 2 /* f16 planes, after GELU */, OUT_SCORE = 3 };
 
 struct F16Args {
     int N, K, M, stages;
@@ -68,8 +68,8 @@ struct F16Args {
     float inv;                // what takes the scale of x out of a sum (a power of two)
     const float* row_inv;     // the same per activation row, or null
     float* y; int ldy;        // OUT_F32
-    uint16_t* yp[3];          // OUT_BF16 (two planes, or three), OUT_GELU (two): planes, ldy elements apart
-    float out_scale, out_lift;   // OUT_GELU: scale and lift of the planes
+    uint16_t* yp[3];          // OUT_PLANES, OUT_GELU: planes (three only of bf16), ldy elements apart
+    float out_scale, out_lift;   // scale and lift of f16 planes
     const int* targets; float4* stats; float* tlogit;      // OUT_SCORE
     int* status;
     long long wait_cycles;
@@ -356,6 +356,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
                         uint32_t t[2];
                         split2_f16(gelu_f(v0) * a.out_scale, gelu_f(v1) * a.out_scale, a.out_lift, t);
                         w[0] = t[0]; w[1] = t[1];
+                    } else if (a.out_scale != 0.0f) {
+                        uint32_t t[2];
+                        split2_f16(v0 * a.out_scale, v1 * a.out_scale, a.out_lift, t);
+                        w[0] = t[0]; w[1] = t[1]; w[2] = 0;
                     } else if (a.yp[2]) {
                         split2<3>(v0, v1, w);
                     } else {
@@ -369,7 +373,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
                         *(uint32_t*)(a.yp[0] + at) = o0;
                         *(uint32_t*)(a.yp[1] + at) = o1;
                     }
-                    if (MODE == OUT_BF16 && a.yp[2]) {
+                    if (MODE == OUT_PLANES && a.yp[2]) {
                         const uint32_t g2 = __shfl_xor_sync(0xffffffffu, w[2], 1);
                         if (real && 2 * i + odd < left) *(uint32_t*)(a.yp[2] + at) = __byte_perm(w[2], g2, odd ? 0x3276 : 0x5410);
                     }
@@ -587,11 +591,11 @@ int launch_gemm_f16(const F16Mat& w, const Planes& x, const float* row_inv, cons
     a.bias = bias; a.residual = residual; a.gelu = epi == EPI_GELU; a.row_inv = row_inv; a.y = y; a.ldy = ldy; a.status = status;
     if (epi != EPI_NONE && epi != EPI_GELU) return fail(FC_E_ARG, "epilogue %d is not one of this entry's", epi);
     if (y) return launch_f16<OUT_F32>(w, x, a, M, exact, st);
-    if (!yp || (epi == EPI_GELU && yp->n != 2) || (w.N & 31) || (ldy & 7) || residual || row_inv || (epi == EPI_GELU) != (yp->scale != 0.0f))
-        return fail(FC_E_SHAPE, "plane output needs N %% 32 == 0, ldy %% 8 == 0, bf16 planes (behind GELU two f16 planes) and no residual");
+    if (!yp || (epi == EPI_GELU && yp->n != 2) || (w.N & 31) || (ldy & 7) || residual || row_inv || (epi == EPI_GELU && yp->scale == 0.0f) || (yp->scale != 0.0f && yp->n != 2))
+        return fail(FC_E_SHAPE, "plane output needs N %% 32 == 0, ldy %% 8 == 0, bf16 planes or two f16 planes (behind GELU these) and no residual");
     for (int p = 0; p < yp->n; ++p) a.yp[p] = (uint16_t*)yp->p[p];
     a.out_scale = yp->scale; a.out_lift = yp->lift;
-    return epi == EPI_GELU ? launch_f16<OUT_GELU>(w, x, a, M, exact, st) : launch_f16<OUT_BF16>(w, x, a, M, exact, st);
+    return epi == EPI_GELU ? launch_f16<OUT_GELU>(w, x, a, M, exact, st) : launch_f16<OUT_PLANES>(w, x, a, M, exact, st);
 }
 
 int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st, bool exact) {
