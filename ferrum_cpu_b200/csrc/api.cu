@@ -723,9 +723,10 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
     const size_t n = (size_t)M * w->w.K;
     CallScratch scratch;
     Planes x;
-    if (planes == 2 && w->w.f16_exact && f16_rows(w->w.K, M)) {
+    const size_t nw = (size_t)w->w.N * w->w.K;
+    // (no more scratch than the pool keeps: with more, every call would take memory from the driver)
+    if (planes == 2 && w->w.f16_exact && f16_rows(w->w.K, M) && 4 * (n + nw + M) <= kScratchKept) {
         // both operands as f16 planes, and the rows' scales behind them
-        const size_t nw = (size_t)w->w.N * w->w.K;
         FC_TRY(scratch.take(w->device, 4 * (n + nw + M), st));
         if (scratch.p) {
             __half* p = (__half*)scratch.p;

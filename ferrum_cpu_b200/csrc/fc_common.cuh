@@ -67,6 +67,7 @@ struct Arena {
 };
 // scratch.cu — device memory of one call, taken and given back in the order of its stream. take leaves p null when there is no
 // memory; the other failures are errors. A device's pool lives while weights are retained on it.
+constexpr uint64_t kScratchKept = (uint64_t)256 << 20;   // what a device's pool keeps between calls
 int scratch_retain(int device);
 void scratch_release(int device);
 struct CallScratch {

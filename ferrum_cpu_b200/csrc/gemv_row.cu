@@ -21,7 +21,9 @@
 //    `ks` of them share a row;
 //  - few rows take few warps per CTA, spread over all SMs.
 // Bound: issue and latency. In a chain 768 -> 768 takes 1.8 us, 3072 -> 768 2.8, 2048 -> 2048 3.2, 2048 -> 16384 12.5 (2.8 TB/s;
-// 12.4 when the matrix comes from L2), 2048 -> 32000 21; the sum of the launches of a step is what a token costs.
+// 12.4 when the matrix comes from L2), 2048 -> 32000 21; the sum of the launches of a step is what a token costs. (Taken with one level an
+// instruction; packed pairs took 5 % off a step of 16 blocks of 2048, 43.1 -> 40.9 ms for 64 tokens. Asking for a warp's second task ahead
+// of the wait as well: 43.0.)
 // (The kernel this replaced streamed 32 KB tiles through a shared-memory ring with a block barrier per tile: about 5.5 us
 // for every product of a step, however small.)
 #include <algorithm>

@@ -3,7 +3,7 @@
 // A product on a caller's stream returns before its kernels run, so its scratch can belong neither to the weight (two streams
 // would share it) nor to a growing buffer (a capture could not make it). It is taken from a pool per device in the order of
 // the stream and given back in that order: calls that may overlap get memory of their own, a captured call becomes an
-// allocation node of its graph, and what the pool keeps between calls is bounded by kKeptBytes and shared by all weights of
+// allocation node of its graph, and what the pool keeps between calls is bounded by kScratchKept and shared by all weights of
 // the device. The pool never makes one stream wait for another. The last weight of a device returns it whole.
 #include <mutex>
 
@@ -12,7 +12,6 @@
 namespace fc {
 
 namespace {
-constexpr uint64_t kKeptBytes = (uint64_t)256 << 20;
 struct Pool {
     cudaMemPool_t pool = nullptr;
     int weights = 0;
@@ -33,7 +32,7 @@ int scratch_retain(int device) {
         props.location.id = device;
         cudaMemPool_t pool = nullptr;
         FC_CUDA(cudaMemPoolCreate(&pool, &props));
-        uint64_t keep = kKeptBytes;
+        uint64_t keep = kScratchKept;
         int no = 0;
         cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
         if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no);

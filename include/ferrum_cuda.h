@@ -38,8 +38,11 @@ extern "C" {
 
 /* Math modes of the window forward (scoring, primes) and of the linears with M >= 2. Decode steps are
  * f32-equivalent in both. */
-#define FC_MATH_FP32 0      /* tcgen05 kind::f16, activations as three bf16 planes (their f32 value exactly), f32 accumulate */
-#define FC_MATH_BF16X3 1    /* the same with two planes (2^-17 relative) */
+#define FC_MATH_FP32 0      /* tcgen05 kind::f16, f32 accumulate: exact int8 levels against three bf16 planes of the activations (their f32
+                               value exactly), or, in GPT-2 models of width 512 and more, exact f16 planes of the weights against f16 planes of
+                               the activations (2^-23 relative), with sums no further from 64 bits */
+#define FC_MATH_BF16X3 1    /* the same against two bf16 planes (2^-17 relative), or f16 planes with sums kept longer in the tensor core
+                               (about 5e-7 of a product) */
 
 /* Dimensions of a gpt2-architecture GGUF (ferrum_core/src/loader/gpt2.rs:201-215). */
 typedef struct fc_config {
@@ -156,7 +159,8 @@ int fc_q8_0_linear(int device, const float* x, const void* wq, const float* bias
  * Operands are read and written in the stream's order, bias_dev included: it may be what the call ahead
  * on the stream writes. Few rows (K <= 3072 and M <= 4, or M * N * K below 2^25 with K rounded up to 256)
  * run on f32 FMA in both math modes and need no scratch. More are first split into bf16 planes (two in
- * FC_MATH_BF16X3 when K is a multiple of 64, else three: 4 or 6 bytes an element). That scratch belongs
+ * FC_MATH_BF16X3 when K is a multiple of 64, else three: 4 or 6 bytes an element); in FC_MATH_BF16X3 from 512 and K / 2 rows on (up to 256 MiB)
+ * both x and the weight become f16 planes (4 bytes an element of either). That scratch belongs
  * to the call, not to the weight: it is taken from a pool in the order of the stream and given back in
  * the same order, so that a call may be captured into a graph without a call before it (it becomes an
  * allocation node; such a graph cannot be a child node). Between calls the pool keeps 256 MiB at most
@@ -203,7 +207,8 @@ int fc_q8_0_linear_dev_noalloc(const fc_qweight* w, const float* x_dev, const fl
 
 /* ---- model ------------------------------------------------------------------------ */
 /* Validates as loader/gpt2.rs + loader/mod.rs:147-154 (d % n_head == 0, K % 32 == 0),
- * uploads and repacks the weights on `device`. */
+ * uploads and repacks the weights on `device`. Models in FC_MATH_BF16X3, and those of width 512 and more, also keep their
+ * matrices as f16 planes for window forwards (4 bytes a weight), unless there is no memory for them. */
 int fc_model_create(const fc_config* cfg, const fc_weights* w, int device, fc_model** out);
 /* The same from a GGUF file, without the f32 expansion of the matrices (the direct path the
  * reference names as future work, loader/decode.rs:99-100). Reads a gpt2-architecture GGUF
