@@ -720,7 +720,7 @@ def main():
             "gpu_launches": int(launches),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
                          "traffic": None, "peak_kind": peak_kind,
-                         "what": "chain of dependent launches (five per block, eight tokens per graph): %.1f MB algorithmic per token" % (bpt / 1e6)},
+                         "what": "chain of dependent launches (two per block, eight tokens per graph): %.1f MB algorithmic per token" % (bpt / 1e6)},
             "clocks": clocks,
         }
         if args.workload == "both":
