@@ -105,6 +105,24 @@ def test_top_k_draws_at_the_edges_of_the_candidate_list(V, k, levels):
         assert got == want or levels or k > 40
 
 
+@pytest.mark.parametrize("V", [8191, 8192, 8193, 9215, 8 * 1024 + 129, 20001, 51199, 51200])
+def test_top_k_draws_of_rows_that_several_blocks_share(V):
+    """Rows below and above the length from which eight blocks share the passes, with ragged last lines; a penalised window that
+    repeats ids and one too long for shared memory; equal values that overflow the candidate list; a row without mass. k <= 40 values
+    are kept and no sum of so many rounds by more than k ulp, which no draw of these seeds meets: the token is the reference's."""
+    logits = synth.Rng(V).normal(V, 2.5)
+    window = list(synth.token_ids(9, 200, V)) + [0, V - 1, int(np.argmax(logits))] * 3
+    for recent in ((), window, window * 6):
+        for seed in range(1, 7):
+            want, got = _pair(logits, seed, recent=recent, temperature=0.8, top_k=40, top_p=0.95, repetition_penalty=1.1)
+            assert want == got
+    flat = np.zeros(V, np.float32)
+    flat[V // 2:] = -50.0
+    assert _pair(flat, 3, top_k=40)[1] < V // 2               # ties at the cut are all kept
+    want, got = _pair(np.full(V, np.nan, np.float32), 5, top_k=40)
+    assert 0 <= got < V and want == got                       # no mass: the uniform fallback
+
+
 def test_greedy_with_penalty_matches_exactly_on_vocabulary_sized_rows():
     V = 50257
     logp = synth.Rng(6).normal(V, 2.5)
