@@ -286,7 +286,7 @@ static int launch_head(fc_stream* s, const float* x, int mode, const BlockRow* t
     int n_stats = 0;
     if (tail) FC_TRY(launch_head_row(step_mat(m->head), m->head.N, *tail, s->logits, s->stats, &n_stats, s->state, m->st));
     else FC_TRY(launch_gemv_row(m->head, x, RowNorm{m->lnfg, m->lnfb, 1e-5f}, nullptr, nullptr, EPI_NONE, s->logits, s->state, m->st, s->stats, &n_stats));
-    return launch_step_finish(s->logits, m->cfg.vocab, s->stats, n_stats, mode == STEP_PROBS ? s->probs : nullptr, s->queue, s->queue_cap, s->state,
+    return launch_step_finish(s->logits, m->cfg.vocab, s->stats, n_stats, tail ? kHeadSpan : 0, mode == STEP_PROBS ? s->probs : nullptr, s->queue, s->queue_cap, s->state,
                               m->st);
 }
 

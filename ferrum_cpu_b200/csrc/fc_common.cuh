@@ -215,6 +215,8 @@ int launch_mlp_half(const BlockRow& r, const StepMat (&up)[2] /* up, or gate and
                     cudaStream_t st);
 
 // head_row.cu — the product behind those: N logits and, with stats, per CTA the largest and the mass around it (kRowStats entries at most).
+// stats[c], c < *n_stats: over the rows of which (row / kHeadSpan) % *n_stats is c.
+constexpr int kHeadSpan = 32;
 int launch_head_row(const StepMat& w, int N, const BlockRow& r, float* logits, float2* stats, int* n_stats, const StepState* state, cudaStream_t st);
 
 // Windows of rows that share a forward pass: window b holds rows starts[b] .. starts[b + 1] (device array of B + 1), or, with
@@ -288,7 +290,7 @@ int launch_layernorm_planes(const float* x, const float* g, const float* b, cons
 // Decode tail over logits[V]: softmax statistics, optional probs[V], optional greedy select
 // (append to queue) — and always the end-of-step bookkeeping (pos, fed).
 // The tail behind a head product with stats: probabilities (probs set) or the greedy pick, then the step's advance.
-int launch_step_finish(const float* logits, int V, const float2* stats, int n_stats, float* probs_or_null, int* queue, int queue_cap,
+int launch_step_finish(const float* logits, int V, const float2* stats, int n_stats, int span, float* probs_or_null, int* queue, int queue_cap,
                        StepState* state, cudaStream_t st);
 // End-of-step bookkeeping alone (steps that skip the head).
 int launch_step_advance_pdl(StepState* state, cudaStream_t st);

@@ -16,6 +16,7 @@ namespace fc {
 namespace {
 
 constexpr int T = 512, W = T / 32, RB = 2, MAX_PARTS = 16;
+static_assert(RB * W == kHeadSpan, "consecutive rows of a CTA");
 
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) { return (uint64_t)__float_as_uint(hi) << 32 | __float_as_uint(lo); }
 // Levels 2 i and 2 i + 1 of a unit's word against two elements of the row.

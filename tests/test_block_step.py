@@ -34,6 +34,30 @@ def test_tokens_and_probabilities(d, heads, ff, ctx, prompt, new, vocab):
     om.close()
 
 
+# one CTA of the head and as many as the chip has, a last span that is not full, rows that no CTA reaches a second time
+@pytest.mark.parametrize("vocab", [31, 515, 4736, 9501])
+@pytest.mark.parametrize("rows", ["ties", "flat", "nan"])
+def test_pick_reads_the_rows_that_reach_the_largest(vocab, rows):
+    """Equal rows all over the head: the first of them is picked. Rows that all lie within the bound, and rows without mass: the first."""
+    sm = synth.SynthModel(1, 512, 8, 2048, 32, vocab, seed=vocab, perturb=True)
+    table = synth.q8_0_dequantize(sm.token_embd, vocab * 512).reshape(vocab, 512)
+    if rows == "ties":
+        table = table[np.arange(vocab) % 131]
+    elif rows == "flat":
+        table[:] = table[0]
+    else:
+        sm.out_norm_g[:] = np.nan
+    sm.token_embd[:] = synth.q8_0_quantize(table)
+    om, gm = O.OracleModel(sm), fcb.CudaSlm(sm.config, sm.weights)
+    ids = synth.token_ids(4, 3, vocab)
+    want = om.generate_greedy(ids, 12)[0]
+    assert (want < min(vocab, 131) if rows == "ties" else want == 0).all()
+    gm.set_decode_mode(1)                                   # the prompt by the same step, not by the persistent kernel
+    assert np.array_equal(gm.generate_tokens(ids, 12)[0], want)
+    gm.close()
+    om.close()
+
+
 def test_scores_of_minus_infinity_and_huge_rows():
     """A row without a finite logit ends as it does in the step of five launches: no id beyond the vocabulary, no hang."""
     sm = synth.SynthModel(1, 512, 8, 2048, 32, 515, seed=3)
