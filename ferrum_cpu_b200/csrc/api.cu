@@ -458,10 +458,7 @@ static int model_planes(const fc_model* m) {
     const fc_config& c = m->cfg;
     return c.math_mode == FC_MATH_BF16X3 && c.d_model % 64 == 0 && c.d_ff % 64 == 0 ? 2 : 3;
 }
-// Width from which on the f32 mode runs on f16 planes: its sums there are no further from 64 bits than those of the level GEMM.
-constexpr int kExactF16 = 512;
-// The matrices of a model as f16 planes (a two-plane model, or one whose products are long enough), and the scales of the activation planes. A scale is the largest power of two
-// that keeps scale x bound within f16, where the bound holds for every input: a LayerNorm's row has norm at most sqrt(d) max|g| +
+// The matrices of a two-plane model as f16 planes, and the scales of the activation planes. A scale is the largest power of two that keeps scale x bound within f16, where the bound holds for every input: a LayerNorm's row has norm at most sqrt(d) max|g| +
 // |b|, an element of a product at most the norm of its weight row times that (+ bias), a mixture of value rows and GELU at
 // most what goes into them. The 1 % is for rounding. Without memory for the planes (4 bytes a weight), with a matrix that f16
 // cannot hold or a bound that is not a finite number, the model stays on the level GEMM.
@@ -571,18 +568,15 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
     const int d = c.d_model, F = c.d_ff;
     cudaStream_t st = m->st;
     const bool tc_attn = tensor_attention(m);
-    // f16 planes, unless a few rows are better off where K is split over CTAs (prompts of 64 / 101 / 250 ids, 12 x 768: 1014 / 1033 / 1120 us
-    // on them, 932 / 1207 / 1469 split; 24 x 1024: 2273 / 2315 / 2506 and 2235 / 2449 / 3123)
-    const bool f16 = m->f16 && (planes == 2 || d >= kExactF16) && (!split_k || R > 64);
-    // the attention of the f32 mode keeps three bf16 planes: two of f16 take 9 % off a batch of mixed requests, but its log-probabilities are up to
-    // 16 % further from 64 bits then (those of the two-plane mode half as far as with bf16: 8.5e-8 for 1.6e-7)
-    const bool f16_heads = f16 && planes == 2;
-    m->pqkv.n = planes;
-    m->pn.n = m->patt.n = m->phid.n = f16 ? 2 : planes;
-    m->pn.lift = m->patt.lift = f16_lift(d, planes == 3);
-    m->phid.lift = f16_lift(F, planes == 3);
+    // f16 planes in the two-plane mode (never in the f32 mode: two of them are a bit short of an f32), unless a few rows are better off where K is
+    // split over CTAs (prompts of 64 / 101 / 250 ids, 12 x 768: 1014 / 1033 / 1120 us on them, 932 / 1207 / 1469 split; 24 x 1024: 2273 / 2315 /
+    // 2506 and 2235 / 2449 / 3123)
+    const bool f16 = m->f16 && planes == 2 && (!split_k || R > 64);
+    m->pqkv.n = m->pn.n = m->patt.n = m->phid.n = planes;
+    m->pn.lift = m->patt.lift = f16_lift(d);
+    m->phid.lift = f16_lift(F);
     auto product = [&](const QMat& q, const F16Mat& h, const Planes& x, const float* bias, const float* residual, int epi, float* y, const Planes* yp) {
-        return f16 ? launch_gemm_f16(h, x, nullptr, bias, residual, epi, y, yp, R, q.N, status, st, planes == 3)
+        return f16 ? launch_gemm_f16(h, x, nullptr, bias, residual, epi, y, yp, R, q.N, status, st)
                    : launch_gemm_q8_tc(q, x, bias, residual, epi, y, yp, R, q.N, status, st, split_k);
     };
     FC_CUDA(cudaMemsetAsync(m->err_d, 0, sizeof(int), st));
@@ -597,7 +591,7 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
     for (int l = 0; l < c.n_layer; ++l) {
         const LayerDev& L = m->layers[l];
         m->pn.scale = f16 ? L.f16.n1 : 0.0f;
-        m->pqkv.scale = f16_heads ? L.f16.heads : 0.0f;
+        m->pqkv.scale = f16 ? L.f16.heads : 0.0f;
         m->patt.scale = f16 ? L.f16.att : 0.0f;
         m->phid.scale = f16 ? L.f16.hid : 0.0f;
         FC_TRY(launch_layernorm_planes(m->x, L.ln1g, L.ln1b, nullptr, R, d, m->pn, st));
@@ -606,7 +600,7 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
         } else {
             FC_TRY(product(L.qkv, L.f16.qkv, m->pn, L.qkv_b, nullptr, EPI_NONE, m->qkv, nullptr));
             FC_TRY(on_qkv(l));
-            if (tc_attn) FC_TRY(f16_heads ? launch_split_f16(m->qkv, m->pqkv, (size_t)R * 3 * d, st) : launch_split_planes(m->qkv, m->pqkv, (size_t)R * 3 * d, st));
+            if (tc_attn) FC_TRY(f16 ? launch_split_f16(m->qkv, m->pqkv, (size_t)R * 3 * d, st) : launch_split_planes(m->qkv, m->pqkv, (size_t)R * 3 * d, st));
         }
         if (tc_attn) {
             FC_TRY(launch_attn_prefill_tc(m->pqkv, win, R, d, c.n_head, m->patt, status, st));
@@ -640,12 +634,11 @@ static int score_device(fc_model* m, const ScoreSlot& s, const Windows& win, int
     // the head's epilogue keeps (max, sum of exponentials, first argmax) per row and 128-column tile and the
     // target's logit: [rows][V] logits never reach memory (scoring.rs:175-181 needs one number per row)
     if (f16) {
-        m->pn.n = 2;
         m->pn.scale = m->lnf_scale;
-        m->pn.lift = f16_lift(d, model_planes(m) == 3);
+        m->pn.lift = f16_lift(d);
     }
     FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, n == R ? nullptr : pick, n, d, m->pn, m->st));
-    if (f16) FC_TRY(launch_gemm_f16_score(m->head_f16, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st, model_planes(m) == 3));
+    if (f16) FC_TRY(launch_gemm_f16_score(m->head_f16, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
     else FC_TRY(launch_gemm_q8_tc_score(m->head, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
     return launch_score_combine(m->head_stats, m->head_tlogit, targets, n, (c.vocab + 127) / 128, c.vocab, s.lp_d(), s.gr_d(), m->st);
 }
@@ -732,10 +725,10 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
             __half* p = (__half*)scratch.p;
             const F16Mat wp = {p, p + nw, w->w.N, w->w.K};
             p += 2 * nw;
-            x.p[0] = p; x.p[1] = p + n; x.n = 2; x.scale = 1.0f; x.lift = f16_lift(w->w.K, false);
+            x.p[0] = p; x.p[1] = p + n; x.n = 2; x.scale = 1.0f; x.lift = f16_lift(w->w.K);
             float* row_inv = (float*)(p + 2 * n);
             FC_TRY(launch_f16_planes(x_dev, M, w->w.K, x, row_inv, w->w, wp, 0, nullptr, st));
-            return launch_gemm_f16(wp, x, row_inv, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, w->status.dev, st, false);
+            return launch_gemm_f16(wp, x, row_inv, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, w->status.dev, st);
         }
     }
     FC_TRY(take_planes(scratch, x, planes, n, w->device, st));
@@ -802,7 +795,7 @@ static int model_build(fc_model* m, const fc_weights* w) {
         FC_TRY(upload_f32(a, s.ln2_g, d, &L.ln2g, st));
         FC_TRY(upload_f32(a, s.ln2_b, d, &L.ln2b, st));
     }
-    if (model_planes(m) == 2 || (d >= kExactF16 && d % 64 == 0 && F % 64 == 0)) FC_TRY(build_f16(m, w));
+    if (model_planes(m) == 2) FC_TRY(build_f16(m, w));
     if (mega_supported(c)) {
         int full = 0;
         FC_TRY(mega_max_grid(&full));

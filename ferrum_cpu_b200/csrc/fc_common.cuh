@@ -237,8 +237,8 @@ struct Planes {
     float scale = 0.0f, lift = 0.0f;
 };
 // The lift of the f16 planes of a product's activations: the share of themselves that sums over K lose, on average, to the tensor
-// core's truncation (gemm_f16.cu), by the stages of 64 whose sums it keeps (one in the f32 mode, else up to four).
-inline float f16_lift(int K, bool exact) { return exact || K <= 64 ? 8.9e-8f : K <= 128 ? 2.8e-7f : K <= 192 ? 4.7e-7f : 6.7e-7f; }
+// core's truncation (gemm_f16.cu), by the stages of 64 whose sums it keeps (up to four).
+inline float f16_lift(int K) { return K <= 64 ? 8.9e-8f : K <= 128 ? 2.8e-7f : K <= 192 ? 4.7e-7f : 6.7e-7f; }
 // Planes of n elements out of a call's scratch; scratch.p stays null when there is no memory.
 int take_planes(CallScratch& scratch, Planes& x, int planes, size_t n, int device, cudaStream_t st);
 // cols (may be null): column k of rows K wide is multiplied by cols[k] first.
@@ -261,11 +261,10 @@ int launch_score_combine(const void* stats, const float* tlogit, const int* targ
                          uint8_t* is_greedy, cudaStream_t st);
 
 // gemm_f16.cu — the same two entries on weights and activations as f16 planes. row_inv (may be null): 1 / scale of each row of x in
-// place of x.scale. Plane output: bf16, or behind GELU f16 of yp->scale. A row's result does not depend on the rows beside it. exact:
-// the sums of the f32 mode.
+// place of x.scale. Plane output: bf16, or behind GELU f16 of yp->scale. A row's result does not depend on the rows beside it.
 int launch_gemm_f16(const F16Mat& w, const Planes& x, const float* row_inv, const float* bias, const float* residual, int epi, float* y, const Planes* yp,
-                    int M, int ldy, int* status, cudaStream_t st, bool exact);
-int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st, bool exact);
+                    int M, int ldy, int* status, cudaStream_t st);
+int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st);
 // x [M][K] as f16 planes scaled row by row (row_inv [M]: 1 / scale) and w as exact f16 planes, in one launch; either may be empty.
 // top (may be null): raised to the bits of the largest square norm of the weight rows from `from` on (finite and positive).
 int launch_f16_planes(const float* x, int M, int K, const Planes& out /* lift counts, scale does not */, float* row_inv, const QMat& w, const F16Mat& planes, int from, unsigned* top,

@@ -1,7 +1,7 @@
 // Q8_0 GEMM with the weight as two f16 planes:
 //     Y[M][N] = X[M][K] · dequant(W[N][K])ᵀ + bias (+GELU) (+residual), or the softmax records of the LM head
 //
-// The product of the two-plane math mode (FC_MATH_BF16X3), and of window forwards in the f32 mode. A Q8_0 weight d·q has at most 19
+// The product of the two-plane math mode (FC_MATH_BF16X3). A Q8_0 weight d·q has at most 19
 // significant bits (11 of the f16 scale, 8 of the level) and is a whole multiple of 2^-24, so hi = f16(d·q) and lo = d·q - hi hold it
 // EXACTLY, as long as d·128 does not overflow f16 (QMat::f16_exact, checked at upload). An activation, scaled by a power of two
 // that keeps it in range, is hi + lo to 2^-23 relative. Three MMAs per step, hi·hi + hi·lo + lo·hi, drop 2^-24 of a product, and no
@@ -9,8 +9,9 @@
 //
 // gemm_tc.cu multiplies the levels instead (two MMAs per step with bf16 planes of x) and has to fold every 32-wide k-block
 // into registers by the block's scale: its drain is what bounds it, at half the rate of the pipe, and its two bf16 planes of x
-// leave 2^-17. It stays for the f32 linear, for narrow models in the f32 mode (below a width of 512 its sums are the more exact
-// ones), for matrices that f16 does not hold, and for few rows of a prime or of a caller's own, which it splits over K.
+// leave 2^-17. It stays for the f32 mode (three bf16 planes are an f32 exactly, two of f16 are not: its three products here took 16 %
+// off a batch of mixed requests, with a product at K = 768 at 1.08e-7 from 64 bits for 1.03e-7), for matrices that f16 does not hold, and for few
+// rows of a prime or of a caller's own, which it splits over K.
 //
 // The tensor core truncates its f32 sums: towards zero, once per MMA. Over all of K that is 1.05e-9 of the result per k (measured
 // on one MMA per 16 k: 1.1e-6 at K = 1024, 4.2e-6 at 4096; three times as much here), where two bf16 planes of x are 2.5e-6 off
@@ -18,11 +19,6 @@
 // on average the same share of a sum (2.8e-7 with two stages a group, 6.7e-7 with four), and the activations are lifted by it
 // (f16_lift). Error against 64 bits (relative, 2-norm) at K = 1024: two-plane mode 5.0e-7 (levels and bf16 planes: 2.5e-6; groups of 8:
 // 1.7e-6, and no faster).
-//
-// The f32 mode (FC_MATH_FP32) of models of width 512 and more is the same kernel with one stage a group, drained once per 12
-// MMAs. Its error at K = 768 / 1024 / 3072 / 4096: 1.08e-7 / 1.15e-7 / 1.54e-7 / 1.70e-7 (levels with three bf16 planes: 1.03e-7 / 1.15e-7 /
-// 1.84e-7 / 2.10e-7); of the log-probabilities of 12 x 768 and 24 x 1024 on windows of 32, 256 and 1024 ids 3.3e-8 / 3.3e-8 / 3.2e-8 and 3.7e-8 /
-// 3.6e-8 / 3.5e-8 (3.4e-8 / 3.3e-8 / 3.3e-8 and 3.7e-8 / 3.7e-8 / 3.7e-8). Groups of half a stage are no more exact (1.3e-7 at 768) and slower.
 //
 // One CTA per SM, 640 threads (registers 104 a thread of the drain, 64 of the others):
 //   warps 0-15  drain: a group's sums from TMEM into registers (lane = weight row, column = activation row); after the last
@@ -52,7 +48,7 @@ using namespace tc;
 namespace {
 
 constexpr int BK = 64;                                  // k per stage: one 128-byte swizzle row of f16
-constexpr int KGROUP = 4;                               // stages whose sums stay in TMEM in the two-plane mode; in the f32 mode one
+constexpr int KGROUP = 4;                               // stages whose sums stay in TMEM
 constexpr int W_BYTES = 128 * BK * 2;                   // one plane of the CTA's weight tile of a stage
 constexpr int DRAIN_WARPS = 16, TMA_WARP = 16, MMA_WARP = 17, THREADS = 640;
 constexpr int MAX_STAGES = 6;
@@ -63,7 +59,6 @@ enum Mode : int { OUT_F32 = 0, OUT_PLANES = 1 /* bf16 planes, or f16 planes of a
 
 struct F16Args {
     int N, K, M, stages;
-    int exact;                // the f32 mode
     const float* bias; const float* residual; int gelu;
     float inv;                // what takes the scale of x out of a sum (a power of two)
     const float* row_inv;     // the same per activation row, or null
@@ -181,12 +176,11 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
             const uint64_t desc = smem_desc(sb);
             const uint32_t dhi = (uint32_t)(desc >> 32);
             uint32_t w = (uint32_t)desc, ph = 0, aph = 1;
-            const int per_group = a.exact ? 1 : KGROUP;
             int s = 0, buf = 0;
             bool ok = true;
             for (int tile = group; tile < n_tiles && ok; tile += n_groups) {
                 for (int kb = 0, in_group = 0; kb < nst && ok; ++kb) {
-                    const bool first = in_group == 0, last = ++in_group == per_group || kb == nst - 1;
+                    const bool first = in_group == 0, last = ++in_group == KGROUP || kb == nst - 1;
                     if (last) in_group = 0;
                     ok = (!first || wait_bar(acc_empty + 8 * buf, aph, abort, a)) && wait_bar(full + 8 * s, ph, abort, a);
                     if (!ok) break;
@@ -224,7 +218,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
     // -------------------------------------------------------------------- drain and finish
     const int quarter = warp & 3, part = warp >> 2;                                 // 32 TMEM lanes, a quarter of the columns
     const uint32_t taddr0 = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part * CW);
-    const int groups = a.exact ? nst : (nst + KGROUP - 1) / KGROUP;
+    const int groups = (nst + KGROUP - 1) / KGROUP;
     uint32_t fph = 0;
     int buf = 0;
     for (int tile = group; tile < n_tiles; tile += n_groups) {
@@ -533,7 +527,7 @@ int launch_one(const CUtensorMap (&map)[4], F16Args a, int tiles, int sms, cudaS
 }
 
 template <int MODE>
-int launch_f16(const F16Mat& w, const Planes& x, F16Args a, int M, bool exact, cudaStream_t st) {
+int launch_f16(const F16Mat& w, const Planes& x, F16Args a, int M, cudaStream_t st) {
     static int sms[64] = {};
     int dev = 0;
     FC_CUDA(cudaGetDevice(&dev));
@@ -544,7 +538,6 @@ int launch_f16(const F16Mat& w, const Planes& x, F16Args a, int M, bool exact, c
     const TileChoice t = choose_tile(M, w.N, w.K, MODE, sms[dev]);
     a.N = w.N; a.K = w.K; a.M = M;
     a.inv = 1.0f / x.scale;
-    a.exact = exact;
     a.wait_cycles = g_debug.wait_cycles; a.withhold = g_debug.withhold;
     CUtensorMap map[4];
     FC_TRY(encode_plane(&map[0], w.hi, w.N, w.K, 128, true));
@@ -586,23 +579,23 @@ int launch_split_f16(const float* x, const Planes& out, size_t n, cudaStream_t s
 }
 
 int launch_gemm_f16(const F16Mat& w, const Planes& x, const float* row_inv, const float* bias, const float* residual, int epi, float* y, const Planes* yp,
-                    int M, int ldy, int* status, cudaStream_t st, bool exact) {
+                    int M, int ldy, int* status, cudaStream_t st) {
     F16Args a = {};
     a.bias = bias; a.residual = residual; a.gelu = epi == EPI_GELU; a.row_inv = row_inv; a.y = y; a.ldy = ldy; a.status = status;
     if (epi != EPI_NONE && epi != EPI_GELU) return fail(FC_E_ARG, "epilogue %d is not one of this entry's", epi);
-    if (y) return launch_f16<OUT_F32>(w, x, a, M, exact, st);
+    if (y) return launch_f16<OUT_F32>(w, x, a, M, st);
     if (!yp || (epi == EPI_GELU && yp->n != 2) || (w.N & 31) || (ldy & 7) || residual || row_inv || (epi == EPI_GELU && yp->scale == 0.0f) || (yp->scale != 0.0f && yp->n != 2))
         return fail(FC_E_SHAPE, "plane output needs N %% 32 == 0, ldy %% 8 == 0, bf16 planes or two f16 planes (behind GELU these) and no residual");
     for (int p = 0; p < yp->n; ++p) a.yp[p] = (uint16_t*)yp->p[p];
     a.out_scale = yp->scale; a.out_lift = yp->lift;
-    return epi == EPI_GELU ? launch_f16<OUT_GELU>(w, x, a, M, exact, st) : launch_f16<OUT_PLANES>(w, x, a, M, exact, st);
+    return epi == EPI_GELU ? launch_f16<OUT_GELU>(w, x, a, M, st) : launch_f16<OUT_PLANES>(w, x, a, M, st);
 }
 
-int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st, bool exact) {
+int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st) {
     if (!targets || !stats || !tlogit) return fail(FC_E_ARG, "the scoring epilogue needs targets, stats and tlogit");
     F16Args a = {};
     a.targets = targets; a.stats = (float4*)stats; a.tlogit = tlogit; a.status = status;
-    return launch_f16<OUT_SCORE>(w, x, a, M, exact, st);
+    return launch_f16<OUT_SCORE>(w, x, a, M, st);
 }
 
 }  // namespace fc

@@ -39,10 +39,9 @@ extern "C" {
 /* Math modes of the window forward (scoring, primes) and of the linears with M >= 2. Decode steps are
  * f32-equivalent in both. */
 #define FC_MATH_FP32 0      /* tcgen05 kind::f16, f32 accumulate: exact int8 levels against three bf16 planes of the activations (their f32
-                               value exactly), or, in GPT-2 models of width 512 and more, exact f16 planes of the weights against f16 planes of
-                               the activations (2^-23 relative), with sums no further from 64 bits */
-#define FC_MATH_BF16X3 1    /* the same against two bf16 planes (2^-17 relative), or f16 planes with sums kept longer in the tensor core
-                               (about 5e-7 of a product) */
+                               value exactly) */
+#define FC_MATH_BF16X3 1    /* the same against two bf16 planes (2^-17 relative), or exact f16 planes of the weights against two f16 planes of
+                               the activations, with sums kept longer in the tensor core (about 5e-7 of a product) */
 
 /* Dimensions of a gpt2-architecture GGUF (ferrum_core/src/loader/gpt2.rs:201-215). */
 typedef struct fc_config {
