@@ -2034,7 +2034,7 @@ int fc_debug_withhold_scratch(int on) {
 int fc_debug_set_wait_budget(long long cycles, int withhold_producers) {
     if (cycles <= 0) return fail(FC_E_ARG, "fc_debug_set_wait_budget: cycles = %lld", cycles);
     g_debug.wait_cycles = cycles;
-    g_debug.withhold = withhold_producers != 0;
+    g_debug.withhold = withhold_producers == 2 ? 2 : withhold_producers != 0;
     return FC_OK;
 }
 

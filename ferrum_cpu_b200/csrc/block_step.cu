@@ -112,7 +112,7 @@ struct Waits {
     int* status;
     StepState* state;                // a wait that runs out fails the step, so that nothing behind it writes or advances
     long long cycles;
-    int withhold;                    // test hook: the clusters' first CTAs send nothing of the row
+    int withhold;                    // test hook: the clusters' first CTAs send nothing of the row (1), no hidden unit (2)
 };
 __device__ __forceinline__ bool received(const uint64_t* bar, const Waits& w) {
     uint32_t ok;
@@ -212,7 +212,7 @@ struct RowNormed {
             float q = 0.0f;
             if (lane < mine) { const float a = v.x - m, c = v.y - m, e = v.z - m, f = v.w - m; q = (a * a + c * c) + (e * e + f * f); }
             q = warp_sum(q);
-            if (!(waits.withhold && rank == 0)) {
+            if (!(waits.withhold == 1 && rank == 0)) {
                 if (lane < mine) send(&s.xr[u], &s.bar, wid, v);
                 if (lane == 0) send(&s.stat[rank], &s.bar, wid, make_float2(m, q));
             }
@@ -589,14 +589,15 @@ __global__ void __launch_bounds__(T, 2) mlp_half_kernel(const MlpHalf a) {
     w.run(rs.xs[0], rs.xs[COPIES - 1], d >> 3, r);
 #pragma unroll
     for (int i = 0; i < HB; ++i)
-        if (lane < C && u0 + i < share) {
+        if (lane < C && u0 + i < share && !(waits.withhold == 2 && rank == 0)) {
             const int e = rank * share + u0 + i;
             float v;
             if constexpr (RMS) v = __fmul_rn(__fdiv_rn(r[2 * i], __fadd_rn(1.0f, expf(-r[2 * i]))), r[2 * i + 1]);
             else v = gelu_f(r[i]);
             send(&hid[e ^ ((e >> 3) & 12)], &bar, lane, KIND == LEVELS ? v * down_scale[i] : v);
         }
-    if (!received(&bar, waits)) { outstay(); return; }
+    // a warp goes on, or gives up, as a whole: what follows exchanges among its lanes, and nothing among warps
+    if (!__all_sync(0xffffffffu, received(&bar, waits))) { outstay(); return; }
     // eight threads that read the same quarter of their units meet every bank once: quarter j of unit u lies at j ^ (u / 2) % 4
     ulonglong2 v[4];
 #pragma unroll

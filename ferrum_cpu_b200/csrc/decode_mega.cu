@@ -321,7 +321,7 @@ __device__ bool produce_params(Cta& k, const float* lnpack, const float* biaspac
 
 __device__ void producer(Cta& k) {
     const MegaParams& p = k.p;
-    if (p.withhold) return;   // test hook: nothing is copied, the consumers' first wait runs out
+    if (p.withhold == 1) return;   // test hook: nothing is copied, the consumers' first wait runs out
     for (int step = 0; step < p.n_steps; ++step) {
         for (int l = 0; l < p.L; ++l) {
             const MegaLayer& L = k.layers[l];

@@ -150,7 +150,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
 
     if (warp >= TMA_WARP) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-        if (warp == TMA_WARP && !a.withhold && elect_one()) {
+        if (warp == TMA_WARP && a.withhold != 1 && elect_one()) {
             // ------------------------------------------------------------ TMA producer
             int s = 0;
             uint32_t ph = 1;

@@ -244,7 +244,7 @@ gemm_q8_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
 
     if (warp >= TMA_WARP) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-        if (warp == TMA_WARP && !a.withhold && elect_one()) {
+        if (warp == TMA_WARP && a.withhold != 1 && elect_one()) {
             // ------------------------------------------------------------ TMA producer
             int s = 0;
             uint32_t ph = 1;

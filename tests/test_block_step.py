@@ -86,6 +86,36 @@ def test_a_wait_that_runs_out_feeds_nothing():
     om.close()
 
 
+@pytest.mark.parametrize("kind", ["gpt2", "llama", "levels"])
+def test_hidden_units_that_never_come_feed_nothing(kind):
+    """The wait inside the MLP half runs out in every warp of a cluster; the step fails as a whole and the next one is as if it had not been."""
+    if kind == "gpt2":
+        sm = synth.SynthModel(2, 512, 8, 2048, 64, 515, seed=5, perturb=True)
+        om, gm = O.OracleModel(sm), fcb.CudaSlm(sm.config, sm.weights)
+        gm.set_decode_mode(1)
+        gpu, cpu = gm.feed, om.feed
+    else:
+        prec = {"llama": None, "levels": 0}[kind]
+        sm = synth.SynthLlama(515, 512, 2, 8, 2, 64, 2048, 64, seed=5, perturb=True)
+        om, gm = O.OracleLlama(sm, threads=4, **({} if prec is None else {"prec": prec})), CudaLlama.from_synth(sm, prec=prec)
+        cache = gm.new_cache()
+        om.clear()
+        gpu, cpu = lambda t: gm.forward_one(t, cache), om.forward_one
+    for t in (3, 11):
+        gpu(t), cpu(t)
+    _lib.check(_lib.lib().fc_debug_set_wait_budget(200000, 2))
+    try:
+        with pytest.raises(fcb.FerrumCudaError) as e:
+            gpu(7)
+    finally:
+        _lib.check(_lib.lib().fc_debug_set_wait_budget(4000000000, 0))
+    assert e.value.code == _lib.FC_E_TIMEOUT
+    got, want = gpu(7), cpu(7)
+    assert np.abs(got - want).max() < (2e-5 if kind == "gpt2" else 2e-4 * max(1.0, float(np.abs(want).max())))
+    gm.close()
+    om.close()
+
+
 # both pairings of the rotation with and without a tail that is not rotated, grouped heads, weights as stored and on rows of levels,
 # and caches longer than a CTA of a head holds
 @pytest.mark.parametrize("d,heads,kv,ff,ctx,rope_dim,rope_type,prec", [(512, 8, 2, 2048, 40, 64, 0, None), (512, 8, 8, 1024, 33, 48, 1, 0),
