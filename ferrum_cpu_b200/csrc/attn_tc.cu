@@ -20,7 +20,7 @@
 //   warp 4      TMA: Q once, then a K tile and a V tile (64 keys) per step;
 //   warp 5      tcgen05.mma issue: 12 (24) MMAs for the score tile, as many for P·V (V is consumed
 //               MN-major, exactly as TMA lays out its [keys][hd] rows).
-// Every mbarrier wait is bounded; on a timeout the status word is raised and the CTA leaves.
+// Every mbarrier wait is bounded; on a timeout the status word is raised and the CTA leaves, each warp as a whole.
 //
 // Bound: tensor pipe / MUFU. 4·hd·T(T+1)/2 algorithmic FLOP per (window, head).
 #include "pdl.cuh"
@@ -43,7 +43,6 @@ struct Smem {
 };
 constexpr int SOFTMAX_WARPS = 4, TMA_WARP = 4, MMA_WARP = 5, THREADS = 6 * 32;
 constexpr int TMEM_COLS = 128;         // score tile: columns 0..63, P·V tile: columns 64..127
-constexpr long long WAIT_CYCLES = 4000000000LL;
 // f32 sums, M = 128, N = 64; B K-major for Q·Kᵀ, MN-major (bit 16) for P·V
 constexpr uint32_t BF16 = (1u << 7) | (1u << 10);        // operand types; without: f16
 constexpr uint32_t IDESC_S = (1u << 4) | ((uint32_t)(KT >> 3) << 17) | ((uint32_t)(QT >> 4) << 24);
@@ -83,13 +82,13 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* b, uint32_t pa
         : "=r"(ok) : "r"(s32(b)), "r"(parity), "r"(2000u) : "memory");
     return ok != 0;
 }
-__device__ bool wait_bar(Bars* bars, unsigned long long* b, uint32_t parity, int* status) {
+template <class Args>
+__device__ bool wait_bar(Bars* bars, unsigned long long* b, uint32_t parity, const Args& a) {
     const long long t0 = clock64();
     while (!mbar_try_wait(b, parity)) {
         if (bars->abort) return false;
-        if (clock64() - t0 > WAIT_CYCLES) {
-            bars->abort = 1;
-            atomicExch(status, FC_E_TIMEOUT);
+        if (clock64() - t0 > a.wait_cycles) {
+            tc::give_up(&bars->abort, a);
             return false;
         }
     }
@@ -146,6 +145,8 @@ struct AttnArgs {
     float unscale;               // f16 planes: 1 / their scale
     float out_scale, out_lift;   // not 0: two f16 planes of out_scale (1 + out_lift) times the output
     int* status;
+    long long wait_cycles;       // budget of every mbarrier wait
+    int withhold;                // test hook: 1: nothing is copied
 };
 
 }  // namespace
@@ -194,17 +195,17 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
     pdl_trigger();
 
     if (warp == TMA_WARP) {
-        if (tc::elect_one()) {
+        if (a.withhold != 1 && tc::elect_one()) {
             mbar_expect_tx(&bars->q_full, P * Q_BYTES);
 #pragma unroll
             for (int p = 0; p < P; ++p) tma_load_2d(smem + OFF_Q + p * Q_BYTES, &maps.q[p], h * HD, row0 + q0, &bars->q_full);
             for (int kt = 0; kt < n_kt; ++kt) {
                 const uint32_t par = (kt & 1) ^ 1;
-                if (!wait_bar(bars, &bars->k_empty, par, a.status)) break;
+                if (!wait_bar(bars, &bars->k_empty, par, a)) break;
                 mbar_expect_tx(&bars->k_full, P * KV_BYTES);
 #pragma unroll
                 for (int p = 0; p < P; ++p) tma_load_2d(smem + OFF_K + p * KV_BYTES, &maps.kv[p], a.k_col + (h / a.group) * HD, row0 + kt * KT, &bars->k_full);
-                if (!wait_bar(bars, &bars->v_empty, par, a.status)) break;
+                if (!wait_bar(bars, &bars->v_empty, par, a)) break;
                 mbar_expect_tx(&bars->v_full, P * KV_BYTES);
 #pragma unroll
                 for (int p = 0; p < P; ++p) tma_load_2d(smem + OFF_V + p * KV_BYTES, &maps.kv[p], a.v_col + (h / a.group) * HD, row0 + kt * KT, &bars->v_full);
@@ -215,11 +216,11 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
             const uint32_t sb = s32(smem);
             const uint64_t dq = smem_desc(sb + OFF_Q), dk = smem_desc(sb + OFF_K), dv = smem_desc(sb + OFF_V), dp = smem_desc(sb + OFF_P);
             constexpr uint64_t QS = Q_BYTES / 16, KS = KV_BYTES / 16, PS = P_BYTES / 16;   // from plane to plane, in descriptor units
-            bool ok = wait_bar(bars, &bars->q_full, 0, a.status);
+            bool ok = wait_bar(bars, &bars->q_full, 0, a);
             // score tile kt: its keys have landed and the softmax warps have read the previous one out of TMEM
             auto issue_scores = [&](int kt) -> bool {
                 const uint32_t par = kt & 1;
-                if (!(wait_bar(bars, &bars->k_full, par, a.status) && wait_bar(bars, &bars->s_empty, par ^ 1, a.status))) return false;
+                if (!(wait_bar(bars, &bars->k_full, par, a) && wait_bar(bars, &bars->s_empty, par ^ 1, a))) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 each_term<P>([&](int i, int j, bool first) {
 #pragma unroll
@@ -240,8 +241,8 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
                     if (!ok) break;
                 }
                 // P·V tile: P is in shared memory, the previous P·V tile has been folded in
-                ok = wait_bar(bars, &bars->v_full, par, a.status) && wait_bar(bars, &bars->p_full, par, a.status) &&
-                     wait_bar(bars, &bars->o_empty, par ^ 1, a.status);
+                ok = wait_bar(bars, &bars->v_full, par, a) && wait_bar(bars, &bars->p_full, par, a) &&
+                     wait_bar(bars, &bars->o_empty, par ^ 1, a);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 each_term<P>([&](int i, int j, bool first) {
@@ -269,7 +270,7 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
         bool ok = true;
         for (int kt = 0; kt < n_kt && ok; ++kt) {
             const uint32_t par = kt & 1;
-            ok = wait_bar(bars, &bars->s_full, par, a.status);
+            ok = __all_sync(0xffffffffu, wait_bar(bars, &bars->s_full, par, a));   // loads, votes and barriers below are a warp's
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint32_t s0[32], s1[32];
@@ -318,7 +319,7 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
                 for (int c = 0; c < HD; ++c) o[c] *= corr;
             }
             // fold in this tile's P·V
-            ok = wait_bar(bars, &bars->o_full, par, a.status);
+            ok = __all_sync(0xffffffffu, wait_bar(bars, &bars->o_full, par, a));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             tmem_ld32(lane_addr + HD, s0);
@@ -353,6 +354,10 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (bars->abort) {                                     // copies and MMAs may be in flight for a few microseconds more
+        const long long t0 = clock64();
+        while (clock64() - t0 < 200000) __nanosleep(200);
+    }
     __syncthreads();
     if (warp == MMA_WARP) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -410,7 +415,7 @@ static int launch_attn_tc(const Planes& qkv, const Windows& w, int R, int H, int
     a.win = w; a.k_col = H * HD; a.v_col = (H + KV) * HD; a.group = H / KV; a.ldo = H * HD;
     a.unscale = F16 ? 1.0f / qkv.scale : 1.0f;
     a.out_scale = out.scale; a.out_lift = out.lift;
-    a.status = status;
+    a.status = status; a.wait_cycles = g_debug.wait_cycles; a.withhold = g_debug.withhold;
     dim3 grid((w.T + QT - 1) / QT, H, w.B);
     FC_CUDA(launch_pdl(attn_prefill_tc_kernel<P, F16>, grid, dim3(THREADS), SMEM_BYTES<P>, st, maps, a));
     FC_LAUNCHED();

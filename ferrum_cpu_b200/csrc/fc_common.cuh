@@ -41,7 +41,8 @@ inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 // Test hooks (fc_debug_set_wait_budget): the cycle budget of every bounded device-side wait, and a
 // switch that makes the producers of the pipelined kernels withhold their copies (1), or a kernel's second exchange come to nothing
-// (2: the hidden units of a decode step's block), so that a test can make a wait run out without faulting, trapping or hanging anything.
+// (2: the hidden units of a decode step's block; in a tensor-core GEMM one of four warps gives up by itself), so that a test can
+// make a wait run out without faulting, trapping or hanging anything.
 struct DebugKnobs {
     long long wait_cycles = 4000000000LL;   // ~2 s at 1.9 GHz
     int withhold = 0;

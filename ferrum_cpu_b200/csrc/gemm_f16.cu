@@ -34,7 +34,7 @@
 // their own, with the planes made (levels in gemm_tc.cu): 4096 x 1024 x 4096 73 us (109), 32768 x 768 x 2304 239 us = 1.46 PFLOP/s executed
 // (348), 32768 x 3072 x 768 322 us (450).
 //
-// Every wait is bounded; a wait that runs out raises the status word and all roles leave.
+// Every wait is bounded; a wait that runs out raises the status word and all roles leave, in whatever order they learn of it.
 #include <algorithm>
 #include <type_traits>
 
@@ -68,7 +68,7 @@ struct F16Args {
     const int* targets; float4* stats; float* tlogit;      // OUT_SCORE
     int* status;
     long long wait_cycles;
-    int withhold;
+    int withhold;             // test hooks
 };
 
 constexpr int BAR_FULL = 0, BAR_EMPTY = BAR_FULL + 8 * MAX_STAGES, BAR_ACC_FULL = BAR_EMPTY + 8 * MAX_STAGES, BAR_ACC_EMPTY = BAR_ACC_FULL + 16;
@@ -221,13 +221,15 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
     const int groups = (nst + KGROUP - 1) / KGROUP;
     uint32_t fph = 0;
     int buf = 0;
+    const bool quits = a.withhold == 2 && quarter == 1;                             // test hook: one warp of each part gives up alone
+    if (quits && lane == 0) give_up(abort, a);
     for (int tile = group; tile < n_tiles; tile += n_groups) {
         uint64_t acc[CW / 2];
 #pragma unroll
         for (int i = 0; i < CW / 2; ++i) acc[i] = 0;
-        bool ok = true;
+        bool ok = !quits;
 #pragma unroll 1
-        for (int g = 0; g < groups; ++g) {
+        for (int g = 0; g < groups && ok; ++g) {
             ok = __all_sync(0xffffffffu, wait_bar(acc_full + 8 * buf, fph, abort, a));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -247,6 +249,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
             buf ^= 1;
             if (buf == 0) fph ^= 1;
         }
+        // behind the vote the records of the tile before are read, too
+        if (MODE == OUT_SCORE) ok = all_of_128(1 + part, ok);
         if (!ok) break;
         const int n = (tile % tiles_n) * (128 * CG) + rank * 128 + quarter * 32 + lane;
         const int m0 = (tile / tiles_n) * NT + part * CW, left = a.M - m0;
@@ -257,7 +261,6 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
             // four quarters meet in shared memory. Lanes l and l + 16 end up with column 16 j + l of its warp.
             const float kLog2e = 1.4426950408889634f;
             const int nq = n - lane;
-            asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");            // the records of the tile before are read
 #pragma unroll
             for (int j = 0; j < CW / 16; ++j) {
                 float e[16], my_max = -INFINITY;

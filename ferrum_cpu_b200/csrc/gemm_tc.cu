@@ -35,7 +35,7 @@
 // distributed shared memory in rank order, so that a few activation rows still occupy the GPU and results stay
 // reproducible.
 //
-// Every wait is bounded; a wait that runs out raises the status word and all roles leave.
+// Every wait is bounded; a wait that runs out raises the status word and all roles leave, in whatever order they learn of it.
 // Bound: weight bytes for a few rows, the drain for many (2·M·N·K algorithmic FLOP, planes x that executed). Measured with the
 // split of X into planes (of the f32 form this replaced: CUDA-core FMA, 42 TFLOP/s):
 //     32768 x 768 x 2304   2 planes 348 us = 334 TFLOP/s   3 planes 369 us = 314 TFLOP/s
@@ -87,7 +87,7 @@ struct TcArgs {
     const int* targets; float4* stats; float* tlogit;
     int* status;
     long long wait_cycles;    // budget of every mbarrier wait
-    int withhold;             // test hook: the TMA producer issues nothing, so the waits on its stages run out
+    int withhold;             // test hooks. 1: the TMA producer issues nothing, so the waits on its stages run out
 };
 
 // Barriers and flags at the end of the shared memory, by byte offset.
@@ -331,7 +331,7 @@ gemm_q8_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
                     r.q[i] = have ? __ldg(src + (2 * kb + hk) * 2 + i) : make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);   // biased zeros
             };
             auto put = [&](Row& r, int kb) {
-                ok = wait_bar<true>(empty + 8 * s, ph, abort, a);
+                ok = __all_sync(0xffffffffu, wait_bar<true>(empty + 8 * s, ph, abort, a));
                 if (!ok) return;
                 scales[slot * 256 + row * 2 + hk] = r.d;
                 slot = slot == a.stages + SCALE_EXTRA - 1 ? 0 : slot + 1;
@@ -376,14 +376,16 @@ gemm_q8_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
         int slot = 0;
         uint32_t fph = 0;                                                           // phase of the acc_full barriers
         int buf = 0;
+        const bool quits = a.withhold == 2 && quarter == 1;                         // test hook: one warp of each part gives up alone
+        if (quits && lane == 0) give_up(abort, a);
         for (int tile = group; tile < n_tiles; tile += n_groups) {
             uint64_t acc[CW / 2];
 #pragma unroll
             for (int i = 0; i < CW / 2; ++i) acc[i] = 0;
-            bool ok = true;
+            bool ok = !quits;
             __half2 sc = __half2half2(__float2half(0.0f));
 #pragma unroll 1
-            for (int b = 2 * st0; b < min(2 * st1, nb); ++b) {
+            for (int b = 2 * st0; b < min(2 * st1, nb) && ok; ++b) {
                 ok = __all_sync(0xffffffffu, wait_bar(acc_full + 8 * buf, fph, abort, a));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -408,6 +410,8 @@ gemm_q8_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
                 }
                 if (++buf == a.bufs) { buf = 0; fph ^= 1; }
             }
+            // behind the vote the records of the tile before are read, too
+            if (MODE == OUT_SCORE) ok = all_of_128(1 + part, ok);
             if (!ok) break;
             const int n = (tile % tiles_n) * (128 * CG) + (CG == 2 ? rank * 128 : 0) + quarter * 32 + lane;
             const int m0 = (tile / tiles_n) * a.nt + part * cw;
@@ -427,7 +431,6 @@ gemm_q8_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
                 const float kLog2e = 1.4426950408889634f;
                 const bool real = n < a.N;
                 const int nq = n - lane;
-                asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");        // the records of the tile before are read
 #pragma unroll
                 for (int j = 0; j < CW / 32; ++j) {
                     float e[32], my_max = -INFINITY;

@@ -59,6 +59,11 @@ __device__ __forceinline__ bool mbar_sleep(uint32_t b, uint32_t parity) {
         : "=r"(ok) : "r"(b), "r"(parity), "r"(1000u) : "memory");
     return ok != 0;
 }
+template <class Args>
+__device__ __forceinline__ void give_up(volatile int* abort, const Args& a) {
+    *abort = 1;
+    atomicExch(a.status, FC_E_TIMEOUT);
+}
 // Bounded wait. Returns false (after raising the status word) when the budget runs out or another role of this CTA
 // already gave up. SLEEP: for the producers, which wait most of the time and are stages ahead.
 template <bool SLEEP = false, class Args>
@@ -68,12 +73,19 @@ __device__ __forceinline__ bool wait_bar(uint32_t b, uint32_t parity, volatile i
     while (!(SLEEP ? mbar_sleep(b, parity) : mbar_poll(b, parity, 256))) {
         if (*abort) return false;
         if (clock64() - t0 > a.wait_cycles) {
-            *abort = 1;
-            atomicExch(a.status, FC_E_TIMEOUT);
+            give_up(abort, a);
             return false;
         }
     }
     return true;
+}
+// Warps that meet at a named barrier (128 threads) go on together or not at all: a wait that ran out in one of them may have been
+// completed for another. Every warp votes once per tile, whatever its own wait said.
+__device__ __forceinline__ bool all_of_128(int barrier, bool ok) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %2, 0;\n\tbarrier.cta.red.and.pred p, %1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(r) : "r"(barrier), "r"((uint32_t)ok) : "memory");
+    return r != 0;
 }
 // mbar: shared::cluster address of the barrier the bytes complete on; with CG = 2 it may be the pair's other CTA's.
 template <int CG>

@@ -519,7 +519,7 @@ float fc_last_score_ms(const fc_model* m);
  * request timeout, slm_server/src/model_thread.rs:48-56). This hook sets that budget for launches
  * made afterwards by this process and, with withhold_producers != 0, makes the producer warps of
  * those kernels copy nothing (2: their copies come, and a later exchange does not: the hidden units
- * of a decode step's block), so that a test can watch a wait run out and the handle stay usable.
+ * of a decode step's block, a warp's share of a tensor-core product), so that a test can watch a wait run out and the handle stay usable.
  * Nothing faults, traps or waits without a limit. Not for production use: restore
  * (4000000000, 0) afterwards. */
 int fc_debug_set_wait_budget(long long cycles, int withhold_producers);

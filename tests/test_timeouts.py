@@ -102,3 +102,23 @@ def test_prime_times_out_and_recovers(ctx):
     for got, p in zip(gm.decode_batch(prompts, 5), prompts):
         assert np.array_equal(got, om.generate_greedy(p, 5)[0])
     gm.close()
+
+
+@pytest.mark.parametrize("hook", [1, 2])
+@pytest.mark.parametrize("mode", [fcb.FC_MATH_FP32, fcb.FC_MATH_BF16X3])
+def test_scoring_with_heads_of_64(mode, hook):
+    """Nothing is copied, in the tensor-core attention either; or one warp of those that share a tile's records gives up while the others
+    get their sums. All of them leave, and the next call is whole."""
+    sm = synth.SynthModel(1, 128, 2, 256, 96, 1000, seed=4, perturb=True, math_mode=mode)
+    gm, om = fcb.CudaSlm(sm.config, sm.weights), O.OracleModel(sm, threads=2)
+    ids = synth.token_ids(1, 96, 1000)
+    _lib.check(_lib.lib().fc_debug_set_wait_budget(SHORT, hook))
+    try:
+        with pytest.raises(fcb.FerrumCudaError) as e:
+            gm.token_logprobs(ids, 1)
+    finally:
+        _lib.check(_lib.lib().fc_debug_set_wait_budget(DEFAULT, 0))
+    assert e.value.code == _lib.FC_E_TIMEOUT
+    lp = gm.token_logprobs(ids, 1, per_token=True)[1]
+    assert np.abs(lp - om.token_logprobs(ids, 1)[3]).max() < 1e-3
+    gm.close()
