@@ -218,8 +218,10 @@ struct RowNormed {
             }
             if (r.x_out && first && wid == 0 && lane < mine && !done) ((float4*)r.x_out)[u] = v;
         }
-        // a warp without columns of its own waits at the block barrier instead: one that polls is late to wake
-        const bool ok = 32 * wid >= units || received(&s.bar, waits);
+        // a warp without columns of its own waits at the block barrier instead: one that polls is late to wake, and without a wait it
+        // may not read what the peers send
+        if (32 * wid >= units) return __syncthreads_and(true);
+        const bool ok = received(&s.bar, waits);
         // the CTAs' means and squares are merged around the common mean (n (m - mean)^2 is what a CTA's own mean left out)
         float2 st[C];
 #pragma unroll
