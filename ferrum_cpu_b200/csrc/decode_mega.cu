@@ -148,9 +148,8 @@ struct HeadWork {
     int spi;           // strips per ring item
     int kb;            // tiles per strip (K / 32)
     int strip_bytes;
-    int ks[2];         // K parts per strip: full item, last (shorter) item
-    int pad;
-    unsigned unit[2][CWARPS];   // per warp: strip | first tile << 8 | end tile << 16 (0xffffffff: idle)
+    int ks;            // K parts per strip
+    unsigned unit[CWARPS];   // per warp: strip | first tile << 8 | end tile << 16 (0xffffffff: idle)
 };
 static_assert(W_KINDS * 32 + sizeof(HeadWork) <= 512, "work descriptors");
 __device__ void make_head_work(HeadWork* w, int N, int K, int c, int G) {
@@ -158,20 +157,13 @@ __device__ void make_head_work(HeadWork* w, int N, int K, int c, int G) {
     w->kb = K >> 5;
     w->strip_bytes = mega_strip_bytes(K);
     w->spi = max(1, min(SLOT_BYTES / w->strip_bytes, CWARPS));
-    w->pad = 0;
-    const int n = w->s1 - w->s0;
-    const int ns_v[2] = {min(w->spi, max(n, 1)), n > 0 ? n - ((n - 1) / w->spi) * w->spi : 1};
-    for (int v = 0; v < 2; ++v) {
-        const int ns = ns_v[v], ks = max(1, min(w->kb, CWARPS / ns));
-        w->ks[v] = ks;
-        for (int u = 0; u < CWARPS; ++u) {
-            if (u < ns * ks) {
-                const int strip = u / ks, part = u - strip * ks;
-                w->unit[v][u] = (unsigned)strip | (unsigned)(part * w->kb / ks) << 8 | (unsigned)((part + 1) * w->kb / ks) << 16;
-            } else {
-                w->unit[v][u] = 0xffffffffu;
-            }
-        }
+    // One split of K for every strip, in whichever CTA and item it lies (a last item may leave warps idle): equal rows have equal
+    // logits, and the first of them is picked.
+    const int most = max(1, min(w->spi, (mega_strips(N) + G - 1) / G)), ks = max(1, min(w->kb, CWARPS / most));
+    w->ks = ks;
+    for (int u = 0; u < CWARPS; ++u) {
+        const int strip = u / ks, part = u - strip * ks;
+        w->unit[u] = strip < most ? (unsigned)strip | (unsigned)(part * w->kb / ks) << 8 | (unsigned)((part + 1) * w->kb / ks) << 16 : 0xffffffffu;
     }
 }
 
@@ -537,12 +529,11 @@ __device__ bool consume_head(Cta& k, float* lg) {
     const float* xsc = k.xsc();
     for (int s = wk.s0; s < wk.s1; s += wk.spi) {
         const int ns = min(wk.spi, wk.s1 - s);
-        const int var = ns == wk.spi ? 0 : 1;
         const int slot = k.item % SLOTS;
         if (!consumer_wait(k, &k.ctrl->full[slot], (k.item / SLOTS) & 1)) return false;
         float* ps = k.psum + (k.item & 1) * 256;
-        const unsigned unit = wk.unit[var][wid];
-        if (unit != 0xffffffffu) {
+        const unsigned unit = wk.unit[wid];
+        if ((int)(unit & 0xff) < ns) {
             const int strip = unit & 0xff, kb0 = (unit >> 8) & 0xff, kb1 = (unit >> 16) & 0xff;
             const unsigned char* tile = k.slot_q(slot) + strip * wk.strip_bytes + kb0 * kMegaTileBytes;
             float acc0 = 0.0f, acc1 = 0.0f;
@@ -570,7 +561,7 @@ __device__ bool consume_head(Cta& k, float* lg) {
         consumer_sync();                                   // slot fully read, partial sums visible
         if (lane == 0) mbar_arrive(&k.ctrl->empty[slot]);
         if (k.tid < ns * kMegaStripRows) {
-            const int strip = k.tid >> 3, r = k.tid & 7, ks = wk.ks[var];
+            const int strip = k.tid >> 3, r = k.tid & 7, ks = wk.ks;
             float v = 0.0f;
             for (int part = 0; part < ks; ++part) v += ps[(strip * ks + part) * 8 + r];
             const int n = (s + strip) * kMegaStripRows + r;

@@ -58,6 +58,26 @@ def test_pick_reads_the_rows_that_reach_the_largest(vocab, rows):
     om.close()
 
 
+# the persistent kernel, the chain, what a new stream takes (a prompt on the persistent kernel, or as a window), and streams in lock step;
+# widths whose heads give a CTA fewer strips than an item holds, and more
+@pytest.mark.parametrize("d,heads", [(128, 2), (512, 8), (768, 12)])
+@pytest.mark.parametrize("vocab", [515, 4736, 9501, 50257])
+@pytest.mark.parametrize("mode,prompt", [(0, 3), (1, 3), (2, 3), (2, 80), ("batch", 5)])
+def test_the_first_of_equal_rows_is_picked(d, heads, vocab, mode, prompt):
+    sm = synth.SynthModel(1, d, heads, 256, 128, vocab, seed=vocab, perturb=True)
+    blocks = sm.token_embd.reshape(vocab, d // 32 * 34)
+    blocks[:] = blocks[np.arange(vocab) % 131]
+    gm = fcb.CudaSlm(sm.config, sm.weights)
+    ids = synth.token_ids(4, 2 * prompt, vocab).reshape(2, prompt)
+    if mode == "batch":
+        got = np.concatenate(gm.decode_batch(ids, 12))
+    else:
+        gm.set_decode_mode(mode)
+        got = gm.generate_tokens(ids[0], 12)[0]
+    assert (got < min(vocab, 131)).all()
+    gm.close()
+
+
 def test_scores_of_minus_infinity_and_huge_rows():
     """A row without a finite logit ends as it does in the step of five launches: no id beyond the vocabulary, no hang."""
     sm = synth.SynthModel(1, 512, 8, 2048, 32, 515, seed=3)
