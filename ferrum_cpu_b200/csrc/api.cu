@@ -573,8 +573,7 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
     // 2506 and 2235 / 2449 / 3123)
     const bool f16 = m->f16 && planes == 2 && (!split_k || R > 64);
     m->pqkv.n = m->pn.n = m->patt.n = m->phid.n = planes;
-    m->pn.lift = m->patt.lift = f16_lift(d);
-    m->phid.lift = f16_lift(F);
+    m->pqkv.lo = 1.0f;                                               // the attention adds both planes' products in one place
     auto product = [&](const QMat& q, const F16Mat& h, const Planes& x, const float* bias, const float* residual, int epi, float* y, const Planes* yp) {
         return f16 ? launch_gemm_f16(h, x, nullptr, bias, residual, epi, y, yp, R, q.N, status, st)
                    : launch_gemm_q8_tc(q, x, bias, residual, epi, y, yp, R, q.N, status, st, split_k);
@@ -635,7 +634,6 @@ static int score_device(fc_model* m, const ScoreSlot& s, const Windows& win, int
     // target's logit: [rows][V] logits never reach memory (scoring.rs:175-181 needs one number per row)
     if (f16) {
         m->pn.scale = m->lnf_scale;
-        m->pn.lift = f16_lift(d);
     }
     FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, n == R ? nullptr : pick, n, d, m->pn, m->st));
     if (f16) FC_TRY(launch_gemm_f16_score(m->head_f16, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
@@ -725,7 +723,7 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
             __half* p = (__half*)scratch.p;
             const F16Mat wp = {p, p + nw, w->w.N, w->w.K};
             p += 2 * nw;
-            x.p[0] = p; x.p[1] = p + n; x.n = 2; x.scale = 1.0f; x.lift = f16_lift(w->w.K);
+            x.p[0] = p; x.p[1] = p + n; x.n = 2; x.scale = 1.0f;
             float* row_inv = (float*)(p + 2 * n);
             FC_TRY(launch_f16_planes(x_dev, M, w->w.K, x, row_inv, w->w, wp, 0, nullptr, st));
             return launch_gemm_f16(wp, x, row_inv, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, w->status.dev, st);

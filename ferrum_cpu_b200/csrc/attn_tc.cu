@@ -143,7 +143,7 @@ struct AttnArgs {
     int ldo;                     // row stride of the output planes (= query heads x 64)
     uint16_t* out[3];            // [R][ldo] bf16 planes, or
     float unscale;               // f16 planes: 1 / their scale
-    float out_scale, out_lift;   // not 0: two f16 planes of out_scale (1 + out_lift) times the output
+    float out_scale, out_lo;     // not 0: f16 planes of out_scale times the output, the second times out_lo
     int* status;
     long long wait_cycles;       // budget of every mbarrier wait
     int withhold;                // test hook: 1: nothing is copied
@@ -302,7 +302,7 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
                 uint32_t w[4][P];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    if constexpr (F16) split2_f16(p[2 * e], p[2 * e + 1], 0.0f, w[e]);
+                    if constexpr (F16) split2_f16(p[2 * e], p[2 * e + 1], 1.0f, w[e]);
                     else split2<P>(p[2 * e], p[2 * e + 1], w[e]);
                 }
 #pragma unroll
@@ -341,7 +341,7 @@ attn_prefill_tc_kernel(const __grid_constant__ AttnMaps maps, const AttnArgs a) 
                     const float v0 = o[8 * c + 2 * e] * inv, v1 = o[8 * c + 2 * e + 1] * inv;
                     if (a.out_scale != 0.0f) {
                         uint32_t t[2];
-                        split2_f16(v0 * a.out_scale, v1 * a.out_scale, a.out_lift, t);
+                        split2_f16(v0 * a.out_scale, v1 * a.out_scale, a.out_lo, t);
                         w[e][0] = t[0]; w[e][1] = t[1];
                     } else {
                         split2<P>(v0, v1, w[e]);
@@ -414,7 +414,7 @@ static int launch_attn_tc(const Planes& qkv, const Windows& w, int R, int H, int
     }
     a.win = w; a.k_col = H * HD; a.v_col = (H + KV) * HD; a.group = H / KV; a.ldo = H * HD;
     a.unscale = F16 ? 1.0f / qkv.scale : 1.0f;
-    a.out_scale = out.scale; a.out_lift = out.lift;
+    a.out_scale = out.scale; a.out_lo = out.lo;
     a.status = status; a.wait_cycles = g_debug.wait_cycles; a.withhold = g_debug.withhold;
     dim3 grid((w.T + QT - 1) / QT, H, w.B);
     FC_CUDA(launch_pdl(attn_prefill_tc_kernel<P, F16>, grid, dim3(THREADS), SMEM_BYTES<P>, st, maps, a));
@@ -423,6 +423,7 @@ static int launch_attn_tc(const Planes& qkv, const Windows& w, int R, int H, int
 }
 
 int launch_attn_prefill_tc_gqa(const Planes& qkv, const Windows& w, int R, int H, int KV, const Planes& out, int* status, cudaStream_t st) {
+    if (qkv.scale != 0.0f && qkv.lo != 1.0f) return fail(FC_E_ARG, "the attention's planes add up as they are");
     if (qkv.scale != 0.0f) return launch_attn_tc<2, true>(qkv, w, R, H, KV, out, status, st);
     return qkv.n == 3 ? launch_attn_tc<3, false>(qkv, w, R, H, KV, out, status, st) : launch_attn_tc<2, false>(qkv, w, R, H, KV, out, status, st);
 }

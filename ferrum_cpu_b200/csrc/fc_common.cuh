@@ -109,7 +109,7 @@ struct QMat {
     bool f16_exact = false;   // two f16 planes hold every weight exactly (largest scale x 128 within f16); else unknown
 };
 constexpr int kRowPad = 128;
-// A Q8_0 matrix as two f16 planes [N][K] whose sum it is, exactly (gemm_f16.cu).
+// A Q8_0 matrix as two f16 planes [N][K], hi and kRest times the rest, exactly (gemm_f16.cu).
 struct F16Mat {
     void *hi = nullptr, *lo = nullptr;
     int N = 0, K = 0;
@@ -230,16 +230,16 @@ struct Windows {
 };
 
 // An f32 matrix as n bf16 planes whose sum it is: 2 planes hold it to 2^-17 relative (FC_MATH_BF16X3), 3 exactly
-// (FC_MATH_FP32). The form in which activations reach the tensor cores. With a scale (a power of two) they are two f16 planes of
-// scale (1 + lift) times the matrix, for gemm_f16.cu; whoever sets it vouches for scale x values within f16's range.
+// (FC_MATH_FP32). The form in which activations reach the tensor cores. With a scale (a power of two) they are two f16 planes: hi of
+// scale times the matrix, and lo times what that leaves; whoever sets it vouches for scale x values within f16's range. kRest is the lo of
+// whatever gemm_f16.cu multiplies, weights included: it brings a remainder of 2^-11 up to where hi is, so that elements down to
+// 2^-13 keep 2^-23 of themselves (without it, down to 2^-2).
+constexpr float kRest = 2048.0f;
 struct Planes {
     void* p[3] = {nullptr, nullptr, nullptr};
     int n = 0;
-    float scale = 0.0f, lift = 0.0f;
+    float scale = 0.0f, lo = kRest;
 };
-// The lift of the f16 planes of a product's activations: the share of themselves that sums over K lose, on average, to the tensor
-// core's truncation (gemm_f16.cu), by the stages of 64 whose sums it keeps (up to four).
-inline float f16_lift(int K) { return K <= 64 ? 8.9e-8f : K <= 128 ? 2.8e-7f : K <= 192 ? 4.7e-7f : 6.7e-7f; }
 // Planes of n elements out of a call's scratch; scratch.p stays null when there is no memory.
 int take_planes(CallScratch& scratch, Planes& x, int planes, size_t n, int device, cudaStream_t st);
 // cols (may be null): column k of rows K wide is multiplied by cols[k] first.
@@ -268,7 +268,7 @@ int launch_gemm_f16(const F16Mat& w, const Planes& x, const float* row_inv, cons
 int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st);
 // x [M][K] as f16 planes scaled row by row (row_inv [M]: 1 / scale) and w as exact f16 planes, in one launch; either may be empty.
 // top (may be null): raised to the bits of the largest square norm of the weight rows from `from` on (finite and positive).
-int launch_f16_planes(const float* x, int M, int K, const Planes& out /* lift counts, scale does not */, float* row_inv, const QMat& w, const F16Mat& planes, int from, unsigned* top,
+int launch_f16_planes(const float* x, int M, int K, const Planes& out /* its scale does not count */, float* row_inv, const QMat& w, const F16Mat& planes, int from, unsigned* top,
                       cudaStream_t st);
 // Whether a caller's own two-plane product of M rows is better off there.
 bool f16_rows(int K, int M);

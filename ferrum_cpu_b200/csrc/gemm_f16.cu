@@ -5,7 +5,8 @@
 // significant bits (11 of the f16 scale, 8 of the level) and is a whole multiple of 2^-24, so hi = f16(d·q) and lo = d·q - hi hold it
 // EXACTLY, as long as d·128 does not overflow f16 (QMat::f16_exact, checked at upload). An activation, scaled by a power of two
 // that keeps it in range, is hi + lo to 2^-23 relative. Three MMAs per step, hi·hi + hi·lo + lo·hi, drop 2^-24 of a product, and no
-// scale is left to apply: k-blocks add up in TMEM, and the tensor pipe is what bounds the kernel.
+// scale is left to apply: k-blocks add up in TMEM, and the tensor pipe is what bounds the kernel. The lo planes hold kRest = 2^11 times
+// their values: an element 2^28 below the largest of its row (of the scale's bound, in a window forward) still keeps 2^-23 of itself.
 //
 // gemm_tc.cu multiplies the levels instead (two MMAs per step with bf16 planes of x) and has to fold every 32-wide k-block
 // into registers by the block's scale: its drain is what bounds it, at half the rate of the pipe, and its two bf16 planes of x
@@ -13,19 +14,23 @@
 // off a batch of mixed requests, with a product at K = 768 at 1.08e-7 from 64 bits for 1.03e-7), for matrices that f16 does not hold, and for few
 // rows of a prime or of a caller's own, which it splits over K.
 //
-// The tensor core truncates its f32 sums: towards zero, once per MMA. Over all of K that is 1.05e-9 of the result per k (measured
-// on one MMA per 16 k: 1.1e-6 at K = 1024, 4.2e-6 at 4096; three times as much here), where two bf16 planes of x are 2.5e-6 off
-// whatever K is. So sums stay in TMEM for KGROUP stages and then go into f32 registers, rounded to nearest. What they lose on the way is
-// on average the same share of a sum (2.8e-7 with two stages a group, 6.7e-7 with four), and the activations are lifted by it
-// (f16_lift). Error against 64 bits (relative, 2-norm) at K = 1024: two-plane mode 5.0e-7 (levels and bf16 planes: 2.5e-6; groups of 8:
-// 1.7e-6, and no faster).
+// The tensor core truncates its f32 sums: towards zero, once per MMA, by up to an ulp of the whole sum however small what is added. So
+// the small terms (hi·lo, lo·hi) have sums of their own, which 1 / kRest brings to where truncation does not count, and the sums of hi·hi
+// stay in TMEM for FIRST = 6 stages of a tile, then for KGROUP = 3 at a time, and go into f32 registers, rounded to nearest. Sums that need no rounding
+// lose nothing. Error against 64 bits on normal draws (relative, 2-norm) at K = 512 / 768 / 1024 / 3072 / 4096: 4.4e-7 / 4.0e-7 / 3.7e-7 / 3.2e-7 /
+// 3.1e-7. Levels and two bf16 planes: 2.5e-6. All three terms in one sum, four stages: 8e-7, in groups of one stage 1.4e-7 and a tenth slower.
+//
+// With a place each, the 512 columns hold no second buffer. The order of a tile's MMAs makes up for it: at a group's end the drain
+// reads the sums of hi·hi (some 1000 cycles from commit to issuer) while the small terms of that stage and the next group's first run, and a
+// tile's first and last small terms come behind the main terms of two stages. The first group is long because the drain is in the epilogue of the
+// tile before: with 4 + 4 stages 4096 x 1024 x 4096 took 102 us, 98 now (two buffers, one sum: 97).
 //
 // One CTA per SM, 640 threads (registers 104 a thread of the drain, 64 of the others):
 //   warps 0-15  drain: a group's sums from TMEM into registers (lane = weight row, column = activation row); after the last
 //               group bias / GELU / residual or the softmax records, and the stores. With 8 warps of twice the columns the GELU
 //               epilogue was latency-bound: 32768 x 768 x 3072 390 us, now 298
 //   warp 16     TMA: both planes of the weight and of the activations, 64 k a stage
-//   warp 17     MMA issue and the TMEM allocation: two buffers of up to 256 columns, so that a group is read while the next runs.
+//   warp 17     MMA issue and the TMEM allocation: up to 256 columns for the sums of hi·hi, as many for the small terms'.
 //               One elected thread (tc.cuh: elect_one) issues an MMA in about 30 cycles; behind lane == 0 it took 74
 // CG = 2: a pair of CTAs shares a tile of 256 weight rows (each holds 128 of them and half of the activation rows). CG = 1
 // takes few rows. The order of a row's sums depends on K alone, so a row's result does not depend on the rows beside it.
@@ -48,11 +53,12 @@ using namespace tc;
 namespace {
 
 constexpr int BK = 64;                                  // k per stage: one 128-byte swizzle row of f16
-constexpr int KGROUP = 4;                               // stages whose sums stay in TMEM
+constexpr int FIRST = 6, KGROUP = 3;                    // stages whose sums stay in TMEM: a tile's first ones, then so many at a time
+static_assert(FIRST >= 2, "the first two stages of a tile are one group");
 constexpr int W_BYTES = 128 * BK * 2;                   // one plane of the CTA's weight tile of a stage
 constexpr int DRAIN_WARPS = 16, TMA_WARP = 16, MMA_WARP = 17, THREADS = 640;
 constexpr int MAX_STAGES = 6;
-constexpr int TMEM_COLS = 512, ACC_COLS = 256;
+constexpr int TMEM_COLS = 512, REST = 256;              // the sums of hi·hi, and from column REST on those of the small terms
 constexpr int SMEM_LIMIT = 227 * 1024;
 
 enum Mode : int { OUT_F32 = 0, OUT_PLANES = 1 /* bf16 planes, or f16 planes of a scale */, OUT_GELU = 2 /* f16 planes, after GELU */, OUT_SCORE = 3 };
@@ -64,15 +70,15 @@ struct F16Args {
     const float* row_inv;     // the same per activation row, or null
     float* y; int ldy;        // OUT_F32
     uint16_t* yp[3];          // OUT_PLANES, OUT_GELU: planes (three only of bf16), ldy elements apart
-    float out_scale, out_lift;   // scale and lift of f16 planes
+    float out_scale, out_lo;  // f16 planes: of out_scale times the output, the second times out_lo
     const int* targets; float4* stats; float* tlogit;      // OUT_SCORE
     int* status;
     long long wait_cycles;
     int withhold;             // test hooks
 };
 
-constexpr int BAR_FULL = 0, BAR_EMPTY = BAR_FULL + 8 * MAX_STAGES, BAR_ACC_FULL = BAR_EMPTY + 8 * MAX_STAGES, BAR_ACC_EMPTY = BAR_ACC_FULL + 16;
-constexpr int BAR_TMEM = BAR_ACC_EMPTY + 16, BAR_ABORT = BAR_TMEM + 4, BAR_BYTES = BAR_ABORT + 4;
+constexpr int BAR_FULL = 0, BAR_EMPTY = BAR_FULL + 8 * MAX_STAGES, BAR_ACC_FULL = BAR_EMPTY + 8 * MAX_STAGES, BAR_ACC_EMPTY = BAR_ACC_FULL + 8;
+constexpr int BAR_REST_FULL = BAR_ACC_EMPTY + 8, BAR_REST_EMPTY = BAR_REST_FULL + 8, BAR_TMEM = BAR_REST_EMPTY + 8, BAR_ABORT = BAR_TMEM + 4, BAR_BYTES = BAR_ABORT + 4;
 
 __device__ __forceinline__ void add2(uint64_t& acc, uint64_t v) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(v)); }
 
@@ -92,6 +98,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
     volatile int* abort = (volatile int*)(tail + BAR_ABORT);
     const uint32_t sb = s32(smem), full = s32(tail) + BAR_FULL, empty = s32(tail) + BAR_EMPTY;
     const uint32_t acc_full = s32(tail) + BAR_ACC_FULL, acc_empty = s32(tail) + BAR_ACC_EMPTY;
+    const uint32_t rest_full = s32(tail) + BAR_REST_FULL, rest_empty = s32(tail) + BAR_REST_EMPTY;
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int rank = CG == 2 ? (int)(blockIdx.x & 1) : 0;
     const int group = blockIdx.x / CG, n_groups = gridDim.x / CG;                   // CTAs or pairs take tiles in turn
@@ -105,10 +112,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
             mbar_init(full + 8 * s, 1);
             mbar_init(empty + 8 * s, 1);
         }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(acc_full + 8 * b, 1);
-            mbar_init(acc_empty + 8 * b, DRAIN_WARPS * CG);
-        }
+        mbar_init(acc_full, 1);
+        mbar_init(acc_empty, DRAIN_WARPS * CG);
+        mbar_init(rest_full, 1);
+        mbar_init(rest_empty, DRAIN_WARPS * CG);
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -132,7 +139,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
     pdl_wait();                                                                     // set up while the kernel ahead still ran
     pdl_trigger();
     // the barriers the pair's MMA issuer waits on are the leader's
-    const uint32_t full_leader = CG == 2 ? mapa(full, 0) : full, acc_empty_leader = CG == 2 ? mapa(acc_empty, 0) : acc_empty;
+    const uint32_t full_leader = CG == 2 ? mapa(full, 0) : full, acc_empty_leader = CG == 2 ? mapa(acc_empty, 0) : acc_empty,
+                   rest_empty_leader = CG == 2 ? mapa(rest_empty, 0) : rest_empty;
 
     // Every role ends here: nobody leaves while a peer may still reach this CTA's shared memory or barriers. After an
     // aborted wait, copies and MMAs may be in flight for a few microseconds more: outstay them.
@@ -175,32 +183,72 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
             constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(8 * CG) << 24);
             const uint64_t desc = smem_desc(sb);
             const uint32_t dhi = (uint32_t)(desc >> 32);
-            uint32_t w = (uint32_t)desc, ph = 0, aph = 1;
-            int s = 0, buf = 0;
+            const uint32_t rest = tmem + REST;
+            uint32_t w = (uint32_t)desc, ph = 0, aph = 1, rph = 1;
+            auto main_terms = [&](auto accumulate) {
+                const uint32_t x = w + 2 * W_BYTES / 16;                            // descriptors count 16 bytes
+                umma<CG, decltype(accumulate)::value>(tmem, w, x, dhi, idesc);
+#pragma unroll
+                for (int k = 1; k < BK / 16; ++k) umma<CG, true>(tmem, w + 2 * k, x + 2 * k, dhi, idesc);
+            };
+            auto small_terms = [&](uint32_t w, auto accumulate) {
+                const uint32_t x = w + 2 * W_BYTES / 16;
+                umma<CG, decltype(accumulate)::value>(rest, w + W_BYTES / 16, x, dhi, idesc);
+#pragma unroll
+                for (int k = 1; k < BK / 16; ++k) umma<CG, true>(rest, w + W_BYTES / 16 + 2 * k, x + 2 * k, dhi, idesc);
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k) umma<CG, true>(rest, w + 2 * k, x + X_BYTES / 16 + 2 * k, dhi, idesc);
+            };
+            const std::integral_constant<bool, true> add;
+            const std::integral_constant<bool, false> set;
+            int s = 0;
             bool ok = true;
             for (int tile = group; tile < n_tiles && ok; tile += n_groups) {
-                for (int kb = 0, in_group = 0; kb < nst && ok; ++kb) {
-                    const bool first = in_group == 0, last = ++in_group == KGROUP || kb == nst - 1;
-                    if (last) in_group = 0;
-                    ok = (!first || wait_bar(acc_empty + 8 * buf, aph, abort, a)) && wait_bar(full + 8 * s, ph, abort, a);
+                uint32_t held = 0, held_empty = 0;
+                bool holds = false;
+                for (int kb = 0, left = 0; kb < nst; ++kb) {
+                    ok = wait_bar(full + 8 * s, ph, abort, a);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t acc = tmem + buf * ACC_COLS, x = w + 2 * W_BYTES / 16;      // descriptors count 16 bytes
-                    // the small terms first: they meet a small accumulator
-                    if (first) umma<CG, false>(acc, w + W_BYTES / 16, x, dhi, idesc);
-                    else umma<CG, true>(acc, w + W_BYTES / 16, x, dhi, idesc);
-#pragma unroll
-                    for (int k = 1; k < BK / 16; ++k) umma<CG, true>(acc, w + W_BYTES / 16 + 2 * k, x + 2 * k, dhi, idesc);
-#pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) umma<CG, true>(acc, w + 2 * k, x + X_BYTES / 16 + 2 * k, dhi, idesc);
-#pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) umma<CG, true>(acc, w + 2 * k, x + 2 * k, dhi, idesc);
-                    umma_commit<CG>(empty + 8 * s);
-                    if (last) {
-                        umma_commit<CG>(acc_full + 8 * buf);
-                        buf ^= 1;
-                        if (buf == 0) aph ^= 1;
+                    const bool begins = left == 0, ahead = begins && kb > 0;
+                    if (begins) {
+                        // the sums' place is read while the small terms of this stage and the one before run
+                        left = min(kb == 0 ? FIRST : KGROUP, nst - kb);
+                        if (ahead) small_terms(w, add);
+                        ok = wait_bar(acc_empty, aph, abort, a);
+                        if (!ok) break;
+                        aph ^= 1;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        main_terms(set);
+                    } else {
+                        main_terms(add);
                     }
+                    if (--left == 0) umma_commit<CG>(acc_full);
+                    if (!ahead && (kb == 0 ? nst > 1 : kb == nst - 2 && kb > 1)) {
+                        // a tile's first and last small terms come behind the main terms of two stages: the drain reads the small terms of
+                        // the tile before, and the main terms of this one, meanwhile
+                        held = w;
+                        held_empty = empty + 8 * s;
+                        holds = true;
+                    } else {
+                        const bool starts = kb == (nst > 1);
+                        if (starts) {
+                            ok = wait_bar(rest_empty, rph, abort, a);
+                            if (!ok) break;
+                            rph ^= 1;
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        }
+                        if (holds) {
+                            if (starts) small_terms(held, set);
+                            else small_terms(held, add);
+                            umma_commit<CG>(held_empty);
+                            holds = false;
+                        }
+                        if (kb == 0) small_terms(w, set);
+                        else if (!ahead) small_terms(w, add);
+                        umma_commit<CG>(empty + 8 * s);
+                    }
+                    if (kb == nst - 1) umma_commit<CG>(rest_full);
                     w += STAGE / 16;
                     if (++s == a.stages) { s = 0; ph ^= 1; w = (uint32_t)desc; }
                 }
@@ -218,9 +266,24 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
     // -------------------------------------------------------------------- drain and finish
     const int quarter = warp & 3, part = warp >> 2;                                 // 32 TMEM lanes, a quarter of the columns
     const uint32_t taddr0 = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part * CW);
-    const int groups = (nst + KGROUP - 1) / KGROUP;
-    uint32_t fph = 0;
-    int buf = 0;
+    const int groups = 1 + (max(nst - FIRST, 0) + KGROUP - 1) / KGROUP;
+    // the warp's columns from column `col` on, pair by pair, and the word that they are read
+    auto take = [&](int col, uint32_t bar, auto put) {
+        constexpr int LW = CW % 32 == 0 ? 32 : CW % 16 == 0 ? 16 : 8;
+#pragma unroll
+        for (int o = 0; o < CW; o += LW) {
+            uint32_t r[LW];
+            tmem_ld_n<LW>(taddr0 + (uint32_t)(col + o), r, 0);
+            tmem_wait<LW>(r);
+            if (o + LW == CW) {
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                if (lane == 0) mbar_arrive_cluster(bar);
+            }
+#pragma unroll
+            for (int i = 0; i < LW / 2; ++i) put(o / 2 + i, pack2(r[2 * i], r[2 * i + 1]));
+        }
+    };
+    uint32_t fph = 0, rph = 0;
     const bool quits = a.withhold == 2 && quarter == 1;                             // test hook: one warp of each part gives up alone
     if (quits && lane == 0) give_up(abort, a);
     for (int tile = group; tile < n_tiles; tile += n_groups) {
@@ -230,24 +293,18 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
         bool ok = !quits;
 #pragma unroll 1
         for (int g = 0; g < groups && ok; ++g) {
-            ok = __all_sync(0xffffffffu, wait_bar(acc_full + 8 * buf, fph, abort, a));
+            ok = __all_sync(0xffffffffu, wait_bar(acc_full, fph, abort, a));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            constexpr int LW = CW % 32 == 0 ? 32 : CW % 16 == 0 ? 16 : 8;
-#pragma unroll
-            for (int o = 0; o < CW; o += LW) {
-                uint32_t r[LW];
-                tmem_ld_n<LW>(taddr0 + (uint32_t)(buf * ACC_COLS + o), r, 0);
-                tmem_wait<LW>(r);
-                if (o + LW == CW) {
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    if (lane == 0) mbar_arrive_cluster(acc_empty_leader + 8 * buf);
-                }
-#pragma unroll
-                for (int i = 0; i < LW / 2; ++i) add2(acc[o / 2 + i], pack2(r[2 * i], r[2 * i + 1]));
-            }
-            buf ^= 1;
-            if (buf == 0) fph ^= 1;
+            take(0, acc_empty_leader, [&](int i, uint64_t v) { add2(acc[i], v); });
+            fph ^= 1;
+        }
+        ok = __all_sync(0xffffffffu, ok && wait_bar(rest_full, rph, abort, a));
+        if (ok) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t share = pack2(__float_as_uint(1.0f / kRest), __float_as_uint(1.0f / kRest));
+            take(REST, rest_empty_leader, [&](int i, uint64_t v) { fma2(acc[i], v, share); });
+            rph ^= 1;
         }
         // behind the vote the records of the tile before are read, too
         if (MODE == OUT_SCORE) ok = all_of_128(1 + part, ok);
@@ -257,60 +314,19 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
         const bool real = n < a.N;
         const float bias = a.bias && real ? __ldg(a.bias + n) : 0.0f;
         if constexpr (MODE == OUT_SCORE) {
-            // softmax records of (activation row, 128 weight rows): each warp reduces its 32 lanes per column, the
-            // four quarters meet in shared memory. Lanes l and l + 16 end up with column 16 j + l of its warp.
-            const float kLog2e = 1.4426950408889634f;
+            // each warp reduces its 32 lanes per column, the four quarters meet in shared memory
             const int nq = n - lane;
+            auto records = [&](auto w, const int c0) {
+                constexpr int W = decltype(w)::value;
+                score_records<W>([&](int i) { return ((i & 1) ? hi_f(acc[(c0 + i) / 2]) : lo_f(acc[(c0 + i) / 2])) * a.inv; }, lane, nq < a.N ? nq : 0x7fffffff - 64, real,
+                                 m0 + c0, a.M, W, a.targets, a.tlogit, recs + quarter * NT + part * CW + c0);
+            };
 #pragma unroll
-            for (int j = 0; j < CW / 16; ++j) {
-                float e[16], my_max = -INFINITY;
-                int my_idx = 0x7fffffff;
-                const int mt = m0 + j * 16 + (lane & 15);
-                const int tgt = mt < a.M ? __ldg(a.targets + mt) : -1;
-                const uint32_t hits = __ballot_sync(0xffffffffu, tgt >= nq && tgt < nq + 32);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const float v = ((i & 1) ? hi_f(acc[j * 8 + i / 2]) : lo_f(acc[j * 8 + i / 2])) * a.inv;
-                    const float t = real ? v : -INFINITY;
-                    const float mx = redux_max(t);
-                    const uint32_t at = __ballot_sync(0xffffffffu, t == mx);
-                    e[i] = real ? ex2((v - mx) * kLog2e) : 0.0f;
-                    if ((lane & 15) == i) { my_max = mx; my_idx = nq + __ffs(at) - 1; }
-                    if (hits >> i & 1) {                                             // some lane's row is the target of column i
-                        const int tg = __shfl_sync(0xffffffffu, tgt, i);
-                        if (n == tg) a.tlogit[m0 + j * 16 + i] = v;
-                    }
-                }
-                // transposing sum: 8 + 4 + 2 + 1 exchanges leave lanes l and l + 16 with halves of the sum of column l
-#pragma unroll
-                for (int o = 8; o > 0; o >>= 1) {
-#pragma unroll
-                    for (int i = 0; i < o; ++i) {
-                        const bool up = lane & o;
-                        const float keep = up ? e[i + o] : e[i], send = up ? e[i] : e[i + o];
-                        e[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-                    }
-                }
-                e[0] += __shfl_xor_sync(0xffffffffu, e[0], 16);
-                if (lane < 16)
-                    recs[quarter * NT + part * CW + j * 16 + lane] = make_float4(my_max, e[0], __int_as_float(nq < a.N ? my_idx : 0x7fffffff), 0.0f);
-            }
+            for (int c0 = 0; c0 + 16 <= CW; c0 += 16) records(std::integral_constant<int, 16>(), c0);
             asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");
             const int c = quarter * 32 + lane, m = m0 + c;
             const int t128 = (tile % tiles_n) * CG + rank, n128 = (a.N + 127) / 128;
-            if (c < CW && m < a.M && t128 < n128) {
-                float mx = -INFINITY, sum = 0.0f;
-                int idx = 0x7fffffff;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) mx = fmaxf(mx, recs[q * NT + part * CW + c].x);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float4 r = recs[q * NT + part * CW + c];
-                    if (r.x > -INFINITY || r.y != 0.0f) sum += r.y * ex2((r.x - mx) * kLog2e);
-                    if (r.x == mx) idx = min(idx, __float_as_int(r.z));
-                }
-                a.stats[(size_t)m * n128 + t128] = make_float4(mx, sum, __int_as_float(idx), 0.0f);
-            }
+            if (c < CW && m < a.M && t128 < n128) a.stats[(size_t)m * n128 + t128] = merge_records(recs + part * CW + c, NT);
         } else if constexpr (MODE == OUT_F32) {
             // the residual may be the output itself, so the compiler cannot move loads above the stores ahead of them: a batch
             // of them is asked for first
@@ -351,11 +367,11 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
                     uint32_t w[3];
                     if (MODE == OUT_GELU) {
                         uint32_t t[2];
-                        split2_f16(gelu_f(v0) * a.out_scale, gelu_f(v1) * a.out_scale, a.out_lift, t);
+                        split2_f16(gelu_f(v0) * a.out_scale, gelu_f(v1) * a.out_scale, a.out_lo, t);
                         w[0] = t[0]; w[1] = t[1];
                     } else if (a.out_scale != 0.0f) {
                         uint32_t t[2];
-                        split2_f16(v0 * a.out_scale, v1 * a.out_scale, a.out_lift, t);
+                        split2_f16(v0 * a.out_scale, v1 * a.out_scale, a.out_lo, t);
                         w[0] = t[0]; w[1] = t[1]; w[2] = 0;
                     } else if (a.yp[2]) {
                         split2<3>(v0, v1, w);
@@ -385,7 +401,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
 // Rows of x as f16 planes, each scaled by a power of two that brings its largest element into [2^14, 2^15), and rows of a Q8_0
 // matrix as exact f16 planes; a warp per row. top (null or a zeroed word): bits of the largest square norm among the weight rows from
 // `from` on.
-__global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict__ x, int M, int K, float lift, __half* __restrict__ xh, __half* __restrict__ xl,
+__global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict__ x, int M, int K, __half* __restrict__ xh, __half* __restrict__ xl,
                                                          float* __restrict__ row_inv, const QMat w, __half* __restrict__ wh,
                                                          __half* __restrict__ wl, int from, unsigned* __restrict__ top) {
     constexpr int HELD = 8;
@@ -411,8 +427,8 @@ __global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict
         const float s = __uint_as_float((uint32_t)se << 23);
         auto put = [&](int u, const float4& v) {
             uint32_t p[2], q[2];
-            split2_f16(v.x * s, v.y * s, lift, p);
-            split2_f16(v.z * s, v.w * s, lift, q);
+            split2_f16(v.x * s, v.y * s, kRest, p);
+            split2_f16(v.z * s, v.w * s, kRest, q);
             ((uint2*)(xh + (size_t)row * K))[u] = make_uint2(p[0], q[0]);
             ((uint2*)(xl + (size_t)row * K))[u] = make_uint2(p[1], q[1]);
         };
@@ -438,7 +454,7 @@ __global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict
             // 0x6400 | u is 1024 + u in f16: less 1152 it is the level, exactly
             const uint32_t t = __byte_perm((&u.x)[i >> 1], 0x64646464u, (i & 1) ? 0x4342 : 0x4140);
             const __half2 lv = __hsub2(*(const __half2*)&t, __half2half2(__ushort_as_half((unsigned short)0x6480)));
-            const __half2 h = __hmul2(lv, d2), r = __hfma2(lv, d2, __hneg2(h));       // the rounding's remainder, exactly
+            const __half2 h = __hmul2(lv, d2), r = __hmul2(__hfma2(lv, d2, __hneg2(h)), __float2half2_rn(kRest));   // the rounding's remainder, exactly
             hi[i] = *(const uint32_t*)&h;
             lo[i] = *(const uint32_t*)&r;
             if (top) {
@@ -460,12 +476,12 @@ __global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict
 }
 
 // x [n] as f16 planes of out.scale times its values.
-__global__ void __launch_bounds__(256) split_f16_kernel(const float4* __restrict__ x, uint2* __restrict__ hi, uint2* __restrict__ lo, float scale, float lift, size_t n4) {
+__global__ void __launch_bounds__(256) split_f16_kernel(const float4* __restrict__ x, uint2* __restrict__ hi, uint2* __restrict__ lo, float scale, float rest, size_t n4) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
         const float4 v = x[i];
         uint32_t p[2], q[2];
-        split2_f16(v.x * scale, v.y * scale, lift, p);
-        split2_f16(v.z * scale, v.w * scale, lift, q);
+        split2_f16(v.x * scale, v.y * scale, rest, p);
+        split2_f16(v.z * scale, v.w * scale, rest, q);
         hi[i] = make_uint2(p[0], q[0]);
         lo[i] = make_uint2(p[1], q[1]);
     }
@@ -537,7 +553,7 @@ int launch_f16(const F16Mat& w, const Planes& x, F16Args a, int M, cudaStream_t 
     if (dev >= 64) return fail(FC_E_ARG, "device %d out of range", dev);
     if (!sms[dev]) FC_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
     if (M <= 0) return FC_OK;
-    if (x.n != 2 || x.scale == 0.0f || !w.hi || w.K % 32) return fail(FC_E_SHAPE, "the f16 GEMM takes two f16 planes of either side and K %% 32 == 0 (K = %d)", w.K);
+    if (x.n != 2 || x.scale == 0.0f || x.lo != kRest || !w.hi || w.K % 32) return fail(FC_E_SHAPE, "the f16 GEMM takes two f16 planes of either side and K %% 32 == 0 (K = %d)", w.K);
     const TileChoice t = choose_tile(M, w.N, w.K, MODE, sms[dev]);
     a.N = w.N; a.K = w.K; a.M = M;
     a.inv = 1.0f / x.scale;
@@ -566,7 +582,7 @@ bool f16_rows(int K, int M) { return M >= 512 && M >= K / 2; }
 int launch_f16_planes(const float* x, int M, int K, const Planes& out, float* row_inv, const QMat& w, const F16Mat& planes, int from, unsigned* top,
                       cudaStream_t st) {
     if (K % 4 || w.K % 16) return fail(FC_E_SHAPE, "f16 planes: row lengths %d, %d", K, w.K);
-    f16_planes_kernel<<<(M + w.N + 7) / 8, 256, 0, st>>>(x, M, K, out.lift, (__half*)out.p[0], (__half*)out.p[1], row_inv, w, (__half*)planes.hi, (__half*)planes.lo,
+    f16_planes_kernel<<<(M + w.N + 7) / 8, 256, 0, st>>>(x, M, K, (__half*)out.p[0], (__half*)out.p[1], row_inv, w, (__half*)planes.hi, (__half*)planes.lo,
                                                          from, top);
     FC_LAUNCHED();
     return FC_OK;
@@ -576,7 +592,7 @@ int launch_split_f16(const float* x, const Planes& out, size_t n, cudaStream_t s
     if (n % 4 || out.n != 2 || out.scale == 0.0f) return fail(FC_E_SHAPE, "split_f16: %zu elements into %d planes", n, out.n);
     const size_t n4 = n / 4;
     split_f16_kernel<<<(int)std::max<size_t>(1, std::min<size_t>((n4 + 255) / 256, 148 * 8)), 256, 0, st>>>(
-        (const float4*)x, (uint2*)out.p[0], (uint2*)out.p[1], out.scale, out.lift, n4);
+        (const float4*)x, (uint2*)out.p[0], (uint2*)out.p[1], out.scale, out.lo, n4);
     FC_LAUNCHED();
     return FC_OK;
 }
@@ -590,7 +606,7 @@ int launch_gemm_f16(const F16Mat& w, const Planes& x, const float* row_inv, cons
     if (!yp || (epi == EPI_GELU && yp->n != 2) || (w.N & 31) || (ldy & 7) || residual || row_inv || (epi == EPI_GELU && yp->scale == 0.0f) || (yp->scale != 0.0f && yp->n != 2))
         return fail(FC_E_SHAPE, "plane output needs N %% 32 == 0, ldy %% 8 == 0, bf16 planes or two f16 planes (behind GELU these) and no residual");
     for (int p = 0; p < yp->n; ++p) a.yp[p] = (uint16_t*)yp->p[p];
-    a.out_scale = yp->scale; a.out_lift = yp->lift;
+    a.out_scale = yp->scale; a.out_lo = yp->lo;
     return epi == EPI_GELU ? launch_f16<OUT_GELU>(w, x, a, M, st) : launch_f16<OUT_PLANES>(w, x, a, M, st);
 }
 

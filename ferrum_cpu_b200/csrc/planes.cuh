@@ -25,21 +25,20 @@ __device__ __forceinline__ void split2(float v0, float v1, uint32_t (&w)[P]) {
         }
     }
 }
-// Two f32 values -> f16 hi and lo terms: together 2^-23 relative, while the values stay below 65504 and lo above 2^-24. lift: what the
-// pair stands for is v (1 + lift), see Planes.
-__device__ __forceinline__ void split2_f16(float v0, float v1, float lift, uint32_t (&w)[2]) {
+// Two f32 values -> f16 hi, and the remainder times lo: v to 2^-23 of itself or 2^-25 / lo, whichever is more, below 65504.
+__device__ __forceinline__ void split2_f16(float v0, float v1, float lo, uint32_t (&w)[2]) {
     const __half2 h = __floats2half2_rn(v0, v1);
     const float2 hf = __half22float2(h);
-    const __half2 l = __floats2half2_rn(fmaf(v0, lift, v0 - hf.x), fmaf(v1, lift, v1 - hf.y));
+    const __half2 l = __floats2half2_rn((v0 - hf.x) * lo, (v1 - hf.y) * lo);
     w[0] = *(const uint32_t*)&h;
     w[1] = *(const uint32_t*)&l;
 }
-constexpr int F16X2 = -2;   // in the place of a number of planes: two f16 planes of out.scale times the value
+constexpr int F16X2 = -2;   // in the place of a number of planes: two f16 planes of out.scale times the value, the second times out.lo
 template <int P>
 __device__ __forceinline__ void store_planes(const Planes& out, size_t i, float v) {
     constexpr int N = P == F16X2 ? 2 : P;
     uint32_t w[N];
-    if constexpr (P == F16X2) split2_f16(v * out.scale, 0.0f, out.lift, w);
+    if constexpr (P == F16X2) split2_f16(v * out.scale, 0.0f, out.lo, w);
     else split2<P>(v, 0.0f, w);
 #pragma unroll
     for (int p = 0; p < N; ++p) ((uint16_t*)out.p[p])[i] = (uint16_t)w[p];
@@ -49,8 +48,8 @@ __device__ __forceinline__ void store_planes4(const Planes& out, size_t i4, floa
     constexpr int N = P == F16X2 ? 2 : P;
     uint32_t a[N], b[N];
     if constexpr (P == F16X2) {
-        split2_f16(v.x * out.scale, v.y * out.scale, out.lift, a);
-        split2_f16(v.z * out.scale, v.w * out.scale, out.lift, b);
+        split2_f16(v.x * out.scale, v.y * out.scale, out.lo, a);
+        split2_f16(v.z * out.scale, v.w * out.scale, out.lo, b);
     } else {
         split2<P>(v.x, v.y, a);
         split2<P>(v.z, v.w, b);

@@ -195,6 +195,60 @@ __device__ __forceinline__ float ex2(float v) {
     return r;
 }
 
+// Softmax records of W activation rows (columns of a warp's tile), each over the warp's 32 weight rows: v(i) is the lane's logit of column i,
+// of weight row n = n0 + lane (not real: beyond the matrix). rec[c] = (largest, sum of exp(logit - largest), first row that attains it);
+// a target's own logit goes to tlogit. cols: columns that there are, rows of x from m0 on.
+template <int W, class V>
+__device__ __forceinline__ void score_records(V v, int lane, int n0, bool real, int m0, int M, int cols, const int* targets, float* tlogit, float4* rec) {
+    const float kLog2e = 1.4426950408889634f;
+    float e[W], my_max = -INFINITY;
+    int my_idx = 0x7fffffff;
+    const int col = lane & (W - 1);
+    const int tgt = col < cols && m0 + col < M ? __ldg(targets + m0 + col) : -1;
+    const uint32_t hits = __ballot_sync(0xffffffffu, tgt >= n0 && tgt < n0 + 32);
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+        const float x = v(i);
+        const float t = real ? x : -INFINITY;
+        const float mx = redux_max(t);
+        const uint32_t at = __ballot_sync(0xffffffffu, t == mx);
+        e[i] = real ? ex2((x - mx) * kLog2e) : 0.0f;
+        if (col == i) { my_max = mx; my_idx = n0 + __ffs(at) - 1; }
+        if (hits >> i & 1) {                                                 // some lane's row is the target of column i
+            const int tg = __shfl_sync(0xffffffffu, tgt, i);
+            if (n0 + lane == tg) tlogit[m0 + i] = x;
+        }
+    }
+    // transposing sum: W/2 + .. + 1 exchanges leave the lanes that agree in their low bits with parts of the sum of one column
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) {
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const bool up = lane & o;
+            const float keep = up ? e[i + o] : e[i], send = up ? e[i] : e[i + o];
+            e[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (int o = W; o < 32; o <<= 1) e[0] += __shfl_xor_sync(0xffffffffu, e[0], o);
+    if (lane < W && col < cols) rec[lane] = make_float4(my_max, e[0], __int_as_float(my_idx), 0.0f);
+}
+// The records of a column over the four quarters of 128 weight rows, `stride` apart.
+__device__ __forceinline__ float4 merge_records(const float4* rec, int stride) {
+    const float kLog2e = 1.4426950408889634f;
+    float mx = -INFINITY, sum = 0.0f;
+    int idx = 0x7fffffff;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) mx = fmaxf(mx, rec[q * stride].x);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float4 r = rec[q * stride];
+        if (r.x > -INFINITY || r.y != 0.0f) sum += r.y * ex2((r.x - mx) * kLog2e);
+        if (r.x == mx) idx = min(idx, __float_as_int(r.z));
+    }
+    return make_float4(mx, sum, __int_as_float(idx), 0.0f);
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

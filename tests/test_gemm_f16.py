@@ -75,3 +75,47 @@ def test_scales_at_the_ends_of_f16(scales):
     bound = _bound(x, w, k) if max(scales) < 512 else 2.0**-16 * (np.abs(x).astype(np.float64) @ np.abs(w).T)
     assert (np.abs(got - want) <= bound).all()
     qw.close()
+
+
+# stages of 64: the last small terms behind the first ones, one and two groups, a group of one stage
+@pytest.mark.parametrize("k", [192, 256, 384, 448, 640, 704, 1024])
+def test_orders_of_a_tile(k):
+    n, m = 300, 1100
+    raw, w = _weight(n, k, 10)
+    x = np.random.RandomState(11).standard_normal((m, k)).astype(np.float32)
+    qw = fcb.QWeight(raw, n, k)
+    assert (np.abs(_run(qw, x, n) - x.astype(np.float64) @ w.T) <= _bound(x, w, k)).all()
+    qw.close()
+
+
+@pytest.mark.parametrize("k", [128, 1024])
+def test_sums_that_need_no_rounding_are_exact(k):
+    """One element of few bits a row: its product, rounded once. Whole numbers on one scale: their sum."""
+    n, m = 256, 1024
+    raw, w = _weight(n, k, 12)
+    qw = fcb.QWeight(raw, n, k)
+    x = np.zeros((m, k), np.float32)
+    x[np.arange(m), np.arange(m) % k] = 1.375 * 2.0 ** (np.arange(m) % 9 - 4)
+    assert np.array_equal(_run(qw, x, n), (x.astype(np.float64) @ w.T).astype(np.float32))
+    qw.close()
+    raw, w = _weight(n, k, 13, np.array([2.0**-10]))
+    qw = fcb.QWeight(raw, n, k)
+    x = np.random.RandomState(14).randint(-3, 4, (m, k)).astype(np.float32)
+    assert np.array_equal(_run(qw, x, n), x.astype(np.float64) @ w.T)
+    qw.close()
+
+
+@pytest.mark.parametrize("size", [1e4, 1e6, 1e8])
+def test_an_element_that_no_weight_reads(size):
+    """However large it is, the others keep their bits: 2^-36 of the row's scale, which is at most 2^14 / size, is 2^-23 of an element of 1."""
+    n, k, m = 200, 256, 700
+    raw, w = _weight(n, k, 15)
+    raw.reshape(n, k // 32, 34)[:, 2, 2 + 9] = 0
+    w[:, 73] = 0.0
+    x = np.random.RandomState(16).standard_normal((m, k)).astype(np.float32)
+    x[:, 73] = size
+    qw = fcb.QWeight(raw, n, k)
+    got, want = _run(qw, x, n), x.astype(np.float64) @ w.T
+    x[:, 73] = 0.0
+    assert (np.abs(got - want) <= _bound(x, w, k) + 2.0**-36 * size * 2.0**-14 * np.abs(w).sum(1)).all()
+    qw.close()
