@@ -89,7 +89,7 @@ int upload_q8(Arena& ar, const void* host, int N, int K, QMat* out, cudaStream_t
 // A block's matrices as f16 planes and the scales of the activation planes that meet them (gemm_f16.cu).
 struct LayerF16 {
     F16Mat qkv, out, up, down;
-    float n1 = 0.0f, heads = 0.0f, att = 0.0f, n2 = 0.0f, hid = 0.0f;
+    float n1 = 0.0f, heads = 0.0f, att = 0.0f, n2 = 0.0f, hid = 0.0f;   // 0: bf16 planes
 };
 struct LayerDev {
     QMat qkv, out, up, down;
@@ -204,7 +204,7 @@ struct fc_model {
     float* pos = nullptr;
     float *lnfg = nullptr, *lnfb = nullptr;
     std::vector<LayerDev> layers;
-    bool f16 = false;                          // window forwards run on f16 planes: LayerDev::f16, and
+    bool f16 = false;                          // window forwards run on f16 planes where they have a scale: LayerDev::f16, and
     F16Mat head_f16;
     float lnf_scale = 0.0f;
     // prefill workspace for ws_rows rows
@@ -458,66 +458,118 @@ static int model_planes(const fc_model* m) {
     const fc_config& c = m->cfg;
     return c.math_mode == FC_MATH_BF16X3 && c.d_model % 64 == 0 && c.d_ff % 64 == 0 ? 2 : 3;
 }
-// The matrices of a two-plane model as f16 planes, and the scales of the activation planes. A scale is the largest power of two that keeps scale x bound within f16, where the bound holds for every input: a LayerNorm's row has norm at most sqrt(d) max|g| +
+// The matrices of a two-plane model as f16 planes, and the scales of the activation planes that meet them. A scale is the largest power of two
+// that keeps scale x bound within f16, where the bound holds for every input: a LayerNorm's row has norm at most sqrt(d) max|g| +
 // |b|, an element of a product at most the norm of its weight row times that (+ bias), a mixture of value rows and GELU at
-// most what goes into them. The 1 % is for rounding. Without memory for the planes (4 bytes a weight), with a matrix that f16
-// cannot hold or a bound that is not a finite number, the model stays on the level GEMM.
+// most what goes into them. The 1 % is for rounding.
+// One gain, bias or weight row far above the others makes the bound useless to them: what an f16 pair leaves of an element does not shrink
+// with it any more below 2^-13 (planes of products, 2^-36 is lost of a scaled element) or 2^-2 (the attention's, 2^-25). A scale is therefore 0,
+// and its planes stay bf16 (2^-17 of each element), where an element of the usual size of the least gain, bias or row would not keep 2^-17 with
+// some bits to spare: 8 for elements below that size, 4 in the attention. Normal draws of 12 x 768 are 2^20 and 2^13 above the two lines.
+// Without memory for the planes (4 bytes a weight) or with a matrix that f16 cannot hold the whole model stays on the level GEMM.
 static int build_f16(fc_model* m, const fc_weights* w) {
     const fc_config& c = m->cfg;
     const int d = c.d_model, F = c.d_ff;
-    bool ok = m->head.f16_exact;
+    bool held = m->head.f16_exact;
     size_t weights = (size_t)c.vocab * d;
     for (const LayerDev& L : m->layers) {
-        ok = ok && L.qkv.f16_exact && L.out.f16_exact && L.up.f16_exact && L.down.f16_exact;
+        held = held && L.qkv.f16_exact && L.out.f16_exact && L.up.f16_exact && L.down.f16_exact;
         weights += (size_t)4 * d * d + (size_t)2 * d * F;
     }
-    if (!ok) return FC_OK;
+    if (!held) return FC_OK;
     void* mem = nullptr;
-    const size_t tops_at = weights * 4, tops_bytes = (size_t)c.n_layer * 3 * sizeof(unsigned);
-    const cudaError_t e = cudaMalloc(&mem, tops_at + tops_bytes);
+    constexpr int NORMS = 6;                                         // a layer's words: two each of the query and key, the value and the up rows
+    const size_t norms_at = weights * 4, norms_bytes = (size_t)c.n_layer * NORMS * sizeof(unsigned);
+    const cudaError_t e = cudaMalloc(&mem, norms_at + norms_bytes);
     if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); return FC_OK; }
     FC_CUDA(e);
     m->arena.ptrs.push_back(mem);
-    unsigned* tops_d = (unsigned*)((char*)mem + tops_at);
-    FC_CUDA(cudaMemsetAsync(tops_d, 0, tops_bytes, m->st));
+    unsigned* norms_d = (unsigned*)((char*)mem + norms_at);
+    FC_CUDA(cudaMemsetAsync(norms_d, 0, norms_bytes, m->st));
     char* at = (char*)mem;
-    auto make = [&](const QMat& q, F16Mat* f, int from, unsigned* top) -> int {
-        const size_t bytes = (size_t)q.N * q.K * 2;
-        *f = F16Mat{at, at + bytes, q.N, q.K};
-        at += 2 * bytes;
-        return launch_f16_planes(nullptr, 0, 4, Planes(), nullptr, q, *f, from, top, m->st);
+    auto make_rows = [&](const QMat& q, const F16Mat& f, int from, int n, unsigned* norms) -> int {
+        const size_t off = (size_t)from * q.K;
+        QMat part = q;
+        part.qu = q.qu + off; part.d = q.d + off / 32; part.N = n;
+        return launch_f16_planes(nullptr, 0, 4, Planes(), nullptr, part, F16Mat{(__half*)f.hi + off, (__half*)f.lo + off, n, q.K}, norms, m->st);
     };
-    FC_TRY(make(m->head, &m->head_f16, 0, nullptr));
+    auto place = [&](const QMat& q) {
+        const size_t bytes = (size_t)q.N * q.K * 2;
+        const F16Mat f = {at, at + bytes, q.N, q.K};
+        at += 2 * bytes;
+        return f;
+    };
+    auto make = [&](const QMat& q, F16Mat* f, unsigned* norms) { *f = place(q); return make_rows(q, *f, 0, q.N, norms); };
+    FC_TRY(make(m->head, &m->head_f16, nullptr));
     for (int l = 0; l < c.n_layer; ++l) {
         LayerDev& L = m->layers[l];
-        FC_TRY(make(L.qkv, &L.f16.qkv, 0, tops_d + 3 * l));
-        FC_TRY(launch_f16_planes(nullptr, 0, 4, Planes(), nullptr, L.qkv, L.f16.qkv, 2 * d, tops_d + 3 * l + 1, m->st));   // the value rows alone
-        FC_TRY(make(L.out, &L.f16.out, 0, nullptr));
-        FC_TRY(make(L.up, &L.f16.up, 0, tops_d + 3 * l + 2));
-        FC_TRY(make(L.down, &L.f16.down, 0, nullptr));
+        unsigned* nw = norms_d + NORMS * l;
+        L.f16.qkv = place(L.qkv);
+        FC_TRY(make_rows(L.qkv, L.f16.qkv, 0, 2 * d, nw));
+        FC_TRY(make_rows(L.qkv, L.f16.qkv, 2 * d, d, nw + 2));
+        FC_TRY(make(L.out, &L.f16.out, nullptr));
+        FC_TRY(make(L.up, &L.f16.up, nw + 4));
+        FC_TRY(make(L.down, &L.f16.down, nullptr));
     }
-    std::vector<float> tops((size_t)c.n_layer * 3);
-    FC_CUDA(cudaMemcpyAsync(tops.data(), tops_d, tops_bytes, cudaMemcpyDeviceToHost, m->st));
+    std::vector<unsigned> norms((size_t)c.n_layer * NORMS);
+    FC_CUDA(cudaMemcpyAsync(norms.data(), norms_d, norms_bytes, cudaMemcpyDeviceToHost, m->st));
     FC_CUDA(cudaStreamSynchronize(m->st));
-    auto most = [](const float* v, size_t n) { double t = 0; for (size_t i = 0; i < n; ++i) t = v[i] != v[i] ? INFINITY : std::max(t, std::fabs((double)v[i])); return t; };
-    auto norm = [](const float* v, size_t n) { double t = 0; for (size_t i = 0; i < n; ++i) t += (double)v[i] * v[i]; return std::sqrt(t); };
-    auto scale = [&](double bound) -> float {
-        bound *= 1.01;
-        ok = ok && bound < 1e30;                                     // false for NaN too
-        return ok && bound > 0 ? (float)std::exp2(std::min(15.0, std::floor(std::log2(65504.0 / bound)))) : 1.0f;
+    struct Range { double most, least; };                            // of magnitudes; least: of those that are not 0 (infinity: none)
+    auto join = [](Range a, Range b) { return Range{std::max(a.most, b.most), std::min(a.least, b.least)}; };
+    auto range = [](const float* v, size_t n) {
+        Range r = {0.0, INFINITY};
+        for (size_t i = 0; i < n; ++i) {
+            const double a = v[i] != v[i] ? INFINITY : std::fabs((double)v[i]);
+            r.most = std::max(r.most, a);
+            if (a > 0) r.least = std::min(r.least, a);
+        }
+        return r;
     };
+    auto rows = [](const unsigned* words) {
+        float sq[2];
+        const unsigned bits[2] = {words[0], ~words[1]};
+        memcpy(sq, bits, sizeof(sq));
+        return words[0] ? Range{std::sqrt((double)sq[0]), std::sqrt((double)sq[1])} : Range{0.0, INFINITY};
+    };
+    auto norm = [](const float* v, size_t n) { double t = 0; for (size_t i = 0; i < n; ++i) t += (double)v[i] * v[i]; return std::sqrt(t); };
+    // What a LayerNorm leaves: elements of at most `most`, usually of `least` or more, in a row of norm `all`.
+    struct Normed { double most, least, all; };
     const double root = std::sqrt((double)d);
+    auto normed = [&](const float* g, const float* b) {
+        const Range rg = range(g, d), rb = range(b, d);
+        Normed r = {root * rg.most + rb.most, INFINITY, root * rg.most + norm(b, d)};
+        for (int i = 0; i < d; ++i) {
+            const double usual = std::max(std::fabs((double)g[i]), std::fabs((double)b[i]));
+            if (usual > 0) r.least = std::min(r.least, usual);
+        }
+        return r;
+    };
+    auto scale = [](double bound, double least, int floor_log2) -> float {
+        bound *= 1.01;
+        if (!(bound < 1e30)) return 0.0f;                            // NaN too
+        const double s = bound > 0 ? std::exp2(std::min(15.0, std::floor(std::log2(65504.0 / bound)))) : 1.0;
+        return s * least >= std::exp2((double)floor_log2) ? (float)s : 0.0f;
+    };
+    constexpr int PRODUCT = -36 + 17 + 8, HEADS = -25 + 17 + 4;
+    bool any = false;
     for (int l = 0; l < c.n_layer; ++l) {
         const fc_layer_weights& s = w->layers[l];
         LayerF16& f = m->layers[l].f16;
-        f.n1 = scale(root * most(s.ln1_g, d) + most(s.ln1_b, d));
-        f.n2 = scale(root * most(s.ln2_g, d) + most(s.ln2_b, d));
-        f.heads = scale(std::sqrt((double)tops[3 * l]) * (root * most(s.ln1_g, d) + norm(s.ln1_b, d)) + most(s.attn_qkv_b, 3 * (size_t)d));
-        f.att = scale(std::sqrt((double)tops[3 * l + 1]) * (root * most(s.ln1_g, d) + norm(s.ln1_b, d)) + most(s.attn_qkv_b + 2 * d, d));
-        f.hid = scale(std::sqrt((double)tops[3 * l + 2]) * (root * most(s.ln2_g, d) + norm(s.ln2_b, d)) + most(s.ffn_up_b, F));
+        const Normed n1 = normed(s.ln1_g, s.ln1_b), n2 = normed(s.ln2_g, s.ln2_b);
+        const unsigned* nw = &norms[(size_t)NORMS * l];
+        const Range v = rows(nw + 2), heads = join(rows(nw), v), up = rows(nw + 4);
+        f.n1 = scale(n1.most, n1.least, PRODUCT);
+        f.n2 = scale(n2.most, n2.least, PRODUCT);
+        f.heads = scale(heads.most * n1.all + range(s.attn_qkv_b, 3 * (size_t)d).most, heads.least * n1.least, HEADS);
+        f.att = scale(v.most * n1.all + range(s.attn_qkv_b + 2 * d, d).most, v.least * n1.least, PRODUCT);
+        f.hid = scale(up.most * n2.all + range(s.ffn_up_b, F).most, up.least * n2.least, PRODUCT);
+        if (f.n1 == 0.0f) f.heads = 0.0f;                            // the level GEMM writes bf16 planes
+        if (f.n2 == 0.0f || f.hid == 0.0f) f.n2 = f.hid = 0.0f;      // each GEMM's GELU leaves planes of its own kind
+        any = any || f.n1 != 0.0f || f.att != 0.0f || f.n2 != 0.0f;
     }
-    m->lnf_scale = scale(root * most(w->out_norm_g, d) + most(w->out_norm_b, d));
-    m->f16 = ok;
+    const Normed nf = normed(w->out_norm_g, w->out_norm_b);
+    m->lnf_scale = scale(nf.most, nf.least, PRODUCT);
+    m->f16 = any || m->lnf_scale != 0.0f;
     return FC_OK;
 }
 // Whether the window attention runs on the tensor cores (heads of 64).
@@ -568,16 +620,15 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
     const int d = c.d_model, F = c.d_ff;
     cudaStream_t st = m->st;
     const bool tc_attn = tensor_attention(m);
-    // f16 planes in the two-plane mode (never in the f32 mode: two of them are a bit short of an f32), unless a few rows are better off where K is
-    // split over CTAs (prompts of 64 / 101 / 250 ids, 12 x 768: 1014 / 1033 / 1120 us on them, 932 / 1207 / 1469 split; 24 x 1024: 2273 / 2315 /
-    // 2506 and 2235 / 2449 / 3123)
-    const bool f16 = m->f16 && planes == 2 && (!split_k || R > 64);
+    // f16 planes in the two-plane mode, where they have a scale (never in the f32 mode: two of them are a bit short of an f32)
+    const bool f16 = m->f16 && planes == 2;
     m->pqkv.n = m->pn.n = m->patt.n = m->phid.n = planes;
     m->pqkv.lo = 1.0f;                                               // the attention adds both planes' products in one place
     auto product = [&](const QMat& q, const F16Mat& h, const Planes& x, const float* bias, const float* residual, int epi, float* y, const Planes* yp) {
-        return f16 ? launch_gemm_f16(h, x, nullptr, bias, residual, epi, y, yp, R, q.N, status, st)
-                   : launch_gemm_q8_tc(q, x, bias, residual, epi, y, yp, R, q.N, status, st, split_k);
+        return x.scale != 0.0f ? launch_gemm_f16(h, x, nullptr, bias, residual, epi, y, yp, R, q.N, status, st)
+                               : launch_gemm_q8_tc(q, x, bias, residual, epi, y, yp, R, q.N, status, st, split_k);
     };
+    auto split = [&](const float* x, const Planes& out, size_t n) { return out.scale != 0.0f ? launch_split_f16(x, out, n, st) : launch_split_planes(x, out, n, st); };
     FC_CUDA(cudaMemsetAsync(m->err_d, 0, sizeof(int), st));
     FC_TRY(launch_embed_rows(m->tok, m->pos, ids, pos, R, win.T, m->x, m->err_d, st));
     // model.rs:58-68: with the statistics switched on, every layer's output is summarised as it appears
@@ -599,13 +650,13 @@ static int forward_blocks_with(fc_model* m, const Windows& win, int R, const int
         } else {
             FC_TRY(product(L.qkv, L.f16.qkv, m->pn, L.qkv_b, nullptr, EPI_NONE, m->qkv, nullptr));
             FC_TRY(on_qkv(l));
-            if (tc_attn) FC_TRY(f16 ? launch_split_f16(m->qkv, m->pqkv, (size_t)R * 3 * d, st) : launch_split_planes(m->qkv, m->pqkv, (size_t)R * 3 * d, st));
+            if (tc_attn) FC_TRY(split(m->qkv, m->pqkv, (size_t)R * 3 * d));
         }
         if (tc_attn) {
             FC_TRY(launch_attn_prefill_tc(m->pqkv, win, R, d, c.n_head, m->patt, status, st));
         } else {
             FC_TRY(launch_attn_prefill(m->qkv, win, d, c.n_head, m->att, st));
-            FC_TRY(f16 ? launch_split_f16(m->att, m->patt, (size_t)R * d, st) : launch_split_planes(m->att, m->patt, (size_t)R * d, st));
+            FC_TRY(split(m->att, m->patt, (size_t)R * d));
         }
         FC_TRY(product(L.out, L.f16.out, m->patt, L.out_b, m->x, EPI_NONE, m->x, nullptr));
         m->pn.scale = f16 ? L.f16.n2 : 0.0f;
@@ -622,7 +673,7 @@ static int score_device(fc_model* m, const ScoreSlot& s, const Windows& win, int
     const int d = c.d_model, n = s.picked;
     const int *ids = (const int*)s.in_d, *pos = ids + R, *pick = pos + R + win.B + 1, *targets = pick + n;
     FC_TRY(forward_blocks_with(m, win, R, ids, pos, model_planes(m), s.status_d(), false, false, [](int) { return FC_OK; }));
-    const bool f16 = m->f16;
+    const bool f16 = m->f16 && m->lnf_scale != 0.0f;
     m->pn.n = model_planes(m);
     m->pn.scale = 0.0f;
     if (m->stats_on) {
@@ -632,9 +683,7 @@ static int score_device(fc_model* m, const ScoreSlot& s, const Windows& win, int
     if (n == 0) return FC_OK;               // the forward was for its statistics
     // the head's epilogue keeps (max, sum of exponentials, first argmax) per row and 128-column tile and the
     // target's logit: [rows][V] logits never reach memory (scoring.rs:175-181 needs one number per row)
-    if (f16) {
-        m->pn.scale = m->lnf_scale;
-    }
+    if (f16) m->pn.scale = m->lnf_scale;
     FC_TRY(launch_layernorm_planes(m->x, m->lnfg, m->lnfb, n == R ? nullptr : pick, n, d, m->pn, m->st));
     if (f16) FC_TRY(launch_gemm_f16_score(m->head_f16, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
     else FC_TRY(launch_gemm_q8_tc_score(m->head, m->pn, targets, m->head_stats, m->head_tlogit, n, s.status_d(), m->st));
@@ -725,7 +774,7 @@ int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bia
             p += 2 * nw;
             x.p[0] = p; x.p[1] = p + n; x.n = 2; x.scale = 1.0f;
             float* row_inv = (float*)(p + 2 * n);
-            FC_TRY(launch_f16_planes(x_dev, M, w->w.K, x, row_inv, w->w, wp, 0, nullptr, st));
+            FC_TRY(launch_f16_planes(x_dev, M, w->w.K, x, row_inv, w->w, wp, nullptr, st));
             return launch_gemm_f16(wp, x, row_inv, bias_dev, nullptr, EPI_NONE, y_dev, nullptr, M, w->w.N, w->status.dev, st);
         }
     }

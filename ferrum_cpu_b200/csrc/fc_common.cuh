@@ -267,8 +267,8 @@ int launch_gemm_f16(const F16Mat& w, const Planes& x, const float* row_inv, cons
                     int M, int ldy, int* status, cudaStream_t st);
 int launch_gemm_f16_score(const F16Mat& w, const Planes& x, const int* targets, void* stats, float* tlogit, int M, int* status, cudaStream_t st);
 // x [M][K] as f16 planes scaled row by row (row_inv [M]: 1 / scale) and w as exact f16 planes, in one launch; either may be empty.
-// top (may be null): raised to the bits of the largest square norm of the weight rows from `from` on (finite and positive).
-int launch_f16_planes(const float* x, int M, int K, const Planes& out /* its scale does not count */, float* row_inv, const QMat& w, const F16Mat& planes, int from, unsigned* top,
+// norms (null, or two zeroed words): the bits of the largest square norm of a weight row, and the complement of those of the smallest but 0.
+int launch_f16_planes(const float* x, int M, int K, const Planes& out /* its scale does not count */, float* row_inv, const QMat& w, const F16Mat& planes, unsigned* norms,
                       cudaStream_t st);
 // Whether a caller's own two-plane product of M rows is better off there.
 bool f16_rows(int K, int M);

@@ -399,11 +399,11 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap wh, const __grid_constant__ 
 }
 
 // Rows of x as f16 planes, each scaled by a power of two that brings its largest element into [2^14, 2^15), and rows of a Q8_0
-// matrix as exact f16 planes; a warp per row. top (null or a zeroed word): bits of the largest square norm among the weight rows from
-// `from` on.
+// matrix as exact f16 planes; a warp per row. norms: null, or two zeroed words: bits of the largest square norm of a weight row, and the
+// complement of the bits of the smallest that is not 0.
 __global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict__ x, int M, int K, __half* __restrict__ xh, __half* __restrict__ xl,
                                                          float* __restrict__ row_inv, const QMat w, __half* __restrict__ wh,
-                                                         __half* __restrict__ wl, int from, unsigned* __restrict__ top) {
+                                                         __half* __restrict__ wl, unsigned* __restrict__ norms) {
     constexpr int HELD = 8;
     pdl_trigger();
     const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict
             const __half2 h = __hmul2(lv, d2), r = __hmul2(__hfma2(lv, d2, __hneg2(h)), __float2half2_rn(kRest));   // the rounding's remainder, exactly
             hi[i] = *(const uint32_t*)&h;
             lo[i] = *(const uint32_t*)&r;
-            if (top) {
+            if (norms) {
                 const float2 f = __half22float2(h);
                 norm = fmaf(f.x, f.x, fmaf(f.y, f.y, norm));
             }
@@ -468,10 +468,13 @@ __global__ void __launch_bounds__(256) f16_planes_kernel(const float* __restrict
         pl[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         pl[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
     }
-    if (top && n >= from) {
+    if (norms) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) norm += __shfl_xor_sync(0xffffffffu, norm, o);
-        if (lane == 0) atomicMax(top, __float_as_uint(norm));                          // squares: the order of the bits is theirs
+        if (lane == 0 && norm > 0.0f) {                                                // squares: the order of the bits is theirs
+            atomicMax(norms, __float_as_uint(norm));
+            atomicMax(norms + 1, ~__float_as_uint(norm));
+        }
     }
 }
 
@@ -579,11 +582,10 @@ int launch_f16(const F16Mat& w, const Planes& x, F16Args a, int M, cudaStream_t 
 // 32.3 (26.8), 1024 rows 33.0 (37.2), 1536 rows 43.6 (49.3); N = 4096: 512 rows 53.7 (47.4), 1024 rows 82 (81), 1536 rows 103 (119).
 bool f16_rows(int K, int M) { return M >= 512 && M >= K / 2; }
 
-int launch_f16_planes(const float* x, int M, int K, const Planes& out, float* row_inv, const QMat& w, const F16Mat& planes, int from, unsigned* top,
-                      cudaStream_t st) {
+int launch_f16_planes(const float* x, int M, int K, const Planes& out, float* row_inv, const QMat& w, const F16Mat& planes, unsigned* norms, cudaStream_t st) {
     if (K % 4 || w.K % 16) return fail(FC_E_SHAPE, "f16 planes: row lengths %d, %d", K, w.K);
     f16_planes_kernel<<<(M + w.N + 7) / 8, 256, 0, st>>>(x, M, K, (__half*)out.p[0], (__half*)out.p[1], row_inv, w, (__half*)planes.hi, (__half*)planes.lo,
-                                                         from, top);
+                                                         norms);
     FC_LAUNCHED();
     return FC_OK;
 }

@@ -206,7 +206,7 @@ int fc_q8_0_linear_dev_noalloc(const fc_qweight* w, const float* x_dev, const fl
 
 /* ---- model ------------------------------------------------------------------------ */
 /* Validates as loader/gpt2.rs + loader/mod.rs:147-154 (d % n_head == 0, K % 32 == 0),
- * uploads and repacks the weights on `device`. Models in FC_MATH_BF16X3, and those of width 512 and more, also keep their
+ * uploads and repacks the weights on `device`. Models in FC_MATH_BF16X3 also keep their
  * matrices as f16 planes for window forwards (4 bytes a weight), unless there is no memory for them. */
 int fc_model_create(const fc_config* cfg, const fc_weights* w, int device, fc_model** out);
 /* The same from a GGUF file, without the f32 expansion of the matrices (the direct path the

@@ -51,3 +51,15 @@ def test_f32_mode_holds_every_element(where):
     ids = synth.token_ids(1, 3 * 64, 515).reshape(3, 64)
     plain, wide = (_logprobs(_spread(512, 8, 2048, where, size, fcb.FC_MATH_FP32), ids) for size in (0.0, 1e8))
     assert np.array_equal(plain, wide)
+
+
+@pytest.mark.parametrize("size", [0.0, 1e4, 1e6, 1e8, 1e12])
+@pytest.mark.parametrize("where", PLACES)
+def test_two_plane_mode_keeps_its_precision(where, size):
+    """Activations to 2^-17 of each element (f16 planes hold more, where a scale of all elements allows it) behind whatever nobody reads. An element
+    is off by 2^-17 / sqrt(3) at random, so is a logit (they have a size of 1/2), nine products in a row add up to 3 times that, and 4.5 times
+    it is what 192 rows show; behind f16 planes alone 1e12 is off by 0.2."""
+    ids = synth.token_ids(1, 3 * 64, 515).reshape(3, 64)
+    want = _logprobs(_spread(512, 8, 2048, where, 0.0, fcb.FC_MATH_FP32), ids)
+    got = _logprobs(_spread(512, 8, 2048, where, size, fcb.FC_MATH_BF16X3), ids)
+    assert np.abs(got - want).max() < 4.5 * 3 * 2.0**-17 / np.sqrt(3) / 2
