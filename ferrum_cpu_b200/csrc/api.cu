@@ -200,6 +200,7 @@ struct fc_model {
     cudaStream_t st = nullptr;
     Arena arena;       // weights
     Arena ws_arena;    // prefill workspace
+    Arena f16_arena;   // the weights as f16 planes, given back when anything else of the model finds no memory
     QMat tok, head;
     float* pos = nullptr;
     float *lnfg = nullptr, *lnfb = nullptr;
@@ -466,7 +467,9 @@ static int model_planes(const fc_model* m) {
 // with it any more below 2^-13 (planes of products, 2^-36 is lost of a scaled element) or 2^-2 (the attention's, 2^-25). A scale is therefore 0,
 // and its planes stay bf16 (2^-17 of each element), where an element of the usual size of the least gain, bias or row would not keep 2^-17 with
 // some bits to spare: 8 for elements below that size, 4 in the attention. Normal draws of 12 x 768 are 2^20 and 2^13 above the two lines.
-// Without memory for the planes (4 bytes a weight) or with a matrix that f16 cannot hold the whole model stays on the level GEMM.
+// With a matrix that f16 cannot hold the whole model stays on the level GEMM, and so it does where the planes (4 bytes a weight) would take
+// more than a quarter of the free memory: three times as much stays free for caches, workspaces and other models, which did with 1.06 bytes a weight
+// before there were planes.
 static int build_f16(fc_model* m, const fc_weights* w) {
     const fc_config& c = m->cfg;
     const int d = c.d_model, F = c.d_ff;
@@ -480,10 +483,13 @@ static int build_f16(fc_model* m, const fc_weights* w) {
     void* mem = nullptr;
     constexpr int NORMS = 6;                                         // a layer's words: two each of the query and key, the value and the up rows
     const size_t norms_at = weights * 4, norms_bytes = (size_t)c.n_layer * NORMS * sizeof(unsigned);
+    size_t free_bytes = 0, total_bytes = 0;
+    FC_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+    if (norms_at + norms_bytes > free_bytes / 4) return FC_OK;
     const cudaError_t e = cudaMalloc(&mem, norms_at + norms_bytes);
     if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); return FC_OK; }
     FC_CUDA(e);
-    m->arena.ptrs.push_back(mem);
+    m->f16_arena.ptrs.push_back(mem);
     unsigned* norms_d = (unsigned*)((char*)mem + norms_at);
     FC_CUDA(cudaMemsetAsync(norms_d, 0, norms_bytes, m->st));
     char* at = (char*)mem;
@@ -570,16 +576,25 @@ static int build_f16(fc_model* m, const fc_weights* w) {
     const Normed nf = normed(w->out_norm_g, w->out_norm_b);
     m->lnf_scale = scale(nf.most, nf.least, PRODUCT);
     m->f16 = any || m->lnf_scale != 0.0f;
+    if (!m->f16) m->f16_arena.release();
     return FC_OK;
+}
+// What a model allocates besides. Where there is no memory the planes are given back, and it is tried again: whoever had room for a stream,
+// a workspace or a batch without them has it with them. `make` leaves nothing behind when it fails.
+template <class Make>
+static int with_room(fc_model* m, Make make) {
+    const bool starved = m->f16 && g_debug.withhold_scratch == 2;
+    const int rc = starved ? fail(FC_E_CUDA, "no memory (test hook)") : make();
+    if (rc == FC_OK || !m->f16 || !(starved || cudaGetLastError() == cudaErrorMemoryAllocation)) return rc;
+    FC_CUDA(cudaStreamSynchronize(m->st));
+    m->f16 = false;
+    m->f16_arena.release();
+    return make();
 }
 // Whether the window attention runs on the tensor cores (heads of 64).
 static bool tensor_attention(const fc_model* m) { return m->cfg.d_model == m->cfg.n_head * 64; }
 
-static int ensure_workspace(fc_model* m, int rows, int planes) {
-    if (rows <= m->ws_rows && planes <= m->ws_planes) return FC_OK;
-    rows = std::max(rows, m->ws_rows);
-    planes = std::max(planes, m->ws_planes);
-    FC_CUDA(cudaStreamSynchronize(m->st));
+static int make_workspace(fc_model* m, int rows, int planes) {
     m->ws_arena.release();
     m->ws_rows = m->ws_planes = 0;
     const fc_config& c = m->cfg;
@@ -607,6 +622,13 @@ static int ensure_workspace(fc_model* m, int rows, int planes) {
     m->ws_rows = rows;
     m->ws_planes = planes;
     return FC_OK;
+}
+static int ensure_workspace(fc_model* m, int rows, int planes) {
+    if (rows <= m->ws_rows && planes <= m->ws_planes) return FC_OK;
+    rows = std::max(rows, m->ws_rows);
+    planes = std::max(planes, m->ws_planes);
+    FC_CUDA(cudaStreamSynchronize(m->st));
+    return with_room(m, [&] { return make_workspace(m, rows, planes); });
 }
 
 // Sequential::forward (model.rs:51-71) through every block, on the R rows of `win` (device arrays: their ids, and their
@@ -842,7 +864,6 @@ static int model_build(fc_model* m, const fc_weights* w) {
         FC_TRY(upload_f32(a, s.ln2_g, d, &L.ln2g, st));
         FC_TRY(upload_f32(a, s.ln2_b, d, &L.ln2b, st));
     }
-    if (model_planes(m) == 2) FC_TRY(build_f16(m, w));
     if (mega_supported(c)) {
         int full = 0;
         FC_TRY(mega_max_grid(&full));
@@ -915,6 +936,7 @@ static int model_build(fc_model* m, const fc_weights* w) {
         }
         if (!m->mega_tables.empty()) m->mega_grid = m->mega_tables[0].grid;
     }
+    if (model_planes(m) == 2) FC_TRY(build_f16(m, w));            // last: out of what the model's own tables leave
     FC_CUDA(cudaStreamSynchronize(st));
     return FC_OK;
 }
@@ -956,6 +978,7 @@ void fc_model_free(fc_model* m) {
     m->pool.clear();
     m->arena.release();
     m->ws_arena.release();
+    m->f16_arena.release();
     for (ScoreSlot& s : m->slot) s.release();
     if (m->batch.graph) cudaGraphExecDestroy(m->batch.graph);
     if (m->batch.graph4) cudaGraphExecDestroy(m->batch.graph4);
@@ -1233,10 +1256,7 @@ int fc_predict_next(fc_model* m, const int32_t* ids, int n, float* probs) {
 }
 
 // ----------------------------------------------------------------------------- streams
-int fc_stream_create(fc_model* m, fc_stream** out) {
-    if (!m || !out) return fail(FC_E_ARG, "fc_stream_create: null argument");
-    *out = nullptr;
-    FC_CUDA(cudaSetDevice(m->device));
+static int stream_create(fc_model* m, fc_stream** out) {
     const fc_config& c = m->cfg;
     fc_stream* s = new fc_stream;
     s->m = m;
@@ -1278,6 +1298,12 @@ int fc_stream_create(fc_model* m, fc_stream** out) {
     if (rc != FC_OK) { fc_stream_free(s); return rc; }
     *out = s;
     return FC_OK;
+}
+int fc_stream_create(fc_model* m, fc_stream** out) {
+    if (!m || !out) return fail(FC_E_ARG, "fc_stream_create: null argument");
+    *out = nullptr;
+    FC_CUDA(cudaSetDevice(m->device));
+    return with_room(m, [&] { return stream_create(m, out); });
 }
 
 void fc_stream_free(fc_stream* s) {
@@ -1929,8 +1955,8 @@ int fc_decode_batch(fc_model* m, int n_streams, const int32_t* prompts, int prom
         return FC_OK;
     }
     FC_TRY(check_ids(m, prompts, (size_t)n_streams * prompt_len));
-    FC_TRY(batch_make_frags(m));
-    FC_TRY(batch_ensure(m, std::min(n_streams, kBatchMaxStreams), max_new));
+    FC_TRY(with_room(m, [&] { return batch_make_frags(m); }));
+    FC_TRY(with_room(m, [&] { return batch_ensure(m, std::min(n_streams, kBatchMaxStreams), max_new); }));
     BatchCtx& b = m->batch;
     cudaStream_t st = m->st;
     FC_CUDA(cudaEventRecord(m->ev0, st));
@@ -2074,7 +2100,7 @@ int fc_decode_batch_multi(fc_model* const* models, int n_models, int n_streams, 
 }
 
 int fc_debug_withhold_scratch(int on) {
-    g_debug.withhold_scratch = on != 0;
+    g_debug.withhold_scratch = on == 2 ? 2 : on != 0;
     return FC_OK;
 }
 

@@ -46,7 +46,7 @@ inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 struct DebugKnobs {
     long long wait_cycles = 4000000000LL;   // ~2 s at 1.9 GHz
     int withhold = 0;
-    int withhold_scratch = 0;               // CallScratch finds no memory
+    int withhold_scratch = 0;               // 1: CallScratch finds no memory; 2: a model that holds f16 planes finds none for anything else
 };
 extern DebugKnobs g_debug;
 

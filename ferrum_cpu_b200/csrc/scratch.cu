@@ -53,7 +53,7 @@ void scratch_release(int device) {
 
 int CallScratch::take(int device, size_t bytes, cudaStream_t st) {
     st_ = st;
-    if (g_debug.withhold_scratch) return FC_OK;
+    if (g_debug.withhold_scratch == 1) return FC_OK;
     const cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, g_pools[device].pool, st);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();

@@ -207,7 +207,9 @@ int fc_q8_0_linear_dev_noalloc(const fc_qweight* w, const float* x_dev, const fl
 /* ---- model ------------------------------------------------------------------------ */
 /* Validates as loader/gpt2.rs + loader/mod.rs:147-154 (d % n_head == 0, K % 32 == 0),
  * uploads and repacks the weights on `device`. Models in FC_MATH_BF16X3 also keep their
- * matrices as f16 planes for window forwards (4 bytes a weight), unless there is no memory for them. */
+ * matrices as f16 planes for window forwards (4 bytes a weight), where that takes at most a quarter of the device's free memory. They are
+ * given back when a workspace, a stream or a batch of the model finds no memory; window forwards then run as where there never were any,
+ * on two bf16 planes. */
 int fc_model_create(const fc_config* cfg, const fc_weights* w, int device, fc_model** out);
 /* The same from a GGUF file, without the f32 expansion of the matrices (the direct path the
  * reference names as future work, loader/decode.rs:99-100). Reads a gpt2-architecture GGUF
@@ -523,7 +525,8 @@ float fc_last_score_ms(const fc_model* m);
  * Nothing faults, traps or waits without a limit. Not for production use: restore
  * (4000000000, 0) afterwards. */
 int fc_debug_set_wait_budget(long long cycles, int withhold_producers);
-/* With on != 0 the products on callers' streams find no memory for their scratch (restore with 0). */
+/* With 1 the products on callers' streams find no memory for their scratch, with 2 a model that holds f16 planes finds none for a
+ * workspace, a stream or a batch (restore with 0). */
 int fc_debug_withhold_scratch(int on);
 
 #ifdef __cplusplus

@@ -1,10 +1,12 @@
 """Window forwards of models whose activations have parts far apart in size. An element that no weight reads (its column of levels is
 zero) or that GELU turns into zero leaves the function as it is, whatever its size: only what the products hold of the others may change."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import ferrum_cpu_b200 as fcb
-from ferrum_cpu_b200 import synth
+from ferrum_cpu_b200 import _lib, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -63,3 +65,31 @@ def test_two_plane_mode_keeps_its_precision(where, size):
     want = _logprobs(_spread(512, 8, 2048, where, 0.0, fcb.FC_MATH_FP32), ids)
     got = _logprobs(_spread(512, 8, 2048, where, size, fcb.FC_MATH_BF16X3), ids)
     assert np.abs(got - want).max() < 4.5 * 3 * 2.0**-17 / np.sqrt(3) / 2
+
+
+def test_planes_make_room():
+    """A workspace, a stream or a batch that finds no memory gets that of the f16 planes; forwards go on without them."""
+    ids = synth.token_ids(1, 4 * 64, 515).reshape(4, 64)
+    sm = _spread(512, 8, 2048, "ln1_b", 0.0, fcb.FC_MATH_BF16X3)
+    want = _logprobs(_spread(512, 8, 2048, "ln1_b", 0.0, fcb.FC_MATH_FP32), ids)
+
+    def stream(gm):
+        s = C.c_void_p()
+        _lib.check(_lib.lib().fc_stream_create(gm._m, C.byref(s)))
+        _lib.lib().fc_stream_free(s)
+
+    uses = [lambda gm: gm.score_sequences(ids), stream, lambda gm: gm.decode_batch(ids[:, :4], 3)]
+    left = []
+    for use in uses:
+        gm = fcb.CudaSlm(sm.config, sm.weights)
+        few = gm.score_sequences(ids[:1])[1]
+        _lib.check(_lib.lib().fc_debug_withhold_scratch(2))
+        try:
+            use(gm)
+        finally:
+            _lib.check(_lib.lib().fc_debug_withhold_scratch(0))
+        left.append(gm.score_sequences(ids)[1])
+        assert not np.array_equal(left[-1][:1], few)             # no longer on f16 planes
+        gm.close()
+    assert all(np.array_equal(lp, left[0]) for lp in left[1:])
+    assert np.abs(left[0] - want).max() < 4.5 * 3 * 2.0**-17 / np.sqrt(3) / 2
