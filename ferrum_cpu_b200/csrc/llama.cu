@@ -570,6 +570,13 @@ int read_state(fc_llama_cache* s, StepState* out) {
     return FC_OK;
 }
 
+// What a step that failed on the device comes to. Nothing behind it advanced: the cache ends where the state does.
+int step_error(fc_llama_cache* s, const StepState& hs) {
+    if (!hs.error) return FC_OK;
+    s->host_pos = std::min(s->host_pos, hs.pos);
+    return fail(hs.error, hs.error == FC_E_TIMEOUT ? "a bounded wait inside a decode step ran out" : "the decode step rejected a token or position on the device");
+}
+
 // Queues ids behind what the queue holds and feeds them; the last one with the head when asked.
 int feed_ids(fc_llama_cache* s, const int32_t* ids, int n, int head_on_last) {
     fc_llama* m = s->m;
@@ -950,8 +957,7 @@ int fc_llama_forward_one(fc_llama_cache* s, int32_t token, float* logits) {
     if (logits) FC_CUDA(cudaMemcpyAsync(logits, s->logits, (size_t)m->cfg.vocab * 4, cudaMemcpyDeviceToHost, m->st));
     StepState hs;
     FC_TRY(read_state(s, &hs));
-    if (hs.error) { s->host_pos -= 1; return fail(hs.error, "the decode step rejected a token or position on the device"); }
-    return FC_OK;
+    return step_error(s, hs);
 }
 
 int fc_llama_prime(fc_llama_cache* s, const int32_t* ids, int n, float* logits) {
@@ -966,8 +972,7 @@ int fc_llama_prime(fc_llama_cache* s, const int32_t* ids, int n, float* logits) 
     if (logits) FC_CUDA(cudaMemcpyAsync(logits, s->logits, (size_t)m->cfg.vocab * 4, cudaMemcpyDeviceToHost, m->st));
     StepState hs;
     FC_TRY(read_state(s, &hs));
-    if (hs.error) return fail(hs.error, "the decode step rejected a token or position on the device");
-    return FC_OK;
+    return step_error(s, hs);
 }
 
 int fc_llama_generate(fc_llama_cache* s, const int32_t* prompt, int n, int max_new, const fc_sampling* params,
@@ -1035,7 +1040,7 @@ int fc_llama_generate(fc_llama_cache* s, const int32_t* prompt, int n, int max_n
         if (free_run && made > 0) FC_CUDA(cudaMemcpyAsync(out, s->queue + n, (size_t)made * 4, cudaMemcpyDeviceToHost, st));
         StepState hs;
         rc = read_state(s, &hs);
-        if (rc == FC_OK && hs.error) rc = fail(hs.error, "the decode step rejected a token or position on the device");
+        if (rc == FC_OK) rc = step_error(s, hs);
         if (rc == FC_OK) FC_CUDA(cudaEventElapsedTime(&s->last_decode_ms, s->ev0, s->ev1));
     }
     FC_CUDA(cudaMemcpy(rng_state, s->rng_d, 8, cudaMemcpyDeviceToHost));

@@ -168,3 +168,35 @@ def test_llama_steps_past_the_held_rows():
         if t % 97 == 0 or t > 1290:
             assert np.abs(got - want).max() < 2e-4, t
     gm.close()
+
+
+@pytest.mark.parametrize("prec", [None, 0])
+@pytest.mark.parametrize("what", ["forward_one", "prime", "generate"])
+def test_a_llama_wait_that_runs_out_feeds_nothing(what, prec):
+    """The row never comes: the call says so, the cache ends where its last whole step left it, and goes on from there."""
+    sm = synth.SynthLlama(515, 512, 2, 8, 2, 64, 2048, 64, seed=5, perturb=True)
+    om, gm = O.OracleLlama(sm, threads=4, **({} if prec is None else {"prec": prec})), CudaLlama.from_synth(sm, prec=prec)
+    cache = gm.new_cache()
+    ids = [3, 11, 5]
+    om.clear()
+    for t in ids:
+        gm.forward_one(t, cache), om.forward_one(t)
+    greedy = _lib.FcSampling(0.0, 0, 1.0, 1.0)
+    gm.generate(ids, 12, greedy, cache=cache)               # with graphs of every kind
+    gm.prime(ids, cache)
+    calls = {"forward_one": lambda: gm.forward_one(7, cache), "prime": lambda: gm.prime(ids, cache), "generate": lambda: gm.generate(ids, 12, greedy, cache=cache)}
+    _lib.check(_lib.lib().fc_debug_set_wait_budget(200000, 1))
+    try:
+        with pytest.raises(fcb.FerrumCudaError) as e:
+            calls[what]()
+    finally:
+        _lib.check(_lib.lib().fc_debug_set_wait_budget(4000000000, 0))
+    assert e.value.code == _lib.FC_E_TIMEOUT and "wait" in str(e.value)
+    assert cache.pos() == (3 if what == "forward_one" else 0)
+    if what != "forward_one":
+        for t in ids:
+            gm.forward_one(t, cache)
+    got, want = gm.forward_one(7, cache), om.forward_one(7)
+    assert np.abs(got - want).max() < 2e-4 * max(1.0, float(np.abs(want).max()))
+    gm.close()
+    om.close()
