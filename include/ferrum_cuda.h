@@ -173,8 +173,9 @@ void fc_qweight_free(fc_qweight* w);
 int fc_q8_0_linear_dev(const fc_qweight* w, const float* x_dev, const float* bias_dev, float* y_dev,
                        int M, int math_mode, void* cuda_stream);
 
-/* The same product as fc_q8_0_linear_dev in FC_MATH_BF16X3, for callers that must not
- * allocate device memory. No counterpart in the reference (it never leaves the host heap).
+/* The product of fc_q8_0_linear_dev in FC_MATH_BF16X3 on two bf16 planes, for callers that must not
+ * allocate device memory: bit for bit the same below 512 or K / 2 rows, and to the mode's 2^-17 of an activation from there on,
+ * where that entry takes f16 planes. No counterpart in the reference (it never leaves the host heap).
  *
  * Who needs it: a serving loop that handed all free device memory to its own pool at
  * start-up, so a cudaMalloc inside the library would fail; or a latency-critical thread that

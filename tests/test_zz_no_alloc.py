@@ -4,8 +4,9 @@ Some hosts of this library cannot call cudaMalloc while they serve: all free dev
 given to their own pool at start-up, or the calling thread must not block on the driver's
 allocation lock. For them the library keeps the scratch of the tensor-core linear (the bf16
 planes of the activations and a status word) in a fixed device array. This file checks, through
-the C ABI, that the variant computes exactly what fc_q8_0_linear_dev computes, twice in a row
-(the array keeps the previous call's contents), and that it refuses sizes beyond the array.
+the C ABI, that the variant computes exactly what fc_q8_0_linear_dev computes on bf16 planes, twice in a row
+(the array keeps the previous call's contents), the same to 2^-16 from the rows on where the latter takes f16 planes, and that
+it refuses sizes beyond the array.
 
 Collected last on purpose: a run that stops at the first failure has then already run every
 other test."""
@@ -42,6 +43,25 @@ def test_noalloc_linear_matches_the_allocating_entry_point_twice():
         assert torch.equal(got, want), f"call {call}: max abs diff {(got - want).abs().max().item():.3e}"
         ref = x.double() @ torch.from_numpy(synth.q8_0_dequantize(wq, n * k).reshape(n, k)).double().cuda().T + bias.double()
         assert (got.double() - ref).abs().max().item() <= 1e-4 * ref.abs().max().item()
+    qw.close()
+
+
+@pytest.mark.parametrize("m,n,k", [(512, 300, 1024), (1024, 1000, 2048)])
+def test_noalloc_linear_from_the_rows_on_where_the_other_takes_f16_planes(m, n, k):
+    """Two bf16 planes leave 2^-17 of an activation, two f16 planes 2^-23, and either sum less than 2^-17 of the terms."""
+    import torch
+
+    wq = synth.q8_0_quantize(synth.Rng(5).normal(n * k, 0.02))
+    qw = fcb.QWeight(wq, n, k)
+    x = torch.from_numpy(synth.Rng(7).normal(m * k, 1.0).reshape(m, k)).cuda()
+    want, got = torch.zeros(m, n, device="cuda"), torch.zeros(m, n, device="cuda")
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    qw.linear_dev(x.data_ptr(), None, want.data_ptr(), m, fcb.FC_MATH_BF16X3, stream)
+    qw.linear_dev_noalloc(x.data_ptr(), None, got.data_ptr(), m, stream)
+    torch.cuda.synchronize()
+    terms = x.double().abs() @ torch.from_numpy(np.abs(synth.q8_0_dequantize(wq, n * k).reshape(n, k))).double().cuda().T
+    assert ((got - want).abs().double() <= 2.0**-16 * terms).all()
+    assert not torch.equal(got, want)
     qw.close()
 
 
