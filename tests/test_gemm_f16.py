@@ -17,22 +17,27 @@ def _weight(n, k, seed, scales=None):
 
 
 def _bound(x, w, k):
-    # per element, of sum |x||w|: 48 truncations of 2^-23 in a group of 256 k, one rounding a group, three plane terms and the bias
+    # per element, of sum |x||w|: 24 truncations of 2^-23 in a group (up to 384 k, then 192), one rounding a group, three plane terms and the
+    # bias; the small terms' truncations are 2^-11 of that
     s = np.abs(x).astype(np.float64) @ np.abs(w).T
-    return (48 * 2.0**-23 + (k / 256 + 6) * 2.0**-24) * s
+    return (24 * 2.0**-23 + (k / 192 + 6) * 2.0**-24) * s
 
 
 def _run(qw, x, n, bias=None):
     import torch
     xd, y = torch.from_numpy(x).cuda(), torch.full((x.shape[0], n), float("nan"), device="cuda")
     b = torch.from_numpy(bias).cuda() if bias is not None else None
+    fcb.take_launch_count()
     qw.linear_dev(xd.data_ptr(), b.data_ptr() if b is not None else None, y.data_ptr(), x.shape[0], fcb.FC_MATH_BF16X3)
+    # small products run on f32 FMA, in one launch; the tensor core's have a launch for the planes
+    small = qw.k <= 3072 and x.shape[0] * n * ((qw.k + 255) // 256 * 256) < 2**25
+    assert fcb.take_launch_count() == (1 if small else 2)
     torch.cuda.synchronize()
     return y.cpu().numpy()
 
 
 @pytest.mark.parametrize("m,n,k", [(512, 1, 64), (513, 127, 128), (575, 129, 320), (769, 257, 256), (1024, 1000, 768), (2305, 300, 832),
-                                   (4096, 2048, 64)])
+                                   (4096, 2048, 64), (131072, 1, 64), (2050, 1, 4096), (1600, 127, 3136), (2080, 128, 192)])
 def test_matches_64_bit_sums(m, n, k):
     raw, w = _weight(n, k, 1)
     x = np.random.RandomState(2).standard_normal((m, k)).astype(np.float32)
@@ -41,11 +46,14 @@ def test_matches_64_bit_sums(m, n, k):
     want = x.astype(np.float64) @ w.T + bias
     got = _run(qw, x, n, bias)
     assert (np.abs(got - want) <= _bound(x, w, k) + 2.0**-24 * np.abs(want)).all()
+    # no bf16 planes, which leave 2.5e-6
+    assert np.linalg.norm(got - want) < 1e-6 * np.linalg.norm(want)
     qw.close()
 
 
-def test_rows_of_any_magnitude_and_their_neighbours():
-    n, k, m = 160, 128, 600
+@pytest.mark.parametrize("n", [160, 264])                # on f32 FMA, and on f16 planes
+def test_rows_of_any_magnitude_and_their_neighbours(n):
+    k, m = 128, 600
     raw, w = _weight(n, k, 4)
     x = np.random.RandomState(5).standard_normal((m, k)).astype(np.float32)
     x *= np.float32(10.0) ** np.random.RandomState(6).randint(-30, 31, (m, 1)).astype(np.float32)
@@ -63,10 +71,11 @@ def test_rows_of_any_magnitude_and_their_neighbours():
     qw.close()
 
 
+@pytest.mark.parametrize("n", [130, 258])                # on f32 FMA, and on the tensor core
 @pytest.mark.parametrize("scales", [(2.0**-24, 3 * 2.0**-24, 1.5 * 2.0**-14), (511.5, 400.0), (512.0, 600.0, 1e-3)])
-def test_scales_at_the_ends_of_f16(scales):
+def test_scales_at_the_ends_of_f16(scales, n):
     """Subnormal scales, the largest that f16 planes hold, and scales beyond (which the level kernel takes)."""
-    n, k, m = 130, 192, 512
+    k, m = 192, 512
     raw, w = _weight(n, k, 8, np.array(scales))
     x = np.random.RandomState(9).standard_normal((m, k)).astype(np.float32)
     qw = fcb.QWeight(raw, n, k)
@@ -74,6 +83,8 @@ def test_scales_at_the_ends_of_f16(scales):
     # the level kernel splits x to 2^-17, each term of a product once more
     bound = _bound(x, w, k) if max(scales) < 512 else 2.0**-16 * (np.abs(x).astype(np.float64) @ np.abs(w).T)
     assert (np.abs(got - want) <= bound).all()
+    # on f16 planes if these hold the weights, else on levels and bf16 planes
+    assert n < 258 or (np.linalg.norm(got - want) < 1e-6 * np.linalg.norm(want)) == (max(scales) < 512)
     qw.close()
 
 
