@@ -473,7 +473,7 @@ def main():
     ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--score-math", choices=["bf16x3", "fp32"], default="bf16x3",
-                    help="math mode of the scoring GEMMs: activations as two bf16 planes, or as three (exact)")
+                    help="math mode of the scoring GEMMs: two 16-bit planes of the activations, or three (exact)")
     args = ap.parse_args()
     rank = int(os.environ.get("RANK", "0"))
     local = int(os.environ.get("LOCAL_RANK", "0"))
@@ -768,8 +768,8 @@ def main():
             "n_gpus": world, "steps": args.score_steps, "ms_per_step": step_ms, "scaling": "strong" if world > 1 else "n/a",
             "config": {"workload": "configs[2]: %d sequences x %d ids, full-window prefill, per-token log-probs, %d windows per forward"
                        % (N_SEQ, SEQ_LEN, bw),
-                       "math": "linear layers: tcgen05 kind::f16, exact weight levels, f32 activations as %d bf16 planes, f32 accumulate"
-                               % (2 if args.score_math == "bf16x3" else 3)},
+                       "math": "linear layers: tcgen05 kind::f16, f32 accumulate, " + ("weights and activations as two f16 planes"
+                               if args.score_math == "bf16x3" else "exact weight levels, f32 activations as three bf16 planes")},
             "dtype": "bf16x3" if args.score_math == "bf16x3" else "f32",
             "e2e": {"value": positions / e2e_s, "unit": "positions/s", "h2d_bytes_per_step": per * SEQ_LEN * 4,
                     "d2h_bytes_per_step": per * SEQ_LEN * 4 + per * 24},

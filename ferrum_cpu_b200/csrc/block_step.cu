@@ -31,7 +31,7 @@ namespace fc {
 
 namespace {
 
-constexpr int T = 384, W = T / 32;             // threads and warps of a CTA (512 with a row of 1024: 339 us a token, 384 326)
+constexpr int T = 384, W = T / 32;             // threads and warps of a CTA (512 with a row of 1024: 339 us a token, 384 317)
 constexpr int MAX_D = 1024;
 constexpr int MAX_PARTS = 16;
 constexpr int MAX_SLICE = 512;                 // hidden units of a cluster

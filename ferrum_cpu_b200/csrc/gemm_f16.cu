@@ -36,8 +36,8 @@
 // takes few rows. The order of a row's sums depends on K alone, so a row's result does not depend on the rows beside it.
 //
 // Bound: the tensor pipe at the clock the power limit leaves. A stage of a 256-row tile takes 1547 cycles, its MMAs 1536. In a loop of
-// their own, with the planes made (levels in gemm_tc.cu): 4096 x 1024 x 4096 73 us (109), 32768 x 768 x 2304 239 us = 1.46 PFLOP/s executed
-// (348), 32768 x 3072 x 768 322 us (450).
+// their own, with the planes made (levels in gemm_tc.cu): 4096 x 1024 x 4096 72 us (109), 32768 x 768 x 2304 234 us = 1.49 PFLOP/s executed
+// (348), 16384 x 3072 x 768 161 us.
 //
 // Every wait is bounded; a wait that runs out raises the status word and all roles leave, in whatever order they learn of it.
 #include <algorithm>
@@ -578,8 +578,13 @@ int launch_f16(const F16Mat& w, const Planes& x, F16Args a, int M, cudaStream_t 
 }  // namespace
 
 // A call of its own pays for turning the weight into planes, 5 bytes a weight, and has no split of K for few rows. Us on this kernel
-// (on the levels): 512 rows x 1024 x 2048 18.6 (20.8), x 4096 24.8 (24.8); 256 rows 17.1 (18.7), 20.8 (20.9); K = 3072, N = 1024: 512 rows
-// 32.3 (26.8), 1024 rows 33.0 (37.2), 1536 rows 43.6 (49.3); N = 4096: 512 rows 53.7 (47.4), 1024 rows 82 (81), 1536 rows 103 (119).
+// (on the levels), back to back, for N = 512 / 1024 / 4096:
+//     K = 1024    512 rows 16.6 / 18.5 / 24.8 (14.5 / 16.6 / 22.8)    768 rows 16.7 / 18.6 / 28.9 (16.6 / 20.2 / 35.1)
+//     K = 2048    768 rows 26.8 / 26.8 / 45.3 (20.6 / 26.9 / 57.2)   1024 rows 26.9 / 26.8 / 55.3 (21.6 / 30.8 / 59.6)
+//     K = 3072   1024 rows 36.8 / 36.8 / 77.9 (24.8 / 36.0 / 81.5)   1536 rows 35.1 / 43.2 / 103 (35.1 / 46.3 / 118)
+//     K = 4096   1536 rows 45.3 / 53.7 / 140 (41.2 / 57.6 / 155)     2048 rows 51.6 / 57.7 / 185 (45.4 / 61.7 / 168)
+// The line lies where most shapes have gone over. Near it this kernel may be the slower one by up to 25 % (small N, whose levels split K), and
+// large N would gain by it from fewer rows on; where both are close its results are, which are five times nearer to 64 bits.
 bool f16_rows(int K, int M) { return M >= 512 && M >= K / 2; }
 
 int launch_f16_planes(const float* x, int M, int K, const Planes& out, float* row_inv, const QMat& w, const F16Mat& planes, unsigned* norms, cudaStream_t st) {

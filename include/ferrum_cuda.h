@@ -41,7 +41,9 @@ extern "C" {
 #define FC_MATH_FP32 0      /* tcgen05 kind::f16, f32 accumulate: exact int8 levels against three bf16 planes of the activations (their f32
                                value exactly) */
 #define FC_MATH_BF16X3 1    /* the same against two bf16 planes (2^-17 relative), or exact f16 planes of the weights against two f16 planes of
-                               the activations, with sums kept longer in the tensor core (about 4e-7 of a product) */
+                               the activations, with sums kept longer in the tensor core (about 4e-7 of a product): in a linear with
+                               a scale for every row (elements below 2^-33 of its largest keep less than 2^-17), in a model where a
+                               layer's one scale leaves all elements 2^-17 */
 
 /* Dimensions of a gpt2-architecture GGUF (ferrum_core/src/loader/gpt2.rs:201-215). */
 typedef struct fc_config {
